@@ -270,6 +270,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   // (local attention only: over a whole sentence the second window costs the attention kernel more than the GEMM it replaces)
   { const char* pe = std::getenv("LINMT_ATT_FOLD"); att_fold_ = att_merge_ && o.attention_mode == LINMT_ATT_LOCAL_P_GENERAL && !(pe && std::atoi(pe) == 0); }
   { const char* pe = std::getenv("LINMT_TC_PERSIST"); persist_ = !(pe && std::atoi(pe) == 0); }
+  { const char* pe = std::getenv("LINMT_TC_ROWS"); rows_ = !(pe && std::atoi(pe) == 0); }
   { const char* pe = std::getenv("LINMT_TC_PAIR"); pair_ = !(pe && std::atoi(pe) == 0); }
   { const char* pe = std::getenv("LINMT_PDL"); pdl_ = use_tc_ && !(pe && std::atoi(pe) == 0); }   // LINMT_PDL=0: test knob
   // fp32 weights on the tensor cores: the f16 pair by default (3 partial products), bf16 planes on request

@@ -7,6 +7,7 @@
 #include "engine.h"
 #include "gemm_tc.cuh"
 #include "gemm_tc_pair.cuh"
+#include "gemm_tc_rows.cuh"
 #include "step_kernels.cuh"
 
 namespace linmt {
@@ -135,6 +136,37 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   const long ntile_cols = (N + bn - 1) / bn;
   const bool pair = ppair || (pair_ && fmt_ == 1 && nt == 2 && bk == 64 && splits == 1 && mt >= 2 && bn % 16 == 0 &&
                     tc::make_shape(bn, nt, bk, fmt_).stages < 3 && (long)((mt + 1) & ~1) * ntile_cols <= n_sm_ && ws_parts_ == 1);
+  // Few rows: the weight-streaming kernel (gemm_tc_rows.cuh), where the rows are the narrow side of the MMA.  Its gain
+  // shrinks as the rows fill the 128-row tile (gate product, us against this file's one-tile kernel: 8.7 / 13.8 at 12
+  // rows, 10.2 / 14.8 at 32, 11.4 / 15.8 at 64; bf16 6.3 / 13.0 at 12, 9.0 / 13.0 at 64); a product of many column
+  // tiles and one k slice is finished by too few warps for more than 48 rows (vocabulary 12.7 / 14.7 us at 12 rows,
+  // 14.7 / 15.1 at 48, 17.3 / 15.1 at 64).
+  {
+    tc::RowsShape rs;
+    if (rows_ && ws_parts_ == 1 && M <= tc::kRowsMax && (M <= 48 || N <= 128 * n_sm_) && tc::make_shape_rows(M, N, K, nt, fmt_, n_sm_, drain >= K / 32, &rs)) {
+      tc::Planes a = A;
+      for (int t = 0; t < 3; ++t) if (a.p[t]) a.p[t] += a_col0;
+      const CUtensorMap* xm = b_maps(a, a_rows_cap, K, rs.rp, 64);
+      const CUtensorMap* wm = b_maps(W, N, K, tc::BM, 64);
+      if (!xm || !wm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
+      tc::TmapSet tm;
+      std::memcpy(tm.a, xm, sizeof(tm.a));
+      std::memcpy(tm.b, wm, sizeof(tm.b));
+      rs.pdl = (pdl_ && pdl_gemm_) ? 1 : 0;
+      if constexpr (Epi::kHasPmax) {
+        if (e.pmax) {      // block maxima of 32 columns
+          const int slots = 4 * ((N + tc::BM - 1) / tc::BM);
+          if (slots > e.pmax_ld) { e.pmax = nullptr; pmax_slots_ = 0; }
+          else pmax_slots_ = slots;
+        }
+      }
+      if (nt == 2) CK((tc::launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream)));
+      else if (fmt_ == 1) CK((tc::launch_gemm_tc_rows<1, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream)));
+      else CK((tc::launch_gemm_tc_rows<1, 0, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream)));
+      LAUNCHED();
+      return LINMT_OK;
+    }
+  }
   const CUtensorMap* am = a_maps(A, a_col0, a_rows_cap, K, bk);
   const CUtensorMap* bm = b_maps(W, N, K, pair ? bn / 2 : bn, bk);
   if (!am || !bm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");

@@ -493,6 +493,41 @@ struct TcEpiLstm {
       }
     __syncwarp();
   }
+  // Row form (gemm_tc_rows.cuh): a lane holds four consecutive accumulator columns = the gates of one hidden unit.
+  // preload() reads what does not depend on the accumulator, so that it can be in flight while the product runs.
+  struct Pre { float4 x, b; float c; };
+  __device__ __forceinline__ Pre preload(int row, int col) const {
+    Pre p;
+    p.b = *reinterpret_cast<const float4*>(bias + col);
+    p.x = xw ? *reinterpret_cast<const float4*>(xw + (size_t)x_row(row) * x_ld + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    p.c = c_prev[(size_t)c_src_row(row) * ldc + (col >> 2)];
+    return p;
+  }
+  __device__ __forceinline__ void finish_row(bool valid, int row, int col, int /*lane*/, const float4& v, const Pre& p) const {
+    if (!valid) return;
+    const int j = col >> 2;
+    const size_t i1 = (size_t)row * h_out1.ld + h1_col0 + j, i2 = (size_t)row * h_out2.ld + h2_col0 + j;
+    if (row_len == nullptr || pos < row_len[row]) {
+      const float gi = sigmoid_fast((v.x + p.x.x) + p.b.x);
+      const float gf = sigmoid_fast((v.y + p.x.y) + p.b.y);
+      const float gg = tanh_fast((v.z + p.x.z) + p.b.z);
+      const float go = sigmoid_fast((v.w + p.x.w) + p.b.w);
+      const float c = gf * p.c + gi * gg;
+      const float h = go * tanh_fast(c);
+      c_out[(size_t)row * ldc + j] = c;
+      split_store(h_out1, nt, i1, h);
+      if (h_out2.p[0]) split_store(h_out2, nt, i2, h);
+      if (h_f32) h_f32[(size_t)row * hf_row_stride + j] = planes_value(h, nt);
+    } else {
+      c_out[(size_t)row * ldc + j] = p.c;
+      const size_t ip = (size_t)row * h_prev.ld + hp_col0 + j;
+      for (int t = 0; t < nt; ++t) {
+        const __nv_bfloat16 hv = h_prev.p[t][ip];
+        h_out1.p[t][i1] = hv;
+        if (h_out2.p[0]) h_out2.p[t][i2] = hv;
+      }
+    }
+  }
 };
 
 // out = tanh(acc [+ add] + bias) as bf16 planes (the attentional state).  `add` is an optional fp32 term per
@@ -517,6 +552,18 @@ struct TcEpiBiasTanh {
       }
       split_store4(out, nt, idx + 4 * q, tanh_fast(a.x + b.x), tanh_fast(a.y + b.y), tanh_fast(a.z + b.z), tanh_fast(a.w + b.w));
     }
+  }
+  struct Pre { float4 a, b; };   // row form, see TcEpiLstm
+  __device__ __forceinline__ Pre preload(int row, int col) const {
+    Pre p;
+    p.b = *reinterpret_cast<const float4*>(bias + col);
+    p.a = add ? *reinterpret_cast<const float4*>(add + (size_t)row * ld_add + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return p;
+  }
+  __device__ __forceinline__ void finish_row(bool valid, int row, int col, int /*lane*/, const float4& v, const Pre& p) const {
+    if (!valid) return;
+    split_store4(out, nt, (size_t)row * out.ld + col_off + col, tanh_fast((v.x + p.a.x) + p.b.x), tanh_fast((v.y + p.a.y) + p.b.y),
+                 tanh_fast((v.z + p.a.z) + p.b.z), tanh_fast((v.w + p.a.w) + p.b.w));
   }
 };
 
@@ -623,6 +670,31 @@ struct TcEpiF32 {
   __device__ __forceinline__ void block(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, int slot) const {
     const float m = stage_store(row0, lane, M, col_first, nch, v, sbuf, kEpiScratchStride);
     pmax_store(row0 + lane, M, slot, m);
+  }
+  // Row form, see TcEpiLstm; a warp holds 32 columns of four rows (lane & 3 = row), the block maxima are theirs.
+  struct Pre { float4 b; };
+  __device__ __forceinline__ Pre preload(int, int col) const {
+    Pre p;
+    p.b = bias ? *reinterpret_cast<const float4*>(bias + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return p;
+  }
+  __device__ __forceinline__ void finish_row(bool valid, int row, int col, int lane, const float4& v, const Pre& p) const {
+    float m = -INFINITY;
+    if (valid) {
+      float4 r = make_float4(v.x + p.b.x, v.y + p.b.y, v.z + p.b.z, v.w + p.b.w);
+      if (col < split) { r.x = tanh_fast(r.x); r.y = tanh_fast(r.y); r.z = tanh_fast(r.z); r.w = tanh_fast(r.w); }
+      if (out16) {
+        r.x = __half2float(__float2half_rn(r.x)); r.y = __half2float(__float2half_rn(r.y));
+        r.z = __half2float(__float2half_rn(r.z)); r.w = __half2float(__float2half_rn(r.w));
+      }
+      store4((size_t)row * ld + col, r);
+      m = max4(m, r, col);
+    }
+    if (pmax) {
+#pragma unroll
+      for (int o = 16; o > 2; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if (lane < 4 && valid) pmax[(size_t)row * pmax_ld + (col >> 5)] = m;
+    }
   }
 };
 

@@ -8,6 +8,7 @@
 #include "gemm_simt.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc_pair.cuh"
+#include "gemm_tc_rows.cuh"
 #include "step_kernels.cuh"
 
 namespace {
@@ -81,11 +82,21 @@ int linmt_k_gemm(const float* X, const float* W, float* Y, int32_t R, int32_t K,
     const bool pair = !(pair_env && std::atoi(pair_env) == 0) && fmt == 1 && nt == 2 && bk == 64 && splits == 1 && mt >= 2 && bn % 16 == 0 &&
                       tc::make_shape(bn, nt, bk, fmt).stages < 3 && (long)((mt + 1) & ~1) * ((Np + bn - 1) / bn) <= n_sm &&
                       tc::max_resident_pairs<2, 64, 1, tc::TcEpiF32>() > 0;
-    for (int t = 0; t < nt; ++t)
+    // ... and its rule for few rows (LINMT_TC_ROWS=0 keeps the one-tile kernel)
+    tc::RowsShape rs;
+    const char* rows_env = std::getenv("LINMT_TC_ROWS");
+    const bool few = !(rows_env && std::atoi(rows_env) == 0) && (R <= 48 || Np <= 128 * n_sm) && tc::make_shape_rows(R, Np, Kp, nt, fmt, n_sm, false, &rs);
+    if (few) {
+      for (int t = 0; t < nt; ++t)
+        if (!tc::make_tmap(&tm.a[t], A.p[t], R, Kp, Kp, rs.rp, 64) || !tc::make_tmap(&tm.b[t], B.p[t], Np, Kp, Kp, tc::BM, 64)) return LINMT_ECUDA;
+    }
+    for (int t = 0; t < nt && !few; ++t)
       if (!tc::make_tmap(&tm.b[t], B.p[t], Np, Kp, Kp, pair ? bn / 2 : bn, bk)) return LINMT_ECUDA;
     tc::Shape sh = pair ? tc::make_shape_pair(bn, nt, bk, fmt) : tc::make_shape(bn, nt, bk, fmt);
     sh.splits = splits;
-    cudaError_t le = pair ? tc::launch_gemm_tc_pair<2, 64, 1, tc::TcEpiF32>(tm, R, Np, Kp, sh, e, derr.as<int>(), 0, nullptr, nullptr)
+    cudaError_t le = few && nt == 2 ? tc::launch_gemm_tc_rows<2, 1, tc::TcEpiF32>(tm, R, Np, Kp, rs, e, derr.as<int>(), 0)
+                   : few ? tc::launch_gemm_tc_rows<1, 0, tc::TcEpiF32>(tm, R, Np, Kp, rs, e, derr.as<int>(), 0)
+                   : pair ? tc::launch_gemm_tc_pair<2, 64, 1, tc::TcEpiF32>(tm, R, Np, Kp, sh, e, derr.as<int>(), 0, nullptr, nullptr)
                           : tc::launch_gemm_tc(tm, R, Np, Kp, sh, e, derr.as<int>(), 0, dws.as<float>(), dcnt.as<int>());
     KCK(le);
     KCK(cudaDeviceSynchronize());

@@ -90,3 +90,19 @@ def test_gemm_on_cta_pairs_vs_float64_and_one_tile(cuda_lib):
     # a last row tile that is partly empty (700 = 5 x 128 + 60 rows)
     Y5 = decoder.k_gemm(X[:700], W, "tensor", "fp32")
     assert (np.abs(Y5 - ref[:700]) <= 1e-6 * scale[:700] + 1e-7).all()
+
+
+@pytest.mark.parametrize("prec,tol", [("fp32", 1e-6), ("bf16", 4e-3)])
+@pytest.mark.parametrize("R,K,N", [(1, 64, 128), (3, 200, 130), (16, 2048, 4096), (17, 1000, 3000), (32, 130, 20000), (33, 2048, 4096),
+                                   (49, 700, 20000), (64, 1024, 391), (65, 256, 512)])
+def test_gemm_few_rows_vs_float64(cuda_lib, R, K, N, prec, tol):
+    """The weight-streaming product for up to 64 rows: edges of its row groups (4), MMA widths (16), of the change from
+    half to whole SMs (33) and to the other kernels (49 rows of many columns, 65), K slices of unequal length."""
+    from linmt_b200 import decoder
+    rng = np.random.default_rng(R + K + N)
+    X = rng.uniform(-1, 1, (R, K)).astype(np.float32)
+    W = rng.uniform(-0.08, 0.08, (K, N)).astype(np.float32)
+    Y = decoder.k_gemm(X, W, "tensor", prec)
+    ref = X.astype(np.float64) @ W.astype(np.float64)
+    scale = np.abs(X).astype(np.float64) @ np.abs(W).astype(np.float64)
+    assert (np.abs(Y - ref) <= tol * scale + 1e-7).all(), float((np.abs(Y - ref) / scale).max())
