@@ -18,6 +18,7 @@
 #include <thread>
 
 #include "gemm_simt.cuh"
+#include "gemm_tc_rows.cuh"
 #include "step_kernels.cuh"
 
 namespace linmt {
@@ -246,6 +247,7 @@ int Engine::alloc_state(DevState& s) {
   CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));   // rows past a sentence's end are never written, but read as GEMM operand rows by the fold
   if (att_fold_) DA(s.hs_wc1, (size_t)B * opt.max_src_len * Hp);
   DA(s.enc_x, (size_t)B * Hp);
+  if (enc_rows_) DA(s.enc_pre, (size_t)enc_rows_ * 4 * Hp);
   for (int i = 0; i < 2; ++i) {
     s.enc_h[i].resize(L); s.enc_c[i].resize(L);
     for (int l = 0; l < L; ++l) { DA(s.enc_h[i][l], (size_t)B * Hp); DA(s.enc_c[i][l], (size_t)B * Hp); }
@@ -318,6 +320,11 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
     CK(cudaMemset(d_splitk_counters_, 0, sizeof(int) * kSplitKMaxTiles));
     if (pair_ && !pairs_available()) pair_ = false;   // (a device that cannot co-schedule two such CTAs keeps the one-tile kernels)
   }
+  // panels of the layer-by-layer encoder: all positions of a batch if that is at most 16384 rows (0.27 GB of input parts)
+  if (use_tc_ && rows_ && (nt_ == 1 || fmt_ == 1)) {
+    const int nb = std::min(B, tc::kRowsMax);
+    enc_rows_ = std::min(opt.max_src_len * nb, std::max(16384, nb));
+  }
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);
   for (int i = 0; i < nm; ++i) {
     int rc = pack_model(blobs[i], models_[i]);
@@ -333,11 +340,14 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   DA(d_tok_, R); DA(d_parent_, R); DA(d_score_, R);
   DA(d_hist_tok_, (size_t)Tcap * R); DA(d_hist_parent_, (size_t)Tcap * R);
   DA(d_fin_t_, (size_t)B * fin_cap); DA(d_fin_b_, (size_t)B * fin_cap); DA(d_fin_n_, B);
+  DA(d_rows_done_, B);
+  CK(cudaMemset(d_rows_done_, 0, sizeof(int) * B));
   DA(d_fin_score_, (size_t)B * fin_cap); DA(d_fin_final_, (size_t)B * fin_cap);
   if (nm > 1) DA(d_combined_, (size_t)R * Vp);
   DA(d_cand_idx_, (size_t)R * kk); DA(d_cand_logp_, (size_t)R * kk); DA(d_eos_logp_, R); DA(d_row_stats_, 2 * (size_t)R);
   pmax_ld_ = 4 * ((Vp + 47) / 48) + 4;   // four column blocks per tile, tiles at least 48 wide
   DA(d_pmax_, (size_t)R * pmax_ld_);
+  DA(d_psum_, (size_t)std::min(R, tc::kRowsMax) * pmax_ld_);
   if (o.print_info) {
     DA(d_rec_align_, (size_t)Tcap * R * rec_win); DA(d_rec_lo_, (size_t)Tcap * R); DA(d_rec_vit_, (size_t)Tcap * R);
   }
@@ -351,6 +361,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
 // sentences of the batch advance together, one position per round; a row stops changing
 // once its sentence is consumed.  Top-layer states go to hs[b][pos].
 int Engine::run_encoder(int n, int Smax) {
+  hs_sent_ = opt.max_src_len; hs_pos_ = 1;
   for (int mi = 0; mi < n_models; ++mi) {
     DevModel& m = models_[mi];
     DevState& s = states_[mi];
@@ -474,11 +485,12 @@ int Engine::launch_attention(int mi, int t, int rows, const float* u_alt, float*
   DevModel& m = models_[mi];
   DevState& s = states_[mi];
   const int ldp = att_merge_ ? 3 * Hp : 2 * Hp;
-  const size_t smem = sizeof(float) * (win + 8);
   // fold: the weighted sum runs over W_c1 . hs and the kernel writes htilde (ctx_planes = the htilde panel)
   const AttFold af = fold ? AttFold{s.hs_wc1, s.proj + 2 * Hp, 3 * Hp, m.att_bout} : AttFold{nullptr, nullptr, 0, nullptr};
-  CK(tc::launch_k(pdl_, attention_kernel, dim3(rows), dim3(256), smem, stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
-                  (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, k, (int)opt.max_src_len, (int)opt.attention_mode,
+  const bool wide = rows <= n_sm_;   // a CTA of 1024 threads per SM
+  CK(tc::launch_k(pdl_, wide ? attention_kernel<1024> : attention_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256),
+                  wide ? attention_smem<1024>(win) : attention_smem<256>(win), stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
+                  (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, k, hs_sent_, hs_pos_, (int)opt.attention_mode,
                   (int)opt.attention_d, win, ra, rl, rv, ctx_planes, nt, rec_win, ens_member_code(mi), at, af));
   LAUNCHED();
   return LINMT_OK;
@@ -493,6 +505,8 @@ int Engine::step_tail(int t, int rows) {
     trace_dev_.logits = (n_models == 1) ? s.logits : d_combined_;
     trace_dev_.ld_logits = Vp;
     trace_dev_.row_stats = d_row_stats_;
+    SelectArgs sel{BeamState{d_tok_, d_score_, d_parent_, d_hist_tok_, d_hist_parent_, d_fin_t_, d_fin_b_, d_fin_score_, d_fin_n_, fin_cap, R},
+                   d_steps_, d_orig_, d_rows_done_, t, k, opt.penalty, opt.diversity, TraceDev{}};
     if (n_models == 1) {
       if (int rc = kt(KC_SOFTMAX)) return rc;
       TopkRefine rf{};
@@ -507,8 +521,14 @@ int Engine::step_tail(int t, int rows) {
         rf.eps_coef = 1.1f * (1.0f / 1024.0f) * m0.voc_wnorm_max;
       }
       if (refine_) trace_dev_.rf = rf;
-      CK(launch_softmax_topk(s.logits, Vp, V, kk, rows, o, 1, stream, pdl_, d_pmax_, pmax_ld_, pmax_slots_, refine_ ? &rf : nullptr,
-                             logits16_ ? s.logits16 : nullptr));
+      sel.tr = trace_dev_;
+      if (pblocks_) {
+        const LogitBlocks bl{d_pmax_, d_psum_, pmax_ld_, pmax_slots_};
+        CK(tc::launch_k(pdl_, topk_blocks_kernel, dim3(rows), dim3(kTopkBlocksThreads), topk_blocks_smem(bl.n, rf.a0 ? rf.K : 0), stream,
+                        (const float*)s.logits, logits16_ ? (const __half*)s.logits16 : (const __half*)nullptr, Vp, V, kk, o, 1, bl, rf, sel));
+      } else
+        CK(launch_softmax_topk(s.logits, Vp, V, kk, rows, o, 1, stream, pdl_, d_pmax_, pmax_ld_, pmax_slots_, refine_ ? &rf : nullptr,
+                               logits16_ ? s.logits16 : nullptr, sel));
     } else {
       // EnsembleFactory::EnsemblesModels (src/decoder.h:1910-1931): mean of the members'
       // probabilities, renormalised -- written as log(mean p) so that the log-softmax of the
@@ -520,19 +540,12 @@ int Engine::step_tail(int t, int rows) {
       CK(tc::launch_k(pdl_, ensemble_combine_kernel, dim3(rows), dim3(256), 0, stream, er, Vp, V, (int)opt.ensemble_mode, d_combined_));
       LAUNCHED();
       if (int rc = kt(KC_SOFTMAX)) return rc;
-      CK(launch_softmax_topk(d_combined_, Vp, V, kk, rows, o, opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0, stream, pdl_));
+      sel.tr = trace_dev_;
+      CK(launch_softmax_topk(d_combined_, Vp, V, kk, rows, o, opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0, stream, pdl_, nullptr, 0, 0, nullptr, nullptr, sel));
     }
     LAUNCHED();
   }
-  {
-    BeamState bs{d_tok_, d_score_, d_parent_, d_hist_tok_, d_hist_parent_, d_fin_t_, d_fin_b_, d_fin_score_, d_fin_n_, fin_cap, R};
-    const size_t smem = (size_t)k * kk * 24 + 16;
-    if (int rc = kt(KC_SELECT)) return rc;
-    CK(tc::launch_k(pdl_, beam_select_kernel, dim3(n_act), dim3(256), smem, stream, bs, (const int32_t*)d_cand_idx_, (const float*)d_cand_logp_,
-                    (const float*)d_eos_logp_, (const int32_t*)d_steps_, (const int32_t*)d_orig_, t, k, opt.penalty, opt.diversity, trace_dev_));
-    LAUNCHED();
-    if (int rc = kt(KC_END)) return rc;
-  }
+  if (int rc = kt(KC_END)) return rc;
   CK(cudaGetLastError());
   stats.decoder_row_steps += rows;
   stats.sentence_steps += n_act;

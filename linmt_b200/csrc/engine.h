@@ -50,6 +50,9 @@ struct TcState {
   tc::Planes panel_ht{};             // [R][Hp]   htilde
   tc::Planes hs_planes{};            // [B * max_src][Hp]  the encoder's top states as operand planes (attention fold)
   std::vector<tc::Planes> encp[2];   // [L] x [B][2Hp]  below | h_prev, double buffered over positions
+  // encoder layer by layer (few sentences): block p of n rows = the state after p positions of the chunk
+  tc::Planes enc_in{};               // [rows][Hp] the first layer's input
+  std::vector<tc::Planes> enc_seq;   // [L] x [rows + n][Hp]
 };
 
 struct DevState {
@@ -62,6 +65,7 @@ struct DevState {
   float* hs = nullptr;                               // [B][max_src][Hp]
   float* hs_wc1 = nullptr;                           // [B][max_src][Hp]  W_c1 . hs (tensor path with the attention fold)
   float* enc_x = nullptr;                            // [B][Hp]
+  float* enc_pre = nullptr;                          // [rows][4Hp]  W_x . input of every position (encoder layer by layer)
   std::vector<float*> enc_h[2], enc_c[2];            // [L] x [B][Hp], double buffered
 };
 
@@ -109,6 +113,7 @@ class Engine {
   int run_encoder(int n, int Smax);
   int run_decoder_step(int mi, int t, int rows);
   int run_encoder_tc(int n, int Smax);
+  int run_encoder_layers_tc(int n, int Smax);   // few sentences: layer by layer
   int run_decoder_step_tc(int mi, int t, int rows);
   int step_tail(int t, int rows);
   bool pairs_available();   // clusters of two GEMM CTAs can be scheduled on the current device (engine_tc.cu)
@@ -121,7 +126,7 @@ class Engine {
   const CUtensorMap* a_maps(const tc::Planes& p, int col0, int rows_cap, int K, int bk);
   const CUtensorMap* b_maps(const tc::Planes& p, int rows, int K, int bn, int bk);
   template <class Epi>
-  int tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e, int nt = 0, int drain = 0);
+  int tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e, int nt = 0, int drain = 0, int x_row0 = 0);
 
   bool use_tc_ = false;
   // encoder wavefront: one stream per layer, a small ring of events per layer
@@ -153,6 +158,10 @@ class Engine {
   std::map<std::tuple<const void*, int, int, int, int>, std::array<CUtensorMap, 3>> tmap_cache_;
 
   const int32_t* cur_ids_ = nullptr;
+  // row of the encoder states of sentence b after position p: b * hs_sent_ + p * hs_pos_
+  int hs_sent_ = 0, hs_pos_ = 1;
+  int enc_rows_ = 0;                    // rows (positions x sentences) the layer-by-layer encoder takes at a time
+  int enc_final_row_ = -1;              // its final states: first row in enc_seq (-1: the other encoder ran)
   TraceDev trace_dev_{};
   size_t trace_pt_member_stride_ = 0;   // floats between two members' p_t records in the device trace buffer
   int enc_final_buf_ = 0;
@@ -170,12 +179,15 @@ class Engine {
   int32_t *d_tok_ = nullptr, *d_parent_ = nullptr, *d_hist_tok_ = nullptr, *d_hist_parent_ = nullptr;
   float* d_score_ = nullptr;
   int32_t *d_fin_t_ = nullptr, *d_fin_b_ = nullptr, *d_fin_n_ = nullptr;
+  int32_t* d_rows_done_ = nullptr;   // per sentence: rows whose softmax of this step is done (SelectArgs)
   float *d_fin_score_ = nullptr, *d_fin_final_ = nullptr;
   float* d_combined_ = nullptr;  // [R][Vp] ensemble-combined log-values (n_models > 1)
   int32_t* d_cand_idx_ = nullptr;
   float *d_cand_logp_ = nullptr, *d_eos_logp_ = nullptr, *d_row_stats_ = nullptr;
   float* d_pmax_ = nullptr;   // [R][pmax_ld_] block maxima of the logits, by-product of the vocabulary GEMM
+  float* d_psum_ = nullptr;   // [min(R, 64)][pmax_ld_] sums of exponentials of the same blocks (few rows)
   int pmax_ld_ = 0;
+  bool pblocks_ = false;      // the last vocabulary GEMM left maxima and sums of 32-column blocks
   int pmax_slots_ = 0;        // slots the last vocabulary GEMM filled (0 = none: the softmax finds its own maxima)
   // alignment records (print_info)
   float* d_rec_align_ = nullptr;

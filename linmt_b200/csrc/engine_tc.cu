@@ -3,6 +3,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <algorithm>
 
 #include "engine.h"
 #include "gemm_tc.cuh"
@@ -67,6 +68,12 @@ int Engine::alloc_state_tc(TcState& s) {
   if ((rc = alloc_planes(s.panel_top, R, 2 * Hp))) return rc;
   if ((rc = alloc_planes(s.panel_ht, R, Hp))) return rc;
   if (att_fold_ && (rc = alloc_planes(s.hs_planes, (size_t)B * opt.max_src_len, Hp))) return rc;
+  if (enc_rows_) {
+    if ((rc = alloc_planes(s.enc_in, enc_rows_, Hp))) return rc;
+    s.enc_seq.resize(L);
+    for (int l = 0; l < L; ++l)
+      if ((rc = alloc_planes(s.enc_seq[l], (size_t)enc_rows_ + tc::kRowsMax, Hp))) return rc;
+  }
   for (int i = 0; i < 2; ++i) {
     s.encp[i].resize(L);
     for (int l = 0; l < L; ++l)
@@ -101,7 +108,7 @@ const CUtensorMap* Engine::b_maps(const tc::Planes& p, int rows, int K, int bn, 
 
 // C[M][N] = A[:, a_col0 : a_col0+K] . W[N][K]^T with the tile width chosen for this shape.
 template <class Epi>
-int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e_in, int nt, int drain) {
+int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e_in, int nt, int drain, int x_row0) {
   Epi e = e_in;
   if (nt <= 0 || nt > nt_) nt = nt_;
   int bn = 0, splits = 1;
@@ -158,15 +165,18 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
           const int slots = 4 * ((N + tc::BM - 1) / tc::BM);
           if (slots > e.pmax_ld) { e.pmax = nullptr; pmax_slots_ = 0; }
           else pmax_slots_ = slots;
+          pblocks_ = e.pmax && topk_blocks_smem(slots, K) <= kBlocksSmemMax;
+          e.psum = pblocks_ ? d_psum_ : nullptr;
         }
       }
-      if (nt == 2) CK((tc::launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream)));
-      else if (fmt_ == 1) CK((tc::launch_gemm_tc_rows<1, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream)));
-      else CK((tc::launch_gemm_tc_rows<1, 0, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream)));
+      if (nt == 2) CK((tc::launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
+      else if (fmt_ == 1) CK((tc::launch_gemm_tc_rows<1, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
+      else CK((tc::launch_gemm_tc_rows<1, 0, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
       LAUNCHED();
       return LINMT_OK;
     }
   }
+  if (x_row0) return fail(LINMT_EINVAL, "internal: a row offset needs the few-rows kernel");
   const CUtensorMap* am = a_maps(A, a_col0, a_rows_cap, K, bk);
   const CUtensorMap* bm = b_maps(W, N, K, pair ? bn / 2 : bn, bk);
   if (!am || !bm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
@@ -254,7 +264,9 @@ int Engine::build_xw_tables() {
 // events for the cross-layer edges.  Besides the true dependencies, (l, p) waits for (l+1, p-2),
 // the last reader of the double-buffered input slot it overwrites.
 int Engine::run_encoder_tc(int n, int Smax) {
+  if (rows_ && n <= tc::kRowsMax && enc_rows_) return run_encoder_layers_tc(n, Smax);
   constexpr int kRing = 4;
+  hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;
   if (enc_streams_.empty()) {
     enc_streams_.resize(L);
     enc_events_.assign(L, std::vector<cudaEvent_t>(kRing));
@@ -322,6 +334,67 @@ int Engine::run_encoder_tc(int n, int Smax) {
   return LINMT_OK;
 }
 
+// Encoder for few sentences (up to 64), layer by layer.  A layer's input part W_x . x_p of ALL positions is one GEMM; what
+// is left of the recurrence per position is W_h . h (half of the layer's weights, which then stay in L2 from one position
+// to the next) in the few-rows kernel, with the input part added in its epilogue.  L x S short launches instead of S
+// rounds of L launches on L streams that each read the whole layer from HBM: one sentence of 30 words 1.28 -> 0.75 ms.
+// Block p of a layer's sequence panel holds its states after p positions (block 0 the state before): operand of the next
+// position and, as a whole, of the next layer's input GEMM.  Sources longer than the panels are taken in chunks.
+int Engine::run_encoder_layers_tc(int n, int Smax) {
+  hs_sent_ = 1; hs_pos_ = n;
+  const int per = enc_rows_ / n;               // positions per chunk
+  pdl_gemm_ = true;
+  for (int mi = 0; mi < n_models; ++mi) {
+    DevModel& m = models_[mi];
+    DevState& s = states_[mi];
+    TcState& ts = tc_states_[mi];
+    for (int l = 0; l < L; ++l) {
+      CK(cudaMemsetAsync(s.enc_c[0][l], 0, sizeof(float) * (size_t)n * Hp, stream));
+      for (int t = 0; t < nt_; ++t) CK(cudaMemsetAsync(ts.enc_seq[l].p[t], 0, sizeof(uint16_t) * (size_t)n * Hp, stream));
+    }
+    for (int p0 = 0; p0 < Smax; p0 += per) {
+      const int np = std::min(per, Smax - p0);
+      enc_embed_seq_kernel<<<dim3(n, np, nt_), 128, 0, stream>>>(cur_ids_, d_off_, d_len_, m.p_emb_src, desc.vocab_src, ts.enc_in, Hp, p0);
+      LAUNCHED();
+      for (int l = 0; l < L; ++l) {
+        const tc::Planes& seq = ts.enc_seq[l];
+        if (p0 > 0)   // the state the previous chunk ended with
+          for (int t = 0; t < nt_; ++t)
+            CK(cudaMemcpyAsync(seq.p[t], seq.p[t] + (size_t)per * n * Hp, sizeof(uint16_t) * (size_t)n * Hp, cudaMemcpyDeviceToDevice, stream));
+        tc::Planes in = l == 0 ? ts.enc_in : ts.enc_seq[l - 1];
+        if (l > 0) for (int t = 0; t < nt_; ++t) in.p[t] += (size_t)n * Hp;
+        tc::TcEpiF32 ei{nullptr, s.enc_pre, 4 * Hp, 0};
+        if (int rc = tc_gemm(in, 0, enc_rows_, m.p_enc_w[l], np * n, 4 * Hp, Hp, ei)) return rc;
+        tc::Planes wh = m.p_enc_w[l];
+        for (int t = 0; t < nt_; ++t) wh.p[t] += Hp;
+        for (int q = 0; q < np; ++q) {
+          const int pos = p0 + q;
+          tc::TcEpiLstm e{};
+          e.bias = m.enc_b[l]; e.c_prev = s.enc_c[pos & 1][l]; e.ldc = Hp; e.c_out = s.enc_c[(pos & 1) ^ 1][l];
+          e.xw = s.enc_pre + (size_t)q * n * 4 * Hp; e.x_ld = 4 * Hp;
+          e.h_out1 = seq; e.h1_col0 = 0;
+          e.h_prev = seq; e.hp_col0 = 0;
+          for (int t = 0; t < nt_; ++t) { e.h_out1.p[t] += (size_t)(q + 1) * n * Hp; e.h_prev.p[t] += (size_t)q * n * Hp; }
+          e.h_out2 = no_planes(); e.h2_col0 = 0;
+          e.h_f32 = (l == L - 1) ? s.hs + (size_t)pos * n * Hp : nullptr;
+          e.hf_row_stride = Hp;
+          e.row_len = d_len_; e.pos = pos; e.nt = nt_;
+          if (int rc = tc_gemm(seq, 0, enc_rows_ + tc::kRowsMax, wh, n, 4 * Hp, Hp, e, 0, 0, q * n)) return rc;
+        }
+        if (l == L - 1 && att_fold_) {
+          // W_c1 applied to the encoder states, once: the attention sums these rows (see AttFold in step_kernels.cuh)
+          tc::Planes top = seq;
+          for (int t = 0; t < nt_; ++t) top.p[t] += (size_t)n * Hp;
+          tc::TcEpiF32 e{nullptr, s.hs_wc1 + (size_t)p0 * n * Hp, Hp, 0};
+          if (int rc = tc_gemm(top, 0, enc_rows_, m.p_att_out_w, np * n, Hp, Hp, e)) return rc;
+        }
+      }
+      enc_final_row_ = np * n;
+    }
+  }
+  return LINMT_OK;
+}
+
 // One decoder forward, tensor-core path (see Engine::run_decoder_step).
 int Engine::run_decoder_step_tc(int mi, int t, int rows) {
   DevModel& m = models_[mi];
@@ -345,7 +418,8 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
       for (int p = 0; p < nt_; ++p) {
         const __nv_bfloat16* src;
         long long sst;
-        if (t == 0) { src = ts.encp[fb][l].p[p] + Hp; sst = (long long)ts.encp[fb][l].ld * 2; }
+        if (t == 0 && enc_final_row_ >= 0) { src = ts.enc_seq[l].p[p] + (size_t)enc_final_row_ * Hp; sst = (long long)Hp * 2; }
+        else if (t == 0) { src = ts.encp[fb][l].p[p] + Hp; sst = (long long)ts.encp[fb][l].ld * 2; }
         else { src = hcur_planes(l).p[p] + hcur_col0(l); sst = (long long)hcur_planes(l).ld * 2; }
         add(src, sst, hprev_planes(l).p[p] + Hp, (long long)hprev_planes(l).ld * 2, Hp * 2, 0);
       }
@@ -440,7 +514,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
   {
     tc::TcEpiF32 e{m.voc_b, s.logits, Vp, 0};
     if (logits16_) e.out16 = s.logits16;   // the softmax of this step is their only reader
-    pmax_slots_ = 0;
+    pmax_slots_ = 0; pblocks_ = false;
     if (n_models == 1 && pmax_on_) { e.pmax = d_pmax_; e.pmax_ld = pmax_ld_; e.n_valid = V; }
     if (int rc = kt(KC_VOCAB)) return rc;
     // Logits feed only the softmax of their own step: the tensor core's truncation bias over one

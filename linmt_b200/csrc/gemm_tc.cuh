@@ -327,6 +327,7 @@ struct TcEpiLstm {
   // the first decoder layer's product then costs a row lookup instead of a third of the GEMM.
   const float* xw = nullptr; const int32_t* x_tok = nullptr; int x_ld = 0; int x_vocab = 0; int x_unk = 0;
   __device__ __forceinline__ int x_row(int row) const {
+    if (!x_tok) return row;    // one row of the table per row of the product (encoder: the input's share of every position)
     const int t = x_tok[row];
     return (t < 0 || t >= x_vocab) ? x_unk : t;
   }
@@ -576,6 +577,7 @@ struct TcEpiF32 {
   // 64 columns (tile column block `slot`) of every row, over columns < n_valid, at pmax[row * pmax_ld + slot].
   // The softmax kernel then needs no first sweep over the row for its maximum and its top-k threshold.
   float* pmax = nullptr; int pmax_ld = 0; int n_valid = 0;
+  float* psum = nullptr;    // row form only: sum of exp(z - maximum) of the same block
   // Optional half-precision output (out16 set: `out` is not written): logits whose few values that matter one by one
   // are recomputed by their consumer and which otherwise only enter a sum of exponentials go out as fp16, half
   // the bytes to write and to sweep.  The block maxima are then those of the ROUNDED values (elements of the row).
@@ -680,8 +682,8 @@ struct TcEpiF32 {
   }
   __device__ __forceinline__ void finish_row(bool valid, int row, int col, int lane, const float4& v, const Pre& p) const {
     float m = -INFINITY;
+    float4 r = make_float4(v.x + p.b.x, v.y + p.b.y, v.z + p.b.z, v.w + p.b.w);
     if (valid) {
-      float4 r = make_float4(v.x + p.b.x, v.y + p.b.y, v.z + p.b.z, v.w + p.b.w);
       if (col < split) { r.x = tanh_fast(r.x); r.y = tanh_fast(r.y); r.z = tanh_fast(r.z); r.w = tanh_fast(r.w); }
       if (out16) {
         r.x = __half2float(__float2half_rn(r.x)); r.y = __half2float(__float2half_rn(r.y));
@@ -694,6 +696,16 @@ struct TcEpiF32 {
 #pragma unroll
       for (int o = 16; o > 2; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       if (lane < 4 && valid) pmax[(size_t)row * pmax_ld + (col >> 5)] = m;
+      if (psum) {
+        float q = 0.f;
+        if (valid && m > -INFINITY) {
+          q = (col < n_valid ? __expf(r.x - m) : 0.f) + (col + 1 < n_valid ? __expf(r.y - m) : 0.f);
+          q += (col + 2 < n_valid ? __expf(r.z - m) : 0.f) + (col + 3 < n_valid ? __expf(r.w - m) : 0.f);
+        }
+#pragma unroll
+        for (int o = 16; o > 2; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        if (lane < 4 && valid) psum[(size_t)row * pmax_ld + (col >> 5)] = q;
+      }
     }
   }
 };

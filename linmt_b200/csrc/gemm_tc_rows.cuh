@@ -105,7 +105,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 
 template <int NT, int FMT, class Epi>
 __global__ void __launch_bounds__(kRowsThreads, 2)
-gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, RowsShape sh, Epi epi, int* __restrict__ err_flag) {
+gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int x_row0, RowsShape sh, Epi epi, int* __restrict__ err_flag) {
   constexpr int PC = product_code(NT, FMT);
   static_assert(NT == 1 || PC == kF16PairCode, "one plane or the f16 pair");
   constexpr int W_BYTES = BM * 128;            // one plane of a weight k-block (64 deep)
@@ -170,7 +170,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, Row
   pdl_wait();    // from here on the previous kernel's results are visible
   if (warp == 0 && !is_w && lane < 2 * NT)
     for (int kb = 0; kb < prex; ++kb)
-      tma_load_2d(xbase + (uint32_t)(kb * NT * X_BYTES + pl * X_BYTES), map, (kb0 + kb) * 64, 0, xbars + 8u * kb);
+      tma_load_2d(xbase + (uint32_t)(kb * NT * X_BYTES + pl * X_BYTES), map, (kb0 + kb) * 64, x_row0, xbars + 8u * kb);
   // what the epilogue of this warp's first unit reads is requested now and used after the accumulators are complete
   auto unit_row = [&](int i) { return ((rank + splits * i) >> 2) * 4 + (lane & 3); };
   auto unit_col = [&](int i) { return n0 + ((rank + splits * i) & 3) * 32 + (lane & ~3); };    // of the lane's four columns
@@ -197,7 +197,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, Row
         ++kw;
         if (++ws == WS) { ws = 0; wph ^= 1u; }
       } else {
-        if (!is_w && lane < 2 * NT) tma_load_2d(xbase + (uint32_t)(xs * NT * X_BYTES + pl * X_BYTES), map, (kb0 + kx) * 64, 0, fb);
+        if (!is_w && lane < 2 * NT) tma_load_2d(xbase + (uint32_t)(xs * NT * X_BYTES + pl * X_BYTES), map, (kb0 + kx) * 64, x_row0, fb);
         ++kx;
         if (++xs == XS) { xs = 0; xph ^= 1u; }
       }
@@ -304,8 +304,9 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, Row
   if (threadIdx.x == 0 && *abort_flag) atomicExch(err_flag, 1);
 }
 
+// x_row0: first row of the product in the activations' tensor map
 template <int NT, int FMT, class Epi>
-inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st) {
+inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0 = 0) {
   static bool optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_rows_kernel<NT, FMT, Epi>, optin_done, kRowsSmemWhole); e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
@@ -325,7 +326,7 @@ inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, c
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tc_rows_kernel<NT, FMT, Epi>, tm, M, N, K, sh, epi, err_flag);
+  return cudaLaunchKernelEx(&cfg, gemm_tc_rows_kernel<NT, FMT, Epi>, tm, M, N, K, x_row0, sh, epi, err_flag);
 }
 
 }  // namespace tc

@@ -146,7 +146,26 @@ static __global__ void enc_embed_planes_kernel(const int32_t* __restrict__ ids, 
   }
 }
 
+// The same for every position at once (encoder layer by layer): row (pos * n + b) of dst.  grid = (n, positions, nt).
+static __global__ void enc_embed_seq_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ off, const int32_t* __restrict__ len,
+                                            tc::Planes emb, int vocab, tc::Planes dst, int Hp, int pos0) {
+  tc::pdl_launch_dependents();
+  tc::pdl_wait();
+  const int b = blockIdx.x, t = blockIdx.z, pos = pos0 + blockIdx.y;
+  const int S = len[b];
+  uint4* d = reinterpret_cast<uint4*>(dst.p[t] + (size_t)(blockIdx.y * gridDim.x + b) * dst.ld);
+  int tok = pos < S ? ids[off[b] + (S - 1 - pos)] : 0;
+  if (tok < 0 || tok >= vocab) tok = 0;
+  const uint4* src = reinterpret_cast<const uint4*>(emb.p[t] + (size_t)tok * emb.ld);
+  for (int i = threadIdx.x; i < Hp / 8; i += blockDim.x) d[i] = src[i];
+}
+
 // ---------------------------------------------------------------------------------------
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
 // Block-wide sum in a fixed order (deterministic).
 __device__ __forceinline__ float block_sum(float v, float* red) {
 #pragma unroll
@@ -155,8 +174,14 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   __syncthreads();
   if (l == 0) red[w] = v;
   __syncthreads();
-  float t = 0.f;
   const int nw = blockDim.x >> 5;
+  if (nw > 8) {
+    float t = l < nw ? red[l] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+  }
+  float t = 0.f;
   for (int i = 0; i < nw; ++i) t += red[i];
   return t;
 }
@@ -167,7 +192,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // CreateIndicesKernel, LoadInHSKernel, ElemReduceKernelLarge, AlignmentReductionKernel,
 // CreateCTKernel).
 //   proj [rows][2*Hp]: tanh(W_p h) | W_a^T h      (global_dot: `u` = h_top itself)
-//   hs   [B][max_src][Hp]: top encoder state after consuming reversed position p
+//   hs   row sent * hs_sent + p * hs_pos: top encoder state of a sentence after consuming reversed position p
 //   ctx  [rows][Hp] fp32 and/or ctx_planes (bf16 planes, columns [0,Hp) of the panel)
 //   rec_align [rows][rec_win] / rec_lo [rows] / rec_vit [rows]: alignment record of this step
 //   (may be null).  win = 2D+1 for local attention, max_src for the global modes.
@@ -176,7 +201,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 //   (rec_win = max_src, rec_lo = 0), the first member writes it, the others add to it in member order,
 //   and the last one takes the vote: the position of the largest summed score, the search starting from
 //   "none, 0" (EnsembleFactory::EnsemblesModels, src/decoder.h:1934-1964).
-// grid = rows, block = 256, dynamic smem = (win + 8) floats.  The kernel is a chain of L2 round trips, not
+// grid = rows, block = THREADS, dynamic smem = attention_smem<THREADS>(win).  The kernel is a chain of L2 round trips, not
 // of bytes.  (Three variations were tried and measured no faster: the window's states kept in shared memory
 // between the score sweep and the context sweep -- 86 KB per CTA costs the occupancy the halved traffic buys;
 // one CTA per group of beams of a sentence reading every state row once for all of them -- a quarter of the
@@ -200,25 +225,31 @@ struct AttFold {
   const float* add; int ld_add;   // element (row, j) at add[row * ld_add + j]
   const float* bias;    // [Hp]
 };
-// (six CTAs per SM: 888 resident CTAs hold the 768 rows of a full step in one wave; at five, 28 rows ran as a second wave)
-static __global__ void __launch_bounds__(256, 6) attention_kernel(const float* __restrict__ proj, int ldp, const float* __restrict__ u_alt, int ldu,
+// THREADS = 256: six CTAs per SM, so that the 888 resident CTAs hold the 768 rows of a full step in one wave (at five, 28
+// rows ran as a second wave).  THREADS = 1024 for a step whose rows leave SMs empty: one window position per warp and the
+// context in four groups of positions instead of chains of three and 21 dependent rounds of loads (one sentence: 18.1 us
+// per step with 256 threads).
+template <int THREADS>
+static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) attention_kernel(const float* __restrict__ proj, int ldp, const float* __restrict__ u_alt, int ldu,
                                  const float* __restrict__ vp, const float* __restrict__ hs,
                                  const int32_t* __restrict__ src_len, float* __restrict__ ctx, int H, int Hp,
-                                 int k, int max_src, int mode, int D, int win, float* __restrict__ rec_align,
+                                 int k, int hs_sent, int hs_pos, int mode, int D, int win, float* __restrict__ rec_align,
                                  int32_t* __restrict__ rec_lo, int32_t* __restrict__ rec_vit, tc::Planes ctx_planes, int nt,
                                  int rec_win, int ens, AttTrace at, AttFold fold) {
   tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
   extern __shared__ float sm[];
+  constexpr int kGroups = THREADS / 256;    // of window positions, in the context sum
   float* e = sm;            // [win]
-  float* red = sm + win;    // [8]
+  float* red = sm + win;    // [THREADS / 32]
+  float4* csum = reinterpret_cast<float4*>(sm + ((win + THREADS / 32 + 3) & ~3));   // [kGroups - 1][256] partial contexts
   __shared__ float s_pt;
   __shared__ int s_lo, s_hi;
   const int r = blockIdx.x;
   const int sent = r / k;
   const int S = src_len[sent];
   const float* u = u_alt ? (u_alt + (size_t)r * ldu) : (proj + (size_t)r * ldp + Hp);
-  const float* hsb = hs + (size_t)sent * max_src * Hp;
+  const float* hsb = hs + (size_t)sent * hs_sent * Hp;
 
   if (mode == 0) {
     float part = 0.f;
@@ -241,12 +272,18 @@ static __global__ void __launch_bounds__(256, 6) attention_kernel(const float* _
   const int W = hi - lo + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int w = warp; w < W; w += nw) {
-    const float* hrow = hsb + (size_t)(S - 1 - (lo + w)) * Hp;
+    const float* hrow = hsb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp;
     float acc = 0.f;
-    for (int j = lane * 4; j < Hp; j += 128) {
+    auto dot4 = [&](int j) {
       const float4 a = *reinterpret_cast<const float4*>(hrow + j);
       const float4 b = *reinterpret_cast<const float4*>(u + j);
       acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
+    };
+    if (THREADS > 256) {
+#pragma unroll 8
+      for (int j = lane * 4; j < Hp; j += 128) dot4(j);
+    } else {
+      for (int j = lane * 4; j < Hp; j += 128) dot4(j);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -313,14 +350,13 @@ static __global__ void __launch_bounds__(256, 6) attention_kernel(const float* _
   }
   // context: CreateCTKernel, deep_rnn_kernel.h:1250-1260 (sum over window positions in order)
   float* crow = ctx ? ctx + (size_t)r * Hp : nullptr;
-  const float* csb = fold.cs ? fold.cs + (size_t)sent * max_src * Hp : hsb;
-  for (int j = threadIdx.x * 4; j < Hp; j += blockDim.x * 4) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int w = 0; w < W; ++w) {
-      const float a = e[w];
-      const float4 h4 = *reinterpret_cast<const float4*>(csb + (size_t)(S - 1 - (lo + w)) * Hp + j);
-      acc.x += a * h4.x; acc.y += a * h4.y; acc.z += a * h4.z; acc.w += a * h4.w;
-    }
+  const float* csb = fold.cs ? fold.cs + (size_t)sent * hs_sent * Hp : hsb;
+  auto add = [&](float4& acc, int w, int j) {
+    const float a = e[w];
+    const float4 h4 = *reinterpret_cast<const float4*>(csb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp + j);
+    acc.x += a * h4.x; acc.y += a * h4.y; acc.z += a * h4.z; acc.w += a * h4.w;
+  };
+  auto finish = [&](float4 acc, int j) {
     if (fold.cs) {
       // the attentional state: the sums of TcEpiBiasTanh in its order, (W_c1 ctx + W_c2 h) + b
       const float4 g = *reinterpret_cast<const float4*>(fold.add + (size_t)r * fold.ld_add + j);
@@ -333,7 +369,40 @@ static __global__ void __launch_bounds__(256, 6) attention_kernel(const float* _
       const size_t idx = (size_t)r * ctx_planes.ld + j;
       tc::split_store4(ctx_planes, nt, idx, acc.x, acc.y, acc.z, acc.w);
     }
+  };
+  if constexpr (kGroups == 1) {
+    for (int j = threadIdx.x * 4; j < Hp; j += blockDim.x * 4) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int w = 0; w < W; ++w) add(acc, w, j);
+      finish(acc, j);
+    }
+  } else {
+    const int group = threadIdx.x >> 8, w0 = W * group / kGroups, w1 = W * (group + 1) / kGroups;
+    for (int j0 = 0; j0 < Hp; j0 += 1024) {
+      const int j = j0 + (threadIdx.x & 255) * 4;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j < Hp) {
+#pragma unroll 6
+        for (int w = w0; w < w1; ++w) add(acc, w, j);
+      }
+      if (j0 > 0) __syncthreads();      // (the previous pass's partial contexts have been read)
+      if (group > 0 && j < Hp) csum[(group - 1) * 256 + (threadIdx.x & 255)] = acc;
+      __syncthreads();
+      if (group == 0 && j < Hp) {
+#pragma unroll
+        for (int g = 0; g < kGroups - 1; ++g) {
+          const float4 o = csum[g * 256 + threadIdx.x];
+          acc.x += o.x; acc.y += o.y; acc.z += o.z; acc.w += o.w;
+        }
+        finish(acc, j);
+      }
+    }
   }
+}
+
+template <int THREADS>
+inline size_t attention_smem(int win) {
+  return sizeof(float) * (size_t)(((win + THREADS / 32 + 3) & ~3) + (THREADS / 256 - 1) * 1024);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -366,33 +435,420 @@ struct TopkRefine {
 };
 constexpr float kPairInv = 1.0f / 2048.0f;
 
+// ---------------------------------------------------------------------------------------
+// Beam selection for one sentence and one step, all on the device.  Replaces
+// Decoder<T>::ExpandHypothesis (src/decoder.h:355-480) and, on a sentence's last step,
+// Decoder<T>::FinishCurrentHypotheses (src/decoder.h:502-525).
+// Candidate order = (score desc, beam asc, vocab asc), the defined order of the reference's
+// global heap.  START is skipped, EOS goes to the finished list without using a slot.
+struct BeamState {
+  int32_t* tok;        // [R] current token of each slot
+  float* score;        // [R]
+  int32_t* parent;     // [R] parent slot chosen by the last selection
+  int32_t* hist_tok;   // [Tcap][R]
+  int32_t* hist_parent;// [Tcap][R]
+  int32_t* fin_t;      // [B][fin_cap] step at which EOS was produced
+  int32_t* fin_b;      // [B][fin_cap] slot whose history the hypothesis continues
+  float* fin_score;    // [B][fin_cap]
+  int32_t* fin_n;      // [B]
+  int fin_cap;
+  int R;
+};
+struct TraceDev {
+  int32_t* cand_tok; float* cand_logp; int32_t* surv_tok; int32_t* surv_parent; float* surv_score; float* final_logp;
+  const int32_t* force_tok; const int32_t* force_parent; const float* force_score;
+  int Tm;
+  float* pt;                 // [n][Tm+1][k] attention centre of every forward (member 0), or null
+  float* gold_logp;          // [n][Tm][k] log-probability of the forced token of every slot (scoring)
+  const float* logits; int ld_logits; const float* row_stats;   // what gold_logp is computed from
+  TopkRefine rf;             // set when the logits are one-product values: the forced token's logit is recomputed accurately
+};
+// The selection runs inside the softmax kernels: the CTA that finishes a sentence's last row (a counter per sentence)
+// goes on with the sentence's selection, which as a kernel of its own cost a launch and a round trip per step for a
+// microsecond of work (7.7 us per step at one sentence).
+struct SelectArgs {
+  BeamState bs;
+  const int32_t* steps;    // null: no selection (the kernel is called for its own result)
+  const int32_t* orig;
+  int* done;               // [B] rows of the sentence finished in this step; left at zero
+  int t, k;
+  float penalty, diversity;
+  TraceDev tr;
+};
+constexpr int kSelectSmem = kMaxBeam * (kMaxBeam + 1) * 20;   // its shared memory: candidates of the widest beam
+// Candidates of the whole sentence in shared memory, then the walk over them in order, 32 candidates at a time.
+template <int THREADS>
+__device__ __forceinline__ void beam_select_block(const SelectArgs& a, const TopkOut& cand, int sent, int T, int osent, int nf0, unsigned char* smraw) {
+  const BeamState& bs = a.bs;
+  const TraceDev& tr = a.tr;
+  const int k = a.k, kk = k + 1, t = a.t;
+  const int r0 = sent * k;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (t > T) return;
+  if (t == T) {
+    if (warp == 0) {
+      const int n0 = nf0;
+      if (lane < k) {
+        const float lp = __ldcg(cand.eos_logp + r0 + lane);
+        if (tr.final_logp) tr.final_logp[(size_t)osent * k + lane] = lp;
+        const int n = n0 + lane;
+        if (n < bs.fin_cap) {
+          bs.fin_t[(size_t)sent * bs.fin_cap + n] = t;
+          bs.fin_b[(size_t)sent * bs.fin_cap + n] = lane;
+          bs.fin_score[(size_t)sent * bs.fin_cap + n] = bs.score[r0 + lane] + (lp + a.penalty);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) bs.fin_n[sent] = n0 + k < bs.fin_cap ? n0 + k : bs.fin_cap;
+    }
+    return;
+  }
+  const int ncap = k * kk;
+  unsigned long long* key = reinterpret_cast<unsigned long long*>(smraw);   // sortable (score, beam, vocab)
+  float* ss = reinterpret_cast<float*>(key + ncap);   // score, beam and vocabulary id in sorted order
+  int* sb = reinterpret_cast<int*>(ss + ncap);
+  int* sv = sb + ncap;
+  const int cols = (t == 0) ? 1 : k;
+  const int n = cols * kk;
+  for (int c = tid; c < n; c += THREADS) {
+    const int b = c / kk, q = c - b * kk;
+    const float lp = __ldcg(cand.logp + (size_t)(r0 + b) * kk + q);    // (other CTAs' results)
+    const int v = __ldcg(cand.idx + (size_t)(r0 + b) * kk + q);
+    const float rank_penalty = (float)(q + 1) * a.diversity;
+    const float sc = (lp + bs.score[r0 + b]) - rank_penalty;
+    ss[c] = sc; sb[c] = b; sv[c] = v;   // overwritten by the ranking below; keeps every entry valid even for NaN scores
+    // one 64-bit key, larger = earlier: score descending, then beam ascending, then vocabulary id ascending
+    const unsigned int fb = __float_as_uint(sc);
+    const unsigned int ord = (fb & 0x80000000u) ? ~fb : (fb | 0x80000000u);
+    const unsigned int low = 0xFFFFFFFFu - (((unsigned int)b << 24) | ((unsigned int)v & 0xFFFFFFu));
+    key[c] = ((unsigned long long)ord << 32) | low;
+    if (tr.cand_tok) {
+      const size_t off = ((((size_t)osent * tr.Tm + t) * k + b) * kk) + q;
+      tr.cand_tok[off] = v; tr.cand_logp[off] = lp;
+    }
+  }
+  __syncthreads();
+  // (k <= 31: at most 992 candidates, i.e. at most four per thread of a block of 256)
+  constexpr int kPer = (kMaxBeam * (kMaxBeam + 1) + THREADS - 1) / THREADS;
+  int pos[kPer]; float ksc[kPer]; int kb[kPer], kv[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int c = tid + i * THREADS;
+    if (c < n) {
+      const unsigned long long kc = key[c];
+      int p = 0;
+#pragma unroll 4
+      for (int d = 0; d < n; ++d) p += (key[d] > kc) ? 1 : 0;
+      pos[i] = p; ksc[i] = ss[c]; kb[i] = sb[c]; kv[i] = sv[c];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kPer; ++i)
+    if (tid + i * THREADS < n) { ss[pos[i]] = ksc[i]; sb[pos[i]] = kb[i]; sv[pos[i]] = kv[i]; }
+  __syncthreads();
+  __shared__ int s_ntok[kMaxBeam + 1], s_npar[kMaxBeam + 1];
+  __shared__ float s_nscore[kMaxBeam + 1];
+  if (warp == 0) {
+    // START is skipped, EOS leaves the beam without taking a slot as long as slots are free
+    int ns = 0, nf = nf0;
+    for (int p0 = 0; p0 < n && ns < k; p0 += 32) {
+      const int p = p0 + lane;
+      const int v = p < n ? sv[p] : -1;
+      const unsigned take = __ballot_sync(0xffffffffu, v >= 0 && v != kStart && v != kEos);
+      const unsigned below = (1u << lane) - 1u;
+      const int slot = ns + __popc(take & below);            // free slots used before this candidate
+      const bool eos = v == kEos && slot < k;
+      const unsigned ends = __ballot_sync(0xffffffffu, eos);
+      if (((take >> lane) & 1u) && slot < k) { s_ntok[slot] = v; s_npar[slot] = sb[p]; s_nscore[slot] = ss[p] + a.penalty; }
+      const int f = nf + __popc(ends & below);
+      if (eos && f < bs.fin_cap) {
+        bs.fin_t[(size_t)sent * bs.fin_cap + f] = t;
+        bs.fin_b[(size_t)sent * bs.fin_cap + f] = sb[p];
+        bs.fin_score[(size_t)sent * bs.fin_cap + f] = ss[p] + a.penalty;
+      }
+      ns += __popc(take);
+      nf += __popc(ends);
+    }
+    for (int q = ns + lane; q < k; q += 32) { s_ntok[q] = kUnk; s_npar[q] = 0; s_nscore[q] = kDeadScore; }
+    if (lane == 0 && nf > nf0) bs.fin_n[sent] = nf < bs.fin_cap ? nf : bs.fin_cap;
+  }
+  // Scoring (force-decoding): log-probability of the forced token of every slot under its parent's row.
+  // With one-product logits the token's logit is recomputed from both planes of both operands, like the
+  // candidates in the softmax kernel; one warp per slot.
+  __shared__ float s_gold[kMaxBeam + 1];
+  if (tr.force_tok && tr.gold_logp && tr.logits) {
+    for (int b = warp; b < k; b += THREADS / 32) {
+      const size_t off = ((size_t)osent * tr.Tm + t) * k + b;
+      const int npar = tr.force_parent[off];
+      const int prow = r0 + (npar >= 0 && npar < k ? npar : 0);
+      const int gt = tr.force_tok[off] >= 0 ? tr.force_tok[off] : 0;
+      float zv = 0.f;
+      if (tr.rf.a0) {
+        const __half* a0 = tr.rf.a0 + (size_t)prow * tr.rf.lda;
+        const __half* a1 = tr.rf.a1 + (size_t)prow * tr.rf.lda;
+        const __half* w0 = tr.rf.b0 + (size_t)gt * tr.rf.ldb;
+        const __half* w1 = tr.rf.b1 + (size_t)gt * tr.rf.ldb;
+        float acc = 0.f;
+        for (int j = lane; j < tr.rf.K; j += 32) {
+          const float x = fmaf(__half2float(a1[j]), kPairInv, __half2float(a0[j]));
+          const float w = fmaf(__half2float(w1[j]), kPairInv, __half2float(w0[j]));
+          acc = fmaf(x, w, acc);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        zv = acc + (tr.rf.bias ? tr.rf.bias[gt] : 0.f);
+      } else if (lane == 0) {
+        zv = tr.logits[(size_t)prow * tr.ld_logits + gt];
+      }
+      if (lane == 0) s_gold[b] = (zv - __ldcg(tr.row_stats + 2 * prow)) - __ldcg(tr.row_stats + 2 * prow + 1);
+    }
+  }
+  __syncthreads();
+  if (tid < k) {
+    const int b = tid;
+    int ntok = s_ntok[b], npar = s_npar[b];
+    float nscore = s_nscore[b];
+    const size_t off = ((size_t)osent * tr.Tm + t) * k + b;
+    if (tr.surv_tok) { tr.surv_tok[off] = ntok; tr.surv_parent[off] = npar; tr.surv_score[off] = nscore; }
+    if (tr.force_tok) {
+      ntok = tr.force_tok[off]; npar = tr.force_parent[off]; nscore = tr.force_score[off];
+      if (tr.gold_logp && tr.logits) tr.gold_logp[off] = s_gold[b];
+    }
+    bs.tok[r0 + b] = ntok; bs.parent[r0 + b] = npar; bs.score[r0 + b] = nscore;
+    bs.hist_tok[(size_t)t * bs.R + r0 + b] = ntok;
+    bs.hist_parent[(size_t)t * bs.R + r0 + b] = npar;
+  }
+}
+// End of a softmax kernel: row r's results are written; the last row of its sentence selects.
+template <int THREADS>
+__device__ __forceinline__ void select_if_last(const SelectArgs& a, const TopkOut& cand, int r, unsigned char* smraw) {
+  if (!a.steps) return;
+  __shared__ int s_last;
+  const int sent = r / a.k;
+  // what the selection reads first is on its way while the counter answers
+  const int T = a.steps[sent], osent = a.orig[sent], nf0 = a.bs.fin_n[sent];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();       // this row's candidates (all threads', by the barrier) before the counter
+    s_last = atomicAdd(&a.done[sent], 1) == a.k - 1;
+    if (s_last) { a.done[sent] = 0; __threadfence(); }
+  }
+  __syncthreads();
+  if (s_last) beam_select_block<THREADS>(a, cand, sent, T, osent, nf0, smraw);
+}
+
 // Pass 1 finds the row maximum and, from the 256 per-thread maxima, a threshold that at least
 // kk elements reach (the kk-th largest thread maximum).  Pass 2 (the row is L2/L1 resident by
 // then) sums exp(z - max) and collects the few elements at or above the threshold, which are
 // then ranked exactly.  If more elements than the candidate buffer holds reach the threshold
 // (e.g. a row of equal logits) the block falls back to kk exact arg-best sweeps.
 constexpr int kTopkCap = 1024;
+// What both softmax kernels do once the candidates of a row are listed (sh.cv, sh.ci, sh.count) and each thread holds its
+// share `ssum` of the sum of exp(z - rmax): log-sum, accurate values of the candidates (refinement), exact ranking.
+struct TopkShared {
+  float cv[kTopkCap];
+  int ci[kTopkCap];
+  float cd[kTopkCap];   // refinement: change of exp(z - max) per candidate, in buffer order ...
+  float co[kTopkCap];   // ... and in vocabulary order
+  float red[32];
+  int redi[32];
+  int count;
+  float lse, sum, eos, eos_delta;
+};
+// (once a row's results are written, the selection has the memory)
+union TopkSmem {
+  TopkShared sh;
+  unsigned char sel[kSelectSmem];
+};
+template <int THREADS>
+__device__ __forceinline__ void topk_finish(TopkShared& sh, int r, float ssum, float rmax, const float* __restrict__ z, const __half* __restrict__ zh,
+                                            int V, int kk, const TopkOut& out, int normalise, const TopkRefine& rf, const float* s_a) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  auto zat = [&](int i) { return zh ? __half2float(zh[i]) : z[i]; };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
+  if (lane == 0) sh.red[warp] = ssum;
+  __syncthreads();
+  if (warp == 0) {
+    const float bs = warp_sum(lane < THREADS / 32 ? sh.red[lane] : 0.f);
+    if (lane == 0) {
+      sh.sum = bs;
+      if (!rf.a0) sh.lse = normalise ? logf(bs) : -rmax;   // normalise = 0: the row already holds log-probabilities
+    }
+    if (lane == 0 && !rf.a0) {
+      if (out.eos_logp) out.eos_logp[r] = (zat(kEos) - rmax) - sh.lse;
+      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = sh.lse; }
+    }
+  }
+  __syncthreads();
+  int n = sh.count;
+  if (rf.a0 && n > kTopkCap) {
+    // More elements than the buffer holds reach the widened threshold (a nearly flat row): pick the kk best
+    // of the one-product logits by exact sweeps and make those the candidates.  Their values are refined
+    // like any others below; an element within the error bound just beyond the kk-th can be missed here,
+    // which on a row this flat is a tie within the tolerance.
+    float last_v = INFINITY;
+    int last_i = -1;
+    for (int round = 0; round < kk; ++round) {
+      float bv = -INFINITY;
+      int bi = 0x7fffffff;
+      for (int i = tid; i < V; i += THREADS) {
+        const float v = zat(i);
+        const bool after = (v < last_v) || (v == last_v && i > last_i);
+        if (after && better(v, i, bv, bi)) { bv = v; bi = i; }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+      }
+      __syncthreads();
+      if (lane == 0) { sh.red[warp] = bv; sh.redi[warp] = bi; }
+      __syncthreads();
+      bv = sh.red[0]; bi = sh.redi[0];
+      for (int w = 1; w < THREADS / 32; ++w) if (better(sh.red[w], sh.redi[w], bv, bi)) { bv = sh.red[w]; bi = sh.redi[w]; }
+      if (tid == 0) { sh.cv[round] = bv; sh.ci[round] = bi; }
+      last_v = bv; last_i = bi;
+    }
+    __syncthreads();
+    n = 0;
+    while (n < kk && sh.ci[n] != 0x7fffffff) ++n;   // fewer than kk elements in the row
+    __syncthreads();
+    if (tid == 0) sh.count = n;
+  }
+  if (rf.a0) {
+    // accurate values for the candidates (and for EOS, whose log-probability is always reported): one
+    // warp per candidate, fp32 FMAs over the two planes of both operands.  Each also yields the term by
+    // which the row's sum of exponentials changes when the accurate value replaces the one-product one:
+    // on a peaked row the few dominant logits ARE the normaliser, and their fp16-product error would
+    // otherwise go straight into every log-probability of the row.
+    const int nc = n;
+    for (int c = warp; c <= nc; c += THREADS / 32) {
+      const int v = (c < nc) ? sh.ci[c] : kEos;
+      const __half* w0 = rf.b0 + (size_t)v * rf.ldb;
+      const __half* w1 = rf.b1 + (size_t)v * rf.ldb;
+      // (what the sum is completed with is requested together with the weights)
+      const float bias = rf.bias ? rf.bias[v] : 0.f;
+      const float za = (c < nc) ? sh.cv[c] : zat(kEos);
+      float acc = 0.f;
+      auto dot4 = [&](int j) {
+        const uint2 q0 = *reinterpret_cast<const uint2*>(w0 + j);
+        const uint2 q1 = *reinterpret_cast<const uint2*>(w1 + j);
+        const __half2 h00 = *reinterpret_cast<const __half2*>(&q0.x), h01 = *reinterpret_cast<const __half2*>(&q0.y);
+        const __half2 h10 = *reinterpret_cast<const __half2*>(&q1.x), h11 = *reinterpret_cast<const __half2*>(&q1.y);
+        const float2 b00 = __half22float2(h00), b01 = __half22float2(h01), b10 = __half22float2(h10), b11 = __half22float2(h11);
+        acc = fmaf(s_a[j + 0], fmaf(b10.x, kPairInv, b00.x), acc);
+        acc = fmaf(s_a[j + 1], fmaf(b10.y, kPairInv, b00.y), acc);
+        acc = fmaf(s_a[j + 2], fmaf(b11.x, kPairInv, b01.x), acc);
+        acc = fmaf(s_a[j + 3], fmaf(b11.y, kPairInv, b01.y), acc);
+      };
+      if (THREADS > 256) {     // few rows: registers to spare for eight rounds of loads in flight
+#pragma unroll 8
+        for (int j = lane * 4; j < rf.K; j += 128) dot4(j);
+      } else {
+        for (int j = lane * 4; j < rf.K; j += 128) dot4(j);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) {
+        const float zv = acc + bias;
+        const float delta = __expf(zv - rmax) - __expf(za - rmax);
+        if (c < nc) { sh.cv[c] = zv; sh.cd[c] = delta; }
+        else { sh.eos = zv; sh.eos_delta = delta; }
+      }
+    }
+    __syncthreads();
+    // the correction is summed in vocabulary order, so the result does not depend on the order in which
+    // the candidates happened to enter the buffer
+    for (int c = tid; c < nc; c += THREADS) {
+      const int i = sh.ci[c];
+      int pos = 0;
+      for (int d = 0; d < nc; ++d) pos += (sh.ci[d] < i) ? 1 : 0;
+      sh.co[pos] = sh.cd[c];
+    }
+    __syncthreads();
+    if (warp == 0) {
+      float corr = 0.f;
+      bool eos_listed = false;
+      for (int c = lane; c < nc; c += 32) { corr += sh.co[c]; eos_listed = eos_listed || (sh.ci[c] == kEos); }
+      corr = warp_sum(corr);
+      if (!__any_sync(0xffffffffu, eos_listed)) corr += sh.eos_delta;
+      if (lane == 0) {
+      const float bs = sh.sum + corr;
+      sh.lse = normalise ? logf(bs > 0.f ? bs : sh.sum) : -rmax;
+      if (out.eos_logp) out.eos_logp[r] = (sh.eos - rmax) - sh.lse;
+      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = sh.lse; }
+      }
+    }
+    __syncthreads();
+  }
+  const float rlse = sh.lse;
+  if (n <= kTopkCap) {
+    // exact ranking of the candidates: value descending, index ascending
+    for (int c = tid; c < n; c += THREADS) {
+      const float v = sh.cv[c];
+      const int i = sh.ci[c];
+      int rank = 0;
+      for (int d = 0; d < n; ++d) rank += better(sh.cv[d], sh.ci[d], v, i) ? 1 : 0;
+      if (rank < kk) {
+        out.idx[(size_t)r * kk + rank] = i;
+        out.logp[(size_t)r * kk + rank] = (v - rmax) - rlse;
+      }
+    }
+    for (int q = n + tid; q < kk; q += THREADS) {  // fewer than kk elements in the row
+      out.idx[(size_t)r * kk + q] = -1;
+      out.logp[(size_t)r * kk + q] = -INFINITY;
+    }
+    return;
+  }
+  // ---- fallback: kk sweeps, each picking the best element after the previous pick ----
+  float last_v = INFINITY;
+  int last_i = -1;
+  for (int round = 0; round < kk; ++round) {
+    float bv = -INFINITY;
+    int bi = 0x7fffffff;
+    for (int i = tid; i < V; i += THREADS) {
+      const float v = zat(i);
+      const bool after = (v < last_v) || (v == last_v && i > last_i);
+      if (after && better(v, i, bv, bi)) { bv = v; bi = i; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+    }
+    __syncthreads();
+    if (lane == 0) { sh.red[warp] = bv; sh.redi[warp] = bi; }
+    __syncthreads();
+    bv = sh.red[0]; bi = sh.redi[0];
+    for (int w = 1; w < THREADS / 32; ++w) if (better(sh.red[w], sh.redi[w], bv, bi)) { bv = sh.red[w]; bi = sh.redi[w]; }
+    if (tid == 0) {
+      const bool valid = bi != 0x7fffffff;
+      out.idx[(size_t)r * kk + round] = valid ? bi : -1;
+      out.logp[(size_t)r * kk + round] = valid ? ((bv - rmax) - rlse) : -INFINITY;
+    }
+    last_v = bv; last_i = bi;
+  }
+}
+
 static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float* __restrict__ logits, int ld, int V, int kk, TopkOut out,
                                                                   int normalise, const float* __restrict__ pmax, int pmax_ld, int n_slots, TopkRefine rf,
-                                                                  const __half* __restrict__ logits16) {
+                                                                  const __half* __restrict__ logits16, const __grid_constant__ SelectArgs sel) {
   extern __shared__ float s_a[];   // [rf.K] the row's activations in fp32 (refinement only)
   tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
   __shared__ float s_tmax[256];
-  __shared__ float s_cv[kTopkCap];
-  __shared__ int s_ci[kTopkCap];
-  __shared__ float s_red[8];
-  __shared__ int s_redi[8];
-  __shared__ float s_cd[kTopkCap];   // refinement: change of exp(z - max) per candidate, in buffer order ...
-  __shared__ float s_co[kTopkCap];   // ... and in vocabulary order
-  __shared__ int s_count;
-  __shared__ float s_tau, s_max, s_lse, s_sum, s_eos, s_eos_delta;
+  __shared__ __align__(16) unsigned char s_union[sizeof(TopkSmem)];
+  TopkShared& sh = *reinterpret_cast<TopkShared*>(s_union);
+  __shared__ float s_tau, s_max;
   const int r = blockIdx.x, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
   const float* z = logits + (size_t)r * ld;
   // fp16 logits (refinement mode only: the candidates' values are recomputed, the rest only enter the sum)
   const __half* zh = logits16 ? logits16 + (size_t)r * ld : nullptr;
-  auto zat = [&](int i) { return zh ? __half2float(zh[i]) : z[i]; };
   const int V4 = V & ~3;
   // ---- pass 1: maxima (four independent 16-byte loads in flight per thread) -- or, when the GEMM that
   // produced the logits left the maxima of disjoint column blocks of every row (pmax), just those ----
@@ -422,7 +878,7 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
     for (int i = V4 + tid; i < V; i += 256) m = fmaxf(m, z[i]);
   }
   s_tmax[tid] = m;
-  if (tid == 0) s_count = 0;
+  if (tid == 0) sh.count = 0;
   __syncthreads();
   if (kk <= 32) {
     // Threshold from 32 group maxima (group = the 8 threads with the same lane): each is an
@@ -465,21 +921,21 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
     for (int sl = tid; sl < n_slots; sl += 256) {
       const float v = pmax[(size_t)r * pmax_ld + sl];
       if (v >= tau0) {
-        const int pos = atomicAdd(&s_count, 1);
-        if (pos < kTopkCap) s_cv[pos] = v;
+        const int pos = atomicAdd(&sh.count, 1);
+        if (pos < kTopkCap) sh.cv[pos] = v;
       }
     }
     __syncthreads();
-    const int m2 = s_count;
+    const int m2 = sh.count;
     if (m2 <= kTopkCap)
       for (int c = tid; c < m2; c += 256) {
-        const float v = s_cv[c];
+        const float v = sh.cv[c];
         int rank = 0;
-        for (int d = 0; d < m2; ++d) rank += (s_cv[d] > v || (s_cv[d] == v && d < c)) ? 1 : 0;
+        for (int d = 0; d < m2; ++d) rank += (sh.cv[d] > v || (sh.cv[d] == v && d < c)) ? 1 : 0;
         if (rank == kk - 1) s_tau = v;
       }
     __syncthreads();
-    if (tid == 0) s_count = 0;
+    if (tid == 0) sh.count = 0;
     __syncthreads();
   }
   float tau = s_tau;
@@ -495,10 +951,10 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) s_red[warp] = ss;
+    if (lane == 0) sh.red[warp] = ss;
     __syncthreads();
     float tot = 0.f;
-    for (int w = 0; w < 8; ++w) tot += s_red[w];
+    for (int w = 0; w < 8; ++w) tot += sh.red[w];
     tau -= 2.0f * (rf.eps_coef * sqrtf(tot) + 1e-5f);   // + fp16 subnormals and the accumulator's own rounding
     if (zh) tau -= 2.0f * 4.9e-4f * fmaxf(fabsf(rmax), fabsf(tau));   // and the rounding of the stored value (2^-11 relative)
     __syncthreads();
@@ -508,8 +964,8 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
   auto visit = [&](float v, int i) {
     ssum += __expf(v - rmax);  // arguments in [-few, 0]: ~1e-7 relative on the sum of V terms
     if (v >= tau) {
-      const int pos = atomicAdd(&s_count, 1);
-      if (pos < kTopkCap) { s_cv[pos] = v; s_ci[pos] = i; }
+      const int pos = atomicAdd(&sh.count, 1);
+      if (pos < kTopkCap) { sh.cv[pos] = v; sh.ci[pos] = i; }
     }
   };
   {
@@ -523,8 +979,8 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (v[u] >= tau) {
-            const int pos = atomicAdd(&s_count, 1);
-            if (pos < kTopkCap) { s_cv[pos] = v[u]; s_ci[pos] = i + u; }
+            const int pos = atomicAdd(&sh.count, 1);
+            if (pos < kTopkCap) { sh.cv[pos] = v[u]; sh.ci[pos] = i + u; }
           }
       }
     };
@@ -566,170 +1022,144 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
     for (int j = V4 + tid; j < V; j += 256) visit(z[j], j);
     }
   }
+  topk_finish<256>(sh, r, ssum, rmax, z, zh, V, kk, out, normalise, rf, s_a);
+  select_if_last<256>(sel, out, r, s_union);
+}
+
+// The same result when the GEMM that produced the logits left, for every block of 32 columns of a row, the block's maximum
+// AND its sum of exp(z - maximum) (gemm_tc_rows.cuh): the row itself is not swept.  The maximum, the sum and the threshold
+// come from the blocks (938 pairs for 30,000 classes), and only blocks whose maximum reaches the threshold are looked into.
+// For few rows, whose one CTA each has an SM to itself and is bound by the chain of its memory round trips, not by bytes
+// (one sentence at 12 rows, 30k classes: 22.2 us per step sweeping).
+// grid = rows, dynamic smem = topk_blocks_smem
+constexpr int kBlockCols = 32;
+constexpr int kBlocksSmemMax = 23 * 1024;   // of dynamic shared memory beside the candidate lists: wider rows are swept
+struct LogitBlocks {
+  const float* max; const float* sum; int ld; int n;
+};
+inline size_t topk_blocks_smem(int n_blocks, int refine_K) { return sizeof(float) * (size_t)(2 * n_blocks + refine_K); }
+constexpr int kTopkBlocksThreads = 1024;
+static __global__ void __launch_bounds__(kTopkBlocksThreads, 1) topk_blocks_kernel(const float* __restrict__ logits, const __half* __restrict__ logits16, int ld, int V, int kk,
+                                                                           TopkOut out, int normalise, LogitBlocks bl, TopkRefine rf, const __grid_constant__ SelectArgs sel) {
+  constexpr int THREADS = kTopkBlocksThreads;
+  tc::pdl_launch_dependents();
+  tc::pdl_wait();
+  extern __shared__ float dyn[];
+  float* s_m = dyn;                  // [n] block maxima
+  float* s_q = dyn + bl.n;           // [n] block sums
+  float* s_a = dyn + 2 * bl.n;       // [rf.K] activations (refinement)
+  __shared__ __align__(16) unsigned char s_union[sizeof(TopkSmem)];
+  TopkShared& sh = *reinterpret_cast<TopkShared*>(s_union);
+  __shared__ float s_tmax[THREADS];
+  __shared__ float s_tau, s_max;
+  const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* z = logits ? logits + (size_t)r * ld : nullptr;
+  const __half* zh = logits16 ? logits16 + (size_t)r * ld : nullptr;
+  float m = -INFINITY;
+  for (int b = tid; b < bl.n; b += THREADS) {
+    const float v = bl.max[(size_t)r * bl.ld + b];
+    s_q[b] = bl.sum[(size_t)r * bl.ld + b];
+    s_m[b] = v;
+    m = fmaxf(m, v);
+  }
+  float ss = 0.f;
+  if (rf.a0)
+    for (int j = tid; j < rf.K; j += THREADS) {
+      const float a = __half2float(rf.a0[(size_t)r * rf.lda + j]) + __half2float(rf.a1[(size_t)r * rf.lda + j]) * kPairInv;
+      s_a[j] = a;
+      ss = fmaf(a, a, ss);
+    }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
-  if (lane == 0) s_red[warp] = ssum;
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (lane == 0) sh.red[warp] = ss;
+  s_tmax[tid] = m;
+  if (tid == 0) sh.count = 0;
   __syncthreads();
-  if (tid == 0) {
-    float bs = 0.f;
-    for (int w = 0; w < 8; ++w) bs += s_red[w];
-    s_sum = bs;
-    s_lse = normalise ? logf(bs) : -rmax;   // normalise = 0: the row already holds log-probabilities
-    if (!rf.a0) {
-      if (out.eos_logp) out.eos_logp[r] = (zat(kEos) - rmax) - s_lse;
-      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = s_lse; }
+  if (warp == 0) {
+    // threshold from 32 group maxima, as in softmax_topk_kernel (kk <= 32)
+    float g = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < THREADS / 32; ++w) g = fmaxf(g, s_tmax[w * 32 + lane]);
+    float bm = g;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const float o = __shfl_sync(0xffffffffu, g, j);
+      rank += (o > g || (o == g && j < lane)) ? 1 : 0;
+    }
+    if (rank == kk - 1) s_tau = g;
+    if (lane == 0) s_max = bm;
+  }
+  __syncthreads();
+  const float rmax = s_max;
+  // the sum, and the blocks that reach the threshold
+  const float tau0 = s_tau;
+  float ssum = 0.f;
+  for (int b = tid; b < bl.n; b += THREADS) {
+    const float v = s_m[b];
+    if (v > -INFINITY) ssum = fmaf(s_q[b], __expf(v - rmax), ssum);
+    if (v >= tau0) {
+      const int pos = atomicAdd(&sh.count, 1);
+      if (pos < kTopkCap) sh.cv[pos] = v;
     }
   }
   __syncthreads();
-  int n = s_count;
-  if (rf.a0 && n > kTopkCap) {
-    // More elements than the buffer holds reach the widened threshold (a nearly flat row): pick the kk best
-    // of the one-product logits by exact sweeps and make those the candidates.  Their values are refined
-    // like any others below; an element within the error bound just beyond the kk-th can be missed here,
-    // which on a row this flat is a tie within the tolerance.
-    float last_v = INFINITY;
-    int last_i = -1;
-    for (int round = 0; round < kk; ++round) {
-      float bv = -INFINITY;
-      int bi = 0x7fffffff;
-      for (int i = tid; i < V; i += 256) {
-        const float v = zat(i);
-        const bool after = (v < last_v) || (v == last_v && i > last_i);
-        if (after && better(v, i, bv, bi)) { bv = v; bi = i; }
+  {
+    // tighter: the kk-th largest of those maxima is still reached by kk elements
+    const int m2 = sh.count;
+    if (m2 <= kTopkCap)
+      for (int c = tid; c < m2; c += THREADS) {
+        const float v = sh.cv[c];
+        int rank = 0;
+        for (int d = 0; d < m2; ++d) rank += (sh.cv[d] > v || (sh.cv[d] == v && d < c)) ? 1 : 0;
+        if (rank == kk - 1) s_tau = v;
+      }
+  }
+  __syncthreads();
+  if (tid == 0) sh.count = 0;
+  __syncthreads();
+  float tau = s_tau;
+  if (rf.a0) {     // every logit is within eps of its accurate value (see softmax_topk_kernel)
+    const float tot = warp_sum(lane < THREADS / 32 ? sh.red[lane] : 0.f);
+    tau -= 2.0f * (rf.eps_coef * sqrtf(tot) + 1e-5f);
+    if (zh) tau -= 2.0f * 4.9e-4f * fmaxf(fabsf(rmax), fabsf(tau));
+  }
+  // each warp tests 32 blocks at a time and reads those that reach the threshold, two at a time
+  for (int b0 = warp * 32; b0 < bl.n; b0 += THREADS) {
+    unsigned hit = __ballot_sync(0xffffffffu, b0 + lane < bl.n && s_m[b0 + lane] >= tau);
+    while (hit) {
+      int i[2];
+      float v[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int b = hit ? b0 + __ffs(hit) - 1 : -1;
+        hit &= hit - 1;
+        i[u] = b >= 0 ? b * kBlockCols + lane : V;
+        v[u] = i[u] < V ? (zh ? __half2float(zh[i[u]]) : z[i[u]]) : -INFINITY;
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-      }
-      __syncthreads();
-      if (lane == 0) { s_red[warp] = bv; s_redi[warp] = bi; }
-      __syncthreads();
-      bv = s_red[0]; bi = s_redi[0];
-      for (int w = 1; w < 8; ++w) if (better(s_red[w], s_redi[w], bv, bi)) { bv = s_red[w]; bi = s_redi[w]; }
-      if (tid == 0) { s_cv[round] = bv; s_ci[round] = bi; }
-      last_v = bv; last_i = bi;
+      for (int u = 0; u < 2; ++u)
+        if (i[u] < V && v[u] >= tau) {
+          const int pos = atomicAdd(&sh.count, 1);
+          if (pos < kTopkCap) { sh.cv[pos] = v[u]; sh.ci[pos] = i[u]; }
+        }
     }
-    __syncthreads();
-    n = 0;
-    while (n < kk && s_ci[n] != 0x7fffffff) ++n;   // fewer than kk elements in the row
-    __syncthreads();
-    if (tid == 0) s_count = n;
   }
-  if (rf.a0) {
-    // accurate values for the candidates (and for EOS, whose log-probability is always reported): one
-    // warp per candidate, fp32 FMAs over the two planes of both operands.  Each also yields the term by
-    // which the row's sum of exponentials changes when the accurate value replaces the one-product one:
-    // on a peaked row the few dominant logits ARE the normaliser, and their fp16-product error would
-    // otherwise go straight into every log-probability of the row.
-    const int nc = n;
-    for (int c = warp; c <= nc; c += 8) {
-      const int v = (c < nc) ? s_ci[c] : kEos;
-      const __half* w0 = rf.b0 + (size_t)v * rf.ldb;
-      const __half* w1 = rf.b1 + (size_t)v * rf.ldb;
-      float acc = 0.f;
-      for (int j = lane * 4; j < rf.K; j += 128) {
-        const uint2 q0 = *reinterpret_cast<const uint2*>(w0 + j);
-        const uint2 q1 = *reinterpret_cast<const uint2*>(w1 + j);
-        const __half2 h00 = *reinterpret_cast<const __half2*>(&q0.x), h01 = *reinterpret_cast<const __half2*>(&q0.y);
-        const __half2 h10 = *reinterpret_cast<const __half2*>(&q1.x), h11 = *reinterpret_cast<const __half2*>(&q1.y);
-        const float2 b00 = __half22float2(h00), b01 = __half22float2(h01), b10 = __half22float2(h10), b11 = __half22float2(h11);
-        acc = fmaf(s_a[j + 0], fmaf(b10.x, kPairInv, b00.x), acc);
-        acc = fmaf(s_a[j + 1], fmaf(b10.y, kPairInv, b00.y), acc);
-        acc = fmaf(s_a[j + 2], fmaf(b11.x, kPairInv, b01.x), acc);
-        acc = fmaf(s_a[j + 3], fmaf(b11.y, kPairInv, b01.y), acc);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) {
-        const float zv = acc + (rf.bias ? rf.bias[v] : 0.f);
-        const float za = (c < nc) ? s_cv[c] : zat(kEos);
-        const float delta = __expf(zv - rmax) - __expf(za - rmax);
-        if (c < nc) { s_cv[c] = zv; s_cd[c] = delta; }
-        else { s_eos = zv; s_eos_delta = delta; }
-      }
-    }
-    __syncthreads();
-    // the correction is summed in vocabulary order, so the result does not depend on the order in which
-    // the candidates happened to enter the buffer
-    bool eos_listed = false;
-    for (int c = tid; c < nc; c += 256) {
-      const int i = s_ci[c];
-      int pos = 0;
-      for (int d = 0; d < nc; ++d) pos += (s_ci[d] < i) ? 1 : 0;
-      s_co[pos] = s_cd[c];
-    }
-    __syncthreads();
-    if (tid == 0) {
-      float corr = 0.f;
-      for (int c = 0; c < nc; ++c) { corr += s_co[c]; eos_listed = eos_listed || (s_ci[c] == kEos); }
-      if (!eos_listed) corr += s_eos_delta;
-      const float bs = s_sum + corr;
-      s_lse = normalise ? logf(bs > 0.f ? bs : s_sum) : -rmax;
-      if (out.eos_logp) out.eos_logp[r] = (s_eos - rmax) - s_lse;
-      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = s_lse; }
-    }
-    __syncthreads();
-  }
-  const float rlse = s_lse;
-  if (n <= kTopkCap) {
-    // exact ranking of the candidates: value descending, index ascending
-    for (int c = tid; c < n; c += 256) {
-      const float v = s_cv[c];
-      const int i = s_ci[c];
-      int rank = 0;
-      for (int d = 0; d < n; ++d) rank += better(s_cv[d], s_ci[d], v, i) ? 1 : 0;
-      if (rank < kk) {
-        out.idx[(size_t)r * kk + rank] = i;
-        out.logp[(size_t)r * kk + rank] = (v - rmax) - rlse;
-      }
-    }
-    for (int q = n + tid; q < kk; q += 256) {  // fewer than kk elements in the row
-      out.idx[(size_t)r * kk + q] = -1;
-      out.logp[(size_t)r * kk + q] = -INFINITY;
-    }
-    return;
-  }
-  // ---- fallback: kk sweeps, each picking the best element after the previous pick ----
-  float last_v = INFINITY;
-  int last_i = -1;
-  for (int round = 0; round < kk; ++round) {
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int i = tid; i < V; i += 256) {
-      const float v = zat(i);
-      const bool after = (v < last_v) || (v == last_v && i > last_i);
-      if (after && better(v, i, bv, bi)) { bv = v; bi = i; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-    }
-    __syncthreads();
-    if (lane == 0) { s_red[warp] = bv; s_redi[warp] = bi; }
-    __syncthreads();
-    bv = s_red[0]; bi = s_redi[0];
-    for (int w = 1; w < 8; ++w) if (better(s_red[w], s_redi[w], bv, bi)) { bv = s_red[w]; bi = s_redi[w]; }
-    if (tid == 0) {
-      const bool valid = bi != 0x7fffffff;
-      out.idx[(size_t)r * kk + round] = valid ? bi : -1;
-      out.logp[(size_t)r * kk + round] = valid ? ((bv - rmax) - rlse) : -INFINITY;
-    }
-    last_v = bv; last_i = bi;
-  }
+  __syncthreads();     // (sh.red has been read by every warp)
+  topk_finish<THREADS>(sh, r, ssum, rmax, z, zh, V, kk, out, normalise, rf, s_a);
+  select_if_last<THREADS>(sel, out, r, s_union);
 }
 
 inline cudaError_t launch_softmax_topk(const float* logits, int ld, int V, int kk, int rows, const TopkOut& out, int normalise,
                                        cudaStream_t st, bool pdl = false, const float* pmax = nullptr, int pmax_ld = 0, int n_slots = 0,
-                                       const TopkRefine* refine = nullptr, const __half* logits16 = nullptr) {
+                                       const TopkRefine* refine = nullptr, const __half* logits16 = nullptr, const SelectArgs& sel = SelectArgs{}) {
   if (n_slots <= 0) pmax = nullptr;
   TopkRefine rf{};
   if (refine) rf = *refine;
   const size_t smem = rf.a0 ? sizeof(float) * (size_t)rf.K : 0;
-  return tc::launch_k(pdl, softmax_topk_kernel, dim3(rows), dim3(256), smem, st, logits, ld, V, kk, out, normalise, pmax, pmax_ld, n_slots, rf, refine ? logits16 : (const __half*)nullptr);
+  return tc::launch_k(pdl, softmax_topk_kernel, dim3(rows), dim3(256), smem, st, logits, ld, V, kk, out, normalise, pmax, pmax_ld, n_slots, rf, refine ? logits16 : (const __half*)nullptr, sel);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -821,176 +1251,6 @@ static __global__ void __launch_bounds__(256) ensemble_combine_kernel(EnsembleRo
     o[j] = (mode == 0) ? logf((float)acc) : (float)acc;
   }
   (void)inv_n;
-}
-
-// ---------------------------------------------------------------------------------------
-// Beam selection for one sentence and one step, all on the device.  Replaces
-// Decoder<T>::ExpandHypothesis (src/decoder.h:355-480) and, on a sentence's last step,
-// Decoder<T>::FinishCurrentHypotheses (src/decoder.h:502-525).
-// Candidate order = (score desc, beam asc, vocab asc), the defined order of the reference's
-// global heap.  START is skipped, EOS goes to the finished list without using a slot.
-struct BeamState {
-  int32_t* tok;        // [R] current token of each slot
-  float* score;        // [R]
-  int32_t* parent;     // [R] parent slot chosen by the last selection
-  int32_t* hist_tok;   // [Tcap][R]
-  int32_t* hist_parent;// [Tcap][R]
-  int32_t* fin_t;      // [B][fin_cap] step at which EOS was produced
-  int32_t* fin_b;      // [B][fin_cap] slot whose history the hypothesis continues
-  float* fin_score;    // [B][fin_cap]
-  int32_t* fin_n;      // [B]
-  int fin_cap;
-  int R;
-};
-struct TraceDev {
-  int32_t* cand_tok; float* cand_logp; int32_t* surv_tok; int32_t* surv_parent; float* surv_score; float* final_logp;
-  const int32_t* force_tok; const int32_t* force_parent; const float* force_score;
-  int Tm;
-  float* pt;                 // [n][Tm+1][k] attention centre of every forward (member 0), or null
-  float* gold_logp;          // [n][Tm][k] log-probability of the forced token of every slot (scoring)
-  const float* logits; int ld_logits; const float* row_stats;   // what gold_logp is computed from
-  TopkRefine rf;             // set when the logits are one-product values: the forced token's logit is recomputed accurately
-};
-// grid = active sentences, block = 256, dynamic smem = k*kk*24 + 8 bytes
-static __global__ void __launch_bounds__(256) beam_select_kernel(BeamState bs, const int32_t* __restrict__ cand_idx, const float* __restrict__ cand_logp,
-                                   const float* __restrict__ eos_logp, const int32_t* __restrict__ steps,
-                                   const int32_t* __restrict__ orig, int t, int k, float penalty, float diversity,
-                                   TraceDev tr) {
-  tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
-  tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
-  extern __shared__ unsigned char smraw[];
-  const int kk = k + 1;
-  const int ncap = k * kk;
-  float* cs = reinterpret_cast<float*>(smraw);   // candidate score
-  int* cb = reinterpret_cast<int*>(cs + ncap);   // beam
-  int* cv = cb + ncap;                           // vocab id
-  int* order = cv + ncap;                        // sorted position -> candidate
-  unsigned long long* key = reinterpret_cast<unsigned long long*>(order + ncap);  // sortable (score, beam, vocab)
-  const int sent = blockIdx.x;
-  const int T = steps[sent];
-  const int r0 = sent * k;
-  const int osent = orig[sent];
-  if (t > T) return;
-  if (t == T) {
-    if (threadIdx.x == 0) {
-      int n = bs.fin_n[sent];
-      for (int b = 0; b < k; ++b) {
-        const float lp = eos_logp[r0 + b];
-        if (tr.final_logp) tr.final_logp[(size_t)osent * k + b] = lp;
-        if (n < bs.fin_cap) {
-          bs.fin_t[(size_t)sent * bs.fin_cap + n] = t;
-          bs.fin_b[(size_t)sent * bs.fin_cap + n] = b;
-          bs.fin_score[(size_t)sent * bs.fin_cap + n] = bs.score[r0 + b] + (lp + penalty);
-          ++n;
-        }
-      }
-      bs.fin_n[sent] = n;
-    }
-    return;
-  }
-  const int cols = (t == 0) ? 1 : k;
-  const int n = cols * kk;
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const int b = c / kk, q = c - b * kk;
-    const float lp = cand_logp[(size_t)(r0 + b) * kk + q];
-    const int v = cand_idx[(size_t)(r0 + b) * kk + q];
-    const float rank_penalty = (float)(q + 1) * diversity;
-    cs[c] = (lp + bs.score[r0 + b]) - rank_penalty;
-    cb[c] = b; cv[c] = v;
-    order[c] = c;  // overwritten by the ranking below; keeps every entry valid even for NaN scores
-    {
-      // one 64-bit key, larger = earlier: score descending, then beam ascending, then vocabulary id ascending
-      const unsigned int fb = __float_as_uint(cs[c]);
-      const unsigned int ord = (fb & 0x80000000u) ? ~fb : (fb | 0x80000000u);
-      const unsigned int low = 0xFFFFFFFFu - (((unsigned int)b << 24) | ((unsigned int)v & 0xFFFFFFu));
-      key[c] = ((unsigned long long)ord << 32) | low;
-    }
-    if (tr.cand_tok) {
-      const size_t off = ((((size_t)osent * tr.Tm + t) * k + b) * kk) + q;
-      tr.cand_tok[off] = v; tr.cand_logp[off] = lp;
-    }
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    const unsigned long long kc = key[c];
-    int pos = 0;
-    for (int d = 0; d < n; ++d) pos += (key[d] > kc) ? 1 : 0;
-    order[pos] = c;
-  }
-  __syncthreads();
-  // The walk itself is serial (START is skipped, EOS leaves the beam without taking a slot), but it
-  // only touches shared memory; every global write happens afterwards, one thread per slot.
-  __shared__ int s_ntok[kMaxBeam + 1], s_npar[kMaxBeam + 1];
-  __shared__ float s_nscore[kMaxBeam + 1];
-  if (threadIdx.x == 0) {
-    int ns = 0;
-    int nf = bs.fin_n[sent];
-    for (int p = 0; p < n && ns < k; ++p) {
-      const int c = order[p];
-      const int v = cv[c];
-      if (v == kStart || v < 0) continue;
-      if (v == kEos) {
-        if (nf < bs.fin_cap) {
-          bs.fin_t[(size_t)sent * bs.fin_cap + nf] = t;
-          bs.fin_b[(size_t)sent * bs.fin_cap + nf] = cb[c];
-          bs.fin_score[(size_t)sent * bs.fin_cap + nf] = cs[c] + penalty;
-          ++nf;
-        }
-        continue;
-      }
-      s_ntok[ns] = v; s_npar[ns] = cb[c]; s_nscore[ns] = cs[c] + penalty;
-      ++ns;
-    }
-    for (; ns < k; ++ns) { s_ntok[ns] = kUnk; s_npar[ns] = 0; s_nscore[ns] = kDeadScore; }
-    bs.fin_n[sent] = nf;
-  }
-  // Scoring (force-decoding): log-probability of the forced token of every slot under its parent's row.
-  // With one-product logits the token's logit is recomputed from both planes of both operands, like the
-  // candidates in the softmax kernel; one warp per slot.
-  __shared__ float s_gold[kMaxBeam + 1];
-  if (tr.force_tok && tr.gold_logp && tr.logits) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int b = warp; b < k; b += (int)(blockDim.x >> 5)) {
-      const size_t off = ((size_t)osent * tr.Tm + t) * k + b;
-      const int npar = tr.force_parent[off];
-      const int prow = r0 + (npar >= 0 && npar < k ? npar : 0);
-      const int gt = tr.force_tok[off] >= 0 ? tr.force_tok[off] : 0;
-      float zv = 0.f;
-      if (tr.rf.a0) {
-        const __half* a0 = tr.rf.a0 + (size_t)prow * tr.rf.lda;
-        const __half* a1 = tr.rf.a1 + (size_t)prow * tr.rf.lda;
-        const __half* w0 = tr.rf.b0 + (size_t)gt * tr.rf.ldb;
-        const __half* w1 = tr.rf.b1 + (size_t)gt * tr.rf.ldb;
-        float acc = 0.f;
-        for (int j = lane; j < tr.rf.K; j += 32) {
-          const float a = fmaf(__half2float(a1[j]), kPairInv, __half2float(a0[j]));
-          const float w = fmaf(__half2float(w1[j]), kPairInv, __half2float(w0[j]));
-          acc = fmaf(a, w, acc);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        zv = acc + (tr.rf.bias ? tr.rf.bias[gt] : 0.f);
-      } else if (lane == 0) {
-        zv = tr.logits[(size_t)prow * tr.ld_logits + gt];
-      }
-      if (lane == 0) s_gold[b] = (zv - tr.row_stats[2 * prow]) - tr.row_stats[2 * prow + 1];
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < k) {
-    const int b = threadIdx.x;
-    int ntok = s_ntok[b], npar = s_npar[b];
-    float nscore = s_nscore[b];
-    const size_t off = ((size_t)osent * tr.Tm + t) * k + b;
-    if (tr.surv_tok) { tr.surv_tok[off] = ntok; tr.surv_parent[off] = npar; tr.surv_score[off] = nscore; }
-    if (tr.force_tok) {
-      ntok = tr.force_tok[off]; npar = tr.force_parent[off]; nscore = tr.force_score[off];
-      if (tr.gold_logp && tr.logits) tr.gold_logp[off] = s_gold[b];
-    }
-    bs.tok[r0 + b] = ntok; bs.parent[r0 + b] = npar; bs.score[r0 + b] = nscore;
-    bs.hist_tok[(size_t)t * bs.R + r0 + b] = ntok;
-    bs.hist_parent[(size_t)t * bs.R + r0 + b] = npar;
-  }
 }
 
 // ---------------------------------------------------------------------------------------
