@@ -69,6 +69,7 @@ Engine::~Engine() {
   for (void* p : allocs_) cudaFree(p);
   for (void* p : trace_allocs_) cudaFree(p);
   if (h_meta_) cudaFreeHost(h_meta_);
+  if (h_stage_) cudaFreeHost(h_stage_);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   for (auto e : kt_ev_) cudaEventDestroy(e);
@@ -335,11 +336,13 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
     if ((rc = alloc_state(states_[i]))) return rc;
     if (use_tc_ && (rc = alloc_state_tc(tc_states_[i]))) return rc;
   }
-  DA(d_off_, B + 1); DA(d_len_, B); DA(d_steps_, B); DA(d_orig_, B);
-  CK(cudaMallocHost(&h_meta_, sizeof(int32_t) * 4 * (B + 1)));
-  DA(d_tok_, R); DA(d_parent_, R); DA(d_score_, R);
+  // what one copy brings in and what one memset clears at the start of a decode lies together
+  DA(d_off_, 4 * (B + 1)); d_len_ = d_off_ + (B + 1); d_steps_ = d_off_ + 2 * (B + 1); d_orig_ = d_off_ + 3 * (B + 1);
+  CK(cudaMallocHost(&h_meta_, sizeof(int32_t) * (4 * (B + 1) + 1)));
+  h_err_ = h_meta_ + 4 * (B + 1);
+  DA(d_tok_, 3 * (size_t)R + B); d_parent_ = d_tok_ + R; d_score_ = reinterpret_cast<float*>(d_tok_ + 2 * (size_t)R); d_fin_n_ = d_tok_ + 3 * (size_t)R;
   DA(d_hist_tok_, (size_t)Tcap * R); DA(d_hist_parent_, (size_t)Tcap * R);
-  DA(d_fin_t_, (size_t)B * fin_cap); DA(d_fin_b_, (size_t)B * fin_cap); DA(d_fin_n_, B);
+  DA(d_fin_t_, (size_t)B * fin_cap); DA(d_fin_b_, (size_t)B * fin_cap);
   DA(d_rows_done_, B);
   CK(cudaMemset(d_rows_done_, 0, sizeof(int) * B));
   DA(d_fin_score_, (size_t)B * fin_cap); DA(d_fin_final_, (size_t)B * fin_cap);
@@ -580,14 +583,9 @@ int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, co
   if (max_len < Tm + 2) return fail(LINMT_EINVAL, "max_len smaller than max steps + 2");
   CK(cudaSetDevice(opt.device));
   CK(cudaEventRecord(ev0_, stream));
-  CK(cudaMemcpyAsync(d_off_, m_off, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemcpyAsync(d_len_, m_len, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemcpyAsync(d_steps_, m_steps, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemcpyAsync(d_orig_, m_orig, sizeof(int32_t) * n, cudaMemcpyHostToDevice, stream));
-  CK(cudaMemsetAsync(d_tok_, 0, sizeof(int32_t) * R, stream));     // START = 0 (src/decoder.h:339-342)
-  CK(cudaMemsetAsync(d_parent_, 0, sizeof(int32_t) * R, stream));
-  CK(cudaMemsetAsync(d_score_, 0, sizeof(float) * R, stream));
-  CK(cudaMemsetAsync(d_fin_n_, 0, sizeof(int32_t) * B, stream));
+  CK(cudaMemcpyAsync(d_off_, h_meta_, sizeof(int32_t) * 4 * (B + 1), cudaMemcpyHostToDevice, stream));
+  // tokens START = 0 (src/decoder.h:339-342), parents, scores, finished counts
+  CK(cudaMemsetAsync(d_tok_, 0, sizeof(int32_t) * (3 * (size_t)R + B), stream));
   cur_ids_ = d_ids;
   trace_dev_ = TraceDev{};
   if (trace_dev) {
@@ -632,11 +630,10 @@ int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, co
 }
 
 int Engine::finish_timing() {
+  CK(cudaMemcpyAsync(h_err_, d_tc_err_, sizeof(int), cudaMemcpyDeviceToHost, stream));
   CK(cudaStreamSynchronize(stream));
   if (use_tc_) {
-    int herr = 0;
-    CK(cudaMemcpy(&herr, d_tc_err_, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) return fail(LINMT_ECUDA, "a tensor-core GEMM gave up waiting on a barrier (results of this call are invalid)");
+    if (*h_err_) return fail(LINMT_ECUDA, "a tensor-core GEMM gave up waiting on a barrier (results of this call are invalid)");
   }
   CK(cudaEventElapsedTime(&stats.last_decode_ms, ev0_, ev1_));
   for (int c = 0; c < KC_COUNT; ++c) { class_ms[c] = 0.f; class_launches[c] = 0; }
@@ -663,42 +660,96 @@ int Engine::kt(int cls) {
   return LINMT_OK;
 }
 
-// Host-pointer front of decode_core: copies ids in, results out, in chunks of max_batch.
+// Order in which sentences are put into device batches: longest decode first, so that a batch's sentences end together
+// (a batch runs as many steps as its longest sentence).
+std::vector<int> batch_order(const int32_t* src_off, int n, const int32_t* steps) {
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    if (steps[a] != steps[b]) return steps[a] > steps[b];
+    return src_off[a + 1] - src_off[a] > src_off[b + 1] - src_off[b];
+  });
+  return order;
+}
+
+int Engine::reserve_host(size_t bytes) {
+  if (bytes <= h_stage_cap_) return LINMT_OK;
+  if (h_stage_) cudaFreeHost(h_stage_);
+  h_stage_ = nullptr; h_stage_cap_ = 0;
+  if (cudaMallocHost(&h_stage_, bytes) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMallocHost failed (host staging)");
+  h_stage_cap_ = bytes;
+  return LINMT_OK;
+}
+
+// One device batch of decode_host: sentences idx[0..cn) of the caller's arrays, results to their rows of the caller's
+// outputs.  Ids go in and results come out through one pinned buffer, one copy each way.
+int Engine::decode_chunk(const HostJob& jb, const int* idx, int cn, const linmt_trace* td, int Tm_all) {
+  const int nb = opt.nbest;
+  std::vector<int32_t> off(cn + 1, 0), st(cn);
+  for (int i = 0; i < cn; ++i) {
+    const int s = idx[i];
+    off[i + 1] = off[i] + std::max(0, jb.src_off[s + 1] - jb.src_off[s]);
+    st[i] = jb.steps[s];
+  }
+  const size_t n_ids = (size_t)off[cn];
+  // staging buffers grow with the longest input seen; the outgrown buffer is freed (the previous chunk's
+  // work on it ended with the synchronisation in finish_timing)
+  if (n_ids > d_ids_cap_) {
+    if (int rc_ = regrow(&d_ids_, n_ids + 1024)) return rc_;
+    d_ids_cap_ = n_ids + 1024;
+  }
+  const size_t need = (size_t)cn * nb, ml = (size_t)jb.max_len, per_align = ml * opt.max_src_len;
+  // device results of the batch, one behind the other: len, score, tok, vit, align
+  const size_t n_tok = need * ml, n_out = 2 * need + n_tok + (jb.out_vit ? n_tok : 0) + (jb.out_align ? need * per_align : 0);
+  if (n_out > out_cap_) {
+    if (int rc_ = regrow(&d_out_, n_out)) return rc_;
+    out_cap_ = n_out;
+  }
+  int32_t* d_len = d_out_;
+  float* d_score = reinterpret_cast<float*>(d_out_ + need);
+  int32_t* d_tok = d_out_ + 2 * need;
+  int32_t* d_vit = d_tok + n_tok;
+  float* d_align = reinterpret_cast<float*>(d_out_ + n_out - (jb.out_align ? need * per_align : 0));
+  if (int rc = reserve_host(std::max(n_ids, n_out) * 4)) return rc;
+  for (int i = 0; i < cn; ++i)
+    if (off[i + 1] > off[i]) std::memcpy(h_stage_ + off[i], jb.src_ids + jb.src_off[idx[i]], sizeof(int32_t) * (off[i + 1] - off[i]));
+  CK(cudaMemcpyAsync(d_ids_, h_stage_, n_ids * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+  int rc = decode_core(d_ids_, off.data(), cn, st.data(), jb.max_len, d_tok, d_len, d_score, jb.out_vit ? d_vit : nullptr,
+                       jb.out_align ? d_align : nullptr, td, Tm_all);
+  if (rc) { cudaStreamSynchronize(stream); return rc; }
+  CK(cudaMemcpyAsync(h_stage_, d_out_, n_out * 4, cudaMemcpyDeviceToHost, stream));
+  if ((rc = finish_timing())) return rc;
+  const int32_t* h = h_stage_;
+  for (int i = 0; i < cn; ++i) {
+    const size_t o = (size_t)idx[i] * nb, q = (size_t)i * nb;
+    std::memcpy(jb.out_len + o, h + q, sizeof(int32_t) * nb);
+    std::memcpy(jb.out_score + o, h + need + q, sizeof(float) * nb);
+    std::memcpy(jb.out_tok + o * ml, h + 2 * need + q * ml, sizeof(int32_t) * nb * ml);
+    if (jb.out_vit) std::memcpy(jb.out_vit + o * ml, h + 2 * need + n_tok + q * ml, sizeof(int32_t) * nb * ml);
+    if (jb.out_align)
+      std::memcpy(jb.out_align + o * per_align, h + (n_out - need * per_align) + q * per_align, sizeof(float) * nb * per_align);
+  }
+  return LINMT_OK;
+}
+
+// Host-pointer front of decode_core: device batches of at most max_batch sentences, filled in the order of batch_order;
+// a call with a trace keeps the caller's order (its records are laid out by it).
 int Engine::decode_host(const int32_t* src_ids, const int32_t* src_off, int n, const int32_t* steps, int max_len,
                         int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align,
                         const linmt_trace* trace) {
   if (n < 0 || !src_ids || !src_off || !steps || !out_tok || !out_len || !out_score) return fail(LINMT_EINVAL, "null argument");
   if (out_align && !opt.print_info) return fail(LINMT_EINVAL, "alignments need print_info = 1");
   CK(cudaSetDevice(opt.device));
-  const int nb = opt.nbest;
+  const HostJob jb{src_ids, src_off, steps, max_len, out_tok, out_len, out_score, out_vit, out_align};
   int Tm_all = 0;
   for (int i = 0; i < n; ++i) Tm_all = std::max(Tm_all, steps[i]);
   float total_ms = 0.f, gemm_ms = 0.f;
   int gemm_launches = 0;
+  std::vector<int> order;
+  if (trace || n <= B) { order.resize(n); std::iota(order.begin(), order.end(), 0); }
+  else order = batch_order(src_off, n, steps);
   for (int c0 = 0; c0 < n; c0 += B) {
     const int cn = std::min(B, n - c0);
-    const int32_t base = src_off[c0];
-    const size_t n_ids = (size_t)(src_off[c0 + cn] - base);
-    // staging buffers grow with the longest input seen; the outgrown buffer is freed (the previous chunk's
-    // work on it ended with the synchronisation in finish_timing)
-    if (n_ids > d_ids_cap_) {
-      if (int rc_ = regrow(&d_ids_, n_ids + 1024)) return rc_;
-      d_ids_cap_ = n_ids + 1024;
-    }
-    const size_t need = (size_t)cn * nb;
-    if (need > out_cap_len_ || max_len > out_cap_maxlen_) {
-      const size_t ml = std::max<size_t>(max_len, out_cap_maxlen_);
-      const size_t cap = std::max<size_t>(need, (size_t)B * nb);
-      int rc_;
-      if ((rc_ = regrow(&d_out_tok_, cap * ml)) || (rc_ = regrow(&d_out_vit_, cap * ml)) || (rc_ = regrow(&d_out_len_, cap)) ||
-          (rc_ = regrow(&d_out_score_, cap)))
-        return rc_;
-      if (opt.print_info && (rc_ = regrow(&d_out_align_, cap * ml * opt.max_src_len))) return rc_;
-      out_cap_len_ = cap; out_cap_maxlen_ = ml;
-    }
-    CK(cudaMemcpyAsync(d_ids_, src_ids + base, n_ids * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-    std::vector<int32_t> off(cn + 1);
-    for (int i = 0; i <= cn; ++i) off[i] = src_off[c0 + i] - base;
     // per-chunk device trace buffers
     linmt_trace td{};
     std::vector<std::pair<void*, std::pair<void*, size_t>>> copy_back;  // (device, (host, bytes))
@@ -746,18 +797,9 @@ int Engine::decode_host(const int32_t* src_ids, const int32_t* src_off, int n, c
       if ((rc = mk(n_s, 4, nullptr, trace->force_parent ? trace->force_parent + (size_t)c0 * Tm_all * k : nullptr, (void**)&td.force_parent))) return rc;
       if ((rc = mk(n_s, 4, nullptr, trace->force_score ? trace->force_score + (size_t)c0 * Tm_all * k : nullptr, (void**)&td.force_score))) return rc;
     }
-    int rc = decode_core(d_ids_, off.data(), cn, steps + c0, max_len, d_out_tok_, d_out_len_, d_out_score_,
-                         out_vit ? d_out_vit_ : nullptr, out_align ? d_out_align_ : nullptr, trace ? &td : nullptr, Tm_all);
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(out_tok + (size_t)c0 * nb * max_len, d_out_tok_, need * max_len * 4, cudaMemcpyDeviceToHost, stream));
-    CK(cudaMemcpyAsync(out_len + (size_t)c0 * nb, d_out_len_, need * 4, cudaMemcpyDeviceToHost, stream));
-    CK(cudaMemcpyAsync(out_score + (size_t)c0 * nb, d_out_score_, need * 4, cudaMemcpyDeviceToHost, stream));
-    if (out_vit) CK(cudaMemcpyAsync(out_vit + (size_t)c0 * nb * max_len, d_out_vit_, need * max_len * 4, cudaMemcpyDeviceToHost, stream));
-    if (out_align)
-      CK(cudaMemcpyAsync(out_align + (size_t)c0 * nb * max_len * opt.max_src_len, d_out_align_,
-                         need * max_len * opt.max_src_len * 4, cudaMemcpyDeviceToHost, stream));
+    if (int rc = decode_chunk(jb, order.data() + c0, cn, trace ? &td : nullptr, Tm_all)) return rc;
     for (auto& cb : copy_back) CK(cudaMemcpyAsync(cb.second.first, cb.first, cb.second.second, cudaMemcpyDeviceToHost, stream));
-    if ((rc = finish_timing())) return rc;
+    if (!copy_back.empty()) CK(cudaStreamSynchronize(stream));
     total_ms += stats.last_decode_ms; gemm_ms += stats.last_gemm_ms; gemm_launches += stats.last_gemm_launches;
   }
   stats.last_decode_ms = total_ms; stats.last_gemm_ms = gemm_ms; stats.last_gemm_launches = gemm_launches;
@@ -875,28 +917,20 @@ int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* s
   const int B = g0.B;
   if (e->n_engines() == 1 || trace || n <= B || !src_ids || !src_off || !steps || !out_tok || !out_len || !out_score)
     return g0.decode_host(src_ids, src_off, n, steps, max_len, out_tok, out_len, out_score, out_vit, out_align, trace);
-  // several devices: the job is cut into device batches of consecutive sentences; each device's host thread
-  // takes the next batch when it is free, the batches with the most decoder forwards first
+  // several devices: the same device batches as on one, dealt to the devices' host threads as they become free, the
+  // batches with the most decoder forwards first (they are in that order)
+  if (out_align && !g0.opt.print_info) { g0.err = "alignments need print_info = 1"; return LINMT_EINVAL; }
+  const linmt::Engine::HostJob jb{src_ids, src_off, steps, max_len, out_tok, out_len, out_score, out_vit, out_align};
+  const std::vector<int> sents = linmt::batch_order(src_off, n, steps);
   const int nchunks = (n + B - 1) / B;
-  std::vector<long long> cost(nchunks, 0);
-  for (int c = 0; c < nchunks; ++c) {
-    int tm = 0;
-    const int cn = std::min(B, n - c * B);
-    for (int i = 0; i < cn; ++i) tm = std::max(tm, steps[c * B + i]);
-    cost[c] = (long long)(tm + 1) * cn;
-  }
   std::vector<int> order(nchunks);
   std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-  const size_t nb = (size_t)g0.opt.nbest, ml = (size_t)max_len, ms = (size_t)g0.opt.max_src_len;
   std::vector<float> ms_per_engine(e->n_engines(), 0.f);
   std::mutex stat_mutex;
   int rc = linmt::run_on_engines(e, order, [&](Engine& g, int c) -> int {
-    const size_t c0 = (size_t)c * B;
-    const int cn = std::min(B, n - (int)c0);
-    int r = g.decode_host(src_ids, src_off + c0, cn, steps + c0, max_len, out_tok + c0 * nb * ml, out_len + c0 * nb,
-                          out_score + c0 * nb, out_vit ? out_vit + c0 * nb * ml : nullptr,
-                          out_align ? out_align + c0 * nb * ml * ms : nullptr, nullptr);
+    const int cn = std::min(B, n - c * B);
+    if (cudaSetDevice(g.opt.device) != cudaSuccess) { g.err = "cudaSetDevice failed"; return LINMT_ECUDA; }
+    int r = g.decode_chunk(jb, sents.data() + (size_t)c * B, cn, nullptr, 0);
     if (r == LINMT_OK) {
       std::lock_guard<std::mutex> lock(stat_mutex);
       for (int i = 0; i < e->n_engines(); ++i)

@@ -83,6 +83,12 @@ class Engine {
                   int32_t* d_out_tok, int32_t* d_out_len, float* d_out_score, int32_t* d_out_vit, float* d_out_align,
                   const linmt_trace* trace_dev, int trace_Tm);
   int finish_timing();
+  // a decode call's arrays (linmt_decode_batch)
+  struct HostJob {
+    const int32_t *src_ids, *src_off, *steps; int max_len;
+    int32_t *out_tok, *out_len; float* out_score; int32_t* out_vit; float* out_align;
+  };
+  int decode_chunk(const HostJob& jb, const int* idx, int cn, const linmt_trace* trace_dev, int Tm_all);
   int decode_host(const int32_t* src_ids, const int32_t* src_off, int n, const int32_t* steps, int max_len,
                   int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align,
                   const linmt_trace* trace);
@@ -165,7 +171,6 @@ class Engine {
   TraceDev trace_dev_{};
   size_t trace_pt_member_stride_ = 0;   // floats between two members' p_t records in the device trace buffer
   int enc_final_buf_ = 0;
-  size_t out_cap_maxlen_ = 0;
   std::vector<DevModel> models_;
   std::vector<DevState> states_;
   std::vector<void*> allocs_;
@@ -174,7 +179,8 @@ class Engine {
 
   // batch metadata (device) and pinned staging
   int32_t *d_off_ = nullptr, *d_len_ = nullptr, *d_steps_ = nullptr, *d_orig_ = nullptr;
-  int32_t* h_meta_ = nullptr;  // pinned [4][B+1]
+  int32_t* h_meta_ = nullptr;  // pinned [4][B+1], then the error flag
+  int32_t* h_err_ = nullptr;
   // beam state
   int32_t *d_tok_ = nullptr, *d_parent_ = nullptr, *d_hist_tok_ = nullptr, *d_hist_parent_ = nullptr;
   float* d_score_ = nullptr;
@@ -195,9 +201,11 @@ class Engine {
   // host staging for decode_host
   int32_t* d_ids_ = nullptr;
   size_t d_ids_cap_ = 0;
-  int32_t *d_out_tok_ = nullptr, *d_out_len_ = nullptr, *d_out_vit_ = nullptr;
-  float *d_out_score_ = nullptr, *d_out_align_ = nullptr;
-  size_t out_cap_len_ = 0;
+  int32_t* d_out_ = nullptr;      // results of a device batch: len | score | tok | vit | align
+  size_t out_cap_ = 0;
+  int32_t* h_stage_ = nullptr;    // pinned: ids of a batch, then its results
+  size_t h_stage_cap_ = 0;
+  int reserve_host(size_t bytes);
   // trace buffers (device), sized on demand
   std::vector<void*> trace_allocs_;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
@@ -227,6 +235,7 @@ struct linmt_engine {
 };
 
 namespace linmt {
+std::vector<int> batch_order(const int32_t* src_off, int n, const int32_t* steps);
 // Runs job(engine, item) for item = order[0], order[1], ... on the engines of a handle, one host thread per
 // engine, each taking the next item when it is free.  Returns the first error; engine 0's `err` names it.
 int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::function<int(Engine&, int)>& job);

@@ -39,7 +39,8 @@ struct RowsShape {
   int rp, units;       // rows rounded up to 16 = N of the MMA; rows rounded up to 4 = units of 4 rows x 32 columns
   int wstages, xstages, recv_bytes, smem_bytes;   // rings of weight and activation k-blocks
   int splits;          // K slices = cluster size
-  int leads, acc_stride, stacked, tmem_cols;
+  int leads, acc_stride, tmem_cols;
+  int alias;           // the partial sums' buffer lies in the rings (and waits until the whole cluster is done with them)
   int pdl;
 };
 
@@ -48,14 +49,21 @@ inline bool rows_set_splits(RowsShape* s, int K, int nt) {
   // partial sums: the units are dealt to the CTAs of the cluster, 512 bytes a slice
   s->recv_bytes = (s->units + s->splits - 1) / s->splits * s->splits * 512;
   const int w = nt * BM * 128, x = nt * s->rp * 128;
-  const int room = (s->tmem_cols == 512 ? kRowsSmemWhole : kRowsSmemHalf) - s->recv_bytes - kRowsBarBytes;
   const int nkb = (K / 64 + s->splits - 1) / s->splits;
-  s->wstages = (room - 2 * x) / w;
-  if (s->wstages > nkb) s->wstages = nkb;
-  if (s->wstages > kMaxStages) s->wstages = kMaxStages;
-  s->xstages = (room - s->wstages * w) / x;
-  if (s->xstages > s->wstages) s->xstages = s->wstages;
-  s->smem_bytes = s->wstages * w + s->xstages * x + s->recv_bytes + kRowsBarBytes;
+  for (s->alias = 0; s->alias < 2; ++s->alias) {
+    const int room = (s->tmem_cols == 512 ? kRowsSmemWhole : kRowsSmemHalf) - (s->alias ? 0 : s->recv_bytes) - kRowsBarBytes;
+    s->wstages = (room - 2 * x) / w;
+    if (s->wstages > nkb) s->wstages = nkb;
+    if (s->wstages > kMaxStages) s->wstages = kMaxStages;
+    if (s->wstages < 1) continue;
+    s->xstages = (room - s->wstages * w) / x;
+    if (s->xstages > s->wstages) s->xstages = s->wstages;
+    if (s->wstages >= 2 || nkb == 1 || s->alias) break;
+  }
+  if (s->alias > 1) return false;
+  const int rings = s->wstages * w + s->xstages * x;
+  if (s->alias && rings < s->recv_bytes) return false;
+  s->smem_bytes = rings + (s->alias ? 0 : s->recv_bytes) + kRowsBarBytes;
   const int least = s->tmem_cols == 512 ? kRowsSmemHalf + 3072 : kRowsSmemMin;
   if (s->smem_bytes < least) s->smem_bytes = least;
   return s->wstages >= 1 && s->xstages >= 1;
@@ -67,26 +75,30 @@ inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, b
   if (!(nt == 1 || (nt == 2 && fmt == 1))) return false;
   RowsShape s{};
   s.rp = (rows + 15) & ~15; s.units = (rows + 3) & ~3;
-  // f16 pair: w0 meets both planes of the activations in ONE instruction (N = 2 rp, the planes lie one behind the other),
-  // so an accumulator holds w0 x0 | w0 x1
-  s.tmem_cols = nt == 2 && s.rp > 32 ? 512 : 256;
-  s.stacked = nt == 2;
-  s.acc_stride = nt == 2 ? 2 * s.rp : s.rp;
-  s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
-  if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
   const int tiles = (N + BM - 1) / BM, nkb = K / 64;
   // One 128-column tile per cluster; K slices to fill the machine once.  CTAs of half an SM: measured best with as many
   // slices as a portable cluster has (4096 x 2048 at 12 rows: 10.2, 9.1, 8.7 us at 4, 6, 8 slices -- the more of the
   // weights are in flight when the activations arrive); CTAs of a whole SM: clusters of four are the largest of which
-  // the device holds enough at once (8.1 us at 4, 14 us at 6 slices, 3072 x 1024 at 64 rows).
-  const bool whole = s.tmem_cols == 512;
-  s.splits = (whole ? n_sm : 2 * n_sm) / tiles;
-  s.splits = s.splits < 1 ? 1 : (s.splits > (whole ? 4 : 8) ? (whole ? 4 : 8) : s.splits);
-  if (s.splits > nkb) s.splits = nkb;
-  if (!rows_set_splits(&s, K, nt)) return false;
-  if (nt == 2 && !one_chain && (nkb + s.splits - 1) / s.splits > 3 * s.leads) return false;   // a chain is at most three k-blocks
-  *out = s;
-  return true;
+  // the device holds enough at once (8.1 us at 4, 14 us at 6 slices, 3072 x 1024 at 64 rows) -- for more rows than the
+  // accumulators of half an SM's TMEM serve.  One plane and few rows: a CTA's slice fits its ring whole at half as many
+  // slices (4096 x 2048 at 12 rows: 6.2 us at 4, 6.6 at 8; at 64 rows 9.5 and 8.0).
+  for (int whole = 0; whole < 2; ++whole) {
+    s.splits = (whole || (nt == 1 && s.rp <= 32) ? n_sm : 2 * n_sm) / tiles;
+    s.splits = s.splits < 1 ? 1 : (s.splits > (whole ? 4 : 8) ? (whole ? 4 : 8) : s.splits);
+    if (s.splits > nkb) s.splits = nkb;
+    s.tmem_cols = whole ? 512 : 256;
+    // f16 pair: w0 meets both planes of the activations in ONE instruction (N = 2 rp, the planes lie one behind the
+    // other), so an accumulator holds w0 x0 | w0 x1
+    s.acc_stride = nt * s.rp;
+    s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
+    if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
+    const bool chains = nt == 1 || one_chain || (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
+    if (s.leads >= 1 && chains && rows_set_splits(&s, K, nt)) {
+      *out = s;
+      return true;
+    }
+  }
+  return false;
 }
 
 // four floats into the shared memory of a CTA of the cluster, their bytes counted on a barrier there
@@ -114,8 +126,9 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   const int X_BYTES = sh.rp * 128;             // one plane of an activation k-block
   const int WS = sh.wstages, XS = sh.xstages;
   const uint32_t xbase = base + (uint32_t)(WS * NT * W_BYTES);
-  const uint32_t recv = xbase + (uint32_t)(XS * NT * X_BYTES);
-  const uint32_t bars = recv + (uint32_t)sh.recv_bytes;   // W full[WS], W empty[WS], X full[XS], X empty[XS], accum, recv
+  const uint32_t rings_end = xbase + (uint32_t)(XS * NT * X_BYTES);
+  const uint32_t recv = sh.alias ? base : rings_end;
+  const uint32_t bars = rings_end + (sh.alias ? 0u : (uint32_t)sh.recv_bytes);   // W full[WS], W empty[WS], X full[XS], X empty[XS], accum, recv
   const uint32_t xbars = bars + 16u * WS, accum_bar = xbars + 16u * XS, recv_bar = accum_bar + 8u;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(rows_smem + (recv_bar + 8u - base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(rows_smem + (recv_bar + 12u - base));
@@ -204,7 +217,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     }
   } else if (warp <= issuers && lane == 0) {
     // warp 1: w0 times the activations (both planes of the f16 pair), warp 2 (f16 pair): w1 x0
-    const uint32_t idesc = make_idesc(BM, sh.stacked && warp == 1 ? 2 * sh.rp : sh.rp, FMT);
+    const uint32_t idesc = make_idesc(BM, NT == 2 && warp == 1 ? 2 * sh.rp : sh.rp, FMT);
     const int chain = NT == 1 ? nkb : (nkb + sh.leads - 1) / sh.leads;   // k-blocks per leading accumulator
     int ws = 0, xs = 0, in_chain = 0;
     uint32_t wph = 0, xph = 0;
@@ -231,7 +244,12 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   // Partial sums of a unit: [slice][32 columns][4 rows].
   const int q = warp & 3, half = warp >> 2;
   if (splits > 1) cluster_wait();
-  if (mbar_wait(accum_bar, 0, abort_flag)) {
+  const bool done = mbar_wait(accum_bar, 0, abort_flag);
+  if (sh.alias) {        // nobody writes into a ring that is still being read
+    __syncwarp();
+    if (splits > 1) cluster_sync_all(); else __syncthreads();
+  }
+  if (done) {
     tc_fence_after();
     const int chain = (nkb + sh.leads - 1) / sh.leads;
     const int used = NT == 1 ? 1 : (nkb + chain - 1) / chain;
@@ -243,7 +261,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
       for (int a = 0; a < ML; ++a)
         if (a < used) {
           tmem_ld8(at + (uint32_t)(a * sh.acc_stride), lead[a]);
-          if (NT > 1 && sh.stacked) tmem_ld8(at + (uint32_t)(a * sh.acc_stride + sh.rp), cross[a]);
+          if (NT > 1) tmem_ld8(at + (uint32_t)(a * sh.acc_stride + sh.rp), cross[a]);
         }
       if (NT > 1) tmem_ld8(at + (uint32_t)(sh.leads * sh.acc_stride), cross[ML]);
       tmem_wait_ld();
@@ -257,7 +275,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
           for (int a = 0; a < ML; ++a)
             if (a < used) {
               if (a > 0) v[i] += __uint_as_float(lead[a][i]);
-              if (sh.stacked) c += __uint_as_float(cross[a][i]);
+              c += __uint_as_float(cross[a][i]);
             }
           v[i] = fmaf(c, kF16PairInvScale, v[i]);
         }
