@@ -350,7 +350,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   DA(d_cand_idx_, (size_t)R * kk); DA(d_cand_logp_, (size_t)R * kk); DA(d_eos_logp_, R); DA(d_row_stats_, 2 * (size_t)R);
   pmax_ld_ = 4 * ((Vp + 47) / 48) + 4;   // four column blocks per tile, tiles at least 48 wide
   DA(d_pmax_, (size_t)R * pmax_ld_);
-  DA(d_psum_, (size_t)std::min(R, tc::kRowsMax) * pmax_ld_);
+  DA(d_psum_, (size_t)tc::kRowsMax * pmax_ld_);
   if (o.print_info) {
     DA(d_rec_align_, (size_t)Tcap * R * rec_win); DA(d_rec_lo_, (size_t)Tcap * R); DA(d_rec_vit_, (size_t)Tcap * R);
   }
@@ -459,7 +459,7 @@ int Engine::run_decoder_step(int mi, int t, int rows) {
     int32_t* rl = d_rec_lo_ ? d_rec_lo_ + (size_t)t * R : nullptr;
     int32_t* rv = d_rec_vit_ ? d_rec_vit_ + (size_t)t * R : nullptr;
     if (int rc = kt(KC_ATTENTION)) return rc;
-    if (int rc = launch_attention(mi, t, rows, u_alt, s.ctx, tc::Planes{}, 0, ra, rl, rv)) return rc;
+    if (int rc = launch_attention(mi, t, rows, k, u_alt, s.ctx, tc::Planes{}, 0, ra, rl, rv)) return rc;
   }
   // 5. attentional state htilde = tanh(W_c1 ctx + W_c2 h + b)
   {
@@ -481,7 +481,7 @@ int Engine::run_decoder_step(int mi, int t, int rows) {
 }
 
 // Attention of one decoder forward (both GEMM families).
-int Engine::launch_attention(int mi, int t, int rows, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
+int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
                              float* ra, int32_t* rl, int32_t* rv, bool fold) {
   // the record of member mi: [n][Tm+1][k] at pt + mi * (sentences of this device batch's record) * (Tm+1) * k
   const AttTrace at{trace_dev_.pt ? trace_dev_.pt + (size_t)mi * trace_pt_member_stride_ : nullptr, d_orig_, trace_dev_.Tm + 1, t};
@@ -493,10 +493,22 @@ int Engine::launch_attention(int mi, int t, int rows, const float* u_alt, float*
   const bool wide = rows <= n_sm_;   // a CTA of 1024 threads per SM
   CK(tc::launch_k(pdl_, wide ? attention_kernel<1024> : attention_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256),
                   wide ? attention_smem<1024>(win) : attention_smem<256>(win), stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
-                  (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, k, hs_sent_, hs_pos_, (int)opt.attention_mode,
+                  (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, kb, hs_sent_, hs_pos_, (int)opt.attention_mode,
                   (int)opt.attention_d, win, ra, rl, rv, ctx_planes, nt, rec_win, ens_member_code(mi), at, af));
   LAUNCHED();
   return LINMT_OK;
+}
+
+TopkRefine Engine::refinement(const tc::Planes& ht) const {
+  const DevModel& m = models_[0];
+  TopkRefine rf{};
+  rf.a0 = reinterpret_cast<const __half*>(ht.p[0]); rf.a1 = reinterpret_cast<const __half*>(ht.p[1]);
+  rf.lda = ht.ld;
+  rf.b0 = reinterpret_cast<const __half*>(m.p_voc_w.p[0]); rf.b1 = reinterpret_cast<const __half*>(m.p_voc_w.p[1]);
+  rf.ldb = m.p_voc_w.ld;
+  rf.bias = m.voc_b; rf.K = Hp;
+  rf.eps_coef = 1.1f * (1.0f / 1024.0f) * m.voc_wnorm_max;
+  return rf;
 }
 
 // Log-softmax statistics + per-beam top-(k+1), then beam selection (both paths).
@@ -513,16 +525,7 @@ int Engine::step_tail(int t, int rows) {
     if (n_models == 1) {
       if (int rc = kt(KC_SOFTMAX)) return rc;
       TopkRefine rf{};
-      if (refine_) {
-        const TcState& ts = tc_states_[0];
-        const DevModel& m0 = models_[0];
-        rf.a0 = reinterpret_cast<const __half*>(ts.panel_ht.p[0]); rf.a1 = reinterpret_cast<const __half*>(ts.panel_ht.p[1]);
-        rf.lda = ts.panel_ht.ld;
-        rf.b0 = reinterpret_cast<const __half*>(m0.p_voc_w.p[0]); rf.b1 = reinterpret_cast<const __half*>(m0.p_voc_w.p[1]);
-        rf.ldb = m0.p_voc_w.ld;
-        rf.bias = m0.voc_b; rf.K = Hp;
-        rf.eps_coef = 1.1f * (1.0f / 1024.0f) * m0.voc_wnorm_max;
-      }
+      if (refine_) rf = refinement(tc_states_[0].panel_ht);
       if (refine_) trace_dev_.rf = rf;
       sel.tr = trace_dev_;
       if (pblocks_) {
@@ -806,6 +809,82 @@ int Engine::decode_host(const int32_t* src_ids, const int32_t* src_off, int n, c
   return LINMT_OK;
 }
 
+// Log-probabilities of given targets (linmt_score_batch), in device batches of max_batch sentences, longest target first.
+int Engine::score_host(const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids, const int32_t* tgt_off, int n,
+                       float* out_logprob, float* out_token_logp, int max_tgt) {
+  CK(cudaSetDevice(opt.device));
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  auto tlen = [&](int i) { return tgt_off[i + 1] - tgt_off[i]; };
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return tlen(a) > tlen(b); });
+  float total_ms = 0.f;
+  for (int c0 = 0; c0 < n; c0 += B) {
+    const int cn = std::min(B, n - c0);
+    const int* idx = order.data() + c0;
+    const int steps = tlen(idx[0]) + 1;        // forwards: one per token and one for EOS
+    int Smax = 0;
+    size_t n_ids = 0;
+    for (int i = 0; i < cn; ++i) {
+      const int len = src_off[idx[i] + 1] - src_off[idx[i]];
+      if (len < 1) return fail(LINMT_EINVAL, "empty source sentence");
+      if (len > opt.max_src_len) return fail(LINMT_ELIMIT, "source sentence longer than max_src_len");
+      h_meta_[i] = (int32_t)n_ids; h_meta_[(B + 1) + i] = len; h_meta_[2 * (B + 1) + i] = steps - 1; h_meta_[3 * (B + 1) + i] = i;
+      n_ids += len;
+      Smax = std::max(Smax, len);
+    }
+    std::vector<int> n_act(steps, 0);
+    size_t rows = 0;
+    for (int t = 0; t < steps; ++t) {
+      while (n_act[t] < cn && tlen(idx[n_act[t]]) >= t) ++n_act[t];
+      rows += n_act[t];
+    }
+    // ids | tokens read [steps][cn] | tokens asked for [rows], up in one copy; log-probabilities [rows] back
+    const size_t n_up = n_ids + (size_t)steps * cn + rows;
+    if (n_up + rows > score_io_cap_) {
+      if (int rc = regrow(&score_io_, n_up + rows)) return rc;
+      score_io_cap_ = n_up + rows;
+    }
+    if (int rc = reserve_host((n_up + rows) * 4)) return rc;
+    int32_t *h_tok = h_stage_ + n_ids, *h_gold = h_tok + (size_t)steps * cn;
+    for (int i = 0; i < cn; ++i)
+      std::memcpy(h_stage_ + h_meta_[i], src_ids + src_off[idx[i]], sizeof(int32_t) * h_meta_[(B + 1) + i]);
+    size_t row = 0;
+    for (int t = 0; t < steps; ++t)
+      for (int i = 0; i < cn; ++i) {
+        const int32_t* tgt = tgt_ids + tgt_off[idx[i]];
+        h_tok[(size_t)t * cn + i] = t == 0 || i >= n_act[t] ? kStart : tgt[t - 1];
+        if (i < n_act[t]) h_gold[row++] = t < tlen(idx[i]) ? tgt[t] : kEos;
+      }
+    CK(cudaEventRecord(ev0_, stream));
+    CK(cudaMemcpyAsync(d_off_, h_meta_, sizeof(int32_t) * 4 * (B + 1), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(score_io_, h_stage_, n_up * 4, cudaMemcpyHostToDevice, stream));
+    cur_ids_ = score_io_;
+    trace_dev_ = TraceDev{};
+    kt_used_ = 0; rec_flops_ = 0.0;
+    float* d_logp = reinterpret_cast<float*>(score_io_ + n_up);
+    int rc = score_core_tc(cn, Smax, n_act, score_io_ + n_ids, score_io_ + n_ids + (size_t)steps * cn, d_logp);
+    if (rc) { cudaStreamSynchronize(stream); return rc; }
+    if ((rc = kt(KC_END))) return rc;
+    CK(cudaEventRecord(ev1_, stream));
+    const float* h_logp = reinterpret_cast<const float*>(h_stage_ + n_up);
+    CK(cudaMemcpyAsync(h_stage_ + n_up, d_logp, rows * 4, cudaMemcpyDeviceToHost, stream));
+    if ((rc = finish_timing())) return rc;
+    total_ms += stats.last_decode_ms;
+    row = 0;
+    for (int i = 0; i < cn; ++i) out_logprob[idx[i]] = 0.f;
+    for (int t = 0; t < steps; ++t)
+      for (int i = 0; i < n_act[t]; ++i, ++row) {
+        out_logprob[idx[i]] += h_logp[row];
+        if (out_token_logp) out_token_logp[(size_t)idx[i] * (max_tgt + 1) + t] = h_logp[row];
+      }
+    if (out_token_logp)
+      for (int i = 0; i < cn; ++i)
+        for (int t = tlen(idx[i]) + 1; t <= max_tgt; ++t) out_token_logp[(size_t)idx[i] * (max_tgt + 1) + t] = 0.f;
+  }
+  stats.last_decode_ms = total_ms;
+  return LINMT_OK;
+}
+
 int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::function<int(Engine&, int)>& job) {
   const int ne = h->n_engines();
   if (ne == 1 || order.size() <= 1) {
@@ -968,7 +1047,8 @@ int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* sr
     Tm = std::max(Tm, steps[i]);
   }
   if (out_token_logp && max_tgt < Tm) { g.err = "max_tgt smaller than the longest target"; return LINMT_EINVAL; }
-  // every beam slot is forced to the given token: slot b continues slot b
+  if (g.scores_rows()) return g.score_host(src_ids, src_off, tgt_ids, tgt_off, n, out_logprob, out_token_logp, max_tgt);
+  // CUDA-core path: a forced decode; every beam slot is forced to the given token, slot b continues slot b
   std::vector<int32_t> ftok((size_t)n * Tm * k, 2), fpar((size_t)n * Tm * k, 0);
   std::vector<float> fscore((size_t)n * Tm * k, 0.f), gold((size_t)n * Tm * k, 0.f), fin((size_t)n * k, 0.f);
   for (int i = 0; i < n; ++i)

@@ -89,6 +89,9 @@ class Engine {
     int32_t *out_tok, *out_len; float* out_score; int32_t* out_vit; float* out_align;
   };
   int decode_chunk(const HostJob& jb, const int* idx, int cn, const linmt_trace* trace_dev, int Tm_all);
+  int score_host(const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids, const int32_t* tgt_off, int n,
+                 float* out_logprob, float* out_token_logp, int max_tgt);
+  bool scores_rows() const { return use_tc_; }    // (the CUDA-core path scores through a forced decode)
   int decode_host(const int32_t* src_ids, const int32_t* src_off, int n, const int32_t* steps, int max_len,
                   int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align,
                   const linmt_trace* trace);
@@ -120,10 +123,16 @@ class Engine {
   int run_decoder_step(int mi, int t, int rows);
   int run_encoder_tc(int n, int Smax);
   int run_encoder_layers_tc(int n, int Smax);   // few sentences: layer by layer
-  int run_decoder_step_tc(int mi, int t, int rows);
+  // a step of scoring: the tokens read, where every member's htilde goes and where the previous step's is
+  struct ScoreStep { const int32_t* tok; const tc::Planes* ht; const tc::Planes* ht_prev; };
+  int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr);
+  int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax);
+  int score_core_tc(int n, int Smax, const std::vector<int>& n_act, const int32_t* d_tok, const int32_t* d_gold, float* d_logp);
+  int reserve_score(size_t rows);
+  TopkRefine refinement(const tc::Planes& ht) const;    // of one-product logits of these attentional states
   int step_tail(int t, int rows);
   bool pairs_available();   // clusters of two GEMM CTAs can be scheduled on the current device (engine_tc.cu)
-  int launch_attention(int mi, int t, int rows, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
+  int launch_attention(int mi, int t, int rows, int kb, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
                        float* rec_align, int32_t* rec_lo, int32_t* rec_vit, bool fold = false);
   int alloc_state_tc(TcState& s);
   int build_xw_tables();   // dec_xw of every model (tensor path, xw_table_)
@@ -191,7 +200,7 @@ class Engine {
   int32_t* d_cand_idx_ = nullptr;
   float *d_cand_logp_ = nullptr, *d_eos_logp_ = nullptr, *d_row_stats_ = nullptr;
   float* d_pmax_ = nullptr;   // [R][pmax_ld_] block maxima of the logits, by-product of the vocabulary GEMM
-  float* d_psum_ = nullptr;   // [min(R, 64)][pmax_ld_] sums of exponentials of the same blocks (few rows)
+  float* d_psum_ = nullptr;   // [64][pmax_ld_] sums of exponentials of the same blocks (few rows)
   int pmax_ld_ = 0;
   bool pblocks_ = false;      // the last vocabulary GEMM left maxima and sums of 32-column blocks
   int pmax_slots_ = 0;        // slots the last vocabulary GEMM filled (0 = none: the softmax finds its own maxima)
@@ -206,6 +215,26 @@ class Engine {
   int32_t* h_stage_ = nullptr;    // pinned: ids of a batch, then its results
   size_t h_stage_cap_ = 0;
   int reserve_host(size_t bytes);
+  // scoring workspace, made at the first call and kept
+  std::vector<tc::Planes> score_ht_;
+  size_t score_rows_ = 0;
+  int score_q_ = 0;
+  std::vector<float*> score_logits_;
+  __half* score_logits16_ = nullptr;
+  float *score_combined_ = nullptr, *score_candp_ = nullptr, *score_eos_ = nullptr, *score_stats_ = nullptr, *score_pmax_ = nullptr;
+  int32_t *score_idx_ = nullptr, *score_io_ = nullptr;
+  size_t score_io_cap_ = 0;
+  template <class T> int dalloc_bytes(T** p, size_t bytes) {
+    void* q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMalloc failed (scoring workspace)");
+    allocs_.push_back(q);
+    *p = static_cast<T*>(q);
+    return LINMT_OK;
+  }
+  void release(void* p) {
+    for (auto it = allocs_.begin(); p && it != allocs_.end(); ++it)
+      if (*it == p) { allocs_.erase(it); cudaFree(p); return; }
+  }
   // trace buffers (device), sized on demand
   std::vector<void*> trace_allocs_;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;

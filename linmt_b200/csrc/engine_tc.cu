@@ -396,12 +396,18 @@ int Engine::run_encoder_layers_tc(int n, int Smax) {
 }
 
 // One decoder forward, tensor-core path (see Engine::run_decoder_step).
-int Engine::run_decoder_step_tc(int mi, int t, int rows) {
+int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   DevModel& m = models_[mi];
   DevState& s = states_[mi];
   TcState& ts = tc_states_[mi];
   const bool feed = desc.feed_input && t > 0;
   pdl_gemm_ = true;
+  // scoring: one row per sentence continues itself, its tokens are given, and every step's htilde is kept
+  const int kb = sc ? 1 : k;
+  const int32_t* tok = sc ? sc->tok : d_tok_;
+  const int32_t* parent = sc ? nullptr : d_parent_;
+  const tc::Planes ht = sc ? sc->ht[mi] : ts.panel_ht;
+  const tc::Planes ht_prev = sc ? sc->ht_prev[mi] : ts.panel_ht;
   // where h_cur of layer l lives after its GEMM: the input slot of the consumer panel
   auto hcur_planes = [&](int l) -> const tc::Planes& { return (l + 1 < L) ? ts.panel[l + 1] : ts.panel_top; };
   auto hcur_col0 = [&](int l) { return (l + 1 < L) ? 0 : Hp; };
@@ -429,14 +435,14 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
     }
     if (feed)
       for (int p = 0; p < nt_; ++p)
-        add(ts.panel_ht.p[p], (long long)ts.panel_ht.ld * 2, ts.panel1.p[p] + 2 * Hp, (long long)ts.panel1.ld * 2, Hp * 2, 0);
+        add(ht_prev.p[p], (long long)ht_prev.ld * 2, ts.panel1.p[p] + 2 * Hp, (long long)ts.panel1.ld * 2, Hp * 2, 0);
     if (!m.dec_xw)   // with the input-term table the embedding never enters the GEMM
       for (int p = 0; p < nt_; ++p)
         add(m.p_emb_tgt.p[p], (long long)m.p_emb_tgt.ld * 2, ts.panel1.p[p], (long long)ts.panel1.ld * 2, Hp * 2, 1);
     jobs.n = nj;
     dim3 grid(rows, (nj + kGatherJobsPerBlock - 1) / kGatherJobsPerBlock);
     if (int rc = kt(KC_GATHER)) return rc;
-    CK(tc::launch_k(pdl_, row_gather_kernel, grid, dim3(128), 0, stream, jobs, (const int32_t*)d_parent_, (const int32_t*)d_tok_, V, k, t == 0 ? 1 : 0));
+    CK(tc::launch_k(pdl_, row_gather_kernel, grid, dim3(128), 0, stream, jobs, parent, tok, V, kb, t == 0 ? 1 : 0));
     LAUNCHED();
   }
   // 2. LSTM stack
@@ -448,7 +454,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
     else {
       e.c_prev = (t & 1) ? s.c_cur[l] : s.c_prev[l];
       e.c_out = (t & 1) ? s.c_prev[l] : s.c_cur[l];
-      e.c_parent = d_parent_; e.c_k = k;
+      e.c_parent = parent; e.c_k = kb;
     }
     e.h_out1 = hcur_planes(l); e.h1_col0 = hcur_col0(l);
     e.h_out2 = no_planes(); e.h2_col0 = 0;
@@ -462,7 +468,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
       // K columns (h_prev | htilde_prev) only: the x columns of panel and weights are skipped, their term comes from the table
       tc::Planes wrest = m.p_dec_w[0];
       for (int p = 0; p < 3; ++p) if (wrest.p[p]) wrest.p[p] += Hp;
-      e.xw = m.dec_xw; e.x_tok = d_tok_; e.x_ld = 4 * Hp; e.x_vocab = V; e.x_unk = kUnk;
+      e.xw = m.dec_xw; e.x_tok = tok; e.x_ld = 4 * Hp; e.x_vocab = V; e.x_unk = kUnk;
       K -= Hp;
       rc = tc_gemm(hprev_planes(0), Hp, R, wrest, rows, 4 * Hp, K, e);
     } else {
@@ -490,15 +496,16 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
   }
   // 4. scores, softmax x Gaussian, context (written into the attention-output panel)
   {
-    float* ra = d_rec_align_ ? d_rec_align_ + (size_t)t * R * rec_win : nullptr;
-    int32_t* rl = d_rec_lo_ ? d_rec_lo_ + (size_t)t * R : nullptr;
-    int32_t* rv = d_rec_vit_ ? d_rec_vit_ + (size_t)t * R : nullptr;
+    const bool rec = d_rec_align_ && !sc;
+    float* ra = rec ? d_rec_align_ + (size_t)t * R * rec_win : nullptr;
+    int32_t* rl = rec ? d_rec_lo_ + (size_t)t * R : nullptr;
+    int32_t* rv = rec ? d_rec_vit_ + (size_t)t * R : nullptr;
     if (int rc = kt(KC_ATTENTION)) return rc;
-    if (int rc = launch_attention(mi, t, rows, u_alt, nullptr, att_fold_ ? ts.panel_ht : ts.panel_top, nt_, ra, rl, rv, att_fold_)) return rc;
+    if (int rc = launch_attention(mi, t, rows, kb, u_alt, nullptr, att_fold_ ? ht : ts.panel_top, nt_, ra, rl, rv, att_fold_)) return rc;
   }
   // 5. htilde = tanh(W_c1 ctx + W_c2 h + b) (with the fold the attention kernel has written it already)
   if (!att_fold_) {
-    tc::TcEpiBiasTanh e{m.att_bout, ts.panel_ht, 0, nt_};
+    tc::TcEpiBiasTanh e{m.att_bout, ht, 0, nt_};
     if (int rc0 = kt(KC_ATTOUT)) return rc0;
     int rc;
     if (att_merge_) {
@@ -511,19 +518,109 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows) {
     if (rc) return rc;
   }
   // 6. logits
-  {
-    tc::TcEpiF32 e{m.voc_b, s.logits, Vp, 0};
-    if (logits16_) e.out16 = s.logits16;   // the softmax of this step is their only reader
-    pmax_slots_ = 0; pblocks_ = false;
-    if (n_models == 1 && pmax_on_) { e.pmax = d_pmax_; e.pmax_ld = pmax_ld_; e.n_valid = V; }
-    if (int rc = kt(KC_VOCAB)) return rc;
-    // Logits feed only the softmax of their own step: the tensor core's truncation bias over one
-    // K = Hp chain (~32 ulp of the accumulator, 2e-7 relative on a log-probability) does not
-    // accumulate over steps as it does through the recurrent products, so this GEMM runs its
-    // leading product as one chain (no intermediate drains: 5 % faster).
-    int rc = tc_gemm(ts.panel_ht, 0, R, m.p_voc_w, rows, Vp, Hp, e, nt_vocab_, Hp / 32);
-    if (rc) return rc;
+  if (sc) return LINMT_OK;
+  if (int rc = kt(KC_VOCAB)) return rc;
+  return vocab_gemm(mi, ts.panel_ht, R, rows, s.logits, s.logits16, d_pmax_);
+}
+
+// Logits of `rows` attentional states.
+int Engine::vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax) {
+  DevModel& m = models_[mi];
+  tc::TcEpiF32 e{m.voc_b, logits, Vp, 0};
+  if (logits16_) e.out16 = logits16;   // the softmax of this step is their only reader
+  pmax_slots_ = 0; pblocks_ = false;
+  if (n_models == 1 && pmax_on_) { e.pmax = pmax; e.pmax_ld = pmax_ld_; e.n_valid = V; }
+  // Logits feed only the softmax of their own step: the tensor core's truncation bias over one
+  // K = Hp chain (~32 ulp of the accumulator, 2e-7 relative on a log-probability) does not
+  // accumulate over steps as it does through the recurrent products, so this GEMM runs its
+  // leading product as one chain (no intermediate drains: 5 % faster).
+  return tc_gemm(ht, 0, rows_cap, m.p_voc_w, rows, Vp, Hp, e, nt_vocab_, Hp / 32);
+}
+
+// Scores of given targets, tensor-core path: one device batch of n sentences, longest target first.  Nothing of a step
+// depends on the step's logits, so only the recurrence runs step by step, on ONE row per sentence (a forced decode ran a
+// row per beam slot), and the vocabulary product, its softmax and the given tokens' log-probabilities follow for all
+// positions together.
+//   n_act[t] sentences run step t; d_tok [steps][n] the tokens read (START first); d_gold / d_logp the tokens asked for
+//   (EOS last) and their log-probabilities, packed: the first n_act[t] sentences of step 0, of step 1, ...
+int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const int32_t* d_tok, const int32_t* d_gold, float* d_logp) {
+  const int steps = (int)n_act.size();
+  size_t rows_all = 0;
+  for (int a : n_act) rows_all += a;
+  if (int rc = reserve_score(rows_all)) return rc;
+  if (int rc = run_encoder_tc(n, Smax)) return rc;
+  enc_final_buf_ = Smax & 1;
+  std::vector<tc::Planes> prev = score_ht_, cur = score_ht_;
+  size_t row = 0;
+  for (int t = 0; t < steps; ++t) {
+    for (int mi = 0; mi < n_models; ++mi) {
+      for (int p = 0; p < nt_; ++p) cur[mi].p[p] = score_ht_[mi].p[p] + row * Hp;
+      const ScoreStep sc{d_tok + (size_t)t * n, cur.data(), prev.data()};
+      if (int rc = run_decoder_step_tc(mi, t, n_act[t], &sc)) return rc;
+    }
+    prev = cur;
+    row += n_act[t];
+    stats.decoder_row_steps += n_act[t];
+    stats.sentence_steps += n_act[t];
   }
+  for (size_t r0 = 0; r0 < rows_all; r0 += score_q_) {
+    const int rows = (int)std::min<size_t>(score_q_, rows_all - r0);
+    TopkOut o{score_idx_, score_candp_, score_eos_, score_stats_};
+    TopkRefine rf{};
+    for (int mi = 0; mi < n_models; ++mi) {
+      tc::Planes a = score_ht_[mi];
+      for (int p = 0; p < nt_; ++p) a.p[p] += r0 * Hp;
+      if (mi == 0 && refine_) rf = refinement(a);
+      if (int rc = vocab_gemm(mi, a, (int)std::min<size_t>(score_q_, score_rows_ - r0), rows, score_logits_[mi], score_logits16_, score_pmax_)) return rc;
+    }
+    const float* logits = score_logits_[0];
+    int normalise = 1;
+    if (n_models > 1) {
+      EnsembleRows er{};
+      for (int mi = 0; mi < n_models; ++mi) er.logits[mi] = score_logits_[mi];
+      er.n = n_models;
+      CK(tc::launch_k(pdl_, ensemble_combine_kernel, dim3(rows), dim3(256), 0, stream, er, Vp, V, (int)opt.ensemble_mode, score_combined_));
+      LAUNCHED();
+      logits = score_combined_;
+      normalise = opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0;
+    }
+    CK(launch_softmax_topk(logits, Vp, V, kk, rows, o, normalise, stream, pdl_, score_pmax_, pmax_ld_, pmax_slots_, refine_ ? &rf : nullptr,
+                           logits16_ ? score_logits16_ : nullptr));
+    LAUNCHED();
+    CK(tc::launch_k(pdl_, gold_logp_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, d_gold + r0, rows, logits, Vp, V, (const float*)score_stats_, rf, d_logp + r0));
+    LAUNCHED();
+  }
+  return LINMT_OK;
+}
+
+// Workspace of score_core_tc, kept between calls: attentional states of every position, and logits of as many rows at a
+// time as 64 Mi values hold.
+int Engine::reserve_score(size_t rows) {
+  int rc;
+  if (rows > score_rows_) {
+    for (auto& p : score_ht_)
+      for (int t = 0; t < nt_; ++t) release(p.p[t]);
+    tmap_cache_.clear();      // (maps of the released panels)
+    score_rows_ = 0;
+    score_ht_.assign(n_models, tc::Planes{});
+    for (int mi = 0; mi < n_models; ++mi)
+      if ((rc = alloc_planes(score_ht_[mi], rows, Hp))) return rc;
+    score_rows_ = rows;
+  }
+  if (score_q_) return LINMT_OK;
+  const size_t cap = std::max<size_t>(128, (((size_t)64 << 20) / Vp) & ~(size_t)127);
+  score_logits_.assign(n_models, nullptr);
+  if (logits16_) {
+    if ((rc = dalloc_bytes(&score_logits16_, cap * Vp * 2))) return rc;
+  } else {
+    for (int mi = 0; mi < n_models; ++mi)
+      if ((rc = dalloc_bytes(&score_logits_[mi], cap * Vp * 4))) return rc;
+  }
+  if (n_models > 1 && (rc = dalloc_bytes(&score_combined_, cap * Vp * 4))) return rc;
+  if ((rc = dalloc_bytes(&score_idx_, cap * kk * 4)) || (rc = dalloc_bytes(&score_candp_, cap * kk * 4)) || (rc = dalloc_bytes(&score_eos_, cap * 4)) ||
+      (rc = dalloc_bytes(&score_stats_, cap * 8)) || (rc = dalloc_bytes(&score_pmax_, cap * pmax_ld_ * 4)))
+    return rc;
+  score_q_ = (int)cap;
   return LINMT_OK;
 }
 

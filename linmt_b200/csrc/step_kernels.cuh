@@ -93,7 +93,7 @@ static __global__ void row_gather_kernel(GatherJobs jobs, const int32_t* __restr
   const int r = blockIdx.x;
   const int j0 = blockIdx.y * kGatherJobsPerBlock;
   const int sent = r / k;
-  const long long prow = src_per_sentence ? sent : sent * k + parent[r];
+  const long long prow = src_per_sentence ? sent : parent ? sent * k + parent[r] : r;
   // every thread moves 16 bytes of up to four jobs at a time: all loads first, then the stores
   const unsigned char* src[kGatherJobsPerBlock];
   unsigned char* dst[kGatherJobsPerBlock];
@@ -1160,6 +1160,34 @@ inline cudaError_t launch_softmax_topk(const float* logits, int ld, int V, int k
   if (refine) rf = *refine;
   const size_t smem = rf.a0 ? sizeof(float) * (size_t)rf.K : 0;
   return tc::launch_k(pdl, softmax_topk_kernel, dim3(rows), dim3(256), smem, st, logits, ld, V, kk, out, normalise, pmax, pmax_ld, n_slots, rf, refine ? logits16 : (const __half*)nullptr, sel);
+}
+
+// Log-probability of one given token per row (scoring), from the row's softmax statistics; with one-product logits the
+// token's logit is recomputed from both planes of both operands, like the candidates above.  One warp per row.
+static __global__ void __launch_bounds__(256) gold_logp_kernel(const int32_t* __restrict__ gold, int rows, const float* __restrict__ logits, int ld, int V,
+                                                               const float* __restrict__ row_stats, TopkRefine rf, float* __restrict__ out) {
+  tc::pdl_launch_dependents();
+  tc::pdl_wait();
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  int g = gold[r];
+  if (g < 0) g = 0;
+  if (g >= V) g = kUnk;
+  float zv = 0.f;
+  if (rf.a0) {
+    const __half *a0 = rf.a0 + (size_t)r * rf.lda, *a1 = rf.a1 + (size_t)r * rf.lda;
+    const __half *w0 = rf.b0 + (size_t)g * rf.ldb, *w1 = rf.b1 + (size_t)g * rf.ldb;
+    float acc = 0.f;
+    for (int j = lane; j < rf.K; j += 32) {
+      const float x = fmaf(__half2float(a1[j]), kPairInv, __half2float(a0[j]));
+      const float w = fmaf(__half2float(w1[j]), kPairInv, __half2float(w0[j]));
+      acc = fmaf(x, w, acc);
+    }
+    zv = warp_sum(acc) + (rf.bias ? rf.bias[g] : 0.f);
+  } else {
+    zv = logits[(size_t)r * ld + g];
+  }
+  if (lane == 0) out[r] = (zv - row_stats[2 * r]) - row_stats[2 * r + 1];
 }
 
 // ---------------------------------------------------------------------------------------

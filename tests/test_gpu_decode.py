@@ -551,3 +551,22 @@ def test_file_mode_on_two_devices(cuda_lib, tmp_path):
         ds.close()
         outs.append((tmp_path / f"{name}.out").read_text())
     assert outs[0] == outs[1] and outs[0].count("================") == len(lines)
+
+
+@pytest.mark.parametrize("n_sent,beam,members,max_batch", [(1, 1, 1, 8), (8, 3, 1, 3), (8, 2, 2, 8), (37, 1, 1, 16)])
+def test_scores_match_a_forced_decode(cuda_lib, c1, n_sent, beam, members, max_batch):
+    """linmt_score_batch runs one row per sentence and all vocabulary products after the recurrence; the CUDA-core path
+    scores through a forced decode.  Ragged targets, several device batches, ensembles, one sentence."""
+    from linmt_b200 import decoder
+    c, blob, _ = c1
+    blobs = [blob] + [synth.make_blob(c.desc, 30 + m) for m in range(1, members)]
+    sents = synth.make_sentences(n_sent, 1, 20, c.desc.Vs, 1.1, 5, lambda s: s + 1)
+    rng = np.random.default_rng(n_sent)
+    targets = [rng.integers(0, c.desc.V, size=int(m)) for m in rng.integers(1, 25, size=n_sent)]
+    res = []
+    for path in ("auto", "simt"):
+        dec = decoder.Decoder(c.desc, blobs, beam=beam, max_batch=max_batch, max_src_len=32, max_steps=64, gemm_path=path)
+        res.append(dec.score(sents, targets))
+        dec.close()
+    np.testing.assert_allclose(res[0][1], res[1][1], rtol=RTOL_FP32, atol=1e-6)
+    np.testing.assert_allclose(res[0][0], res[1][0], rtol=RTOL_FP32)
