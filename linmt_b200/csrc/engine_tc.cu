@@ -197,15 +197,17 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   }
   // many waves of tiles whose leading product is one chain: one persistent CTA per SM
   const long tiles = (long)((M + tc::BM - 1) / tc::BM) * ((N + bn - 1) / bn);
+  if constexpr (Epi::kHasBlock) {
   if (ppair) {
     const int pdl = sh.pdl;
-    sh = tc::make_shape_persist_pair(bn, nt, bk, fmt_);
+    sh = tc::make_shape_persist_pair(bn, fmt_);
     sh.pdl = pdl;
-    if (fmt_ == 1) CK((tc::launch_gemm_tc_persist_pair<1, 64, 1, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_)));
-    else CK((tc::launch_gemm_tc_persist_pair<1, 64, 0, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_)));
+    if (fmt_ == 1) CK((tc::launch_gemm_tc_persist_pair<1, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_)));
+    else CK((tc::launch_gemm_tc_persist_pair<0, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_)));
     LAUNCHED();
     ++stats.pair_launches;
     return LINMT_OK;
+  }
   }
   if (persist_ && splits == 1 && tiles > n_sm_ && ((nt == 2 && drain >= K / 32) || one_plane_logits)) {
     if (nt == 1) {

@@ -185,6 +185,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// The warp's number and one elected lane, both in a form that the compiler knows to be uniform over the warp: the
+// operands of tcgen05.mma are uniform registers, and a loop that only one lane enters has to move every one of them over
+// for every instruction.  The issuing loops are therefore run by the whole warp, with the instruction itself under the
+// elected lane.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // Shared-memory matrix descriptor of a K-major tile whose rows are 64 bytes (BK bf16) with
 // the 64-byte swizzle TMA wrote (8-row groups 512 bytes apart), or 128-byte rows with the
 // 128-byte swizzle (groups 1024 bytes apart).
@@ -300,6 +311,7 @@ __device__ __forceinline__ float tanh_fast(float x) {
 // 32 different lines per instruction; staging a block of up to 64 columns and storing it back
 // with consecutive lanes on consecutive addresses cuts the memory-pipe passes 4-8x (measured: the
 // epilogue was 7.6-7.9 us of a 29-36 us tile).
+constexpr int kStagedStride = 36;                        // floats per row of a persistent kernel's staging area: two 16-column chunks + 4
 constexpr int kEpiBlockChunks = 4;                       // 16-column chunks a warp owns at most
 constexpr int kEpiScratchStride = 68;                    // floats per staged row (64 + 4: conflict-free float4 rows)
 constexpr int kEpiScratchBytes = kEpiStagingBytes / kEpiWarps;   // per warp: 32 x 68 floats, or the LSTM epilogue's c | h planes | h
@@ -386,31 +398,44 @@ struct TcEpiLstm {
   static constexpr bool kHasBlock = true;
   static constexpr bool kHasPmax = false;
   __device__ __forceinline__ void block(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, int /*slot*/) const {
+    block_of<kEpiBlockChunks, 3>(row0, lane, M, col_first, nch, v, sbuf);
+  }
+  // up to two chunks at a time in a small staging area of the warp's own (persistent kernels, one plane)
+  __device__ __forceinline__ float staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf) const {
+    block_of<2, 1>(row0, lane, M, col_first, nch, v, sbuf);
+    return 0.f;
+  }
+  // CH = most chunks, PL = planes there is room for
+  template <int CH, int PL>
+  __device__ __forceinline__ void block_of(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf) const {
+    constexpr int CS = 4 * CH + 4;           // floats per staged row of c (and of h in fp32)
+    constexpr int HS = CH == 4 ? 24 : 12;    // 16-bit values per staged row of an h plane
+    constexpr int XS = 16 * CH + 4;          // floats per staged row of the input term
     const int nq = nch;                      // float4 groups (4 hidden units each) per row
     const int j_first = col_first >> 2;
     const int row = row0 + lane;
     const bool valid = row < M;
     const bool active = valid && ((row_len == nullptr) || (pos < row_len[row]));
-    float* cs = sbuf;                                            // [32][20] floats: c_prev in, c out
-    unsigned short* hs = reinterpret_cast<unsigned short*>(sbuf + 32 * 20);   // [planes][32][24] 16-bit
-    float* hf = sbuf + 32 * 20 + 3 * 32 * 12;                    // [32][20] floats: h in fp32 (only if h_f32)
+    float* cs = sbuf;                                            // [32][CS] floats: c_prev in, c out
+    unsigned short* hs = reinterpret_cast<unsigned short*>(sbuf + 32 * CS);   // [planes][32][HS] 16-bit
+    float* hf = sbuf + 32 * CS + PL * 32 * HS / 2;               // [32][CS] floats: h in fp32 (only if h_f32)
     if (xw) {
       // the rows of the input-term table for this block, staged coalesced, then added lane = row
       const int nq4 = 4 * nch;
       for (int s = lane; s < 32 * nq4; s += 32) {
         const int r = s / nq4, g = s - r * nq4;
         if (row0 + r < M)
-          *reinterpret_cast<float4*>(sbuf + r * kEpiScratchStride + 4 * g) =
+          *reinterpret_cast<float4*>(sbuf + r * XS + 4 * g) =
               *reinterpret_cast<const float4*>(xw + (size_t)x_row(row0 + r) * x_ld + col_first + 4 * g);
       }
       __syncwarp();
       if (valid) {
 #pragma unroll
-        for (int ci = 0; ci < kEpiBlockChunks; ++ci) {
+        for (int ci = 0; ci < CH; ++ci) {
           if (ci < nch) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const float4 t = *reinterpret_cast<const float4*>(sbuf + lane * kEpiScratchStride + 16 * ci + 4 * q);
+              const float4 t = *reinterpret_cast<const float4*>(sbuf + lane * XS + 16 * ci + 4 * q);
               v[ci][4 * q] += t.x; v[ci][4 * q + 1] += t.y; v[ci][4 * q + 2] += t.z; v[ci][4 * q + 3] += t.w;
             }
           }
@@ -422,15 +447,15 @@ struct TcEpiLstm {
     for (int s = lane; s < 32 * nq; s += 32) {
       const int r = s / nq, g = s - r * nq;
       if (row0 + r < M)
-        *reinterpret_cast<float4*>(cs + r * 20 + 4 * g) =
+        *reinterpret_cast<float4*>(cs + r * CS + 4 * g) =
             *reinterpret_cast<const float4*>(c_prev + (size_t)c_src_row(row0 + r) * ldc + j_first + 4 * g);
     }
     __syncwarp();
     if (active) {
 #pragma unroll
-      for (int ci = 0; ci < kEpiBlockChunks; ++ci) {
+      for (int ci = 0; ci < CH; ++ci) {
         if (ci < nch) {
-          const float4 cp = *reinterpret_cast<const float4*>(cs + lane * 20 + 4 * ci);
+          const float4 cp = *reinterpret_cast<const float4*>(cs + lane * CS + 4 * ci);
           const float cpv[4] = {cp.x, cp.y, cp.z, cp.w};
           float c[4], h[4];
 #pragma unroll
@@ -443,9 +468,9 @@ struct TcEpiLstm {
             c[u] = gf * cpv[u] + gi * gg;
             h[u] = go * tanh_fast(c[u]);
           }
-          *reinterpret_cast<float4*>(cs + lane * 20 + 4 * ci) = make_float4(c[0], c[1], c[2], c[3]);
+          *reinterpret_cast<float4*>(cs + lane * CS + 4 * ci) = make_float4(c[0], c[1], c[2], c[3]);
           if (h_f32)
-            *reinterpret_cast<float4*>(hf + lane * 20 + 4 * ci) =
+            *reinterpret_cast<float4*>(hf + lane * CS + 4 * ci) =
                 make_float4(planes_value(h[0], nt), planes_value(h[1], nt), planes_value(h[2], nt), planes_value(h[3], nt));
           // planes of h: 4 units = 8 bytes per plane
           unsigned short q0[4], q1[4], q2[4];
@@ -460,9 +485,9 @@ struct TcEpiLstm {
               q2[u] = __bfloat16_as_ushort(__float2bfloat16_rn(r1 - __bfloat162float(b1)));
             }
           }
-          *reinterpret_cast<uint2*>(hs + (0 * 32 + lane) * 24 + 4 * ci) = make_uint2(q0[0] | ((uint32_t)q0[1] << 16), q0[2] | ((uint32_t)q0[3] << 16));
-          if (nt > 1) *reinterpret_cast<uint2*>(hs + (1 * 32 + lane) * 24 + 4 * ci) = make_uint2(q1[0] | ((uint32_t)q1[1] << 16), q1[2] | ((uint32_t)q1[3] << 16));
-          if (nt > 2) *reinterpret_cast<uint2*>(hs + (2 * 32 + lane) * 24 + 4 * ci) = make_uint2(q2[0] | ((uint32_t)q2[1] << 16), q2[2] | ((uint32_t)q2[3] << 16));
+          *reinterpret_cast<uint2*>(hs + (0 * 32 + lane) * HS + 4 * ci) = make_uint2(q0[0] | ((uint32_t)q0[1] << 16), q0[2] | ((uint32_t)q0[3] << 16));
+          if (nt > 1) *reinterpret_cast<uint2*>(hs + (1 * 32 + lane) * HS + 4 * ci) = make_uint2(q1[0] | ((uint32_t)q1[1] << 16), q1[2] | ((uint32_t)q1[3] << 16));
+          if (nt > 2) *reinterpret_cast<uint2*>(hs + (2 * 32 + lane) * HS + 4 * ci) = make_uint2(q2[0] | ((uint32_t)q2[1] << 16), q2[2] | ((uint32_t)q2[3] << 16));
         }
       }
     } else if (valid) {
@@ -470,7 +495,7 @@ struct TcEpiLstm {
       const size_t ip = (size_t)row * h_prev.ld + hp_col0 + j_first;
       for (int t = 0; t < nt; ++t)
         for (int g = 0; g < nch; ++g)
-          *reinterpret_cast<uint2*>(hs + (t * 32 + lane) * 24 + 4 * g) = *reinterpret_cast<const uint2*>(h_prev.p[t] + ip + 4 * g);
+          *reinterpret_cast<uint2*>(hs + (t * 32 + lane) * HS + 4 * g) = *reinterpret_cast<const uint2*>(h_prev.p[t] + ip + 4 * g);
     }
     const unsigned active_mask = __ballot_sync(0xffffffffu, active);
     __syncwarp();
@@ -478,16 +503,16 @@ struct TcEpiLstm {
     for (int s = lane; s < 32 * nq; s += 32) {
       const int r = s / nq, g = s - r * nq;
       if (row0 + r < M) {
-        *reinterpret_cast<float4*>(c_out + (size_t)(row0 + r) * ldc + j_first + 4 * g) = *reinterpret_cast<const float4*>(cs + r * 20 + 4 * g);
+        *reinterpret_cast<float4*>(c_out + (size_t)(row0 + r) * ldc + j_first + 4 * g) = *reinterpret_cast<const float4*>(cs + r * CS + 4 * g);
         if (h_f32 && ((active_mask >> r) & 1u))
-          *reinterpret_cast<float4*>(h_f32 + (size_t)(row0 + r) * hf_row_stride + j_first + 4 * g) = *reinterpret_cast<const float4*>(hf + r * 20 + 4 * g);
+          *reinterpret_cast<float4*>(h_f32 + (size_t)(row0 + r) * hf_row_stride + j_first + 4 * g) = *reinterpret_cast<const float4*>(hf + r * CS + 4 * g);
       }
     }
     for (int t = 0; t < nt; ++t)
       for (int s = lane; s < 32 * nq; s += 32) {
         const int r = s / nq, g = s - r * nq;
         if (row0 + r < M) {
-          const uint2 hv = *reinterpret_cast<const uint2*>(hs + (t * 32 + r) * 24 + 4 * g);
+          const uint2 hv = *reinterpret_cast<const uint2*>(hs + (t * 32 + r) * HS + 4 * g);
           *reinterpret_cast<uint2*>(h_out1.p[t] + (size_t)(row0 + r) * h_out1.ld + h1_col0 + j_first + 4 * g) = hv;
           if (h_out2.p[0]) *reinterpret_cast<uint2*>(h_out2.p[t] + (size_t)(row0 + r) * h_out2.ld + h2_col0 + j_first + 4 * g) = hv;
         }
@@ -669,6 +694,10 @@ struct TcEpiF32 {
     __syncwarp();
     return m;
   }
+  // up to two chunks at a time, see TcEpiLstm; returns the row's maximum over them
+  __device__ __forceinline__ float staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf) const {
+    return stage_store(row0, lane, M, col_first, nch, v, sbuf, kStagedStride);
+  }
   __device__ __forceinline__ void block(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, int slot) const {
     const float m = stage_store(row0, lane, M, col_first, nch, v, sbuf, kEpiScratchStride);
     pmax_store(row0 + lane, M, slot, m);
@@ -770,7 +799,7 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
   __shared__ int s_abort;
 
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;  // M fastest: the CTAs sharing a weight tile run together
   // split-K: this CTA covers k-blocks [kb0, kb0 + nkb) of the K / BK blocks
   const int nkb_total = K / BK;
@@ -797,41 +826,42 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
   const uint32_t tmem_acc = *tmem_slot;
 
   if (warp == 0) {
-    // Producer.  A TMA instruction costs its issuing thread ~150 ns whatever the box size
-    // (measured), so the 2*NT boxes of a stage are issued by 2*NT lanes in one warp instruction:
-    // lane t < NT loads plane t of A, lane NT + t plane t of B.
-    const bool is_a = lane < NT;
-    const int t = is_a ? lane : lane - NT;
-    const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(&tm) + (is_a ? t : 3 + t);  // a[3] then b[3]
-    const uint32_t dst_off = is_a ? (uint32_t)(t * A_BYTES) : (uint32_t)(NT * A_BYTES + t * B_BYTES);
-    const int ycoord = is_a ? m0 : n0;
+    // Producer.
+    const bool one = elect_one();
+    auto load_a = [&](int kb, uint32_t st, uint32_t fb) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) tma_load_2d(st + t * A_BYTES, &tm.a[t], (kb0 + kb) * BK, m0, fb);
+    };
+    auto load_b = [&](int kb, uint32_t st, uint32_t fb) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) tma_load_2d(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], (kb0 + kb) * BK, n0, fb);
+    };
     // First trip round the ring: the weight tiles do not depend on the previous kernel, so they
     // are requested before pdl_wait() and only the activation tiles after it.
     const int npre = nkb < STAGES ? nkb : STAGES;
-    for (int kb = 0; kb < npre; ++kb) {
-      if (lane == 0) mbar_expect_tx(bars + 8u * kb, (uint32_t)STAGE_BYTES);
-      __syncwarp();
-      if (!is_a && lane < 2 * NT) tma_load_2d(base + kb * STAGE_BYTES + dst_off, map, (kb0 + kb) * BK, ycoord, bars + 8u * kb);
-    }
+    if (one)
+      for (int kb = 0; kb < npre; ++kb) {
+        mbar_expect_tx(bars + 8u * kb, (uint32_t)STAGE_BYTES);
+        load_b(kb, base + kb * STAGE_BYTES, bars + 8u * kb);
+      }
     pdl_wait();   // the activations are the previous kernel's output
-    if (is_a)
-      for (int kb = 0; kb < npre; ++kb) tma_load_2d(base + kb * STAGE_BYTES + dst_off, map, (kb0 + kb) * BK, ycoord, bars + 8u * kb);
+    if (one)
+      for (int kb = 0; kb < npre; ++kb) load_a(kb, base + kb * STAGE_BYTES, bars + 8u * kb);
     int s = npre == STAGES ? 0 : npre; uint32_t ph = npre == STAGES ? 1u : 0u;
     uint32_t st = base + s * STAGE_BYTES, fb = bars + 8u * s, eb = bars + 8u * (STAGES + s);
     for (int kb = npre; kb < nkb; ++kb) {
-      int ok = 1;
-      if (lane == 0) {
-        ok = mbar_wait(eb, ph ^ 1u, &s_abort) ? 1 : 0;
-        if (ok) mbar_expect_tx(fb, (uint32_t)STAGE_BYTES);
+      if (!mbar_wait(eb, ph ^ 1u, &s_abort)) break;
+      if (one) {
+        mbar_expect_tx(fb, (uint32_t)STAGE_BYTES);
+        load_a(kb, st, fb);
+        load_b(kb, st, fb);
       }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      if (lane < 2 * NT) tma_load_2d(st + dst_off, map, (kb0 + kb) * BK, ycoord, fb);
       st += STAGE_BYTES; fb += 8u; eb += 8u;
       if (++s == STAGES) { s = 0; ph ^= 1u; st = base; fb = bars; eb = bars + 8u * STAGES; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       const uint32_t idesc = make_idesc(BM, BN, FMT);
       int s = 0; uint32_t ph = 0;
       uint32_t st = base, fb = bars, eb = bars + 8u * STAGES;
@@ -842,9 +872,11 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
         const uint64_t b0 = make_desc<BKT>(st + NT * A_BYTES);         // plane 0 of B, k-step 0
         if (NP == 1) {
           // plain bf16: one accumulation chain
+          if (one) {
 #pragma unroll
-          for (int ks = 0; ks < BK / UMMA_K; ++ks)
-            umma_bf16(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (kb | ks) ? 1u : 0u);
+            for (int ks = 0; ks < BK / UMMA_K; ++ks)
+              umma_bf16(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (kb | ks) ? 1u : 0u);
+          }
         } else {
           // (the small cross terms are the other issuing warp's)
           // leading product: accumulator 0 holds only kDrainEvery k-blocks at a time; the epilogue
@@ -855,19 +887,22 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
             if (!mbar_wait(main_free, (uint32_t)((d - 1) & 1), &s_abort)) break;
             tc_fence_after();
           }
+          if (one) {
 #pragma unroll
-          for (int ks = 0; ks < BK / UMMA_K; ++ks)
-            umma_bf16(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (in_chunk | ks) ? 1u : 0u);
-          if (in_chunk == kDrainEvery - 1 || kb == nkb - 1) umma_commit(main_full);
+            for (int ks = 0; ks < BK / UMMA_K; ++ks)
+              umma_bf16(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (in_chunk | ks) ? 1u : 0u);
+            if (in_chunk == kDrainEvery - 1 || kb == nkb - 1) umma_commit(main_full);
+          }
         }
-        umma_commit(eb);
+        if (one) umma_commit(eb);
         st += STAGE_BYTES; fb += 8u; eb += 8u;
         if (++s == STAGES) { s = 0; ph ^= 1u; st = base; fb = bars; eb = bars + 8u * STAGES; }
       }
-      umma_commit(accum_bar);
+      if (one) umma_commit(accum_bar);
     }
   } else if (warp == kIssue2Warp) {
-    if (NP > 1 && lane == 0) {
+    if (NP > 1) {
+      const bool one = elect_one();
       // second issuer: the small cross terms, one long chain in accumulator 1
       const uint32_t idesc = make_idesc(BM, BN, FMT);
       const uint32_t acc1 = tmem_acc + (uint32_t)acc_stride(BN);
@@ -879,20 +914,22 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
         tc_fence_after();
         const uint64_t a0 = make_desc<BKT>(st);
         const uint64_t b0 = make_desc<BKT>(st + NT * A_BYTES);
+        if (one) {
 #pragma unroll
-        for (int ks = 0; ks < BK / UMMA_K; ++ks) {
+          for (int ks = 0; ks < BK / UMMA_K; ++ks) {
 #pragma unroll
-          for (int p = 0; p < NP - 1; ++p) {
-            const uint64_t ad = a0 + (uint64_t)(((prod_a(PC, p) * A_BYTES) >> 4) + ks * 2);
-            const uint64_t bd = b0 + (uint64_t)prod_b(PC, p) * bstep + (uint64_t)(ks * 2);
-            umma_bf16(acc1, ad, bd, idesc, (kb | ks | p) ? 1u : 0u);
+            for (int p = 0; p < NP - 1; ++p) {
+              const uint64_t ad = a0 + (uint64_t)(((prod_a(PC, p) * A_BYTES) >> 4) + ks * 2);
+              const uint64_t bd = b0 + (uint64_t)prod_b(PC, p) * bstep + (uint64_t)(ks * 2);
+              umma_bf16(acc1, ad, bd, idesc, (kb | ks | p) ? 1u : 0u);
+            }
           }
+          umma_commit(eb);
         }
-        umma_commit(eb);
         st += STAGE_BYTES; fb += 8u; eb += 8u;
         if (++s == STAGES) { s = 0; ph ^= 1u; st = base; fb = bars; eb = bars + 8u * STAGES; }
       }
-      umma_commit(accum_bar);
+      if (one) umma_commit(accum_bar);
     }
   } else {
     // epilogue: warp w may touch TMEM lanes 32*(w%4) .. +31; the four warps of a lane quadrant
@@ -1068,7 +1105,7 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
   __shared__ int s_abort;
 
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int mt = (M + BM - 1) / BM;
   const int ntile = mt * ((N + BN - 1) / BN);
   const int nkb = K / BK;
@@ -1090,31 +1127,30 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
   const uint32_t tmem_acc = *tmem_slot;
 
   if (warp == 0) {
-    const bool is_a = lane < NT;
-    const int t = is_a ? lane : lane - NT;
-    const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(&tm) + (is_a ? t : 3 + t);
-    const uint32_t dst_off = is_a ? (uint32_t)(t * A_BYTES) : (uint32_t)(NT * A_BYTES + t * B_BYTES);
+    const bool one = elect_one();
     int s = 0; uint32_t ph = 0;
     uint32_t st = base, fb = bars, eb = bars + 8u * STAGES;
     pdl_wait();
     bool live = true;
     for (int tile = blockIdx.x; tile < ntile && live; tile += gridDim.x) {
-      const int ycoord = is_a ? (tile % mt) * BM : (tile / mt) * BN;
+      const int ya = (tile % mt) * BM, yb = (tile / mt) * BN;
       for (int kb = 0; kb < nkb; ++kb) {
-        int ok = 1;
-        if (lane == 0) {
-          ok = mbar_wait(eb, ph ^ 1u, &s_abort) ? 1 : 0;
-          if (ok) mbar_expect_tx(fb, (uint32_t)STAGE_BYTES);
+        if (!mbar_wait(eb, ph ^ 1u, &s_abort)) { live = false; break; }
+        if (one) {
+          mbar_expect_tx(fb, (uint32_t)STAGE_BYTES);
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            tma_load_2d(st + t * A_BYTES, &tm.a[t], kb * BK, ya, fb);
+            tma_load_2d(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], kb * BK, yb, fb);
+          }
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) { live = false; break; }
-        if (lane < 2 * NT) tma_load_2d(st + dst_off, map, kb * BK, ycoord, fb);
         st += STAGE_BYTES; fb += 8u; eb += 8u;
         if (++s == STAGES) { s = 0; ph ^= 1u; st = base; fb = bars; eb = bars + 8u * STAGES; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const bool one = elect_one();
       const uint32_t idesc = make_idesc(BM, BN, FMT);
       const uint32_t acc1 = tmem_acc + (uint32_t)acc_stride(BN);
       const uint64_t bstep = (uint64_t)(B_BYTES >> 4);
@@ -1133,7 +1169,7 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
           tc_fence_after();
           const uint64_t a0 = make_desc<BKT>(st);
           const uint64_t b0 = make_desc<BKT>(st + NT * A_BYTES);
-          if (NP > 1) {
+          if (NP > 1 && one) {
 #pragma unroll
             for (int ks = 0; ks < BK / UMMA_K; ++ks) {
 #pragma unroll
@@ -1144,14 +1180,16 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
               }
             }
           }
+          if (one) {
 #pragma unroll
-          for (int ks = 0; ks < BK / UMMA_K; ++ks)
-            umma_bf16(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (kb | ks) ? 1u : 0u);
-          umma_commit(eb);
+            for (int ks = 0; ks < BK / UMMA_K; ++ks)
+              umma_bf16(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (kb | ks) ? 1u : 0u);
+            umma_commit(eb);
+          }
           st += STAGE_BYTES; fb += 8u; eb += 8u;
           if (++s == STAGES) { s = 0; ph ^= 1u; st = base; fb = bars; eb = bars + 8u * STAGES; }
         }
-        umma_commit(accum_full);
+        if (one) umma_commit(accum_full);
       }
     }
   } else {
@@ -1321,11 +1359,10 @@ inline cudaError_t launch_gemm_tc(const TmapSet& tm, int M, int N, int K, const 
 
 // Persistent launch (see gemm_tc_persist_kernel): one or two planes per operand, no split-K.  One-plane
 // launches get a staging area of their own beside a ring of one stage less.
-constexpr int kPersistStageStride = 36;   // floats per staged row: two 16-column chunks + 4
 inline Shape make_shape_persist(int bn, int nt, int bk, int fmt) {
   Shape s = make_shape(bn, nt, bk, fmt);
   if (nt == 1) {
-    const int stg = kEpiWarps * 32 * kPersistStageStride * 4;
+    const int stg = kEpiWarps * 32 * kStagedStride * 4;
     s.stages = (SMEM_BUDGET - stg) / s.stage_bytes;
     if (s.stages > kMaxStages) s.stages = kMaxStages;
     s.smem_bytes = s.stages * s.stage_bytes + stg + 1024 + 256;
@@ -1338,7 +1375,7 @@ inline cudaError_t launch_gemm_tc_persist(const TmapSet& tm, int M, int N, int K
   if ((sh.nt != 2 && sh.nt != 1) || K % sh.bk || sh.stages < 2) return cudaErrorInvalidValue;
   const int tiles = ((M + BM - 1) / BM) * ((N + sh.bn - 1) / sh.bn);
   const dim3 grid(tiles < n_sm ? tiles : n_sm);
-  const int stride = sh.nt == 1 ? kPersistStageStride : 0;
+  const int stride = sh.nt == 1 ? kStagedStride : 0;
 #define LINMT_PERSIST_CASE(NTV, BKV, FMTV)                                                                                   \
   {                                                                                                                          \
     static bool optin_done[kMaxDevices] = {};                                                                                \

@@ -98,7 +98,7 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   __shared__ int s_abort;
 
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();     // 0 = leader (even blockIdx.x), 1 = peer
   const bool leader = rank == 0;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
@@ -125,38 +125,42 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   const uint32_t tmem_acc = *tmem_slot;
 
   if (warp == 0) {
-    // Producer (both CTAs): lanes 0..NT-1 the planes of this CTA's A rows, lanes NT..2NT-1 the planes of its half of B.
-    const bool is_a = lane < NT;
-    const int t = is_a ? lane : lane - NT;
-    const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(&tm) + (is_a ? (t < 3 ? t : 0) : 3 + (t < 3 ? t : 0));
-    const uint32_t dst_off = is_a ? (uint32_t)(t * A_BYTES) : (uint32_t)(NT * A_BYTES + t * B_BYTES);
-    const int ycoord = is_a ? m0 : n0 + (int)rank * BH;
+    // Producer (both CTAs): the planes of this CTA's A rows and of its half of B, issued by the elected lane.
+    const bool one = elect_one();
     const uint32_t full0 = cluster_map(bars, 0u);           // the leader's full barriers, as cluster addresses
     const uint32_t tx_bytes = 2u * (uint32_t)STAGE_BYTES;   // both CTAs' boxes
+    const int yb = n0 + (int)rank * BH;
+    auto load_a = [&](int kb, uint32_t st, uint32_t fb) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) tma_load_2d_pair(st + t * A_BYTES, &tm.a[t], (kb0 + kb) * BK, m0, fb);
+    };
+    auto load_b = [&](int kb, uint32_t st, uint32_t fb) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) tma_load_2d_pair(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], (kb0 + kb) * BK, yb, fb);
+    };
     const int npre = nkb < STAGES ? nkb : STAGES;
-    for (int kb = 0; kb < npre; ++kb) {
-      if (lane == 0 && leader) mbar_expect_tx(bars + 8u * kb, tx_bytes);
-      __syncwarp();
-      if (!is_a && lane < 2 * NT) tma_load_2d_pair(base + kb * STAGE_BYTES + dst_off, map, (kb0 + kb) * BK, ycoord, full0 + 8u * kb);
-    }
+    if (one)
+      for (int kb = 0; kb < npre; ++kb) {
+        if (leader) mbar_expect_tx(bars + 8u * kb, tx_bytes);
+        load_b(kb, base + kb * STAGE_BYTES, full0 + 8u * kb);
+      }
     pdl_wait();
-    if (is_a)
-      for (int kb = 0; kb < npre; ++kb) tma_load_2d_pair(base + kb * STAGE_BYTES + dst_off, map, (kb0 + kb) * BK, ycoord, full0 + 8u * kb);
+    if (one)
+      for (int kb = 0; kb < npre; ++kb) load_a(kb, base + kb * STAGE_BYTES, full0 + 8u * kb);
     int s = npre == STAGES ? 0 : npre; uint32_t ph = npre == STAGES ? 1u : 0u;
     for (int kb = npre; kb < nkb; ++kb) {
-      const uint32_t st = base + s * STAGE_BYTES, eb = bars + 8u * (STAGES + s);
-      int ok = 1;
-      if (lane == 0) {
-        ok = mbar_wait(eb, ph ^ 1u, &s_abort) ? 1 : 0;       // this CTA's copy of the stage-free barrier
-        if (ok && leader) mbar_expect_tx(bars + 8u * s, tx_bytes);
+      const uint32_t st = base + s * STAGE_BYTES;
+      if (!mbar_wait(bars + 8u * (STAGES + s), ph ^ 1u, &s_abort)) break;       // this CTA's copy of the stage-free barrier
+      if (one) {
+        if (leader) mbar_expect_tx(bars + 8u * s, tx_bytes);
+        load_a(kb, st, full0 + 8u * s);
+        load_b(kb, st, full0 + 8u * s);
       }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
-      if (lane < 2 * NT) tma_load_2d_pair(st + dst_off, map, (kb0 + kb) * BK, ycoord, full0 + 8u * s);
       if (++s == STAGES) { s = 0; ph ^= 1u; }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool one = elect_one();
       // leading product of the pair's 256 x BN tile into accumulator 0 (of both CTAs)
       const uint32_t idesc = make_idesc(2 * BM, BN, FMT);
       int s = 0; uint32_t ph = 0;
@@ -172,17 +176,20 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
           if (!mbar_wait(main_free, (uint32_t)((d - 1) & 1), &s_abort)) break;
           tc_fence_after();
         }
+        if (one) {
 #pragma unroll
-        for (int ks = 0; ks < BK / UMMA_K; ++ks)
-          umma_f16_pair(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (in_chunk | ks) ? 1u : 0u);
-        if (in_chunk == kDrainEvery - 1 || kb == nkb - 1) umma_commit_pair(main_full);
-        umma_commit_pair(eb);
+          for (int ks = 0; ks < BK / UMMA_K; ++ks)
+            umma_f16_pair(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (in_chunk | ks) ? 1u : 0u);
+          if (in_chunk == kDrainEvery - 1 || kb == nkb - 1) umma_commit_pair(main_full);
+          umma_commit_pair(eb);
+        }
         if (++s == STAGES) { s = 0; ph ^= 1u; }
       }
-      umma_commit_pair(accum_bar);
+      if (one) umma_commit_pair(accum_bar);
     }
   } else if (warp == kIssue2Warp) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool one = elect_one();
       const uint32_t idesc = make_idesc(2 * BM, BN, FMT);
       const uint32_t acc1 = tmem_acc + (uint32_t)acc_stride(BN);
       const uint64_t bstep = (uint64_t)(B_BYTES >> 4);
@@ -193,19 +200,21 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
         tc_fence_after();
         const uint64_t a0 = make_desc<BKT>(st);
         const uint64_t b0 = make_desc<BKT>(st + NT * A_BYTES);
+        if (one) {
 #pragma unroll
-        for (int ks = 0; ks < BK / UMMA_K; ++ks) {
+          for (int ks = 0; ks < BK / UMMA_K; ++ks) {
 #pragma unroll
-          for (int p = 0; p < NP - 1; ++p) {
-            const uint64_t ad = a0 + (uint64_t)(((prod_a(PC, p) * A_BYTES) >> 4) + ks * 2);
-            const uint64_t bd = b0 + (uint64_t)prod_b(PC, p) * bstep + (uint64_t)(ks * 2);
-            umma_f16_pair(acc1, ad, bd, idesc, (kb | ks | p) ? 1u : 0u);
+            for (int p = 0; p < NP - 1; ++p) {
+              const uint64_t ad = a0 + (uint64_t)(((prod_a(PC, p) * A_BYTES) >> 4) + ks * 2);
+              const uint64_t bd = b0 + (uint64_t)prod_b(PC, p) * bstep + (uint64_t)(ks * 2);
+              umma_f16_pair(acc1, ad, bd, idesc, (kb | ks | p) ? 1u : 0u);
+            }
           }
+          umma_commit_pair(eb);
         }
-        umma_commit_pair(eb);
         if (++s == STAGES) { s = 0; ph ^= 1u; }
       }
-      umma_commit_pair(accum_bar);
+      if (one) umma_commit_pair(accum_bar);
     }
   } else {
     // epilogue (both CTAs, each on the rows of its own TMEM): the one-tile kernel's
@@ -356,61 +365,59 @@ inline cudaError_t launch_gemm_tc_pair(const TmapSet& tm, int M, int N, int K, c
                             splits > 1 ? ws : (float*)nullptr, counters);
 }
 
-// ---- persistent form on CTA pairs (many-wave GEMMs: the vocabulary projection) ---------------------------
-// gemm_tc_persist_kernel with every SM pair walking over 256 x BN tiles: pair p takes pair tiles p, p + pairs, ...
-// (row pair fastest); CTA `rank` of the pair owns row tile 2 * (row pair) + rank of each.  Loads, barriers and
-// TMEM hand-over as in gemm_tc_pair_kernel; the tensor core may start the next tile once the epilogue warps of
-// BOTH CTAs have copied their accumulator rows out (they arrive on the leader's barrier).
-inline Shape make_shape_persist_pair(int bn, int nt, int bk, int fmt) {
-  Shape s = make_shape_pair(bn, nt, bk, fmt);
-  if (nt == 1) {
-    const int stg = kEpiWarps * 32 * kPersistStageStride * 4;
-    s.stages = (SMEM_BUDGET - stg) / s.stage_bytes;
-    if (s.stages > kMaxStages) s.stages = kMaxStages;
-    s.smem_bytes = s.stages * s.stage_bytes + stg + 1024 + 256;
-  }
+// ---- persistent form on CTA pairs (one-plane GEMMs of many tiles) ------------------------------------------
+// Every SM pair walks over 256 x BN tiles: pair p takes pair tiles p, p + pairs, ... (row pair fastest); CTA `rank` of the
+// pair owns row tile 2 * (row pair) + rank of each.  Loads and barriers as in gemm_tc_pair_kernel, one plane per operand.
+// Two accumulators of up to 256 columns each: while the tensor cores are on one tile, the epilogue warps take the other
+// out of TMEM, two 16-column chunks at a time through a staging area of their own, so that neither waits for the other.
+// What bounds it is what an SM takes in (128 + BN / 2 operand rows per k-block and CTA), hence tiles as wide as the
+// columns allow.  Measured against one accumulator: see persist_pair_bn.
+inline Shape make_shape_persist_pair(int bn, int fmt) {
+  Shape s = make_shape_pair(bn, 1, 64, fmt);
+  const int stg = kEpiWarps * 32 * kStagedStride * 4;
+  s.stages = (SMEM_BUDGET - stg) / s.stage_bytes;
+  if (s.stages > kMaxStages) s.stages = kMaxStages;
+  s.smem_bytes = s.stages * s.stage_bytes + stg + 1024 + 256;
   return s;
 }
 
-template <int NT, int BKT, int FMT, class Epi>
+template <int FMT, class Epi>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, int STAGES, Epi epi,
-                            int* __restrict__ err_flag, int stage_stride) {
-  constexpr int PC = product_code(NT, FMT);
-  constexpr int NP = num_products(PC);
-  constexpr int A_BYTES = BM * BKT * 2;
-  constexpr int BK = BKT;
+gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, int STAGES, Epi epi, int* __restrict__ err_flag) {
+  constexpr int BK = 64;
+  constexpr int A_BYTES = BM * BK * 2;
+  constexpr int STG_WARP = 32 * kStagedStride * 4;
+  constexpr uint32_t kAccCols = TMEM_COLS / 2;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - raw);
   const int BH = BN >> 1;
-  const int B_BYTES = BH * BK * 2;
-  const int STAGE_BYTES = NT * (A_BYTES + B_BYTES);
-  const int STG_WARP = 32 * stage_stride * 4;
-  const int RING = (stage_stride > 0 ? STAGES * STAGE_BYTES : ring_bytes(STAGES, STAGE_BYTES));
+  const int STAGE_BYTES = A_BYTES + BH * BK * 2;
+  const int RING = STAGES * STAGE_BYTES;
   const int PRE = RING + kEpiWarps * STG_WARP;
-  const uint32_t bars = base + PRE;   // full[STAGES], empty[STAGES], accum_full, tmem_free
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + PRE + 8 * (2 * STAGES + 3));
+  const uint32_t bars = base + PRE;   // full[STAGES], empty[STAGES], accum_full[2], tmem_free[2]
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + PRE + 8 * (2 * STAGES + 4));
   __shared__ int s_abort;
 
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
-  const int mt = (M + BM - 1) / BM;
-  const int mt2 = (mt + 1) >> 1;                       // row pairs
+  const int mt2 = ((M + BM - 1) / BM + 1) >> 1;        // row pairs
   const int ntile = mt2 * ((N + BN - 1) / BN);        // pair tiles
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int nkb = K / BK;
   const uint32_t accum_full = bars + 8u * (2 * STAGES);
-  const uint32_t tmem_free = accum_full + 8u;
+  const uint32_t tmem_free = accum_full + 16u;
 
   if (threadIdx.x == 0) {
     s_abort = 0;
     for (int s = 0; s < STAGES; ++s) { mbar_init(bars + 8u * s, 1); mbar_init(bars + 8u * (STAGES + s), 1); }
-    mbar_init(accum_full, 1);
-    mbar_init(tmem_free, 2 * kEpiWarps);   // both CTAs' epilogue warps (the leader's copy is the one waited on)
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(accum_full + 8u * b, 1);
+      mbar_init(tmem_free + 8u * b, 2 * kEpiWarps);   // both CTAs' epilogue warps (the leader's copy is the one waited on)
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -421,136 +428,102 @@ gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, in
   const uint32_t tmem_acc = *tmem_slot;
 
   if (warp == 0) {
-    const bool is_a = lane < NT;
-    const int t = is_a ? lane : lane - NT;
-    const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(&tm) + (is_a ? (t < 3 ? t : 0) : 3 + (t < 3 ? t : 0));
-    const uint32_t dst_off = is_a ? (uint32_t)(t * A_BYTES) : (uint32_t)(NT * A_BYTES + t * B_BYTES);
+    const bool one = elect_one();
     const uint32_t full0 = cluster_map(bars, 0u);
     const uint32_t tx_bytes = 2u * (uint32_t)STAGE_BYTES;
-    int s = 0; uint32_t ph = 0;
+    auto y_a = [&](int tile) { return ((tile % mt2) * 2 + (int)rank) * BM; };
+    auto y_b = [&](int tile) { return (tile / mt2) * BN + (int)rank * BH; };
+    // first trip round the ring: the weights do not depend on the previous kernel
+    const int npre = nkb < STAGES ? nkb : STAGES;
+    if (one)
+      for (int kb = 0; kb < npre; ++kb) {
+        if (leader) mbar_expect_tx(bars + 8u * kb, tx_bytes);
+        tma_load_2d_pair(base + kb * STAGE_BYTES + A_BYTES, &tm.b[0], kb * BK, y_b(pair), full0 + 8u * kb);
+      }
     pdl_wait();
+    if (one)
+      for (int kb = 0; kb < npre; ++kb) tma_load_2d_pair(base + kb * STAGE_BYTES, &tm.a[0], kb * BK, y_a(pair), full0 + 8u * kb);
+    int s = npre == STAGES ? 0 : npre; uint32_t ph = npre == STAGES ? 1u : 0u;
     bool live = true;
     for (int tile = pair; tile < ntile && live; tile += npairs) {
-      const int ycoord = is_a ? ((tile % mt2) * 2 + (int)rank) * BM : (tile / mt2) * BN + (int)rank * BH;
-      for (int kb = 0; kb < nkb; ++kb) {
-        int ok = 1;
-        if (lane == 0) {
-          ok = mbar_wait(bars + 8u * (STAGES + s), ph ^ 1u, &s_abort) ? 1 : 0;
-          if (ok && leader) mbar_expect_tx(bars + 8u * s, tx_bytes);
+      const int ya = y_a(tile), yb = y_b(tile);
+      for (int kb = tile == pair ? npre : 0; kb < nkb; ++kb) {
+        const uint32_t st = base + s * STAGE_BYTES;
+        if (!mbar_wait(bars + 8u * (STAGES + s), ph ^ 1u, &s_abort)) { live = false; break; }
+        if (one) {
+          if (leader) mbar_expect_tx(bars + 8u * s, tx_bytes);
+          tma_load_2d_pair(st, &tm.a[0], kb * BK, ya, full0 + 8u * s);
+          tma_load_2d_pair(st + A_BYTES, &tm.b[0], kb * BK, yb, full0 + 8u * s);
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) { live = false; break; }
-        if (lane < 2 * NT) tma_load_2d_pair(base + s * STAGE_BYTES + dst_off, map, kb * BK, ycoord, full0 + 8u * s);
         if (++s == STAGES) { s = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
+      const bool one = elect_one();
       const uint32_t idesc = make_idesc(2 * BM, BN, FMT);
-      const uint32_t acc1 = tmem_acc + (uint32_t)acc_stride(BN);
-      const uint64_t bstep = (uint64_t)(B_BYTES >> 4);
       int s = 0; uint32_t ph = 0;
       bool live = true;
       int it = 0;
       for (int tile = pair; tile < ntile && live; tile += npairs, ++it) {
-        if (it > 0) {
-          if (!mbar_wait(tmem_free, (uint32_t)((it - 1) & 1), &s_abort)) break;
+        const int b = it & 1;
+        if (it >= 2) {      // the accumulator's previous tile has been taken out
+          if (!mbar_wait(tmem_free + 8u * b, (uint32_t)(((it >> 1) - 1) & 1), &s_abort)) break;
           tc_fence_after();
         }
         for (int kb = 0; kb < nkb; ++kb) {
           const uint32_t st = base + s * STAGE_BYTES;
           if (!mbar_wait(bars + 8u * s, ph, &s_abort)) { live = false; break; }
           tc_fence_after();
-          const uint64_t a0 = make_desc<BKT>(st);
-          const uint64_t b0 = make_desc<BKT>(st + NT * A_BYTES);
-          if (NP > 1) {
+          const uint64_t a0 = make_desc<BK>(st), b0 = make_desc<BK>(st + A_BYTES);
+          if (one) {
 #pragma unroll
-            for (int ks = 0; ks < BK / UMMA_K; ++ks) {
-#pragma unroll
-              for (int p = 0; p < NP - 1; ++p) {
-                const uint64_t ad = a0 + (uint64_t)(((prod_a(PC, p) * A_BYTES) >> 4) + ks * 2);
-                const uint64_t bd = b0 + (uint64_t)prod_b(PC, p) * bstep + (uint64_t)(ks * 2);
-                umma_f16_pair(acc1, ad, bd, idesc, (kb | ks | p) ? 1u : 0u);
-              }
-            }
+            for (int ks = 0; ks < BK / UMMA_K; ++ks)
+              umma_f16_pair(tmem_acc + kAccCols * b, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (kb | ks) ? 1u : 0u);
+            umma_commit_pair(bars + 8u * (STAGES + s));
           }
-#pragma unroll
-          for (int ks = 0; ks < BK / UMMA_K; ++ks)
-            umma_f16_pair(tmem_acc, a0 + (uint64_t)(ks * 2), b0 + (uint64_t)(ks * 2), idesc, (kb | ks) ? 1u : 0u);
-          umma_commit_pair(bars + 8u * (STAGES + s));
           if (++s == STAGES) { s = 0; ph ^= 1u; }
         }
-        if (live) umma_commit_pair(accum_full);
+        if (live && one) umma_commit_pair(accum_full + 8u * b);
       }
     }
   } else {
     const int q = warp & 3;
     constexpr int kParts = kEpiWarps / 4;
-    constexpr int kChunks = kEpiBlockChunks;
     const int part = (warp - 2) >> 2;
     const int nchunks = BN >> 4;
     const int cpw = (nchunks + kParts - 1) / kParts;
     const int ch0 = part * cpw;
-    const uint32_t astride = (uint32_t)acc_stride(BN);
     const uint32_t lane_base = tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(ch0 * 16);
-    float* sbuf = reinterpret_cast<float*>(base_ptr + (warp - 2) * kEpiScratchBytes);
+    float* own = reinterpret_cast<float*>(base_ptr + RING + (warp - 2) * STG_WARP);
     const uint32_t tmem_free_leader = cluster_map(tmem_free, 0u);
     pdl_wait();
     int it = 0;
     for (int tile = pair; tile < ntile; tile += npairs, ++it) {
-      const int m0 = ((tile % mt2) * 2 + (int)rank) * BM, n0 = (tile / mt2) * BN;
-      const int row0 = m0 + q * 32;
+      const int b = it & 1;
+      const int row0 = ((tile % mt2) * 2 + (int)rank) * BM + q * 32, n0 = (tile / mt2) * BN;
       int nmine = nchunks - ch0; nmine = nmine < 0 ? 0 : (nmine > cpw ? cpw : nmine);
       {
         const int left = (N - (n0 + ch0 * 16) + 15) >> 4;
         if (left < nmine) nmine = left < 0 ? 0 : left;
       }
-      if (!mbar_wait_sleepy(accum_full, (uint32_t)(it & 1), &s_abort)) break;
+      if (!mbar_wait_sleepy(accum_full + 8u * b, (uint32_t)((it >> 1) & 1), &s_abort)) break;
       tc_fence_after();
-      float macc[kChunks][16];
+      float m = -INFINITY;
 #pragma unroll
-      for (int ci = 0; ci < kChunks; ++ci) {
-        if (ci < nmine) {
-          tmem_ld16(lane_base + (uint32_t)(ci * 16), macc[ci]);
-          if (NP > 1) {
-            float sm[16];
-            tmem_ld16(lane_base + astride + (uint32_t)(ci * 16), sm);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) macc[ci][i] += FMT ? sm[i] * kF16PairInvScale : sm[i];
-          }
+      for (int c0 = 0; c0 < kEpiBlockChunks; c0 += 2) {
+        const int nc = nmine - c0 < 2 ? nmine - c0 : 2;
+        float v[2][16];
+        if (nc > 0) tmem_ld16(lane_base + kAccCols * b + (uint32_t)(c0 * 16), v[0]);
+        if (nc > 1) tmem_ld16(lane_base + kAccCols * b + (uint32_t)(c0 * 16 + 16), v[1]);
+        if (c0 + 2 >= kEpiBlockChunks) {     // everything is in registers: the tensor cores may have the accumulator
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(tmem_free_leader + 8u * b);
         }
+        if (nc > 0 && row0 < M) m = fmaxf(m, epi.staged(row0, lane, M, n0 + (ch0 + c0) * 16, nc, v, own));
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(tmem_free_leader);   // the pair's tensor cores may start the next tile
-      const bool last = tile + npairs >= ntile;
-      const int slot = (tile / mt2) * kParts + part;
-      if constexpr (Epi::kHasPmax) {
-        if (stage_stride > 0) {
-          float* own = reinterpret_cast<float*>(base_ptr + RING + (warp - 2) * STG_WARP);
-          float m = -INFINITY;
-#pragma unroll
-          for (int c0 = 0; c0 < kChunks; c0 += 2) {
-            if (c0 < nmine) {
-              const int nc = nmine - c0 < 2 ? nmine - c0 : 2;
-              m = fmaxf(m, epi.stage_store(row0, lane, M, n0 + (ch0 + c0) * 16, nc, macc + c0, own, stage_stride));
-            }
-          }
-          epi.pmax_store(row0 + lane, M, slot, m);
-          continue;
-        }
-      }
-      if (last && Epi::kHasBlock) {
-        // the last tile's accumulators are complete, so neither tensor core reads a ring any more
-        if (nmine > 0) epi.block(row0, lane, M, n0 + ch0 * 16, nmine, macc, sbuf, slot);
-        else if constexpr (Epi::kHasPmax) epi.pmax_store(row0 + lane, M, slot, -INFINITY);
-      } else if constexpr (Epi::kHasPmax) {
-        epi.direct_block(row0 + lane, M, n0 + ch0 * 16, nmine, macc, slot);
-      } else if (row0 + lane < M) {
-#pragma unroll
-        for (int ci = 0; ci < kChunks; ++ci)
-          if (ci < nmine) epi(row0 + lane, n0 + (ch0 + ci) * 16, macc[ci]);
-      }
+      if constexpr (Epi::kHasPmax) epi.pmax_store(row0 + lane, M, (tile / mt2) * kParts + part, m);
     }
   }
   tc_fence_before();
@@ -560,16 +533,15 @@ gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, in
 }
 
 // One cluster of two CTAs per SM pair (at most n_sm / 2 pairs); B tensor maps with a box of bn / 2 rows.
-template <int NT, int BKT, int FMT, class Epi>
+template <int FMT, class Epi>
 inline cudaError_t launch_gemm_tc_persist_pair(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
                                                cudaStream_t st, int n_sm) {
-  if (K % sh.bk || sh.stages < 2 || sh.bn % 16) return cudaErrorInvalidValue;
+  if (K % 64 || sh.stages < 2 || sh.bn % 16 || sh.bn > 256) return cudaErrorInvalidValue;
   static bool optin_done[kMaxDevices] = {};
-  if (cudaError_t e = ensure_smem_optin(gemm_tc_persist_pair_kernel<NT, BKT, FMT, Epi>, optin_done); e != cudaSuccess) return e;
+  if (cudaError_t e = ensure_smem_optin(gemm_tc_persist_pair_kernel<FMT, Epi>, optin_done); e != cudaSuccess) return e;
   const int mt2 = ((M + BM - 1) / BM + 1) / 2;
   const int tiles = mt2 * ((N + sh.bn - 1) / sh.bn);
   const int pairs = tiles < n_sm / 2 ? tiles : n_sm / 2;
-  const int stride = sh.nt == 1 ? kPersistStageStride : 0;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = (size_t)sh.smem_bytes; cfg.stream = st;
   cudaLaunchAttribute attr[2];
@@ -579,7 +551,7 @@ inline cudaError_t launch_gemm_tc_persist_pair(const TmapSet& tm, int M, int N, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = sh.pdl ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_tc_persist_pair_kernel<NT, BKT, FMT, Epi>, tm, M, N, K, sh.bn, sh.stages, epi, err_flag, stride);
+  return cudaLaunchKernelEx(&cfg, gemm_tc_persist_pair_kernel<FMT, Epi>, tm, M, N, K, sh.bn, sh.stages, epi, err_flag);
 }
 
 // How many CTA pairs of the one-tile pair kernel the current device holds at once (0: clusters of two such CTAs

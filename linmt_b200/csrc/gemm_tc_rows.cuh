@@ -134,7 +134,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   volatile int* abort_flag = reinterpret_cast<volatile int*>(rows_smem + (recv_bar + 12u - base));
 
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BM;
   const int splits = sh.splits, rank = blockIdx.z;
   const int nkb_total = K / 64;
@@ -155,21 +155,26 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect_tx(recv_bar, (uint32_t)(n_own * (splits - 1) * 512));   // the neighbours' share
   }
-  // the producer: lanes < NT the planes of the weights, lanes NT .. 2 NT - 1 those of the activations
-  const bool is_w = lane < NT;
-  const int pl = is_w ? lane : lane - NT;
-  const CUtensorMap* map = reinterpret_cast<const CUtensorMap*>(&tm) + (is_w ? 3 + (pl < 3 ? pl : 0) : (pl < 3 ? pl : 0));
+  const bool one = elect_one();
+  auto load_w = [&](int kb, int stage) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) tma_load_2d(base + (uint32_t)((stage * NT + t) * W_BYTES), &tm.b[t], (kb0 + kb) * 64, n0, bars + 8u * stage);
+  };
+  auto load_x = [&](int kb, int stage) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) tma_load_2d(xbase + (uint32_t)((stage * NT + t) * X_BYTES), &tm.a[t], (kb0 + kb) * 64, x_row0, xbars + 8u * stage);
+  };
   const int prew = nkb < WS ? nkb : WS, prex = nkb < XS ? nkb : XS;
   if (warp == 0) {
-    if (!is_w && lane < 2 * NT) asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");   // its descriptor is there when the wait ends
-    __syncwarp();
-    for (int kb = 0; kb < prew; ++kb) {
-      if (lane == 0) mbar_expect_tx(bars + 8u * kb, (uint32_t)(NT * W_BYTES));
-      __syncwarp();
-      if (is_w) tma_load_2d(base + (uint32_t)(kb * NT * W_BYTES + pl * W_BYTES), map, (kb0 + kb) * 64, n0, bars + 8u * kb);
-    }
-    if (lane == 0)
+    if (one) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) asm volatile("prefetch.tensormap [%0];" ::"l"(&tm.a[t]) : "memory");   // there when the wait ends
+      for (int kb = 0; kb < prew; ++kb) {
+        mbar_expect_tx(bars + 8u * kb, (uint32_t)(NT * W_BYTES));
+        load_w(kb, kb);
+      }
       for (int kb = 0; kb < prex; ++kb) mbar_expect_tx(xbars + 8u * kb, (uint32_t)(NT * X_BYTES));
+    }
     __syncwarp();
   } else if (warp == 1) {
     tmem_alloc(recv_bar + 8u, (uint32_t)sh.tmem_cols);
@@ -181,9 +186,8 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   const uint32_t tmem = *tmem_slot;
 
   pdl_wait();    // from here on the previous kernel's results are visible
-  if (warp == 0 && !is_w && lane < 2 * NT)
-    for (int kb = 0; kb < prex; ++kb)
-      tma_load_2d(xbase + (uint32_t)(kb * NT * X_BYTES + pl * X_BYTES), map, (kb0 + kb) * 64, x_row0, xbars + 8u * kb);
+  if (warp == 0 && one)
+    for (int kb = 0; kb < prex; ++kb) load_x(kb, kb);
   // what the epilogue of this warp's first unit reads is requested now and used after the accumulators are complete
   auto unit_row = [&](int i) { return ((rank + splits * i) >> 2) * 4 + (lane & 3); };
   auto unit_col = [&](int i) { return n0 + ((rank + splits * i) & 3) * 32 + (lane & ~3); };    // of the lane's four columns
@@ -197,25 +201,19 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     while (kw < nkb || kx < nkb) {
       // the ring that is behind goes first (with equal depths: alternately)
       const bool do_w = kx >= nkb || (kw < nkb && kw <= kx);
-      int ok = 1;
-      const uint32_t fb = do_w ? bars + 8u * ws : xbars + 8u * xs;
-      if (lane == 0) {
-        ok = (do_w ? mbar_wait(bars + 8u * (WS + ws), wph ^ 1u, abort_flag) : mbar_wait(xbars + 8u * (XS + xs), xph ^ 1u, abort_flag)) ? 1 : 0;
-        if (ok) mbar_expect_tx(fb, (uint32_t)(do_w ? NT * W_BYTES : NT * X_BYTES));
-      }
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) break;
       if (do_w) {
-        if (is_w) tma_load_2d(base + (uint32_t)(ws * NT * W_BYTES + pl * W_BYTES), map, (kb0 + kw) * 64, n0, fb);
+        if (!mbar_wait(bars + 8u * (WS + ws), wph ^ 1u, abort_flag)) break;
+        if (one) { mbar_expect_tx(bars + 8u * ws, (uint32_t)(NT * W_BYTES)); load_w(kw, ws); }
         ++kw;
         if (++ws == WS) { ws = 0; wph ^= 1u; }
       } else {
-        if (!is_w && lane < 2 * NT) tma_load_2d(xbase + (uint32_t)(xs * NT * X_BYTES + pl * X_BYTES), map, (kb0 + kx) * 64, x_row0, fb);
+        if (!mbar_wait(xbars + 8u * (XS + xs), xph ^ 1u, abort_flag)) break;
+        if (one) { mbar_expect_tx(xbars + 8u * xs, (uint32_t)(NT * X_BYTES)); load_x(kx, xs); }
         ++kx;
         if (++xs == XS) { xs = 0; xph ^= 1u; }
       }
     }
-  } else if (warp <= issuers && lane == 0) {
+  } else if (warp <= issuers) {
     // warp 1: w0 times the activations (both planes of the f16 pair), warp 2 (f16 pair): w1 x0
     const uint32_t idesc = make_idesc(BM, NT == 2 && warp == 1 ? 2 * sh.rp : sh.rp, FMT);
     const int chain = NT == 1 ? nkb : (nkb + sh.leads - 1) / sh.leads;   // k-blocks per leading accumulator
@@ -228,15 +226,17 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
       tc_fence_after();
       const uint64_t w0 = make_desc<64>(base + (uint32_t)(ws * NT * W_BYTES) + woff), x0 = make_desc<64>(xbase + (uint32_t)(xs * NT * X_BYTES));
       if (warp == 1 && in_chain == chain) { in_chain = 0; acc += (uint32_t)sh.acc_stride; }
+      if (one) {
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) umma_bf16(acc, w0 + (uint64_t)(ks * 2), x0 + (uint64_t)(ks * 2), idesc, (in_chain | ks) ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks) umma_bf16(acc, w0 + (uint64_t)(ks * 2), x0 + (uint64_t)(ks * 2), idesc, (in_chain | ks) ? 1u : 0u);
+        umma_commit(bars + 8u * (WS + ws));
+        umma_commit(xbars + 8u * (XS + xs));
+      }
       ++in_chain;
-      umma_commit(bars + 8u * (WS + ws));
-      umma_commit(xbars + 8u * (XS + xs));
       if (++ws == WS) { ws = 0; wph ^= 1u; }
       if (++xs == XS) { xs = 0; xph ^= 1u; }
     }
-    umma_commit(accum_bar);
+    if (one) umma_commit(accum_bar);
   }
   __syncwarp();
 
