@@ -266,7 +266,7 @@ int Engine::build_xw_tables() {
 // events for the cross-layer edges.  Besides the true dependencies, (l, p) waits for (l+1, p-2),
 // the last reader of the double-buffered input slot it overwrites.
 int Engine::run_encoder_tc(int n, int Smax) {
-  if (rows_ && n <= tc::kRowsMax && enc_rows_) return run_encoder_layers_tc(n, Smax);
+  if (rows_ && n <= 64 && enc_rows_) return run_encoder_layers_tc(n, Smax);
   constexpr int kRing = 4;
   hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;
   if (enc_streams_.empty()) {

@@ -1,6 +1,6 @@
 // gemm_tc_rows.cuh -- the tensor-core GEMM for FEW activation rows (a decoder step of a sentence or a small batch).
 //
-//   C[R][N] = A[R][K] . Wt[N][K]^T   with R <= 128, N and K in the thousands
+//   C[R][N] = A[R][K] . Wt[N][K]^T   with R <= 128 (one plane: 64), N and K in the thousands
 //
 // With few rows the product is a stream of weights: every weight byte comes in once and meets R rows.  The kernel of
 // gemm_tc.cuh puts the rows on the 128-wide M side of the MMA, holds a whole SM's shared memory and joins K slices
@@ -25,7 +25,8 @@ namespace linmt {
 namespace tc {
 
 constexpr int kRowsThreads = 256;       // warp 0 TMA, warps 1 and 2 issue MMAs, then all eight finish rows
-constexpr int kRowsMax = 64;
+constexpr int kRowsMax = 128;
+constexpr int rows_max(int nt) { return nt == 1 ? 64 : 128; }    // (one plane, 96 rows: 9.5 us in the one-tile kernel, 10.5 here)
 constexpr int kRowsMaxLeads = 4;
 // Shared memory of a CTA that shares its SM with one of the next kernel's (SM: 228 KB, 1 KB of it per CTA reserved), and
 // the least it asks for: with less, a third CTA would fit whose TMEM allocation waits for the other two, and CTAs of one
@@ -39,7 +40,7 @@ struct RowsShape {
   int rp, units;       // rows rounded up to 16 = N of the MMA; rows rounded up to 4 = units of 4 rows x 32 columns
   int wstages, xstages, recv_bytes, smem_bytes;   // rings of weight and activation k-blocks
   int splits;          // K slices = cluster size
-  int leads, acc_stride, tmem_cols;
+  int leads, acc_stride, stacked, tmem_cols;
   int alias;           // the partial sums' buffer lies in the rings (and waits until the whole cluster is done with them)
   int pdl;
 };
@@ -71,7 +72,7 @@ inline bool rows_set_splits(RowsShape* s, int K, int nt) {
 
 // one_chain: the leading product may be one long chain per accumulator (logits, see gemm_tc_persist_kernel)
 inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, bool one_chain, RowsShape* out) {
-  if (rows < 1 || rows > kRowsMax || K % 64 || K < 64 || N % 16) return false;
+  if (rows < 1 || rows > rows_max(nt) || K % 64 || K < 64 || N % 16) return false;
   if (!(nt == 1 || (nt == 2 && fmt == 1))) return false;
   RowsShape s{};
   s.rp = (rows + 15) & ~15; s.units = (rows + 3) & ~3;
@@ -88,8 +89,10 @@ inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, b
     if (s.splits > nkb) s.splits = nkb;
     s.tmem_cols = whole ? 512 : 256;
     // f16 pair: w0 meets both planes of the activations in ONE instruction (N = 2 rp, the planes lie one behind the
-    // other), so an accumulator holds w0 x0 | w0 x1
-    s.acc_stride = nt * s.rp;
+    // other), so an accumulator holds w0 x0 | w0 x1; beyond 64 rows an instruction per product takes as long, and the
+    // columns are better spent on short chains
+    s.stacked = nt == 2 && s.rp <= 64;
+    s.acc_stride = s.stacked ? 2 * s.rp : (s.rp + 31) & ~31;
     s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
     if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
     const bool chains = nt == 1 || one_chain || (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
@@ -214,8 +217,8 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
       }
     }
   } else if (warp <= issuers) {
-    // warp 1: w0 times the activations (both planes of the f16 pair), warp 2 (f16 pair): w1 x0
-    const uint32_t idesc = make_idesc(BM, NT == 2 && warp == 1 ? 2 * sh.rp : sh.rp, FMT);
+    // warp 1: w0 times the activations (both planes of the f16 pair if stacked), warp 2 (f16 pair): w1 x0, and w0 x1 if not
+    const uint32_t idesc = make_idesc(BM, sh.stacked && warp == 1 ? 2 * sh.rp : sh.rp, FMT);
     const int chain = NT == 1 ? nkb : (nkb + sh.leads - 1) / sh.leads;   // k-blocks per leading accumulator
     int ws = 0, xs = 0, in_chain = 0;
     uint32_t wph = 0, xph = 0;
@@ -229,6 +232,11 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
       if (one) {
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) umma_bf16(acc, w0 + (uint64_t)(ks * 2), x0 + (uint64_t)(ks * 2), idesc, (in_chain | ks) ? 1u : 0u);
+        if (NT == 2 && warp == 2 && !sh.stacked) {      // w0 x1
+          const uint64_t wl = w0 - (uint64_t)(W_BYTES >> 4), x1 = x0 + (uint64_t)(X_BYTES >> 4);
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks) umma_bf16(acc, wl + (uint64_t)(ks * 2), x1 + (uint64_t)(ks * 2), idesc, 1u);
+        }
         umma_commit(bars + 8u * (WS + ws));
         umma_commit(xbars + 8u * (XS + xs));
       }
@@ -261,7 +269,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
       for (int a = 0; a < ML; ++a)
         if (a < used) {
           tmem_ld8(at + (uint32_t)(a * sh.acc_stride), lead[a]);
-          if (NT > 1) tmem_ld8(at + (uint32_t)(a * sh.acc_stride + sh.rp), cross[a]);
+          if (NT > 1 && sh.stacked) tmem_ld8(at + (uint32_t)(a * sh.acc_stride + sh.rp), cross[a]);
         }
       if (NT > 1) tmem_ld8(at + (uint32_t)(sh.leads * sh.acc_stride), cross[ML]);
       tmem_wait_ld();
@@ -275,7 +283,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
           for (int a = 0; a < ML; ++a)
             if (a < used) {
               if (a > 0) v[i] += __uint_as_float(lead[a][i]);
-              c += __uint_as_float(cross[a][i]);
+              if (sh.stacked) c += __uint_as_float(cross[a][i]);
             }
           v[i] = fmaf(c, kF16PairInvScale, v[i]);
         }

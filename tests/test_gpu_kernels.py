@@ -94,10 +94,12 @@ def test_gemm_on_cta_pairs_vs_float64_and_one_tile(cuda_lib):
 
 @pytest.mark.parametrize("prec,tol", [("fp32", 1e-6), ("bf16", 4e-3)])
 @pytest.mark.parametrize("R,K,N", [(1, 64, 128), (3, 200, 130), (16, 2048, 4096), (17, 1000, 3000), (32, 130, 20000), (33, 2048, 4096),
-                                   (49, 700, 20000), (64, 1024, 391), (65, 256, 512)])
+                                   (49, 700, 20000), (64, 1024, 391), (65, 256, 512), (96, 2048, 4096), (128, 1024, 3000), (129, 2048, 4096),
+                                   (500, 1000, 4096)])
 def test_gemm_few_rows_vs_float64(cuda_lib, R, K, N, prec, tol):
-    """The weight-streaming product for up to 64 rows: edges of its row groups (4), MMA widths (16), of the change from
-    half to whole SMs (33) and to the other kernels (49 rows of many columns, 65), K slices of unequal length."""
+    """The weight-streaming product for few rows: edges of its row groups (4), MMA widths (16), of the change from half to
+    whole SMs and to one MMA per product (65), to the other kernels (49 rows of many columns, 65 / 129), K slices of unequal
+    length; and narrow tiles beyond."""
     from linmt_b200 import decoder
     rng = np.random.default_rng(R + K + N)
     X = rng.uniform(-1, 1, (R, K)).astype(np.float32)
