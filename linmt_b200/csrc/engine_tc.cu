@@ -140,6 +140,18 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
     ppair = true;
     bn = 208;
   }
+  // ... and the gate product of one plane, where one tile per CTA is more than one wave (beyond 1024 rows; measured at N =
+  // 4096, K = 2048: 22.4 / 28.3 us at 1280 rows, 25.7 / 30.6 at 1536): rounds of 3.9 + 0.0215 * width us, and a prologue
+  // and last epilogue of 4 + 0.033 * width.
+  if (Epi::kHasBlock && !Epi::kHasPmax && pair_ && persist_ && nt == 1 && splits == 1 && bk == 64 && mt > 8 && ws_parts_ == 1) {
+    double best = 1e30;
+    for (int w = 96; w <= 256; w += 16) {
+      const long t = (long)((mt + 1) / 2) * ((N + w - 1) / w), rounds = (t + n_sm_ / 2 - 1) / (n_sm_ / 2);
+      const double cost = 4.0 + 0.033 * w + rounds * (3.9 + 0.0215 * w) * K / 2048.0;
+      if (cost < best) { best = cost; bn = w; }
+    }
+    ppair = true;
+  }
   const long ntile_cols = (N + bn - 1) / bn;
   const bool pair = ppair || (pair_ && fmt_ == 1 && nt == 2 && bk == 64 && splits == 1 && mt >= 2 && bn % 16 == 0 &&
                     tc::make_shape(bn, nt, bk, fmt_).stages < 3 && (long)((mt + 1) & ~1) * ntile_cols <= n_sm_ && ws_parts_ == 1);
