@@ -323,7 +323,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   }
   // panels of the layer-by-layer encoder: all positions of a batch if that is at most 16384 rows (0.27 GB of input parts)
   if (use_tc_ && rows_ && (nt_ == 1 || fmt_ == 1)) {
-    const int nb = std::min(B, tc::kRowsMax);
+    const int nb = std::min(B, 64);
     enc_rows_ = std::min(opt.max_src_len * nb, std::max(16384, nb));
   }
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);
@@ -349,8 +349,8 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   if (nm > 1) DA(d_combined_, (size_t)R * Vp);
   DA(d_cand_idx_, (size_t)R * kk); DA(d_cand_logp_, (size_t)R * kk); DA(d_eos_logp_, R); DA(d_row_stats_, 2 * (size_t)R);
   pmax_ld_ = 4 * ((Vp + 47) / 48) + 4;   // four column blocks per tile, tiles at least 48 wide
-  DA(d_pmax_, (size_t)R * pmax_ld_);
-  DA(d_psum_, (size_t)tc::kRowsMax * pmax_ld_);
+  DA(d_pmax_, (size_t)nm * R * pmax_ld_);    // per member
+  DA(d_psum_, (size_t)nm * R * pmax_ld_);
   if (o.print_info) {
     DA(d_rec_align_, (size_t)Tcap * R * rec_win); DA(d_rec_lo_, (size_t)Tcap * R); DA(d_rec_vit_, (size_t)Tcap * R);
   }
@@ -499,6 +499,17 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
   return LINMT_OK;
 }
 
+// Softmax statistics and top-k of rows whose logits vocab_gemm has just produced, from the block statistics it left if it did.
+cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, const float* pmax, const float* psum, int rows, const TopkOut& o, int normalise,
+                                 const TopkRefine* rf, const SelectArgs& sel) {
+  if (!logits16_) logits16 = nullptr;
+  if (!pblocks_) return launch_softmax_topk(logits, Vp, V, kk, rows, o, normalise, stream, pdl_, pmax, pmax_ld_, pmax_slots_, rf, logits16, sel);
+  const LogitBlocks bl{pmax, psum, pmax_ld_, pmax_slots_, pmax_tile_, pmax_part_};
+  const bool wide = rows <= n_sm_;
+  return tc::launch_k(pdl_, wide ? topk_blocks_kernel<1024> : topk_blocks_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256), topk_blocks_smem(bl.n, rf ? rf->K : 0), stream,
+                      logits, logits16, Vp, V, kk, o, normalise, bl, rf ? *rf : TopkRefine{}, sel);
+}
+
 TopkRefine Engine::refinement(const tc::Planes& ht) const {
   const DevModel& m = models_[0];
   TopkRefine rf{};
@@ -528,26 +539,29 @@ int Engine::step_tail(int t, int rows) {
       if (refine_) rf = refinement(tc_states_[0].panel_ht);
       if (refine_) trace_dev_.rf = rf;
       sel.tr = trace_dev_;
-      if (pblocks_) {
-        const LogitBlocks bl{d_pmax_, d_psum_, pmax_ld_, pmax_slots_};
-        CK(tc::launch_k(pdl_, topk_blocks_kernel, dim3(rows), dim3(kTopkBlocksThreads), topk_blocks_smem(bl.n, rf.a0 ? rf.K : 0), stream,
-                        (const float*)s.logits, logits16_ ? (const __half*)s.logits16 : (const __half*)nullptr, Vp, V, kk, o, 1, bl, rf, sel));
-      } else
-        CK(launch_softmax_topk(s.logits, Vp, V, kk, rows, o, 1, stream, pdl_, d_pmax_, pmax_ld_, pmax_slots_, refine_ ? &rf : nullptr,
-                               logits16_ ? s.logits16 : nullptr, sel));
+      CK(softmax_topk(s.logits, s.logits16, d_pmax_, d_psum_, rows, o, 1, refine_ ? &rf : nullptr, sel));
     } else {
       // EnsembleFactory::EnsemblesModels (src/decoder.h:1910-1931): mean of the members'
       // probabilities, renormalised -- written as log(mean p) so that the log-softmax of the
       // combined row IS the renormalisation; or the plain mean of log-probabilities.
+      // Combination, softmax and top-k are one kernel unless the combined row itself is asked for (scores of forced tokens).
       EnsembleRows er{};
       for (int mi = 0; mi < n_models; ++mi) er.logits[mi] = states_[mi].logits;
       er.n = n_models;
-      if (int rc = kt(KC_COMBINE)) return rc;
-      CK(tc::launch_k(pdl_, ensemble_combine_kernel, dim3(rows), dim3(256), 0, stream, er, Vp, V, (int)opt.ensemble_mode, d_combined_));
-      LAUNCHED();
-      if (int rc = kt(KC_SOFTMAX)) return rc;
       sel.tr = trace_dev_;
-      CK(launch_softmax_topk(d_combined_, Vp, V, kk, rows, o, opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0, stream, pdl_, nullptr, 0, 0, nullptr, nullptr, sel));
+      if (int rc = kt(KC_COMBINE)) return rc;
+      const size_t smem = sizeof(float) * (size_t)((V + 127) / 128);
+      if (trace_dev_.gold_logp || smem > (size_t)kBlocksSmemMax) {
+        CK(tc::launch_k(pdl_, ensemble_combine_kernel, dim3(rows), dim3(256), 0, stream, er, Vp, V, (int)opt.ensemble_mode, d_combined_));
+        LAUNCHED();
+        if (int rc = kt(KC_SOFTMAX)) return rc;
+        CK(launch_softmax_topk(d_combined_, Vp, V, kk, rows, o, opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0, stream, pdl_, nullptr, 0, 0, nullptr, nullptr, sel));
+      } else {
+        const bool wide = rows <= n_sm_;
+        const LogitBlocks bl{d_pmax_, d_psum_, pmax_ld_, pblocks_ ? pmax_slots_ : 0, pmax_tile_, pmax_part_};
+        CK(tc::launch_k(pdl_, wide ? ensemble_topk_kernel<1024> : ensemble_topk_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256), smem, stream, er, Vp, V, kk,
+                        (int)opt.ensemble_mode, o, bl, (long long)R * pmax_ld_, d_combined_, sel));
+      }
     }
     LAUNCHED();
   }

@@ -126,7 +126,10 @@ class Engine {
   // a step of scoring: the tokens read, where every member's htilde goes and where the previous step's is
   struct ScoreStep { const int32_t* tok; const tc::Planes* ht; const tc::Planes* ht_prev; };
   int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr);
-  int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax);
+  void note_blocks(float** pmax, float** psum, int ld, int N, int K, int tile, int part);
+  int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum);
+  cudaError_t softmax_topk(const float* logits, const __half* logits16, const float* pmax, const float* psum, int rows, const TopkOut& o, int normalise,
+                           const TopkRefine* rf, const SelectArgs& sel);
   int score_core_tc(int n, int Smax, const std::vector<int>& n_act, const int32_t* d_tok, const int32_t* d_gold, float* d_logp);
   int reserve_score(size_t rows);
   TopkRefine refinement(const tc::Planes& ht) const;    // of one-product logits of these attentional states
@@ -199,10 +202,11 @@ class Engine {
   float* d_combined_ = nullptr;  // [R][Vp] ensemble-combined log-values (n_models > 1)
   int32_t* d_cand_idx_ = nullptr;
   float *d_cand_logp_ = nullptr, *d_eos_logp_ = nullptr, *d_row_stats_ = nullptr;
-  float* d_pmax_ = nullptr;   // [R][pmax_ld_] block maxima of the logits, by-product of the vocabulary GEMM
-  float* d_psum_ = nullptr;   // [64][pmax_ld_] sums of exponentials of the same blocks (few rows)
+  float* d_pmax_ = nullptr;   // [members][R][pmax_ld_] block maxima of the logits, by-product of the vocabulary GEMM ...
+  float* d_psum_ = nullptr;   // ... and the blocks' sums of exp(z - maximum)
   int pmax_ld_ = 0;
-  bool pblocks_ = false;      // the last vocabulary GEMM left maxima and sums of 32-column blocks
+  bool pblocks_ = false;      // the last vocabulary GEMM left both, for pmax_slots_ blocks: four of pmax_part_ columns per tile of pmax_tile_
+  int pmax_tile_ = 1, pmax_part_ = 1;
   int pmax_slots_ = 0;        // slots the last vocabulary GEMM filled (0 = none: the softmax finds its own maxima)
   // alignment records (print_info)
   float* d_rec_align_ = nullptr;
@@ -221,7 +225,7 @@ class Engine {
   int score_q_ = 0;
   std::vector<float*> score_logits_;
   __half* score_logits16_ = nullptr;
-  float *score_combined_ = nullptr, *score_candp_ = nullptr, *score_eos_ = nullptr, *score_stats_ = nullptr, *score_pmax_ = nullptr;
+  float *score_combined_ = nullptr, *score_candp_ = nullptr, *score_eos_ = nullptr, *score_stats_ = nullptr, *score_pmax_ = nullptr, *score_psum_ = nullptr;
   int32_t *score_idx_ = nullptr, *score_io_ = nullptr;
   size_t score_io_cap_ = 0;
   template <class T> int dalloc_bytes(T** p, size_t bytes) {

@@ -130,14 +130,15 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   // CTA pairs (gemm_tc_pair.cuh) where the one-tile shape has room for two stages only: an even number of row
   // tiles (an odd one is rounded up, which must still fit one wave), split operands, 64-deep stages, K not split
   const int mt = (M + tc::BM - 1) / tc::BM;
-  // The many-wave one-plane logits GEMM has a persistent pair form as well: worth it for an even number of row tiles
-  // (measured at N = 30016, K = 1024: 56.2 against 61.7 us at 768 rows, 24.5 against 27.7 at 192; an odd number of
-  // row tiles wastes half a pair and loses), with 208-wide tiles.
+  // The many-wave one-plane logits GEMM has a persistent pair form as well (measured at K = 1024, against one tile per CTA:
+  // N = 30016 23.6 / 29.5 us at 256 rows, 51 / 57 at 640, 55 / 71 at 768; N = 80000 104 / 124 at 512; three row tiles, a
+  // quarter of the pair idle, are equal), with 208-wide tiles.
   const bool one_plane_logits = nt == 1 && Epi::kHasPmax;   // the fp32-output GEMMs: vocabulary projection
+  // (the block statistics depend on the tile width, so the width is the pair's whether or not pairs may run)
   bool ppair = false;
-  if (pair_ && persist_ && one_plane_logits && splits == 1 && bk == 64 && mt % 2 == 0 && ws_parts_ == 1 &&
-      (long)mt * ((N + bn - 1) / bn) > n_sm_ && (long)(mt / 2) * ((N + 207) / 208) > n_sm_ / 2) {
-    ppair = true;
+  if (one_plane_logits && splits == 1 && bk == 64 && mt >= 2 && ws_parts_ == 1 &&
+      (long)mt * ((N + bn - 1) / bn) > n_sm_ && (long)((mt + 1) / 2) * ((N + 207) / 208) > n_sm_ / 2) {
+    ppair = pair_ && persist_;
     bn = 208;
   }
   // ... and the gate product of one plane, where one tile per CTA is more than one wave (beyond 1024 rows; measured at N =
@@ -174,11 +175,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
       rs.pdl = (pdl_ && pdl_gemm_) ? 1 : 0;
       if constexpr (Epi::kHasPmax) {
         if (e.pmax) {      // block maxima of 32 columns
-          const int slots = 4 * ((N + tc::BM - 1) / tc::BM);
-          if (slots > e.pmax_ld) { e.pmax = nullptr; pmax_slots_ = 0; }
-          else pmax_slots_ = slots;
-          pblocks_ = e.pmax && topk_blocks_smem(slots, K) <= kBlocksSmemMax;
-          e.psum = pblocks_ ? d_psum_ : nullptr;
+          note_blocks(&e.pmax, &e.psum, e.pmax_ld, N, K, tc::BM, 32);
         }
       }
       if (nt == 2) CK((tc::launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
@@ -202,9 +199,8 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   if constexpr (Epi::kHasPmax) {
     // block maxima for the softmax: four column blocks per tile; not from the split-K fix-up path
     if (e.pmax) {
-      const int slots = 4 * ((N + bn - 1) / bn);
-      if (splits > 1 || slots > e.pmax_ld) { e.pmax = nullptr; pmax_slots_ = 0; }
-      else pmax_slots_ = slots;
+      if (splits > 1) e.pmax = e.psum = nullptr;
+      else note_blocks(&e.pmax, &e.psum, e.pmax_ld, N, K, bn, ((bn >> 4) + 3) / 4 * 16);
     }
   }
   // many waves of tiles whose leading product is one chain: one persistent CTA per SM
@@ -221,6 +217,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
     return LINMT_OK;
   }
   }
+  if constexpr (Epi::kHasPmax) {
   if (persist_ && splits == 1 && tiles > n_sm_ && ((nt == 2 && drain >= K / 32) || one_plane_logits)) {
     if (nt == 1) {
       const int pdl = sh.pdl;
@@ -230,6 +227,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
     CK(tc::launch_gemm_tc_persist(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_));
     LAUNCHED();
     return LINMT_OK;
+  }
   }
   if (pair) {
     CK((tc::launch_gemm_tc_pair<2, 64, 1, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, nullptr, nullptr)));
@@ -534,16 +532,25 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   // 6. logits
   if (sc) return LINMT_OK;
   if (int rc = kt(KC_VOCAB)) return rc;
-  return vocab_gemm(mi, ts.panel_ht, R, rows, s.logits, s.logits16, d_pmax_);
+  return vocab_gemm(mi, ts.panel_ht, R, rows, s.logits, s.logits16, d_pmax_ + (size_t)mi * R * pmax_ld_, d_psum_ + (size_t)mi * R * pmax_ld_);
+}
+
+// What block statistics a vocabulary GEMM is going to leave: four blocks of `part` columns per tile of `tile`.
+void Engine::note_blocks(float** pmax, float** psum, int ld, int N, int K, int tile, int part) {
+  const int slots = 4 * ((N + tile - 1) / tile);
+  if (slots > ld) { *pmax = *psum = nullptr; return; }
+  pmax_slots_ = slots; pmax_tile_ = tile; pmax_part_ = part;
+  if (topk_blocks_smem(slots, K) > (size_t)kBlocksSmemMax) *psum = nullptr;
+  pblocks_ = *psum != nullptr;
 }
 
 // Logits of `rows` attentional states.
-int Engine::vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax) {
+int Engine::vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum) {
   DevModel& m = models_[mi];
   tc::TcEpiF32 e{m.voc_b, logits, Vp, 0};
   if (logits16_) e.out16 = logits16;   // the softmax of this step is their only reader
   pmax_slots_ = 0; pblocks_ = false;
-  if (n_models == 1 && pmax_on_) { e.pmax = pmax; e.pmax_ld = pmax_ld_; e.n_valid = V; }
+  if (pmax_on_ && pmax) { e.pmax = pmax; e.psum = psum; e.pmax_ld = pmax_ld_; e.n_valid = V; }
   // Logits feed only the softmax of their own step: the tensor core's truncation bias over one
   // K = Hp chain (~32 ulp of the accumulator, 2e-7 relative on a log-probability) does not
   // accumulate over steps as it does through the recurrent products, so this GEMM runs its
@@ -585,7 +592,7 @@ int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const 
       tc::Planes a = score_ht_[mi];
       for (int p = 0; p < nt_; ++p) a.p[p] += r0 * Hp;
       if (mi == 0 && refine_) rf = refinement(a);
-      if (int rc = vocab_gemm(mi, a, (int)std::min<size_t>(score_q_, score_rows_ - r0), rows, score_logits_[mi], score_logits16_, score_pmax_)) return rc;
+      if (int rc = vocab_gemm(mi, a, (int)std::min<size_t>(score_q_, score_rows_ - r0), rows, score_logits_[mi], score_logits16_, n_models == 1 ? score_pmax_ : nullptr, score_psum_)) return rc;
     }
     const float* logits = score_logits_[0];
     int normalise = 1;
@@ -598,8 +605,7 @@ int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const 
       logits = score_combined_;
       normalise = opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0;
     }
-    CK(launch_softmax_topk(logits, Vp, V, kk, rows, o, normalise, stream, pdl_, score_pmax_, pmax_ld_, pmax_slots_, refine_ ? &rf : nullptr,
-                           logits16_ ? score_logits16_ : nullptr));
+    CK(softmax_topk(logits, score_logits16_, score_pmax_, score_psum_, rows, o, normalise, refine_ ? &rf : nullptr, SelectArgs{}));
     LAUNCHED();
     CK(tc::launch_k(pdl_, gold_logp_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, d_gold + r0, rows, logits, Vp, V, (const float*)score_stats_, rf, d_logp + r0));
     LAUNCHED();
@@ -632,7 +638,8 @@ int Engine::reserve_score(size_t rows) {
   }
   if (n_models > 1 && (rc = dalloc_bytes(&score_combined_, cap * Vp * 4))) return rc;
   if ((rc = dalloc_bytes(&score_idx_, cap * kk * 4)) || (rc = dalloc_bytes(&score_candp_, cap * kk * 4)) || (rc = dalloc_bytes(&score_eos_, cap * 4)) ||
-      (rc = dalloc_bytes(&score_stats_, cap * 8)) || (rc = dalloc_bytes(&score_pmax_, cap * pmax_ld_ * 4)))
+      (rc = dalloc_bytes(&score_stats_, cap * 8)) || (rc = dalloc_bytes(&score_pmax_, cap * pmax_ld_ * 4)) ||
+      (rc = dalloc_bytes(&score_psum_, cap * pmax_ld_ * 4)))
     return rc;
   score_q_ = (int)cap;
   return LINMT_OK;

@@ -290,6 +290,9 @@ __device__ __forceinline__ void split_store4(const Planes& pl, int nt, size_t id
   }
 }
 
+// 2^x (2 ulp), results below the normal range to zero
+__device__ __forceinline__ float exp2f_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+
 // Activation functions of the fused epilogues.  The hardware exponential (ex2.approx, 2 ulp) and
 // reciprocal keep the ABSOLUTE error of both below ~1.5e-7 -- what the matrix products that consume h
 // care about -- at a third of the instructions of expf / tanhf; around zero, where
@@ -401,9 +404,10 @@ struct TcEpiLstm {
     block_of<kEpiBlockChunks, 3>(row0, lane, M, col_first, nch, v, sbuf);
   }
   // up to two chunks at a time in a small staging area of the warp's own (persistent kernels, one plane)
-  __device__ __forceinline__ float staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf) const {
+  struct Stat {};
+  static __device__ __forceinline__ Stat no_stat() { return Stat{}; }
+  __device__ __forceinline__ void staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, Stat&) const {
     block_of<2, 1>(row0, lane, M, col_first, nch, v, sbuf);
-    return 0.f;
   }
   // CH = most chunks, PL = planes there is room for
   template <int CH, int PL>
@@ -602,7 +606,7 @@ struct TcEpiF32 {
   // 64 columns (tile column block `slot`) of every row, over columns < n_valid, at pmax[row * pmax_ld + slot].
   // The softmax kernel then needs no first sweep over the row for its maximum and its top-k threshold.
   float* pmax = nullptr; int pmax_ld = 0; int n_valid = 0;
-  float* psum = nullptr;    // row form only: sum of exp(z - maximum) of the same block
+  float* psum = nullptr;    // optional: sum of exp(z - maximum) of the same block, so that nobody has to sweep the row for it
   // Optional half-precision output (out16 set: `out` is not written): logits whose few values that matter one by one
   // are recomputed by their consumer and which otherwise only enter a sum of exponentials go out as fp16, half
   // the bytes to write and to sweep.  The block maxima are then those of the ROUNDED values (elements of the row).
@@ -638,8 +642,60 @@ struct TcEpiF32 {
   // staged per row, then stored with a row's 16 float4 on consecutive lanes.
   static constexpr bool kHasBlock = true;
   static constexpr bool kHasPmax = true;
-  __device__ __forceinline__ void pmax_store(int row, int M, int slot, float m) const {
-    if (pmax && row < M) pmax[(size_t)row * pmax_ld + slot] = m;
+  struct Stat { float m, s; };       // maximum and sum of exp(z - maximum) of some columns of a row
+  static __device__ __forceinline__ Stat no_stat() { return Stat{-INFINITY, 0.f}; }
+  __device__ __forceinline__ void merge(Stat& a, const Stat& b) const {
+    if (b.m == -INFINITY) return;
+    const float m = fmaxf(a.m, b.m);
+    if (psum) a.s = a.s * __expf(a.m - m) + b.s * __expf(b.m - m);    // (a.m = -inf: 0)
+    a.m = m;
+  }
+  // Of finished values v[0 .. nch), two chunks at a time: every kernel forms a block's statistics in the same steps, so
+  // that which of them runs does not show in the results.
+  template <int CH>
+  __device__ __forceinline__ Stat stat_of(int col_first, int nch, const float (*v)[16]) const {
+    Stat st = no_stat();
+    if (!pmax) return st;
+#pragma unroll
+    for (int c0 = 0; c0 < CH; c0 += 2) {
+      Stat h = no_stat();
+      if (col_first + 16 * (c0 + 2) <= n_valid && c0 + 2 <= nch) {      // both chunks whole: nothing to test
+#pragma unroll
+        for (int ci = c0; ci < c0 + 2 && ci < CH; ++ci)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) h.m = fmaxf(h.m, v[ci][i]);
+        if (psum) {
+#pragma unroll
+          for (int ci = c0; ci < c0 + 2 && ci < CH; ++ci)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) h.s += exp2f_fast((v[ci][i] - h.m) * 1.4426950408889634f);
+        }
+      } else {
+#pragma unroll
+        for (int ci = c0; ci < c0 + 2 && ci < CH; ++ci)
+          if (ci < nch) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (col_first + 16 * ci + i < n_valid) h.m = fmaxf(h.m, v[ci][i]);
+          }
+        if (psum && h.m > -INFINITY) {
+#pragma unroll
+          for (int ci = c0; ci < c0 + 2 && ci < CH; ++ci)
+            if (ci < nch) {
+#pragma unroll
+              for (int i = 0; i < 16; ++i) h.s += col_first + 16 * ci + i < n_valid ? __expf(v[ci][i] - h.m) : 0.f;
+            }
+        }
+      }
+      merge(st, h);
+    }
+    return st;
+  }
+  __device__ __forceinline__ void stat_store(int row, int M, int slot, const Stat& st) const {
+    if (pmax && row < M) {
+      pmax[(size_t)row * pmax_ld + slot] = st.m;
+      if (psum) psum[(size_t)row * pmax_ld + slot] = st.s;
+    }
   }
   __device__ __forceinline__ float max4(float m, const float4& r, int c) const {
     if (c + 0 < n_valid) m = fmaxf(m, r.x);
@@ -650,7 +706,6 @@ struct TcEpiF32 {
   }
   // the same block without staging (row-per-lane stores), for callers whose staging area is busy
   __device__ __forceinline__ void direct_block(int row, int M, int col_first, int nch, float (*v)[16], int slot) const {
-    float m = -INFINITY;
     if (row < M) {
 #pragma unroll
       for (int ci = 0; ci < kEpiBlockChunks; ++ci) {
@@ -660,47 +715,54 @@ struct TcEpiF32 {
           for (int q = 0; q < 4; ++q) {
             const float4 r = finish4(make_float4(v[ci][4 * q], v[ci][4 * q + 1], v[ci][4 * q + 2], v[ci][4 * q + 3]), col0 + 4 * q);
             store4((size_t)row * ld + col0 + 4 * q, r);
-            m = max4(m, r, col0 + 4 * q);
+            v[ci][4 * q] = r.x; v[ci][4 * q + 1] = r.y; v[ci][4 * q + 2] = r.z; v[ci][4 * q + 3] = r.w;
           }
         }
       }
     }
-    pmax_store(row, M, slot, m);
+    stat_store(row, M, slot, stat_of<kEpiBlockChunks>(col_first, nch, v));
   }
-  // Stages nch (<= 4) chunks of this warp's 32 rows with `stride` floats per row (>= 16 * nch + 4) and
-  // stores them with consecutive lanes on consecutive addresses; returns this lane's (= row's) maximum
-  // over the valid columns.
-  __device__ __forceinline__ float stage_store(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf,
-                                               int stride) const {
-    float m = -INFINITY;
+  // Stages nch (<= CH) chunks of this warp's 32 rows with `stride` floats per row (>= 16 * nch + 4) and
+  // stores them with consecutive lanes on consecutive addresses; returns this lane's (= row's) statistics
+  // of the valid columns.
+  template <int CH>
+  __device__ __forceinline__ Stat stage_store(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf,
+                                              int stride) const {
 #pragma unroll
-    for (int ci = 0; ci < kEpiBlockChunks; ++ci) {
+    for (int ci = 0; ci < CH; ++ci) {
       if (ci < nch) {
         const int col0 = col_first + 16 * ci;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float4 r = finish4(make_float4(v[ci][4 * q], v[ci][4 * q + 1], v[ci][4 * q + 2], v[ci][4 * q + 3]), col0 + 4 * q);
           *reinterpret_cast<float4*>(sbuf + lane * stride + 16 * ci + 4 * q) = r;
-          m = max4(m, r, col0 + 4 * q);
+          v[ci][4 * q] = r.x; v[ci][4 * q + 1] = r.y; v[ci][4 * q + 2] = r.z; v[ci][4 * q + 3] = r.w;
         }
       }
     }
     __syncwarp();
     const int nq = 4 * nch;   // float4 per row
-    for (int s = lane; s < 32 * nq; s += 32) {
-      const int r = s / nq, g = s - r * nq;
-      if (row0 + r < M) store4((size_t)(row0 + r) * ld + col_first + 4 * g, *reinterpret_cast<const float4*>(sbuf + r * stride + 4 * g));
+    if (nch == 2 && row0 + 32 <= M) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int r = 4 * i + (lane >> 3), g = lane & 7;
+        store4((size_t)(row0 + r) * ld + col_first + 4 * g, *reinterpret_cast<const float4*>(sbuf + r * stride + 4 * g));
+      }
+    } else {
+      for (int s = lane; s < 32 * nq; s += 32) {
+        const int r = s / nq, g = s - r * nq;
+        if (row0 + r < M) store4((size_t)(row0 + r) * ld + col_first + 4 * g, *reinterpret_cast<const float4*>(sbuf + r * stride + 4 * g));
+      }
     }
     __syncwarp();
-    return m;
+    return stat_of<CH>(col_first, nch, v);
   }
-  // up to two chunks at a time, see TcEpiLstm; returns the row's maximum over them
-  __device__ __forceinline__ float staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf) const {
-    return stage_store(row0, lane, M, col_first, nch, v, sbuf, kStagedStride);
+  // up to two chunks at a time, see TcEpiLstm; merged into the row's statistics
+  __device__ __forceinline__ void staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, Stat& st) const {
+    merge(st, stage_store<2>(row0, lane, M, col_first, nch, v, sbuf, kStagedStride));
   }
   __device__ __forceinline__ void block(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, int slot) const {
-    const float m = stage_store(row0, lane, M, col_first, nch, v, sbuf, kEpiScratchStride);
-    pmax_store(row0 + lane, M, slot, m);
+    stat_store(row0 + lane, M, slot, stage_store<kEpiBlockChunks>(row0, lane, M, col_first, nch, v, sbuf, kEpiScratchStride));
   }
   // Row form, see TcEpiLstm; a warp holds 32 columns of four rows (lane & 3 = row), the block maxima are theirs.
   struct Pre { float4 b; };
@@ -962,7 +1024,7 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
         if (Epi::kHasBlock) {
           const int slot = (int)blockIdx.y * kParts + part;
           if (nmine > 0) epi.block(row0, lane, M, n0 + ch0 * 16, nmine, macc, sbuf, slot);
-          else if constexpr (Epi::kHasPmax) epi.pmax_store(row, M, slot, -INFINITY);
+          else if constexpr (Epi::kHasPmax) epi.stat_store(row, M, slot, Epi::no_stat());
         } else if (row < M) {
 #pragma unroll
           for (int ci = 0; ci < kChunks; ++ci)
@@ -1079,14 +1141,13 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
 // TMEM back at once, and write their tile to memory while the tensor core is already on the next
 // one -- the ~7 us of prologue and epilogue that every tile of a multi-wave launch used to pay is
 // paid once per CTA.  Stores: the staging area of the one-tile kernel is the stage ring, which is busy
-// here, so either the launch sets aside a small staging area of its own (stage_stride > 0: 32 rows x
-// stage_stride floats per epilogue warp, two 16-column chunks at a time -- the one-plane launches, whose
-// ring leaves the room), or tiles go out with row-per-lane stores and only a CTA's last tile, with the
-// ring idle, is staged there.  No split-K, no intermediate drains.
+// here; one-plane launches, whose ring leaves the room, set a small staging area aside for every epilogue warp (two
+// 16-column chunks at a time), the others store row per lane.  No split-K, no intermediate drains.  Epilogues with
+// block statistics only (TcEpiF32).
 template <int NT, int BKT, int FMT, class Epi>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, int STAGES, Epi epi,
-                       int* __restrict__ err_flag, int stage_stride) {
+                       int* __restrict__ err_flag) {
   constexpr int PC = product_code(NT, FMT);
   constexpr int NP = num_products(PC);
   constexpr int A_BYTES = BM * BKT * 2;
@@ -1097,8 +1158,8 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
   unsigned char* base_ptr = smem_raw + (base - raw);
   const int B_BYTES = BN * BK * 2;
   const int STAGE_BYTES = NT * (A_BYTES + B_BYTES);
-  const int STG_WARP = 32 * stage_stride * 4;                    // bytes of a warp's own staging area (0: none)
-  const int RING = (stage_stride > 0 ? STAGES * STAGE_BYTES : ring_bytes(STAGES, STAGE_BYTES));
+  constexpr int STG_WARP = NT == 1 ? 32 * kStagedStride * 4 : 0;  // bytes of a warp's own staging area
+  const int RING = NT == 1 ? STAGES * STAGE_BYTES : ring_bytes(STAGES, STAGE_BYTES);
   const int PRE = RING + kEpiWarps * STG_WARP;                   // ring, then the staging areas, then the barriers
   const uint32_t bars = base + PRE;   // full[STAGES], empty[STAGES], accum_full, tmem_free
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(base_ptr + PRE + 8 * (2 * STAGES + 3));
@@ -1202,7 +1263,6 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
     const int ch0 = part * cpw;
     const uint32_t astride = (uint32_t)acc_stride(BN);
     const uint32_t lane_base = tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(ch0 * 16);
-    float* sbuf = reinterpret_cast<float*>(base_ptr + (warp - 2) * kEpiScratchBytes);
     pdl_wait();
     int it = 0;
     for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x, ++it) {
@@ -1231,34 +1291,21 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tmem_free);   // the tensor core may start the next tile
-      const bool last = tile + (int)gridDim.x >= ntile;
       const int slot = (tile / mt) * kParts + part;
-      if constexpr (Epi::kHasPmax) {
-        if (stage_stride > 0) {
-          // this warp's own staging area: as many chunks at a time as a staged row holds
-          float* own = reinterpret_cast<float*>(base_ptr + RING + (warp - 2) * STG_WARP);
-          float m = -INFINITY;
+      if constexpr (NT == 1) {
+        // this warp's own staging area: as many chunks at a time as a staged row holds
+        float* own = reinterpret_cast<float*>(base_ptr + RING + (warp - 2) * STG_WARP);
+        auto st = Epi::no_stat();
 #pragma unroll
-          for (int c0 = 0; c0 < kChunks; c0 += 2) {   // two chunks at a time (stage_stride >= 36); static indices keep macc in registers
-            if (c0 < nmine) {
-              const int nc = nmine - c0 < 2 ? nmine - c0 : 2;
-              m = fmaxf(m, epi.stage_store(row0, lane, M, n0 + (ch0 + c0) * 16, nc, macc + c0, own, stage_stride));
-            }
+        for (int c0 = 0; c0 < kChunks; c0 += 2) {   // two chunks at a time; static indices keep macc in registers
+          if (c0 < nmine) {
+            const int nc = nmine - c0 < 2 ? nmine - c0 : 2;
+            epi.staged(row0, lane, M, n0 + (ch0 + c0) * 16, nc, macc + c0, own, st);
           }
-          epi.pmax_store(row0 + lane, M, slot, m);
-          continue;
         }
-      }
-      if (last && Epi::kHasBlock) {
-        // the ring is idle from here on: stage and store coalesced
-        if (nmine > 0) epi.block(row0, lane, M, n0 + ch0 * 16, nmine, macc, sbuf, slot);
-        else if constexpr (Epi::kHasPmax) epi.pmax_store(row0 + lane, M, slot, -INFINITY);
-      } else if constexpr (Epi::kHasPmax) {
+        epi.stat_store(row0 + lane, M, slot, st);
+      } else {
         epi.direct_block(row0 + lane, M, n0 + ch0 * 16, nmine, macc, slot);
-      } else if (row0 + lane < M) {
-#pragma unroll
-        for (int ci = 0; ci < kChunks; ++ci)
-          if (ci < nmine) epi(row0 + lane, n0 + (ch0 + ci) * 16, macc[ci]);
       }
     }
   }
@@ -1375,13 +1422,12 @@ inline cudaError_t launch_gemm_tc_persist(const TmapSet& tm, int M, int N, int K
   if ((sh.nt != 2 && sh.nt != 1) || K % sh.bk || sh.stages < 2) return cudaErrorInvalidValue;
   const int tiles = ((M + BM - 1) / BM) * ((N + sh.bn - 1) / sh.bn);
   const dim3 grid(tiles < n_sm ? tiles : n_sm);
-  const int stride = sh.nt == 1 ? kStagedStride : 0;
 #define LINMT_PERSIST_CASE(NTV, BKV, FMTV)                                                                                   \
   {                                                                                                                          \
     static bool optin_done[kMaxDevices] = {};                                                                                \
     if (cudaError_t e = ensure_smem_optin(gemm_tc_persist_kernel<NTV, BKV, FMTV, Epi>, optin_done); e != cudaSuccess) return e; \
     return launch_k(sh.pdl != 0, gemm_tc_persist_kernel<NTV, BKV, FMTV, Epi>, grid, dim3(kThreads), (size_t)sh.smem_bytes, st, tm, M, N, K, \
-                    sh.bn, sh.stages, epi, err_flag, stride);                                                                \
+                    sh.bn, sh.stages, epi, err_flag);                                                                \
   }
   if (sh.nt == 1) {
     if (sh.fmt == 1 && sh.bk == 64) LINMT_PERSIST_CASE(1, 64, 1)
@@ -1419,8 +1465,8 @@ inline int pick_bn(int M, int N, int n_sm) {
 // waves * (k-blocks-per-CTA of those + ~8-13 us of prologue/epilogue per tile), plus the cost of
 // writing and re-reading partial tiles when K is split (only worth it for tiles up to 176 wide).
 // ws_floats bounds the split-K workspace (splits * padded rows * N floats).
-// The f16 pair with 64-deep stages, measured (two issuing threads): a k-block costs ~490 ns while the
-// issuing threads are the limit (tiles up to ~100 wide) and 120 + 3.6 * bn ns beyond (the tensor pipe at
+// The f16 pair with 64-deep stages, measured: a k-block costs ~400 ns on narrow tiles (an MMA of 128 rows has a floor of
+// ~65 clocks however narrow it is) and 120 + 3.6 * bn ns on wider ones (the tensor pipe at
 // its practical rate); per tile ~6 us + 12 ns per column of prologue and epilogue; a split adds ~2 us plus
 // 0.28 ns per partial-tile element that is written and read back (valid rows only).
 inline void pick_shape_f16(int M, int N, int K, int n_sm, size_t ws_floats, int max_tiles, int* bn_out, int* splits_out) {
@@ -1432,7 +1478,7 @@ inline void pick_shape_f16(int M, int N, int K, int n_sm, size_t ws_floats, int 
   for (int bn = 256; bn >= 64; bn -= 16) {
     const long tiles = (long)mt * ((N + bn - 1) / bn);
     const double wide = 120.0 + 3.6 * bn;
-    const double per_kb = wide > 490.0 ? wide : 490.0;
+    const double per_kb = wide > 400.0 ? wide : 400.0;
     for (int s = 1; s <= 6; ++s) {
       if (s > 1 && (bn > 208 || nkb / s < 2 || tiles > max_tiles || (size_t)s * mt * BM * (size_t)N > ws_floats)) break;
       const long waves = (tiles * s + n_sm - 1) / n_sm;

@@ -244,7 +244,7 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
         if (Epi::kHasBlock) {
           const int slot = (int)blockIdx.y * kParts + part;
           if (nmine > 0) epi.block(row0, lane, M, n0 + ch0 * 16, nmine, macc, sbuf, slot);
-          else if constexpr (Epi::kHasPmax) epi.pmax_store(row, M, slot, -INFINITY);
+          else if constexpr (Epi::kHasPmax) epi.stat_store(row, M, slot, Epi::no_stat());
         } else if (row < M) {
 #pragma unroll
           for (int ci = 0; ci < kChunks; ++ci)
@@ -371,7 +371,7 @@ inline cudaError_t launch_gemm_tc_pair(const TmapSet& tm, int M, int N, int K, c
 // Two accumulators of up to 256 columns each: while the tensor cores are on one tile, the epilogue warps take the other
 // out of TMEM, two 16-column chunks at a time through a staging area of their own, so that neither waits for the other.
 // What bounds it is what an SM takes in (128 + BN / 2 operand rows per k-block and CTA), hence tiles as wide as the
-// columns allow.  Measured against one accumulator: see persist_pair_bn.
+// columns allow.  Measured against one accumulator: see the dispatch.
 inline Shape make_shape_persist_pair(int bn, int fmt) {
   Shape s = make_shape_pair(bn, 1, 64, fmt);
   const int stg = kEpiWarps * 32 * kStagedStride * 4;
@@ -509,7 +509,7 @@ gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, in
       }
       if (!mbar_wait_sleepy(accum_full + 8u * b, (uint32_t)((it >> 1) & 1), &s_abort)) break;
       tc_fence_after();
-      float m = -INFINITY;
+      auto st = Epi::no_stat();
 #pragma unroll
       for (int c0 = 0; c0 < kEpiBlockChunks; c0 += 2) {
         const int nc = nmine - c0 < 2 ? nmine - c0 : 2;
@@ -521,9 +521,9 @@ gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, in
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(tmem_free_leader + 8u * b);
         }
-        if (nc > 0 && row0 < M) m = fmaxf(m, epi.staged(row0, lane, M, n0 + (ch0 + c0) * 16, nc, v, own));
+        if (nc > 0 && row0 < M) epi.staged(row0, lane, M, n0 + (ch0 + c0) * 16, nc, v, own, st);
       }
-      if constexpr (Epi::kHasPmax) epi.pmax_store(row0 + lane, M, (tile / mt2) * kParts + part, m);
+      if constexpr (Epi::kHasPmax) epi.stat_store(row0 + lane, M, (tile / mt2) * kParts + part, st);
     }
   }
   tc_fence_before();

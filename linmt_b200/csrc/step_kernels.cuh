@@ -1026,22 +1026,22 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
   select_if_last<256>(sel, out, r, s_union);
 }
 
-// The same result when the GEMM that produced the logits left, for every block of 32 columns of a row, the block's maximum
-// AND its sum of exp(z - maximum) (gemm_tc_rows.cuh): the row itself is not swept.  The maximum, the sum and the threshold
-// come from the blocks (938 pairs for 30,000 classes), and only blocks whose maximum reaches the threshold are looked into.
-// For few rows, whose one CTA each has an SM to itself and is bound by the chain of its memory round trips, not by bytes
-// (one sentence at 12 rows, 30k classes: 22.2 us per step sweeping).
+// The same result when the GEMM that produced the logits left, for every block of up to 64 columns of a row, the block's
+// maximum AND its sum of exp(z - maximum) (TcEpiF32): the row itself is not swept.  The maximum, the sum and the threshold
+// come from the blocks (580 or 940 pairs for 30,000 classes), and only blocks whose maximum reaches the threshold are
+// looked into.  THREADS = 1024 for few rows, whose one CTA each has an SM to itself and is bound by the chain of its memory
+// round trips (one sentence at 12 rows, 30k classes: 22.2 us per step sweeping, 13.1 so); 256 otherwise, where the sweep
+// read what the GEMM had just written.
 // grid = rows, dynamic smem = topk_blocks_smem
-constexpr int kBlockCols = 32;
 constexpr int kBlocksSmemMax = 23 * 1024;   // of dynamic shared memory beside the candidate lists: wider rows are swept
 struct LogitBlocks {
   const float* max; const float* sum; int ld; int n;
+  int tile, part;     // columns of a GEMM tile and of one of its four blocks (the last one of a tile may be narrower)
 };
 inline size_t topk_blocks_smem(int n_blocks, int refine_K) { return sizeof(float) * (size_t)(2 * n_blocks + refine_K); }
-constexpr int kTopkBlocksThreads = 1024;
-static __global__ void __launch_bounds__(kTopkBlocksThreads, 1) topk_blocks_kernel(const float* __restrict__ logits, const __half* __restrict__ logits16, int ld, int V, int kk,
+template <int THREADS>
+static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) topk_blocks_kernel(const float* __restrict__ logits, const __half* __restrict__ logits16, int ld, int V, int kk,
                                                                            TopkOut out, int normalise, LogitBlocks bl, TopkRefine rf, const __grid_constant__ SelectArgs sel) {
-  constexpr int THREADS = kTopkBlocksThreads;
   tc::pdl_launch_dependents();
   tc::pdl_wait();
   extern __shared__ float dyn[];
@@ -1126,24 +1126,25 @@ static __global__ void __launch_bounds__(kTopkBlocksThreads, 1) topk_blocks_kern
     tau -= 2.0f * (rf.eps_coef * sqrtf(tot) + 1e-5f);
     if (zh) tau -= 2.0f * 4.9e-4f * fmaxf(fabsf(rmax), fabsf(tau));
   }
-  // each warp tests 32 blocks at a time and reads those that reach the threshold, two at a time
+  // each warp tests 32 blocks at a time and reads those that reach the threshold
   for (int b0 = warp * 32; b0 < bl.n; b0 += THREADS) {
     unsigned hit = __ballot_sync(0xffffffffu, b0 + lane < bl.n && s_m[b0 + lane] >= tau);
     while (hit) {
-      int i[2];
+      const int b = b0 + __ffs(hit) - 1;
+      hit &= hit - 1;
+      const int in_tile = (b & 3) * bl.part, c0 = (b >> 2) * bl.tile + in_tile;
+      const int end = c0 + (bl.tile - in_tile < bl.part ? bl.tile - in_tile : bl.part);
       float v[2];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
-        const int b = hit ? b0 + __ffs(hit) - 1 : -1;
-        hit &= hit - 1;
-        i[u] = b >= 0 ? b * kBlockCols + lane : V;
-        v[u] = i[u] < V ? (zh ? __half2float(zh[i[u]]) : z[i[u]]) : -INFINITY;
+        const int i = c0 + lane + 32 * u;
+        v[u] = i < end && i < V ? (zh ? __half2float(zh[i]) : z[i]) : -INFINITY;
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u)
-        if (i[u] < V && v[u] >= tau) {
+        if (v[u] >= tau && v[u] > -INFINITY) {
           const int pos = atomicAdd(&sh.count, 1);
-          if (pos < kTopkCap) { sh.cv[pos] = v[u]; sh.ci[pos] = i[u]; }
+          if (pos < kTopkCap) { sh.cv[pos] = v[u]; sh.ci[pos] = c0 + lane + 32 * u; }
         }
     }
   }
@@ -1279,6 +1280,156 @@ static __global__ void __launch_bounds__(256) ensemble_combine_kernel(EnsembleRo
     o[j] = (mode == 0) ? logf((float)acc) : (float)acc;
   }
   (void)inv_n;
+}
+
+// Ensembles: combination, log-softmax and top-kk of a row in one pass over the members' logits.  A member's maximum and
+// log-sum come from its block statistics if the GEMM left them (otherwise from a sweep of its own); the pass then forms the
+// combined value of every class -- mean of the probabilities (mode 0) or of the log-probabilities (mode 1), accumulated
+// in double like the reference's loop -- keeps the maximum of every 128 classes and the sum, and only the blocks that reach
+// the threshold are formed again to list their candidates.  The combined row itself is never written, and the logits are
+// read once: (M + 1/16) x V x 4 bytes a row instead of (2 M + 2) x V x 4.  M = 4 at up to 384 rows, 30k classes: the two
+// kernels took 224 us per step.
+// THREADS = 1024 for rows that leave SMs empty.  grid = rows, dynamic smem = ceil(V / 128) floats.
+template <int THREADS>
+static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1) ensemble_topk_kernel(EnsembleRows er, int ld, int V, int kk, int mode, TopkOut out, LogitBlocks bl,
+                                                                                             long long bl_member, float* __restrict__ combined, const __grid_constant__ SelectArgs sel) {
+  tc::pdl_launch_dependents();
+  tc::pdl_wait();
+  constexpr int kWarps = THREADS / 32;
+  extern __shared__ float s_bm[];            // [ceil(V / 128)] block maxima of the combined values
+  __shared__ __align__(16) unsigned char s_union[sizeof(TopkSmem)];
+  TopkShared& sh = *reinterpret_cast<TopkShared*>(s_union);
+  __shared__ float s_m[8][kWarps], s_s[8][kWarps];
+  __shared__ float s_c[8];                   // maximum + log-sum of a member
+  __shared__ float s_tmax[THREADS], s_tau, s_eos[2];
+  const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int m = 0; m < er.n; ++m) {
+    float mx = -INFINITY, sum = 0.f;
+    auto join = [&](float om, float os) {
+      const float nm = fmaxf(mx, om);
+      sum = (nm == -INFINITY) ? 0.f : sum * __expf(mx - nm) + os * __expf(om - nm);
+      mx = nm;
+    };
+    if (bl.n > 0) {
+      const float* bm = bl.max + m * bl_member + (size_t)r * bl.ld;
+      const float* bs = bl.sum + m * bl_member + (size_t)r * bl.ld;
+      for (int b = tid; b < bl.n; b += THREADS) join(bm[b], bs[b]);
+    } else {
+      const float* z = er.logits[m] + (size_t)r * ld;
+      for (int i = tid * 4; i < V; i += THREADS * 4) {
+        const float4 q = *reinterpret_cast<const float4*>(z + i);     // (rows are padded)
+        const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) if (i + u < V) join(v[u], 1.f);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float om = __shfl_xor_sync(0xffffffffu, mx, o), os = __shfl_xor_sync(0xffffffffu, sum, o);
+      join(om, os);
+    }
+    if (lane == 0) { s_m[m][warp] = mx; s_s[m][warp] = sum; }
+  }
+  if (tid == 0) sh.count = 0;
+  __syncthreads();
+  if (tid < er.n) {
+    float mx = s_m[tid][0], sum = s_s[tid][0];
+    for (int w = 1; w < kWarps; ++w) {
+      const float om = s_m[tid][w], os = s_s[tid][w];
+      const float nm = fmaxf(mx, om);
+      sum = (nm == -INFINITY) ? 0.f : sum * __expf(mx - nm) + os * __expf(om - nm);
+      mx = nm;
+    }
+    s_c[tid] = mx + logf(sum);
+  }
+  __syncthreads();
+  // four classes from i on; what is compared is the mean probability (mode 0) or the mean log-probability (mode 1)
+  const double n_members = er.n;
+  const bool pow2 = (er.n & (er.n - 1)) == 0;        // then the division is an exact product
+  const double inv_members = 1.0 / n_members;
+  auto combine4 = [&](int i) {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int m0 = 0; m0 < er.n; m0 += 4) {
+      float4 q[4];      // four members' loads in flight
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (m0 + m < er.n) q[m] = *reinterpret_cast<const float4*>(er.logits[m0 + m] + (size_t)r * ld + i);
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+        if (m0 + m < er.n) {
+          const float c = s_c[m0 + m];
+          const float l[4] = {q[m].x - c, q[m].y - c, q[m].z - c, q[m].w - c};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) a[u] += mode == 0 ? (double)expf(l[u]) : (double)l[u];
+        }
+    }
+    if (pow2) return make_float4((float)(a[0] * inv_members), (float)(a[1] * inv_members), (float)(a[2] * inv_members), (float)(a[3] * inv_members));
+    return make_float4((float)(a[0] / n_members), (float)(a[1] / n_members), (float)(a[2] / n_members), (float)(a[3] / n_members));
+  };
+  float tmax = -INFINITY, psum = 0.f;
+  for (int b = warp; b * 128 < V; b += kWarps) {
+    const int i = b * 128 + lane * 4;
+    float bm = -INFINITY;
+    if (i < V) {
+      const float4 w = combine4(i);
+      const float v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u < V) {
+          bm = fmaxf(bm, v[u]);
+          psum += v[u];
+          if (i + u == kEos) s_eos[kEos] = mode == 0 ? logf(v[u]) : v[u];
+        }
+    }
+    tmax = fmaxf(tmax, bm);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+    if (lane == 0) s_bm[b] = bm;
+  }
+  // threshold: the kk-th largest of 32 maxima over disjoint classes (kk <= 32), reached by kk classes
+  s_tmax[tid] = tmax;
+  __syncthreads();
+  if (warp == 0) {
+    float g = -INFINITY;
+    for (int w = 0; w < kWarps; ++w) g = fmaxf(g, s_tmax[w * 32 + lane]);
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const float o = __shfl_sync(0xffffffffu, g, j);
+      rank += (o > g || (o == g && j < lane)) ? 1 : 0;
+    }
+    if (rank == kk - 1) s_tau = g;
+  }
+  __syncthreads();
+  // (probabilities that differ may have the same logarithm, and then the lower index is the better one)
+  const float tau = mode == 0 ? s_tau * (1.0f - 1e-6f) : s_tau;
+  for (int b = warp; b * 128 < V; b += kWarps) {
+    if (s_bm[b] < tau) continue;
+    const int i = b * 128 + lane * 4;
+    if (i >= V) continue;
+    const float4 w = combine4(i);
+    const float v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u < V && v[u] >= tau) {
+        const int pos = atomicAdd(&sh.count, 1);
+        if (pos < kTopkCap) { sh.cv[pos] = mode == 0 ? logf(v[u]) : v[u]; sh.ci[pos] = i + u; }
+      }
+  }
+  __syncthreads();
+  const float* z = s_eos;     // (of the row, only EOS is asked for by index ...)
+  if (sh.count > kTopkCap) {  // ... unless more classes than the list holds reach the threshold: then it is swept
+    float* row = combined + (size_t)r * ld;
+    for (int i = tid * 4; i < V; i += THREADS * 4) {
+      const float4 w = combine4(i);
+      *reinterpret_cast<float4*>(row + i) = mode == 0 ? make_float4(logf(w.x), logf(w.y), logf(w.z), logf(w.w)) : w;
+    }
+    __threadfence_block();
+    __syncthreads();
+    z = row;
+  }
+  topk_finish<THREADS>(sh, r, psum, 0.f, z, nullptr, V, kk, out, mode == 0 ? 1 : 0, TopkRefine{}, nullptr);
+  select_if_last<THREADS>(sel, out, r, s_union);
 }
 
 // ---------------------------------------------------------------------------------------
