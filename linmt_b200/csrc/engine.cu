@@ -403,7 +403,6 @@ int Engine::run_encoder(int n, int Smax) {
 int Engine::run_decoder_step(int mi, int t, int rows) {
   DevModel& m = models_[mi];
   DevState& s = states_[mi];
-  const int n_act = rows / k;
   // 1. reorder states through the parents, look up the new tokens' embeddings
   {
     PrepArrays pa{};

@@ -237,6 +237,20 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) attent
                                  int32_t* __restrict__ rec_lo, int32_t* __restrict__ rec_vit, tc::Planes ctx_planes, int nt,
                                  int rec_win, int ens, AttTrace at, AttFold fold) {
   tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
+  if (THREADS > 256) {
+    // Few rows: the weights of a step have displaced the encoder's states from L2.  While the projection runs, the k CTAs
+    // of a sentence ask for them again (a hint; nothing is read here, so the length may still be an earlier step's).
+    const int sent = blockIdx.x / k, S = src_len[sent];
+    const char* h0 = reinterpret_cast<const char*>(hs + (size_t)sent * hs_sent * Hp);
+    const char* c0 = fold.cs ? reinterpret_cast<const char*>(fold.cs + (size_t)sent * hs_sent * Hp) : nullptr;
+    const int lines = Hp / 32;
+    for (int i = (blockIdx.x - sent * k) * THREADS + threadIdx.x; i < S * lines; i += k * THREADS) {
+      const int pos = i / lines;
+      const size_t off = (size_t)pos * hs_pos * Hp * 4 + (size_t)(i - pos * lines) * 128;
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(h0 + off));
+      if (c0) asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + off));
+    }
+  }
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
   extern __shared__ float sm[];
   constexpr int kGroups = THREADS / 256;    // of window positions, in the context sum
@@ -307,7 +321,8 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) attent
     for (int w = lane; w < W; w += 32) {
       float a = e[w];
       if (mode == 0) {
-        const float tmp = expf((-1 * powf(pt - (float)(lo + w), 2.0f)) / (2 * sigma_sq));
+        const float d = pt - (float)(lo + w);
+        const float tmp = expf(-(d * d) / (2 * sigma_sq));
         if (0 != sum) a = (a / sum) * tmp;
       } else if (0 != sum) a = a / sum;
       e[w] = a;
@@ -475,7 +490,7 @@ struct SelectArgs {
   float penalty, diversity;
   TraceDev tr;
 };
-constexpr int kSelectSmem = kMaxBeam * (kMaxBeam + 1) * 20;   // its shared memory: candidates of the widest beam
+constexpr int kSelectSmem = kMaxBeam * (kMaxBeam + 1) * 16;   // its shared memory: candidates of the widest beam
 // Candidates of the whole sentence in shared memory, then the walk over them in order, 32 candidates at a time.
 template <int THREADS>
 __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const TopkOut& cand, int sent, int T, int osent, int nf0, unsigned char* smraw) {
@@ -503,11 +518,8 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     }
     return;
   }
-  const int ncap = k * kk;
-  unsigned long long* key = reinterpret_cast<unsigned long long*>(smraw);   // sortable (score, beam, vocab)
-  float* ss = reinterpret_cast<float*>(key + ncap);   // score, beam and vocabulary id in sorted order
-  int* sb = reinterpret_cast<int*>(ss + ncap);
-  int* sv = sb + ncap;
+  unsigned long long* key = reinterpret_cast<unsigned long long*>(smraw);   // sortable (score, beam, vocabulary id)
+  unsigned long long* order = key + k * kk;                                 // the same in order
   const int cols = (t == 0) ? 1 : k;
   const int n = cols * kk;
   for (int c = tid; c < n; c += THREADS) {
@@ -516,7 +528,6 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     const int v = __ldcg(cand.idx + (size_t)(r0 + b) * kk + q);
     const float rank_penalty = (float)(q + 1) * a.diversity;
     const float sc = (lp + bs.score[r0 + b]) - rank_penalty;
-    ss[c] = sc; sb[c] = b; sv[c] = v;   // overwritten by the ranking below; keeps every entry valid even for NaN scores
     // one 64-bit key, larger = earlier: score descending, then beam ascending, then vocabulary id ascending
     const unsigned int fb = __float_as_uint(sc);
     const unsigned int ord = (fb & 0x80000000u) ? ~fb : (fb | 0x80000000u);
@@ -528,24 +539,24 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     }
   }
   __syncthreads();
-  // (k <= 31: at most 992 candidates, i.e. at most four per thread of a block of 256)
-  constexpr int kPer = (kMaxBeam * (kMaxBeam + 1) + THREADS - 1) / THREADS;
-  int pos[kPer]; float ksc[kPer]; int kb[kPer], kv[kPer];
-#pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int c = tid + i * THREADS;
-    if (c < n) {
-      const unsigned long long kc = key[c];
-      int p = 0;
+  // a thread counts the candidates before its own; four of a large block share one (a warp per candidate with ballots
+  // was slower: 156 candidates, 7000 clocks in a block of 1024 and 20000 in one of 256)
+  const int share = THREADS > 256 && n <= THREADS / 4 ? 4 : 1;
+  for (int c0 = 0; c0 < n; c0 += THREADS / share) {
+    const int c = c0 + tid / share;
+    const unsigned long long kc = c < n ? key[c] : 0ull;
+    int p = 0;
 #pragma unroll 4
-      for (int d = 0; d < n; ++d) p += (key[d] > kc) ? 1 : 0;
-      pos[i] = p; ksc[i] = ss[c]; kb[i] = sb[c]; kv[i] = sv[c];
+    for (int d = tid & (share - 1); d < n; d += share) {
+      const unsigned long long kd = key[d];
+      p += (kd > kc || (kd == kc && d < c)) ? 1 : 0;
     }
+    if (share > 1) {
+      p += __shfl_xor_sync(0xffffffffu, p, 1);
+      p += __shfl_xor_sync(0xffffffffu, p, 2);
+    }
+    if (c < n && (tid & (share - 1)) == 0) order[p] = kc;
   }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < kPer; ++i)
-    if (tid + i * THREADS < n) { ss[pos[i]] = ksc[i]; sb[pos[i]] = kb[i]; sv[pos[i]] = kv[i]; }
   __syncthreads();
   __shared__ int s_ntok[kMaxBeam + 1], s_npar[kMaxBeam + 1];
   __shared__ float s_nscore[kMaxBeam + 1];
@@ -554,18 +565,21 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     int ns = 0, nf = nf0;
     for (int p0 = 0; p0 < n && ns < k; p0 += 32) {
       const int p = p0 + lane;
-      const int v = p < n ? sv[p] : -1;
+      const unsigned long long ko = p < n ? order[p] : 0ull;
+      const unsigned int low = 0xFFFFFFFFu - (unsigned int)ko, ord = (unsigned int)(ko >> 32);
+      const int v = p < n && (low & 0xFFFFFFu) != 0xFFFFFFu ? (int)(low & 0xFFFFFFu) : -1, b = (int)(low >> 24);
+      const float sc = __uint_as_float((ord & 0x80000000u) ? (ord & 0x7FFFFFFFu) : ~ord);
       const unsigned take = __ballot_sync(0xffffffffu, v >= 0 && v != kStart && v != kEos);
       const unsigned below = (1u << lane) - 1u;
       const int slot = ns + __popc(take & below);            // free slots used before this candidate
       const bool eos = v == kEos && slot < k;
       const unsigned ends = __ballot_sync(0xffffffffu, eos);
-      if (((take >> lane) & 1u) && slot < k) { s_ntok[slot] = v; s_npar[slot] = sb[p]; s_nscore[slot] = ss[p] + a.penalty; }
+      if (((take >> lane) & 1u) && slot < k) { s_ntok[slot] = v; s_npar[slot] = b; s_nscore[slot] = sc + a.penalty; }
       const int f = nf + __popc(ends & below);
       if (eos && f < bs.fin_cap) {
         bs.fin_t[(size_t)sent * bs.fin_cap + f] = t;
-        bs.fin_b[(size_t)sent * bs.fin_cap + f] = sb[p];
-        bs.fin_score[(size_t)sent * bs.fin_cap + f] = ss[p] + a.penalty;
+        bs.fin_b[(size_t)sent * bs.fin_cap + f] = b;
+        bs.fin_score[(size_t)sent * bs.fin_cap + f] = sc + a.penalty;
       }
       ns += __popc(take);
       nf += __popc(ends);
@@ -629,13 +643,18 @@ __device__ __forceinline__ void select_if_last(const SelectArgs& a, const TopkOu
   // what the selection reads first is on its way while the counter answers
   const int T = a.steps[sent], osent = a.orig[sent], nf0 = a.bs.fin_n[sent];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();       // this row's candidates (all threads', by the barrier) before the counter
-    s_last = atomicAdd(&a.done[sent], 1) == a.k - 1;
-    if (s_last) { a.done[sent] = 0; __threadfence(); }
+  bool last = true;        // (a greedy sentence has one row)
+  if (a.k > 1) {
+    if (threadIdx.x == 0) {
+      int before;            // releases this row's candidates (all threads', by the barrier) and acquires the other rows'
+      asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(before) : "l"(a.done + sent) : "memory");
+      s_last = before == a.k - 1;
+      if (s_last) a.done[sent] = 0;
+    }
+    __syncthreads();
+    last = s_last;
   }
-  __syncthreads();
-  if (s_last) beam_select_block<THREADS>(a, cand, sent, T, osent, nf0, smraw);
+  if (last) beam_select_block<THREADS>(a, cand, sent, T, osent, nf0, smraw);
 }
 
 // Pass 1 finds the row maximum and, from the 256 per-thread maxima, a threshold that at least
@@ -653,8 +672,9 @@ struct TopkShared {
   float co[kTopkCap];   // ... and in vocabulary order
   float red[32];
   int redi[32];
-  int count;
-  float lse, sum, eos, eos_delta;
+  float part[32];       // the warps' shares of the sum
+  int count, n_blocks;
+  float lse, eos, eos_delta;
 };
 // (once a row's results are written, the selection has the memory)
 union TopkSmem {
@@ -666,22 +686,9 @@ __device__ __forceinline__ void topk_finish(TopkShared& sh, int r, float ssum, f
                                             int V, int kk, const TopkOut& out, int normalise, const TopkRefine& rf, const float* s_a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   auto zat = [&](int i) { return zh ? __half2float(zh[i]) : z[i]; };
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ssum += __shfl_xor_sync(0xffffffffu, ssum, o);
-  if (lane == 0) sh.red[warp] = ssum;
-  __syncthreads();
-  if (warp == 0) {
-    const float bs = warp_sum(lane < THREADS / 32 ? sh.red[lane] : 0.f);
-    if (lane == 0) {
-      sh.sum = bs;
-      if (!rf.a0) sh.lse = normalise ? logf(bs) : -rmax;   // normalise = 0: the row already holds log-probabilities
-    }
-    if (lane == 0 && !rf.a0) {
-      if (out.eos_logp) out.eos_logp[r] = (zat(kEos) - rmax) - sh.lse;
-      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = sh.lse; }
-    }
-  }
-  __syncthreads();
+  ssum = warp_sum(ssum);
+  if (lane == 0) sh.part[warp] = ssum;
+  const float z_eos = !rf.a0 && warp == 0 ? zat(kEos) : 0.f;
   int n = sh.count;
   if (rf.a0 && n > kTopkCap) {
     // More elements than the buffer holds reach the widened threshold (a nearly flat row): pick the kk best
@@ -759,31 +766,77 @@ __device__ __forceinline__ void topk_finish(TopkShared& sh, int r, float ssum, f
         else { sh.eos = zv; sh.eos_delta = delta; }
       }
     }
-    __syncthreads();
-    // the correction is summed in vocabulary order, so the result does not depend on the order in which
-    // the candidates happened to enter the buffer
-    for (int c = tid; c < nc; c += THREADS) {
+  }
+  __syncthreads();
+  // The rest is a warp's work while the candidates are no more than its lanes (13 to 17 at a beam of 12): in registers,
+  // without a barrier.  The correction is summed in vocabulary order, so the result does not depend on the order in
+  // which the candidates happened to enter the buffer.
+  if (n <= 32) {
+    if (warp != 0) return;
+    const bool in = lane < n;
+    const float v = in ? sh.cv[lane] : -INFINITY;
+    const int i = in ? sh.ci[lane] : 0x7fffffff;
+    float sum = warp_sum(lane < THREADS / 32 ? sh.part[lane] : 0.f);
+    int pos = 0, rank = 0;
+#pragma unroll 4
+    for (int d = 0; d < n; ++d) {
+      const float ov = __shfl_sync(0xffffffffu, v, d);
+      const int oi = __shfl_sync(0xffffffffu, i, d);
+      pos += oi < i ? 1 : 0;
+      rank += better(ov, oi, v, i) ? 1 : 0;
+    }
+    float eos = z_eos;
+    if (rf.a0) {
+      if (in) sh.co[pos] = sh.cd[lane];
+      __syncwarp();
+      float corr = warp_sum(in ? sh.co[lane] : 0.f);
+      if (!__any_sync(0xffffffffu, in && i == kEos)) corr += sh.eos_delta;
+      if (sum + corr > 0.f) sum += corr;
+      eos = sh.eos;
+    }
+    const float lse = normalise ? logf(sum) : -rmax;   // normalise = 0: the row already holds log-probabilities
+    if (in && rank < kk) {
+      out.idx[(size_t)r * kk + rank] = i;
+      out.logp[(size_t)r * kk + rank] = (v - rmax) - lse;
+    }
+    if (n + lane < kk) {       // fewer than kk elements in the row
+      out.idx[(size_t)r * kk + n + lane] = -1;
+      out.logp[(size_t)r * kk + n + lane] = -INFINITY;
+    }
+    if (lane == 0) {
+      if (out.eos_logp) out.eos_logp[r] = (eos - rmax) - lse;
+      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = lse; }
+    }
+    return;
+  }
+  if (rf.a0 && n <= kTopkCap) {
+    for (int c = tid; c < n; c += THREADS) {
       const int i = sh.ci[c];
       int pos = 0;
-      for (int d = 0; d < nc; ++d) pos += (sh.ci[d] < i) ? 1 : 0;
+      for (int d = 0; d < n; ++d) pos += (sh.ci[d] < i) ? 1 : 0;
       sh.co[pos] = sh.cd[c];
     }
     __syncthreads();
-    if (warp == 0) {
+  }
+  if (warp == 0) {
+    float sum = warp_sum(lane < THREADS / 32 ? sh.part[lane] : 0.f);
+    float eos = z_eos;
+    if (rf.a0) {
       float corr = 0.f;
       bool eos_listed = false;
-      for (int c = lane; c < nc; c += 32) { corr += sh.co[c]; eos_listed = eos_listed || (sh.ci[c] == kEos); }
+      for (int c = lane; c < n; c += 32) { corr += sh.co[c]; eos_listed = eos_listed || (sh.ci[c] == kEos); }
       corr = warp_sum(corr);
       if (!__any_sync(0xffffffffu, eos_listed)) corr += sh.eos_delta;
-      if (lane == 0) {
-      const float bs = sh.sum + corr;
-      sh.lse = normalise ? logf(bs > 0.f ? bs : sh.sum) : -rmax;
-      if (out.eos_logp) out.eos_logp[r] = (sh.eos - rmax) - sh.lse;
-      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = sh.lse; }
-      }
+      if (sum + corr > 0.f) sum += corr;
+      eos = sh.eos;
     }
-    __syncthreads();
+    if (lane == 0) {
+      sh.lse = normalise ? logf(sum) : -rmax;
+      if (out.eos_logp) out.eos_logp[r] = (eos - rmax) - sh.lse;
+      if (out.row_stats) { out.row_stats[2 * r] = rmax; out.row_stats[2 * r + 1] = sh.lse; }
+    }
   }
+  __syncthreads();
   const float rlse = sh.lse;
   if (n <= kTopkCap) {
     // exact ranking of the candidates: value descending, index ascending
@@ -1022,6 +1075,7 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
     for (int j = V4 + tid; j < V; j += 256) visit(z[j], j);
     }
   }
+  __syncthreads();
   topk_finish<256>(sh, r, ssum, rmax, z, zh, V, kk, out, normalise, rf, s_a);
   select_if_last<256>(sel, out, r, s_union);
 }
@@ -1051,10 +1105,17 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) topk_b
   __shared__ __align__(16) unsigned char s_union[sizeof(TopkSmem)];
   TopkShared& sh = *reinterpret_cast<TopkShared*>(s_union);
   __shared__ float s_tmax[THREADS];
-  __shared__ float s_tau, s_max;
+  __shared__ float s_tau, s_max, s_eps;
   const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float* z = logits ? logits + (size_t)r * ld : nullptr;
   const __half* zh = logits16 ? logits16 + (size_t)r * ld : nullptr;
+  // (the activations are requested before the blocks are waited for; K is a multiple of 64)
+  uint2 q0 = make_uint2(0u, 0u), q1 = make_uint2(0u, 0u);
+  auto act_load = [&](int j) {
+    q0 = *reinterpret_cast<const uint2*>(rf.a0 + (size_t)r * rf.lda + j);
+    q1 = *reinterpret_cast<const uint2*>(rf.a1 + (size_t)r * rf.lda + j);
+  };
+  if (rf.a0 && tid * 4 < rf.K) act_load(tid * 4);
   float m = -INFINITY;
   for (int b = tid; b < bl.n; b += THREADS) {
     const float v = bl.max[(size_t)r * bl.ld + b];
@@ -1062,18 +1123,21 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) topk_b
     s_m[b] = v;
     m = fmaxf(m, v);
   }
-  float ss = 0.f;
-  if (rf.a0)
-    for (int j = tid; j < rf.K; j += THREADS) {
-      const float a = __half2float(rf.a0[(size_t)r * rf.lda + j]) + __half2float(rf.a1[(size_t)r * rf.lda + j]) * kPairInv;
-      s_a[j] = a;
-      ss = fmaf(a, a, ss);
-    }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if (lane == 0) sh.red[warp] = ss;
   s_tmax[tid] = m;
-  if (tid == 0) sh.count = 0;
+  if (tid == 0) { sh.count = 0; sh.n_blocks = 0; s_tau = -INFINITY; }
+  if (rf.a0) {
+    float ss = 0.f;
+    for (int j = tid * 4; j < rf.K; j += THREADS * 4) {
+      if (j >= THREADS * 4) act_load(j);
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&q0.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&q0.y));
+      const float2 g0 = __half22float2(*reinterpret_cast<const __half2*>(&q1.x)), g1 = __half22float2(*reinterpret_cast<const __half2*>(&q1.y));
+      const float4 a = make_float4(f0.x + g0.x * kPairInv, f0.y + g0.y * kPairInv, f1.x + g1.x * kPairInv, f1.y + g1.y * kPairInv);
+      s_a[j] = a.x; s_a[j + 1] = a.y; s_a[j + 2] = a.z; s_a[j + 3] = a.w;
+      ss = fmaf(a.x, a.x, ss); ss = fmaf(a.y, a.y, ss); ss = fmaf(a.z, a.z, ss); ss = fmaf(a.w, a.w, ss);
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) sh.red[warp] = ss;
+  }
   __syncthreads();
   if (warp == 0) {
     // threshold from 32 group maxima, as in softmax_topk_kernel (kk <= 32)
@@ -1090,65 +1154,71 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) topk_b
       rank += (o > g || (o == g && j < lane)) ? 1 : 0;
     }
     if (rank == kk - 1) s_tau = g;
-    if (lane == 0) s_max = bm;
+    const float tot = rf.a0 ? warp_sum(lane < THREADS / 32 ? sh.red[lane] : 0.f) : 0.f;
+    if (lane == 0) { s_max = bm; s_eps = rf.a0 ? 2.0f * (rf.eps_coef * sqrtf(tot) + 1e-5f) : 0.f; }
   }
   __syncthreads();
-  const float rmax = s_max;
-  // the sum, and the blocks that reach the threshold
-  const float tau0 = s_tau;
+  const float rmax = s_max, tau0 = s_tau, eps = s_eps;
+  // refinement: every logit is within eps of its accurate value (see softmax_topk_kernel)
+  auto lowered = [&](float t) {
+    if (!rf.a0) return t;
+    t -= eps;
+    return zh ? t - 2.0f * 4.9e-4f * fmaxf(fabsf(rmax), fabsf(t)) : t;
+  };
+  // the sum, and the list of the blocks that reach the (lowered) threshold: sh.cd their maxima, sh.co their numbers
+  float* lv = sh.cd;
+  int* lb = reinterpret_cast<int*>(sh.co);
   float ssum = 0.f;
+  float tau = lowered(tau0);
   for (int b = tid; b < bl.n; b += THREADS) {
     const float v = s_m[b];
     if (v > -INFINITY) ssum = fmaf(s_q[b], __expf(v - rmax), ssum);
-    if (v >= tau0) {
-      const int pos = atomicAdd(&sh.count, 1);
-      if (pos < kTopkCap) sh.cv[pos] = v;
+    if (v >= tau) {
+      const int pos = atomicAdd(&sh.n_blocks, 1);
+      if (pos < kTopkCap) { lv[pos] = v; lb[pos] = b; }
     }
   }
   __syncthreads();
-  {
-    // tighter: the kk-th largest of those maxima is still reached by kk elements
-    const int m2 = sh.count;
-    if (m2 <= kTopkCap)
-      for (int c = tid; c < m2; c += THREADS) {
-        const float v = sh.cv[c];
-        int rank = 0;
-        for (int d = 0; d < m2; ++d) rank += (sh.cv[d] > v || (sh.cv[d] == v && d < c)) ? 1 : 0;
-        if (rank == kk - 1) s_tau = v;
+  const int n_list = sh.n_blocks;
+  // tighter: the kk-th largest of those maxima is still reached by kk elements (a warp ranks a block)
+  if (n_list <= kTopkCap)
+    for (int c = warp; c < n_list; c += THREADS / 32) {
+      const float v = lv[c];
+      int rank = 0;
+      for (int d0 = 0; d0 < n_list; d0 += 32) {
+        const int d = d0 + lane;
+        const float o = d < n_list ? lv[d] : -INFINITY;
+        rank += __popc(__ballot_sync(0xffffffffu, d < n_list && (o > v || (o == v && d < c))));
       }
-  }
-  __syncthreads();
-  if (tid == 0) sh.count = 0;
-  __syncthreads();
-  float tau = s_tau;
-  if (rf.a0) {     // every logit is within eps of its accurate value (see softmax_topk_kernel)
-    const float tot = warp_sum(lane < THREADS / 32 ? sh.red[lane] : 0.f);
-    tau -= 2.0f * (rf.eps_coef * sqrtf(tot) + 1e-5f);
-    if (zh) tau -= 2.0f * 4.9e-4f * fmaxf(fabsf(rmax), fabsf(tau));
-  }
-  // each warp tests 32 blocks at a time and reads those that reach the threshold
-  for (int b0 = warp * 32; b0 < bl.n; b0 += THREADS) {
-    unsigned hit = __ballot_sync(0xffffffffu, b0 + lane < bl.n && s_m[b0 + lane] >= tau);
-    while (hit) {
-      const int b = b0 + __ffs(hit) - 1;
-      hit &= hit - 1;
-      const int in_tile = (b & 3) * bl.part, c0 = (b >> 2) * bl.tile + in_tile;
-      const int end = c0 + (bl.tile - in_tile < bl.part ? bl.tile - in_tile : bl.part);
-      float v[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int i = c0 + lane + 32 * u;
-        v[u] = i < end && i < V ? (zh ? __half2float(zh[i]) : z[i]) : -INFINITY;
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-        if (v[u] >= tau && v[u] > -INFINITY) {
-          const int pos = atomicAdd(&sh.count, 1);
-          if (pos < kTopkCap) { sh.cv[pos] = v[u]; sh.ci[pos] = c0 + lane + 32 * u; }
-        }
+      if (rank == kk - 1 && lane == 0) s_tau = v;
     }
+  __syncthreads();
+  tau = lowered(s_tau);
+  // a warp reads a block
+  auto read_block = [&](int b) {
+    const int in_tile = (b & 3) * bl.part, c0 = (b >> 2) * bl.tile + in_tile;
+    const int end = c0 + (bl.tile - in_tile < bl.part ? bl.tile - in_tile : bl.part);
+    float v[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = c0 + lane + 32 * u;
+      v[u] = i < end && i < V ? (zh ? __half2float(zh[i]) : z[i]) : -INFINITY;
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (v[u] >= tau && v[u] > -INFINITY) {
+        const int pos = atomicAdd(&sh.count, 1);
+        if (pos < kTopkCap) { sh.cv[pos] = v[u]; sh.ci[pos] = c0 + lane + 32 * u; }
+      }
+  };
+  if (n_list <= kTopkCap) {
+    for (int c = warp; c < n_list; c += THREADS / 32)
+      if (lv[c] >= tau) read_block(lb[c]);
+  } else {
+    for (int b = warp; b < bl.n; b += THREADS / 32)
+      if (s_m[b] >= tau) read_block(b);
   }
-  __syncthreads();     // (sh.red has been read by every warp)
+  __syncthreads();     // (the list has been read by every warp)
   topk_finish<THREADS>(sh, r, ssum, rmax, z, zh, V, kk, out, normalise, rf, s_a);
   select_if_last<THREADS>(sel, out, r, s_union);
 }
