@@ -289,6 +289,23 @@ __device__ __forceinline__ void split_store4(const Planes& pl, int nt, size_t id
     }
   }
 }
+__device__ __forceinline__ void split_store2(const Planes& pl, int nt, size_t idx, float x0, float x1) {
+  if (pl.fmt == 1) {
+    unsigned short a0, a1, b0, b1;
+    f16_pair(x0, a0, a1);
+    f16_pair(x1, b0, b1);
+    *reinterpret_cast<uint32_t*>(pl.p[0] + idx) = (uint32_t)a0 | ((uint32_t)b0 << 16);
+    *reinterpret_cast<uint32_t*>(pl.p[1] + idx) = (uint32_t)a1 | ((uint32_t)b1 << 16);
+    return;
+  }
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+    if (t < nt) {
+      const __nv_bfloat162 b(__float2bfloat16(x0), __float2bfloat16(x1));
+      *reinterpret_cast<__nv_bfloat162*>(pl.p[t] + idx) = b;
+      x0 -= __bfloat162float(b.x); x1 -= __bfloat162float(b.y);
+    }
+}
 
 // 2^x (2 ulp), results below the normal range to zero
 __device__ __forceinline__ float exp2f_fast(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }

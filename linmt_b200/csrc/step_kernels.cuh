@@ -167,27 +167,8 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 // Block-wide sum in a fixed order (deterministic).
-__device__ __forceinline__ float block_sum(float v, float* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  const int nw = blockDim.x >> 5;
-  if (nw > 8) {
-    float t = l < nw ? red[l] : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    return t;
-  }
-  float t = 0.f;
-  for (int i = 0; i < nw; ++i) t += red[i];
-  return t;
-}
-
 // ---------------------------------------------------------------------------------------
-// Attention for one decoder row (AttentionNode::ForwardProp, src/layer_attention.h:243-483,
+// Attention of a step (AttentionNode::ForwardProp, src/layer_attention.h:243-483,
 // kernels k12-k20: Sgemm m=1, SigmoidKernel, AlignmentPosKernel, LowerUpperKernel,
 // CreateIndicesKernel, LoadInHSKernel, ElemReduceKernelLarge, AlignmentReductionKernel,
 // CreateCTKernel).
@@ -201,12 +182,6 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 //   (rec_win = max_src, rec_lo = 0), the first member writes it, the others add to it in member order,
 //   and the last one takes the vote: the position of the largest summed score, the search starting from
 //   "none, 0" (EnsembleFactory::EnsemblesModels, src/decoder.h:1934-1964).
-// grid = rows, block = THREADS, dynamic smem = attention_smem<THREADS>(win).  The kernel is a chain of L2 round trips, not
-// of bytes.  (Three variations were tried and measured no faster: the window's states kept in shared memory
-// between the score sweep and the context sweep -- 86 KB per CTA costs the occupancy the halved traffic buys;
-// one CTA per group of beams of a sentence reading every state row once for all of them -- a quarter of the
-// CTAs, the same chain of round trips in each; and loads issued in batches of eight ahead of the arithmetic --
-// the registers cost more occupancy than the batching hides latency.)
 // Optional record of the attention centre p_t of every row of a forward (local attention): the parity tests
 // use it to tell a window that was cut on the other side of an integer apart from an error.
 struct AttTrace {
@@ -225,26 +200,36 @@ struct AttFold {
   const float* add; int ld_add;   // element (row, j) at add[row * ld_add + j]
   const float* bias;    // [Hp]
 };
-// THREADS = 256: six CTAs per SM, so that the 888 resident CTAs hold the 768 rows of a full step in one wave (at five, 28
-// rows ran as a second wave).  THREADS = 1024 for a step whose rows leave SMs empty: one window position per warp and the
-// context in four groups of positions instead of chains of three and 21 dependent rounds of loads (one sentence: 18.1 us
-// per step with 256 threads).
-template <int THREADS>
-static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) attention_kernel(const float* __restrict__ proj, int ldp, const float* __restrict__ u_alt, int ldu,
+// A CTA serves G beams of a sentence (a group): their windows overlap almost everywhere, so an encoder state is read once
+// for all of them -- for the scores by a warp per position, for the context by a thread per four columns -- and meets G
+// vectors, the scores' in shared memory.  The kernel is a chain of L2 round trips (centre, scores, context), so a group
+// costs little more time than one row, while the rows of a step become fewer waves of CTAs.  Against a CTA of 256 threads
+// per row: 1536 rows, window 21 44 -> 32 us per step; 640 rows, whole sources of up to 100 words 49 -> 28; 768 rows 26 -> 19.
+// G = 1, THREADS = 1024 for a step whose rows leave SMs empty: one position per warp and the context in four ranges of
+// positions (one sentence: 18.1 us per step with 256 threads, 10 so).  grid = sentences * groups, dynamic smem =
+// attention_smem
+template <int G, int THREADS>
+static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attention_kernel(const float* __restrict__ proj, int ldp, const float* __restrict__ u_alt, int ldu,
                                  const float* __restrict__ vp, const float* __restrict__ hs,
                                  const int32_t* __restrict__ src_len, float* __restrict__ ctx, int H, int Hp,
-                                 int k, int hs_sent, int hs_pos, int mode, int D, int win, float* __restrict__ rec_align,
+                                 int k, int groups, int hs_sent, int hs_pos, int mode, int D, float* __restrict__ rec_align,
                                  int32_t* __restrict__ rec_lo, int32_t* __restrict__ rec_vit, tc::Planes ctx_planes, int nt,
                                  int rec_win, int ens, AttTrace at, AttFold fold) {
   tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
-  if (THREADS > 256) {
-    // Few rows: the weights of a step have displaced the encoder's states from L2.  While the projection runs, the k CTAs
+  constexpr int kWarps = THREADS / 32;
+  constexpr int kRanges = THREADS > 512 ? THREADS / 256 : 1;    // of positions, in the context sum
+  constexpr int GP = G == 3 ? 4 : G;                            // beams per position in e, for vector loads
+  const int sent = blockIdx.x / groups, q = blockIdx.x - sent * groups;
+  const int per = (k + groups - 1) / groups, b0 = q * per;
+  const int nb = k - b0 < per ? k - b0 : per;          // beams of this group, 1 .. G
+  const int S = src_len[sent];
+  if (THREADS > 512) {
+    // Few rows: the weights of a step have displaced the encoder's states from L2.  While the projection runs, the CTAs
     // of a sentence ask for them again (a hint; nothing is read here, so the length may still be an earlier step's).
-    const int sent = blockIdx.x / k, S = src_len[sent];
     const char* h0 = reinterpret_cast<const char*>(hs + (size_t)sent * hs_sent * Hp);
     const char* c0 = fold.cs ? reinterpret_cast<const char*>(fold.cs + (size_t)sent * hs_sent * Hp) : nullptr;
     const int lines = Hp / 32;
-    for (int i = (blockIdx.x - sent * k) * THREADS + threadIdx.x; i < S * lines; i += k * THREADS) {
+    for (int i = q * THREADS + threadIdx.x; i < S * lines; i += groups * THREADS) {
       const int pos = i / lines;
       const size_t off = (size_t)pos * hs_pos * Hp * 4 + (size_t)(i - pos * lines) * 128;
       asm volatile("prefetch.global.L2 [%0];" ::"l"(h0 + off));
@@ -252,172 +237,251 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) attent
     }
   }
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
-  extern __shared__ float sm[];
-  constexpr int kGroups = THREADS / 256;    // of window positions, in the context sum
-  float* e = sm;            // [win]
-  float* red = sm + win;    // [THREADS / 32]
-  float4* csum = reinterpret_cast<float4*>(sm + ((win + THREADS / 32 + 3) & ~3));   // [kGroups - 1][256] partial contexts
-  __shared__ float s_pt;
-  __shared__ int s_lo, s_hi;
-  const int r = blockIdx.x;
-  const int sent = r / k;
-  const int S = src_len[sent];
-  const float* u = u_alt ? (u_alt + (size_t)r * ldu) : (proj + (size_t)r * ldp + Hp);
+  extern __shared__ __align__(16) float sm[];
+  float* su = sm;                                           // [G][Hp] what the states are multiplied with, and then
+  float4* csum = reinterpret_cast<float4*>(sm);             // [kRanges - 1][256] partial contexts (G = 1)
+  float* e = sm + G * (Hp > (kRanges - 1) * 1024 ? Hp : (kRanges - 1) * 1024);    // [positions][GP], from the first position of all windows on
+  __shared__ float s_red[G][kWarps];
+  __shared__ float s_pt[G];
+  __shared__ int s_lo[G], s_hi[G];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r0 = sent * k + b0;
   const float* hsb = hs + (size_t)sent * hs_sent * Hp;
+  auto row_of = [&](int g) { return r0 + (g < nb ? g : nb - 1); };
 
-  if (mode == 0) {
-    float part = 0.f;
-    const float* t1 = proj + (size_t)r * ldp;
-    for (int j = threadIdx.x; j < H; j += blockDim.x) part = fmaf(vp[j], t1[j], part);
-    const float dot = block_sum(part, red);
-    if (threadIdx.x == 0) {
-      const float sg = (float)(1.0 / (1.0 + exp(-1.0 * (double)dot)));  // SigmoidKernel, deep_rnn_kernel.h:1075-1080
-      const float pt = (float)S * sg;
-      s_pt = pt;
-      s_lo = (0 > (int)pt - D) ? 0 : ((int)pt - D);                       // LowerUpperKernel, :1094-1100
-      s_hi = ((S - 1) < (int)pt + D) ? (S - 1) : ((int)pt + D);
-      if (at.pt) at.pt[((size_t)at.orig[sent] * at.T1 + at.t) * k + (r - sent * k)] = pt;
-    }
-  } else if (threadIdx.x == 0) {
-    s_pt = 0.f; s_lo = 0; s_hi = S - 1;
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    const float* u = u_alt ? (u_alt + (size_t)row_of(g) * ldu) : (proj + (size_t)row_of(g) * ldp + Hp);
+    for (int j = tid * 4; j < Hp; j += THREADS * 4) *reinterpret_cast<float4*>(su + g * Hp + j) = *reinterpret_cast<const float4*>(u + j);
   }
-  __syncthreads();
-  const int lo = s_lo, hi = s_hi;
-  const int W = hi - lo + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int w = warp; w < W; w += nw) {
-    const float* hrow = hsb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp;
-    float acc = 0.f;
-    auto dot4 = [&](int j) {
-      const float4 a = *reinterpret_cast<const float4*>(hrow + j);
-      const float4 b = *reinterpret_cast<const float4*>(u + j);
-      acc = fmaf(a.x, b.x, acc); acc = fmaf(a.y, b.y, acc); acc = fmaf(a.z, b.z, acc); acc = fmaf(a.w, b.w, acc);
-    };
-    if (THREADS > 256) {
-#pragma unroll 8
-      for (int j = lane * 4; j < Hp; j += 128) dot4(j);
-    } else {
-      for (int j = lane * 4; j < Hp; j += 128) dot4(j);
+  if (mode == 0) {
+    // each 256 threads take every other beam
+    constexpr int kPart = THREADS / 256, kMine = (G + kPart - 1) / kPart;
+    const int first = G > 1 ? tid >> 8 : 0;
+    constexpr int kStep = G > 1 ? 256 : THREADS;
+    float part[kMine] = {};
+    for (int j = G > 1 ? tid & 255 : tid; j < H; j += kStep) {
+      const float v = vp[j];
+#pragma unroll
+      for (int i = 0; i < kMine; ++i) part[i] = fmaf(v, proj[(size_t)row_of(first + i * kPart) * ldp + j], part[i]);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) e[w] = acc;
+    for (int i = 0; i < kMine; ++i) {
+      const int g = first + i * kPart;
+      part[i] = warp_sum(part[i]);
+      if (lane == 0 && g < G) s_red[g][G > 1 ? warp & 7 : warp] = part[i];
+    }
+    __syncthreads();
+    if (warp < nb) {
+      float dot = 0.f;
+      if (G > 1) {
+        for (int i = 0; i < 8; ++i) dot += s_red[warp][i];
+      } else {
+        dot = warp_sum(lane < kWarps ? s_red[0][lane] : 0.f);
+      }
+      if (lane == 0) {
+        const float sg = (float)(1.0 / (1.0 + exp(-1.0 * (double)dot)));  // SigmoidKernel, deep_rnn_kernel.h:1075-1080
+        const float pt = (float)S * sg;
+        s_pt[warp] = pt;
+        s_lo[warp] = (0 > (int)pt - D) ? 0 : ((int)pt - D);                       // LowerUpperKernel, :1094-1100
+        s_hi[warp] = ((S - 1) < (int)pt + D) ? (S - 1) : ((int)pt + D);
+        if (at.pt) at.pt[((size_t)at.orig[sent] * at.T1 + at.t) * k + b0 + warp] = pt;
+      }
+    }
+  } else if (tid < nb) {
+    s_pt[tid] = 0.f; s_lo[tid] = 0; s_hi[tid] = S - 1;
   }
   __syncthreads();
-  if (warp == 0) {
+  int lo = s_lo[0], hi = s_hi[0];     // of all windows
+#pragma unroll
+  for (int g = 1; g < G; ++g)
+    if (g < nb) { lo = min(lo, s_lo[g]); hi = max(hi, s_hi[g]); }
+  const int W = hi - lo + 1;
+  // scores: two positions at a time meet the vectors read from shared memory, which would otherwise be the bound
+  constexpr int kAtOnce = G > 1 ? 2 : 1;
+  for (int w = warp; w < W; w += kWarps * kAtOnce) {
+    const int w2 = kAtOnce > 1 && w + kWarps < W ? w + kWarps : w;
+    const float* ha = hsb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp;
+    const float* hb = hsb + (size_t)(S - 1 - (lo + w2)) * hs_pos * Hp;
+    float acc[kAtOnce][G] = {};
+    auto dot4 = [&](int j) {
+      float4 a[kAtOnce];
+      a[0] = *reinterpret_cast<const float4*>(ha + j);
+      if (kAtOnce > 1) a[kAtOnce - 1] = *reinterpret_cast<const float4*>(hb + j);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float4 b = *reinterpret_cast<const float4*>(su + g * Hp + j);
+#pragma unroll
+        for (int p = 0; p < kAtOnce; ++p) {
+          float& c = acc[p][g];
+          c = fmaf(a[p].x, b.x, c); c = fmaf(a[p].y, b.y, c); c = fmaf(a[p].z, b.z, c); c = fmaf(a[p].w, b.w, c);
+        }
+      }
+    };
+#pragma unroll (THREADS > 512 ? 8 : G > 1 ? 2 : 4)
+    for (int j = lane * 4; j < Hp; j += 128) dot4(j);
+#pragma unroll
+    for (int p = 0; p < kAtOnce; ++p)
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const float v = warp_sum(acc[p][g]);
+        if (lane == 0) e[(p ? w2 : w) * GP + g] = v;
+      }
+  }
+  __syncthreads();
+  if (warp < nb) {
     // AlignmentReductionKernel, deep_rnn_kernel.h:1197-1241 (max starts at 0, no renormalisation
     // after the Gaussian), one lane per window position instead of one thread per beam
+    const int g = warp, wlo = s_lo[g], whi = s_hi[g];
+    const int w0 = wlo - lo, w1 = whi - lo + 1;     // its window among the positions
+    float* eg = e + g;
     float mx = 0.f;
-    for (int w = lane; w < W; w += 32) mx = fmaxf(mx, e[w]);
+    for (int w = w0 + lane; w < w1; w += 32) mx = fmaxf(mx, eg[w * GP]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     float sum = 0.f;
-    for (int w = lane; w < W; w += 32) { const float ev = expf(e[w] - mx); e[w] = ev; sum += ev; }
+    for (int w = w0 + lane; w < w1; w += 32) { const float ev = expf(eg[w * GP] - mx); eg[w * GP] = ev; sum += ev; }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float sigma_sq = ((float)D * (float)D) / 4.0f;
-    const float pt = s_pt;
+    const float pt = s_pt[g];
     float best = 0.f; int besti = 0x7fffffff;
-    for (int w = lane; w < W; w += 32) {
-      float a = e[w];
+    for (int w = w0 + lane; w < w1; w += 32) {
+      float a = eg[w * GP];
       if (mode == 0) {
         const float d = pt - (float)(lo + w);
         const float tmp = expf(-(d * d) / (2 * sigma_sq));
         if (0 != sum) a = (a / sum) * tmp;
       } else if (0 != sum) a = a / sum;
-      e[w] = a;
+      eg[w * GP] = a;
       if (a > best) { best = a; besti = lo + w; }  // viterbi vote, src/decoder.h:1948-1962 (first maximum)
     }
+    if (G > 1)
+      for (int w = lane; w < W; w += 32)
+        if (w < w0 || w >= w1) eg[w * GP] = 0.f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ob = __shfl_xor_sync(0xffffffffu, best, o);
       const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
       if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
     }
-    if (lane == 0 && rec_lo && ens == 0) { rec_lo[r] = lo; rec_vit[r] = (best > 0.f) ? besti : -1; }
+    if (lane == 0 && rec_lo && ens == 0) { rec_lo[r0 + g] = wlo; rec_vit[r0 + g] = (best > 0.f) ? besti : -1; }
+  } else if (G > 1 && warp < G) {
+    for (int w = lane; w < W; w += 32) e[w * GP + warp] = 0.f;
   }
   __syncthreads();
-  if (rec_align && ens == 0)
-    for (int w = threadIdx.x; w < rec_win; w += blockDim.x) rec_align[(size_t)r * rec_win + w] = (w < W) ? e[w] : 0.f;
-  if (rec_align && ens != 0) {
-    float* row = rec_align + (size_t)r * rec_win;
-    for (int sp = threadIdx.x; sp < rec_win; sp += blockDim.x) {
-      const float a = (sp >= lo && sp <= hi) ? e[sp - lo] : 0.f;
-      row[sp] = (ens == 1) ? (0.f + a) : (row[sp] + a);
-    }
-    if (ens == 3) {
-      __syncthreads();
-      if (warp == 0) {
-        float best = 0.f; int besti = 0x7fffffff;
-        for (int sp = lane; sp < rec_win; sp += 32) {
-          const float a = row[sp];
-          if (a > best) { best = a; besti = sp; }
-        }
+  if (rec_align)
+    for (int g = 0; g < nb; ++g) {
+      float* row = rec_align + (size_t)(r0 + g) * rec_win;
+      const float* eg = e + g;
+      const int wlo = s_lo[g], whi = s_hi[g];
+      if (ens == 0) {
+        for (int w = tid; w < rec_win; w += THREADS) row[w] = (wlo + w <= whi) ? eg[(wlo - lo + w) * GP] : 0.f;
+        continue;
+      }
+      for (int sp = tid; sp < rec_win; sp += THREADS) {
+        const float a = (sp >= wlo && sp <= whi) ? eg[(sp - lo) * GP] : 0.f;
+        row[sp] = (ens == 1) ? (0.f + a) : (row[sp] + a);
+      }
+      if (ens == 3) {
+        __syncthreads();
+        if (warp == 0) {
+          float best = 0.f; int besti = 0x7fffffff;
+          for (int sp = lane; sp < rec_win; sp += 32) {
+            const float a = row[sp];
+            if (a > best) { best = a; besti = sp; }
+          }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
-          if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
+          for (int o = 16; o > 0; o >>= 1) {
+            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
+            if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
+          }
+          if (lane == 0) { rec_lo[r0 + g] = 0; rec_vit[r0 + g] = (best > 0.f) ? besti : -1; }
         }
-        if (lane == 0) { rec_lo[r] = 0; rec_vit[r] = (best > 0.f) ? besti : -1; }
       }
     }
-  }
-  // context: CreateCTKernel, deep_rnn_kernel.h:1250-1260 (sum over window positions in order)
-  float* crow = ctx ? ctx + (size_t)r * Hp : nullptr;
+  // context: CreateCTKernel, deep_rnn_kernel.h:1250-1260
   const float* csb = fold.cs ? fold.cs + (size_t)sent * hs_sent * Hp : hsb;
-  auto add = [&](float4& acc, int w, int j) {
-    const float a = e[w];
-    const float4 h4 = *reinterpret_cast<const float4*>(csb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp + j);
-    acc.x += a * h4.x; acc.y += a * h4.y; acc.z += a * h4.z; acc.w += a * h4.w;
-  };
-  auto finish = [&](float4 acc, int j) {
-    if (fold.cs) {
-      // the attentional state: the sums of TcEpiBiasTanh in its order, (W_c1 ctx + W_c2 h) + b
-      const float4 g = *reinterpret_cast<const float4*>(fold.add + (size_t)r * fold.ld_add + j);
-      const float4 b = *reinterpret_cast<const float4*>(fold.bias + j);
-      acc.x = tc::tanh_fast((acc.x + g.x) + b.x); acc.y = tc::tanh_fast((acc.y + g.y) + b.y);
-      acc.z = tc::tanh_fast((acc.z + g.z) + b.z); acc.w = tc::tanh_fast((acc.w + g.w) + b.w);
-    }
-    if (crow) *reinterpret_cast<float4*>(crow + j) = acc;
-    if (ctx_planes.p[0]) {  // tensor-core path: the context goes straight into its operand panel
-      const size_t idx = (size_t)r * ctx_planes.ld + j;
-      tc::split_store4(ctx_planes, nt, idx, acc.x, acc.y, acc.z, acc.w);
-    }
-  };
-  if constexpr (kGroups == 1) {
-    for (int j = threadIdx.x * 4; j < Hp; j += blockDim.x * 4) {
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int w = 0; w < W; ++w) add(acc, w, j);
-      finish(acc, j);
+  const float* col0 = csb + (size_t)(S - 1 - lo) * hs_pos * Hp;
+  const size_t step = (size_t)hs_pos * Hp;
+  if constexpr (kRanges == 1) {
+    // a thread has two columns of every beam and sums the positions in order
+    for (int j = tid * 2; j < Hp; j += THREADS * 2) {
+      float2 acc[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) acc[g] = make_float2(0.f, 0.f);
+      const float* col = col0 + j;
+#pragma unroll 6
+      for (int w = 0; w < W; ++w) {
+        const float2 h = *reinterpret_cast<const float2*>(col - w * step);
+        float a[GP];
+        if constexpr (GP == 4) {
+          *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(e + w * GP);
+        } else if constexpr (GP == 2) {
+          *reinterpret_cast<float2*>(a) = *reinterpret_cast<const float2*>(e + w * GP);
+        } else {
+          a[0] = e[w];
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) { acc[g].x += a[g] * h.x; acc[g].y += a[g] * h.y; }
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        if (g >= nb) break;
+        const int r = r0 + g;
+        float2 c = acc[g];
+        if (fold.cs) {
+          // the attentional state: the sums of TcEpiBiasTanh in its order, (W_c1 ctx + W_c2 h) + b
+          const float2 a = *reinterpret_cast<const float2*>(fold.add + (size_t)r * fold.ld_add + j);
+          const float2 b = *reinterpret_cast<const float2*>(fold.bias + j);
+          c.x = tc::tanh_fast((c.x + a.x) + b.x); c.y = tc::tanh_fast((c.y + a.y) + b.y);
+        }
+        if (ctx) *reinterpret_cast<float2*>(ctx + (size_t)r * Hp + j) = c;
+        if (ctx_planes.p[0])    // tensor-core path: the context goes straight into its operand panel
+          tc::split_store2(ctx_planes, nt, (size_t)r * ctx_planes.ld + j, c.x, c.y);
+      }
     }
   } else {
-    const int group = threadIdx.x >> 8, w0 = W * group / kGroups, w1 = W * (group + 1) / kGroups;
+    const int range = tid >> 8, c = tid & 255, w0 = W * range / kRanges, w1 = W * (range + 1) / kRanges;
     for (int j0 = 0; j0 < Hp; j0 += 1024) {
-      const int j = j0 + (threadIdx.x & 255) * 4;
+      const int j = j0 + c * 4;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       if (j < Hp) {
+        const float* col = col0 + j;
 #pragma unroll 6
-        for (int w = w0; w < w1; ++w) add(acc, w, j);
+        for (int w = w0; w < w1; ++w) {
+          const float a = e[w];
+          const float4 h4 = *reinterpret_cast<const float4*>(col - w * step);
+          acc.x += a * h4.x; acc.y += a * h4.y; acc.z += a * h4.z; acc.w += a * h4.w;
+        }
       }
       if (j0 > 0) __syncthreads();      // (the previous pass's partial contexts have been read)
-      if (group > 0 && j < Hp) csum[(group - 1) * 256 + (threadIdx.x & 255)] = acc;
+      if (range > 0 && j < Hp) csum[(range - 1) * 256 + c] = acc;
       __syncthreads();
-      if (group == 0 && j < Hp) {
+      if (range == 0 && j < Hp) {
 #pragma unroll
-        for (int g = 0; g < kGroups - 1; ++g) {
-          const float4 o = csum[g * 256 + threadIdx.x];
-          acc.x += o.x; acc.y += o.y; acc.z += o.z; acc.w += o.w;
+        for (int o = 0; o < kRanges - 1; ++o) {
+          const float4 p = csum[o * 256 + c];
+          acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
         }
-        finish(acc, j);
+        if (fold.cs) {
+          const float4 a = *reinterpret_cast<const float4*>(fold.add + (size_t)r0 * fold.ld_add + j);
+          const float4 b = *reinterpret_cast<const float4*>(fold.bias + j);
+          acc.x = tc::tanh_fast((acc.x + a.x) + b.x); acc.y = tc::tanh_fast((acc.y + a.y) + b.y);
+          acc.z = tc::tanh_fast((acc.z + a.z) + b.z); acc.w = tc::tanh_fast((acc.w + a.w) + b.w);
+        }
+        if (ctx) *reinterpret_cast<float4*>(ctx + (size_t)r0 * Hp + j) = acc;
+        if (ctx_planes.p[0]) tc::split_store4(ctx_planes, nt, (size_t)r0 * ctx_planes.ld + j, acc.x, acc.y, acc.z, acc.w);
       }
     }
   }
 }
 
-template <int THREADS>
-inline size_t attention_smem(int win) {
-  return sizeof(float) * (size_t)(((win + THREADS / 32 + 3) & ~3) + (THREADS / 256 - 1) * 1024);
+// `positions`: the window of one beam, the whole source where windows are joined
+inline size_t attention_smem(int G, int threads, int Hp, int positions) {
+  const int parts = threads > 512 ? (threads / 256 - 1) * 1024 : 0, gp = G == 3 ? 4 : G;
+  return sizeof(float) * (size_t)(G * (Hp > parts ? Hp : parts) + gp * positions);
 }
 
 // ---------------------------------------------------------------------------------------

@@ -570,3 +570,26 @@ def test_scores_match_a_forced_decode(cuda_lib, c1, n_sent, beam, members, max_b
         dec.close()
     np.testing.assert_allclose(res[0][1], res[1][1], rtol=RTOL_FP32, atol=1e-6)
     np.testing.assert_allclose(res[0][0], res[1][0], rtol=RTOL_FP32)
+
+
+@pytest.mark.parametrize("attention,n_sent,beam,members", [("local_p_general", 150, 1, 1), ("local_p_general", 149, 2, 1), ("global_general", 149, 5, 1),
+                                                           ("local_p_general", 80, 12, 1), ("local_p_general", 149, 3, 2)])
+def test_attention_of_beam_groups(cuda_lib, c1, attention, n_sent, beam, members):
+    """Steps of more rows than SMs: the attention's CTAs serve groups of one to three beams (the last one of a sentence
+    may be smaller) with windows of their own.  Against the same search, forced, in small batches of a CTA per row."""
+    from linmt_b200 import decoder
+    c, blob, _ = c1
+    blobs = [blob] + [synth.make_blob(c.desc, 30 + m) for m in range(1, members)]
+    sents = synth.make_sentences(n_sent, 1, 30, c.desc.Vs, 1.1, 5, lambda s: s + 1)
+    kw = dict(beam=beam, attention=attention, print_info=True, max_src_len=32, max_steps=64)
+    big = decoder.Decoder(c.desc, blobs, max_batch=n_sent, **kw)
+    a = big.decode(sents, trace=True, want_align=True)
+    small = decoder.Decoder(c.desc, blobs, max_batch=8, **kw)
+    b = small.decode(sents, trace=True, force=a, want_align=True)
+    big.close(); small.close()
+    for i in range(n_sent):
+        T = int(sents.steps[i])
+        x, y = a["cand_logp"][i, :T], b["cand_logp"][i, :T]
+        np.testing.assert_allclose(x[0, 0], y[0, 0], rtol=RTOL_FP32, atol=1e-5)
+        np.testing.assert_allclose(x[1:], y[1:], rtol=RTOL_FP32, atol=1e-5)
+    np.testing.assert_allclose(a["align"], b["align"], atol=1e-4)
