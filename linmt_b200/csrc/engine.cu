@@ -654,8 +654,8 @@ int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, co
     a.fin_final = d_fin_final_; a.win = rec_win; a.k = k; a.nbest = opt.nbest; a.max_len = max_len; a.max_src = opt.max_src_len;
     a.lp_alpha = opt.lp_alpha; a.cp_beta = opt.cp_beta; a.min_ratio = opt.min_ratio;
     a.out_tok = d_out_tok; a.out_len = d_out_len; a.out_score = d_out_score; a.out_vit = d_out_vit; a.out_align = d_out_align;
-    const size_t smem = 4 * ((size_t)opt.max_src_len * sizeof(float) + (size_t)max_len * sizeof(int));
-    finalize_kernel<<<n, 128, smem, stream>>>(a);
+    const FinalizeShape f = finalize_shape(max_len, k);
+    finalize_kernel<<<n, 32 * f.warps, f.smem, stream>>>(a, f.par_bytes);
     LAUNCHED();
     CK(cudaGetLastError());
   }
