@@ -1757,7 +1757,9 @@ static __global__ void __launch_bounds__(512) finalize_kernel(FinalizeArgs a, in
   }
   __syncthreads();
   const int osent = a.orig[sent];
-  for (int q = warp; q < a.nbest; q += nw) {
+  for (int q0 = 0; q0 < a.nbest; q0 += nw) {
+    const int q = q0 + warp;
+    if (q < a.nbest) {
     const size_t ob = (size_t)osent * a.nbest + q;
     // positions past the hypothesis (all of them when fewer than nbest passed the filter) read START / "no
     // alignment", so that a result does not carry what an earlier decode left in the buffer
@@ -1769,10 +1771,8 @@ static __global__ void __launch_bounds__(512) finalize_kernel(FinalizeArgs a, in
     if (a.out_align)
       for (size_t j = (size_t)n_used * a.max_src + lane; j < (size_t)a.max_len * a.max_src; j += 32)
         a.out_align[ob * a.max_len * a.max_src + j] = 0.f;
-    if (q >= s_nb) {
-      if (lane == 0) { a.out_len[ob] = 0; a.out_score[ob] = 0.f; }
-      continue;
-    }
+    if (q >= s_nb && lane == 0) { a.out_len[ob] = 0; a.out_score[ob] = 0.f; }
+    if (q < s_nb) {
     const int h = s_best[q];
     const int t = ft[h];
     const int n = t + 2;
@@ -1790,21 +1790,26 @@ static __global__ void __launch_bounds__(512) finalize_kernel(FinalizeArgs a, in
       if (p <= t) ot[p] = a.bs.hist_tok[(size_t)(p - 1) * R + r0 + path[p + 1]];      // the word chosen after forward p - 1
       if (ov) ov[p] = a.rec_vit ? a.rec_vit[(size_t)(p - 1) * R + r0 + path[p]] : -1;
     }
-    __syncwarp();
-    if (a.out_align && tracked) {
-      float* oa = a.out_align + ob * a.max_len * a.max_src;
-      for (int p = 0; p < n; ++p) {
+    }
+    }
+    if (!a.out_align || !tracked) continue;
+    // alignments: the steps of this round's hypotheses are dealt to all warps
+    __syncthreads();
+    for (int z = 0; z < nw && q0 + z < s_nb; ++z) {
+      const int n = ft[s_best[q0 + z]] + 2;
+      const int* zpath = reinterpret_cast<int*>(smraw) + z * a.max_len;
+      float* oa = a.out_align + ((size_t)osent * a.nbest + q0 + z) * a.max_len * a.max_src;
+      for (int p = warp; p < n; p += nw) {
         float part = 0.f;
         const bool norm = (a.cp_beta != 0.f) && p >= 2;
         size_t row = 0; int lo = 0;
-        if (p >= 1) { row = (size_t)(p - 1) * R + r0 + path[p]; lo = a.rec_lo[row]; }
+        if (p >= 1) { row = (size_t)(p - 1) * R + r0 + zpath[p]; lo = a.rec_lo[row]; }
         if (norm) {
           for (int s = lane; s < S; s += 32) {
             const int w = s - lo;
             part += ((w >= 0 && w < a.win) ? a.rec_align[row * a.win + w] : 0.f) + 0.01f;
           }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          part = warp_sum(part);
         }
         for (int s = lane; s < a.max_src; s += 32) {
           float v = 0.f;
@@ -1817,7 +1822,7 @@ static __global__ void __launch_bounds__(512) finalize_kernel(FinalizeArgs a, in
         }
       }
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
