@@ -417,6 +417,7 @@ struct TcEpiLstm {
   // same way.  Rows past their length (encoder) keep c and copy h_prev.
   static constexpr bool kHasBlock = true;
   static constexpr bool kHasPmax = false;
+  static constexpr bool kHasPrefetch = true;
   __device__ __forceinline__ void block(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, int /*slot*/) const {
     block_of<kEpiBlockChunks, 3>(row0, lane, M, col_first, nch, v, sbuf);
   }
@@ -426,7 +427,20 @@ struct TcEpiLstm {
   __device__ __forceinline__ void staged(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf, Stat&) const {
     block_of<2, 1>(row0, lane, M, col_first, nch, v, sbuf);
   }
-  // CH = most chunks, PL = planes there is room for
+  // What a block is going to read besides the accumulator, asked into L2 while the product runs (rows of a table far
+  // larger than L2; the cell state).
+  __device__ __forceinline__ void prefetch(int row0, int lane, int M, int col_first, int nch) const {
+    const int row = row0 + lane;
+    if (row >= M || nch <= 0) return;
+    if (xw) {
+      const char* x = reinterpret_cast<const char*>(xw + (size_t)x_row(row) * x_ld + col_first);
+      for (int b = 0; b < nch; b += 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + 64 * b));
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(x + 64 * nch - 4));
+    }
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(c_prev + (size_t)c_src_row(row) * ldc + (col_first >> 2)));
+  }
+  // CH = most chunks, PL = planes there is room for.  The loads of a block are issued four at a time, their row numbers
+  // looked up once: as a loop of load and staging store each was a round trip of its own.
   template <int CH, int PL>
   __device__ __forceinline__ void block_of(int row0, int lane, int M, int col_first, int nch, float (*v)[16], float* sbuf) const {
     constexpr int CS = 4 * CH + 4;           // floats per staged row of c (and of h in fp32)
@@ -440,14 +454,24 @@ struct TcEpiLstm {
     float* cs = sbuf;                                            // [32][CS] floats: c_prev in, c out
     unsigned short* hs = reinterpret_cast<unsigned short*>(sbuf + 32 * CS);   // [planes][32][HS] 16-bit
     float* hf = sbuf + 32 * CS + PL * 32 * HS / 2;               // [32][CS] floats: h in fp32 (only if h_f32)
+    const unsigned inv = (65536u + nq - 1) / nq;                 // s / nq for s < 512 = s * inv >> 16
+    const int c_row = valid ? c_src_row(row) : 0;
     if (xw) {
       // the rows of the input-term table for this block, staged coalesced, then added lane = row
-      const int nq4 = 4 * nch;
-      for (int s = lane; s < 32 * nq4; s += 32) {
-        const int r = s / nq4, g = s - r * nq4;
-        if (row0 + r < M)
-          *reinterpret_cast<float4*>(sbuf + r * XS + 4 * g) =
-              *reinterpret_cast<const float4*>(xw + (size_t)x_row(row0 + r) * x_ld + col_first + 4 * g);
+      const int my_x = valid ? x_row(row) : 0;
+      for (int i0 = 0; i0 < nq; ++i0) {
+        float4 t[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int s = lane + 32 * (4 * i0 + u), r = (int)(((unsigned)(s >> 2) * inv) >> 16), g = s - r * 4 * nq;
+          const int xr = __shfl_sync(0xffffffffu, my_x, r);
+          t[u] = row0 + r < M ? __ldg(reinterpret_cast<const float4*>(xw + (size_t)xr * x_ld + col_first + 4 * g)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int s = lane + 32 * (4 * i0 + u), r = (int)(((unsigned)(s >> 2) * inv) >> 16), g = s - r * 4 * nq;
+          *reinterpret_cast<float4*>(sbuf + r * XS + 4 * g) = t[u];
+        }
       }
       __syncwarp();
       if (valid) {
@@ -465,11 +489,21 @@ struct TcEpiLstm {
       __syncwarp();
     }
     // c_prev: coalesced load into the staging area
-    for (int s = lane; s < 32 * nq; s += 32) {
-      const int r = s / nq, g = s - r * nq;
-      if (row0 + r < M)
-        *reinterpret_cast<float4*>(cs + r * CS + 4 * g) =
-            *reinterpret_cast<const float4*>(c_prev + (size_t)c_src_row(row0 + r) * ldc + j_first + 4 * g);
+    {
+      float4 t[CH];
+#pragma unroll
+      for (int u = 0; u < CH; ++u)
+        if (u < nq) {
+          const int s = lane + 32 * u, r = (int)(((unsigned)s * inv) >> 16), g = s - r * nq;
+          const int cr = __shfl_sync(0xffffffffu, c_row, r);
+          t[u] = row0 + r < M ? *reinterpret_cast<const float4*>(c_prev + (size_t)cr * ldc + j_first + 4 * g) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+      for (int u = 0; u < CH; ++u)
+        if (u < nq) {
+          const int s = lane + 32 * u, r = (int)(((unsigned)s * inv) >> 16), g = s - r * nq;
+          *reinterpret_cast<float4*>(cs + r * CS + 4 * g) = t[u];
+        }
     }
     __syncwarp();
     if (active) {
@@ -481,7 +515,7 @@ struct TcEpiLstm {
           float c[4], h[4];
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
-            const float4 b = *reinterpret_cast<const float4*>(bias + col_first + 16 * ci + 4 * u);
+            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col_first + 16 * ci + 4 * u));
             const float gi = sigmoid_fast(v[ci][4 * u + 0] + b.x);
             const float gf = sigmoid_fast(v[ci][4 * u + 1] + b.y);
             const float gg = tanh_fast(v[ci][4 * u + 2] + b.z);
@@ -522,7 +556,7 @@ struct TcEpiLstm {
     __syncwarp();
     // coalesced stores
     for (int s = lane; s < 32 * nq; s += 32) {
-      const int r = s / nq, g = s - r * nq;
+      const int r = (int)(((unsigned)s * inv) >> 16), g = s - r * nq;
       if (row0 + r < M) {
         *reinterpret_cast<float4*>(c_out + (size_t)(row0 + r) * ldc + j_first + 4 * g) = *reinterpret_cast<const float4*>(cs + r * CS + 4 * g);
         if (h_f32 && ((active_mask >> r) & 1u))
@@ -531,7 +565,7 @@ struct TcEpiLstm {
     }
     for (int t = 0; t < nt; ++t)
       for (int s = lane; s < 32 * nq; s += 32) {
-        const int r = s / nq, g = s - r * nq;
+        const int r = (int)(((unsigned)s * inv) >> 16), g = s - r * nq;
         if (row0 + r < M) {
           const uint2 hv = *reinterpret_cast<const uint2*>(hs + (t * 32 + r) * HS + 4 * g);
           *reinterpret_cast<uint2*>(h_out1.p[t] + (size_t)(row0 + r) * h_out1.ld + h1_col0 + j_first + 4 * g) = hv;
@@ -586,6 +620,7 @@ struct TcEpiBiasTanh {
   const float* add = nullptr; int ld_add = 0;
   static constexpr bool kHasBlock = false;
   static constexpr bool kHasPmax = false;
+  static constexpr bool kHasPrefetch = false;
   __device__ __forceinline__ void block(int, int, int, int, int, float (*)[16], float*, int) const {}
   __device__ __forceinline__ void operator()(int row, int col0, const float* v) const {
     const size_t idx = (size_t)row * out.ld + col_off + col0;
@@ -659,6 +694,7 @@ struct TcEpiF32 {
   // staged per row, then stored with a row's 16 float4 on consecutive lanes.
   static constexpr bool kHasBlock = true;
   static constexpr bool kHasPmax = true;
+  static constexpr bool kHasPrefetch = false;
   struct Stat { float m, s; };       // maximum and sum of exp(z - maximum) of some columns of a row
   static __device__ __forceinline__ Stat no_stat() { return Stat{-INFINITY, 0.f}; }
   __device__ __forceinline__ void merge(Stat& a, const Stat& b) const {
@@ -1035,6 +1071,7 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
     // with split-K the tile's partial sum goes to the workspace; the last CTA of the tile adds them up
     float* wrow = ws ? ws + ((size_t)blockIdx.z * ((size_t)gridDim.x * BM) + (size_t)row) * (size_t)N : nullptr;
     pdl_wait();   // before the first global access of these warps (the hardware wait is over long before)
+    if constexpr (Epi::kHasPrefetch) epi.prefetch(row0, lane, M, n0 + ch0 * 16, nmine);
     float macc[kChunks][16];
     auto finish = [&]() {
       if (splits == 1) {

@@ -238,6 +238,7 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     float* wrow = ws ? ws + ((size_t)blockIdx.z * ((size_t)gridDim.x * BM) + (size_t)row) * (size_t)N : nullptr;
     const uint32_t main_free_leader = cluster_map(main_free, 0u);
     pdl_wait();
+    if constexpr (Epi::kHasPrefetch) epi.prefetch(row0, lane, M, n0 + ch0 * 16, nmine);
     float macc[kChunks][16];
     auto finish = [&]() {
       if (splits == 1) {
@@ -507,6 +508,7 @@ gemm_tc_persist_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, in
         const int left = (N - (n0 + ch0 * 16) + 15) >> 4;
         if (left < nmine) nmine = left < 0 ? 0 : left;
       }
+      if constexpr (Epi::kHasPrefetch) epi.prefetch(row0, lane, M, n0 + ch0 * 16, nmine);
       if (!mbar_wait_sleepy(accum_full + 8u * b, (uint32_t)((it >> 1) & 1), &s_abort)) break;
       tc_fence_after();
       auto st = Epi::no_stat();
