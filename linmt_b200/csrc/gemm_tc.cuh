@@ -665,13 +665,14 @@ struct TcEpiF32 {
   __half* out16 = nullptr;
   __device__ __forceinline__ float4 finish4(float4 r, int col0) const {
     if (bias) {
-      const float4 b = *reinterpret_cast<const float4*>(bias + col0);
+      const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col0));
       r.x += b.x; r.y += b.y; r.z += b.z; r.w += b.w;
     }
     if (col0 < split) { r.x = tanh_fast(r.x); r.y = tanh_fast(r.y); r.z = tanh_fast(r.z); r.w = tanh_fast(r.w); }
     if (out16) {
-      r.x = __half2float(__float2half_rn(r.x)); r.y = __half2float(__float2half_rn(r.y));
-      r.z = __half2float(__float2half_rn(r.z)); r.w = __half2float(__float2half_rn(r.w));
+      // (two values to a conversion: a single one is a slow instruction)
+      const float2 lo = __half22float2(__floats2half2_rn(r.x, r.y)), hi = __half22float2(__floats2half2_rn(r.z, r.w));
+      r = make_float4(lo.x, lo.y, hi.x, hi.y);
     }
     return r;
   }
@@ -713,15 +714,20 @@ struct TcEpiF32 {
     for (int c0 = 0; c0 < CH; c0 += 2) {
       Stat h = no_stat();
       if (col_first + 16 * (c0 + 2) <= n_valid && c0 + 2 <= nch) {      // both chunks whole: nothing to test
+        // (four chains: one of 32 dependent steps was most of the time of this)
+        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
         for (int ci = c0; ci < c0 + 2 && ci < CH; ++ci)
 #pragma unroll
-          for (int i = 0; i < 16; ++i) h.m = fmaxf(h.m, v[ci][i]);
+          for (int i = 0; i < 16; ++i) m4[i & 3] = fmaxf(m4[i & 3], v[ci][i]);
+        h.m = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         if (psum) {
+          float s4[4] = {};
 #pragma unroll
           for (int ci = c0; ci < c0 + 2 && ci < CH; ++ci)
 #pragma unroll
-            for (int i = 0; i < 16; ++i) h.s += exp2f_fast((v[ci][i] - h.m) * 1.4426950408889634f);
+            for (int i = 0; i < 16; ++i) s4[i & 3] += exp2f_fast((v[ci][i] - h.m) * 1.4426950408889634f);
+          h.s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
         }
       } else {
 #pragma unroll
