@@ -1422,10 +1422,10 @@ static __global__ void __launch_bounds__(256) ensemble_combine_kernel(EnsembleRo
 // in double like the reference's loop -- keeps the maximum of every 128 classes and the sum, and only the blocks that reach
 // the threshold are formed again to list their candidates.  The combined row itself is never written, and the logits are
 // read once: (M + 1/16) x V x 4 bytes a row instead of (2 M + 2) x V x 4.  M = 4 at up to 384 rows, 30k classes: the two
-// kernels took 224 us per step.
+// kernels took 224 us per step, this one 91, and 76 with the next block's loads in flight.
 // THREADS = 1024 for rows that leave SMs empty.  grid = rows, dynamic smem = ceil(V / 128) floats.
 template <int THREADS>
-static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1) ensemble_topk_kernel(EnsembleRows er, int ld, int V, int kk, int mode, TopkOut out, LogitBlocks bl,
+static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : 1) ensemble_topk_kernel(const __grid_constant__ EnsembleRows er, int ld, int V, int kk, int mode, TopkOut out, LogitBlocks bl,
                                                                                              long long bl_member, float* __restrict__ combined, const __grid_constant__ SelectArgs sel) {
   tc::pdl_launch_dependents();
   tc::pdl_wait();
@@ -1481,31 +1481,40 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1) ensemb
   const double n_members = er.n;
   const bool pow2 = (er.n & (er.n - 1)) == 0;        // then the division is an exact product
   const double inv_members = 1.0 / n_members;
-  auto combine4 = [&](int i) {
+  auto load4 = [&](int i, float4* q) {      // the first four members' loads, in flight together
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+      if (m < er.n) q[m] = *reinterpret_cast<const float4*>(er.logits[m] + (size_t)r * ld + i);
+  };
+  auto combine4 = [&](int i, float4* q) {
     double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int m0 = 0; m0 < er.n; m0 += 4) {
-      float4 q[4];      // four members' loads in flight
+    auto add = [&](int m, const float4& v) {
+      const float c = s_c[m];
+      const float l[4] = {v.x - c, v.y - c, v.z - c, v.w - c};
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
-        if (m0 + m < er.n) q[m] = *reinterpret_cast<const float4*>(er.logits[m0 + m] + (size_t)r * ld + i);
+      for (int u = 0; u < 4; ++u) a[u] += mode == 0 ? (double)expf(l[u]) : (double)l[u];
+    };
 #pragma unroll
-      for (int m = 0; m < 4; ++m)
-        if (m0 + m < er.n) {
-          const float c = s_c[m0 + m];
-          const float l[4] = {q[m].x - c, q[m].y - c, q[m].z - c, q[m].w - c};
-#pragma unroll
-          for (int u = 0; u < 4; ++u) a[u] += mode == 0 ? (double)expf(l[u]) : (double)l[u];
-        }
-    }
+    for (int m = 0; m < 4; ++m)
+      if (m < er.n) add(m, q[m]);
+#pragma unroll 1
+    for (int m = 4; m < er.n; ++m) add(m, *reinterpret_cast<const float4*>(er.logits[m] + (size_t)r * ld + i));
     if (pow2) return make_float4((float)(a[0] * inv_members), (float)(a[1] * inv_members), (float)(a[2] * inv_members), (float)(a[3] * inv_members));
     return make_float4((float)(a[0] / n_members), (float)(a[1] / n_members), (float)(a[2] / n_members), (float)(a[3] / n_members));
   };
   float tmax = -INFINITY, psum = 0.f;
+  // (the next block's loads are in flight while a block is combined: its latency was most of the kernel)
+  float4 next[4] = {};
+  if (warp * 128 + lane * 4 < V) load4(warp * 128 + lane * 4, next);
   for (int b = warp; b * 128 < V; b += kWarps) {
     const int i = b * 128 + lane * 4;
     float bm = -INFINITY;
+    float4 q[4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) q[m] = next[m];
+    if (i + kWarps * 128 < V) load4(i + kWarps * 128, next);
     if (i < V) {
-      const float4 w = combine4(i);
+      const float4 w = combine4(i, q);
       const float v[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int u = 0; u < 4; ++u)
@@ -1541,7 +1550,9 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1) ensemb
     if (s_bm[b] < tau) continue;
     const int i = b * 128 + lane * 4;
     if (i >= V) continue;
-    const float4 w = combine4(i);
+    float4 q[4];
+    load4(i, q);
+    const float4 w = combine4(i, q);
     const float v[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
     for (int u = 0; u < 4; ++u)
@@ -1555,7 +1566,9 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 4 : 1) ensemb
   if (sh.count > kTopkCap) {  // ... unless more classes than the list holds reach the threshold: then it is swept
     float* row = combined + (size_t)r * ld;
     for (int i = tid * 4; i < V; i += THREADS * 4) {
-      const float4 w = combine4(i);
+      float4 q[4];
+      load4(i, q);
+      const float4 w = combine4(i, q);
       *reinterpret_cast<float4*>(row + i) = mode == 0 ? make_float4(logf(w.x), logf(w.y), logf(w.z), logf(w.w)) : w;
     }
     __threadfence_block();
