@@ -41,8 +41,7 @@ C2_TRAFFIC_BYTES = {
     "lstm_gemm": 43.5e6,        # first layer 45.74 MB (with input-term table rows), the others 42.72 MB
     "vocab_gemm": 77.2e6,       # 63.40 MB read (the weights) + 13.82 MB written (fp16 logits, most of them still in L2)
     "attn_proj_gemm": 15.8e6, "attn_out_gemm": 10.56e6,
-    "softmax_topk": 56.0e6,     # the fp16 logits once + candidates' weight rows (cold-cache capture)
-    "gather": 10.66e6, "attention": 19.55e6, "beam_select": 0.11e6,
+    "gather": 10.66e6,          # (softmax and attention: no capture of their present kernels)
 }
 
 
@@ -385,14 +384,14 @@ def run_ours(args):
             roof("vocab_gemm", f"vocabulary GEMM [rows,H]x[H,V] ({args.gemm_path} path)", "tensor", 2.0 * rs * H * V * M, voc_products),
             roof("attn_proj_gemm", "attention projections GEMM [rows,H]x[H,3H] (W_p | W_a^T | W_c2)", "tensor", 2.0 * rs * H * 3 * H * M, gate_products),
             roof("attn_out_gemm", "attention output GEMM [rows,H]x[H,H] (W_c1) + tanh", "tensor", 2.0 * rs * H * H * M, gate_products),
-            roof("softmax_topk", "log-softmax statistics + per-row top-(k+1), one pass over the logits" + (" (fp16)" if logits16 else ""), "hbm",
-                 rs * V * (2.0 if logits16 else 4.0)),
-            roof("ensemble_combine", "ensemble combination of the members' distributions", "hbm", rs * V * 4.0 * (M + 1)),
+            roof("softmax_topk", "log-softmax and per-row top-(k+1) from the logits GEMM's block statistics"
+                 + (", accurate logits of the candidates" if logits16 else "") + ", beam selection", "hbm",
+                 rs * (V / 52 * 8.0 + (c.beam + 2) * (Hp * 4.0 if logits16 else 208.0))),
+            roof("ensemble_combine", "ensemble combination of the members' distributions, softmax, top-(k+1), beam selection", "hbm", rs * V * 4.0 * M),
             roof("gather", "beam reordering of the recurrent state (h planes of every layer, attentional state)", "hbm",
                  rs * (L + 1) * nt * Hp * 2.0 * 2 * M),
             roof("attention", "attention: p_t, window scores, softmax x Gaussian, weighted sum of W_c1-mapped states, tanh -> attentional state", "hbm",
                  (ss * 2 * 21 * Hp * 4.0 + rs * (3 * Hp * 4.0 + nt * Hp * 2.0)) * M),
-            roof("beam_select", "beam selection (k(k+1) candidates per sentence)", "hbm", rs * (c.beam + 1) * 8.0),
         ]
         blocks = [b_ for b_ in blocks if b_]
         blocks.sort(key=lambda b_: -b_["share_of_step"])
