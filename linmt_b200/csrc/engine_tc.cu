@@ -159,11 +159,11 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   // Few rows: the weight-streaming kernel (gemm_tc_rows.cuh), where the rows are the narrow side of the MMA.  Its gain
   // shrinks as the rows fill the 128-row tile (gate product, us against this file's one-tile kernel: 8.7 / 13.8 at 12
   // rows, 10.2 / 14.8 at 32, 11.4 / 15.8 at 64; bf16 6.3 / 13.0 at 12, 9.0 / 13.0 at 64); a product of many column
-  // tiles and one k slice is finished by too few warps for more than 48 rows (vocabulary 12.7 / 14.7 us at 12 rows,
-  // 14.7 / 15.1 at 48, 17.3 / 15.1 at 64).
+  // tiles and one k slice is finished by too few warps for more than 48 rows of the f16 pair (one plane, vocabulary with
+  // block statistics in the decode: 12.7 us at 12 rows, 18.9 at 64 against 19.6 in the one-tile kernel).
   {
     tc::RowsShape rs;
-    if (rows_ && ws_parts_ == 1 && M <= tc::kRowsMax && (M <= 48 || N <= 128 * n_sm_) && tc::make_shape_rows(M, N, K, nt, fmt_, n_sm_, drain >= K / 32, &rs)) {
+    if (rows_ && ws_parts_ == 1 && M <= tc::kRowsMax && (nt == 1 || M <= 48 || N <= 128 * n_sm_) && tc::make_shape_rows(M, N, K, nt, fmt_, n_sm_, drain >= K / 32, &rs)) {
       tc::Planes a = A;
       for (int t = 0; t < 3; ++t) if (a.p[t]) a.p[t] += a_col0;
       const CUtensorMap* xm = b_maps(a, a_rows_cap, K, rs.rp, 64);
