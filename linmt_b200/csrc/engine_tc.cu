@@ -130,13 +130,16 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   // CTA pairs (gemm_tc_pair.cuh) where the one-tile shape has room for two stages only: an even number of row
   // tiles (an odd one is rounded up, which must still fit one wave), split operands, 64-deep stages, K not split
   const int mt = (M + tc::BM - 1) / tc::BM;
+  // (a row offset is for the few-rows kernel and the one-tile kernel, which takes it where the former declines; its
+  // products are those of up to 64 sentences, a single row tile)
+  const bool may_pair = ws_parts_ == 1 && x_row0 == 0;
   // The many-wave one-plane logits GEMM has a persistent pair form as well (measured at K = 1024, against one tile per CTA:
   // N = 30016 23.6 / 29.5 us at 256 rows, 51 / 57 at 640, 55 / 71 at 768; N = 80000 104 / 124 at 512; three row tiles, a
   // quarter of the pair idle, are equal), with 208-wide tiles.
   const bool one_plane_logits = nt == 1 && Epi::kHasPmax;   // the fp32-output GEMMs: vocabulary projection
   // (the block statistics depend on the tile width, so the width is the pair's whether or not pairs may run)
   bool ppair = false;
-  if (one_plane_logits && splits == 1 && bk == 64 && mt >= 2 && ws_parts_ == 1 &&
+  if (one_plane_logits && splits == 1 && bk == 64 && mt >= 2 && may_pair &&
       (long)mt * ((N + bn - 1) / bn) > n_sm_ && (long)((mt + 1) / 2) * ((N + 207) / 208) > n_sm_ / 2) {
     ppair = pair_ && persist_;
     bn = 208;
@@ -144,7 +147,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   // ... and the gate product of one plane, where one tile per CTA is more than one wave (beyond 1024 rows; measured at N =
   // 4096, K = 2048: 22.4 / 28.3 us at 1280 rows, 25.7 / 30.6 at 1536): rounds of 3.9 + 0.0215 * width us, and a prologue
   // and last epilogue of 4 + 0.033 * width.
-  if (Epi::kHasBlock && !Epi::kHasPmax && pair_ && persist_ && nt == 1 && splits == 1 && bk == 64 && mt > 8 && ws_parts_ == 1) {
+  if (Epi::kHasBlock && !Epi::kHasPmax && pair_ && persist_ && nt == 1 && splits == 1 && bk == 64 && mt > 8 && may_pair) {
     double best = 1e30;
     for (int w = 96; w <= 256; w += 16) {
       const long t = (long)((mt + 1) / 2) * ((N + w - 1) / w), rounds = (t + n_sm_ / 2 - 1) / (n_sm_ / 2);
@@ -155,7 +158,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   }
   const long ntile_cols = (N + bn - 1) / bn;
   const bool pair = ppair || (pair_ && fmt_ == 1 && nt == 2 && bk == 64 && splits == 1 && mt >= 2 && bn % 16 == 0 &&
-                    tc::make_shape(bn, nt, bk, fmt_).stages < 3 && (long)((mt + 1) & ~1) * ntile_cols <= n_sm_ && ws_parts_ == 1);
+                    tc::make_shape(bn, nt, bk, fmt_).stages < 3 && (long)((mt + 1) & ~1) * ntile_cols <= n_sm_ && may_pair);
   // Few rows: the weight-streaming kernel (gemm_tc_rows.cuh), where the rows are the narrow side of the MMA.  Its gain
   // shrinks as the rows fill the 128-row tile (gate product, us against this file's one-tile kernel: 8.7 / 13.8 at 12
   // rows, 10.2 / 14.8 at 32, 11.4 / 15.8 at 64; bf16 6.3 / 13.0 at 12, 9.0 / 13.0 at 64); a product of many column
@@ -185,7 +188,6 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
       return LINMT_OK;
     }
   }
-  if (x_row0) return fail(LINMT_EINVAL, "internal: a row offset needs the few-rows kernel");
   const CUtensorMap* am = a_maps(A, a_col0, a_rows_cap, K, bk);
   const CUtensorMap* bm = b_maps(W, N, K, pair ? bn / 2 : bn, bk);
   if (!am || !bm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
@@ -218,7 +220,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   }
   }
   if constexpr (Epi::kHasPmax) {
-  if (persist_ && splits == 1 && tiles > n_sm_ && ((nt == 2 && drain >= K / 32) || one_plane_logits)) {
+  if (persist_ && splits == 1 && x_row0 == 0 && tiles > n_sm_ && ((nt == 2 && drain >= K / 32) || one_plane_logits)) {
     if (nt == 1) {
       const int pdl = sh.pdl;
       sh = tc::make_shape_persist(bn, nt, bk, fmt_);   // a ring of one stage less, staging areas of its own
@@ -236,7 +238,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
     return LINMT_OK;
   }
   CK(tc::launch_gemm_tc(tm, M, N, K, sh, e, d_tc_err_, stream, d_splitk_ws_ + (size_t)ws_part_ * ws_floats,
-                        d_splitk_counters_ + ws_part_ * max_tiles));
+                        d_splitk_counters_ + ws_part_ * max_tiles, x_row0));
   LAUNCHED();
   return LINMT_OK;
 }
@@ -348,7 +350,7 @@ int Engine::run_encoder_tc(int n, int Smax) {
 
 // Encoder for few sentences (up to 64), layer by layer.  A layer's input part W_x . x_p of ALL positions is one GEMM; what
 // is left of the recurrence per position is W_h . h (half of the layer's weights, which then stay in L2 from one position
-// to the next) in the few-rows kernel, with the input part added in its epilogue.  L x S short launches instead of S
+// to the next) in the few-rows kernel, or for wide models in the one-tile kernel, with the input part added in the epilogue.  L x S short launches instead of S
 // rounds of L launches on L streams that each read the whole layer from HBM: one sentence of 30 words 1.28 -> 0.75 ms.
 // Block p of a layer's sequence panel holds its states after p positions (block 0 the state before): operand of the next
 // position and, as a whole, of the next layer's input GEMM.  Sources longer than the panels are taken in chunks.

@@ -902,7 +902,7 @@ __device__ __forceinline__ bool mbar_wait_sleepy(uint32_t bar, uint32_t parity, 
 // ---- kernel -------------------------------------------------------------------------------
 template <int NT, int BKT, int FMT, class Epi>
 __global__ void __launch_bounds__(kThreadsMain, 1)
-gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, int STAGES, int kDrainEvery, Epi epi,
+gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int a_row0, int BN, int STAGES, int kDrainEvery, Epi epi,
                int* __restrict__ err_flag, int splits, float* __restrict__ ws, int* __restrict__ tile_counters) {
   constexpr int PC = product_code(NT, FMT);
   constexpr int NP = num_products(PC);
@@ -949,9 +949,10 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int BN, 
   if (warp == 0) {
     // Producer.
     const bool one = elect_one();
+    const int ya = a_row0 + m0;      // (rows past the product's last one are read and not used)
     auto load_a = [&](int kb, uint32_t st, uint32_t fb) {
 #pragma unroll
-      for (int t = 0; t < NT; ++t) tma_load_2d(st + t * A_BYTES, &tm.a[t], (kb0 + kb) * BK, m0, fb);
+      for (int t = 0; t < NT; ++t) tma_load_2d(st + t * A_BYTES, &tm.a[t], (kb0 + kb) * BK, ya, fb);
     };
     auto load_b = [&](int kb, uint32_t st, uint32_t fb) {
 #pragma unroll
@@ -1432,36 +1433,37 @@ inline cudaError_t ensure_smem_optin(Kernel* kernel, bool* done_per_device, int 
 
 template <int NT, int BKT, int FMT, class Epi>
 inline cudaError_t launch_gemm_tc_nt(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
-                                     cudaStream_t st, float* ws, int* counters) {
+                                     cudaStream_t st, float* ws, int* counters, int a_row0) {
   static bool optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_kernel<NT, BKT, FMT, Epi>, optin_done); e != cudaSuccess) return e;
   const int splits = (sh.splits > 1 && ws && counters) ? sh.splits : 1;
   dim3 grid((M + BM - 1) / BM, (N + sh.bn - 1) / sh.bn, splits);
   int drain = (sh.drain > 0 ? sh.drain : kDrainDefault) * 32 / BKT;
   if (drain < 1) drain = 1;
-  return launch_k(sh.pdl != 0, gemm_tc_kernel<NT, BKT, FMT, Epi>, grid, dim3(kThreadsMain), (size_t)sh.smem_bytes, st, tm, M, N, K, sh.bn,
+  return launch_k(sh.pdl != 0, gemm_tc_kernel<NT, BKT, FMT, Epi>, grid, dim3(kThreadsMain), (size_t)sh.smem_bytes, st, tm, M, N, K, a_row0, sh.bn,
                   sh.stages, drain, epi, err_flag, splits, splits > 1 ? ws : (float*)nullptr, counters);
 }
+// a_row0: first row of the product in the activations' tensor map
 template <class Epi>
 inline cudaError_t launch_gemm_tc(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
-                                  cudaStream_t st, float* ws = nullptr, int* counters = nullptr) {
+                                  cudaStream_t st, float* ws = nullptr, int* counters = nullptr, int a_row0 = 0) {
   if (sh.fmt == 1) {
     if (sh.nt == 1) {
-      if (sh.bk == 64) return launch_gemm_tc_nt<1, 64, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
-      return launch_gemm_tc_nt<1, 32, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
+      if (sh.bk == 64) return launch_gemm_tc_nt<1, 64, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
+      return launch_gemm_tc_nt<1, 32, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
     }
     if (sh.nt != 2) return cudaErrorInvalidValue;
-    if (sh.bk == 64) return launch_gemm_tc_nt<2, 64, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
-    return launch_gemm_tc_nt<2, 32, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
+    if (sh.bk == 64) return launch_gemm_tc_nt<2, 64, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
+    return launch_gemm_tc_nt<2, 32, 1, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
   }
   if (sh.bk == 64) {
-    if (sh.nt == 2) return launch_gemm_tc_nt<2, 64, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
-    if (sh.nt == 1) return launch_gemm_tc_nt<1, 64, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
+    if (sh.nt == 2) return launch_gemm_tc_nt<2, 64, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
+    if (sh.nt == 1) return launch_gemm_tc_nt<1, 64, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
     return cudaErrorInvalidValue;  // three planes of 128-byte rows leave room for one stage only
   }
-  if (sh.nt == 3) return launch_gemm_tc_nt<3, 32, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
-  if (sh.nt == 2) return launch_gemm_tc_nt<2, 32, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
-  return launch_gemm_tc_nt<1, 32, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters);
+  if (sh.nt == 3) return launch_gemm_tc_nt<3, 32, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
+  if (sh.nt == 2) return launch_gemm_tc_nt<2, 32, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
+  return launch_gemm_tc_nt<1, 32, 0, Epi>(tm, M, N, K, sh, epi, err_flag, st, ws, counters, a_row0);
 }
 
 // Persistent launch (see gemm_tc_persist_kernel): one or two planes per operand, no split-K.  One-plane

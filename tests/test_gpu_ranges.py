@@ -1,0 +1,36 @@
+"""GPU tests at the far ends of what a handle takes: sizes and batches that no named configuration reaches."""
+import numpy as np
+import pytest
+
+from linmt_b200 import synth
+from parity import RTOL_FP32, compare_forced
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("L,H,counts", [(2, 1600, (64, 49, 48)), (1, 2432, (1, 17, 64))])
+def test_hidden_sizes_beyond_the_few_rows_kernel(cuda_lib, L, H, counts):
+    """The weight-streaming kernel declines K slices of more than three k-blocks per leading accumulator: a recurrent
+    product of 1600 units from 49 sentences on, of 2432 for any number.  The encoder's per-position products then run
+    elsewhere, on rows in the middle of a panel.  Decode (forced) and scores against the CUDA-core path."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(L, H, 100, 60, 1)
+    # Bound of the comparison: a CUDA-core logit is within 4e-6 of its terms' absolute sum, 0.04 x 0.5 x 2432 = 49, of the
+    # exact one, 2e-4; log-probabilities of 100 words are near -4.6, 1e-4 of which is 4.6e-4.  (The peaked family's output
+    # weights are 30 times as large, and the bound 6e-3 against rows of 40: 1.3e-4 relative was seen.)
+    blob = synth.make_blob(d, 3)
+    kw = dict(beam=2, max_batch=64, max_src_len=8, max_steps=12, cp_beta=0.0)
+    tc = decoder.Decoder(d, [blob], **kw)
+    ref = decoder.Decoder(d, [blob], gemm_path="simt", **kw)
+    for n in counts:
+        sents = synth.make_sentences(n, 2, 7, d.Vs, 1.1, n, lambda s: s + 2)
+        r = ref.decode(sents, trace=True)
+        e = tc.decode(sents, trace=True, force=r)
+        worst, bad, skipped, compared = compare_forced(e, r, sents.steps, src_len=sents.lengths())
+        assert worst <= RTOL_FP32 and bad == 0 and skipped <= 0.1 * (skipped + compared), (n, worst, bad, skipped, compared)
+        rng = np.random.default_rng(n)
+        targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 10, size=n)]
+        a, b = tc.score(sents, targets), ref.score(sents, targets)
+        scale = np.abs(b[1]).max(axis=1, keepdims=True)
+        assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), (n, float((np.abs(a[1] - b[1]) / scale).max()))
+    tc.close(); ref.close()
