@@ -16,6 +16,7 @@
 #include <mutex>
 #include <numeric>
 #include <thread>
+#include <type_traits>
 
 #include "gemm_simt.cuh"
 #include "gemm_tc_rows.cuh"
@@ -489,17 +490,25 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
   const int ldp = att_merge_ ? 3 * Hp : 2 * Hp;
   // fold: the weighted sum runs over W_c1 . hs and the kernel writes htilde (ctx_planes = the htilde panel)
   const AttFold af = fold ? AttFold{s.hs_wc1, s.proj + 2 * Hp, 3 * Hp, m.att_bout} : AttFold{nullptr, nullptr, 0, nullptr};
-  auto launch = [&](auto kernel, int threads, int G, int groups, int positions) {
-    return tc::launch_k(pdl_, kernel, dim3(rows / kb * groups), dim3(threads), attention_smem(G, threads, Hp, positions), stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
+  auto launch = [&](auto group, auto block, int groups, int positions) {
+    constexpr int G = decltype(group)::value, kThreads = decltype(block)::value;
+    const size_t smem = attention_smem(G, kThreads, Hp, positions);
+    if (cudaError_t e = tc::allow_smem<attention_kernel<G, kThreads>>(smem); e != cudaSuccess) return e;
+    return tc::launch_k(pdl_, attention_kernel<G, kThreads>, dim3(rows / kb * groups), dim3(kThreads), smem, stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
                         (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, kb, groups, hs_sent_, hs_pos_, (int)opt.attention_mode,
                         (int)opt.attention_d, ra, rl, rv, ctx_planes, nt, rec_win, ens_member_code(mi), at, af);
   };
+  constexpr std::integral_constant<int, 1> one{};
+  constexpr std::integral_constant<int, 2> two{};
+  constexpr std::integral_constant<int, 3> three{};
+  constexpr std::integral_constant<int, 512> half{};
+  constexpr std::integral_constant<int, 1024> whole{};
   // A CTA of 1024 threads per row while that leaves SMs empty, then groups of beams: as many as fill the two CTAs of 512
   // threads that an SM holds, at most three beams in one (1536 rows: 35.2, 32.5, 48.8, 39.7 us with 2, 3, 4, 6: registers
   // spill and the windows of more beams cover more of the source), and fewer where wide models or long sources need the
   // shared memory.  A group's positions are those of all its windows, up to the whole source.
   if (rows <= n_sm_) {
-    CK(launch(attention_kernel<1, 1024>, 1024, 1, kb, win));
+    CK(launch(one, whole, kb, win));
   } else {
     const int sents = rows / kb, src = (int)opt.max_src_len;
     const int want = std::max(1, 2 * n_sm_ / sents);
@@ -508,9 +517,9 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
     const int groups = (kb + per - 1) / per;
     per = (kb + groups - 1) / groups;
     switch (per) {
-      case 1: CK(launch(attention_kernel<1, 512>, 512, 1, groups, win)); break;
-      case 2: CK(launch(attention_kernel<2, 512>, 512, 2, groups, src)); break;
-      default: CK(launch(attention_kernel<3, 512>, 512, 3, groups, src)); break;
+      case 1: CK(launch(one, half, groups, win)); break;
+      case 2: CK(launch(two, half, groups, src)); break;
+      default: CK(launch(three, half, groups, src)); break;
     }
   }
   LAUNCHED();

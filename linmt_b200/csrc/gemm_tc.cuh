@@ -1431,6 +1431,18 @@ inline cudaError_t ensure_smem_optin(Kernel* kernel, bool* done_per_device, int 
   return cudaSuccess;
 }
 
+// The same for kernels that have static shared memory as well and rarely need so much: asked for at the first launch that
+// could pass 48 KB with it (static: at most 24 KB in every kernel of step_kernels.cuh).
+constexpr int kSmemPerBlock = 227 * 1024;
+template <auto Kernel>
+inline cudaError_t allow_smem(size_t dynamic_bytes) {
+  if (dynamic_bytes <= 24 * 1024) return cudaSuccess;
+  static bool done[kMaxDevices] = {};
+  cudaFuncAttributes attr;
+  if (cudaError_t e = cudaFuncGetAttributes(&attr, Kernel); e != cudaSuccess) return e;
+  return ensure_smem_optin(Kernel, done, kSmemPerBlock - (int)attr.sharedSizeBytes);
+}
+
 template <int NT, int BKT, int FMT, class Epi>
 inline cudaError_t launch_gemm_tc_nt(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
                                      cudaStream_t st, float* ws, int* counters, int a_row0) {

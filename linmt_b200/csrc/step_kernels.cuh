@@ -478,7 +478,9 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
   }
 }
 
-// `positions`: the window of one beam, the whole source where windows are joined
+// `positions`: the window of one beam, the whole source where windows are joined.  Wide models and global attention over
+// sources of more than about 9000 words pass 48 KB and are launched with the opt-in (tc::allow_smem): up to 54,000
+// floats for the widest vector and the window of a row together.
 inline size_t attention_smem(int G, int threads, int Hp, int positions) {
   const int parts = threads > 512 ? (threads / 256 - 1) * 1024 : 0, gp = G == 3 ? 4 : G;
   return sizeof(float) * (size_t)(G * (Hp > parts ? Hp : parts) + gp * positions);

@@ -34,3 +34,22 @@ def test_hidden_sizes_beyond_the_few_rows_kernel(cuda_lib, L, H, counts):
         scale = np.abs(b[1]).max(axis=1, keepdims=True)
         assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), (n, float((np.abs(a[1] - b[1]) / scale).max()))
     tc.close(); ref.close()
+
+
+@pytest.mark.parametrize("n", [1, 75])     # two rows, a CTA of 1024 threads each; 150 rows, CTAs of 512 threads
+def test_global_attention_over_long_sources(oracle, cuda_lib, n):
+    """A handle for sources of up to 12,250 words: with a row's vector, its scores pass 48 KB of shared memory."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(1, 64, 200, 100, 1)
+    blob = synth.make_blob(d, 8)
+    rng = np.random.default_rng(n)
+    lens = np.concatenate([[12250], rng.integers(2, 20, size=n - 1)]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    sents = synth.Sentences(synth.zipf_ids(rng, int(off[-1]), 1, d.Vs, 1.1), off, np.full(n, 4, np.int32))
+    kw = dict(beam=2, attention="global_general", cp_beta=0.0, min_ratio=0.0)
+    o = oracle.decode(d, [blob], sents, trace=True, **kw)
+    dec = decoder.Decoder(d, [blob], max_batch=n, max_src_len=12250, max_steps=8, **kw)
+    e = dec.decode(sents, trace=True, force=o)
+    worst, bad, skipped, compared = compare_forced(e, o, sents.steps, src_len=sents.lengths())
+    assert worst <= RTOL_FP32 and bad == 0 and skipped == 0, (worst, bad, skipped, compared)
+    dec.close()
