@@ -339,6 +339,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   }
   // what one copy brings in and what one memset clears at the start of a decode lies together
   DA(d_off_, 4 * (B + 1)); d_len_ = d_off_ + (B + 1); d_steps_ = d_off_ + 2 * (B + 1); d_orig_ = d_off_ + 3 * (B + 1);
+  CK(cudaMemset(d_off_, 0, sizeof(int32_t) * 4 * (B + 1)));   // (the attention's prefetch may go by a length before the first copy)
   CK(cudaMallocHost(&h_meta_, sizeof(int32_t) * (4 * (B + 1) + 1)));
   h_err_ = h_meta_ + 4 * (B + 1);
   DA(d_tok_, 3 * (size_t)R + B); d_parent_ = d_tok_ + R; d_score_ = reinterpret_cast<float*>(d_tok_ + 2 * (size_t)R); d_fin_n_ = d_tok_ + 3 * (size_t)R;

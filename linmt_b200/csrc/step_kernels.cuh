@@ -222,10 +222,11 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
   const int sent = blockIdx.x / groups, q = blockIdx.x - sent * groups;
   const int per = (k + groups - 1) / groups, b0 = q * per;
   const int nb = k - b0 < per ? k - b0 : per;          // beams of this group, 1 .. G
-  const int S = src_len[sent];
   if (THREADS > 512) {
     // Few rows: the weights of a step have displaced the encoder's states from L2.  While the projection runs, the CTAs
-    // of a sentence ask for them again (a hint; nothing is read here, so the length may still be an earlier step's).
+    // of a sentence ask for them again.  A hint: no state is read here, and the length this goes by may be an earlier
+    // batch's (or the zero it starts as), which names rows of the same buffer; the one that counts is read below.
+    const int S = src_len[sent];
     const char* h0 = reinterpret_cast<const char*>(hs + (size_t)sent * hs_sent * Hp);
     const char* c0 = fold.cs ? reinterpret_cast<const char*>(fold.cs + (size_t)sent * hs_sent * Hp) : nullptr;
     const int lines = Hp / 32;
@@ -237,6 +238,8 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
     }
   }
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
+  int S;      // (from L2 and not moved: the value above may be in L1)
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(S) : "l"(src_len + sent) : "memory");
   extern __shared__ __align__(16) float sm[];
   float* su = sm;                                           // [G][Hp] what the states are multiplied with, and then
   float4* csum = reinterpret_cast<float4*>(sm);             // [kRanges - 1][256] partial contexts (G = 1)

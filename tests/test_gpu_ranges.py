@@ -53,3 +53,25 @@ def test_global_attention_over_long_sources(oracle, cuda_lib, n):
     worst, bad, skipped, compared = compare_forced(e, o, sents.steps, src_len=sents.lengths())
     assert worst <= RTOL_FP32 and bad == 0 and skipped == 0, (worst, bad, skipped, compared)
     dec.close()
+
+
+@pytest.mark.parametrize("attention", ["local_p_general", "global_general"])
+def test_batches_of_other_lengths_on_one_handle(cuda_lib, attention):
+    """The source lengths of a batch replace those of the batch before while kernels overlap at their boundaries: results
+    on a handle that has just decoded longer or shorter sentences are those of a fresh handle, to the bit."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, 128, 500, 300, 1)
+    blob = synth.make_blob(d, 5)
+    kw = dict(beam=3, attention=attention, print_info=True, cp_beta=0.2, max_batch=8, max_src_len=64, max_steps=64)
+    batches = [synth.make_sentences(n, lo, hi, d.Vs, 1.1, n, lambda s: 12) for n, lo, hi in ((8, 50, 60), (8, 1, 3), (3, 30, 64), (8, 20, 25))]
+    fresh = []
+    for b in batches:
+        dec = decoder.Decoder(d, [blob], **kw)
+        fresh.append(dec.decode(b, want_align=True))
+        dec.close()
+    kept = decoder.Decoder(d, [blob], **kw)
+    for i in (0, 1, 2, 3, 1, 0, 3, 2):
+        out = kept.decode(batches[i], want_align=True)
+        for key in ("tok", "len", "score", "vit", "align"):
+            assert np.array_equal(out[key], fresh[i][key]), (i, key)
+    kept.close()
