@@ -258,6 +258,17 @@ int linmt_decode_file(linmt_engine* e, const char* in_path, const char* out_path
  * gemm_path: LINMT_GEMM_SIMT or LINMT_GEMM_TENSOR; precision: LINMT_PREC_*. */
 int linmt_k_gemm(const float* X, const float* W, float* Y, int32_t R, int32_t K, int32_t N, int32_t gemm_path,
                  int32_t precision, int32_t device);
+/* The vocabulary product of a step as the engine runs it, and the softmax behind it: Y = X[R][K] . W[K][V] + bias, the
+ * statistics that the product leaves per block of columns, and every row's top-kk log-probabilities.
+ *   gemm_path   LINMT_GEMM_AUTO (fp32: one fp16 product, the values rounded to fp16, the candidates recomputed) or
+ *               LINMT_GEMM_TENSOR (fp32: three products); LINMT_PREC_BF16: one bf16 product either way
+ *   block_max, block_sum  [R][ld], ld = 4 * ceil(Vp / 48) + 4, Vp = V rounded up to 128: maximum of a block and sum of
+ *               exp(value - maximum) over it.  Block i covers columns [c, c + info[3]) of tile i / 4, c = (i % 4) * info[3],
+ *               as far as the tile (info[2] columns) and V go
+ *   info [5]    kernel that ran (0 one tile per CTA, 1 few rows, 2 CTA pairs, 3 persistent, 4 persistent pairs), blocks,
+ *               columns of a tile and of a block, 1 if the sums were left too */
+int linmt_k_logits(const float* X, const float* W, const float* bias, int32_t R, int32_t K, int32_t V, int32_t gemm_path, int32_t precision, int32_t kk,
+                   float* Y, float* block_max, float* block_sum, int32_t* info, int32_t* idx, float* logp, float* eos_logp, int32_t device);
 /* Per-row log-softmax statistics and top-kk of logits[R][V]: replaces the softmax kernel
  * (src/deep_rnn_kernel.h:352-429) plus the per-beam top-(k+1) scan of
  * src/decoder.h:401-410.  idx/logp are [R][kk], eos_logp [R]. */

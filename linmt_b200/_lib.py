@@ -37,7 +37,7 @@ class StatsC(C.Structure):
 EXPORTS = ["python_decoder_init", "python_decoder_do_job", "linmt_default_options", "linmt_blob_floats",
            "linmt_create_from_weights", "linmt_create_from_weights_on", "linmt_device_count", "linmt_front_error", "linmt_create", "linmt_destroy", "linmt_last_error", "linmt_beam",
            "linmt_decode_batch", "linmt_decode_batch_device", "linmt_get_stats", "linmt_set_kernel_timing", "linmt_kernel_times",
-           "linmt_translate", "linmt_k_gemm", "linmt_k_softmax_topk", "linmt_gemm_f32_noalloc", "linmt_decode_file", "linmt_score_batch",
+           "linmt_translate", "linmt_k_gemm", "linmt_k_logits", "linmt_k_softmax_topk", "linmt_gemm_f32_noalloc", "linmt_decode_file", "linmt_score_batch",
            "linmt_read_model_file", "python_unk_init", "python_unk_do_job", "linmt_unk_create", "linmt_unk_process", "linmt_unk_destroy"]
 
 _lib = None
@@ -83,6 +83,7 @@ def load():
     lib.linmt_translate.restype = C.c_char_p
     lib.linmt_k_gemm.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                  C.c_int32, C.c_int32]
+    lib.linmt_k_logits.argtypes = [C.c_void_p] * 3 + [C.c_int32] * 6 + [C.c_void_p] * 7 + [C.c_int32]
     lib.linmt_k_softmax_topk.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p,
                                          C.c_void_p, C.c_int32]
     lib.linmt_gemm_f32_noalloc.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32]

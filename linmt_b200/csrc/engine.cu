@@ -350,7 +350,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   DA(d_fin_score_, (size_t)B * fin_cap); DA(d_fin_final_, (size_t)B * fin_cap);
   if (nm > 1) DA(d_combined_, (size_t)R * Vp);
   DA(d_cand_idx_, (size_t)R * kk); DA(d_cand_logp_, (size_t)R * kk); DA(d_eos_logp_, R); DA(d_row_stats_, 2 * (size_t)R);
-  pmax_ld_ = 4 * ((Vp + 47) / 48) + 4;   // four column blocks per tile, tiles at least 48 wide
+  pmax_ld_ = logit_blocks_ld(Vp);
   DA(d_pmax_, (size_t)nm * R * pmax_ld_);    // per member
   DA(d_psum_, (size_t)nm * R * pmax_ld_);
   if (o.print_info) {
@@ -528,14 +528,8 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
 }
 
 // Softmax statistics and top-k of rows whose logits vocab_gemm has just produced, from the block statistics it left if it did.
-cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, const float* pmax, const float* psum, int rows, const TopkOut& o, int normalise,
-                                 const TopkRefine* rf, const SelectArgs& sel) {
-  if (!logits16_) logits16 = nullptr;
-  if (!pblocks_) return launch_softmax_topk(logits, Vp, V, kk, rows, o, normalise, stream, pdl_, pmax, pmax_ld_, pmax_slots_, rf, logits16, sel);
-  const LogitBlocks bl{pmax, psum, pmax_ld_, pmax_slots_, pmax_tile_, pmax_part_};
-  const bool wide = rows <= n_sm_;
-  return tc::launch_k(pdl_, wide ? topk_blocks_kernel<1024> : topk_blocks_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256), topk_blocks_smem(bl.n, rf ? rf->K : 0), stream,
-                      logits, logits16, Vp, V, kk, o, normalise, bl, rf ? *rf : TopkRefine{}, sel);
+cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel) {
+  return launch_topk(logits, logits16_ ? logits16 : nullptr, Vp, V, kk, rows, n_sm_, o, normalise, blocks_, rf, sel, stream, pdl_);
 }
 
 TopkRefine Engine::refinement(const tc::Planes& ht) const {
@@ -546,7 +540,7 @@ TopkRefine Engine::refinement(const tc::Planes& ht) const {
   rf.b0 = reinterpret_cast<const __half*>(m.p_voc_w.p[0]); rf.b1 = reinterpret_cast<const __half*>(m.p_voc_w.p[1]);
   rf.ldb = m.p_voc_w.ld;
   rf.bias = m.voc_b; rf.K = Hp;
-  rf.eps_coef = 1.1f * (1.0f / 1024.0f) * m.voc_wnorm_max;
+  rf.eps_coef = refine_eps(m.voc_wnorm_max);
   return rf;
 }
 
@@ -567,7 +561,7 @@ int Engine::step_tail(int t, int rows) {
       if (refine_) rf = refinement(tc_states_[0].panel_ht);
       if (refine_) trace_dev_.rf = rf;
       sel.tr = trace_dev_;
-      CK(softmax_topk(s.logits, s.logits16, d_pmax_, d_psum_, rows, o, 1, refine_ ? &rf : nullptr, sel));
+      CK(softmax_topk(s.logits, s.logits16, rows, o, 1, refine_ ? &rf : nullptr, sel));
     } else {
       // EnsembleFactory::EnsemblesModels (src/decoder.h:1910-1931): mean of the members'
       // probabilities, renormalised -- written as log(mean p) so that the log-softmax of the
@@ -586,7 +580,7 @@ int Engine::step_tail(int t, int rows) {
         CK(launch_softmax_topk(d_combined_, Vp, V, kk, rows, o, opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0, stream, pdl_, nullptr, 0, 0, nullptr, nullptr, sel));
       } else {
         const bool wide = rows <= n_sm_;
-        const LogitBlocks bl{d_pmax_, d_psum_, pmax_ld_, pblocks_ ? pmax_slots_ : 0, pmax_tile_, pmax_part_};
+        const LogitBlocks bl{d_pmax_, d_psum_, pmax_ld_, blocks_.sum ? blocks_.n : 0, blocks_.tile, blocks_.part};
         CK(tc::launch_k(pdl_, wide ? ensemble_topk_kernel<1024> : ensemble_topk_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256), smem, stream, er, Vp, V, kk,
                         (int)opt.ensemble_mode, o, bl, (long long)R * pmax_ld_, d_combined_, sel));
       }

@@ -126,10 +126,8 @@ class Engine {
   // a step of scoring: the tokens read, where every member's htilde goes and where the previous step's is
   struct ScoreStep { const int32_t* tok; const tc::Planes* ht; const tc::Planes* ht_prev; };
   int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr);
-  void note_blocks(float** pmax, float** psum, int ld, int N, int K, int tile, int part);
   int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum);
-  cudaError_t softmax_topk(const float* logits, const __half* logits16, const float* pmax, const float* psum, int rows, const TopkOut& o, int normalise,
-                           const TopkRefine* rf, const SelectArgs& sel);
+  cudaError_t softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel);
   int score_core_tc(int n, int Smax, const std::vector<int>& n_act, const int32_t* d_tok, const int32_t* d_gold, float* d_logp);
   int reserve_score(size_t rows);
   TopkRefine refinement(const tc::Planes& ht) const;    // of one-product logits of these attentional states
@@ -141,8 +139,7 @@ class Engine {
   int build_xw_tables();   // dec_xw of every model (tensor path, xw_table_)
   int alloc_planes(tc::Planes& p, size_t rows, int ld);
   int to_planes(const std::vector<float>& host, size_t rows, int ld, tc::Planes& dst);
-  const CUtensorMap* a_maps(const tc::Planes& p, int col0, int rows_cap, int K, int bk);
-  const CUtensorMap* b_maps(const tc::Planes& p, int rows, int K, int bn, int bk);
+  const CUtensorMap* maps(const tc::Planes& p, int col0, int rows, int K, int box_rows, int bk);
   template <class Epi>
   int tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e, int nt = 0, int drain = 0, int x_row0 = 0);
 
@@ -205,9 +202,7 @@ class Engine {
   float* d_pmax_ = nullptr;   // [members][R][pmax_ld_] block maxima of the logits, by-product of the vocabulary GEMM ...
   float* d_psum_ = nullptr;   // ... and the blocks' sums of exp(z - maximum)
   int pmax_ld_ = 0;
-  bool pblocks_ = false;      // the last vocabulary GEMM left both, for pmax_slots_ blocks: four of pmax_part_ columns per tile of pmax_tile_
-  int pmax_tile_ = 1, pmax_part_ = 1;
-  int pmax_slots_ = 0;        // slots the last vocabulary GEMM filled (0 = none: the softmax finds its own maxima)
+  LogitBlocks blocks_{};      // what the last vocabulary GEMM left of them
   // alignment records (print_info)
   float* d_rec_align_ = nullptr;
   int32_t *d_rec_lo_ = nullptr, *d_rec_vit_ = nullptr;

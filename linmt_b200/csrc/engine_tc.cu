@@ -6,9 +6,8 @@
 #include <algorithm>
 
 #include "engine.h"
+#include "gemm_plan.cuh"
 #include "gemm_tc.cuh"
-#include "gemm_tc_pair.cuh"
-#include "gemm_tc_rows.cuh"
 #include "step_kernels.cuh"
 
 namespace linmt {
@@ -82,164 +81,47 @@ int Engine::alloc_state_tc(TcState& s) {
   return LINMT_OK;
 }
 
-// Tensor maps are built once per (buffer view, shape) and reused by every launch.
-const CUtensorMap* Engine::a_maps(const tc::Planes& p, int col0, int rows_cap, int K, int bk) {
-  auto key = std::make_tuple((const void*)(p.p[0] + col0), rows_cap, K, p.ld, (int)tc::BM + 1000 * bk);
+// Tensor maps are built once per (buffer view, box) and reused by every launch.
+const CUtensorMap* Engine::maps(const tc::Planes& p, int col0, int rows, int K, int box_rows, int bk) {
+  auto key = std::make_tuple((const void*)(p.p[0] + col0), rows, K, p.ld, box_rows + 1000 * bk);
   auto it = tmap_cache_.find(key);
   if (it == tmap_cache_.end()) {
     std::array<CUtensorMap, 3> m{};
     for (int t = 0; t < nt_; ++t)
-      if (!tc::make_tmap(&m[t], p.p[t] + col0, rows_cap, K, p.ld, tc::BM, bk)) return nullptr;
-    it = tmap_cache_.emplace(key, m).first;
-  }
-  return it->second.data();
-}
-const CUtensorMap* Engine::b_maps(const tc::Planes& p, int rows, int K, int bn, int bk) {
-  auto key = std::make_tuple((const void*)p.p[0], rows, K, p.ld, bn + 1000 * bk);
-  auto it = tmap_cache_.find(key);
-  if (it == tmap_cache_.end()) {
-    std::array<CUtensorMap, 3> m{};
-    for (int t = 0; t < nt_; ++t)
-      if (!tc::make_tmap(&m[t], p.p[t], rows, K, p.ld, bn, bk)) return nullptr;
+      if (!tc::make_tmap(&m[t], p.p[t] + col0, rows, K, p.ld, box_rows, bk)) return nullptr;
     it = tmap_cache_.emplace(key, m).first;
   }
   return it->second.data();
 }
 
-// C[M][N] = A[:, a_col0 : a_col0+K] . W[N][K]^T with the tile width chosen for this shape.
+// C[M][N] = A[:, a_col0 : a_col0+K] . W[N][K]^T on the kernel and in the shape that plan_gemm chooses.
 template <class Epi>
 int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e_in, int nt, int drain, int x_row0) {
   Epi e = e_in;
   if (nt <= 0 || nt > nt_) nt = nt_;
-  int bn = 0, splits = 1;
+  tc::GemmLimits lim;
+  lim.n_sm = n_sm_; lim.parts = ws_parts_; lim.rows = rows_; lim.pair = pair_; lim.persist = persist_;
   // a layer's slice of the split-K workspace: whole 256-byte units, so that every slice starts aligned for the
   // 16-byte partial-tile stores whatever the number of layers sharing it
-  const size_t ws_floats = (kSplitKWsFloats / ws_parts_) & ~(size_t)63;
-  const int max_tiles = kSplitKMaxTiles / ws_parts_;
-  // The encoder runs its L layers as a wavefront on L streams: a GEMM sized for the whole machine would only
-  // queue behind its neighbours, so there each one is shaped for its share of the SMs and they run side by side.
-  const int sm_budget = ws_parts_ > 1 ? (n_sm_ / ws_parts_ > 0 ? n_sm_ / ws_parts_ : 1) : n_sm_;
-  tc::pick_shape(M, N, K, nt, sm_budget, ws_floats, max_tiles, &bn, &splits, fmt_);
-  // one plane (bf16 precision): 64-deep stages with 128-byte rows halve the per-k-block overheads
-  // (measured 1.5x on the gate GEMMs); with split operands only 32-deep stages leave room for a ring
-  // the f16 pair: 64-deep stages as well, except for a weight matrix far larger than L2 under
-  // the widest tiles, where only two such stages fit and four 32-deep ones hide DRAM latency better
-  // (vocabulary GEMM: 143 us against 149 us)
-  int bk = (nt == 1) ? 64 : 32;
-  if (fmt_ == 1 && nt == 2 && K % 64 == 0) bk = (bn >= 240 && (size_t)N * K * 4 > ((size_t)96 << 20)) ? 32 : 64;
-  // CTA pairs (gemm_tc_pair.cuh) where the one-tile shape has room for two stages only: an even number of row
-  // tiles (an odd one is rounded up, which must still fit one wave), split operands, 64-deep stages, K not split
-  const int mt = (M + tc::BM - 1) / tc::BM;
-  // (a row offset is for the few-rows kernel and the one-tile kernel, which takes it where the former declines; its
-  // products are those of up to 64 sentences, a single row tile)
-  const bool may_pair = ws_parts_ == 1 && x_row0 == 0;
-  // The many-wave one-plane logits GEMM has a persistent pair form as well (measured at K = 1024, against one tile per CTA:
-  // N = 30016 23.6 / 29.5 us at 256 rows, 51 / 57 at 640, 55 / 71 at 768; N = 80000 104 / 124 at 512; three row tiles, a
-  // quarter of the pair idle, are equal), with 208-wide tiles.
-  const bool one_plane_logits = nt == 1 && Epi::kHasPmax;   // the fp32-output GEMMs: vocabulary projection
-  // (the block statistics depend on the tile width, so the width is the pair's whether or not pairs may run)
-  bool ppair = false;
-  if (one_plane_logits && splits == 1 && bk == 64 && mt >= 2 && may_pair &&
-      (long)mt * ((N + bn - 1) / bn) > n_sm_ && (long)((mt + 1) / 2) * ((N + 207) / 208) > n_sm_ / 2) {
-    ppair = pair_ && persist_;
-    bn = 208;
-  }
-  // ... and the gate product of one plane, where one tile per CTA is more than one wave (beyond 1024 rows; measured at N =
-  // 4096, K = 2048: 22.4 / 28.3 us at 1280 rows, 25.7 / 30.6 at 1536): rounds of 3.9 + 0.0215 * width us, and a prologue
-  // and last epilogue of 4 + 0.033 * width.
-  if (Epi::kHasBlock && !Epi::kHasPmax && pair_ && persist_ && nt == 1 && splits == 1 && bk == 64 && mt > 8 && may_pair) {
-    double best = 1e30;
-    for (int w = 96; w <= 256; w += 16) {
-      const long t = (long)((mt + 1) / 2) * ((N + w - 1) / w), rounds = (t + n_sm_ / 2 - 1) / (n_sm_ / 2);
-      const double cost = 4.0 + 0.033 * w + rounds * (3.9 + 0.0215 * w) * K / 2048.0;
-      if (cost < best) { best = cost; bn = w; }
-    }
-    ppair = true;
-  }
-  const long ntile_cols = (N + bn - 1) / bn;
-  const bool pair = ppair || (pair_ && fmt_ == 1 && nt == 2 && bk == 64 && splits == 1 && mt >= 2 && bn % 16 == 0 &&
-                    tc::make_shape(bn, nt, bk, fmt_).stages < 3 && (long)((mt + 1) & ~1) * ntile_cols <= n_sm_ && may_pair);
-  // Few rows: the weight-streaming kernel (gemm_tc_rows.cuh), where the rows are the narrow side of the MMA.  Its gain
-  // shrinks as the rows fill the 128-row tile (gate product, us against this file's one-tile kernel: 8.7 / 13.8 at 12
-  // rows, 10.2 / 14.8 at 32, 11.4 / 15.8 at 64; bf16 6.3 / 13.0 at 12, 9.0 / 13.0 at 64); a product of many column
-  // tiles and one k slice is finished by too few warps for more than 48 rows of the f16 pair (one plane, vocabulary with
-  // block statistics in the decode: 12.7 us at 12 rows, 18.9 at 64 against 19.6 in the one-tile kernel).
-  {
-    tc::RowsShape rs;
-    if (rows_ && ws_parts_ == 1 && M <= tc::kRowsMax && (nt == 1 || M <= 48 || N <= 128 * n_sm_) && tc::make_shape_rows(M, N, K, nt, fmt_, n_sm_, drain >= K / 32, &rs)) {
-      tc::Planes a = A;
-      for (int t = 0; t < 3; ++t) if (a.p[t]) a.p[t] += a_col0;
-      const CUtensorMap* xm = b_maps(a, a_rows_cap, K, rs.rp, 64);
-      const CUtensorMap* wm = b_maps(W, N, K, tc::BM, 64);
-      if (!xm || !wm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
-      tc::TmapSet tm;
-      std::memcpy(tm.a, xm, sizeof(tm.a));
-      std::memcpy(tm.b, wm, sizeof(tm.b));
-      rs.pdl = (pdl_ && pdl_gemm_) ? 1 : 0;
-      if constexpr (Epi::kHasPmax) {
-        if (e.pmax) {      // block maxima of 32 columns
-          note_blocks(&e.pmax, &e.psum, e.pmax_ld, N, K, tc::BM, 32);
-        }
-      }
-      if (nt == 2) CK((tc::launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
-      else if (fmt_ == 1) CK((tc::launch_gemm_tc_rows<1, 1, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
-      else CK((tc::launch_gemm_tc_rows<1, 0, Epi>(tm, M, N, K, rs, e, d_tc_err_, stream, x_row0)));
-      LAUNCHED();
-      return LINMT_OK;
-    }
-  }
-  const CUtensorMap* am = a_maps(A, a_col0, a_rows_cap, K, bk);
-  const CUtensorMap* bm = b_maps(W, N, K, pair ? bn / 2 : bn, bk);
+  lim.ws_floats = (kSplitKWsFloats / ws_parts_) & ~(size_t)63;
+  lim.max_tiles = kSplitKMaxTiles / ws_parts_;
+  const tc::GemmPlan plan = tc::plan_gemm<Epi>(M, N, K, nt, fmt_, drain, x_row0, lim);
+  const CUtensorMap* am = maps(A, a_col0, a_rows_cap, K, plan.a_box, plan.bk);
+  const CUtensorMap* bm = maps(W, 0, N, K, plan.b_box, plan.bk);
   if (!am || !bm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
   tc::TmapSet tm;
   std::memcpy(tm.a, am, sizeof(tm.a));
   std::memcpy(tm.b, bm, sizeof(tm.b));
-  tc::Shape sh = pair ? tc::make_shape_pair(bn, nt, bk, fmt_) : tc::make_shape(bn, nt, bk, fmt_);
-  sh.splits = splits;
-  if (drain > 0) sh.drain = drain;
-  sh.pdl = (pdl_ && pdl_gemm_) ? 1 : 0;
   if constexpr (Epi::kHasPmax) {
-    // block maxima for the softmax: four column blocks per tile; not from the split-K fix-up path
     if (e.pmax) {
-      if (splits > 1) e.pmax = e.psum = nullptr;
-      else note_blocks(&e.pmax, &e.psum, e.pmax_ld, N, K, bn, ((bn >> 4) + 3) / 4 * 16);
+      blocks_ = logit_blocks(e.pmax, e.psum, e.pmax_ld, N, K, plan.stat_tile, plan.stat_part);
+      e.pmax = blocks_.max; e.psum = blocks_.sum;
     }
   }
-  // many waves of tiles whose leading product is one chain: one persistent CTA per SM
-  const long tiles = (long)((M + tc::BM - 1) / tc::BM) * ((N + bn - 1) / bn);
-  if constexpr (Epi::kHasBlock) {
-  if (ppair) {
-    const int pdl = sh.pdl;
-    sh = tc::make_shape_persist_pair(bn, fmt_);
-    sh.pdl = pdl;
-    if (fmt_ == 1) CK((tc::launch_gemm_tc_persist_pair<1, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_)));
-    else CK((tc::launch_gemm_tc_persist_pair<0, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_)));
-    LAUNCHED();
-    ++stats.pair_launches;
-    return LINMT_OK;
-  }
-  }
-  if constexpr (Epi::kHasPmax) {
-  if (persist_ && splits == 1 && x_row0 == 0 && tiles > n_sm_ && ((nt == 2 && drain >= K / 32) || one_plane_logits)) {
-    if (nt == 1) {
-      const int pdl = sh.pdl;
-      sh = tc::make_shape_persist(bn, nt, bk, fmt_);   // a ring of one stage less, staging areas of its own
-      sh.pdl = pdl;
-    }
-    CK(tc::launch_gemm_tc_persist(tm, M, N, K, sh, e, d_tc_err_, stream, n_sm_));
-    LAUNCHED();
-    return LINMT_OK;
-  }
-  }
-  if (pair) {
-    CK((tc::launch_gemm_tc_pair<2, 64, 1, Epi>(tm, M, N, K, sh, e, d_tc_err_, stream, nullptr, nullptr)));
-    LAUNCHED();
-    ++stats.pair_launches;
-    return LINMT_OK;
-  }
-  CK(tc::launch_gemm_tc(tm, M, N, K, sh, e, d_tc_err_, stream, d_splitk_ws_ + (size_t)ws_part_ * ws_floats,
-                        d_splitk_counters_ + ws_part_ * max_tiles, x_row0));
+  CK(tc::launch_planned(plan, tm, M, N, K, nt, fmt_, pdl_ && pdl_gemm_, e, d_tc_err_, stream, n_sm_, d_splitk_ws_ + (size_t)ws_part_ * lim.ws_floats,
+                        d_splitk_counters_ + ws_part_ * lim.max_tiles, x_row0));
   LAUNCHED();
+  if (plan.on_pairs()) ++stats.pair_launches;
   return LINMT_OK;
 }
 
@@ -537,21 +419,12 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   return vocab_gemm(mi, ts.panel_ht, R, rows, s.logits, s.logits16, d_pmax_ + (size_t)mi * R * pmax_ld_, d_psum_ + (size_t)mi * R * pmax_ld_);
 }
 
-// What block statistics a vocabulary GEMM is going to leave: four blocks of `part` columns per tile of `tile`.
-void Engine::note_blocks(float** pmax, float** psum, int ld, int N, int K, int tile, int part) {
-  const int slots = 4 * ((N + tile - 1) / tile);
-  if (slots > ld) { *pmax = *psum = nullptr; return; }
-  pmax_slots_ = slots; pmax_tile_ = tile; pmax_part_ = part;
-  if (topk_blocks_smem(slots, K) > (size_t)kBlocksSmemMax) *psum = nullptr;
-  pblocks_ = *psum != nullptr;
-}
-
 // Logits of `rows` attentional states.
 int Engine::vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum) {
   DevModel& m = models_[mi];
   tc::TcEpiF32 e{m.voc_b, logits, Vp, 0};
   if (logits16_) e.out16 = logits16;   // the softmax of this step is their only reader
-  pmax_slots_ = 0; pblocks_ = false;
+  blocks_ = LogitBlocks{};
   if (pmax_on_ && pmax) { e.pmax = pmax; e.psum = psum; e.pmax_ld = pmax_ld_; e.n_valid = V; }
   // Logits feed only the softmax of their own step: the tensor core's truncation bias over one
   // K = Hp chain (~32 ulp of the accumulator, 2e-7 relative on a log-probability) does not
@@ -607,7 +480,7 @@ int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const 
       logits = score_combined_;
       normalise = opt.ensemble_mode == LINMT_ENS_PROB_MEAN ? 1 : 0;
     }
-    CK(softmax_topk(logits, score_logits16_, score_pmax_, score_psum_, rows, o, normalise, refine_ ? &rf : nullptr, SelectArgs{}));
+    CK(softmax_topk(logits, score_logits16_, rows, o, normalise, refine_ ? &rf : nullptr, SelectArgs{}));
     LAUNCHED();
     CK(tc::launch_k(pdl_, gold_logp_kernel, dim3((rows + 7) / 8), dim3(256), 0, stream, d_gold + r0, rows, logits, Vp, V, (const float*)score_stats_, rf, d_logp + r0));
     LAUNCHED();

@@ -518,6 +518,7 @@ struct TopkRefine {
   float eps_coef;
 };
 constexpr float kPairInv = 1.0f / 2048.0f;
+inline float refine_eps(float w_norm_max) { return 1.1f * (1.0f / 1024.0f) * w_norm_max; }
 
 // ---------------------------------------------------------------------------------------
 // Beam selection for one sentence and one step, all on the device.  Replaces
@@ -1158,7 +1159,7 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
 // grid = rows, dynamic smem = topk_blocks_smem
 constexpr int kBlocksSmemMax = 23 * 1024;   // of dynamic shared memory beside the candidate lists: wider rows are swept
 struct LogitBlocks {
-  const float* max; const float* sum; int ld; int n;
+  float* max; float* sum; int ld; int n;
   int tile, part;     // columns of a GEMM tile and of one of its four blocks (the last one of a tile may be narrower)
 };
 inline size_t topk_blocks_smem(int n_blocks, int refine_K) { return sizeof(float) * (size_t)(2 * n_blocks + refine_K); }
@@ -1300,6 +1301,26 @@ inline cudaError_t launch_softmax_topk(const float* logits, int ld, int V, int k
   if (refine) rf = *refine;
   const size_t smem = rf.a0 ? sizeof(float) * (size_t)rf.K : 0;
   return tc::launch_k(pdl, softmax_topk_kernel, dim3(rows), dim3(256), smem, st, logits, ld, V, kk, out, normalise, pmax, pmax_ld, n_slots, rf, refine ? logits16 : (const __half*)nullptr, sel);
+}
+
+// What block statistics a logits GEMM of N columns is going to leave in rows of `ld` values: four blocks of `part` columns
+// per tile of `tile`.  n = 0: none, sum = null: the maxima only.
+inline LogitBlocks logit_blocks(float* max, float* sum, int ld, int N, int K, int tile, int part) {
+  const int slots = tile > 0 ? 4 * ((N + tile - 1) / tile) : 0;
+  if (!max || slots < 1 || slots > ld) return LogitBlocks{};
+  if (topk_blocks_smem(slots, K) > (size_t)kBlocksSmemMax) sum = nullptr;
+  return LogitBlocks{max, sum, ld, slots, tile, part};
+}
+// Values a row of block statistics has room for: four column blocks per tile, tiles at least 48 wide.
+inline int logit_blocks_ld(int N) { return 4 * ((N + 47) / 48) + 4; }
+
+// Softmax statistics and top-k (and the selection) of rows of logits, from their block statistics where they have them.
+inline cudaError_t launch_topk(const float* logits, const __half* logits16, int ld, int V, int kk, int rows, int n_sm, const TopkOut& o, int normalise,
+                               const LogitBlocks& bl, const TopkRefine* rf, const SelectArgs& sel, cudaStream_t st, bool pdl) {
+  if (!bl.sum) return launch_softmax_topk(logits, ld, V, kk, rows, o, normalise, st, pdl, bl.max, bl.ld, bl.n, rf, logits16, sel);
+  const bool wide = rows <= n_sm;
+  return tc::launch_k(pdl, wide ? topk_blocks_kernel<1024> : topk_blocks_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256), topk_blocks_smem(bl.n, rf ? rf->K : 0), st,
+                      logits, logits16, ld, V, kk, o, normalise, bl, rf ? *rf : TopkRefine{}, sel);
 }
 
 // Log-probability of one given token per row (scoring), from the row's softmax statistics; with one-product logits the

@@ -211,6 +211,30 @@ def k_gemm(X, W, gemm_path="simt", precision="fp32", device=0):
     return Y
 
 
+KERNELS = ("tile", "rows", "pair", "persist", "persist_pair")
+
+
+def k_logits(X, W, bias, kk, gemm_path="auto", precision="fp32", device=0):
+    """The vocabulary product as a step runs it, its block statistics and the softmax behind it: a dict of the logits
+    ``Y``, the ``kernel`` that ran, ``blocks`` (one (first, last + 1) range of columns per block), ``block_max``,
+    ``block_sum`` (None: not left) and ``idx``, ``logp``, ``eos``."""
+    X, W, bias = (np.ascontiguousarray(a, np.float32) for a in (X, W, bias))
+    (R, K), V = X.shape, W.shape[1]
+    ld = 4 * ((-(-V // 128) * 128 + 47) // 48) + 4
+    Y, bm, bs = np.empty((R, V), np.float32), np.empty((R, ld), np.float32), np.empty((R, ld), np.float32)
+    info, idx, lp, eos = np.zeros(5, np.int32), np.empty((R, kk), np.int32), np.empty((R, kk), np.float32), np.empty(R, np.float32)
+    rc = _lib.load().linmt_k_logits(_ptr(X), _ptr(W), _ptr(bias), R, K, V, GEMM[gemm_path], PREC[precision], kk, _ptr(Y), _ptr(bm), _ptr(bs),
+                                    _ptr(info), _ptr(idx), _ptr(lp), _ptr(eos), device)
+    if rc != 0:
+        raise LinmtError(f"linmt_k_logits failed ({rc})")
+    n, tile, part = (int(x) for x in info[1:4])
+    blocks = []
+    for i in range(n):
+        c = i // 4 * tile + i % 4 * part
+        blocks.append((min(c, V), min(c + part, (i // 4 + 1) * tile, V)))
+    return dict(Y=Y, kernel=KERNELS[info[0]], blocks=blocks, block_max=bm[:, :n], block_sum=bs[:, :n] if info[4] else None, idx=idx, logp=lp, eos=eos)
+
+
 def k_softmax_topk(logits, kk, device=0):
     logits = np.ascontiguousarray(logits, np.float32)
     R, V = logits.shape

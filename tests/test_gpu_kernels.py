@@ -108,3 +108,62 @@ def test_gemm_few_rows_vs_float64(cuda_lib, R, K, N, prec, tol):
     ref = X.astype(np.float64) @ W.astype(np.float64)
     scale = np.abs(X).astype(np.float64) @ np.abs(W).astype(np.float64)
     assert (np.abs(Y - ref) <= tol * scale + 1e-7).all(), float((np.abs(Y - ref) / scale).max())
+
+
+@pytest.mark.parametrize("path,prec,R,K,V,kernel", [
+    # one fp16 product, logits rounded to fp16, candidates recomputed (the default): a single column tile, unit edges,
+    # the statistics of 80,000 classes that leave no room for the sums, a partly empty row tile, an odd number of them
+    ("auto", "fp32", 1, 64, 37, "rows"), ("auto", "fp32", 12, 1000, 30000, "rows"), ("auto", "fp32", 64, 1000, 5003, "rows"),
+    ("auto", "fp32", 6, 1000, 80000, "rows"), ("auto", "fp32", 65, 1000, 5003, "tile"), ("auto", "fp32", 128, 1000, 30000, "tile"),
+    ("auto", "fp32", 100, 1000, 40000, "persist"), ("auto", "fp32", 129, 1000, 40000, "persist_pair"), ("auto", "fp32", 300, 1000, 30000, "persist_pair"),
+    # three products
+    ("tensor", "fp32", 12, 1000, 30000, "rows"), ("tensor", "fp32", 128, 1000, 5003, "rows"), ("tensor", "fp32", 65, 1000, 30000, "tile"),
+    ("tensor", "fp32", 129, 1000, 30000, "persist"), ("tensor", "fp32", 768, 1000, 5003, "pair"),
+    # bf16
+    ("auto", "bf16", 48, 1000, 30000, "rows"), ("auto", "bf16", 49, 1000, 30000, "rows"), ("auto", "bf16", 70, 1000, 5003, "tile"),
+    ("auto", "bf16", 100, 1000, 40000, "persist"), ("auto", "bf16", 700, 300, 30000, "persist_pair")])
+def test_vocabulary_product_statistics_and_softmax(cuda_lib, path, prec, R, K, V, kernel):
+    """Every GEMM form a vocabulary product takes: the logits against float64, the maximum of every block of columns (of
+    the values as they are stored) and its sum of exponentials, each column in one block, and the top-kk behind them."""
+    from linmt_b200 import decoder
+    rng = np.random.default_rng(R + K + V)
+    X = rng.uniform(-1, 1, (R, K)).astype(np.float32)
+    W = rng.uniform(-0.08, 0.08, (K, V)).astype(np.float32)
+    bias = rng.uniform(-0.5, 0.5, V).astype(np.float32)
+    kk = min(13, V)
+    out = decoder.k_logits(X, W, bias, kk, path, prec)
+    assert out["kernel"] == kernel
+    ref = X.astype(np.float64) @ W.astype(np.float64) + bias
+    scale = np.abs(X).astype(np.float64) @ np.abs(W).astype(np.float64)
+    Y = out["Y"].astype(np.float64)
+    # both operands rounded to 8 bits (bf16) or 11 (fp16, and the stored value); otherwise 22, and the tensor core's
+    # truncation of a 1000-term sum (2.4e-6 of 3072 terms was measured)
+    if prec == "bf16":
+        bound = 2.0 ** -8 * scale + 1e-6
+    elif path == "auto":
+        bound = 2.0 ** -10 * scale + 2.0 ** -11 * np.abs(ref) + 1e-6
+    else:
+        bound = 2e-6 * scale + 1e-6
+    assert (np.abs(Y - ref) <= bound).all(), float((np.abs(Y - ref) / bound).max())
+    seen = np.zeros(V, int)
+    for i, (c0, c1) in enumerate(out["blocks"]):
+        if c0 >= c1:
+            assert (out["block_max"][:, i] == -np.inf).all()
+            continue
+        seen[c0:c1] += 1
+        m = Y[:, c0:c1].max(1)
+        assert (out["block_max"][:, i] == m).all(), i
+        if out["block_sum"] is not None:
+            np.testing.assert_allclose(out["block_sum"][:, i], np.exp(Y[:, c0:c1] - m[:, None]).sum(1), rtol=1e-5)
+    assert (seen == 1).all()
+    assert (out["block_sum"] is None) == (V == 80000)
+    # with recomputed candidates the result is the exact product's (1e-4 of a row's log-probabilities), otherwise the stored values'
+    z = ref if path == "auto" and prec == "fp32" else Y
+    lp = z - z.max(1, keepdims=True)
+    lp -= np.log(np.exp(lp).sum(1, keepdims=True))
+    tol = 1e-4 * np.abs(lp).max() if z is ref else 1e-5 * np.abs(lp).max()
+    got = np.take_along_axis(lp, out["idx"].astype(np.int64), 1)
+    assert (np.abs(out["logp"] - got) <= tol).all()
+    assert (np.abs(out["logp"] - (-np.sort(-lp, 1)[:, :kk])) <= tol).all()
+    assert (np.sort(out["idx"], 1)[:, 1:] != np.sort(out["idx"], 1)[:, :-1]).all()
+    assert (np.abs(out["eos"] - lp[:, 1]) <= tol).all()
