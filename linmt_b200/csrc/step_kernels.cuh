@@ -1300,6 +1300,8 @@ inline cudaError_t launch_softmax_topk(const float* logits, int ld, int V, int k
   TopkRefine rf{};
   if (refine) rf = *refine;
   const size_t smem = rf.a0 ? sizeof(float) * (size_t)rf.K : 0;
+  // (models of more than 7680 hidden units)
+  if (cudaError_t e = tc::allow_smem<softmax_topk_kernel>(smem); e != cudaSuccess) return e;
   return tc::launch_k(pdl, softmax_topk_kernel, dim3(rows), dim3(256), smem, st, logits, ld, V, kk, out, normalise, pmax, pmax_ld, n_slots, rf, refine ? logits16 : (const __half*)nullptr, sel);
 }
 
