@@ -1,9 +1,11 @@
 """GPU tests at the far ends of what a handle takes: sizes and batches that no named configuration reaches."""
+import os
+
 import numpy as np
 import pytest
 
 from linmt_b200 import synth
-from parity import RTOL_FP32, compare_forced
+from parity import RTOL_FP32, compare_forced, hyps
 
 pytestmark = pytest.mark.gpu
 
@@ -41,17 +43,24 @@ def test_global_attention_over_long_sources(oracle, cuda_lib, n):
     """A handle for sources of up to 12,250 words: with a row's vector, its scores pass 48 KB of shared memory."""
     from linmt_b200 import decoder
     d = synth.ModelDesc(1, 64, 200, 100, 1)
-    blob = synth.make_blob(d, 8)
+    blob = synth.make_blob(d, 8, family="peaked")
     rng = np.random.default_rng(n)
     lens = np.concatenate([[12250], rng.integers(2, 20, size=n - 1)]).astype(np.int32)
     off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
     sents = synth.Sentences(synth.zipf_ids(rng, int(off[-1]), 1, d.Vs, 1.1), off, np.full(n, 4, np.int32))
-    kw = dict(beam=2, attention="global_general", cp_beta=0.0, min_ratio=0.0)
+    kw = dict(beam=2, attention="global_general", cp_beta=0.0, min_ratio=0.0, print_info=1)
     o = oracle.decode(d, [blob], sents, trace=True, **kw)
     dec = decoder.Decoder(d, [blob], max_batch=n, max_src_len=12250, max_steps=8, **kw)
-    e = dec.decode(sents, trace=True, force=o)
+    e = dec.decode(sents, trace=True, force=o, want_align=True)
     worst, bad, skipped, compared = compare_forced(e, o, sents.steps, src_len=sents.lengths())
     assert worst <= RTOL_FP32 and bad == 0 and skipped == 0, (worst, bad, skipped, compared)
+    # every position's weight (a source of 12,250 words has 8e-5 on each): a score is a 64-term fp32 sum, its exponential
+    # and the sum of all of them good to a few 1e-6
+    assert hyps(e, 0) == hyps(o, 0)
+    for i in range(n):
+        if hyps(e, i) == hyps(o, i):
+            m, S = int(o["len"][i, 0]), int(lens[i])
+            np.testing.assert_allclose(e["align"][i, 0, :m, :S], o["align"][i, 0, :m, :S], rtol=5e-5, atol=1e-10)
     dec.close()
 
 
@@ -75,3 +84,84 @@ def test_batches_of_other_lengths_on_one_handle(cuda_lib, attention):
         for key in ("tok", "len", "score", "vit", "align"):
             assert np.array_equal(out[key], fresh[i][key]), (i, key)
     kept.close()
+
+
+def _with_env(env, make):
+    old = {k: os.environ.get(k) for k in env}
+    os.environ.update(env)
+    try:
+        return make()
+    finally:
+        for k, v in old.items():
+            if v is None:
+                os.environ.pop(k, None)
+            else:
+                os.environ[k] = v
+
+
+@pytest.mark.parametrize("attention", ["local_p_general", "global_dot"])
+def test_bf16_batch_of_more_than_1024_rows(oracle, cuda_lib, attention):
+    """128 sentences x 12 beams in bf16: 1536 rows, whose gate products run as persistent CTA pairs until 1024 are left,
+    behind the encoder of more than 64 sentences.  Against the oracle, forced; and the same bits without pairs, since the
+    same products accumulate in the same order.
+
+    Bound: where two implementations sum in different orders, a rounding of the state may fall to the other bf16
+    neighbour, a step of 2^-9.  Logits are 128-term sums that spread by 0.07: 2^-9 of that is 1.4e-4 if every element of
+    one state parts, ten states (layers, context, attentional state, the steps before) 4e-4 in the mean square, ten times
+    that for the far tail.  (Seen: median 2.6e-4, 1.9e-3 at 99.9 %.  Another sentence's rows differ by 6e-2.)"""
+    from linmt_b200 import decoder
+    c = synth.configs()["C1"]
+    blob = c.blobs(family="peaked")[0]
+    sents = synth.make_sentences(128, 3, 20, c.desc.Vs, 1.1, 5, lambda s: min(s + 2, 16))
+    kw = dict(beam=12, precision="bf16", attention=attention, cp_beta=0.0, min_ratio=0.0)
+    o = oracle.decode(c.desc, [blob], sents, trace=True, **kw)
+
+    def run():
+        dec = decoder.Decoder(c.desc, [blob], max_batch=128, max_src_len=32, max_steps=32, **kw)
+        forced, before = dec.decode(sents, trace=True, force=o), dec.stats()["pair_launches"]
+        free = dec.decode(sents)
+        dec.close()
+        return forced, free, before
+
+    forced, free, pairs = run()
+    # a gate launch of every layer in every step of more than 1024 rows
+    wide = sum(1 for t in range(int(sents.steps.max()) + 1) if 12 * int((sents.steps >= t).sum()) > 1024)
+    assert wide >= 3 and pairs >= wide * c.desc.L
+    err = np.concatenate([np.abs(forced["cand_logp"][i, t, :(1 if t == 0 else None)] - o["cand_logp"][i, t, :(1 if t == 0 else None)]).ravel()
+                          for i in range(sents.n) for t in range(int(sents.steps[i]))])
+    assert (err <= 4e-3).mean() >= 0.999 and err.max() <= 1.2e-2, (float((err <= 4e-3).mean()), float(np.median(err)), float(err.max()))
+    forced1, free1, pairs1 = _with_env({"LINMT_TC_PAIR": "0"}, run)
+    assert pairs1 == 0
+    for a, b, keys in ((forced, forced1, ("cand_tok", "cand_logp", "final_logp")), (free, free1, ("tok", "len", "score"))):
+        for key in keys:
+            assert a[key].tobytes() == b[key].tobytes(), key
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("n,longest", [(64, 300), (63, 600), (3, 6000)])
+def test_encoder_in_chunks_of_positions(cuda_lib, precision, n, longest):
+    """The layer-by-layer encoder takes 16,384 rows (positions x sentences) at a time: longer sources continue from the
+    states the chunk before ended with, here after an even and an odd number of positions and more than once.  Against the
+    encoder that runs position by position (the CUDA-core path in fp32; without the few-rows kernel in bf16)."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, 96, 300, 200, 1)
+    blob = synth.make_blob(d, 6, family="peaked")
+    rng = np.random.default_rng(n)
+    lens = np.concatenate([[longest, longest - 1], rng.integers(1, longest, size=n - 2)]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    sents = synth.Sentences(synth.zipf_ids(rng, int(off[-1]), 1, d.Vs, 1.1), off, np.full(n, 6, np.int32))
+    kw = dict(beam=2, precision=precision, max_batch=n, max_src_len=longest, max_steps=8, cp_beta=0.0, min_ratio=0.0)
+    if precision == "fp32":
+        ref = decoder.Decoder(d, [blob], gemm_path="simt", **kw)
+    else:
+        ref = _with_env({"LINMT_TC_ROWS": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    r = ref.decode(sents, trace=True)
+    dec = decoder.Decoder(d, [blob], **kw)
+    e = dec.decode(sents, trace=True, force=r)
+    if precision == "fp32":
+        worst, bad, skipped, compared = compare_forced(e, r, sents.steps, src_len=sents.lengths())
+        assert worst <= RTOL_FP32 and bad == 0 and skipped <= 0.1 * (skipped + compared), (worst, bad, skipped, compared)
+    else:
+        a, b = e["cand_logp"][:, 1:], r["cand_logp"][:, 1:]
+        assert np.abs(a - b).max() <= 1.2e-2, float(np.abs(a - b).max())      # (as for 1536 rows above)
+    ref.close(); dec.close()
