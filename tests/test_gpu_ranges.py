@@ -165,3 +165,63 @@ def test_encoder_in_chunks_of_positions(cuda_lib, precision, n, longest):
         a, b = e["cand_logp"][:, 1:], r["cand_logp"][:, 1:]
         assert np.abs(a - b).max() <= 1.2e-2, float(np.abs(a - b).max())      # (as for 1536 rows above)
     ref.close(); dec.close()
+
+
+@pytest.mark.parametrize("members,mode", [(5, "prob_mean"), (8, "logprob_mean")])
+def test_ensembles_of_more_than_four(oracle, cuda_lib, members, mode):
+    """The combining softmax keeps four members' loads in flight and takes the others in turn."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(1, 64, 1003, 300, 1)
+    blobs = [synth.make_blob(d, 40 + m, family="peaked") for m in range(members)]
+    sents = synth.make_sentences(5, 2, 12, d.Vs, 1.1, 3, lambda s: s + 3)
+    kw = dict(beam=6, nbest=2, cp_beta=0.0, ensemble=mode)
+    o = oracle.decode(d, blobs, sents, trace=True, **kw)
+    dec = decoder.Decoder(d, blobs, max_batch=5, max_src_len=16, max_steps=20, **kw)
+    e = dec.decode(sents, trace=True, force=o)
+    worst, bad, skipped, compared = compare_forced(e, o, sents.steps, src_len=sents.lengths())
+    assert worst <= RTOL_FP32 and bad == 0 and skipped <= 0.1 * (skipped + compared), (worst, bad, skipped, compared)
+    dec.close()
+
+
+@pytest.mark.parametrize("members,precision", [(1, "fp32"), (1, "bf16"), (2, "fp32")])
+def test_rows_of_equal_logits(oracle, cuda_lib, members, precision):
+    """All-zero weights: every class ties, more of them than the candidate lists hold, and the lowest ids win."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(1, 64, 3000, 50, 1)
+    blobs = [np.zeros(synth.blob_floats(d), np.float32)] * members
+    sents = synth.make_sentences(3, 2, 6, d.Vs, 1.1, 3, lambda s: s + 1)
+    kw = dict(beam=4, cp_beta=0.0, precision=precision)
+    o = oracle.decode(d, blobs, sents, trace=True, **kw)
+    dec = decoder.Decoder(d, blobs, max_batch=3, max_src_len=8, max_steps=10, **kw)
+    e = dec.decode(sents, trace=True)
+    for i in range(sents.n):
+        T = int(sents.steps[i])
+        assert (e["cand_tok"][i, 0, 0] == np.arange(5)).all() and (e["cand_tok"][i, 1:T] == np.arange(5)).all()
+        np.testing.assert_allclose(e["cand_logp"][i, 1:T], -np.log(3000.0), rtol=1e-6)
+        assert (e["surv_tok"][i, :T] == o["surv_tok"][i, :T]).all() and (e["surv_parent"][i, :T] == o["surv_parent"][i, :T]).all()
+    dec.close()
+
+
+@pytest.mark.parametrize("steps", [300, 1500, 5900])     # 8 warps, 1 warp, and back-pointers that stay in global memory
+def test_finalisation_of_long_hypotheses(oracle, cuda_lib, steps):
+    """n-best lists with alignments and coverage penalty of hypotheses so long that fewer warps, and then no copy of the
+    back-pointers, fit the shared memory of the finalisation."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(1, 32, 60, 50, 1)
+    blob = synth.make_blob(d, 9, family="peaked")
+    sents = synth.make_sentences(2, 9, 12, d.Vs, 1.1, 3, lambda s: steps if s > 10 else 7)
+    sents.steps[:] = [steps, 7]
+    kw = dict(beam=3, nbest=3, cp_beta=0.2, min_ratio=0.0, print_info=1)
+    o = oracle.decode(d, [blob], sents, trace=True, **kw)
+    dec = decoder.Decoder(d, [blob], max_batch=2, max_src_len=16, max_steps=steps, **kw)
+    e = dec.decode(sents, trace=True, force=o, want_align=True)
+    assert (e["len"] == o["len"]).all()
+    for i in range(2):
+        S = int(sents.lengths()[i])
+        for q in range(3):
+            n = int(o["len"][i, q])
+            assert hyps(e, i, q) == hyps(o, i, q)
+            assert (e["vit"][i, q, :n] == o["vit"][i, q, :n]).mean() >= 0.999
+            assert abs(e["score"][i, q] - o["score"][i, q]) <= RTOL_FP32 * abs(o["score"][i, q])
+            np.testing.assert_allclose(e["align"][i, q, :n, :S], o["align"][i, q, :n, :S], rtol=2e-4, atol=1e-6)
+    dec.close()
