@@ -11,7 +11,7 @@
 
 namespace linmt {
 
-constexpr int kMaxBeam = 31;          // kk = beam + 1 <= 32
+constexpr int kMaxBeam = 31;          // kk = beam + 1 <= 32, the lanes that a threshold is ranked on
 constexpr int kStart = 0, kEos = 1, kUnk = 2;  // src/input_file_preprocess.cc:549-567
 constexpr float kDeadScore = -1e30f;  // score of a hypothesis created when candidates run out
 
@@ -166,7 +166,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// Block-wide sum in a fixed order (deterministic).
 // ---------------------------------------------------------------------------------------
 // Attention of a step (AttentionNode::ForwardProp, src/layer_attention.h:243-483,
 // kernels k12-k20: Sgemm m=1, SigmoidKernel, AlignmentPosKernel, LowerUpperKernel,
@@ -727,8 +726,8 @@ __device__ __forceinline__ void select_if_last(const SelectArgs& a, const TopkOu
   if (last) beam_select_block<THREADS>(a, cand, sent, T, osent, nf0, smraw);
 }
 
-// Pass 1 finds the row maximum and, from the 256 per-thread maxima, a threshold that at least
-// kk elements reach (the kk-th largest thread maximum).  Pass 2 (the row is L2/L1 resident by
+// Pass 1 finds the row maximum and, from 32 maxima over groups of threads, a threshold that at least
+// kk elements reach (the kk-th largest of them).  Pass 2 (the row is L2/L1 resident by
 // then) sums exp(z - max) and collects the few elements at or above the threshold, which are
 // then ranked exactly.  If more elements than the candidate buffer holds reach the threshold
 // (e.g. a row of equal logits) the block falls back to kk exact arg-best sweeps.
@@ -1003,37 +1002,25 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
   s_tmax[tid] = m;
   if (tid == 0) sh.count = 0;
   __syncthreads();
-  if (kk <= 32) {
-    // Threshold from 32 group maxima (group = the 8 threads with the same lane): each is an
-    // element of the row and the groups are disjoint, so at least kk elements reach the kk-th
-    // largest of them; it is a little lower than the kk-th largest thread maximum (a few more
-    // candidates to rank) and costs one warp ~100 instructions instead of 256 x 256 compares.
-    if (warp == 0) {
-      float g = -INFINITY;
+  // Threshold from 32 group maxima (group = the 8 threads with the same lane): each is an
+  // element of the row and the groups are disjoint, so at least kk (at most 32) elements reach the kk-th
+  // largest of them; it is a little lower than the kk-th largest thread maximum (a few more
+  // candidates to rank) and costs one warp ~100 instructions instead of 256 x 256 compares.
+  if (warp == 0) {
+    float g = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) g = fmaxf(g, s_tmax[w * 32 + lane]);
-      float bm = g;
+    for (int w = 0; w < 8; ++w) g = fmaxf(g, s_tmax[w * 32 + lane]);
+    float bm = g;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
-      int rank = 0;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float o = __shfl_sync(0xffffffffu, g, j);
-        rank += (o > g || (o == g && j < lane)) ? 1 : 0;
-      }
-      if (rank == kk - 1) s_tau = g;
-      if (lane == 0) s_max = bm;
-    }
-  } else {
+    for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
     int rank = 0;
-    float bm = -INFINITY;
-    for (int j = 0; j < 256; ++j) {
-      const float o = s_tmax[j];
-      bm = fmaxf(bm, o);
-      rank += (o > m || (o == m && j < tid)) ? 1 : 0;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const float o = __shfl_sync(0xffffffffu, g, j);
+      rank += (o > g || (o == g && j < lane)) ? 1 : 0;
     }
-    if (rank == (kk < 256 ? kk : 256) - 1) s_tau = m;
-    if (tid == 0) s_max = bm;
+    if (rank == kk - 1) s_tau = g;
+    if (lane == 0) s_max = bm;
   }
   __syncthreads();
   if (pmax) {
@@ -1417,7 +1404,6 @@ static __global__ void __launch_bounds__(256) ensemble_combine_kernel(EnsembleRo
   // second sweep: the members' probabilities (or log-probabilities) of four classes at a time, accumulated in
   // double like the reference's loop (src/decoder.h:1913-1921)
   float* o = out + (size_t)r * ld;
-  const float inv_n = 1.0f / er.n;
   for (int i = tid * 4; i < V4; i += 1024) {
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
     for (int m = 0; m < er.n; ++m) {
@@ -1441,7 +1427,6 @@ static __global__ void __launch_bounds__(256) ensemble_combine_kernel(EnsembleRo
     acc /= er.n;
     o[j] = (mode == 0) ? logf((float)acc) : (float)acc;
   }
-  (void)inv_n;
 }
 
 // Ensembles: combination, log-softmax and top-kk of a row in one pass over the members' logits.  A member's maximum and
@@ -1634,7 +1619,8 @@ struct FinalizeArgs {
   int32_t* out_vit;   // [n][nbest][max_len] or null
   float* out_align;   // [n][nbest][max_len][max_src] or null
 };
-// grid = sentences, block = 128, dynamic smem = 4 warps * (max_src floats + max_len ints)
+// grid = sentences, block and dynamic smem = finalize_shape: 1 to 16 warps, a path and row sums of max_len entries for each
+// of them, and the sentence's back-pointers where they fit.
 // The kernel is a chain of memory round trips: following the back-pointers of a hypothesis through global memory was one
 // per step (54 us for 85 steps), and the coverage of a hypothesis two per step.  The sentence's back-pointers come into
 // shared memory first (a byte each), and the coverage reads four steps at a time.
