@@ -23,8 +23,9 @@
 // loads, warp 1 owns TMEM and issues the leading-product MMAs, warps 2..17 run the epilogue
 // (tcgen05.ld -> registers -> fused math -> staging in the idle stage ring -> coalesced stores; four
 // warps per TMEM lane quadrant, each a contiguous block of columns), warp 18 issues the cross-term
-// MMAs.  The issuing threads are the critical path of a narrow tile, so their loops carry descriptors
-// forward by constant increments and everything that can be is a compile-time constant; the waiting
+// MMAs.  The issuing warps are the critical path of a narrow tile (an MMA of 128 rows takes 64 clocks
+// however few its columns), so their loops run on an elected lane (see elect_one), carry descriptors
+// forward by constant increments and have everything that can be as a compile-time constant; the waiting
 // epilogue warps sleep between polls.  A ring of shared-memory stages is handed back and forth with
 // mbarriers; every wait is bounded and reports through an error flag instead of hanging.  All kernels
 // take part in programmatic dependent launch (see pdl_wait below).  A persistent variant
@@ -46,8 +47,8 @@ constexpr int UMMA_K = 16;         // bf16 elements per tcgen05.mma
 constexpr int kEpiWarps = 16;        // epilogue warps: four per TMEM lane quadrant
 constexpr int kThreads = 64 + 32 * kEpiWarps;  // warp 0 TMA, warp 1 MMA, then the epilogue warps
 // The one-tile kernel has a second MMA-issuing warp after the epilogue warps: with split operands the
-// leading product and the cross terms go to different accumulators, so two threads can issue them
-// independently -- a narrow tile is bound by what ONE thread can issue (~58 ns per MMA).
+// leading product and the cross terms go to different accumulators, and the leading one stops for the
+// drains while the other runs on; each accumulator has one issuer, so the order of its sum is fixed.
 constexpr int kIssue2Warp = 2 + kEpiWarps;
 constexpr int kThreadsMain = kThreads + 32;
 constexpr unsigned long long kWaitCycles = 2000000000ull;  // ~1 s at 2 GHz
@@ -1533,12 +1534,14 @@ inline int pick_bn(int M, int N, int n_sm) {
   return best;
 }
 
-// Tile width AND split-K factor from a small cost model (times in ns per k-block, measured):
-// a k-block costs the larger of the issuing thread's time (~58 ns per MMA, whatever its width)
-// and the tensor pipe's (128 x bn x 16 MACs at 4096 MAC/clk); a launch takes
-// waves * (k-blocks-per-CTA of those + ~8-13 us of prologue/epilogue per tile), plus the cost of
-// writing and re-reading partial tiles when K is split (only worth it for tiles up to 176 wide).
-// ws_floats bounds the split-K workspace (splits * padded rows * N floats).
+// Tile width AND split-K factor from a small cost model: a launch takes waves * (k-blocks per CTA times the cost of one,
+// plus 8 us + 20 ns per column of prologue and epilogue), plus the cost of writing and re-reading partial tiles when K is
+// split (only worth it for tiles up to 176 wide).  ws_floats bounds the split-K workspace (splits * padded rows * N floats).
+// The constants for one plane and for bf16 planes are those of an earlier issue loop, in which an MMA cost its
+// issuer 58 ns whatever its width (now: 64 clocks or its columns), and charge too much, the more the narrower
+// the tile.  bf16 gate product, N = 4096, K = 2048, weights from HBM, predicted / measured: 16.4 / 10.4 us at 72 to 128
+// rows (86 tiles of 48 columns), 16.7 / 10.9 at 256, 17.3 / 12.1 at 384, 18.3 / 14.2 at 640, 20.6 / 19.2 at 1024.  The
+// shapes it picks are the ones measured; which others would be faster has not been.
 // The f16 pair with 64-deep stages, measured: a k-block costs ~400 ns on narrow tiles (an MMA of 128 rows has a floor of
 // ~65 clocks however narrow it is) and 120 + 3.6 * bn ns on wider ones (the tensor pipe at
 // its practical rate); per tile ~6 us + 12 ns per column of prologue and epilogue; a split adds ~2 us plus

@@ -11,7 +11,7 @@
 // (the same products accumulate in the same order).  Measured on the decoder's gate product at 768 rows
 // (K = 2048, N = 4096, 176-wide tiles, weights from HBM): 35.8 us against 41.2 us per layer; the one-tile
 // kernel has room for two 76 KB stages there, the pair for four of 54 KB.  Narrower shapes (three or more stages
-// already, bound by the issuing threads) gain nothing, so the host uses pairs only where the one-tile shape is
+// already, bound by the 64 clocks that an MMA takes at least) gain nothing, so the host uses pairs only where the one-tile shape is
 // down to two stages.
 //
 // Protocol (the even CTA of a pair = "leader"):

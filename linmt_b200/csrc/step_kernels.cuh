@@ -1144,7 +1144,10 @@ static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float
 // round trips (one sentence at 12 rows, 30k classes: 22.2 us per step sweeping, 13.1 so); 256 otherwise, where the sweep
 // read what the GEMM had just written.
 // grid = rows, dynamic smem = topk_blocks_smem
-constexpr int kBlocksSmemMax = 23 * 1024;   // of dynamic shared memory beside the candidate lists: wider rows are swept
+// The block statistics of a row and its activations lie in shared memory beside the candidate lists (18 or 21 KB, of the 48
+// a launch may use unasked): rows that need more than this are swept, which includes 80,000 classes in the few-rows kernel's
+// blocks of 32 columns (2500 pairs, 24.1 KB with the activations of 1024 units, 20.0 without).
+constexpr int kBlocksSmemMax = 23 * 1024;
 struct LogitBlocks {
   float* max; float* sum; int ld; int n;
   int tile, part;     // columns of a GEMM tile and of one of its four blocks (the last one of a tile may be narrower)
