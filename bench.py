@@ -35,13 +35,13 @@ UNIT = "tokens/s"
 FALLBACK_TFLOPS = 1590.0  # used only if MEASURED_PEAKS.json is absent
 FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes (read + write) of ONE launch of each kernel class at the full width of the C2 batch (768 rows), from
-# ncu captures of this benchmark's own C2 decode (dram__bytes_read.sum + dram__bytes_write.sum of one launch; the
-# summaries with the capture commands are committed with the profiles).  None = no capture for that class.
+# ncu captures of the kernels that run there (dram__bytes_read.sum + dram__bytes_write.sum of one launch; the
+# summaries with the capture commands are committed with the profiles).  None = no launches of that class there.
 C2_TRAFFIC_BYTES = {
-    "lstm_gemm": 43.5e6,        # first layer 45.74 MB (with input-term table rows), the others 42.72 MB
-    "vocab_gemm": 77.2e6,       # 63.40 MB read (the weights) + 13.82 MB written (fp16 logits, most of them still in L2)
-    "attn_proj_gemm": 15.8e6, "attn_out_gemm": 10.56e6,
-    "gather": 10.66e6,          # (softmax and attention: no capture of their present kernels)
+    "lstm_gemm": 43.1e6,        # first layer 45.4 MB (with input-term table rows), the others 42.3 MB
+    "vocab_gemm": 75.5e6,       # 63.4 MB read (the weights) + 12.1 MB written (fp16 logits, most of them still in L2)
+    "attn_proj_gemm": 15.8e6,
+    "softmax_topk": 14.1e6, "attention": 17.4e6, "gather": 10.0e6,
 }
 
 
