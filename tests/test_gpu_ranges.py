@@ -137,6 +137,28 @@ def test_bf16_batch_of_more_than_1024_rows(oracle, cuda_lib, attention):
             assert a[key].tobytes() == b[key].tobytes(), key
 
 
+def test_full_size_gate_products_on_persistent_pairs(cuda_lib):
+    """The same at the full model size, where a product's 32 k-blocks go round the ring several times and a pair walks over
+    several tiles: 100 sentences x 12 beams, the bits of the one-tile kernels."""
+    from linmt_b200 import decoder
+    c = synth.configs()["C2"]
+    blob = c.blobs()[0]
+    sents = synth.make_sentences(100, 2, 8, c.desc.Vs, 1.1, 5, lambda s: 5)
+
+    def run():
+        dec = decoder.Decoder(c.desc, [blob], beam=12, precision="bf16", max_batch=100, max_src_len=8, max_steps=8, cp_beta=0.0)
+        out = dec.decode(sents, trace=True)
+        pairs = dec.stats()["pair_launches"]
+        dec.close()
+        return out, pairs
+
+    a, pairs = run()
+    b, none = _with_env({"LINMT_TC_PAIR": "0"}, run)
+    assert pairs >= 6 * c.desc.L and none == 0
+    for key in ("cand_tok", "cand_logp", "final_logp", "tok", "score"):
+        assert a[key].tobytes() == b[key].tobytes(), key
+
+
 @pytest.mark.parametrize("precision", ["fp32", "bf16"])
 @pytest.mark.parametrize("n,longest", [(64, 300), (63, 600), (3, 6000)])
 def test_encoder_in_chunks_of_positions(cuda_lib, precision, n, longest):
