@@ -112,6 +112,8 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   tc::TmapSet tm;
   std::memcpy(tm.a, am, sizeof(tm.a));
   std::memcpy(tm.b, bm, sizeof(tm.b));
+  // (one plane and many rows: tensor-bound, and its row tiles read the weights several times over: 1536 rows 29.5 -> 29.9 ms a call as a stream)
+  tm.stream_b = stream_weights_ && decoding_ && (nt > 1 || M <= 256);
   if constexpr (Epi::kHasPmax) {
     if (e.pmax) {
       blocks_ = logit_blocks(e.pmax, e.psum, e.pmax_ld, N, K, plan.stat_tile, plan.stat_part);
@@ -123,6 +125,14 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   LAUNCHED();
   if (plan.on_pairs()) ++stats.pair_launches;
   return LINMT_OK;
+}
+
+// A step reads more weights than L2 has room for beside the states (three quarters of it): they are loaded as a stream.
+bool Engine::weights_stream() const {
+  int l2 = 0;
+  if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, opt.device) != cudaSuccess) { cudaGetLastError(); return false; }
+  const size_t hh = (size_t)Hp * Hp, recurrent = (8 * (size_t)L + 4) * hh, vocab = (size_t)Vp * Hp;
+  return 2 * n_models * (nt_ * recurrent + nt_vocab_ * vocab) > (size_t)l2 / 4 * 3;
 }
 
 bool Engine::pairs_available() { return tc::max_resident_pairs<2, 64, 1, tc::TcEpiLstm>() > 0; }
@@ -160,6 +170,7 @@ int Engine::build_xw_tables() {
 // events for the cross-layer edges.  Besides the true dependencies, (l, p) waits for (l+1, p-2),
 // the last reader of the double-buffered input slot it overwrites.
 int Engine::run_encoder_tc(int n, int Smax) {
+  decoding_ = false;
   if (rows_ && n <= 64 && enc_rows_) return run_encoder_layers_tc(n, Smax);
   constexpr int kRing = 4;
   hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;
@@ -298,6 +309,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   TcState& ts = tc_states_[mi];
   const bool feed = desc.feed_input && t > 0;
   pdl_gemm_ = true;
+  decoding_ = true;
   // scoring: one row per sentence continues itself, its tokens are given, and every step's htilde is kept
   const int kb = sc ? 1 : k;
   const int32_t* tok = sc ? sc->tok : d_tok_;

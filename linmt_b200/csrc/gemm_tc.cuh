@@ -56,6 +56,7 @@ constexpr unsigned long long kWaitCycles = 2000000000ull;  // ~1 s at 2 GHz
 struct alignas(64) TmapSet {
   CUtensorMap a[3];
   CUtensorMap b[3];
+  int stream_b;      // the weights are a stream that L2 cannot hold until they are read again (see weight_policy)
 };
 
 constexpr int A_BYTES = BM * BK * 2;         // one plane of the A tile of a stage
@@ -154,6 +155,24 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+// policy 0: an ordinary load
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t policy) {
+  if (policy == 0) { tma_load_2d(dst, map, x, y, bar); return; }
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy) : "memory");
+}
+// L2 priority of the weights' loads.  The weights of a decoder step of a large model (208 MB for 4 x 1000 / 30k in fp32
+// precision, 134 MB in bf16) pass through L2 (126 MB) between two uses of any of them, and as ordinary lines they take everything
+// else with them: the encoder's states, cell states, biases and block statistics, which the row kernels then fetch from HBM
+// one dependent round trip after another.  As lines that are given up first, they displace each other.  One sentence in
+// fp32 5.72 -> 5.33 ms a call, in bf16 4.43 -> 3.95 (there part of the weights then stays as well), 64 rows 52.1 -> 50.2;
+// with some of the layers kept in L2 instead (one, two or three of four) within 1 % of that or slower.
+__device__ __forceinline__ uint64_t weight_policy(int stream) {
+  uint64_t p = 0;
+  if (stream) asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
 }
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
@@ -950,6 +969,7 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int a_ro
   if (warp == 0) {
     // Producer.
     const bool one = elect_one();
+    const uint64_t policy = weight_policy(tm.stream_b);
     const int ya = a_row0 + m0;      // (rows past the product's last one are read and not used)
     auto load_a = [&](int kb, uint32_t st, uint32_t fb) {
 #pragma unroll
@@ -957,7 +977,7 @@ gemm_tc_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int a_ro
     };
     auto load_b = [&](int kb, uint32_t st, uint32_t fb) {
 #pragma unroll
-      for (int t = 0; t < NT; ++t) tma_load_2d(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], (kb0 + kb) * BK, n0, fb);
+      for (int t = 0; t < NT; ++t) tma_load_2d(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], (kb0 + kb) * BK, n0, fb, policy);
     };
     // First trip round the ring: the weight tiles do not depend on the previous kernel, so they
     // are requested before pdl_wait() and only the activation tiles after it.
@@ -1251,6 +1271,7 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
 
   if (warp == 0) {
     const bool one = elect_one();
+    const uint64_t policy = weight_policy(tm.stream_b);
     int s = 0; uint32_t ph = 0;
     uint32_t st = base, fb = bars, eb = bars + 8u * STAGES;
     pdl_wait();
@@ -1264,7 +1285,7 @@ gemm_tc_persist_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, 
 #pragma unroll
           for (int t = 0; t < NT; ++t) {
             tma_load_2d(st + t * A_BYTES, &tm.a[t], kb * BK, ya, fb);
-            tma_load_2d(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], kb * BK, yb, fb);
+            tma_load_2d(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], kb * BK, yb, fb, policy);
           }
         }
         st += STAGE_BYTES; fb += 8u; eb += 8u;

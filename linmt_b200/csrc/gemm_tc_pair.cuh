@@ -47,6 +47,12 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar, uint64_t policy) {
+  if (policy == 0) { tma_load_2d_pair(dst, map, x, y, bar); return; }
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -127,6 +133,7 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   if (warp == 0) {
     // Producer (both CTAs): the planes of this CTA's A rows and of its half of B, issued by the elected lane.
     const bool one = elect_one();
+    const uint64_t policy = weight_policy(tm.stream_b);
     const uint32_t full0 = cluster_map(bars, 0u);           // the leader's full barriers, as cluster addresses
     const uint32_t tx_bytes = 2u * (uint32_t)STAGE_BYTES;   // both CTAs' boxes
     const int yb = n0 + (int)rank * BH;
@@ -136,7 +143,7 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     };
     auto load_b = [&](int kb, uint32_t st, uint32_t fb) {
 #pragma unroll
-      for (int t = 0; t < NT; ++t) tma_load_2d_pair(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], (kb0 + kb) * BK, yb, fb);
+      for (int t = 0; t < NT; ++t) tma_load_2d_pair(st + NT * A_BYTES + t * B_BYTES, &tm.b[t], (kb0 + kb) * BK, yb, fb, policy);
     };
     const int npre = nkb < STAGES ? nkb : STAGES;
     if (one)

@@ -159,9 +159,10 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     mbar_expect_tx(recv_bar, (uint32_t)(n_own * (splits - 1) * 512));   // the neighbours' share
   }
   const bool one = elect_one();
+  const uint64_t policy = warp == 0 ? weight_policy(tm.stream_b) : 0;
   auto load_w = [&](int kb, int stage) {
 #pragma unroll
-    for (int t = 0; t < NT; ++t) tma_load_2d(base + (uint32_t)((stage * NT + t) * W_BYTES), &tm.b[t], (kb0 + kb) * 64, n0, bars + 8u * stage);
+    for (int t = 0; t < NT; ++t) tma_load_2d(base + (uint32_t)((stage * NT + t) * W_BYTES), &tm.b[t], (kb0 + kb) * 64, n0, bars + 8u * stage, policy);
   };
   auto load_x = [&](int kb, int stage) {
 #pragma unroll
