@@ -361,11 +361,13 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
     if (G > 1)
       for (int w = lane; w < W; w += 32)
         if (w < w0 || w >= w1) eg[w * GP] = 0.f;
+    if (rec_lo && ens == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
-      if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, besti, o);
+        if (ob > best || (ob == best && oi < besti)) { best = ob; besti = oi; }
+      }
     }
     if (lane == 0 && rec_lo && ens == 0) { rec_lo[r0 + g] = wlo; rec_vit[r0 + g] = (best > 0.f) ? besti : -1; }
   } else if (G > 1 && warp < G) {
@@ -588,9 +590,11 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     return;
   }
   unsigned long long* key = reinterpret_cast<unsigned long long*>(smraw);   // sortable (score, beam, vocabulary id)
-  unsigned long long* order = key + k * kk;                                 // the same in order
+  unsigned long long* listed = key + k * kk;                                // those that may be among the survivors
   const int cols = (t == 0) ? 1 : k;
   const int n = cols * kk;
+  __shared__ int s_special[THREADS / 32];      // a warp's candidates that take no slot
+  int special = 0;
   for (int c = tid; c < n; c += THREADS) {
     const int b = c / kk, q = c - b * kk;
     const float lp = __ldcg(cand.logp + (size_t)(r0 + b) * kk + q);    // (other CTAs' results)
@@ -602,29 +606,62 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     const unsigned int ord = (fb & 0x80000000u) ? ~fb : (fb | 0x80000000u);
     const unsigned int low = 0xFFFFFFFFu - (((unsigned int)b << 24) | ((unsigned int)v & 0xFFFFFFu));
     key[c] = ((unsigned long long)ord << 32) | low;
+    special += v < 0 || v == kStart || v == kEos ? 1 : 0;
     if (tr.cand_tok) {
       const size_t off = ((((size_t)osent * tr.Tm + t) * k + b) * kk) + q;
       tr.cand_tok[off] = v; tr.cand_logp[off] = lp;
     }
   }
+  special = __reduce_add_sync(0xffffffffu, special);
+  if (lane == 0) s_special[warp] = special;
   __syncthreads();
-  // a thread counts the candidates before its own; four of a large block share one (a warp per candidate with ballots
-  // was slower: 156 candidates, 7000 clocks in a block of 1024 and 20000 in one of 256)
-  const int share = THREADS > 256 && n <= THREADS / 4 ? 4 : 1;
-  for (int c0 = 0; c0 < n; c0 += THREADS / share) {
-    const int c = c0 + tid / share;
-    const unsigned long long kc = c < n ? key[c] : 0ull;
-    int p = 0;
+  // Only as many candidates as there are slots, and those that take none (START, EOS), have to be in order: the `need` best.
+  // The need-th best of every row's first two (of its first, beyond 16 rows) is a bound that they all reach; what reaches it,
+  // some tens of n, is listed and ranked.  (All n against all n: 2.5 us of the last CTA at 156 candidates, whatever the
+  // threads; 768 rows 29.4 -> 25.3 us a launch, 1536 rows 30.9 -> 25.1.)
+  __shared__ unsigned long long s_bound;
+  __shared__ int s_listed;
+  int n_order = n;
+  const unsigned long long* ranked = key;
+  if (n > 32) {
+    if (warp == 0) {
+      const int need = k + __reduce_add_sync(0xffffffffu, lane < THREADS / 32 ? s_special[lane] : 0);
+      const int firsts = cols > 16 ? 1 : 2, m = firsts * cols;
+      const int b = firsts == 2 ? lane >> 1 : lane, q = firsts == 2 ? lane & 1 : 0;
+      const unsigned long long f = lane < m ? key[b * kk + q] : 0ull;
+      int rank = 0;
 #pragma unroll 4
-    for (int d = tid & (share - 1); d < n; d += share) {
-      const unsigned long long kd = key[d];
-      p += (kd > kc || (kd == kc && d < c)) ? 1 : 0;
+      for (int j = 0; j < m; ++j) {
+        const unsigned long long o = __shfl_sync(0xffffffffu, f, j);
+        rank += o > f || (o == f && j < lane) ? 1 : 0;
+      }
+      if (lane == 0) { s_listed = 0; if (need > m) s_bound = 0ull; }
+      if (lane < m && rank == need - 1) s_bound = f;
     }
-    if (share > 1) {
-      p += __shfl_xor_sync(0xffffffffu, p, 1);
-      p += __shfl_xor_sync(0xffffffffu, p, 2);
+    __syncthreads();
+    const unsigned long long bound = s_bound;
+    for (int c = tid; c < n; c += THREADS) {
+      const unsigned long long kc = key[c];
+      if (kc >= bound) listed[atomicAdd(&s_listed, 1)] = kc;
     }
-    if (c < n && (tid & (share - 1)) == 0) order[p] = kc;
+    __syncthreads();
+    n_order = s_listed;
+    ranked = listed;
+  }
+  // in order, over the keys (32 and fewer are their only reader's)
+  for (int c0 = 0; c0 < n_order; c0 += THREADS) {
+    const int c = c0 + tid;
+    const unsigned long long kc = c < n_order ? ranked[c] : 0ull;
+    int p = 0;
+    if (c < n_order) {
+#pragma unroll 4
+      for (int d = 0; d < n_order; ++d) {
+        const unsigned long long kd = ranked[d];
+        p += (kd > kc || (kd == kc && d < c)) ? 1 : 0;
+      }
+    }
+    if (n <= 32) __syncwarp();
+    if (c < n_order) key[p] = kc;
   }
   __syncthreads();
   __shared__ int s_ntok[kMaxBeam + 1], s_npar[kMaxBeam + 1];
@@ -632,11 +669,11 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
   if (warp == 0) {
     // START is skipped, EOS leaves the beam without taking a slot as long as slots are free
     int ns = 0, nf = nf0;
-    for (int p0 = 0; p0 < n && ns < k; p0 += 32) {
+    for (int p0 = 0; p0 < n_order && ns < k; p0 += 32) {
       const int p = p0 + lane;
-      const unsigned long long ko = p < n ? order[p] : 0ull;
+      const unsigned long long ko = p < n_order ? key[p] : 0ull;
       const unsigned int low = 0xFFFFFFFFu - (unsigned int)ko, ord = (unsigned int)(ko >> 32);
-      const int v = p < n && (low & 0xFFFFFFu) != 0xFFFFFFu ? (int)(low & 0xFFFFFFu) : -1, b = (int)(low >> 24);
+      const int v = p < n_order && (low & 0xFFFFFFu) != 0xFFFFFFu ? (int)(low & 0xFFFFFFu) : -1, b = (int)(low >> 24);
       const float sc = __uint_as_float((ord & 0x80000000u) ? (ord & 0x7FFFFFFFu) : ~ord);
       const unsigned take = __ballot_sync(0xffffffffu, v >= 0 && v != kStart && v != kEos);
       const unsigned below = (1u << lane) - 1u;
@@ -743,7 +780,7 @@ struct TopkShared {
   int redi[32];
   float part[32];       // the warps' shares of the sum
   int count, n_blocks;
-  float lse, eos, eos_delta;
+  float lse, eos, eos_delta, eos_half[2];
 };
 // (once a row's results are written, the selection has the memory)
 union TopkSmem {
@@ -801,38 +838,57 @@ __device__ __forceinline__ void topk_finish(TopkShared& sh, int r, float ssum, f
     // on a peaked row the few dominant logits ARE the normaliser, and their fp16-product error would
     // otherwise go straight into every log-probability of the row.
     const int nc = n;
-    for (int c = warp; c <= nc; c += THREADS / 32) {
-      const int v = (c < nc) ? sh.ci[c] : kEos;
+    // the dot product of a stretch of the row with the same stretch of weight row v, eight values to a lane and load
+    auto dot = [&](int v, int j0, int j1) {
       const __half* w0 = rf.b0 + (size_t)v * rf.ldb;
       const __half* w1 = rf.b1 + (size_t)v * rf.ldb;
-      // (what the sum is completed with is requested together with the weights)
-      const float bias = rf.bias ? rf.bias[v] : 0.f;
-      const float za = (c < nc) ? sh.cv[c] : zat(kEos);
       float acc = 0.f;
-      auto dot4 = [&](int j) {
-        const uint2 q0 = *reinterpret_cast<const uint2*>(w0 + j);
-        const uint2 q1 = *reinterpret_cast<const uint2*>(w1 + j);
-        const __half2 h00 = *reinterpret_cast<const __half2*>(&q0.x), h01 = *reinterpret_cast<const __half2*>(&q0.y);
-        const __half2 h10 = *reinterpret_cast<const __half2*>(&q1.x), h11 = *reinterpret_cast<const __half2*>(&q1.y);
-        const float2 b00 = __half22float2(h00), b01 = __half22float2(h01), b10 = __half22float2(h10), b11 = __half22float2(h11);
-        acc = fmaf(s_a[j + 0], fmaf(b10.x, kPairInv, b00.x), acc);
-        acc = fmaf(s_a[j + 1], fmaf(b10.y, kPairInv, b00.y), acc);
-        acc = fmaf(s_a[j + 2], fmaf(b11.x, kPairInv, b01.x), acc);
-        acc = fmaf(s_a[j + 3], fmaf(b11.y, kPairInv, b01.y), acc);
-      };
-      if (THREADS > 256) {     // few rows: registers to spare for eight rounds of loads in flight
-#pragma unroll 8
-        for (int j = lane * 4; j < rf.K; j += 128) dot4(j);
-      } else {
-        for (int j = lane * 4; j < rf.K; j += 128) dot4(j);
-      }
+#pragma unroll 2
+      for (int j = j0 + lane * 8; j < j1; j += 256) {
+        const uint4 q0 = *reinterpret_cast<const uint4*>(w0 + j), q1 = *reinterpret_cast<const uint4*>(w1 + j);
+        const uint32_t u0[4] = {q0.x, q0.y, q0.z, q0.w}, u1[4] = {q1.x, q1.y, q1.z, q1.w};
+        const float4 x[2] = {*reinterpret_cast<const float4*>(s_a + j), *reinterpret_cast<const float4*>(s_a + j + 4)};
+        const float* xs = reinterpret_cast<const float*>(x);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) {
-        const float zv = acc + bias;
-        const float delta = __expf(zv - rmax) - __expf(za - rmax);
-        if (c < nc) { sh.cv[c] = zv; sh.cd[c] = delta; }
-        else { sh.eos = zv; sh.eos_delta = delta; }
+        for (int i = 0; i < 4; ++i) {
+          const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u0[i])), f1 = __half22float2(*reinterpret_cast<const __half2*>(&u1[i]));
+          acc = fmaf(xs[2 * i], fmaf(f1.x, kPairInv, f0.x), acc);
+          acc = fmaf(xs[2 * i + 1], fmaf(f1.y, kPairInv, f0.y), acc);
+        }
+      }
+      return warp_sum(acc);
+    };
+    auto done = [&](int c, float acc, float bias, float za) {
+      const float zv = acc + bias;
+      const float delta = __expf(zv - rmax) - __expf(za - rmax);
+      if (c < nc) { sh.cv[c] = zv; sh.cd[c] = delta; }
+      else { sh.eos = zv; sh.eos_delta = delta; }
+    };
+    if constexpr (THREADS > 256) {
+      // Few rows: the weight rows come from HBM, and their latency is most of the time.  Two warps share a candidate, so that
+      // all that a lane wants is in flight at once (K = 1024: four loads of 16 bytes): 5.2 us with a warp each.
+      float bias = 0.f, za = 0.f;      // (a thread completes a candidate; what it needs for that is requested first)
+      if (tid <= nc) {
+        const int v = tid < nc ? sh.ci[tid] : kEos;
+        bias = rf.bias ? rf.bias[v] : 0.f;
+        za = tid < nc ? sh.cv[tid] : zat(kEos);
+      }
+      const int half = warp & 1, mid = (rf.K >> 1) & ~7;
+      for (int c = warp >> 1; c <= nc; c += THREADS / 64) {
+        const float acc = dot(c < nc ? sh.ci[c] : kEos, half ? mid : 0, half ? rf.K : mid);
+        if (lane == 0) { if (c < nc) (half ? sh.co : sh.cd)[c] = acc; else sh.eos_half[half] = acc; }
+      }
+      __syncthreads();
+      if (tid <= nc) done(tid, tid < nc ? sh.cd[tid] + sh.co[tid] : sh.eos_half[0] + sh.eos_half[1], bias, za);
+      if (nc == THREADS && tid == 0) done(nc, sh.eos_half[0] + sh.eos_half[1], rf.bias ? rf.bias[kEos] : 0.f, zat(kEos));
+    } else {
+      for (int c = warp; c <= nc; c += THREADS / 32) {
+        const int v = (c < nc) ? sh.ci[c] : kEos;
+        // (what the sum is completed with is requested together with the weights)
+        const float bias = rf.bias ? rf.bias[v] : 0.f;
+        const float za = (c < nc) ? sh.cv[c] : zat(kEos);
+        const float acc = dot(v, 0, rf.K);
+        if (lane == 0) done(c, acc, bias, za);
       }
     }
   }
@@ -959,7 +1015,7 @@ __device__ __forceinline__ void topk_finish(TopkShared& sh, int r, float ssum, f
 static __global__ void __launch_bounds__(256, 6) softmax_topk_kernel(const float* __restrict__ logits, int ld, int V, int kk, TopkOut out,
                                                                   int normalise, const float* __restrict__ pmax, int pmax_ld, int n_slots, TopkRefine rf,
                                                                   const __half* __restrict__ logits16, const __grid_constant__ SelectArgs sel) {
-  extern __shared__ float s_a[];   // [rf.K] the row's activations in fp32 (refinement only)
+  extern __shared__ __align__(16) float s_a[];   // [rf.K] the row's activations in fp32 (refinement only)
   tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
   __shared__ float s_tmax[256];
@@ -1158,7 +1214,7 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) topk_b
                                                                            TopkOut out, int normalise, LogitBlocks bl, TopkRefine rf, const __grid_constant__ SelectArgs sel) {
   tc::pdl_launch_dependents();
   tc::pdl_wait();
-  extern __shared__ float dyn[];
+  extern __shared__ __align__(16) float dyn[];
   float* s_m = dyn;                  // [n] block maxima
   float* s_q = dyn + bl.n;           // [n] block sums
   float* s_a = dyn + 2 * bl.n;       // [rf.K] activations (refinement)

@@ -247,3 +247,30 @@ def test_finalisation_of_long_hypotheses(oracle, cuda_lib, steps):
             assert abs(e["score"][i, q] - o["score"][i, q]) <= RTOL_FP32 * abs(o["score"][i, q])
             np.testing.assert_allclose(e["align"][i, q, :n, :S], o["align"][i, q, :n, :S], rtol=2e-4, atol=1e-6)
     dec.close()
+
+
+@pytest.mark.parametrize("beam", [4, 5, 8, 15, 16, 17, 31])     # up to 32 candidates, two firsts of a row, one first
+@pytest.mark.parametrize("n,family,diversity", [(2, "peaked", 0.0), (60, "peaked", 0.5), (3, "zero", 0.0)])    # 1024 and 256 threads; ties
+def test_selection_from_the_candidates_of_a_step(cuda_lib, beam, n, family, diversity):
+    """A step's survivors follow from its candidates: score descending, then beam, then word; START is skipped, EOS leaves
+    without taking a slot.  Recomputed from the engine's own candidates in fp32 and in its order of operations (the product with a diversity of one half is exact): no tolerance."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(1, 64, 1000, 100, 1)
+    blob = synth.make_blob(d, 5, family="peaked") if family == "peaked" else np.zeros_like(synth.make_blob(d, 5))
+    sents = synth.make_sentences(n, 2, 6, d.Vs, 1.1, 9, lambda s: 8)
+    dec = decoder.Decoder(d, [blob], beam=beam, max_batch=n, max_src_len=8, max_steps=8, cp_beta=0.0, diversity=diversity)
+    e, k, f = dec.decode(sents, trace=True), dec.k, np.float32
+    dec.close()
+    assert k == beam
+    for i in range(n):
+        score = np.zeros(k, f)
+        for t in range(8):
+            cand = []
+            for b in range(1 if t == 0 else k):
+                for q in range(k + 1):
+                    v, lp = int(e["cand_tok"][i, t, b, q]), e["cand_logp"][i, t, b, q]
+                    cand.append((-((lp + score[b]) - f(q + 1) * f(diversity)), b, v))
+            want = [(v, b, -s) for s, b, v in sorted(cand) if v not in (0, 1)][:k]
+            got = list(zip(e["surv_tok"][i, t].tolist(), e["surv_parent"][i, t].tolist(), e["surv_score"][i, t]))
+            assert got == want, (i, t)
+            score = e["surv_score"][i, t].copy()
