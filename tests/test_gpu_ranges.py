@@ -271,6 +271,7 @@ def test_selection_from_the_candidates_of_a_step(cuda_lib, beam, n, family, dive
                     v, lp = int(e["cand_tok"][i, t, b, q]), e["cand_logp"][i, t, b, q]
                     cand.append((-((lp + score[b]) - f(q + 1) * f(diversity)), b, v))
             want = [(v, b, -s) for s, b, v in sorted(cand) if v not in (0, 1)][:k]
+            want += [(2, 0, f(-1e30))] * (k - len(want))       # fewer that survive than slots
             got = list(zip(e["surv_tok"][i, t].tolist(), e["surv_parent"][i, t].tolist(), e["surv_score"][i, t]))
             assert got == want, (i, t)
             score = e["surv_score"][i, t].copy()
