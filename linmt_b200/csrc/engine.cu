@@ -76,6 +76,8 @@ Engine::~Engine() {
   for (auto e : kt_ev_) cudaEventDestroy(e);
   for (auto& v : enc_events_) for (auto e : v) cudaEventDestroy(e);
   if (enc_start_ev_) cudaEventDestroy(enc_start_ev_);
+  for (auto e : mem_events_) if (e) cudaEventDestroy(e);
+  for (auto st : mem_streams_) if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
   for (auto st : enc_streams_) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
   if (stream) cudaStreamDestroy(stream);
 }
@@ -596,6 +598,41 @@ int Engine::step_tail(int t, int rows) {
 }
 
 // ---------------------------------------------------------------------------------------
+// Work of every member of an ensemble, `rows` rows each, that does not depend on the other members': on a stream per member
+// between two points of the main stream.  A member's kernels are a chain in which every product pays its start and its
+// epilogue with most of the chip idle (up to 64 rows) or waiting for its last tiles; another member's fill that in.  Beyond
+// 64 rows each product is shaped for half of the SMs, so that two run side by side in fewer, wider tiles.  Four members of
+// 4 x 1000 / 30k, us a step with the members one after another, on streams shaped for the whole chip, for half of it:
+// 12 rows 382, 327, 365; 48 rows 463, 377, 394; 96 rows 566, 513, 420; 192 rows 768, 710, 649; 384 rows 1020, 974, 939.
+// One after another where an alignment record adds the members up in their order, and where events time the kernels.
+int Engine::each_member(int rows, const std::function<int(int)>& work) {
+  if (!use_tc_ || n_models == 1 || d_rec_align_ || kernel_timing) {
+    for (int mi = 0; mi < n_models; ++mi)
+      if (int rc = work(mi)) return rc;
+    return LINMT_OK;
+  }
+  if (mem_streams_.empty()) {
+    mem_streams_.resize(n_models);
+    mem_events_.resize(n_models + 1);
+    for (auto& st : mem_streams_) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    for (auto& ev : mem_events_) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+  }
+  const cudaStream_t main_stream = stream;
+  CK(cudaEventRecord(mem_events_[n_models], main_stream));
+  int rc = LINMT_OK;
+  for (int mi = 0; mi < n_models; ++mi) {
+    CK(cudaStreamWaitEvent(mem_streams_[mi], mem_events_[n_models], 0));
+    stream = mem_streams_[mi];      // (tc_gemm: with this member's slice of the split-K workspace)
+    ws_part_ = mi; ws_parts_ = n_models; plan_parts_ = rows <= 64 ? 1 : 2;
+    if (rc == LINMT_OK) rc = work(mi);
+    stream = main_stream;
+    ws_part_ = 0; ws_parts_ = 1; plan_parts_ = 0;
+    CK(cudaEventRecord(mem_events_[mi], mem_streams_[mi]));
+    CK(cudaStreamWaitEvent(main_stream, mem_events_[mi], 0));   // (after an error too: the main stream stands for all of them)
+  }
+  return rc;
+}
+
 // Decode of one device batch (n <= max_batch); every data pointer is a device pointer.
 int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, const int32_t* steps_host, int max_len,
                         int32_t* d_out_tok, int32_t* d_out_len, float* d_out_score, int32_t* d_out_vit, float* d_out_align,
@@ -647,8 +684,7 @@ int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, co
     int n_act = 0;
     while (n_act < n && m_steps[n_act] >= t) ++n_act;
     if (n_act == 0) break;
-    for (int mi = 0; mi < n_models; ++mi)
-      if ((rc = use_tc_ ? run_decoder_step_tc(mi, t, n_act * k) : run_decoder_step(mi, t, n_act * k))) return rc;
+    if ((rc = each_member(n_act * k, [&](int mi) { return use_tc_ ? run_decoder_step_tc(mi, t, n_act * k) : run_decoder_step(mi, t, n_act * k); }))) return rc;
     if ((rc = step_tail(t, n_act * k))) return rc;
   }
   {

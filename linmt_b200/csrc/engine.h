@@ -123,6 +123,8 @@ class Engine {
   int run_decoder_step(int mi, int t, int rows);
   int run_encoder_tc(int n, int Smax);
   int run_encoder_layers_tc(int n, int Smax);   // few sentences: layer by layer
+  int encode_member_layers(int mi, int n, int Smax, int per);
+  int each_member(int rows, const std::function<int(int)>& work);
   // a step of scoring: the tokens read, where every member's htilde goes and where the previous step's is
   struct ScoreStep { const int32_t* tok; const tc::Planes* ht; const tc::Planes* ht_prev; };
   int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr);
@@ -170,6 +172,10 @@ class Engine {
   float* d_splitk_ws_ = nullptr;      // split-K partial tiles
   int* d_splitk_counters_ = nullptr;  // one arrival counter per output tile
   static constexpr size_t kSplitKWsFloats = (size_t)16 << 20;  // 64 MiB
+  // ensembles: a stream per member (see each_member)
+  std::vector<cudaStream_t> mem_streams_;
+  std::vector<cudaEvent_t> mem_events_;
+  int plan_parts_ = 0;                // products that run side by side, for the choice of their shapes (0: ws_parts_)
   int ws_part_ = 0, ws_parts_ = 1;    // slice of the workspace a launch may use (concurrent encoder layers get one each)
   static constexpr int kSplitKMaxTiles = 4096;
   std::vector<TcState> tc_states_;

@@ -100,7 +100,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   Epi e = e_in;
   if (nt <= 0 || nt > nt_) nt = nt_;
   tc::GemmLimits lim;
-  lim.n_sm = n_sm_; lim.parts = ws_parts_; lim.rows = rows_; lim.pair = pair_; lim.persist = persist_;
+  lim.n_sm = n_sm_; lim.parts = plan_parts_ ? plan_parts_ : ws_parts_; lim.rows = rows_; lim.pair = pair_; lim.persist = persist_;
   // a layer's slice of the split-K workspace: whole 256-byte units, so that every slice starts aligned for the
   // 16-byte partial-tile stores whatever the number of layers sharing it
   lim.ws_floats = (kSplitKWsFloats / ws_parts_) & ~(size_t)63;
@@ -251,7 +251,12 @@ int Engine::run_encoder_layers_tc(int n, int Smax) {
   hs_sent_ = 1; hs_pos_ = n;
   const int per = enc_rows_ / n;               // positions per chunk
   pdl_gemm_ = true;
-  for (int mi = 0; mi < n_models; ++mi) {
+  enc_final_row_ = (Smax - (Smax - 1) / per * per) * n;     // (of the last chunk)
+  return each_member(n, [&](int mi) { return encode_member_layers(mi, n, Smax, per); });
+}
+
+int Engine::encode_member_layers(int mi, int n, int Smax, int per) {
+  {
     DevModel& m = models_[mi];
     DevState& s = states_[mi];
     TcState& ts = tc_states_[mi];
@@ -296,7 +301,6 @@ int Engine::run_encoder_layers_tc(int n, int Smax) {
           if (int rc = tc_gemm(top, 0, enc_rows_, m.p_att_out_w, np * n, Hp, Hp, e)) return rc;
         }
       }
-      enc_final_row_ = np * n;
     }
   }
   return LINMT_OK;
@@ -461,11 +465,10 @@ int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const 
   std::vector<tc::Planes> prev = score_ht_, cur = score_ht_;
   size_t row = 0;
   for (int t = 0; t < steps; ++t) {
-    for (int mi = 0; mi < n_models; ++mi) {
+    for (int mi = 0; mi < n_models; ++mi)
       for (int p = 0; p < nt_; ++p) cur[mi].p[p] = score_ht_[mi].p[p] + row * Hp;
-      const ScoreStep sc{d_tok + (size_t)t * n, cur.data(), prev.data()};
-      if (int rc = run_decoder_step_tc(mi, t, n_act[t], &sc)) return rc;
-    }
+    const ScoreStep sc{d_tok + (size_t)t * n, cur.data(), prev.data()};
+    if (int rc = each_member(n_act[t], [&](int mi) { return run_decoder_step_tc(mi, t, n_act[t], &sc); })) return rc;
     prev = cur;
     row += n_act[t];
     stats.decoder_row_steps += n_act[t];
