@@ -486,7 +486,7 @@ int Engine::run_decoder_step(int mi, int t, int rows) {
 
 // Attention of one decoder forward (both GEMM families).
 int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
-                             float* ra, int32_t* rl, int32_t* rv, bool fold) {
+                             float* ra, int32_t* rl, int32_t* rv, bool fold, const tc::Planes& ctx2) {
   // the record of member mi: [n][Tm+1][k] at pt + mi * (sentences of this device batch's record) * (Tm+1) * k
   const AttTrace at{trace_dev_.pt ? trace_dev_.pt + (size_t)mi * trace_pt_member_stride_ : nullptr, d_orig_, trace_dev_.Tm + 1, t};
   DevModel& m = models_[mi];
@@ -500,7 +500,7 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
     if (cudaError_t e = tc::allow_smem<attention_kernel<G, kThreads>>(smem); e != cudaSuccess) return e;
     return tc::launch_k(pdl_, attention_kernel<G, kThreads>, dim3(rows / kb * groups), dim3(kThreads), smem, stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
                         (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, kb, groups, hs_sent_, hs_pos_, (int)opt.attention_mode,
-                        (int)opt.attention_d, ra, rl, rv, ctx_planes, nt, rec_win, ens_member_code(mi), at, af);
+                        (int)opt.attention_d, ra, rl, rv, ctx_planes, ctx2, nt, rec_win, ens_member_code(mi), at, af);
   };
   constexpr std::integral_constant<int, 1> one{};
   constexpr std::integral_constant<int, 2> two{};

@@ -44,8 +44,9 @@ struct DevModel {
 // Activation panels of the tensor-core path: every GEMM reads ONE K-contiguous panel, so the
 // producers write straight into the column range of the panel that consumes them.
 struct TcState {
-  tc::Planes panel1{};               // [R][3Hp]  x | h_prev(layer 0) | htilde_prev
-  std::vector<tc::Planes> panel;     // l = 1..L-1: [R][2Hp]  h_cur(l-1) | h_prev(l)
+  // (two of each: rows that continue themselves take turns, see run_decoder_step_tc)
+  tc::Planes panel1[2];              // [R][3Hp]  x | h_prev(layer 0) | htilde_prev
+  std::vector<tc::Planes> panel[2];  // l = 1..L-1: [R][2Hp]  h_cur(l-1) | h_prev(l)
   tc::Planes panel_top{};            // [R][2Hp]  ctx | h_cur(L-1)
   tc::Planes panel_ht{};             // [R][Hp]   htilde
   tc::Planes hs_planes{};            // [B * max_src][Hp]  the encoder's top states as operand planes (attention fold)
@@ -125,8 +126,8 @@ class Engine {
   int run_encoder_layers_tc(int n, int Smax);   // few sentences: layer by layer
   int encode_member_layers(int mi, int n, int Smax, int per);
   int each_member(int rows, const std::function<int(int)>& work);
-  // a step of scoring: the tokens read, where every member's htilde goes and where the previous step's is
-  struct ScoreStep { const int32_t* tok; const tc::Planes* ht; const tc::Planes* ht_prev; };
+  // a step of scoring: the tokens read, and where every member's htilde goes
+  struct ScoreStep { const int32_t* tok; const tc::Planes* ht; };
   int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr);
   int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum);
   cudaError_t softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel);
@@ -137,7 +138,7 @@ class Engine {
   bool weights_stream() const;
   bool pairs_available();   // clusters of two GEMM CTAs can be scheduled on the current device (engine_tc.cu)
   int launch_attention(int mi, int t, int rows, int kb, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
-                       float* rec_align, int32_t* rec_lo, int32_t* rec_vit, bool fold = false);
+                       float* rec_align, int32_t* rec_lo, int32_t* rec_vit, bool fold = false, const tc::Planes& ctx2 = tc::Planes{});
   int alloc_state_tc(TcState& s);
   int build_xw_tables();   // dec_xw of every model (tensor path, xw_table_)
   int alloc_planes(tc::Planes& p, size_t rows, int ld);

@@ -60,10 +60,12 @@ int Engine::to_planes(const std::vector<float>& host, size_t rows, int ld, tc::P
 
 int Engine::alloc_state_tc(TcState& s) {
   int rc;
-  if ((rc = alloc_planes(s.panel1, R, 3 * Hp))) return rc;
-  s.panel.resize(L);
-  for (int l = 1; l < L; ++l)
-    if ((rc = alloc_planes(s.panel[l], R, 2 * Hp))) return rc;
+  for (int i = 0; i < 2; ++i) {
+    if ((rc = alloc_planes(s.panel1[i], R, 3 * Hp))) return rc;
+    s.panel[i].resize(L);
+    for (int l = 1; l < L; ++l)
+      if ((rc = alloc_planes(s.panel[i][l], R, 2 * Hp))) return rc;
+  }
   if ((rc = alloc_planes(s.panel_top, R, 2 * Hp))) return rc;
   if ((rc = alloc_planes(s.panel_ht, R, Hp))) return rc;
   if (att_fold_ && (rc = alloc_planes(s.hs_planes, (size_t)B * opt.max_src_len, Hp))) return rc;
@@ -317,13 +319,23 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   // scoring: one row per sentence continues itself, its tokens are given, and every step's htilde is kept
   const int kb = sc ? 1 : k;
   const int32_t* tok = sc ? sc->tok : d_tok_;
-  const int32_t* parent = sc ? nullptr : d_parent_;
   const tc::Planes ht = sc ? sc->ht[mi] : ts.panel_ht;
-  const tc::Planes ht_prev = sc ? sc->ht_prev[mi] : ts.panel_ht;
+  // Rows that continue themselves (one beam slot, scoring) need no copy of their states between two steps: there are two sets
+  // of panels, and a step writes its states into the other set's h_prev and htilde_prev columns as well, while its own are
+  // being read.  A launch less in a chain of eight to nine.
+  const bool self = sc || (k == 1 && !trace_dev_.force_tok);
+  const int now = self ? t & 1 : 0, next = now ^ 1;
+  const int32_t* parent = self ? nullptr : d_parent_;
+  tc::Planes ht_next = no_planes();      // htilde_prev of the next step
+  if (self && desc.feed_input) {
+    ht_next = ts.panel1[next];
+    for (int p = 0; p < nt_; ++p) ht_next.p[p] += 2 * Hp;
+  }
   // where h_cur of layer l lives after its GEMM: the input slot of the consumer panel
-  auto hcur_planes = [&](int l) -> const tc::Planes& { return (l + 1 < L) ? ts.panel[l + 1] : ts.panel_top; };
+  auto hcur_planes = [&](int l) -> const tc::Planes& { return (l + 1 < L) ? ts.panel[now][l + 1] : ts.panel_top; };
   auto hcur_col0 = [&](int l) { return (l + 1 < L) ? 0 : Hp; };
-  auto hprev_planes = [&](int l) -> const tc::Planes& { return l == 0 ? ts.panel1 : ts.panel[l]; };
+  auto hprev_of = [&](int set, int l) -> const tc::Planes& { return l == 0 ? ts.panel1[set] : ts.panel[set][l]; };
+  auto hprev_planes = [&](int l) -> const tc::Planes& { return hprev_of(now, l); };
   // 1. gather states through the parents into the h_prev slots, look up embeddings
   {
     GatherJobs jobs{};
@@ -332,7 +344,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
       jobs.j[nj++] = GatherJob{static_cast<const unsigned char*>(src), sstride, static_cast<unsigned char*>(dst), dstride, bytes, kind};
     };
     const int fb = enc_final_buf_;
-    for (int l = 0; l < L; ++l) {
+    for (int l = 0; l < L && !(self && t > 0); ++l) {
       for (int p = 0; p < nt_; ++p) {
         const __nv_bfloat16* src;
         long long sst;
@@ -345,17 +357,19 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
       // reads it through the parent index and the two buffers swap roles every step
       if (t == 0) add(s.enc_c[fb][l], (long long)Hp * 4, s.c_prev[l], (long long)Hp * 4, Hp * 4, 0);
     }
-    if (feed)
+    if (feed && !self)
       for (int p = 0; p < nt_; ++p)
-        add(ht_prev.p[p], (long long)ht_prev.ld * 2, ts.panel1.p[p] + 2 * Hp, (long long)ts.panel1.ld * 2, Hp * 2, 0);
+        add(ts.panel_ht.p[p], (long long)ts.panel_ht.ld * 2, ts.panel1[0].p[p] + 2 * Hp, (long long)ts.panel1[0].ld * 2, Hp * 2, 0);
     if (!m.dec_xw)   // with the input-term table the embedding never enters the GEMM
       for (int p = 0; p < nt_; ++p)
-        add(m.p_emb_tgt.p[p], (long long)m.p_emb_tgt.ld * 2, ts.panel1.p[p], (long long)ts.panel1.ld * 2, Hp * 2, 1);
+        add(m.p_emb_tgt.p[p], (long long)m.p_emb_tgt.ld * 2, ts.panel1[now].p[p], (long long)ts.panel1[now].ld * 2, Hp * 2, 1);
     jobs.n = nj;
-    dim3 grid(rows, (nj + kGatherJobsPerBlock - 1) / kGatherJobsPerBlock);
-    if (int rc = kt(KC_GATHER)) return rc;
-    CK(tc::launch_k(pdl_, row_gather_kernel, grid, dim3(128), 0, stream, jobs, parent, tok, V, kb, t == 0 ? 1 : 0));
-    LAUNCHED();
+    if (nj > 0) {
+      dim3 grid(rows, (nj + kGatherJobsPerBlock - 1) / kGatherJobsPerBlock);
+      if (int rc = kt(KC_GATHER)) return rc;
+      CK(tc::launch_k(pdl_, row_gather_kernel, grid, dim3(128), 0, stream, jobs, parent, tok, V, kb, t == 0 ? 1 : 0));
+      LAUNCHED();
+    }
   }
   // 2. LSTM stack
   for (int l = 0; l < L; ++l) {
@@ -369,7 +383,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
       e.c_parent = parent; e.c_k = kb;
     }
     e.h_out1 = hcur_planes(l); e.h1_col0 = hcur_col0(l);
-    e.h_out2 = no_planes(); e.h2_col0 = 0;
+    e.h_out2 = self ? hprev_of(next, l) : no_planes(); e.h2_col0 = Hp;
     e.h_prev = no_planes(); e.hp_col0 = 0;
     e.h_f32 = (l == L - 1 && opt.attention_mode == LINMT_ATT_GLOBAL_DOT) ? s.h_cur[l] : nullptr;
     e.hf_row_stride = Hp;
@@ -413,11 +427,12 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
     int32_t* rl = rec ? d_rec_lo_ + (size_t)t * R : nullptr;
     int32_t* rv = rec ? d_rec_vit_ + (size_t)t * R : nullptr;
     if (int rc = kt(KC_ATTENTION)) return rc;
-    if (int rc = launch_attention(mi, t, rows, kb, u_alt, nullptr, att_fold_ ? ht : ts.panel_top, nt_, ra, rl, rv, att_fold_)) return rc;
+    if (int rc = launch_attention(mi, t, rows, kb, u_alt, nullptr, att_fold_ ? ht : ts.panel_top, nt_, ra, rl, rv, att_fold_, att_fold_ ? ht_next : no_planes())) return rc;
   }
   // 5. htilde = tanh(W_c1 ctx + W_c2 h + b) (with the fold the attention kernel has written it already)
   if (!att_fold_) {
     tc::TcEpiBiasTanh e{m.att_bout, ht, 0, nt_};
+    e.out2 = ht_next;
     if (int rc0 = kt(KC_ATTOUT)) return rc0;
     int rc;
     if (att_merge_) {
@@ -462,14 +477,13 @@ int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const 
   if (int rc = reserve_score(rows_all)) return rc;
   if (int rc = run_encoder_tc(n, Smax)) return rc;
   enc_final_buf_ = Smax & 1;
-  std::vector<tc::Planes> prev = score_ht_, cur = score_ht_;
+  std::vector<tc::Planes> cur = score_ht_;
   size_t row = 0;
   for (int t = 0; t < steps; ++t) {
     for (int mi = 0; mi < n_models; ++mi)
       for (int p = 0; p < nt_; ++p) cur[mi].p[p] = score_ht_[mi].p[p] + row * Hp;
-    const ScoreStep sc{d_tok + (size_t)t * n, cur.data(), prev.data()};
+    const ScoreStep sc{d_tok + (size_t)t * n, cur.data()};
     if (int rc = each_member(n_act[t], [&](int mi) { return run_decoder_step_tc(mi, t, n_act[t], &sc); })) return rc;
-    prev = cur;
     row += n_act[t];
     stats.decoder_row_steps += n_act[t];
     stats.sentence_steps += n_act[t];

@@ -638,6 +638,7 @@ struct TcEpiBiasTanh {
   Planes out; int col_off;
   int nt;
   const float* add = nullptr; int ld_add = 0;
+  Planes out2{};      // a second place for the same (p[0] == nullptr: none)
   static constexpr bool kHasBlock = false;
   static constexpr bool kHasPmax = false;
   static constexpr bool kHasPrefetch = false;
@@ -652,7 +653,9 @@ struct TcEpiBiasTanh {
         const float4 g = *reinterpret_cast<const float4*>(add + (size_t)row * ld_add + col0 + 4 * q);
         a.x += g.x; a.y += g.y; a.z += g.z; a.w += g.w;
       }
-      split_store4(out, nt, idx + 4 * q, tanh_fast(a.x + b.x), tanh_fast(a.y + b.y), tanh_fast(a.z + b.z), tanh_fast(a.w + b.w));
+      a = make_float4(tanh_fast(a.x + b.x), tanh_fast(a.y + b.y), tanh_fast(a.z + b.z), tanh_fast(a.w + b.w));
+      split_store4(out, nt, idx + 4 * q, a.x, a.y, a.z, a.w);
+      if (out2.p[0]) split_store4(out2, nt, (size_t)row * out2.ld + col0 + 4 * q, a.x, a.y, a.z, a.w);
     }
   }
   struct Pre { float4 a, b; };   // row form, see TcEpiLstm
@@ -664,8 +667,9 @@ struct TcEpiBiasTanh {
   }
   __device__ __forceinline__ void finish_row(bool valid, int row, int col, int /*lane*/, const float4& v, const Pre& p) const {
     if (!valid) return;
-    split_store4(out, nt, (size_t)row * out.ld + col_off + col, tanh_fast((v.x + p.a.x) + p.b.x), tanh_fast((v.y + p.a.y) + p.b.y),
-                 tanh_fast((v.z + p.a.z) + p.b.z), tanh_fast((v.w + p.a.w) + p.b.w));
+    const float4 a = make_float4(tanh_fast((v.x + p.a.x) + p.b.x), tanh_fast((v.y + p.a.y) + p.b.y), tanh_fast((v.z + p.a.z) + p.b.z), tanh_fast((v.w + p.a.w) + p.b.w));
+    split_store4(out, nt, (size_t)row * out.ld + col_off + col, a.x, a.y, a.z, a.w);
+    if (out2.p[0]) split_store4(out2, nt, (size_t)row * out2.ld + col, a.x, a.y, a.z, a.w);
   }
 };
 

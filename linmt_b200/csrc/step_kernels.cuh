@@ -173,7 +173,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // CreateCTKernel).
 //   proj [rows][2*Hp]: tanh(W_p h) | W_a^T h      (global_dot: `u` = h_top itself)
 //   hs   row sent * hs_sent + p * hs_pos: top encoder state of a sentence after consuming reversed position p
-//   ctx  [rows][Hp] fp32 and/or ctx_planes (bf16 planes, columns [0,Hp) of the panel)
+//   ctx  [rows][Hp] fp32 and/or ctx_planes (bf16 planes, columns [0,Hp) of the panel) and ctx2 (a second place for the same)
 //   rec_align [rows][rec_win] / rec_lo [rows] / rec_vit [rows]: alignment record of this step
 //   (may be null).  win = 2D+1 for local attention, max_src for the global modes.
 //   ens = 0: one model; the record is the window (rec_win = win) and its first position rec_lo.
@@ -212,7 +212,7 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
                                  const float* __restrict__ vp, const float* __restrict__ hs,
                                  const int32_t* __restrict__ src_len, float* __restrict__ ctx, int H, int Hp,
                                  int k, int groups, int hs_sent, int hs_pos, int mode, int D, float* __restrict__ rec_align,
-                                 int32_t* __restrict__ rec_lo, int32_t* __restrict__ rec_vit, tc::Planes ctx_planes, int nt,
+                                 int32_t* __restrict__ rec_lo, int32_t* __restrict__ rec_vit, tc::Planes ctx_planes, tc::Planes ctx2, int nt,
                                  int rec_win, int ens, AttTrace at, AttFold fold) {
   tc::pdl_launch_dependents();   // see gemm_tc.cuh: the next kernel of the step may start its prologue
   constexpr int kWarps = THREADS / 32;
@@ -444,6 +444,7 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
         if (ctx) *reinterpret_cast<float2*>(ctx + (size_t)r * Hp + j) = c;
         if (ctx_planes.p[0])    // tensor-core path: the context goes straight into its operand panel
           tc::split_store2(ctx_planes, nt, (size_t)r * ctx_planes.ld + j, c.x, c.y);
+        if (ctx2.p[0]) tc::split_store2(ctx2, nt, (size_t)r * ctx2.ld + j, c.x, c.y);
       }
     }
   } else {
@@ -477,6 +478,7 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
         }
         if (ctx) *reinterpret_cast<float4*>(ctx + (size_t)r0 * Hp + j) = acc;
         if (ctx_planes.p[0]) tc::split_store4(ctx_planes, nt, (size_t)r0 * ctx_planes.ld + j, acc.x, acc.y, acc.z, acc.w);
+        if (ctx2.p[0]) tc::split_store4(ctx2, nt, (size_t)r0 * ctx2.ld + j, acc.x, acc.y, acc.z, acc.w);
       }
     }
   }

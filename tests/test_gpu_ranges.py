@@ -275,3 +275,29 @@ def test_selection_from_the_candidates_of_a_step(cuda_lib, beam, n, family, dive
             got = list(zip(e["surv_tok"][i, t].tolist(), e["surv_parent"][i, t].tolist(), e["surv_score"][i, t]))
             assert got == want, (i, t)
             score = e["surv_score"][i, t].copy()
+
+
+@pytest.mark.parametrize("attention", ["local_p_general", "global_general", "global_dot"])
+@pytest.mark.parametrize("L,H,n,precision", [(1, 64, 1, "fp32"), (3, 250, 70, "fp32"), (2, 512, 150, "bf16")])   # few rows, one tile, two
+def test_rows_that_continue_themselves_take_turns_in_two_panels(cuda_lib, attention, L, H, n, precision):
+    """Greedy search and scoring leave a step's states where the next step reads them; a forced search copies them through
+    its parents.  The products are the same, so log-probabilities are the same bits."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(L, H, 400, 300, 1)
+    blob = synth.make_blob(d, 7, family="peaked")
+    sents = synth.make_sentences(n, 1, 9, d.Vs, 1.1, 4, lambda s: s + 3)
+    dec = decoder.Decoder(d, [blob], beam=1, max_batch=n, max_src_len=16, max_steps=16, cp_beta=0.0, attention=attention, precision=precision)
+    free = dec.decode(sents, trace=True)
+    forced = dec.decode(sents, trace=True, force=free)
+    for key in ("cand_tok", "cand_logp", "final_logp"):
+        assert free[key].tobytes() == forced[key].tobytes(), key
+    targets = [free["surv_tok"][i, :s, 0] for i, s in enumerate(sents.steps)]
+    total, per_token = dec.score(sents, targets)
+    dec.close()
+    for i, s in enumerate(sents.steps):      # the chosen word is a candidate of its step, unless that is START or EOS before it
+        t = np.arange(s)
+        hit = (free["cand_tok"][i, t, 0] == free["surv_tok"][i, t, 0][:, None])
+        want = np.where(hit, free["cand_logp"][i, t, 0], 0).sum(axis=1)
+        scale = np.maximum(1, np.abs(free["cand_logp"][i, t, 0]).max(axis=1))
+        tol = (2e-2 if precision == "bf16" else RTOL_FP32) * scale       # scoring multiplies other row counts: sums in another order
+        assert (np.abs(per_token[i, :s] - want) <= tol)[hit.any(axis=1)].all(), i
