@@ -247,8 +247,12 @@ int Engine::alloc_state(DevState& s) {
   DA(s.proj, 3 * rh); DA(s.ctx, rh);
   DA(s.logits, (size_t)R * Vp);
   if (logits16_) DA(s.logits16, (size_t)R * Vp);
-  DA(s.hs, (size_t)B * opt.max_src_len * Hp);
-  CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));   // rows past a sentence's end are never written, but read as GEMM operand rows by the fold
+  if (states16()) {
+    if (int rc = alloc_planes(s.hs16, (size_t)B * opt.max_src_len, Hp)) return rc;
+  } else {
+    DA(s.hs, (size_t)B * opt.max_src_len * Hp);
+    CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));   // rows past a sentence's end are never written, but read as GEMM operand rows by the fold
+  }
   if (att_fold_) DA(s.hs_wc1, (size_t)B * opt.max_src_len * Hp);
   DA(s.enc_x, (size_t)B * Hp);
   if (enc_rows_) DA(s.enc_pre, (size_t)enc_rows_ * 4 * Hp);
@@ -497,10 +501,14 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
   auto launch = [&](auto group, auto block, int groups, int positions) {
     constexpr int G = decltype(group)::value, kThreads = decltype(block)::value;
     const size_t smem = attention_smem(G, kThreads, Hp, positions);
-    if (cudaError_t e = tc::allow_smem<attention_kernel<G, kThreads>>(smem); e != cudaSuccess) return e;
-    return tc::launch_k(pdl_, attention_kernel<G, kThreads>, dim3(rows / kb * groups), dim3(kThreads), smem, stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
-                        (const float*)s.hs, (const int32_t*)d_len_, ctx, H, Hp, kb, groups, hs_sent_, hs_pos_, (int)opt.attention_mode,
+    auto of = [&](auto* hs) {
+      using T = std::remove_const_t<std::remove_pointer_t<decltype(hs)>>;
+      if (cudaError_t e = tc::allow_smem<attention_kernel<G, kThreads, T>>(smem); e != cudaSuccess) return e;
+      return tc::launch_k(pdl_, attention_kernel<G, kThreads, T>, dim3(rows / kb * groups), dim3(kThreads), smem, stream, (const float*)s.proj, ldp, u_alt, Hp, (const float*)m.vp,
+                        (const T*)hs, (const int32_t*)d_len_, ctx, H, Hp, kb, groups, hs_sent_, hs_pos_, (int)opt.attention_mode,
                         (int)opt.attention_d, ra, rl, rv, ctx_planes, ctx2, nt, rec_win, ens_member_code(mi), at, af);
+    };
+    return s.hs16.p[0] ? of((const __nv_bfloat16*)s.hs16.p[0]) : of((const float*)s.hs);
   };
   constexpr std::integral_constant<int, 1> one{};
   constexpr std::integral_constant<int, 2> two{};

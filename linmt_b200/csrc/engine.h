@@ -64,6 +64,7 @@ struct DevState {
   float* logits = nullptr;                           // [R][Vp]
   __half* logits16 = nullptr;                        // [R][Vp]  the same in fp16 (one-product logits whose candidates are recomputed)
   float* hs = nullptr;                               // [B][max_src][Hp]
+  tc::Planes hs16{};                                 // the same in bf16 (one plane: instead of hs)
   float* hs_wc1 = nullptr;                           // [B][max_src][Hp]  W_c1 . hs (tensor path with the attention fold)
   float* enc_x = nullptr;                            // [B][Hp]
   float* enc_pre = nullptr;                          // [rows][4Hp]  W_x . input of every position (encoder layer by layer)
@@ -120,6 +121,8 @@ class Engine {
   int ens_member_code(int mi) const { return n_models == 1 ? 0 : (mi == 0 ? 1 : (mi == n_models - 1 ? 3 : 2)); }
   int pack_model(const float* blob, DevModel& m);
   int alloc_state(DevState& s);
+  // one plane: the encoder's states are rounded to bf16, and kept as that (a sentence's, numbered in 32 bits)
+  bool states16() const { return use_tc_ && nt_ == 1 && (long long)opt.max_src_len * Hp < (1ll << 31); }
   int run_encoder(int n, int Smax);
   int run_decoder_step(int mi, int t, int rows);
   int run_encoder_tc(int n, int Smax);

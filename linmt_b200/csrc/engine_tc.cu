@@ -68,7 +68,7 @@ int Engine::alloc_state_tc(TcState& s) {
   }
   if ((rc = alloc_planes(s.panel_top, R, 2 * Hp))) return rc;
   if ((rc = alloc_planes(s.panel_ht, R, Hp))) return rc;
-  if (att_fold_ && (rc = alloc_planes(s.hs_planes, (size_t)B * opt.max_src_len, Hp))) return rc;
+  if (att_fold_ && !states16() && (rc = alloc_planes(s.hs_planes, (size_t)B * opt.max_src_len, Hp))) return rc;
   if (enc_rows_) {
     if ((rc = alloc_planes(s.enc_in, enc_rows_, Hp))) return rc;
     s.enc_seq.resize(L);
@@ -213,9 +213,9 @@ int Engine::run_encoder_tc(int n, int Smax) {
         tc::TcEpiLstm e{};
         e.bias = m.enc_b[l]; e.c_prev = s.enc_c[in][l]; e.ldc = Hp; e.c_out = s.enc_c[out][l];
         e.h_out1 = ts.encp[out][l]; e.h1_col0 = Hp;
-        if (l + 1 < L) { e.h_out2 = ts.encp[in][l + 1]; e.h2_col0 = 0; } else { e.h_out2 = no_planes(); e.h2_col0 = 0; }
+        if (l + 1 < L) { e.h_out2 = ts.encp[in][l + 1]; e.h2_col0 = 0; } else { e.h_out2 = s.hs16; e.h_out2.ld = (int)opt.max_src_len * Hp; e.h2_col0 = pos * Hp; }
         e.h_prev = ts.encp[in][l]; e.hp_col0 = Hp;
-        e.h_f32 = (l == L - 1) ? s.hs + (size_t)pos * Hp : nullptr;
+        e.h_f32 = (l == L - 1 && s.hs) ? s.hs + (size_t)pos * Hp : nullptr;
         e.hf_row_stride = (long long)opt.max_src_len * Hp;
         e.row_len = d_len_; e.pos = pos; e.nt = nt_;
         stream = sl;  // tc_gemm launches on the member stream, with this layer's slice of the split-K workspace
@@ -234,10 +234,12 @@ int Engine::run_encoder_tc(int n, int Smax) {
       // needs no output GEMM of its own (see AttFold in step_kernels.cuh).  Rows past a sentence's length hold
       // whatever an earlier batch left there; nothing reads their products.
       const size_t rows_all = (size_t)n * opt.max_src_len;
-      tc::split_planes_kernel<<<1024, 256, 0, main_stream>>>(s.hs, ts.hs_planes, nt_, rows_all * Hp);
-      LAUNCHED();
+      if (s.hs) {
+        tc::split_planes_kernel<<<1024, 256, 0, main_stream>>>(s.hs, ts.hs_planes, nt_, rows_all * Hp);
+        LAUNCHED();
+      }
       tc::TcEpiF32 e{nullptr, s.hs_wc1, Hp, 0};
-      if ((rc = tc_gemm(ts.hs_planes, 0, B * (int)opt.max_src_len, m.p_att_out_w, (int)rows_all, Hp, Hp, e))) return rc;
+      if ((rc = tc_gemm(s.hs ? ts.hs_planes : s.hs16, 0, B * (int)opt.max_src_len, m.p_att_out_w, (int)rows_all, Hp, Hp, e))) return rc;
     }
   }
   return LINMT_OK;
@@ -289,8 +291,9 @@ int Engine::encode_member_layers(int mi, int n, int Smax, int per) {
           e.h_out1 = seq; e.h1_col0 = 0;
           e.h_prev = seq; e.hp_col0 = 0;
           for (int t = 0; t < nt_; ++t) { e.h_out1.p[t] += (size_t)(q + 1) * n * Hp; e.h_prev.p[t] += (size_t)q * n * Hp; }
-          e.h_out2 = no_planes(); e.h2_col0 = 0;
-          e.h_f32 = (l == L - 1) ? s.hs + (size_t)pos * n * Hp : nullptr;
+          e.h_out2 = l == L - 1 ? s.hs16 : no_planes(); e.h2_col0 = 0;
+          if (e.h_out2.p[0]) e.h_out2.p[0] += (size_t)pos * n * Hp;
+          e.h_f32 = (l == L - 1 && s.hs) ? s.hs + (size_t)pos * n * Hp : nullptr;
           e.hf_row_stride = Hp;
           e.row_len = d_len_; e.pos = pos; e.nt = nt_;
           if (int rc = tc_gemm(seq, 0, enc_rows_ + tc::kRowsMax, wh, n, 4 * Hp, Hp, e, 0, 0, q * n)) return rc;

@@ -172,7 +172,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // CreateIndicesKernel, LoadInHSKernel, ElemReduceKernelLarge, AlignmentReductionKernel,
 // CreateCTKernel).
 //   proj [rows][2*Hp]: tanh(W_p h) | W_a^T h      (global_dot: `u` = h_top itself)
-//   hs   row sent * hs_sent + p * hs_pos: top encoder state of a sentence after consuming reversed position p
+//   hs   row sent * hs_sent + p * hs_pos: top encoder state of a sentence after consuming reversed position p, in T
 //   ctx  [rows][Hp] fp32 and/or ctx_planes (bf16 planes, columns [0,Hp) of the panel) and ctx2 (a second place for the same)
 //   rec_align [rows][rec_win] / rec_lo [rows] / rec_vit [rows]: alignment record of this step
 //   (may be null).  win = 2D+1 for local attention, max_src for the global modes.
@@ -207,9 +207,20 @@ struct AttFold {
 // G = 1, THREADS = 1024 for a step whose rows leave SMs empty: one position per warp and the context in four ranges of
 // positions (one sentence: 18.1 us per step with 256 threads, 10 so).  grid = sentences * groups, dynamic smem =
 // attention_smem
-template <int G, int THREADS>
+// T: the states as they are stored, fp32 or (one plane: they are rounded to it anyhow) bf16.  The kernel's time beyond its chain
+// is reading them out of L2 twice, for the scores and for the context.
+__device__ __forceinline__ float4 state4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float2 state2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 state2(uint32_t q) { return make_float2(__uint_as_float(q << 16), __uint_as_float(q & 0xffff0000u)); }
+__device__ __forceinline__ float2 state2(const __nv_bfloat16* p) { return state2(*reinterpret_cast<const uint32_t*>(p)); }
+__device__ __forceinline__ float4 state4(const __nv_bfloat16* p) {
+  const uint2 q = *reinterpret_cast<const uint2*>(p);
+  const float2 a = state2(q.x), b = state2(q.y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <int G, int THREADS, class T>
 static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attention_kernel(const float* __restrict__ proj, int ldp, const float* __restrict__ u_alt, int ldu,
-                                 const float* __restrict__ vp, const float* __restrict__ hs,
+                                 const float* __restrict__ vp, const T* __restrict__ hs,
                                  const int32_t* __restrict__ src_len, float* __restrict__ ctx, int H, int Hp,
                                  int k, int groups, int hs_sent, int hs_pos, int mode, int D, float* __restrict__ rec_align,
                                  int32_t* __restrict__ rec_lo, int32_t* __restrict__ rec_vit, tc::Planes ctx_planes, tc::Planes ctx2, int nt,
@@ -228,12 +239,12 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
     const int S = src_len[sent];
     const char* h0 = reinterpret_cast<const char*>(hs + (size_t)sent * hs_sent * Hp);
     const char* c0 = fold.cs ? reinterpret_cast<const char*>(fold.cs + (size_t)sent * hs_sent * Hp) : nullptr;
-    const int lines = Hp / 32;
+    const int lines = Hp / 32;         // (of fp32 rows; every other one where the states are half as wide)
     for (int i = q * THREADS + threadIdx.x; i < S * lines; i += groups * THREADS) {
-      const int pos = i / lines;
-      const size_t off = (size_t)pos * hs_pos * Hp * 4 + (size_t)(i - pos * lines) * 128;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(h0 + off));
-      if (c0) asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + off));
+      const int pos = i / lines, line = i - pos * lines;
+      const size_t row = (size_t)pos * hs_pos * Hp;
+      if (sizeof(T) == 4 || line % 2 == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(h0 + row * sizeof(T) + (size_t)line * (32 * sizeof(T))));
+      if (c0) asm volatile("prefetch.global.L2 [%0];" ::"l"(c0 + row * 4 + (size_t)line * 128));
     }
   }
   tc::pdl_wait();                // nothing below runs before the previous kernel's results are visible
@@ -248,7 +259,7 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
   __shared__ int s_lo[G], s_hi[G];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = sent * k + b0;
-  const float* hsb = hs + (size_t)sent * hs_sent * Hp;
+  const T* hsb = hs + (size_t)sent * hs_sent * Hp;
   auto row_of = [&](int g) { return r0 + (g < nb ? g : nb - 1); };
 
 #pragma unroll
@@ -303,13 +314,13 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
   constexpr int kAtOnce = G > 1 ? 2 : 1;
   for (int w = warp; w < W; w += kWarps * kAtOnce) {
     const int w2 = kAtOnce > 1 && w + kWarps < W ? w + kWarps : w;
-    const float* ha = hsb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp;
-    const float* hb = hsb + (size_t)(S - 1 - (lo + w2)) * hs_pos * Hp;
+    const T* ha = hsb + (size_t)(S - 1 - (lo + w)) * hs_pos * Hp;
+    const T* hb = hsb + (size_t)(S - 1 - (lo + w2)) * hs_pos * Hp;
     float acc[kAtOnce][G] = {};
     auto dot4 = [&](int j) {
       float4 a[kAtOnce];
-      a[0] = *reinterpret_cast<const float4*>(ha + j);
-      if (kAtOnce > 1) a[kAtOnce - 1] = *reinterpret_cast<const float4*>(hb + j);
+      a[0] = state4(ha + j);
+      if (kAtOnce > 1) a[kAtOnce - 1] = state4(hb + j);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         const float4 b = *reinterpret_cast<const float4*>(su + g * Hp + j);
@@ -406,8 +417,8 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
       }
     }
   // context: CreateCTKernel, deep_rnn_kernel.h:1250-1260
-  const float* csb = fold.cs ? fold.cs + (size_t)sent * hs_sent * Hp : hsb;
-  const float* col0 = csb + (size_t)(S - 1 - lo) * hs_pos * Hp;
+  auto context = [&](const auto* csb) {
+  const auto* col0 = csb + (size_t)(S - 1 - lo) * hs_pos * Hp;
   const size_t step = (size_t)hs_pos * Hp;
   if constexpr (kRanges == 1) {
     // a thread has two columns of every beam and sums the positions in order
@@ -415,10 +426,10 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
       float2 acc[G];
 #pragma unroll
       for (int g = 0; g < G; ++g) acc[g] = make_float2(0.f, 0.f);
-      const float* col = col0 + j;
+      const auto* col = col0 + j;
 #pragma unroll 6
       for (int w = 0; w < W; ++w) {
-        const float2 h = *reinterpret_cast<const float2*>(col - w * step);
+        const float2 h = state2(col - w * step);
         float a[GP];
         if constexpr (GP == 4) {
           *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(e + w * GP);
@@ -453,11 +464,11 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
       const int j = j0 + c * 4;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
       if (j < Hp) {
-        const float* col = col0 + j;
+        const auto* col = col0 + j;
 #pragma unroll 6
         for (int w = w0; w < w1; ++w) {
           const float a = e[w];
-          const float4 h4 = *reinterpret_cast<const float4*>(col - w * step);
+          const float4 h4 = state4(col - w * step);
           acc.x += a * h4.x; acc.y += a * h4.y; acc.z += a * h4.z; acc.w += a * h4.w;
         }
       }
@@ -482,6 +493,11 @@ static __global__ void __launch_bounds__(THREADS, THREADS == 512 ? 2 : 1) attent
       }
     }
   }
+  };
+  const float* folded = fold.cs ? fold.cs + (size_t)sent * hs_sent * Hp : nullptr;
+  if constexpr (sizeof(T) == 4) context(folded ? folded : hsb);
+  else if (folded) context(folded);
+  else context(hsb);
 }
 
 // `positions`: the window of one beam, the whole source where windows are joined.  Wide models and global attention over
