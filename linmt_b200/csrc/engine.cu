@@ -329,9 +329,9 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
     stream_weights_ = weights_stream();
     if (pair_ && !pairs_available()) pair_ = false;   // (a device that cannot co-schedule two such CTAs keeps the one-tile kernels)
   }
-  // panels of the layer-by-layer encoder: all positions of a batch if that is at most 16384 rows (0.27 GB of input parts)
+  // panels of the encoder by layers: all positions of a batch if that is at most 16384 rows (0.27 GB of input parts)
   if (use_tc_ && rows_ && (nt_ == 1 || fmt_ == 1)) {
-    const int nb = std::min(B, 64);
+    const int nb = std::min(B, kEncPipelined);
     enc_rows_ = std::min(opt.max_src_len * nb, std::max(16384, nb));
   }
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);

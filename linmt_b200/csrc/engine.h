@@ -128,6 +128,9 @@ class Engine {
   int run_encoder_tc(int n, int Smax);
   int run_encoder_layers_tc(int n, int Smax);   // few sentences: layer by layer
   int encode_member_layers(int mi, int n, int Smax, int per);
+  int run_encoder_pipeline_tc(int n, int Smax);   // more sentences: the layers side by side, a few positions behind each other
+  int encoder_streams();
+  int encode_positions(int mi, int l, int n, int pos0, int np, float* pre, int block);
   int each_member(int rows, const std::function<int(int)>& work);
   // a step of scoring: the tokens read, and where every member's htilde goes
   struct ScoreStep { const int32_t* tok; const tc::Planes* ht; };
@@ -188,6 +191,7 @@ class Engine {
   const int32_t* cur_ids_ = nullptr;
   // row of the encoder states of sentence b after position p: b * hs_sent_ + p * hs_pos_
   int hs_sent_ = 0, hs_pos_ = 1;
+  static constexpr int kEncPipelined = 128;   // sentences that the layers take side by side at most
   int enc_rows_ = 0;                    // rows (positions x sentences) the layer-by-layer encoder takes at a time
   int enc_final_row_ = -1;              // its final states: first row in enc_seq (-1: the other encoder ran)
   TraceDev trace_dev_{};

@@ -163,6 +163,20 @@ int Engine::build_xw_tables() {
   return LINMT_OK;
 }
 
+static constexpr int kEncRing = 4;
+static constexpr int kEncLag = 8;     // positions (64 sentences of 80 words: 3.32, 3.06, 3.20 ms with 4, 8, 14)
+int Engine::encoder_streams() {
+  if (!enc_streams_.empty()) return LINMT_OK;
+  enc_streams_.resize(L);
+  enc_events_.assign(L, std::vector<cudaEvent_t>(kEncRing));
+  for (int l = 0; l < L; ++l) {
+    CK(cudaStreamCreateWithFlags(&enc_streams_[l], cudaStreamNonBlocking));
+    for (int r = 0; r < kEncRing; ++r) CK(cudaEventCreateWithFlags(&enc_events_[l][r], cudaEventDisableTiming));
+  }
+  CK(cudaEventCreateWithFlags(&enc_start_ev_, cudaEventDisableTiming));
+  return LINMT_OK;
+}
+
 // Encoder, tensor-core path (see Engine::run_encoder for the reference procedure).  Panel of
 // layer l at position p: encp[p&1][l] = (input from below | h_prev).  The epilogue writes h to
 // the next position's h_prev slot and to the next layer's input slot of this position.
@@ -171,20 +185,19 @@ int Engine::build_xw_tables() {
 // the SMs (64 rows = one row tile), so the layers run as a wavefront: one stream per layer,
 // events for the cross-layer edges.  Besides the true dependencies, (l, p) waits for (l+1, p-2),
 // the last reader of the double-buffered input slot it overwrites.
+// Which of the three forms: see run_encoder_layers_tc and run_encoder_pipeline_tc.
 int Engine::run_encoder_tc(int n, int Smax) {
   decoding_ = false;
-  if (rows_ && n <= 64 && enc_rows_) return run_encoder_layers_tc(n, Smax);
-  constexpr int kRing = 4;
+  // Measured for 4 x 1000, ms a call of the encoder and two steps.  f16 pair, 80 words, layer by layer / pipelined / as a
+  // wavefront: 24 sentences 2.75, 2.87, 3.45; 32 2.85, 2.87, 3.46; 48 3.28, 2.92, 3.56; 64 3.88, 3.06, 3.62; 96 -, 3.28, 3.72;
+  // 50 words: 32 1.92, 2.15, 2.29; 48 2.17, 2.12, 2.33; 64 2.52, 2.23, 2.38.  One plane, 50 words: 24 1.32, 1.40, 1.39; 32 1.38,
+  // 1.41, 1.38; 64 1.78, 1.41, 1.43; 128 2.26, 1.61, 1.49.  Short sources spend the pipeline's lag filling it.
+  const bool lagged = nt_ > 1 && n_models == 1 && L > 1 && Smax >= 4 * kEncLag;
+  if (rows_ && enc_rows_ && (n <= 32 || (n <= 64 && nt_ > 1 && !lagged))) return run_encoder_layers_tc(n, Smax);
+  if (rows_ && lagged && n <= kEncPipelined && (size_t)n * Smax <= (size_t)enc_rows_) return run_encoder_pipeline_tc(n, Smax);
+  constexpr int kRing = kEncRing;
   hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;
-  if (enc_streams_.empty()) {
-    enc_streams_.resize(L);
-    enc_events_.assign(L, std::vector<cudaEvent_t>(kRing));
-    for (int l = 0; l < L; ++l) {
-      CK(cudaStreamCreateWithFlags(&enc_streams_[l], cudaStreamNonBlocking));
-      for (int r = 0; r < kRing; ++r) CK(cudaEventCreateWithFlags(&enc_events_[l][r], cudaEventDisableTiming));
-    }
-    CK(cudaEventCreateWithFlags(&enc_start_ev_, cudaEventDisableTiming));
-  }
+  if (int rc = encoder_streams()) return rc;
   cudaStream_t main_stream = stream;
   pdl_gemm_ = false;
   for (int mi = 0; mi < n_models; ++mi) {
@@ -245,7 +258,7 @@ int Engine::run_encoder_tc(int n, int Smax) {
   return LINMT_OK;
 }
 
-// Encoder for few sentences (up to 64), layer by layer.  A layer's input part W_x . x_p of ALL positions is one GEMM; what
+// Encoder for few sentences, layer by layer.  A layer's input part W_x . x_p of ALL positions is one GEMM; what
 // is left of the recurrence per position is W_h . h (half of the layer's weights, which then stay in L2 from one position
 // to the next) in the few-rows kernel, or for wide models in the one-tile kernel, with the input part added in the epilogue.  L x S short launches instead of S
 // rounds of L launches on L streams that each read the whole layer from HBM: one sentence of 30 words 1.28 -> 0.75 ms.
@@ -257,6 +270,81 @@ int Engine::run_encoder_layers_tc(int n, int Smax) {
   pdl_gemm_ = true;
   enc_final_row_ = (Smax - (Smax - 1) / per * per) * n;     // (of the last chunk)
   return each_member(n, [&](int mi) { return encode_member_layers(mi, n, Smax, per); });
+}
+
+// Positions pos0 .. pos0 + np of layer l, whose input parts are in `pre`: W_h . h in the few-rows kernel or in the one-tile
+// kernel, with the input part added in the epilogue.  Their states go into the layer's sequence panel from block `block` on.
+int Engine::encode_positions(int mi, int l, int n, int pos0, int np, float* pre, int block) {
+  DevModel& m = models_[mi];
+  DevState& s = states_[mi];
+  const tc::Planes& seq = tc_states_[mi].enc_seq[l];
+  tc::Planes wh = m.p_enc_w[l];
+  for (int t = 0; t < nt_; ++t) wh.p[t] += Hp;
+  for (int q = 0; q < np; ++q) {
+    const int pos = pos0 + q;
+    tc::TcEpiLstm e{};
+    e.bias = m.enc_b[l]; e.c_prev = s.enc_c[pos & 1][l]; e.ldc = Hp; e.c_out = s.enc_c[(pos & 1) ^ 1][l];
+    e.xw = pre + (size_t)q * n * 4 * Hp; e.x_ld = 4 * Hp;
+    e.h_out1 = seq; e.h1_col0 = 0;
+    e.h_prev = seq; e.hp_col0 = 0;
+    for (int t = 0; t < nt_; ++t) { e.h_out1.p[t] += (size_t)(block + q + 1) * n * Hp; e.h_prev.p[t] += (size_t)(block + q) * n * Hp; }
+    e.h_out2 = l == L - 1 ? s.hs16 : no_planes(); e.h2_col0 = 0;
+    if (e.h_out2.p[0]) e.h_out2.p[0] += (size_t)pos * n * Hp;
+    e.h_f32 = (l == L - 1 && s.hs) ? s.hs + (size_t)pos * n * Hp : nullptr;
+    e.hf_row_stride = Hp;
+    e.row_len = d_len_; e.pos = pos; e.nt = nt_;
+    if (int rc = tc_gemm(seq, 0, enc_rows_ + tc::kRowsMax, wh, n, 4 * Hp, Hp, e, 0, 0, (block + q) * n)) return rc;
+  }
+  return LINMT_OK;
+}
+
+// Encoder for more sentences: the layers side by side on a stream each, every one kEncLag positions behind the layer below.
+// As in the form above, the input parts of that many positions are one product, and what is left of the recurrence reads
+// half of a layer's weights, which all layers' together (67 MB in fp32 precision) stay in L2; but every layer's products are
+// shaped for their share of the SMs and run beside the others'.
+int Engine::run_encoder_pipeline_tc(int n, int Smax) {
+  if (int rc = encoder_streams()) return rc;
+  hs_sent_ = 1; hs_pos_ = n; enc_final_row_ = Smax * n;
+  const int share = enc_rows_ / L, lag = std::max(1, std::min(kEncLag, share / n));
+  const cudaStream_t main_stream = stream;
+  for (int mi = 0; mi < n_models; ++mi) {
+    DevModel& m = models_[mi];
+    DevState& s = states_[mi];
+    TcState& ts = tc_states_[mi];
+    for (int l = 0; l < L; ++l) {
+      CK(cudaMemsetAsync(s.enc_c[0][l], 0, sizeof(float) * (size_t)n * Hp, stream));
+      for (int t = 0; t < nt_; ++t) CK(cudaMemsetAsync(ts.enc_seq[l].p[t], 0, sizeof(uint16_t) * (size_t)n * Hp, stream));
+    }
+    enc_embed_seq_kernel<<<dim3(n, Smax, nt_), 128, 0, stream>>>(cur_ids_, d_off_, d_len_, m.p_emb_src, desc.vocab_src, ts.enc_in, Hp, 0);
+    LAUNCHED();
+    CK(cudaEventRecord(enc_start_ev_, main_stream));
+    for (int l = 0; l < L; ++l) CK(cudaStreamWaitEvent(enc_streams_[l], enc_start_ev_, 0));
+    pdl_gemm_ = true;
+    int rc = LINMT_OK;
+    for (int p0 = 0; p0 < Smax && rc == LINMT_OK; p0 += lag) {
+      const int np = std::min(lag, Smax - p0);
+      for (int l = 0; l < L && rc == LINMT_OK; ++l) {
+        if (l > 0) CK(cudaStreamWaitEvent(enc_streams_[l], enc_events_[l - 1][0], 0));
+        stream = enc_streams_[l];       // (tc_gemm: on the layer's stream, with its slice of the split-K workspace)
+        ws_part_ = l; ws_parts_ = L; plan_parts_ = L;
+        float* pre = s.enc_pre + (size_t)l * share * 4 * Hp;
+        tc::TcEpiF32 ei{nullptr, pre, 4 * Hp, 0};
+        rc = l == 0 ? tc_gemm(ts.enc_in, 0, enc_rows_, m.p_enc_w[0], np * n, 4 * Hp, Hp, ei, 0, 0, p0 * n)
+                    : tc_gemm(ts.enc_seq[l - 1], 0, enc_rows_ + tc::kRowsMax, m.p_enc_w[l], np * n, 4 * Hp, Hp, ei, 0, 0, (p0 + 1) * n);
+        if (rc == LINMT_OK) rc = encode_positions(mi, l, n, p0, np, pre, p0);
+        stream = main_stream;
+        ws_part_ = 0; ws_parts_ = 1; plan_parts_ = 0;
+        CK(cudaEventRecord(enc_events_[l][0], enc_streams_[l]));
+      }
+    }
+    for (int l = 0; l < L; ++l) CK(cudaStreamWaitEvent(main_stream, enc_events_[l][0], 0));
+    if (rc != LINMT_OK) return rc;
+    if (att_fold_) {      // W_c1 applied to the encoder states, once (see AttFold in step_kernels.cuh)
+      tc::TcEpiF32 e{nullptr, s.hs_wc1, Hp, 0};
+      if ((rc = tc_gemm(ts.enc_seq[L - 1], 0, enc_rows_ + tc::kRowsMax, m.p_att_out_w, Smax * n, Hp, Hp, e, 0, 0, n))) return rc;
+    }
+  }
+  return LINMT_OK;
 }
 
 int Engine::encode_member_layers(int mi, int n, int Smax, int per) {
@@ -281,23 +369,7 @@ int Engine::encode_member_layers(int mi, int n, int Smax, int per) {
         if (l > 0) for (int t = 0; t < nt_; ++t) in.p[t] += (size_t)n * Hp;
         tc::TcEpiF32 ei{nullptr, s.enc_pre, 4 * Hp, 0};
         if (int rc = tc_gemm(in, 0, enc_rows_, m.p_enc_w[l], np * n, 4 * Hp, Hp, ei)) return rc;
-        tc::Planes wh = m.p_enc_w[l];
-        for (int t = 0; t < nt_; ++t) wh.p[t] += Hp;
-        for (int q = 0; q < np; ++q) {
-          const int pos = p0 + q;
-          tc::TcEpiLstm e{};
-          e.bias = m.enc_b[l]; e.c_prev = s.enc_c[pos & 1][l]; e.ldc = Hp; e.c_out = s.enc_c[(pos & 1) ^ 1][l];
-          e.xw = s.enc_pre + (size_t)q * n * 4 * Hp; e.x_ld = 4 * Hp;
-          e.h_out1 = seq; e.h1_col0 = 0;
-          e.h_prev = seq; e.hp_col0 = 0;
-          for (int t = 0; t < nt_; ++t) { e.h_out1.p[t] += (size_t)(q + 1) * n * Hp; e.h_prev.p[t] += (size_t)q * n * Hp; }
-          e.h_out2 = l == L - 1 ? s.hs16 : no_planes(); e.h2_col0 = 0;
-          if (e.h_out2.p[0]) e.h_out2.p[0] += (size_t)pos * n * Hp;
-          e.h_f32 = (l == L - 1 && s.hs) ? s.hs + (size_t)pos * n * Hp : nullptr;
-          e.hf_row_stride = Hp;
-          e.row_len = d_len_; e.pos = pos; e.nt = nt_;
-          if (int rc = tc_gemm(seq, 0, enc_rows_ + tc::kRowsMax, wh, n, 4 * Hp, Hp, e, 0, 0, q * n)) return rc;
-        }
+        if (int rc = encode_positions(mi, l, n, p0, np, s.enc_pre, 0)) return rc;
         if (l == L - 1 && att_fold_) {
           // W_c1 applied to the encoder states, once: the attention sums these rows (see AttFold in step_kernels.cuh)
           tc::Planes top = seq;

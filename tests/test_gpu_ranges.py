@@ -301,3 +301,25 @@ def test_rows_that_continue_themselves_take_turns_in_two_panels(cuda_lib, attent
         scale = np.maximum(1, np.abs(free["cand_logp"][i, t, 0]).max(axis=1))
         tol = (2e-2 if precision == "bf16" else RTOL_FP32) * scale       # scoring multiplies other row counts: sums in another order
         assert (np.abs(per_token[i, :s] - want) <= tol)[hit.any(axis=1)].all(), i
+
+
+@pytest.mark.parametrize("n,longest", [(33, 32), (64, 45), (65, 33), (128, 40)])     # a last stretch of 8, 5, 1 and 8 positions
+def test_encoder_layers_side_by_side(cuda_lib, n, longest):
+    """Batches of 33 to 128 sentences of 32 and more words in fp32 precision encode with the layers a few positions behind each
+    other; with LINMT_TC_ROWS=0 they do so position by position.  Scores of both agree to the sums' rounding."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(3, 128, 300, 200, 1)
+    blob = synth.make_blob(d, 11, family="peaked")
+    sents = synth.make_sentences(n, 1, longest, d.Vs, 1.1, 6, lambda s: 4)
+    lens = sents.lengths()
+    assert lens.max() >= 32
+    kw = dict(beam=2, max_batch=n, max_src_len=48, max_steps=8, cp_beta=0.0)
+    rng = np.random.default_rng(n)
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 7, size=n)]
+    dec = decoder.Decoder(d, [blob], **kw)
+    ref = _with_env({"LINMT_TC_ROWS": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    a, again, b = dec.score(sents, targets), dec.score(sents, targets), ref.score(sents, targets)
+    dec.close(); ref.close()
+    assert np.array_equal(a[1], again[1])
+    scale = np.maximum(1, np.abs(b[1]).max(axis=1, keepdims=True))
+    assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
