@@ -193,7 +193,7 @@ int Engine::run_encoder_tc(int n, int Smax) {
   // 50 words: 32 1.92, 2.15, 2.29; 48 2.17, 2.12, 2.33; 64 2.52, 2.23, 2.38.  One plane, 50 words: 24 1.32, 1.40, 1.39; 32 1.38,
   // 1.41, 1.38; 64 1.78, 1.41, 1.43; 128 2.26, 1.61, 1.49.  Short sources spend the pipeline's lag filling it.
   const bool lagged = nt_ > 1 && n_models == 1 && L > 1 && Smax >= 4 * kEncLag;
-  if (rows_ && enc_rows_ && (n <= 32 || (n <= 64 && nt_ > 1 && !lagged))) return run_encoder_layers_tc(n, Smax);
+  if (rows_ && enc_rows_ && (n <= kEncLayers || (n <= 64 && nt_ > 1 && !lagged))) return run_encoder_layers_tc(n, Smax);
   if (rows_ && lagged && n <= kEncPipelined && (size_t)n * Smax <= (size_t)enc_rows_) return run_encoder_pipeline_tc(n, Smax);
   constexpr int kRing = kEncRing;
   hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;

@@ -61,7 +61,7 @@ inline GemmPlan plan_gemm(int M, int N, int K, int nt, int fmt, int drain, int a
   if (fmt == 1 && nt == 2 && K % 64 == 0) p.bk = (bn >= 240 && (size_t)N * K * 4 > ((size_t)96 << 20)) ? 32 : 64;
   const int mt = (M + BM - 1) / BM;
   // (a row offset is for the few-rows kernel and the one-tile kernel, which takes it where the former declines; its
-  // products are those of up to 64 sentences, a single row tile)
+  // products are those of up to 128 sentences, a single row tile)
   const bool alone = lim.parts == 1 && a_row0 == 0;
   const bool whole_k = splits == 1 && p.bk == 64;
   // The many-wave one-plane logits GEMM has a persistent pair form (measured at K = 1024, against one tile per CTA:

@@ -1566,7 +1566,8 @@ inline int pick_bn(int M, int N, int n_sm) {
 // issuer 58 ns whatever its width (now: 64 clocks or its columns), and charge too much, the more the narrower
 // the tile.  bf16 gate product, N = 4096, K = 2048, weights from HBM, predicted / measured: 16.4 / 10.4 us at 72 to 128
 // rows (86 tiles of 48 columns), 16.7 / 10.9 at 256, 17.3 / 12.1 at 384, 18.3 / 14.2 at 640, 20.6 / 19.2 at 1024.  The
-// shapes it picks are the ones measured; which others would be faster has not been.
+// shapes it picks are nevertheless within 2 % of the best of every width, split and pair form at 72 to 1024 rows (gates,
+// projections, attention output; both this model and the f16 pair's).
 // The f16 pair with 64-deep stages, measured: a k-block costs ~400 ns on narrow tiles (an MMA of 128 rows has a floor of
 // ~65 clocks however narrow it is) and 120 + 3.6 * bn ns on wider ones (the tensor pipe at
 // its practical rate); per tile ~6 us + 12 ns per column of prologue and epilogue; a split adds ~2 us plus

@@ -639,9 +639,11 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
   // threads; 768 rows 29.4 -> 25.3 us a launch, 1536 rows 30.9 -> 25.1.)
   __shared__ unsigned long long s_bound;
   __shared__ int s_listed;
+  constexpr int kDirect = 64;       // so few are ranked as they are (56 of them by the bound: 4.33 -> 4.38 ms in a call of 69 steps)
   int n_order = n;
   const unsigned long long* ranked = key;
-  if (n > 32) {
+  unsigned long long* order = listed;      // the result, in order
+  if (n > kDirect) {
     if (warp == 0) {
       const int need = k + __reduce_add_sync(0xffffffffu, lane < THREADS / 32 ? s_special[lane] : 0);
       const int firsts = cols > 16 ? 1 : 2, m = firsts * cols;
@@ -665,21 +667,26 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     __syncthreads();
     n_order = s_listed;
     ranked = listed;
+    order = key;
   }
-  // in order, over the keys (32 and fewer are their only reader's)
-  for (int c0 = 0; c0 < n_order; c0 += THREADS) {
-    const int c = c0 + tid;
+  // a thread counts the candidates before its own; four of a large block share one
+  const int share = THREADS > 256 && n_order <= THREADS / 4 ? 4 : 1;
+  for (int c0 = 0; c0 < n_order; c0 += THREADS / share) {
+    const int c = c0 + tid / share;
     const unsigned long long kc = c < n_order ? ranked[c] : 0ull;
     int p = 0;
     if (c < n_order) {
 #pragma unroll 4
-      for (int d = 0; d < n_order; ++d) {
+      for (int d = tid & (share - 1); d < n_order; d += share) {
         const unsigned long long kd = ranked[d];
         p += (kd > kc || (kd == kc && d < c)) ? 1 : 0;
       }
     }
-    if (n <= 32) __syncwarp();
-    if (c < n_order) key[p] = kc;
+    if (share > 1) {
+      p += __shfl_xor_sync(0xffffffffu, p, 1);
+      p += __shfl_xor_sync(0xffffffffu, p, 2);
+    }
+    if (c < n_order && (tid & (share - 1)) == 0) order[p] = kc;
   }
   __syncthreads();
   __shared__ int s_ntok[kMaxBeam + 1], s_npar[kMaxBeam + 1];
@@ -689,7 +696,7 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
     int ns = 0, nf = nf0;
     for (int p0 = 0; p0 < n_order && ns < k; p0 += 32) {
       const int p = p0 + lane;
-      const unsigned long long ko = p < n_order ? key[p] : 0ull;
+      const unsigned long long ko = p < n_order ? order[p] : 0ull;
       const unsigned int low = 0xFFFFFFFFu - (unsigned int)ko, ord = (unsigned int)(ko >> 32);
       const int v = p < n_order && (low & 0xFFFFFFu) != 0xFFFFFFu ? (int)(low & 0xFFFFFFu) : -1, b = (int)(low >> 24);
       const float sc = __uint_as_float((ord & 0x80000000u) ? (ord & 0x7FFFFFFFu) : ~ord);

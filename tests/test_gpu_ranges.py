@@ -249,7 +249,7 @@ def test_finalisation_of_long_hypotheses(oracle, cuda_lib, steps):
     dec.close()
 
 
-@pytest.mark.parametrize("beam", [4, 5, 8, 15, 16, 17, 31])     # up to 32 candidates, two firsts of a row, one first
+@pytest.mark.parametrize("beam", [4, 7, 8, 15, 16, 17, 31])     # up to 64 candidates, two firsts of a row, one first
 @pytest.mark.parametrize("n,family,diversity", [(2, "peaked", 0.0), (60, "peaked", 0.5), (3, "zero", 0.0)])    # 1024 and 256 threads; ties
 def test_selection_from_the_candidates_of_a_step(cuda_lib, beam, n, family, diversity):
     """A step's survivors follow from its candidates: score descending, then beam, then word; START is skipped, EOS leaves
