@@ -612,6 +612,7 @@ int Engine::step_tail(int t, int rows) {
 // 64 rows each product is shaped for half of the SMs, so that two run side by side in fewer, wider tiles.  Four members of
 // 4 x 1000 / 30k, us a step with the members one after another, on streams shaped for the whole chip, for half of it:
 // 12 rows 382, 327, 365; 48 rows 463, 377, 394; 96 rows 566, 513, 420; 192 rows 768, 710, 649; 384 rows 1020, 974, 939.
+// (One plane: shaped for the whole chip, so that the sums are in the order that they have one after another.)
 // One after another where an alignment record adds the members up in their order, and where events time the kernels.
 int Engine::each_member(int rows, const std::function<int(int)>& work) {
   if (!use_tc_ || n_models == 1 || d_rec_align_ || kernel_timing) {
@@ -631,7 +632,7 @@ int Engine::each_member(int rows, const std::function<int(int)>& work) {
   for (int mi = 0; mi < n_models; ++mi) {
     CK(cudaStreamWaitEvent(mem_streams_[mi], mem_events_[n_models], 0));
     stream = mem_streams_[mi];      // (tc_gemm: with this member's slice of the split-K workspace)
-    ws_part_ = mi; ws_parts_ = n_models; plan_parts_ = rows <= 64 ? 1 : 2;
+    ws_part_ = mi; ws_parts_ = n_models; plan_parts_ = rows <= 64 || nt_ == 1 ? 1 : 2;
     if (rc == LINMT_OK) rc = work(mi);
     stream = main_stream;
     ws_part_ = 0; ws_parts_ = 1; plan_parts_ = 0;

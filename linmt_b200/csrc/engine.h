@@ -191,8 +191,8 @@ class Engine {
   const int32_t* cur_ids_ = nullptr;
   // row of the encoder states of sentence b after position p: b * hs_sent_ + p * hs_pos_
   int hs_sent_ = 0, hs_pos_ = 1;
-  // most sentences that are encoded layer by layer whatever the precision and the length, and with the layers side by side
-  static constexpr int kEncLayers = 32, kEncPipelined = 128;
+  // most sentences that are encoded layer by layer, and with the layers side by side
+  static constexpr int kEncLayers = 64, kEncPipelined = 128;
   int enc_rows_ = 0;                    // rows (positions x sentences) the layer-by-layer encoder takes at a time
   int enc_final_row_ = -1;              // its final states: first row in enc_seq (-1: the other encoder ran)
   TraceDev trace_dev_{};

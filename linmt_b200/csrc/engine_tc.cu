@@ -191,9 +191,11 @@ int Engine::run_encoder_tc(int n, int Smax) {
   // Measured for 4 x 1000, ms a call of the encoder and two steps.  f16 pair, 80 words, layer by layer / pipelined / as a
   // wavefront: 24 sentences 2.75, 2.87, 3.45; 32 2.85, 2.87, 3.46; 48 3.28, 2.92, 3.56; 64 3.88, 3.06, 3.62; 96 -, 3.28, 3.72;
   // 50 words: 32 1.92, 2.15, 2.29; 48 2.17, 2.12, 2.33; 64 2.52, 2.23, 2.38.  One plane, 50 words: 24 1.32, 1.40, 1.39; 32 1.38,
-  // 1.41, 1.38; 64 1.78, 1.41, 1.43; 128 2.26, 1.61, 1.49.  Short sources spend the pipeline's lag filling it.
+  // 1.41, 1.38; 64 1.78, 1.41, 1.43; 128 2.26, 1.61, 1.49.  Short sources spend the pipeline's lag filling it.  (One plane stays with the
+  // layers up to 64: another order of sums rounds a state to the other bf16 neighbour now and then, and a near tie of two
+  // hypotheses is decided by that.)
   const bool lagged = nt_ > 1 && n_models == 1 && L > 1 && Smax >= 4 * kEncLag;
-  if (rows_ && enc_rows_ && (n <= kEncLayers || (n <= 64 && nt_ > 1 && !lagged))) return run_encoder_layers_tc(n, Smax);
+  if (rows_ && enc_rows_ && (n <= 32 || (n <= kEncLayers && !lagged))) return run_encoder_layers_tc(n, Smax);
   if (rows_ && lagged && n <= kEncPipelined && (size_t)n * Smax <= (size_t)enc_rows_) return run_encoder_pipeline_tc(n, Smax);
   constexpr int kRing = kEncRing;
   hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;
