@@ -323,3 +323,33 @@ def test_encoder_layers_side_by_side(cuda_lib, n, longest):
     assert np.array_equal(a[1], again[1])
     scale = np.maximum(1, np.abs(b[1]).max(axis=1, keepdims=True))
     assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
+
+
+@pytest.mark.parametrize("hidden", [128, 500])
+@pytest.mark.parametrize("n,longest", [(33, 496), (33, 497), (40, 1000), (64, 256), (64, 257)])     # 16,384 rows, just more, three chunks
+def test_encoder_of_long_sources_takes_chunks(cuda_lib, n, longest, hidden):
+    """33 to 64 sentences so long that the layers' panels do not hold all positions are encoded in chunks, in whichever form
+    reads half of a layer's weights per position, and not position by position: that is told from the launches, L a position
+    against L + 1.  Scores agree to the sums' rounding."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, hidden, 300, 200, 1)
+    blob = synth.make_blob(d, 11, family="peaked")
+    rng = np.random.default_rng(n)
+    lens = np.concatenate([[longest, longest - 1], rng.integers(1, longest, size=n - 2)]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    sents = synth.Sentences(synth.zipf_ids(rng, int(off[-1]), 1, d.Vs, 1.1), off, np.full(n, 1, np.int32))
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 4, size=n)]
+    kw = dict(beam=1, max_batch=n, max_src_len=longest, max_steps=8, cp_beta=0.0)
+    dec = decoder.Decoder(d, [blob], **kw)
+    ref = _with_env({"LINMT_TC_ROWS": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    launches = []
+    for h in (dec, ref):
+        before = h.stats()["kernel_launches"]
+        h.decode(sents)
+        launches.append(h.stats()["kernel_launches"] - before)
+    a, again, b = dec.score(sents, targets), dec.score(sents, targets), ref.score(sents, targets)
+    dec.close(); ref.close()
+    assert launches[1] >= 3 * longest > launches[0] >= 2 * longest, launches
+    assert np.array_equal(a[1], again[1])
+    scale = np.maximum(1, np.abs(b[1]).max(axis=1, keepdims=True))
+    assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
