@@ -1,0 +1,46 @@
+// encoder_form.h -- which form of the tensor-core encoder takes a batch.  Plain C++, so that the rule can be checked without
+// a device.
+#pragma once
+#include <algorithm>
+
+namespace linmt {
+
+// kWavefront   position by position: a layer's whole product per position, a stream per layer
+// kLayers      layer by layer: the input parts of all positions in one product, then W_h . h position by position
+// kPipelined   the layers side by side, each kEncLag positions behind the layer below, with input parts of that many positions
+enum class EncoderForm { kWavefront, kLayers, kPipelined };
+
+// most sentences that are encoded layer by layer, and with the layers side by side; 32 fill a quarter of the row tile that the
+// latter's products take, and are always faster in the few-rows kernel of the former
+constexpr int kEncLayers = 64, kEncPipelined = 128, kEncFew = 32;
+constexpr int kEncLag = 8;     // positions (4 x 1000, 64 sentences of 80 words: 3.32, 3.06, 3.20 ms with 4, 8, 14)
+
+struct EncoderModel {
+  int layers, hp;      // hidden size, rounded up to 64
+  int members;         // of the ensemble (its members are encoded side by side already)
+  bool split;          // fp32 weights (the f16 pair)
+};
+
+// n sentences, the longest of S words, on a handle that has the layers' panels.
+inline EncoderForm encoder_form(const EncoderModel& m, int n, int S) {
+  const EncoderForm other = n <= kEncLayers ? EncoderForm::kLayers : EncoderForm::kWavefront;
+  // (One plane stays with the layers up to 64: another order of sums rounds a state to the other bf16 neighbour now and then,
+  // and a near tie of two hypotheses is decided by that.)
+  if (n <= kEncFew || n > kEncPipelined || !m.split || m.members > 1 || m.layers < 2) return other;
+  // Measured with 2 to 5 layers of 128 to 2048 units and 16 to 96 words (ms of a call with two decoder steps).  A pipeline of L
+  // layers is filled and drained, and pays where the sources are long for that.  Against the wavefront (65 to 128 sentences,
+  // n = 96, pipelined / wavefront at 32, 64 and 96 words): 2 x 1000 1.09 / 1.26, 1.81 / 2.17, 2.56 / 3.07; 3 x 1000 1.48 / 1.51,
+  // 2.36 / 2.63, 3.22 / 3.73; 4 x 1000 1.76 / 1.68, 2.77 / 2.89, 3.69 / 4.35; 5 x 1000 2.27 / 1.90, 3.47 / 3.31, 4.63 / 4.83.
+  if (n > kEncLayers) return S >= kEncLag * std::max(4, 3 * (m.layers - 2)) ? EncoderForm::kPipelined : other;
+  // Against the layers (33 to 64 sentences, n = 33, pipelined / layers): 2 x 128 0.55 / 0.61, 0.88 / 1.02, 1.03 / 1.43; 2 x 1000
+  // 0.97 / 0.76, 1.60 / 1.31, 2.21 / 1.86; 4 x 512 1.00 / 1.01, 1.50 / 1.78, 1.97 / 2.56; 4 x 1000 1.57 / 1.36, 2.44 / 2.43, 3.24 /
+  // 3.52; 5 x 768 1.52 / 1.44, 2.24 / 2.59, 3.01 / 3.76.  Fitted, in us a position: side by side, the longer of issuing L launches
+  // and a product on 1/L of the SMs; one after another, L products of the few-rows kernel, which take a quarter longer from 49
+  // rows on and go from 8.4 to 14 us between 1024 and 1088 units.  What the fit takes is at most 6 % slower than the other.
+  const double h = m.hp / 1024.0, L = m.layers;
+  const double side = std::max(3.2 * L, 8 + 9 * h + 3.5 * h * h * h * (L - 1));
+  const double turn = L * (m.hp <= 1024 ? std::max(6.1, 3.0 + 5.85 * h) : 13.5 + 10 * (h - 1)) * (n > 48 ? 1.22 : 1.0);
+  return S >= 4 * kEncLag && (S + 6 * (L - 1)) * side < S * turn ? EncoderForm::kPipelined : other;
+}
+
+}  // namespace linmt

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/linmt_decoder.h"
+#include "encoder_form.h"
 #include "step_kernels.cuh"
 #include "gemm_tc.cuh"
 #include <array>
@@ -191,10 +192,8 @@ class Engine {
   const int32_t* cur_ids_ = nullptr;
   // row of the encoder states of sentence b after position p: b * hs_sent_ + p * hs_pos_
   int hs_sent_ = 0, hs_pos_ = 1;
-  // most sentences that are encoded layer by layer, and with the layers side by side
-  static constexpr int kEncLayers = 64, kEncPipelined = 128;
-  int enc_rows_ = 0;                    // rows (positions x sentences) the layer-by-layer encoder takes at a time
-  int enc_final_row_ = -1;              // its final states: first row in enc_seq (-1: the other encoder ran)
+  int enc_rows_ = 0;                    // rows (positions x sentences) of the layers' panels (0: position by position only)
+  int enc_final_row_ = -1;              // the final states in the panels: first row in enc_seq (-1: position by position)
   TraceDev trace_dev_{};
   size_t trace_pt_member_stride_ = 0;   // floats between two members' p_t records in the device trace buffer
   int enc_final_buf_ = 0;

@@ -5,6 +5,7 @@
 #include <cstring>
 #include <algorithm>
 
+#include "encoder_form.h"
 #include "engine.h"
 #include "gemm_plan.cuh"
 #include "gemm_tc.cuh"
@@ -164,7 +165,6 @@ int Engine::build_xw_tables() {
 }
 
 static constexpr int kEncRing = 4;
-static constexpr int kEncLag = 8;     // positions (64 sentences of 80 words: 3.32, 3.06, 3.20 ms with 4, 8, 14)
 int Engine::encoder_streams() {
   if (!enc_streams_.empty()) return LINMT_OK;
   enc_streams_.resize(L);
@@ -185,18 +185,15 @@ int Engine::encoder_streams() {
 // the SMs (64 rows = one row tile), so the layers run as a wavefront: one stream per layer,
 // events for the cross-layer edges.  Besides the true dependencies, (l, p) waits for (l+1, p-2),
 // the last reader of the double-buffered input slot it overwrites.
-// Which of the three forms: see run_encoder_layers_tc and run_encoder_pipeline_tc.
+// Which of the three forms: encoder_form (encoder_form.h).
 int Engine::run_encoder_tc(int n, int Smax) {
   decoding_ = false;
-  // Measured for 4 x 1000, ms a call of the encoder and two steps.  f16 pair, 80 words, layer by layer / pipelined / as a
-  // wavefront: 24 sentences 2.75, 2.87, 3.45; 32 2.85, 2.87, 3.46; 48 3.28, 2.92, 3.56; 64 3.88, 3.06, 3.62; 96 -, 3.28, 3.72;
-  // 50 words: 32 1.92, 2.15, 2.29; 48 2.17, 2.12, 2.33; 64 2.52, 2.23, 2.38.  One plane, 50 words: 24 1.32, 1.40, 1.39; 32 1.38,
-  // 1.41, 1.38; 64 1.78, 1.41, 1.43; 128 2.26, 1.61, 1.49.  Short sources spend the pipeline's lag filling it.  (One plane stays with the
-  // layers up to 64: another order of sums rounds a state to the other bf16 neighbour now and then, and a near tie of two
-  // hypotheses is decided by that.)
-  const bool lagged = nt_ > 1 && n_models == 1 && L > 1 && Smax >= 4 * kEncLag;
-  if (rows_ && enc_rows_ && (n <= 32 || (n <= kEncLayers && !lagged))) return run_encoder_layers_tc(n, Smax);
-  if (rows_ && enc_rows_ && lagged && (n <= kEncLayers || (n <= kEncPipelined && (size_t)n * Smax <= (size_t)enc_rows_))) return run_encoder_pipeline_tc(n, Smax);
+  if (enc_rows_)
+    switch (encoder_form(EncoderModel{L, Hp, n_models, nt_ > 1}, n, Smax)) {
+      case EncoderForm::kLayers: return run_encoder_layers_tc(n, Smax);
+      case EncoderForm::kPipelined: return run_encoder_pipeline_tc(n, Smax);
+      case EncoderForm::kWavefront: break;
+    }
   constexpr int kRing = kEncRing;
   hs_sent_ = opt.max_src_len; hs_pos_ = 1; enc_final_row_ = -1;
   if (int rc = encoder_streams()) return rc;
@@ -300,7 +297,7 @@ int Engine::encode_positions(int mi, int l, int n, int pos0, int np, float* pre,
   return LINMT_OK;
 }
 
-// Encoder for more sentences: the layers side by side on a stream each, every one kEncLag positions behind the layer below.
+// Encoder for more sentences and longer sources: the layers side by side on a stream each, every one kEncLag positions behind the layer below.
 // As in the form above, the input parts of that many positions are one product, and what is left of the recurrence reads
 // half of a layer's weights, which all layers' together (67 MB in fp32 precision) stay in L2; but every layer's products are
 // shaped for their share of the SMs and run beside the others'.  Sources longer than the panels are taken in chunks: the

@@ -326,9 +326,9 @@ def test_encoder_layers_side_by_side(cuda_lib, n, longest):
 
 
 @pytest.mark.parametrize("hidden", [128, 500])
-@pytest.mark.parametrize("n,longest", [(33, 496), (33, 497), (40, 1000), (64, 256), (64, 257)])     # 16,384 rows, just more, three chunks
+@pytest.mark.parametrize("n,longest", [(33, 496), (33, 497), (40, 1000), (64, 256), (64, 257), (100, 200)])     # 16,384 rows, just more, three chunks
 def test_encoder_of_long_sources_takes_chunks(cuda_lib, n, longest, hidden):
-    """33 to 64 sentences so long that the layers' panels do not hold all positions are encoded in chunks, in whichever form
+    """33 and more sentences so long that the layers' panels do not hold all positions are encoded in chunks, in whichever form
     reads half of a layer's weights per position, and not position by position: that is told from the launches, L a position
     against L + 1.  Scores agree to the sums' rounding."""
     from linmt_b200 import decoder
