@@ -43,4 +43,11 @@ inline EncoderForm encoder_form(const EncoderModel& m, int n, int S) {
   return S >= 4 * kEncLag && (S + 6 * (L - 1)) * side < S * turn ? EncoderForm::kPipelined : other;
 }
 
+// Sentences that the layers' panels of a handle are made for: those of the forms that its batches, of at most max_batch
+// sentences and max_words words, can take.
+inline int encoder_panel_sentences(const EncoderModel& m, int max_batch, int max_words) {
+  if (max_batch > kEncLayers && encoder_form(m, kEncLayers + 1, max_words) == EncoderForm::kPipelined) return std::min(max_batch, kEncPipelined);
+  return std::min(max_batch, kEncLayers);
+}
+
 }  // namespace linmt

@@ -331,7 +331,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   }
   // panels of the encoder by layers: all positions of a batch if that is at most 16384 rows (0.27 GB of input parts)
   if (use_tc_ && rows_ && (nt_ == 1 || fmt_ == 1)) {
-    const int nb = std::min(B, nt_ == 1 ? kEncLayers : kEncPipelined);     // (see run_encoder_tc)
+    const int nb = encoder_panel_sentences(EncoderModel{L, Hp, nm, nt_ > 1}, B, opt.max_src_len);
     enc_rows_ = std::min(opt.max_src_len * nb, std::max(16384, nb));
   }
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);

@@ -353,3 +353,26 @@ def test_encoder_of_long_sources_takes_chunks(cuda_lib, n, longest, hidden):
     assert np.array_equal(a[1], again[1])
     scale = np.maximum(1, np.abs(b[1]).max(axis=1, keepdims=True))
     assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
+
+
+@pytest.mark.parametrize("layers,members,hidden,longest", [(1, 1, 512, 128), (2, 2, 512, 128), (3, 1, 1024, 24)])
+def test_encoder_panels_only_for_forms_that_run(cuda_lib, layers, members, hidden, longest):
+    """One-layer models, ensembles and handles for short sources never run the layers side by side, so a handle for 128
+    sentences has no larger panels than one for 64: it grows by its encoder states, 12 bytes an element of a position's
+    state, and not by the panels' 20 + 4 L."""
+    import torch
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(layers, hidden, 100, 60, 1)
+    blobs = [synth.make_blob(d, 3 + m) for m in range(members)]
+
+    def held(max_batch):
+        before = torch.cuda.mem_get_info()[0]
+        dec = decoder.Decoder(d, blobs, beam=1, max_batch=max_batch, max_src_len=longest, max_steps=8)
+        after = torch.cuda.mem_get_info()[0]
+        dec.close()
+        return before - after
+
+    held(64)      # (the context's own memory)
+    grown = held(128) - held(64)
+    elements = members * 64 * longest * hidden
+    assert 6 * elements <= grown <= (12 + (20 + 4 * layers) // 2) * elements, grown / elements
