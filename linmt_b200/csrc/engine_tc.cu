@@ -349,8 +349,10 @@ int Engine::run_encoder_pipeline_tc(int n, int Smax) {
       for (int l = 0; l < L; ++l) CK(cudaStreamWaitEvent(main_stream, enc_events_[l][0], 0));
       if (rc != LINMT_OK) return rc;
       if (att_fold_) {      // W_c1 applied to the encoder states, once (see AttFold in step_kernels.cuh)
+        tc::Planes top = ts.enc_seq[L - 1];       // (past block 0; a row offset would keep the product off CTA pairs)
+        for (int t = 0; t < nt_; ++t) top.p[t] += (size_t)n * Hp;
         tc::TcEpiF32 e{nullptr, s.hs_wc1 + (size_t)c0 * n * Hp, Hp, 0};
-        if ((rc = tc_gemm(ts.enc_seq[L - 1], 0, enc_rows_ + tc::kRowsMax, m.p_att_out_w, len * n, Hp, Hp, e, 0, 0, n))) return rc;
+        if ((rc = tc_gemm(top, 0, enc_rows_, m.p_att_out_w, len * n, Hp, Hp, e))) return rc;
       }
     }
   }

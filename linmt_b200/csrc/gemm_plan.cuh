@@ -60,8 +60,8 @@ inline GemmPlan plan_gemm(int M, int N, int K, int nt, int fmt, int drain, int a
   p.bk = nt == 1 ? 64 : 32;
   if (fmt == 1 && nt == 2 && K % 64 == 0) p.bk = (bn >= 240 && (size_t)N * K * 4 > ((size_t)96 << 20)) ? 32 : 64;
   const int mt = (M + BM - 1) / BM;
-  // (a row offset is for the few-rows kernel and the one-tile kernel, which takes it where the former declines; its
-  // products are those of up to 128 sentences, a single row tile)
+  // (a row offset is for the few-rows kernel and the one-tile kernel: the encoder's positions, a single row tile where the
+  // former declines them, and its input parts of eight positions, up to eight row tiles shaped for a share of the SMs)
   const bool alone = lim.parts == 1 && a_row0 == 0;
   const bool whole_k = splits == 1 && p.bk == 64;
   // The many-wave one-plane logits GEMM has a persistent pair form (measured at K = 1024, against one tile per CTA:

@@ -376,3 +376,26 @@ def test_encoder_panels_only_for_forms_that_run(cuda_lib, layers, members, hidde
     grown = held(128) - held(64)
     elements = members * 64 * longest * hidden
     assert 6 * elements <= grown <= (12 + (20 + 4 * layers) // 2) * elements, grown / elements
+
+
+@pytest.mark.parametrize("hidden,n,longest", [(512, 64, 80), (512, 96, 64), (512, 128, 41)])
+def test_attention_output_over_encoder_states_runs_on_pairs(cuda_lib, hidden, n, longest):
+    """The product over all encoder states that follows the layers side by side is the only one of these calls whose shape
+    takes CTA pairs; the same products accumulate in the same order without them."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, hidden, 300, 200, 1)
+    blob = synth.make_blob(d, 11, family="peaked")
+    sents = synth.make_sentences(n, longest, longest, d.Vs, 1.1, 6, lambda s: 3)
+
+    def run():
+        dec = decoder.Decoder(d, [blob], beam=1, max_batch=n, max_src_len=longest, max_steps=8, cp_beta=0.0)
+        out = dec.decode(sents, trace=True)
+        pairs = dec.stats()["pair_launches"]
+        dec.close()
+        return out, pairs
+
+    a, pairs = run()
+    b, none = _with_env({"LINMT_TC_PAIR": "0"}, run)
+    assert pairs == 1 and none == 0
+    for key in ("cand_tok", "cand_logp", "final_logp"):
+        assert a[key].tobytes() == b[key].tobytes(), key
