@@ -399,3 +399,27 @@ def test_attention_output_over_encoder_states_runs_on_pairs(cuda_lib, hidden, n,
     assert pairs == 1 and none == 0
     for key in ("cand_tok", "cand_logp", "final_logp"):
         assert a[key].tobytes() == b[key].tobytes(), key
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("n", [33, 64])     # 132 and 256 rows: the few that two row tiles hold, and all of them
+def test_vocabulary_beyond_l2_on_persistent_pairs(cuda_lib, n, precision):
+    """Weights that L2 cannot hold beside the states (102 MB of vocabulary in one plane) are loaded as a stream, by the
+    persistent pairs of 129 to 256 rows too: the bits of the kernels without pairs."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(1, 512, 100000, 100, 1)
+    blob = synth.make_blob(d, 4, family="peaked")
+    sents = synth.make_sentences(n, 2, 6, d.Vs, 1.1, 5, lambda s: 3)
+
+    def run():
+        dec = decoder.Decoder(d, [blob], beam=4, precision=precision, max_batch=n, max_src_len=8, max_steps=8, cp_beta=0.0)
+        out = dec.decode(sents, trace=True)
+        pairs = dec.stats()["pair_launches"]
+        dec.close()
+        return out, pairs
+
+    a, pairs = run()
+    b, none = _with_env({"LINMT_TC_PAIR": "0"}, run)
+    assert pairs >= 4 and none == 0
+    for key in ("cand_tok", "cand_logp", "final_logp", "tok", "score"):
+        assert a[key].tobytes() == b[key].tobytes(), key
