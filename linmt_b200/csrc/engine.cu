@@ -326,7 +326,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
     DA(d_splitk_ws_, kSplitKWsFloats);
     DA(d_splitk_counters_, kSplitKMaxTiles);
     CK(cudaMemset(d_splitk_counters_, 0, sizeof(int) * kSplitKMaxTiles));
-    stream_weights_ = weights_stream();
+    CK(cudaDeviceGetAttribute(&l2_bytes_, cudaDevAttrL2CacheSize, o.device));
     if (pair_ && !pairs_available()) pair_ = false;   // (a device that cannot co-schedule two such CTAs keeps the one-tile kernels)
   }
   // panels of the encoder by layers: all positions of a batch if that is at most 16384 rows (0.27 GB of input parts)

@@ -142,7 +142,7 @@ class Engine {
   int reserve_score(size_t rows);
   TopkRefine refinement(const tc::Planes& ht) const;    // of one-product logits of these attentional states
   int step_tail(int t, int rows);
-  bool weights_stream() const;
+  bool step_streams(bool scoring, int rows) const;
   bool pairs_available();   // clusters of two GEMM CTAs can be scheduled on the current device (engine_tc.cu)
   int launch_attention(int mi, int t, int rows, int kb, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
                        float* rec_align, int32_t* rec_lo, int32_t* rec_vit, bool fold = false, const tc::Planes& ctx2 = tc::Planes{});
@@ -168,8 +168,8 @@ class Engine {
   bool att_merge_ = false; // tensor path: W_c2 . h_top computed with the attention projections (LINMT_ATT_MERGE=0: test knob)
   bool pmax_on_ = true;    // vocabulary GEMM hands block maxima to the softmax (LINMT_PMAX=0: test knob)
   bool pair_ = true;       // CTA pairs for the GEMM shapes that are down to two stages (LINMT_TC_PAIR=0: test knob)
-  bool stream_weights_ = false;  // the weights of a step do not fit L2
-  bool decoding_ = false;        // the products issued are a decoder step's (or the vocabulary products of scoring)
+  bool stream_weights_ = false;  // the products issued are a step's (or scoring's vocabulary products), whose weights do not fit L2
+  int l2_bytes_ = 0;
   bool rows_ = true;       // weight-streaming kernel for few rows (LINMT_TC_ROWS=0: test knob)
   bool persist_ = true;    // persistent kernel for the many-wave vocabulary GEMM (LINMT_TC_PERSIST=0: test knob)
   bool pdl_gemm_ = false;  // true while the decoder step issues its GEMMs (the encoder's wavefront does not take part)

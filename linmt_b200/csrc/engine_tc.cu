@@ -10,6 +10,7 @@
 #include "gemm_plan.cuh"
 #include "gemm_tc.cuh"
 #include "step_kernels.cuh"
+#include "weight_stream.h"
 
 namespace linmt {
 
@@ -116,7 +117,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   std::memcpy(tm.a, am, sizeof(tm.a));
   std::memcpy(tm.b, bm, sizeof(tm.b));
   // (one plane and many rows: tensor-bound, and its row tiles read the weights several times over: 1536 rows 29.5 -> 29.9 ms a call as a stream)
-  tm.stream_b = stream_weights_ && decoding_ && (nt > 1 || M <= 256);
+  tm.stream_b = stream_weights_ && (nt > 1 || M <= 256);
   if constexpr (Epi::kHasPmax) {
     if (e.pmax) {
       blocks_ = logit_blocks(e.pmax, e.psum, e.pmax_ld, N, K, plan.stat_tile, plan.stat_part);
@@ -130,12 +131,9 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   return LINMT_OK;
 }
 
-// A step reads more weights than L2 has room for beside the states (three quarters of it): they are loaded as a stream.
-bool Engine::weights_stream() const {
-  int l2 = 0;
-  if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, opt.device) != cudaSuccess) { cudaGetLastError(); return false; }
-  const size_t hh = (size_t)Hp * Hp, recurrent = (8 * (size_t)L + 4) * hh, vocab = (size_t)Vp * Hp;
-  return 2 * n_models * (nt_ * recurrent + nt_vocab_ * vocab) > (size_t)l2 / 4 * 3;
+// The weights of a step are loaded as a stream (weight_stream.h).
+bool Engine::step_streams(bool scoring, int rows) const {
+  return weights_stream(StepWeights{L, Hp, Vp, n_models, nt_, nt_vocab_}, (size_t)l2_bytes_, scoring, rows);
 }
 
 bool Engine::pairs_available() { return tc::max_resident_pairs<2, 64, 1, tc::TcEpiLstm>() > 0; }
@@ -187,7 +185,7 @@ int Engine::encoder_streams() {
 // the last reader of the double-buffered input slot it overwrites.
 // Which of the three forms: encoder_form (encoder_form.h).
 int Engine::run_encoder_tc(int n, int Smax) {
-  decoding_ = false;
+  stream_weights_ = false;
   if (enc_rows_)
     switch (encoder_form(EncoderModel{L, Hp, n_models, nt_ > 1}, n, Smax)) {
       case EncoderForm::kLayers: return run_encoder_layers_tc(n, Smax);
@@ -402,7 +400,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   TcState& ts = tc_states_[mi];
   const bool feed = desc.feed_input && t > 0;
   pdl_gemm_ = true;
-  decoding_ = true;
+  stream_weights_ = step_streams(sc != nullptr, rows);
   // scoring: one row per sentence continues itself, its tokens are given, and every step's htilde is kept
   const int kb = sc ? 1 : k;
   const int32_t* tok = sc ? sc->tok : d_tok_;
@@ -575,6 +573,7 @@ int Engine::score_core_tc(int n, int Smax, const std::vector<int>& n_act, const 
     stats.decoder_row_steps += n_act[t];
     stats.sentence_steps += n_act[t];
   }
+  stream_weights_ = step_streams(false, 0);
   for (size_t r0 = 0; r0 < rows_all; r0 += score_q_) {
     const int rows = (int)std::min<size_t>(score_q_, rows_all - r0);
     TopkOut o{score_idx_, score_candp_, score_eos_, score_stats_};
