@@ -423,3 +423,45 @@ def test_vocabulary_beyond_l2_on_persistent_pairs(cuda_lib, n, precision):
     assert pairs >= 4 and none == 0
     for key in ("cand_tok", "cand_logp", "final_logp", "tok", "score"):
         assert a[key].tobytes() == b[key].tobytes(), key
+
+
+@pytest.mark.parametrize("members,n,beam", [(2, 9, 7), (2, 13, 5), (3, 20, 7), (4, 43, 7)])      # 63, 65, 140 and 301 rows
+def test_members_side_by_side(oracle, cuda_lib, members, n, beam):
+    """Members decode on a stream each, beyond 64 rows in products shaped for half of the SMs: forced, against the oracle,
+    and the same bits in every call."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, 128, 20000, 300, 1)
+    blobs = [synth.make_blob(d, 40 + m, family="peaked") for m in range(members)]
+    sents = synth.make_sentences(n, 2, 12, d.Vs, 1.1, 3, lambda s: 2 + s // 3)
+    kw = dict(beam=beam, cp_beta=0.0, min_ratio=0.0)
+    o = oracle.decode(d, blobs, sents, trace=True, **kw)
+    dec = decoder.Decoder(d, blobs, max_batch=n, max_src_len=16, max_steps=20, **kw)
+    e = dec.decode(sents, trace=True, force=o)
+    worst, bad, skipped, compared = compare_forced(e, o, sents.steps, src_len=sents.lengths())
+    assert worst <= RTOL_FP32 and bad == 0 and skipped <= 0.1 * (skipped + compared), (worst, bad, skipped, compared)
+    for _ in range(3):
+        again = dec.decode(sents, trace=True, force=o)
+        for key in ("cand_tok", "cand_logp", "final_logp"):
+            assert e[key].tobytes() == again[key].tobytes(), key
+    dec.close()
+
+
+@pytest.mark.parametrize("attention", ["local_p_general", "global_dot"])
+@pytest.mark.parametrize("members,n,beam", [(3, 12, 5), (2, 40, 5), (3, 45, 7)])      # 60, 200 and 315 rows
+def test_members_side_by_side_in_one_plane(cuda_lib, members, n, beam, attention):
+    """bf16 members on a stream each run the products that they run one after another, as they do while kernels are timed:
+    the same bits, decoded and scored."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, 128, 20000, 300, 1)
+    blobs = [synth.make_blob(d, 40 + m, family="peaked") for m in range(members)]
+    sents = synth.make_sentences(n, 2, 12, d.Vs, 1.1, 3, lambda s: s + 2)
+    rng = np.random.default_rng(n)
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 10, size=n)]
+    dec = decoder.Decoder(d, blobs, beam=beam, precision="bf16", attention=attention, max_batch=n, max_src_len=16, max_steps=20, cp_beta=0.0)
+    side = dec.decode(sents, trace=True), dec.score(sents, targets)
+    dec.set_kernel_timing(True)
+    turn = dec.decode(sents, trace=True), dec.score(sents, targets)
+    dec.close()
+    for key in ("cand_tok", "cand_logp", "final_logp", "tok", "len", "score"):
+        assert side[0][key].tobytes() == turn[0][key].tobytes(), key
+    assert side[1][1].tobytes() == turn[1][1].tobytes()
