@@ -251,7 +251,8 @@ int Engine::alloc_state(DevState& s) {
     if (int rc = alloc_planes(s.hs16, (size_t)B * opt.max_src_len, Hp)) return rc;
   } else {
     DA(s.hs, (size_t)B * opt.max_src_len * Hp);
-    CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));   // rows past a sentence's end are never written, but read as GEMM operand rows by the fold
+    // rows past a sentence's end are never written, but read as GEMM operand rows by the fold
+    CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));
   }
   if (att_fold_) DA(s.hs_wc1, (size_t)B * opt.max_src_len * Hp);
   DA(s.enc_x, (size_t)B * Hp);
@@ -612,6 +613,10 @@ int Engine::step_tail(int t, int rows) {
 // 64 rows each product is shaped for half of the SMs, so that two run side by side in fewer, wider tiles.  Four members of
 // 4 x 1000 / 30k, us a step with the members one after another, on streams shaped for the whole chip, for half of it:
 // 12 rows 382, 327, 365; 48 rows 463, 377, 394; 96 rows 566, 513, 420; 192 rows 768, 710, 649; 384 rows 1020, 974, 939.
+// The line at 64 rows is that model's.  Others, 40 steps of 30-word sentences, ms a call one after another, on streams for the
+// whole chip, for half of it: two of 2 x 1000 96 rows 7.3, 6.6, 5.9, 192 rows 9.0, 7.6, 7.2; eight of 2 x 128 96 rows 18.5, 7.1,
+// 6.6; eight of 3 x 250 96 rows 22.8, 10.9, 10.0, 192 rows 24.5, 11.6, 12.0; two of 3 x 250 66 rows 5.4, 3.8, 4.1, 192 rows 6.1, 4.3,
+// 4.5; three of 5 x 512 66 rows 12.8, 8.3, 9.2, 192 rows 16.0, 9.9, 10.8 (narrow models keep the few-rows kernel's gain longer).
 // (One plane: shaped for the whole chip, so that the sums are in the order that they have one after another.)
 // One after another where an alignment record adds the members up in their order, and where events time the kernels.
 int Engine::each_member(int rows, const std::function<int(int)>& work) {

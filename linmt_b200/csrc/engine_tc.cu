@@ -116,7 +116,8 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   tc::TmapSet tm;
   std::memcpy(tm.a, am, sizeof(tm.a));
   std::memcpy(tm.b, bm, sizeof(tm.b));
-  // (one plane and many rows: tensor-bound, and its row tiles read the weights several times over: 1536 rows 29.5 -> 29.9 ms a call as a stream)
+  // (one plane and many rows: tensor-bound, and its row tiles read the weights several times over: 1536 rows 29.5 -> 29.9 ms a
+  // call as a stream)
   tm.stream_b = stream_weights_ && (nt > 1 || M <= 256);
   if constexpr (Epi::kHasPmax) {
     if (e.pmax) {
@@ -255,11 +256,11 @@ int Engine::run_encoder_tc(int n, int Smax) {
   return LINMT_OK;
 }
 
-// Encoder for few sentences, layer by layer.  A layer's input part W_x . x_p of ALL positions is one GEMM; what
-// is left of the recurrence per position is W_h . h (half of the layer's weights, which then stay in L2 from one position
-// to the next) in the few-rows kernel, or for wide models in the one-tile kernel, with the input part added in the epilogue.  L x S short launches instead of S
-// rounds of L launches on L streams that each read the whole layer from HBM: one sentence of 30 words 1.28 -> 0.75 ms.
-// Block p of a layer's sequence panel holds its states after p positions (block 0 the state before): operand of the next
+// Encoder for few sentences, layer by layer.  A layer's input part W_x . x_p of ALL positions is one GEMM; what is left of the
+// recurrence per position is W_h . h (half of the layer's weights, which then stay in L2 from one position to the next) in the
+// few-rows kernel, or for wide models in the one-tile kernel, with the input part added in the epilogue.  L x S short launches
+// instead of S rounds of L launches on L streams that each read the whole layer from HBM: one sentence of 30 words 1.28 -> 0.75
+// ms.  Block p of a layer's sequence panel holds its states after p positions (block 0 the state before): operand of the next
 // position and, as a whole, of the next layer's input GEMM.  Sources longer than the panels are taken in chunks.
 int Engine::run_encoder_layers_tc(int n, int Smax) {
   hs_sent_ = 1; hs_pos_ = n;
@@ -357,36 +358,35 @@ int Engine::run_encoder_pipeline_tc(int n, int Smax) {
   return LINMT_OK;
 }
 
+// One member, in chunks of `per` positions.
 int Engine::encode_member_layers(int mi, int n, int Smax, int per) {
-  {
-    DevModel& m = models_[mi];
-    DevState& s = states_[mi];
-    TcState& ts = tc_states_[mi];
+  DevModel& m = models_[mi];
+  DevState& s = states_[mi];
+  TcState& ts = tc_states_[mi];
+  for (int l = 0; l < L; ++l) {
+    CK(cudaMemsetAsync(s.enc_c[0][l], 0, sizeof(float) * (size_t)n * Hp, stream));
+    for (int t = 0; t < nt_; ++t) CK(cudaMemsetAsync(ts.enc_seq[l].p[t], 0, sizeof(uint16_t) * (size_t)n * Hp, stream));
+  }
+  for (int p0 = 0; p0 < Smax; p0 += per) {
+    const int np = std::min(per, Smax - p0);
+    enc_embed_seq_kernel<<<dim3(n, np, nt_), 128, 0, stream>>>(cur_ids_, d_off_, d_len_, m.p_emb_src, desc.vocab_src, ts.enc_in, Hp, p0);
+    LAUNCHED();
     for (int l = 0; l < L; ++l) {
-      CK(cudaMemsetAsync(s.enc_c[0][l], 0, sizeof(float) * (size_t)n * Hp, stream));
-      for (int t = 0; t < nt_; ++t) CK(cudaMemsetAsync(ts.enc_seq[l].p[t], 0, sizeof(uint16_t) * (size_t)n * Hp, stream));
-    }
-    for (int p0 = 0; p0 < Smax; p0 += per) {
-      const int np = std::min(per, Smax - p0);
-      enc_embed_seq_kernel<<<dim3(n, np, nt_), 128, 0, stream>>>(cur_ids_, d_off_, d_len_, m.p_emb_src, desc.vocab_src, ts.enc_in, Hp, p0);
-      LAUNCHED();
-      for (int l = 0; l < L; ++l) {
-        const tc::Planes& seq = ts.enc_seq[l];
-        if (p0 > 0)   // the state the previous chunk ended with
-          for (int t = 0; t < nt_; ++t)
-            CK(cudaMemcpyAsync(seq.p[t], seq.p[t] + (size_t)per * n * Hp, sizeof(uint16_t) * (size_t)n * Hp, cudaMemcpyDeviceToDevice, stream));
-        tc::Planes in = l == 0 ? ts.enc_in : ts.enc_seq[l - 1];
-        if (l > 0) for (int t = 0; t < nt_; ++t) in.p[t] += (size_t)n * Hp;
-        tc::TcEpiF32 ei{nullptr, s.enc_pre, 4 * Hp, 0};
-        if (int rc = tc_gemm(in, 0, enc_rows_, m.p_enc_w[l], np * n, 4 * Hp, Hp, ei)) return rc;
-        if (int rc = encode_positions(mi, l, n, p0, np, s.enc_pre, 0)) return rc;
-        if (l == L - 1 && att_fold_) {
-          // W_c1 applied to the encoder states, once: the attention sums these rows (see AttFold in step_kernels.cuh)
-          tc::Planes top = seq;
-          for (int t = 0; t < nt_; ++t) top.p[t] += (size_t)n * Hp;
-          tc::TcEpiF32 e{nullptr, s.hs_wc1 + (size_t)p0 * n * Hp, Hp, 0};
-          if (int rc = tc_gemm(top, 0, enc_rows_, m.p_att_out_w, np * n, Hp, Hp, e)) return rc;
-        }
+      const tc::Planes& seq = ts.enc_seq[l];
+      if (p0 > 0)   // the state the previous chunk ended with
+        for (int t = 0; t < nt_; ++t)
+          CK(cudaMemcpyAsync(seq.p[t], seq.p[t] + (size_t)per * n * Hp, sizeof(uint16_t) * (size_t)n * Hp, cudaMemcpyDeviceToDevice, stream));
+      tc::Planes in = l == 0 ? ts.enc_in : ts.enc_seq[l - 1];
+      if (l > 0) for (int t = 0; t < nt_; ++t) in.p[t] += (size_t)n * Hp;
+      tc::TcEpiF32 ei{nullptr, s.enc_pre, 4 * Hp, 0};
+      if (int rc = tc_gemm(in, 0, enc_rows_, m.p_enc_w[l], np * n, 4 * Hp, Hp, ei)) return rc;
+      if (int rc = encode_positions(mi, l, n, p0, np, s.enc_pre, 0)) return rc;
+      if (l == L - 1 && att_fold_) {
+        // W_c1 applied to the encoder states, once: the attention sums these rows (see AttFold in step_kernels.cuh)
+        tc::Planes top = seq;
+        for (int t = 0; t < nt_; ++t) top.p[t] += (size_t)n * Hp;
+        tc::TcEpiF32 e{nullptr, s.hs_wc1 + (size_t)p0 * n * Hp, Hp, 0};
+        if (int rc = tc_gemm(top, 0, enc_rows_, m.p_att_out_w, np * n, Hp, Hp, e)) return rc;
       }
     }
   }

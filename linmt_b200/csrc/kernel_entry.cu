@@ -1,5 +1,5 @@
 // kernel_entry.cu -- single-kernel entry points of the C ABI (host pointers), used by the
-// parity tests to check one kernel at a time against the CPU checker.
+// parity tests to check one kernel at a time against the CPU oracle.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

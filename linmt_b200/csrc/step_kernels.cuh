@@ -639,7 +639,9 @@ __device__ __forceinline__ void beam_select_block(const SelectArgs& a, const Top
   // threads; 768 rows 29.4 -> 25.3 us a launch, 1536 rows 30.9 -> 25.1.)
   __shared__ unsigned long long s_bound;
   __shared__ int s_listed;
-  constexpr int kDirect = 64;       // so few are ranked as they are (56 of them by the bound: 4.33 -> 4.38 ms in a call of 69 steps)
+  // so few are ranked as they are (a beam of 7: 56 of them by the bound 4.33 -> 4.38 ms in a call of 69 steps; 12: 156 gain by it,
+  // as above; nothing between was measured)
+  constexpr int kDirect = 64;
   int n_order = n;
   const unsigned long long* ranked = key;
   unsigned long long* order = listed;      // the result, in order

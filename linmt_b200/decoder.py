@@ -78,7 +78,7 @@ class Decoder:
 
     def decode(self, sents, *, trace=False, force=None, want_align=False):
         """``sents``: a ``synth.Sentences``.  Returns a dict of numpy arrays shaped like the
-        CPU checker's output."""
+        CPU oracle's output."""
         n = sents.n
         ids = np.ascontiguousarray(sents.ids, np.int32)
         off = np.ascontiguousarray(sents.off, np.int32)

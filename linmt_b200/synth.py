@@ -3,7 +3,7 @@
 The reference project ships no trained model, so every measurement and parity case runs on
 random-initialised weights of the named architecture and on random sentences with the named
 length and token-frequency distributions.  One weight blob is read by both the CUDA engine
-and the CPU checker, so the generator's own RNG is free (numpy ``default_rng``).
+and the CPU oracle, so the generator's own RNG is free (numpy ``default_rng``).
 
 Blob layout = the reference's device memory after ``LoadWeights`` (src/deep_rnn.h:1878-1969):
 matrices in file order, each ``rows x cols`` column-major (src/utility_cu.h:37), i.e. a
