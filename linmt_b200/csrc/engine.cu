@@ -255,6 +255,7 @@ int Engine::alloc_state(DevState& s) {
     CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));
   }
   if (att_fold_) DA(s.hs_wc1, (size_t)B * opt.max_src_len * Hp);
+  if (rec_rows_) DA(s.rec, (size_t)(L + 1) * rec_rows_ * 4 * Hp);
   DA(s.enc_x, (size_t)B * Hp);
   if (enc_rows_) DA(s.enc_pre, (size_t)enc_rows_ * 4 * Hp);
   for (int i = 0; i < 2; ++i) {
@@ -334,6 +335,11 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   if (use_tc_ && rows_ && (nt_ == 1 || fmt_ == 1)) {
     const int nb = encoder_panel_sentences(EncoderModel{L, Hp, nm, nt_ > 1}, B, opt.max_src_len);
     enc_rows_ = std::min(opt.max_src_len * nb, std::max(16384, nb));
+  }
+  // (LINMT_AHEAD=0: test knob.  Narrower models gain nothing: 2 x 128, one row 1.04 -> 1.09 ms a call of 30 steps)
+  {
+    const char* pe = std::getenv("LINMT_AHEAD");
+    if (use_tc_ && rows_ && xw_table_ && nm == 1 && L > 1 && Hp >= 256 && (nt_ == 1 || fmt_ == 1) && !(pe && std::atoi(pe) == 0)) rec_rows_ = std::min(R, k > 1 ? tc::kRowsAhead : kRowsAheadSelf);
   }
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);
   for (int i = 0; i < nm; ++i) {
@@ -540,8 +546,8 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
 }
 
 // Softmax statistics and top-k of rows whose logits vocab_gemm has just produced, from the block statistics it left if it did.
-cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel) {
-  return launch_topk(logits, logits16_ ? logits16 : nullptr, Vp, V, kk, rows, n_sm_, o, normalise, blocks_, rf, sel, stream, pdl_);
+cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel, bool late) {
+  return launch_topk(logits, logits16_ ? logits16 : nullptr, Vp, V, kk, rows, n_sm_, o, normalise, blocks_, rf, sel, stream, pdl_, late);
 }
 
 TopkRefine Engine::refinement(const tc::Planes& ht) const {
@@ -557,7 +563,7 @@ TopkRefine Engine::refinement(const tc::Planes& ht) const {
 }
 
 // Log-softmax statistics + per-beam top-(k+1), then beam selection (both paths).
-int Engine::step_tail(int t, int rows) {
+int Engine::step_tail(int t, int rows, bool ahead) {
   DevState& s = states_[0];
   const int n_act = rows / k;
   {
@@ -573,7 +579,8 @@ int Engine::step_tail(int t, int rows) {
       if (refine_) rf = refinement(tc_states_[0].panel_ht);
       if (refine_) trace_dev_.rf = rf;
       sel.tr = trace_dev_;
-      CK(softmax_topk(s.logits, s.logits16, rows, o, 1, refine_ ? &rf : nullptr, sel));
+      got_late_ = ahead && topk_late(blocks_, rows, n_sm_);
+      CK(softmax_topk(s.logits, s.logits16, rows, o, 1, refine_ ? &rf : nullptr, sel, got_late_));
     } else {
       // EnsembleFactory::EnsemblesModels (src/decoder.h:1910-1931): mean of the members'
       // probabilities, renormalised -- written as log(mean p) so that the log-softmax of the
@@ -694,12 +701,19 @@ int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, co
   // the encoder's final states sit in buffer (Smax & 1)
   enc_final_buf_ = Smax & 1;
   const auto host_t0 = std::chrono::steady_clock::now();
-  for (int t = 0; t <= Tm; ++t) {
-    int n_act = 0;
-    while (n_act < n && m_steps[n_act] >= t) ++n_act;
-    if (n_act == 0) break;
-    if ((rc = each_member(n_act * k, [&](int mi) { return use_tc_ ? run_decoder_step_tc(mi, t, n_act * k) : run_decoder_step(mi, t, n_act * k); }))) return rc;
-    if ((rc = step_tail(t, n_act * k))) return rc;
+  rec_ready_ = false;
+  int n_act = n;
+  for (int t = 0; t <= Tm && n_act > 0; ++t) {
+    int n_next = n_act;       // sentences of the next step
+    while (n_next > 0 && m_steps[n_next - 1] < t + 1) --n_next;
+    const int rows = n_act * k, rows_next = ahead_ok(n_next * k) ? n_next * k : 0;
+    if ((rc = each_member(rows, [&](int mi) { return use_tc_ ? run_decoder_step_tc(mi, t, rows, nullptr, rows_next) : run_decoder_step(mi, t, rows); }))) return rc;
+    if ((rc = step_tail(t, rows, rows_next > 0))) return rc;
+    if (rows_next > 0) {
+      if ((rc = recurrent_ahead(Ahead::kEnds, 0, t, rows_next))) return rc;
+      rec_ready_ = true;
+    }
+    n_act = n_next;
   }
   {
     FinalizeArgs a{};

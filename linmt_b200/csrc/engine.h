@@ -67,6 +67,7 @@ struct DevState {
   float* hs = nullptr;                               // [B][max_src][Hp]
   tc::Planes hs16{};                                 // the same in bf16 (one plane: instead of hs)
   float* hs_wc1 = nullptr;                           // [B][max_src][Hp]  W_c1 . hs (tensor path with the attention fold)
+  float* rec = nullptr;                              // [L + 1][rec_rows_][4Hp]  recurrent products of the step before, by its rows (Engine::recurrent_ahead), in the order of rec_slot
   float* enc_x = nullptr;                            // [B][Hp]
   float* enc_pre = nullptr;                          // [rows][4Hp]  W_x . input of every position (encoder layer by layer)
   std::vector<float*> enc_h[2], enc_c[2];            // [L] x [B][Hp], double buffered
@@ -135,13 +136,22 @@ class Engine {
   int each_member(int rows, const std::function<int(int)>& work);
   // a step of scoring: the tokens read, and where every member's htilde goes
   struct ScoreStep { const int32_t* tok; const tc::Planes* ht; };
-  int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr);
+  int run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc = nullptr, int rows_next = 0);
+  bool ahead_ok(int rows) const;
+  enum class Ahead { kBetween, kEnds };      // which of the recurrent products: the layers' between first and last, those two's
+  // where they are in DevState::rec: the first layer's states, the last one's, the first layer's feed-input, the layers between
+  static constexpr int kRowsAheadSelf = 32;      // rows that continue themselves have no gather to save
+  static constexpr int kRecFeed = 2;
+  int rec_slot(int l) const { return l == 0 ? 0 : l == L - 1 ? 1 : l + 2; }
+  int recurrent_ahead(Ahead which, int mi, int t, int rows);
+  // rows that continue themselves: one beam slot (scoring aside)
+  bool self_rows() const { return k == 1 && !trace_dev_.force_tok; }
   int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum);
-  cudaError_t softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel);
+  cudaError_t softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel, bool late = false);
   int score_core_tc(int n, int Smax, const std::vector<int>& n_act, const int32_t* d_tok, const int32_t* d_gold, float* d_logp);
   int reserve_score(size_t rows);
   TopkRefine refinement(const tc::Planes& ht) const;    // of one-product logits of these attentional states
-  int step_tail(int t, int rows);
+  int step_tail(int t, int rows, bool ahead);
   bool step_streams(bool scoring, int rows) const;
   bool pairs_available();   // clusters of two GEMM CTAs can be scheduled on the current device (engine_tc.cu)
   int launch_attention(int mi, int t, int rows, int kb, const float* u_alt, float* ctx, const tc::Planes& ctx_planes, int nt,
@@ -172,6 +182,10 @@ class Engine {
   int l2_bytes_ = 0;
   bool rows_ = true;       // weight-streaming kernel for few rows (LINMT_TC_ROWS=0: test knob)
   bool persist_ = true;    // persistent kernel for the many-wave vocabulary GEMM (LINMT_TC_PERSIST=0: test knob)
+  bool beside_ = false;      // the products issued leave room for the next one's CTAs (GemmLimits::beside)
+  bool want_late_ = false, got_late_ = false;   // the next product is asked to let its successor start only behind its wait; the last one asked does
+  bool rec_ready_ = false;   // the last step's recurrent products are made (recurrent_ahead)
+  int rec_rows_ = 0;         // rows they have room for
   bool pdl_gemm_ = false;  // true while the decoder step issues its GEMMs (the encoder's wavefront does not take part)
   int fmt_ = 0;       // plane format of every operand: 0 = bf16 planes, 1 = f16 pair
   int nt_vocab_ = 0;  // planes used by the vocabulary GEMM (0 = nt_)

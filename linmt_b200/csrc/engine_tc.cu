@@ -104,12 +104,15 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
   Epi e = e_in;
   if (nt <= 0 || nt > nt_) nt = nt_;
   tc::GemmLimits lim;
+  lim.beside = beside_;
   lim.n_sm = n_sm_; lim.parts = plan_parts_ ? plan_parts_ : ws_parts_; lim.rows = rows_; lim.pair = pair_; lim.persist = persist_;
   // a layer's slice of the split-K workspace: whole 256-byte units, so that every slice starts aligned for the
   // 16-byte partial-tile stores whatever the number of layers sharing it
   lim.ws_floats = (kSplitKWsFloats / ws_parts_) & ~(size_t)63;
   lim.max_tiles = kSplitKMaxTiles / ws_parts_;
   const tc::GemmPlan plan = tc::plan_gemm<Epi>(M, N, K, nt, fmt_, drain, x_row0, lim);
+  got_late_ = want_late_ && plan.kernel == tc::GemmKernel::kRows;
+  want_late_ = false;
   const CUtensorMap* am = maps(A, a_col0, a_rows_cap, K, plan.a_box, plan.bk);
   const CUtensorMap* bm = maps(W, 0, N, K, plan.b_box, plan.bk);
   if (!am || !bm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
@@ -126,7 +129,7 @@ int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::P
     }
   }
   CK(tc::launch_planned(plan, tm, M, N, K, nt, fmt_, pdl_ && pdl_gemm_, e, d_tc_err_, stream, n_sm_, d_splitk_ws_ + (size_t)ws_part_ * lim.ws_floats,
-                        d_splitk_counters_ + ws_part_ * lim.max_tiles, x_row0));
+                        d_splitk_counters_ + ws_part_ * lim.max_tiles, x_row0, got_late_));
   LAUNCHED();
   if (plan.on_pairs()) ++stats.pair_launches;
   return LINMT_OK;
@@ -163,6 +166,9 @@ int Engine::build_xw_tables() {
   return LINMT_OK;
 }
 
+// Up to here the encoder's products of a position are shaped like a step's, so that the next one's weights are under way (4 x 1000, 32
+// positions: one sentence 4.77 -> 4.73 ms a call, eight 14.34 -> 14.16; 64: 0.2 to 2 % slower).
+static constexpr int kBesideSentences = 48;
 static constexpr int kEncRing = 4;
 int Engine::encoder_streams() {
   if (!enc_streams_.empty()) return LINMT_OK;
@@ -186,7 +192,7 @@ int Engine::encoder_streams() {
 // the last reader of the double-buffered input slot it overwrites.
 // Which of the three forms: encoder_form (encoder_form.h).
 int Engine::run_encoder_tc(int n, int Smax) {
-  stream_weights_ = false;
+  stream_weights_ = false; beside_ = n <= kBesideSentences;
   if (enc_rows_)
     switch (encoder_form(EncoderModel{L, Hp, n_models, nt_ > 1}, n, Smax)) {
       case EncoderForm::kLayers: return run_encoder_layers_tc(n, Smax);
@@ -394,7 +400,7 @@ int Engine::encode_member_layers(int mi, int n, int Smax, int per) {
 }
 
 // One decoder forward, tensor-core path (see Engine::run_decoder_step).
-int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
+int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc, int rows_next) {
   DevModel& m = models_[mi];
   DevState& s = states_[mi];
   TcState& ts = tc_states_[mi];
@@ -408,11 +414,16 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   // Rows that continue themselves (one beam slot, scoring) need no copy of their states between two steps: there are two sets
   // of panels, and a step writes its states into the other set's h_prev and htilde_prev columns as well, while its own are
   // being read.  A launch less in a chain of eight to nine.
-  const bool self = sc || (k == 1 && !trace_dev_.force_tok);
+  const bool self = sc || self_rows();
   const int now = self ? t & 1 : 0, next = now ^ 1;
   const int32_t* parent = self ? nullptr : d_parent_;
+  // The recurrent half of every layer's product was made behind the last step (recurrent_ahead); `next`'s first panel takes the
+  // operand of the next one's.
+  const bool have_rec = rec_ready_ && !sc, want_rec = rows_next > 0 && !sc;
+  rec_ready_ = false;
+  beside_ = have_rec;
   tc::Planes ht_next = no_planes();      // htilde_prev of the next step
-  if (self && desc.feed_input) {
+  if ((self || want_rec) && desc.feed_input) {
     ht_next = ts.panel1[next];
     for (int p = 0; p < nt_; ++p) ht_next.p[p] += 2 * Hp;
   }
@@ -422,7 +433,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
   auto hprev_of = [&](int set, int l) -> const tc::Planes& { return l == 0 ? ts.panel1[set] : ts.panel[set][l]; };
   auto hprev_planes = [&](int l) -> const tc::Planes& { return hprev_of(now, l); };
   // 1. gather states through the parents into the h_prev slots, look up embeddings
-  {
+  if (!have_rec) {
     GatherJobs jobs{};
     int nj = 0;
     auto add = [&](const void* src, long long sstride, void* dst, long long dstride, int bytes, int kind) {
@@ -468,14 +479,22 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
       e.c_parent = parent; e.c_k = kb;
     }
     e.h_out1 = hcur_planes(l); e.h1_col0 = hcur_col0(l);
-    e.h_out2 = self ? hprev_of(next, l) : no_planes(); e.h2_col0 = Hp;
+    e.h_out2 = self || (want_rec && l == 0) ? hprev_of(next, l) : no_planes(); e.h2_col0 = Hp;
     e.h_prev = no_planes(); e.hp_col0 = 0;
     e.h_f32 = (l == L - 1 && opt.attention_mode == LINMT_ATT_GLOBAL_DOT) ? s.h_cur[l] : nullptr;
     e.hf_row_stride = Hp;
     e.row_len = nullptr; e.pos = 0; e.nt = nt_;
     int K = (l == 0 && feed) ? 3 * Hp : 2 * Hp;
     int rc;
-    if (l == 0 && m.dec_xw) {
+    if (have_rec && l == 0) {
+      e.xw = m.dec_xw; e.x_tok = tok; e.x_ld = 4 * Hp; e.x_vocab = V; e.x_unk = kUnk;
+      CK(tc::launch_k(pdl_, lstm_cell_kernel, dim3(rows, (Hp + 127) / 128), dim3(128), 0, stream, e, (const float*)s.rec, (const float*)(desc.feed_input ? s.rec + (size_t)kRecFeed * rec_rows_ * 4 * Hp : nullptr), Hp));
+      LAUNCHED();
+      rc = LINMT_OK;
+    } else if (have_rec) {
+      e.xw = s.rec + (size_t)rec_slot(l) * rec_rows_ * 4 * Hp; e.x_ld = 4 * Hp; e.x_parent = true;
+      rc = tc_gemm(hprev_planes(l), 0, R, m.p_dec_w[l], rows, 4 * Hp, Hp, e);
+    } else if (l == 0 && m.dec_xw) {
       // K columns (h_prev | htilde_prev) only: the x columns of panel and weights are skipped, their term comes from the table
       tc::Planes wrest = m.p_dec_w[0];
       for (int p = 0; p < 3; ++p) if (wrest.p[p]) wrest.p[p] += Hp;
@@ -486,10 +505,12 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
       rc = tc_gemm(hprev_planes(l), 0, R, m.p_dec_w[l], rows, 4 * Hp, K, e);
     }
     if (rc) return rc;
-    if (kernel_timing) rec_flops_ += 2.0 * rows * 4.0 * H * (double)((K / Hp) * H);
+    if (kernel_timing) rec_flops_ += 2.0 * rows * 4.0 * H * (double)((have_rec ? (l > 0) : K / Hp) * H);
   }
   // 3. attention projections: tanh(W_p h) | W_a^T h
   if (int rc = kt(KC_PROJ)) return rc;
+  got_late_ = false;
+  want_late_ = want_rec && L > 2;
   const float* u_alt = (opt.attention_mode == LINMT_ATT_GLOBAL_DOT) ? s.h_cur[L - 1] : nullptr;
   if (att_merge_) {
     // ... | W_c2 h: the half of the attention output's pre-activation that needs h_top only (global dot
@@ -505,6 +526,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
     int rc = tc_gemm(ts.panel_top, Hp, R, m.p_att_proj_w, rows, 2 * Hp, Hp, e);
     if (rc) return rc;
   }
+  want_late_ = false;
   // 4. scores, softmax x Gaussian, context (written into the attention-output panel)
   {
     const bool rec = d_rec_align_ && !sc;
@@ -513,6 +535,8 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
     int32_t* rv = rec ? d_rec_vit_ + (size_t)t * R : nullptr;
     if (int rc = kt(KC_ATTENTION)) return rc;
     if (int rc = launch_attention(mi, t, rows, kb, u_alt, nullptr, att_fold_ ? ht : ts.panel_top, nt_, ra, rl, rv, att_fold_, att_fold_ ? ht_next : no_planes())) return rc;
+    if (want_rec)
+      if (int rc = recurrent_ahead(Ahead::kBetween, mi, t, rows_next)) return rc;
   }
   // 5. htilde = tanh(W_c1 ctx + W_c2 h + b) (with the fold the attention kernel has written it already)
   if (!att_fold_) {
@@ -529,10 +553,76 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc) {
     }
     if (rc) return rc;
   }
+  beside_ = false;
   // 6. logits
   if (sc) return LINMT_OK;
   if (int rc = kt(KC_VOCAB)) return rc;
   return vocab_gemm(mi, ts.panel_ht, R, rows, s.logits, s.logits16, d_pmax_ + (size_t)mi * R * pmax_ld_, d_psum_ + (size_t)mi * R * pmax_ld_);
+}
+
+// The recurrent halves of the next step's LSTM products, W_h . h of every layer (and W_feed . htilde of the first), of the rows
+// as they are: which row continues which is not needed for them, only for their sum with the rest, whose epilogue reads the
+// parent's row.  With few rows a step is a chain of launches that wait for each other, and the weights' stream stands still
+// while the attention, the softmax and the selection run on a few SMs; these products run beside them, those of the layers
+// between beside the attention, the rest beside the softmax.  What is left of the chain is half a product a layer, none of the
+// first (lstm_cell_kernel adds up its terms), and no state is gathered.  48 steps, ms a call without / with: 4 x 1000 / 30k 1 row
+// 3.92 / 3.81, 12 rows 4.74 / 4.02, 24 4.88 / 4.34, 60 5.57 / 5.47, in bf16 5 rows 3.41 / 3.22; 2 x 1000 12 rows 3.55 / 3.08, 48 3.69 / 3.46;
+// 3 x 250 / 5k 12 rows 2.50 / 2.36; beyond 48 rows their CTAs take longer than what they run beside (kRowsAhead; 32, kRowsAheadSelf, where there is no gather to save).
+//
+// They start without a wait for the kernel before them in the stream (RowsShape::ahead).  Before the attention that is where the
+// projections have let the attention start only behind their own wait, and it these products: the layers' states are complete.
+// Before the softmax, where that has let them start only behind its wait: all of the step is.  (The LATE instances; got_late_ says
+// whether the launch was one of them.)  At their end they do wait, for those who wait for them.
+bool Engine::ahead_ok(int rows) const {
+  tc::RowsShape sh;
+  return rows > 0 && rows <= rec_rows_ && tc::make_shape_ahead(rows, 4 * Hp, Hp, nt_, fmt_, n_sm_, 1, &sh);   // (more products: fewer slices each, see there)
+}
+
+int Engine::recurrent_ahead(Ahead which, int mi, int t, int rows) {
+  DevModel& m = models_[mi];
+  DevState& s = states_[mi];
+  TcState& ts = tc_states_[mi];
+  const int now = self_rows() ? t & 1 : 0, next = now ^ 1;     // the sets of panels, see run_decoder_step_tc
+  constexpr int kSegs = 3;      // (at most five layers)
+  struct Part { tc::Planes a; int a_col0, layer, w_col0; } part[kSegs];
+  int segs = 0, slot = 0;
+  if (which == Ahead::kBetween) {
+    slot = rec_slot(1);
+    for (int l = 1; l + 1 < L; ++l) part[segs++] = Part{ts.panel[now][l + 1], 0, l, Hp};
+  } else {
+    part[segs++] = Part{ts.panel1[next], Hp, 0, Hp};
+    part[segs++] = Part{ts.panel_top, Hp, L - 1, Hp};
+    if (desc.feed_input) part[segs++] = Part{ts.panel1[next], 2 * Hp, 0, 2 * Hp};
+  }
+  if (segs == 0) return LINMT_OK;
+  tc::RowsShape sh;
+  if (!tc::make_shape_ahead(rows, 4 * Hp, Hp, nt_, fmt_, n_sm_, segs, &sh)) return fail(LINMT_EINVAL, "internal: no shape for the recurrent products");
+  sh.pdl = pdl_ ? 1 : 0;
+  sh.ahead = pdl_ && got_late_ ? 1 : 0;
+  tc::TmapSets<kSegs> tms{};
+  for (int i = 0; i < segs; ++i) {
+    tc::Planes w = m.p_dec_w[part[i].layer];
+    for (int p = 0; p < nt_; ++p) w.p[p] += part[i].w_col0;
+    const CUtensorMap* am = maps(part[i].a, part[i].a_col0, R, Hp, sh.rp, 64);
+    const CUtensorMap* bm = maps(w, 0, 4 * Hp, Hp, tc::BM, 64);
+    if (!am || !bm) return fail(LINMT_ECUDA, "cuTensorMapEncodeTiled failed");
+    std::memcpy(tms.s[i].a, am, sizeof(tms.s[i].a));
+    std::memcpy(tms.s[i].b, bm, sizeof(tms.s[i].b));
+    tms.s[i].stream_b = stream_weights_;
+  }
+  const size_t stride = (size_t)rec_rows_ * 4 * Hp;
+  const tc::TcEpiParts e{s.rec + slot * stride, (long long)stride, 4 * Hp};
+  auto launch = [&](auto nt, auto fmt) {
+    return tc::launch_gemm_tc_rows_of<decltype(nt)::value, decltype(fmt)::value, tc::TcEpiParts, kSegs, false>(tms, segs, rows, 4 * Hp, Hp, sh, e, d_tc_err_, stream, 0);
+  };
+  constexpr std::integral_constant<int, 0> zero{};
+  constexpr std::integral_constant<int, 1> one{};
+  constexpr std::integral_constant<int, 2> two{};
+  if (int rc = kt(KC_LSTM)) return rc;
+  if (kernel_timing) rec_flops_ += 2.0 * rows * 4.0 * H * (double)(segs * H);
+  CK(nt_ == 2 ? launch(two, one) : launch(one, zero));
+  LAUNCHED();
+  return LINMT_OK;
 }
 
 // Logits of `rows` attentional states.

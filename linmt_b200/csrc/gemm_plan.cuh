@@ -16,6 +16,7 @@ struct GemmLimits {
   int parts = 1;          // products that run side by side, each shaped for its share of the SMs (encoder wavefront)
   size_t ws_floats = 0;   // split-K workspace and its tile counters, of this product alone
   int max_tiles = 0;
+  bool beside = false;    // few rows: the next product's CTAs are to find room beside this one's
   bool rows = true, pair = true, persist = true;    // kernel forms that may be used (tests switch them off)
 };
 
@@ -41,7 +42,7 @@ inline GemmPlan plan_gemm(int M, int N, int K, int nt, int fmt, int drain, int a
   // tiles and one k slice is finished by too few warps for more than 48 rows of the f16 pair (one plane, vocabulary with
   // block statistics in the decode: 12.7 us at 12 rows, 18.9 at 64 against 19.6 in the one-tile kernel).
   if (lim.rows && lim.parts == 1 && M <= kRowsMax && (nt == 1 || M <= 48 || N <= 128 * lim.n_sm) &&
-      make_shape_rows(M, N, K, nt, fmt, lim.n_sm, drain >= K / 32, &p.rs)) {
+      make_shape_rows(M, N, K, nt, fmt, lim.n_sm, drain >= K / 32, lim.beside, &p.rs)) {
     p.kernel = GemmKernel::kRows;
     p.a_box = p.rs.rp; p.b_box = BM;
     if (Epi::kHasPmax) { p.stat_tile = BM; p.stat_part = 32; }
@@ -114,19 +115,20 @@ inline GemmPlan plan_gemm(int M, int N, int K, int nt, int fmt, int drain, int a
   return p;
 }
 
-// The tensor maps of `tm` have the plan's boxes; ws and counters are those the limits were given for.
+// The tensor maps of `tm` have the plan's boxes; ws and counters are those the limits were given for.  late: the next kernel may
+// start only once this one is past its wait (the few-rows kernel's offer, with fp32 results).
 template <class Epi>
 inline cudaError_t launch_planned(const GemmPlan& p, const TmapSet& tm, int M, int N, int K, int nt, int fmt, bool pdl, const Epi& e, int* err_flag,
-                                  cudaStream_t st, int n_sm, float* ws, int* counters, int a_row0 = 0) {
+                                  cudaStream_t st, int n_sm, float* ws, int* counters, int a_row0 = 0, bool late = false) {
   Shape sh = p.sh;
   sh.pdl = pdl ? 1 : 0;
   switch (p.kernel) {
     case GemmKernel::kRows: {
       RowsShape rs = p.rs;
       rs.pdl = pdl ? 1 : 0;
-      if (nt == 2) return launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, err_flag, st, a_row0);
-      if (fmt == 1) return launch_gemm_tc_rows<1, 1, Epi>(tm, M, N, K, rs, e, err_flag, st, a_row0);
-      return launch_gemm_tc_rows<1, 0, Epi>(tm, M, N, K, rs, e, err_flag, st, a_row0);
+      if (nt == 2) return launch_gemm_tc_rows<2, 1, Epi>(tm, M, N, K, rs, e, err_flag, st, a_row0, late);
+      if (fmt == 1) return launch_gemm_tc_rows<1, 1, Epi>(tm, M, N, K, rs, e, err_flag, st, a_row0, late);
+      return launch_gemm_tc_rows<1, 0, Epi>(tm, M, N, K, rs, e, err_flag, st, a_row0, late);
     }
     case GemmKernel::kPersistPair:
       if constexpr (Epi::kHasBlock) {

@@ -378,8 +378,9 @@ struct TcEpiLstm {
   // to the accumulator of row r with tok = x_tok[r] (out-of-range ids count as x_unk) -- the embedding part of
   // the first decoder layer's product then costs a row lookup instead of a third of the GEMM.
   const float* xw = nullptr; const int32_t* x_tok = nullptr; int x_ld = 0; int x_vocab = 0; int x_unk = 0;
+  bool x_parent = false;     // (without x_tok) the row of `xw` is the parent's, as c_prev's is
   __device__ __forceinline__ int x_row(int row) const {
-    if (!x_tok) return row;    // one row of the table per row of the product (encoder: the input's share of every position)
+    if (!x_tok) return x_parent ? c_src_row(row) : row;    // one row of the table per row of the product (encoder: the input's share of every position)
     const int t = x_tok[row];
     return (t < 0 || t >= x_vocab) ? x_unk : t;
   }
@@ -435,6 +436,7 @@ struct TcEpiLstm {
   // this lane's row.  sbuf = this warp's staging area.  c_prev comes in and c goes out through
   // the staging area with consecutive lanes on consecutive addresses; h goes out as planes the
   // same way.  Rows past their length (encoder) keep c and copy h_prev.
+  static constexpr bool kLate = false;      // (an instance of the few-rows kernel that lets its successor start late)
   static constexpr bool kHasBlock = true;
   static constexpr bool kHasPmax = false;
   static constexpr bool kHasPrefetch = true;
@@ -639,6 +641,7 @@ struct TcEpiBiasTanh {
   int nt;
   const float* add = nullptr; int ld_add = 0;
   Planes out2{};      // a second place for the same (p[0] == nullptr: none)
+  static constexpr bool kLate = false;
   static constexpr bool kHasBlock = false;
   static constexpr bool kHasPmax = false;
   static constexpr bool kHasPrefetch = false;
@@ -670,6 +673,17 @@ struct TcEpiBiasTanh {
     const float4 a = make_float4(tanh_fast((v.x + p.a.x) + p.b.x), tanh_fast((v.y + p.a.y) + p.b.y), tanh_fast((v.z + p.a.z) + p.b.z), tanh_fast((v.w + p.a.w) + p.b.w));
     split_store4(out, nt, (size_t)row * out.ld + col_off + col, a.x, a.y, a.z, a.w);
     if (out2.p[0]) split_store4(out2, nt, (size_t)row * out2.ld + col, a.x, a.y, a.z, a.w);
+  }
+};
+
+// fp32 out, one result per segment of a launch (row form only).
+struct TcEpiParts {
+  float* out; long long stride; int ld;
+  __device__ __forceinline__ TcEpiParts of(int seg) const { return TcEpiParts{out + seg * stride, 0, ld}; }
+  struct Pre {};
+  __device__ __forceinline__ Pre preload(int, int) const { return Pre{}; }
+  __device__ __forceinline__ void finish_row(bool valid, int row, int col, int /*lane*/, const float4& v, const Pre&) const {
+    if (valid) *reinterpret_cast<float4*>(out + (size_t)row * ld + col) = v;
   }
 };
 
@@ -717,6 +731,7 @@ struct TcEpiF32 {
   }
   // Block form (see TcEpiLstm::block): bias / tanh in registers, the block of up to 64 columns
   // staged per row, then stored with a row's 16 float4 on consecutive lanes.
+  static constexpr bool kLate = true;
   static constexpr bool kHasBlock = true;
   static constexpr bool kHasPmax = true;
   static constexpr bool kHasPrefetch = false;

@@ -18,6 +18,8 @@
 // (the tensor core truncates on every accumulate): the K range of a CTA is dealt to `leads` accumulators, each chain
 // at most three k-blocks, and the cross terms have columns of their own.  All of them are added in fp32 registers.
 #pragma once
+#include <type_traits>
+
 #include "gemm_tc.cuh"
 #include "gemm_tc_pair.cuh"
 
@@ -43,6 +45,7 @@ struct RowsShape {
   int leads, acc_stride, stacked, tmem_cols;
   int alias;           // the partial sums' buffer lies in the rings (and waits until the whole cluster is done with them)
   int pdl;
+  int ahead;           // (several products in a launch) reads nothing of the kernel before it, and waits for that only at its end
 };
 
 // Everything that follows from the split.
@@ -71,7 +74,9 @@ inline bool rows_set_splits(RowsShape* s, int K, int nt) {
 }
 
 // one_chain: the leading product may be one long chain per accumulator (logits, see gemm_tc_persist_kernel)
-inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, bool one_chain, RowsShape* out) {
+// beside: a CTA per SM at most, so that the next product's are all in flight beside them, their rings full, when this one's
+// results arrive (4096 x 1024 and 3072 x 1024 in a chain, 12 rows: 80 against 84 us a step with 256 and 192 CTAs, which take turns)
+inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, bool one_chain, bool beside, RowsShape* out) {
   if (rows < 1 || rows > rows_max(nt) || K % 64 || K < 64 || N % 16) return false;
   if (!(nt == 1 || (nt == 2 && fmt == 1))) return false;
   RowsShape s{};
@@ -84,7 +89,7 @@ inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, b
   // accumulators of half an SM's TMEM serve.  One plane and few rows: a CTA's slice fits its ring whole at half as many
   // slices (4096 x 2048 at 12 rows: 6.2 us at 4, 6.6 at 8; at 64 rows 9.5 and 8.0).
   for (int whole = 0; whole < 2; ++whole) {
-    s.splits = (whole || (nt == 1 && s.rp <= 32) ? n_sm : 2 * n_sm) / tiles;
+    s.splits = (whole || beside || (nt == 1 && s.rp <= 32) ? n_sm : 2 * n_sm) / tiles;
     s.splits = s.splits < 1 ? 1 : (s.splits > (whole ? 4 : 8) ? (whole ? 4 : 8) : s.splits);
     if (s.splits > nkb) s.splits = nkb;
     s.tmem_cols = whole ? 512 : 256;
@@ -104,6 +109,37 @@ inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, b
   return false;
 }
 
+// The shape of `segs` products of few rows that run beside other kernels (Engine::recurrent_ahead): as many K slices as fit
+// beside a few whole-SM blocks at once, each with a long stream of weights, where make_shape_rows would have the whole product in
+// flight (three products of 4096 x 1024 as launches of 256 CTAs each behind one another: 24 us more a step than these beside the
+// attention and the softmax, 12 rows).  Half an SM each, so that the next kernel's CTAs find room.
+constexpr int kRowsAhead = 60;
+inline bool make_shape_ahead(int rows, int N, int K, int nt, int fmt, int n_sm, int segs, RowsShape* out) {
+  if (rows < 1 || rows > kRowsAhead || K % 64 || K < 64 || N % 16) return false;
+  if (!(nt == 1 || (nt == 2 && fmt == 1))) return false;
+  RowsShape s{};
+  s.rp = (rows + 15) & ~15; s.units = (rows + 3) & ~3;
+  s.tmem_cols = 256;
+  const int tiles = (N + BM - 1) / BM * segs, nkb = K / 64, places = n_sm * 4 / 3;
+  s.splits = 8;
+  while (s.splits > 1 && tiles * s.splits > places) s.splits >>= 1;
+  for (; s.splits <= 8; s.splits *= 2) {
+    if (s.splits > nkb) s.splits = nkb;
+    for (s.stacked = nt == 2 ? 1 : 0; s.stacked >= 0; --s.stacked) {     // (not stacked: more and shorter chains)
+      s.acc_stride = s.stacked ? 2 * s.rp : (s.rp + 31) & ~31;
+      s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
+      if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
+      const bool chains = nt == 1 || (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
+      if (chains && rows_set_splits(&s, K, nt)) {
+        *out = s;
+        return true;
+      }
+    }
+    if (s.splits == nkb) break;
+  }
+  return false;
+}
+
 // four floats into the shared memory of a CTA of the cluster, their bytes counted on a barrier there
 __device__ __forceinline__ void st_async4(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1,%2,%3,%4}, [%5];"
@@ -118,9 +154,18 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-template <int NT, int FMT, class Epi>
+// Several products of the same shape in one launch: blockIdx.y chooses the operands' maps, and Epi::of(blockIdx.y) the result.
+template <int SEGS>
+struct TmapSets { TmapSet s[SEGS]; };
+
+// LATE: the next kernel may start only once this one is past its wait.  (Template parameters: a kernel's word to the next one is its
+// first instruction, ahead of the first read of its parameters, which cost 1 to 3 % of a chain of small products.)
+template <int NT, int FMT, class Epi, int SEGS, bool LATE>
 __global__ void __launch_bounds__(kRowsThreads, 2)
-gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int x_row0, RowsShape sh, Epi epi, int* __restrict__ err_flag) {
+gemm_tc_rows_kernel(const __grid_constant__ TmapSets<SEGS> tms, int M, int N, int K, int x_row0, RowsShape sh, Epi epi_of, int* __restrict__ err_flag) {
+  auto chosen = [&]() -> std::conditional_t<(SEGS > 1), Epi, const Epi&> { if constexpr (SEGS > 1) return epi_of.of(blockIdx.y); else return epi_of; };
+  const Epi& epi = chosen();
+  const TmapSet& tm = tms.s[SEGS > 1 ? blockIdx.y : 0];
   constexpr int PC = product_code(NT, FMT);
   static_assert(NT == 1 || PC == kF16PairCode, "one plane or the f16 pair");
   constexpr int W_BYTES = BM * 128;            // one plane of a weight k-block (64 deep)
@@ -136,7 +181,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(rows_smem + (recv_bar + 8u - base));
   volatile int* abort_flag = reinterpret_cast<volatile int*>(rows_smem + (recv_bar + 12u - base));
 
-  pdl_launch_dependents();
+  if (!LATE) pdl_launch_dependents();
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BM;
   const int splits = sh.splits, rank = blockIdx.z;
@@ -189,7 +234,8 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
   if (splits > 1) cluster_arrive();     // the barriers above exist (waited for before the first remote write)
   const uint32_t tmem = *tmem_slot;
 
-  pdl_wait();    // from here on the previous kernel's results are visible
+  if (SEGS == 1 || !sh.ahead) pdl_wait();    // from here on the previous kernel's results are visible
+  if (LATE) pdl_launch_dependents();
   if (warp == 0 && one)
     for (int kb = 0; kb < prex; ++kb) load_x(kb, kb);
   // what the epilogue of this warp's first unit reads is requested now and used after the accumulators are complete
@@ -329,15 +375,16 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
     }
   }
   if (threadIdx.x == 0 && *abort_flag) atomicExch(err_flag, 1);
+  if (SEGS > 1 && sh.ahead) pdl_wait();     // (who waits for this kernel waits for the one before it as well)
 }
 
 // x_row0: first row of the product in the activations' tensor map
-template <int NT, int FMT, class Epi>
-inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0 = 0) {
+template <int NT, int FMT, class Epi, int SEGS, bool LATE>
+inline cudaError_t launch_gemm_tc_rows_of(const TmapSets<SEGS>& tms, int segs, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0) {
   static bool optin_done[kMaxDevices] = {};
-  if (cudaError_t e = ensure_smem_optin(gemm_tc_rows_kernel<NT, FMT, Epi>, optin_done, kRowsSmemWhole); e != cudaSuccess) return e;
+  if (cudaError_t e = ensure_smem_optin(gemm_tc_rows_kernel<NT, FMT, Epi, SEGS, LATE>, optin_done, kRowsSmemWhole); e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((N + BM - 1) / BM, 1, sh.splits); cfg.blockDim = dim3(kRowsThreads);
+  cfg.gridDim = dim3((N + BM - 1) / BM, segs, sh.splits); cfg.blockDim = dim3(kRowsThreads);
   cfg.dynamicSmemBytes = (size_t)sh.smem_bytes; cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int na = 0;
@@ -353,7 +400,13 @@ inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, c
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, gemm_tc_rows_kernel<NT, FMT, Epi>, tm, M, N, K, x_row0, sh, epi, err_flag);
+  return cudaLaunchKernelEx(&cfg, gemm_tc_rows_kernel<NT, FMT, Epi, SEGS, LATE>, tms, M, N, K, x_row0, sh, epi, err_flag);
+}
+template <int NT, int FMT, class Epi>
+inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0 = 0, bool late = false) {
+  if constexpr (Epi::kLate)
+    if (late) return launch_gemm_tc_rows_of<NT, FMT, Epi, 1, true>(TmapSets<1>{{tm}}, 1, M, N, K, sh, epi, err_flag, st, x_row0);
+  return launch_gemm_tc_rows_of<NT, FMT, Epi, 1, false>(TmapSets<1>{{tm}}, 1, M, N, K, sh, epi, err_flag, st, x_row0);
 }
 
 }  // namespace tc

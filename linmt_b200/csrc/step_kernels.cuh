@@ -127,6 +127,24 @@ static __global__ void row_gather_kernel(GatherJobs jobs, const int32_t* __restr
   }
 }
 
+// First decoder layer of a step whose recurrent products are there already (Engine::recurrent_ahead): gates of row r = row
+// parent[r] of `pre` (its second part `feed` behind it, or null) plus the input term of its token, which the epilogue's preload looks
+// up.  A thread per hidden unit; grid = (rows, Hp / 128).
+static __global__ void __launch_bounds__(128) lstm_cell_kernel(tc::TcEpiLstm e, const float* __restrict__ pre, const float* __restrict__ feed, int Hp) {
+  tc::pdl_launch_dependents();
+  tc::pdl_wait();
+  const int row = blockIdx.x, col = (blockIdx.y * 128 + threadIdx.x) * 4;
+  if (col >= 4 * Hp) return;
+  const size_t at = (size_t)e.c_src_row(row) * 4 * Hp + col;
+  const tc::TcEpiLstm::Pre p = e.preload(row, col);
+  float4 v = *reinterpret_cast<const float4*>(pre + at);
+  if (feed) {
+    const float4 f = *reinterpret_cast<const float4*>(feed + at);
+    v.x += f.x; v.y += f.y; v.z += f.z; v.w += f.w;
+  }
+  e.finish_row(true, row, col, 0, v, p);
+}
+
 // Encoder input for the tensor-core path: embedding planes of the token at reversed position
 // `pos` into columns [0, Hp) of the layer-0 panel; zeros past the sentence.
 // grid = (B, nt), block = 128
@@ -1236,11 +1254,14 @@ struct LogitBlocks {
   int tile, part;     // columns of a GEMM tile and of one of its four blocks (the last one of a tile may be narrower)
 };
 inline size_t topk_blocks_smem(int n_blocks, int refine_K) { return sizeof(float) * (size_t)(2 * n_blocks + refine_K); }
-template <int THREADS>
+// LATE: the next kernel runs beside this one and reads what this one has waited for, without a wait of its own: it may start
+// only behind that wait.
+template <int THREADS, bool LATE>
 static __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 6 : 1) topk_blocks_kernel(const float* __restrict__ logits, const __half* __restrict__ logits16, int ld, int V, int kk,
                                                                            TopkOut out, int normalise, LogitBlocks bl, TopkRefine rf, const __grid_constant__ SelectArgs sel) {
-  tc::pdl_launch_dependents();
+  if (!LATE) tc::pdl_launch_dependents();
   tc::pdl_wait();
+  if (LATE) tc::pdl_launch_dependents();
   extern __shared__ __align__(16) float dyn[];
   float* s_m = dyn;                  // [n] block maxima
   float* s_q = dyn + bl.n;           // [n] block sums
@@ -1389,12 +1410,15 @@ inline LogitBlocks logit_blocks(float* max, float* sum, int ld, int N, int K, in
 // Values a row of block statistics has room for: four column blocks per tile, tiles at least 48 wide.
 inline int logit_blocks_ld(int N) { return 4 * ((N + 47) / 48) + 4; }
 
-// Softmax statistics and top-k (and the selection) of rows of logits, from their block statistics where they have them.
+// Softmax statistics and top-k (and the selection) of rows of logits, from their block statistics where they have them.  late: see
+// topk_blocks_kernel, where topk_late says that the launch can.
+inline bool topk_late(const LogitBlocks& bl, int rows, int n_sm) { return bl.sum && rows <= n_sm; }
 inline cudaError_t launch_topk(const float* logits, const __half* logits16, int ld, int V, int kk, int rows, int n_sm, const TopkOut& o, int normalise,
-                               const LogitBlocks& bl, const TopkRefine* rf, const SelectArgs& sel, cudaStream_t st, bool pdl) {
+                               const LogitBlocks& bl, const TopkRefine* rf, const SelectArgs& sel, cudaStream_t st, bool pdl, bool late = false) {
   if (!bl.sum) return launch_softmax_topk(logits, ld, V, kk, rows, o, normalise, st, pdl, bl.max, bl.ld, bl.n, rf, logits16, sel);
   const bool wide = rows <= n_sm;
-  return tc::launch_k(pdl, wide ? topk_blocks_kernel<1024> : topk_blocks_kernel<256>, dim3(rows), dim3(wide ? 1024 : 256), topk_blocks_smem(bl.n, rf ? rf->K : 0), st,
+  auto* kernel = !wide ? topk_blocks_kernel<256, false> : late ? topk_blocks_kernel<1024, true> : topk_blocks_kernel<1024, false>;
+  return tc::launch_k(pdl, kernel, dim3(rows), dim3(wide ? 1024 : 256), topk_blocks_smem(bl.n, rf ? rf->K : 0), st,
                       logits, logits16, ld, V, kk, o, normalise, bl, rf ? *rf : TopkRefine{}, sel);
 }
 

@@ -465,3 +465,61 @@ def test_members_side_by_side_in_one_plane(cuda_lib, members, n, beam, attention
     for key in ("cand_tok", "cand_logp", "final_logp", "tok", "len", "score"):
         assert side[0][key].tobytes() == turn[0][key].tobytes(), key
     assert side[1][1].tobytes() == turn[1][1].tobytes()
+
+
+@pytest.mark.parametrize("L,H,n,beam,attention,feed", [
+    (2, 256, 1, 1, "local_p_general", 1), (3, 250, 5, 1, "global_general", 1), (5, 300, 1, 12, "local_p_general", 1),
+    (2, 260, 4, 15, "global_dot", 1),                    # 60 rows, and 45 once a sentence has ended
+    (4, 256, 16, 4, "local_p_general", 0),               # 64 rows, then 60 and fewer
+    (3, 256, 33, 1, "local_p_general", 1)])              # 33 rows, then 32 and fewer
+def test_recurrent_products_ahead_of_their_step(oracle, cuda_lib, L, H, n, beam, attention, feed):
+    """Up to 60 rows (32 of one slot each) the recurrent products of a step are made behind the step before, by the rows that they continue:
+    forced, against the oracle, and against the steps that make them in place; free, the same bits in every call."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(L, H, 2000, 300, feed)
+    blob = synth.make_blob(d, 40, family="peaked")
+    sents = synth.make_sentences(n, 2, 12, d.Vs, 1.1, 3, lambda s: s + 3)
+    kw = dict(beam=beam, attention=attention, cp_beta=0.0, min_ratio=0.0)
+    o = oracle.decode(d, [blob], sents, trace=True, **kw)
+    cap = dict(max_batch=n, max_src_len=16, max_steps=20)
+    dec = decoder.Decoder(d, [blob], **kw, **cap)
+    e = dec.decode(sents, trace=True, force=o)
+    worst, bad, skipped, compared = compare_forced(e, o, sents.steps, src_len=sents.lengths())
+    assert worst <= RTOL_FP32 and bad == 0 and skipped <= 0.1 * (skipped + compared), (worst, bad, skipped, compared)
+    first = dec.decode(sents)
+    for _ in range(3):
+        again = dec.decode(sents)
+        assert first["tok"].tobytes() == again["tok"].tobytes() and first["score"].tobytes() == again["score"].tobytes()
+    before = dec.stats()["kernel_launches"]
+    dec.decode(sents)
+    launches = dec.stats()["kernel_launches"] - before
+    dec.close()
+    ref = _with_env({"LINMT_AHEAD": "0"}, lambda: decoder.Decoder(d, [blob], **kw, **cap))
+    r = ref.decode(sents)
+    before = ref.stats()["kernel_launches"]
+    ref.decode(sents)
+    assert (L == 2 and beam > 1) or ref.stats()["kernel_launches"] - before != launches      # (it ran the other way)
+    ref.close()
+    # scores: sums of up to 15 log-probabilities of the same tokens
+    for i in range(n):
+        if hyps(first, i) == hyps(r, i):
+            np.testing.assert_allclose(first["score"][i, 0], r["score"][i, 0], rtol=RTOL_FP32)
+
+
+@pytest.mark.parametrize("n,beam", [(1, 5), (4, 12), (24, 2)])
+def test_recurrent_products_ahead_in_one_plane(cuda_lib, n, beam):
+    """The same in bf16, forced to the beams of the steps that make them in place: within the bar of bf16 log-probabilities."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(3, 512, 2000, 300, 1)
+    blob = synth.make_blob(d, 40)
+    sents = synth.make_sentences(n, 2, 12, d.Vs, 1.1, 3, lambda s: s + 3)
+    kw = dict(beam=beam, precision="bf16", attention="global_general", cp_beta=0.0, max_batch=n, max_src_len=16, max_steps=20)
+    ref = _with_env({"LINMT_AHEAD": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    r = ref.decode(sents, trace=True)
+    dec = decoder.Decoder(d, [blob], **kw)
+    e = dec.decode(sents, trace=True, force=r)
+    ref.close(); dec.close()
+    for i in range(n):
+        T = int(sents.steps[i])
+        a, b = np.sort(e["cand_logp"][i, 1:T]), np.sort(r["cand_logp"][i, 1:T])
+        assert (np.abs(a - b) <= 2e-2).all(), float(np.abs(a - b).max())
