@@ -36,6 +36,13 @@ constexpr int kRowsMaxLeads = 4;
 constexpr int kRowsSmemHalf = 113 * 1024;
 constexpr int kRowsSmemMin = 78 * 1024;
 constexpr int kRowsSmemWhole = 224 * 1024;     // a CTA that has the SM to itself
+// A CTA that takes all of an SM's TMEM asks for so much shared memory that none of the others fits beside it, as the other
+// kernels with 512 columns do (their staging area alone): a CTA never waits for TMEM that a CTA of another stream holds, whose
+// cluster might in turn wait for one that this CTA's cluster keeps out elsewhere.
+constexpr int kRowsSmemWholeMin = 150 * 1024;
+constexpr int kSmemPerSm = 228 * 1024, kSmemReserved = 1024;       // of an SM; of every block
+static_assert(3 * (kRowsSmemMin + kSmemReserved) > kSmemPerSm && kRowsSmemWholeMin + kRowsSmemMin + 2 * kSmemReserved > kSmemPerSm &&
+              kEpiStagingBytes + kRowsSmemMin + 2 * kSmemReserved > kSmemPerSm, "two CTAs of half the TMEM on an SM, or one of all of it");
 constexpr int kRowsBarBytes = 384;
 
 struct RowsShape {
@@ -68,7 +75,7 @@ inline bool rows_set_splits(RowsShape* s, int K, int nt) {
   const int rings = s->wstages * w + s->xstages * x;
   if (s->alias && rings < s->recv_bytes) return false;
   s->smem_bytes = rings + (s->alias ? 0 : s->recv_bytes) + kRowsBarBytes;
-  const int least = s->tmem_cols == 512 ? kRowsSmemHalf + 3072 : kRowsSmemMin;
+  const int least = s->tmem_cols == 512 ? kRowsSmemWholeMin : kRowsSmemMin;
   if (s->smem_bytes < least) s->smem_bytes = least;
   return s->wstages >= 1 && s->xstages >= 1;
 }
