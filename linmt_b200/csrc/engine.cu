@@ -299,11 +299,31 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   if (fmt_ == 1 && (o.gemm_path == LINMT_GEMM_TENSOR_V16 || (v16x && nm == 1))) nt_vocab_ = 1;
   refine_ = fmt_ == 1 && v16x && nm == 1;
   { const char* pe = std::getenv("LINMT_LOGITS16"); logits16_ = refine_ && !(pe && std::atoi(pe) == 0); }
+  { const char* pe = std::getenv("LINMT_AHEAD"); ahead_ = !(pe && std::atoi(pe) == 0); }      // LINMT_AHEAD=0: test knob
+  { const char* pe = std::getenv("LINMT_LANES"); lanes_ = !(pe && std::atoi(pe) == 0); }
   if (linmt_blob_floats(&d) != blob_floats) return fail(LINMT_EINVAL, "weight blob size does not match the model dimensions");
   if (o.beam <= 0) return fail(LINMT_EINVAL, "--beam-size cannot be <= 0");
   if (o.penalty < 0) return fail(LINMT_EINVAL, "--penalty cannot be < 0");
   if (o.nbest < 1 || o.nbest > 32) return fail(LINMT_EINVAL, "nbest must be in 1..32");
   if (o.max_batch < 1 || o.max_src_len < 1 || o.max_steps < 1) return fail(LINMT_EINVAL, "bad capacity options");
+  return init_state(nullptr, blobs);
+}
+
+int Engine::init_lane(const Engine& of) {
+  desc = of.desc; opt = of.opt; n_models = of.n_models;
+  // (what the environment and the weights decided when the handle was made)
+  use_tc_ = of.use_tc_; xw_table_ = of.xw_table_; pmax_on_ = of.pmax_on_; att_merge_ = of.att_merge_; att_fold_ = of.att_fold_;
+  persist_ = of.persist_; rows_ = of.rows_; pair_ = of.pair_; pdl_ = of.pdl_; ahead_ = of.ahead_; fmt_ = of.fmt_; nt_ = of.nt_;
+  nt_vocab_ = of.nt_vocab_; refine_ = of.refine_; logits16_ = of.logits16_;
+  return init_state(&of, nullptr);
+}
+
+// What is left of a handle's creation once its options are settled: sizes, device buffers, and the weights, packed from `blobs` or
+// those of engine `of`.
+int Engine::init_state(const Engine* of, const float* const* blobs) {
+  const linmt_model_desc& d = desc;
+  const linmt_options& o = opt;
+  const int nm = n_models;
   L = d.layers; H = d.hidden; V = d.vocab_tgt;
   k = std::min<int>(o.beam, (int)std::sqrt((double)V));  // src/decoder.h:1549-1551
   if (k > kMaxBeam) return fail(LINMT_ELIMIT, "beam larger than 31 is not supported");
@@ -336,15 +356,13 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
     const int nb = encoder_panel_sentences(EncoderModel{L, Hp, nm, nt_ > 1}, B, opt.max_src_len);
     enc_rows_ = std::min(opt.max_src_len * nb, std::max(16384, nb));
   }
-  // (LINMT_AHEAD=0: test knob.  Narrower models gain nothing: 2 x 128, one row 1.04 -> 1.09 ms a call of 30 steps)
-  {
-    const char* pe = std::getenv("LINMT_AHEAD");
-    if (use_tc_ && rows_ && xw_table_ && nm == 1 && L > 1 && Hp >= 256 && (nt_ == 1 || fmt_ == 1) && !(pe && std::atoi(pe) == 0)) rec_rows_ = std::min(R, k > 1 ? tc::kRowsAhead : kRowsAheadSelf);
-  }
+  // (narrower models gain nothing: 2 x 128, one row 1.04 -> 1.09 ms a call of 30 steps)
+  if (ahead_ && use_tc_ && rows_ && xw_table_ && nm == 1 && L > 1 && Hp >= 256 && (nt_ == 1 || fmt_ == 1)) rec_rows_ = std::min(R, k > 1 ? tc::kRowsAhead : kRowsAheadSelf);
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);
   for (int i = 0; i < nm; ++i) {
-    int rc = pack_model(blobs[i], models_[i]);
-    if (rc) return rc;
+    int rc = LINMT_OK;
+    if (of) models_[i] = of->models_[i];
+    else if ((rc = pack_model(blobs[i], models_[i]))) return rc;
     // fp16 storage of the logits needs them inside fp16's range with room to spare: |z| <= |w_row| |htilde| + |b| and
     // every component of htilde is below 1 in magnitude
     if (logits16_ && !(models_[i].voc_wnorm_max * std::sqrt((float)H) + models_[i].voc_babs_max < 3.0e4f)) logits16_ = false;
@@ -370,7 +388,7 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   if (o.print_info) {
     DA(d_rec_align_, (size_t)Tcap * R * rec_win); DA(d_rec_lo_, (size_t)Tcap * R); DA(d_rec_vit_, (size_t)Tcap * R);
   }
-  if (use_tc_ && xw_table_) { const int rc_xw = build_xw_tables(); if (rc_xw) return rc_xw; }
+  if (use_tc_ && xw_table_ && !of) { const int rc_xw = build_xw_tables(); if (rc_xw) return rc_xw; }
   CK(cudaDeviceSynchronize());  // every weight upload has landed before the first decode
   return LINMT_OK;
 }
@@ -910,84 +928,76 @@ int Engine::decode_host(const int32_t* src_ids, const int32_t* src_off, int n, c
   return LINMT_OK;
 }
 
-// Log-probabilities of given targets (linmt_score_batch), in device batches of max_batch sentences, longest target first.
-int Engine::score_host(const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids, const int32_t* tgt_off, int n,
-                       float* out_logprob, float* out_token_logp, int max_tgt) {
+// Log-probabilities of given targets (linmt_score_batch): one device batch, sentences idx[0..cn), longest target first.
+int Engine::score_chunk(const ScoreJob& jb, const int* idx, int cn) {
+  const int32_t *src_ids = jb.src_ids, *src_off = jb.src_off, *tgt_ids = jb.tgt_ids, *tgt_off = jb.tgt_off;
+  float *out_logprob = jb.out_logprob, *out_token_logp = jb.out_token_logp;
+  const int max_tgt = jb.max_tgt;
   CK(cudaSetDevice(opt.device));
-  std::vector<int> order(n);
-  std::iota(order.begin(), order.end(), 0);
   auto tlen = [&](int i) { return tgt_off[i + 1] - tgt_off[i]; };
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return tlen(a) > tlen(b); });
-  float total_ms = 0.f;
-  for (int c0 = 0; c0 < n; c0 += B) {
-    const int cn = std::min(B, n - c0);
-    const int* idx = order.data() + c0;
-    const int steps = tlen(idx[0]) + 1;        // forwards: one per token and one for EOS
-    int Smax = 0;
-    size_t n_ids = 0;
-    for (int i = 0; i < cn; ++i) {
-      const int len = src_off[idx[i] + 1] - src_off[idx[i]];
-      if (len < 1) return fail(LINMT_EINVAL, "empty source sentence");
-      if (len > opt.max_src_len) return fail(LINMT_ELIMIT, "source sentence longer than max_src_len");
-      h_meta_[i] = (int32_t)n_ids; h_meta_[(B + 1) + i] = len; h_meta_[2 * (B + 1) + i] = steps - 1; h_meta_[3 * (B + 1) + i] = i;
-      n_ids += len;
-      Smax = std::max(Smax, len);
-    }
-    std::vector<int> n_act(steps, 0);
-    size_t rows = 0;
-    for (int t = 0; t < steps; ++t) {
-      while (n_act[t] < cn && tlen(idx[n_act[t]]) >= t) ++n_act[t];
-      rows += n_act[t];
-    }
-    // ids | tokens read [steps][cn] | tokens asked for [rows], up in one copy; log-probabilities [rows] back
-    const size_t n_up = n_ids + (size_t)steps * cn + rows;
-    if (n_up + rows > score_io_cap_) {
-      if (int rc = regrow(&score_io_, n_up + rows)) return rc;
-      score_io_cap_ = n_up + rows;
-    }
-    if (int rc = reserve_host((n_up + rows) * 4)) return rc;
-    int32_t *h_tok = h_stage_ + n_ids, *h_gold = h_tok + (size_t)steps * cn;
-    for (int i = 0; i < cn; ++i)
-      std::memcpy(h_stage_ + h_meta_[i], src_ids + src_off[idx[i]], sizeof(int32_t) * h_meta_[(B + 1) + i]);
-    size_t row = 0;
-    for (int t = 0; t < steps; ++t)
-      for (int i = 0; i < cn; ++i) {
-        const int32_t* tgt = tgt_ids + tgt_off[idx[i]];
-        h_tok[(size_t)t * cn + i] = t == 0 || i >= n_act[t] ? kStart : tgt[t - 1];
-        if (i < n_act[t]) h_gold[row++] = t < tlen(idx[i]) ? tgt[t] : kEos;
-      }
-    CK(cudaEventRecord(ev0_, stream));
-    CK(cudaMemcpyAsync(d_off_, h_meta_, sizeof(int32_t) * 4 * (B + 1), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(score_io_, h_stage_, n_up * 4, cudaMemcpyHostToDevice, stream));
-    cur_ids_ = score_io_;
-    trace_dev_ = TraceDev{};
-    kt_used_ = 0; rec_flops_ = 0.0;
-    float* d_logp = reinterpret_cast<float*>(score_io_ + n_up);
-    int rc = score_core_tc(cn, Smax, n_act, score_io_ + n_ids, score_io_ + n_ids + (size_t)steps * cn, d_logp);
-    if (rc) { cudaStreamSynchronize(stream); return rc; }
-    if ((rc = kt(KC_END))) return rc;
-    CK(cudaEventRecord(ev1_, stream));
-    const float* h_logp = reinterpret_cast<const float*>(h_stage_ + n_up);
-    CK(cudaMemcpyAsync(h_stage_ + n_up, d_logp, rows * 4, cudaMemcpyDeviceToHost, stream));
-    if ((rc = finish_timing())) return rc;
-    total_ms += stats.last_decode_ms;
-    row = 0;
-    for (int i = 0; i < cn; ++i) out_logprob[idx[i]] = 0.f;
-    for (int t = 0; t < steps; ++t)
-      for (int i = 0; i < n_act[t]; ++i, ++row) {
-        out_logprob[idx[i]] += h_logp[row];
-        if (out_token_logp) out_token_logp[(size_t)idx[i] * (max_tgt + 1) + t] = h_logp[row];
-      }
-    if (out_token_logp)
-      for (int i = 0; i < cn; ++i)
-        for (int t = tlen(idx[i]) + 1; t <= max_tgt; ++t) out_token_logp[(size_t)idx[i] * (max_tgt + 1) + t] = 0.f;
+  const int steps = tlen(idx[0]) + 1;        // forwards: one per token and one for EOS
+  int Smax = 0;
+  size_t n_ids = 0;
+  for (int i = 0; i < cn; ++i) {
+    const int len = src_off[idx[i] + 1] - src_off[idx[i]];
+    if (len < 1) return fail(LINMT_EINVAL, "empty source sentence");
+    if (len > opt.max_src_len) return fail(LINMT_ELIMIT, "source sentence longer than max_src_len");
+    h_meta_[i] = (int32_t)n_ids; h_meta_[(B + 1) + i] = len; h_meta_[2 * (B + 1) + i] = steps - 1; h_meta_[3 * (B + 1) + i] = i;
+    n_ids += len;
+    Smax = std::max(Smax, len);
   }
-  stats.last_decode_ms = total_ms;
+  std::vector<int> n_act(steps, 0);
+  size_t rows = 0;
+  for (int t = 0; t < steps; ++t) {
+    while (n_act[t] < cn && tlen(idx[n_act[t]]) >= t) ++n_act[t];
+    rows += n_act[t];
+  }
+  // ids | tokens read [steps][cn] | tokens asked for [rows], up in one copy; log-probabilities [rows] back
+  const size_t n_up = n_ids + (size_t)steps * cn + rows;
+  if (n_up + rows > score_io_cap_) {
+    if (int rc = regrow(&score_io_, n_up + rows)) return rc;
+    score_io_cap_ = n_up + rows;
+  }
+  if (int rc = reserve_host((n_up + rows) * 4)) return rc;
+  int32_t *h_tok = h_stage_ + n_ids, *h_gold = h_tok + (size_t)steps * cn;
+  for (int i = 0; i < cn; ++i)
+    std::memcpy(h_stage_ + h_meta_[i], src_ids + src_off[idx[i]], sizeof(int32_t) * h_meta_[(B + 1) + i]);
+  size_t row = 0;
+  for (int t = 0; t < steps; ++t)
+    for (int i = 0; i < cn; ++i) {
+      const int32_t* tgt = tgt_ids + tgt_off[idx[i]];
+      h_tok[(size_t)t * cn + i] = t == 0 || i >= n_act[t] ? kStart : tgt[t - 1];
+      if (i < n_act[t]) h_gold[row++] = t < tlen(idx[i]) ? tgt[t] : kEos;
+    }
+  CK(cudaEventRecord(ev0_, stream));
+  CK(cudaMemcpyAsync(d_off_, h_meta_, sizeof(int32_t) * 4 * (B + 1), cudaMemcpyHostToDevice, stream));
+  CK(cudaMemcpyAsync(score_io_, h_stage_, n_up * 4, cudaMemcpyHostToDevice, stream));
+  cur_ids_ = score_io_;
+  trace_dev_ = TraceDev{};
+  kt_used_ = 0; rec_flops_ = 0.0;
+  float* d_logp = reinterpret_cast<float*>(score_io_ + n_up);
+  int rc = score_core_tc(cn, Smax, n_act, score_io_ + n_ids, score_io_ + n_ids + (size_t)steps * cn, d_logp);
+  if (rc) { cudaStreamSynchronize(stream); return rc; }
+  if ((rc = kt(KC_END))) return rc;
+  CK(cudaEventRecord(ev1_, stream));
+  const float* h_logp = reinterpret_cast<const float*>(h_stage_ + n_up);
+  CK(cudaMemcpyAsync(h_stage_ + n_up, d_logp, rows * 4, cudaMemcpyDeviceToHost, stream));
+  if ((rc = finish_timing())) return rc;
+  row = 0;
+  for (int i = 0; i < cn; ++i) out_logprob[idx[i]] = 0.f;
+  for (int t = 0; t < steps; ++t)
+    for (int i = 0; i < n_act[t]; ++i, ++row) {
+      out_logprob[idx[i]] += h_logp[row];
+      if (out_token_logp) out_token_logp[(size_t)idx[i] * (max_tgt + 1) + t] = h_logp[row];
+    }
+  if (out_token_logp)
+    for (int i = 0; i < cn; ++i)
+      for (int t = tlen(idx[i]) + 1; t <= max_tgt; ++t) out_token_logp[(size_t)idx[i] * (max_tgt + 1) + t] = 0.f;
   return LINMT_OK;
 }
 
-int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::function<int(Engine&, int)>& job) {
-  const int ne = h->n_engines();
+int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& job) {
+  const int ne = (int)workers.size();
   if (ne == 1 || order.size() <= 1) {
     for (int item : order)
       if (int rc = job(h->eng, item)) return rc;
@@ -998,7 +1008,7 @@ int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::fu
   std::mutex err_mutex;
   std::string err_text;
   auto worker = [&](int ei) {
-    Engine& g = h->engine(ei);
+    Engine& g = *workers[ei];
     while (first_rc.load() == LINMT_OK) {
       const size_t i = next.fetch_add(1);
       if (i >= order.size()) break;
@@ -1017,6 +1027,16 @@ int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::fu
   return first_rc.load();
 }
 
+// Few rows are a chain of launches in which most of the chip waits, for the next launch or for weights: the device batches of a call
+// that has several run at once, a stream and a host thread each.  ms a batch of 64 sentences of 20 to 30 words with 1, 2, 3 at
+// once: 4 x 1000 / 30k 64 rows 6.4, 5.3, 5.3; 32 rows 5.3, 3.6, 3.3; 256 rows 9.3, 7.8, 7.9; 768 rows 15.2, 14.8, 15.0; in bf16 64 rows
+// 5.0, 3.9, 3.8; scoring 128 sentences in bf16 3.2, 2.3, 2.4; 3 x 250 / 5k 256 rows 4.4, 2.6, 2.0.  (Ensembles' members run side by side
+// already.  Where events time the kernels, one after another.)
+int Engine::lanes_for(int rows) const {
+  if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512) return 1;
+  return rows <= 32 || !step_streams(false, rows) ? 3 : 2;
+}
+
 }  // namespace linmt
 
 // =========================================================================================
@@ -1024,6 +1044,29 @@ int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::fu
 // =========================================================================================
 using linmt::Engine;
 
+std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_device) {
+  std::vector<Engine*> w;
+  const int devices = first_device ? 1 : n_engines();
+  for (int i = 0; i < devices; ++i) w.push_back(&engine(i));
+  const int per = eng.lanes_for(rows);
+  for (int j = 1; j < per && w.size() < items; ++j)
+    for (int i = 0; i < devices && w.size() < items; ++i) {
+      Engine& of = engine(i);
+      // the j-th lane of the i-th device
+      Engine* lane = nullptr;
+      int seen = 0;
+      for (auto& l : lanes)
+        if (l->opt.device == of.opt.device && ++seen == j) lane = l.get();
+      if (!lane && !no_more_lanes) {
+        std::unique_ptr<Engine> l(new (std::nothrow) Engine());
+        if (l && l->init_lane(of) == LINMT_OK) { lane = l.get(); lanes.push_back(std::move(l)); }
+        else { no_more_lanes = true; cudaGetLastError(); }
+      }
+      if (lane) w.push_back(lane);
+    }
+  cudaSetDevice(eng.opt.device);
+  return w;
+}
 
 static std::string g_create_error;
 
@@ -1095,31 +1138,32 @@ int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* s
   if (!e) return LINMT_EINVAL;
   Engine& g0 = e->eng;
   const int B = g0.B;
-  if (e->n_engines() == 1 || trace || n <= B || !src_ids || !src_off || !steps || !out_tok || !out_len || !out_score)
+  if ((g0.kernel_timing && e->n_engines() == 1) || trace || n <= B || !src_ids || !src_off || !steps || !out_tok || !out_len || !out_score)
     return g0.decode_host(src_ids, src_off, n, steps, max_len, out_tok, out_len, out_score, out_vit, out_align, trace);
-  // several devices: the same device batches as on one, dealt to the devices' host threads as they become free, the
-  // batches with the most decoder forwards first (they are in that order)
+  // several device batches: dealt to the engines' host threads as they become free, the batches with the most decoder
+  // forwards first (they are in that order)
   if (out_align && !g0.opt.print_info) { g0.err = "alignments need print_info = 1"; return LINMT_EINVAL; }
   const linmt::Engine::HostJob jb{src_ids, src_off, steps, max_len, out_tok, out_len, out_score, out_vit, out_align};
   const std::vector<int> sents = linmt::batch_order(src_off, n, steps);
   const int nchunks = (n + B - 1) / B;
   std::vector<int> order(nchunks);
   std::iota(order.begin(), order.end(), 0);
-  std::vector<float> ms_per_engine(e->n_engines(), 0.f);
+  const std::vector<Engine*> workers = e->workers(nchunks, B * g0.k, false);
+  std::vector<float> ms_per_engine(workers.size(), 0.f);
   std::mutex stat_mutex;
-  int rc = linmt::run_on_engines(e, order, [&](Engine& g, int c) -> int {
+  int rc = linmt::run_on_engines(e, workers, order, [&](Engine& g, int c) -> int {
     const int cn = std::min(B, n - c * B);
     if (cudaSetDevice(g.opt.device) != cudaSuccess) { g.err = "cudaSetDevice failed"; return LINMT_ECUDA; }
     int r = g.decode_chunk(jb, sents.data() + (size_t)c * B, cn, nullptr, 0);
     if (r == LINMT_OK) {
       std::lock_guard<std::mutex> lock(stat_mutex);
-      for (int i = 0; i < e->n_engines(); ++i)
-        if (&e->engine(i) == &g) ms_per_engine[i] += g.stats.last_decode_ms;
+      for (size_t i = 0; i < workers.size(); ++i)
+        if (workers[i] == &g) ms_per_engine[i] += g.stats.last_decode_ms;
     }
     return r;
   });
   if (rc != LINMT_OK) return rc;
-  // device time of the call = the busiest device's; the counters of the replicas are folded into the handle's
+  // device time of the call = the busiest engine's; the counters of the others are folded into the handle's
   g0.stats.last_decode_ms = *std::max_element(ms_per_engine.begin(), ms_per_engine.end());
   return LINMT_OK;
 }
@@ -1148,7 +1192,26 @@ int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* sr
     Tm = std::max(Tm, steps[i]);
   }
   if (out_token_logp && max_tgt < Tm) { g.err = "max_tgt smaller than the longest target"; return LINMT_EINVAL; }
-  if (g.scores_rows()) return g.score_host(src_ids, src_off, tgt_ids, tgt_off, n, out_logprob, out_token_logp, max_tgt);
+  if (g.scores_rows()) {
+    // device batches of max_batch sentences, longest target first
+    const Engine::ScoreJob jb{src_ids, src_off, tgt_ids, tgt_off, out_logprob, out_token_logp, max_tgt};
+    const int B = g.B, nchunks = (n + B - 1) / B;
+    std::vector<int> sents(n), order(nchunks);
+    std::iota(sents.begin(), sents.end(), 0);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(sents.begin(), sents.end(), [&](int a, int b) { return steps[a] > steps[b]; });
+    const std::vector<Engine*> workers = e->workers(nchunks, B, true);
+    std::vector<float> ms(workers.size(), 0.f);
+    const int rc = linmt::run_on_engines(e, workers, order, [&](Engine& w, int c) -> int {
+      const int r = w.score_chunk(jb, sents.data() + (size_t)c * B, std::min(B, n - c * B));
+      if (r == LINMT_OK)
+        for (size_t i = 0; i < workers.size(); ++i)
+          if (workers[i] == &w) ms[i] += w.stats.last_decode_ms;      // (an engine's own)
+      return r;
+    });
+    if (rc == LINMT_OK) g.stats.last_decode_ms = *std::max_element(ms.begin(), ms.end());
+    return rc;
+  }
   // CUDA-core path: a forced decode; every beam slot is forced to the given token, slot b continues slot b
   std::vector<int32_t> ftok((size_t)n * Tm * k, 2), fpar((size_t)n * Tm * k, 0);
   std::vector<float> fscore((size_t)n * Tm * k, 0.f), gold((size_t)n * Tm * k, 0.f), fin((size_t)n * k, 0.f);
@@ -1188,12 +1251,13 @@ int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* sr
 int linmt_get_stats(const linmt_engine* e, linmt_stats* out) {
   if (!e || !out) return LINMT_EINVAL;
   *out = e->eng.stats;
-  for (const auto& r : e->replicas) {   // launches and forwards of every device
-    out->kernel_launches += r->stats.kernel_launches;
-    out->pair_launches += r->stats.pair_launches;
-    out->decoder_row_steps += r->stats.decoder_row_steps;
-    out->sentence_steps += r->stats.sentence_steps;
-  }
+  for (const auto* others : {&e->replicas, &e->lanes})
+    for (const auto& r : *others) {   // launches and forwards of every engine
+      out->kernel_launches += r->stats.kernel_launches;
+      out->pair_launches += r->stats.pair_launches;
+      out->decoder_row_steps += r->stats.decoder_row_steps;
+      out->sentence_steps += r->stats.sentence_steps;
+    }
   return LINMT_OK;
 }
 

@@ -83,6 +83,10 @@ class Engine {
   Engine() = default;
   ~Engine();
   int init(const linmt_model_desc& d, const float* const* blobs, int n_models, size_t blob_floats, const linmt_options& o);
+  // An engine on the same device with the weights of `of`, which it must not outlive, and state, stream and workspaces of its own.
+  int init_lane(const Engine& of);
+  // Device batches of a call that are worth running at once, of this engine's `rows` each.
+  int lanes_for(int rows) const;
   int decode_core(const int32_t* d_ids, const int32_t* off_host, int n, const int32_t* steps_host, int max_len,
                   int32_t* d_out_tok, int32_t* d_out_len, float* d_out_score, int32_t* d_out_vit, float* d_out_align,
                   const linmt_trace* trace_dev, int trace_Tm);
@@ -93,8 +97,12 @@ class Engine {
     int32_t *out_tok, *out_len; float* out_score; int32_t* out_vit; float* out_align;
   };
   int decode_chunk(const HostJob& jb, const int* idx, int cn, const linmt_trace* trace_dev, int Tm_all);
-  int score_host(const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids, const int32_t* tgt_off, int n,
-                 float* out_logprob, float* out_token_logp, int max_tgt);
+  // a scoring call's arrays (linmt_score_batch), and one device batch of it: sentences idx[0..cn), longest target first
+  struct ScoreJob {
+    const int32_t *src_ids, *src_off, *tgt_ids, *tgt_off;
+    float *out_logprob, *out_token_logp; int max_tgt;
+  };
+  int score_chunk(const ScoreJob& jb, const int* idx, int cn);
   bool scores_rows() const { return use_tc_; }    // (the CUDA-core path scores through a forced decode)
   int decode_host(const int32_t* src_ids, const int32_t* src_off, int n, const int32_t* steps, int max_len,
                   int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align,
@@ -118,6 +126,7 @@ class Engine {
   std::string result_buf;
 
  private:
+  int init_state(const Engine* of, const float* const* blobs);
   int fail(int code, const std::string& msg) { err = msg; return code; }
   // role of member mi in the alignment record of a step: 0 = single model, 1 / 2 / 3 = first / middle / last member
   int ens_member_code(int mi) const { return n_models == 1 ? 0 : (mi == 0 ? 1 : (mi == n_models - 1 ? 3 : 2)); }
@@ -181,6 +190,8 @@ class Engine {
   bool stream_weights_ = false;  // the products issued are a step's (or scoring's vocabulary products), whose weights do not fit L2
   int l2_bytes_ = 0;
   bool rows_ = true;       // weight-streaming kernel for few rows (LINMT_TC_ROWS=0: test knob)
+  bool ahead_ = true;      // recurrent products behind the step before (LINMT_AHEAD=0: test knob)
+  bool lanes_ = true;      // device batches of a call at once (LINMT_LANES=0: test knob)
   bool persist_ = true;    // persistent kernel for the many-wave vocabulary GEMM (LINMT_TC_PERSIST=0: test knob)
   bool beside_ = false;      // the products issued leave room for the next one's CTAs (GemmLimits::beside)
   bool want_late_ = false, got_late_ = false;   // the next product is asked to let its successor start only behind its wait; the last one asked does
@@ -289,13 +300,19 @@ void pack_gate_weights(const float* const* mats, int nseg, int H, int Hp, float*
 struct linmt_engine {
   linmt::Engine eng;
   std::vector<std::unique_ptr<linmt::Engine>> replicas;
+  // Further engines on the devices above, with their weights: a call of several device batches runs some at once (Engine::lanes_for).
+  // Made when such a call first wants them, and kept; where memory does not suffice a call does with what there is.
+  std::vector<std::unique_ptr<linmt::Engine>> lanes;
+  bool no_more_lanes = false;
+  // the engines that share `items` device batches of `rows` rows, on the first device alone or on all
+  std::vector<linmt::Engine*> workers(size_t items, int rows, bool first_device);
   int n_engines() const { return 1 + (int)replicas.size(); }
   linmt::Engine& engine(int i) { return i == 0 ? eng : *replicas[i - 1]; }
 };
 
 namespace linmt {
 std::vector<int> batch_order(const int32_t* src_off, int n, const int32_t* steps);
-// Runs job(engine, item) for item = order[0], order[1], ... on the engines of a handle, one host thread per
+// Runs job(engine, item) for item = order[0], order[1], ... on engines of a handle (linmt_engine::workers), one host thread per
 // engine, each taking the next item when it is free.  Returns the first error; engine 0's `err` names it.
-int run_on_engines(linmt_engine* h, const std::vector<int>& order, const std::function<int(Engine&, int)>& job);
+int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& job);
 }  // namespace linmt

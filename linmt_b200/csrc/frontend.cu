@@ -525,11 +525,11 @@ int linmt_decode_file(linmt_engine* h, const char* in_path, const char* out_path
   const int nb = e.opt.nbest, B = e.opt.max_batch;
   const bool info = e.opt.print_info != 0;
   const bool want_align = info && e.print_align_scores;
-  // one job per device batch; with several devices each device's host thread takes the next batch when it is
+  // one job per device batch; each engine's host thread takes the next batch when it is
   // free (the batches are in descending step count, so the long ones go first)
   std::vector<int> batch_ids;
   for (size_t b0 = 0; b0 < order.size(); b0 += B) batch_ids.push_back((int)(b0 / B));
-  const int rc_all = run_on_engines(h, batch_ids, [&](Engine& g, int bi) -> int {
+  const int rc_all = run_on_engines(h, h->workers(batch_ids.size(), B * e.k, false), batch_ids, [&](Engine& g, int bi) -> int {
     const size_t b0 = (size_t)bi * B;
     const int n = (int)std::min<size_t>(B, order.size() - b0);
     std::vector<int32_t> ids, off(1, 0), steps;

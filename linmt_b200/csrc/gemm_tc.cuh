@@ -32,6 +32,7 @@
 // (gemm_tc_persist_kernel) serves the many-wave vocabulary GEMM; gemm_tc_pair.cuh holds the forms of both kernels
 // that run on CTA pairs (tcgen05 cta_group::2), used where a launch is wide enough for them to pay.
 #pragma once
+#include <atomic>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -1459,7 +1460,7 @@ inline bool make_tmap(CUtensorMap* map, const __nv_bfloat16* ptr, uint64_t rows,
 // it is set once per (kernel, device), for the device that is current at the launch.
 constexpr int kMaxDevices = 64;
 template <class Kernel>
-inline cudaError_t ensure_smem_optin(Kernel* kernel, bool* done_per_device, int bytes = SMEM_BUDGET + 1280) {
+inline cudaError_t ensure_smem_optin(Kernel* kernel, std::atomic<bool>* done_per_device, int bytes = SMEM_BUDGET + 1280) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -1478,7 +1479,7 @@ constexpr int kSmemPerBlock = 227 * 1024;
 template <auto Kernel>
 inline cudaError_t allow_smem(size_t dynamic_bytes) {
   if (dynamic_bytes <= 24 * 1024) return cudaSuccess;
-  static bool done[kMaxDevices] = {};
+  static std::atomic<bool> done[kMaxDevices] = {};
   cudaFuncAttributes attr;
   if (cudaError_t e = cudaFuncGetAttributes(&attr, Kernel); e != cudaSuccess) return e;
   return ensure_smem_optin(Kernel, done, kSmemPerBlock - (int)attr.sharedSizeBytes);
@@ -1487,7 +1488,7 @@ inline cudaError_t allow_smem(size_t dynamic_bytes) {
 template <int NT, int BKT, int FMT, class Epi>
 inline cudaError_t launch_gemm_tc_nt(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
                                      cudaStream_t st, float* ws, int* counters, int a_row0) {
-  static bool optin_done[kMaxDevices] = {};
+  static std::atomic<bool> optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_kernel<NT, BKT, FMT, Epi>, optin_done); e != cudaSuccess) return e;
   const int splits = (sh.splits > 1 && ws && counters) ? sh.splits : 1;
   dim3 grid((M + BM - 1) / BM, (N + sh.bn - 1) / sh.bn, splits);
@@ -1539,7 +1540,7 @@ inline cudaError_t launch_gemm_tc_persist(const TmapSet& tm, int M, int N, int K
   const dim3 grid(tiles < n_sm ? tiles : n_sm);
 #define LINMT_PERSIST_CASE(NTV, BKV, FMTV)                                                                                   \
   {                                                                                                                          \
-    static bool optin_done[kMaxDevices] = {};                                                                                \
+    static std::atomic<bool> optin_done[kMaxDevices] = {};                                                                                \
     if (cudaError_t e = ensure_smem_optin(gemm_tc_persist_kernel<NTV, BKV, FMTV, Epi>, optin_done); e != cudaSuccess) return e; \
     return launch_k(sh.pdl != 0, gemm_tc_persist_kernel<NTV, BKV, FMTV, Epi>, grid, dim3(kThreads), (size_t)sh.smem_bytes, st, tm, M, N, K, \
                     sh.bn, sh.stages, epi, err_flag);                                                                \

@@ -352,7 +352,7 @@ gemm_tc_pair_kernel(const __grid_constant__ TmapSet tm, int M, int N, int K, int
 template <int NT, int BKT, int FMT, class Epi>
 inline cudaError_t launch_gemm_tc_pair(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
                                        cudaStream_t st, float* ws, int* counters) {
-  static bool optin_done[kMaxDevices] = {};
+  static std::atomic<bool> optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_pair_kernel<NT, BKT, FMT, Epi>, optin_done); e != cudaSuccess) return e;
   if (sh.bn % 16) return cudaErrorInvalidValue;
   const int splits = (sh.splits > 1 && ws && counters) ? sh.splits : 1;
@@ -549,7 +549,7 @@ template <int FMT, class Epi>
 inline cudaError_t launch_gemm_tc_persist_pair(const TmapSet& tm, int M, int N, int K, const Shape& sh, const Epi& epi, int* err_flag,
                                                cudaStream_t st, int n_sm) {
   if (K % 64 || sh.stages < 2 || sh.bn % 16 || sh.bn > 256) return cudaErrorInvalidValue;
-  static bool optin_done[kMaxDevices] = {};
+  static std::atomic<bool> optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_persist_pair_kernel<FMT, Epi>, optin_done); e != cudaSuccess) return e;
   const int mt2 = ((M + BM - 1) / BM + 1) / 2;
   const int tiles = mt2 * ((N + sh.bn - 1) / sh.bn);
@@ -570,7 +570,7 @@ inline cudaError_t launch_gemm_tc_persist_pair(const TmapSet& tm, int M, int N, 
 // cannot be scheduled here, e.g. on a partitioned device, and the host must keep to the one-tile kernels).
 template <int NT, int BKT, int FMT, class Epi>
 inline int max_resident_pairs() {
-  static bool optin_done[kMaxDevices] = {};
+  static std::atomic<bool> optin_done[kMaxDevices] = {};
   if (ensure_smem_optin(gemm_tc_pair_kernel<NT, BKT, FMT, Epi>, optin_done) != cudaSuccess) { cudaGetLastError(); return 0; }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2, 1, 1); cfg.blockDim = dim3(kThreadsMain); cfg.dynamicSmemBytes = (size_t)(SMEM_BUDGET + 1280);

@@ -388,7 +388,7 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSets<SEGS> tms, int M, int N, in
 // x_row0: first row of the product in the activations' tensor map
 template <int NT, int FMT, class Epi, int SEGS, bool LATE>
 inline cudaError_t launch_gemm_tc_rows_of(const TmapSets<SEGS>& tms, int segs, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0) {
-  static bool optin_done[kMaxDevices] = {};
+  static std::atomic<bool> optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_rows_kernel<NT, FMT, Epi, SEGS, LATE>, optin_done, kRowsSmemWhole); e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((N + BM - 1) / BM, segs, sh.splits); cfg.blockDim = dim3(kRowsThreads);

@@ -523,3 +523,30 @@ def test_recurrent_products_ahead_in_one_plane(cuda_lib, n, beam):
         T = int(sents.steps[i])
         a, b = np.sort(e["cand_logp"][i, 1:T]), np.sort(r["cand_logp"][i, 1:T])
         assert (np.abs(a - b) <= 2e-2).all(), float(np.abs(a - b).max())
+
+
+@pytest.mark.parametrize("precision,beam,max_batch,n,info", [("fp32", 1, 4, 31, False), ("fp32", 5, 8, 17, True), ("bf16", 3, 16, 70, False),
+                                                             ("fp32", 16, 32, 65, False), ("fp32", 2, 3, 4, False)])     # (the fourth: 512 rows)
+def test_device_batches_of_a_call_at_once(cuda_lib, precision, beam, max_batch, n, info):
+    """A call of several device batches runs some of them at once, decoding and scoring: the bits of one after another, in
+    every call, and its counters are of all of them."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, 256, 3000, 300, 1)
+    blob = synth.make_blob(d, 40, family="peaked")
+    sents = synth.make_sentences(n, 1, 14, d.Vs, 1.1, 3, lambda s: s + 3)
+    rng = np.random.default_rng(n)
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 12, size=n)]
+    kw = dict(beam=beam, precision=precision, max_batch=max_batch, max_src_len=16, max_steps=20, print_info=info, cp_beta=0.2 if info else 0.0)
+    dec = decoder.Decoder(d, [blob], **kw)
+    one = _with_env({"LINMT_LANES": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    for call in range(3):
+        a, b = dec.decode(sents, want_align=info), one.decode(sents, want_align=info)
+        for key in ("tok", "len", "score") + (("vit", "align") if info else ()):
+            assert a[key].tobytes() == b[key].tobytes(), (call, key)
+        for x, y in zip(dec.score(sents, targets), one.score(sents, targets)):
+            assert x.tobytes() == y.tobytes(), call
+    for key in ("kernel_launches", "decoder_row_steps", "sentence_steps"):
+        assert abs(dec.stats()[key] - one.stats()[key]) <= (100 if key == "kernel_launches" else 0), key    # (a handle's and its lanes' creation)
+    short = synth.make_sentences(1, 3, 3, d.Vs, 1.1, 3, lambda s: s + 3)      # one batch, after many
+    assert dec.decode(short)["tok"].tobytes() == one.decode(short)["tok"].tobytes()
+    dec.close(); one.close()
