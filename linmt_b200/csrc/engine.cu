@@ -1034,7 +1034,7 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
 // already.  Where events time the kernels, one after another.)
 int Engine::lanes_for(int rows) const {
   if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512) return 1;
-  return rows <= 32 || !step_streams(false, rows) ? 3 : 2;
+  return rows <= 64 || !step_streams(false, rows) ? 3 : 2;
 }
 
 }  // namespace linmt
@@ -1149,11 +1149,13 @@ int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* s
   std::vector<int> order(nchunks);
   std::iota(order.begin(), order.end(), 0);
   const std::vector<Engine*> workers = e->workers(nchunks, B * g0.k, false);
+  const bool together = nchunks > 1 && g0.lanes_for(B * g0.k) > 1;
   std::vector<float> ms_per_engine(workers.size(), 0.f);
   std::mutex stat_mutex;
   int rc = linmt::run_on_engines(e, workers, order, [&](Engine& g, int c) -> int {
     const int cn = std::min(B, n - c * B);
     if (cudaSetDevice(g.opt.device) != cudaSuccess) { g.err = "cudaSetDevice failed"; return LINMT_ECUDA; }
+    const linmt::Engine::Several several(g, together);
     int r = g.decode_chunk(jb, sents.data() + (size_t)c * B, cn, nullptr, 0);
     if (r == LINMT_OK) {
       std::lock_guard<std::mutex> lock(stat_mutex);
@@ -1201,8 +1203,10 @@ int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* sr
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(sents.begin(), sents.end(), [&](int a, int b) { return steps[a] > steps[b]; });
     const std::vector<Engine*> workers = e->workers(nchunks, B, true);
+    const bool together = nchunks > 1 && g.lanes_for(B) > 1;
     std::vector<float> ms(workers.size(), 0.f);
     const int rc = linmt::run_on_engines(e, workers, order, [&](Engine& w, int c) -> int {
+      const Engine::Several several(w, together);
       const int r = w.score_chunk(jb, sents.data() + (size_t)c * B, std::min(B, n - c * B));
       if (r == LINMT_OK)
         for (size_t i = 0; i < workers.size(); ++i)

@@ -98,14 +98,22 @@ const CUtensorMap* Engine::maps(const tc::Planes& p, int col0, int rows, int K, 
   return it->second.data();
 }
 
+// Products of a device batch that others run beside: up to 64 rows in CTAs of half an SM, as few of them as leave room for another
+// product's; beyond, in tiles for half of the SMs.  4 x 1000 / 30k, ms a call shaped for the whole
+// chip / so: 300 sentences greedily, 64 rows in a batch, 36.2 / 31.4; four batches, greedily 128 rows 25.3 / 21.5; beam 4, 128 rows 23.7 / 20.4, 256 rows
+// 28.6 / 27.1; beam 8, 512 rows 42.5 / 41.2; scoring 128 15.9 / 13.8, in bf16 8.6 / 8.1.  (Products of all positions fill the chip.)
+static constexpr int kSeveralFew = 64, kSeveralMost = 512;
+
 // C[M][N] = A[:, a_col0 : a_col0+K] . W[N][K]^T on the kernel and in the shape that plan_gemm chooses.
 template <class Epi>
 int Engine::tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e_in, int nt, int drain, int x_row0) {
   Epi e = e_in;
   if (nt <= 0 || nt > nt_) nt = nt_;
   tc::GemmLimits lim;
-  lim.beside = beside_;
-  lim.n_sm = n_sm_; lim.parts = plan_parts_ ? plan_parts_ : ws_parts_; lim.rows = rows_; lim.pair = pair_; lim.persist = persist_;
+  lim.beside = beside_ || several_;
+  lim.n_sm = n_sm_; lim.parts = plan_parts_ ? plan_parts_ : ws_parts_;
+  if (several_ && lim.parts == 1 && M > kSeveralFew && M <= kSeveralMost) lim.parts = 2;
+  lim.rows = rows_; lim.pair = pair_; lim.persist = persist_;
   // a layer's slice of the split-K workspace: whole 256-byte units, so that every slice starts aligned for the
   // 16-byte partial-tile stores whatever the number of layers sharing it
   lim.ws_floats = (kSplitKWsFloats / ws_parts_) & ~(size_t)63;

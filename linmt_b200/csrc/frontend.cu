@@ -529,7 +529,9 @@ int linmt_decode_file(linmt_engine* h, const char* in_path, const char* out_path
   // free (the batches are in descending step count, so the long ones go first)
   std::vector<int> batch_ids;
   for (size_t b0 = 0; b0 < order.size(); b0 += B) batch_ids.push_back((int)(b0 / B));
+  const bool together = batch_ids.size() > 1 && e.lanes_for(B * e.k) > 1;
   const int rc_all = run_on_engines(h, h->workers(batch_ids.size(), B * e.k, false), batch_ids, [&](Engine& g, int bi) -> int {
+    const Engine::Several several(g, together);
     const size_t b0 = (size_t)bi * B;
     const int n = (int)std::min<size_t>(B, order.size() - b0);
     std::vector<int32_t> ids, off(1, 0), steps;

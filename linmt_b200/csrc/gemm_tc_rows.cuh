@@ -103,14 +103,17 @@ inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, b
     // f16 pair: w0 meets both planes of the activations in ONE instruction (N = 2 rp, the planes lie one behind the
     // other), so an accumulator holds w0 x0 | w0 x1; beyond 64 rows an instruction per product takes as long, and the
     // columns are better spent on short chains
-    s.stacked = nt == 2 && s.rp <= 64;
-    s.acc_stride = s.stacked ? 2 * s.rp : (s.rp + 31) & ~31;
-    s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
-    if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
-    const bool chains = nt == 1 || one_chain || (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
-    if (s.leads >= 1 && chains && rows_set_splits(&s, K, nt)) {
-      *out = s;
-      return true;
+    // (or not, where that gives short enough chains in half an SM's columns and the SM is to be shared)
+    for (s.stacked = nt == 2 && s.rp <= 64; s.stacked >= 0; --s.stacked) {
+      s.acc_stride = s.stacked ? 2 * s.rp : (s.rp + 31) & ~31;
+      s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
+      if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
+      const bool chains = nt == 1 || one_chain || (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
+      if (s.leads >= 1 && chains && rows_set_splits(&s, K, nt)) {
+        *out = s;
+        return true;
+      }
+      if (!beside) break;
     }
   }
   return false;
