@@ -145,7 +145,7 @@ class Engine {
   int run_encoder_tc(int n, int Smax);
   int run_encoder_layers_tc(int n, int Smax);   // few sentences: layer by layer
   int encode_member_layers(int mi, int n, int Smax, int per);
-  int run_encoder_pipeline_tc(int n, int Smax);   // more sentences: the layers side by side, a few positions behind each other
+  int run_encoder_pipeline_tc(int n, int Smax, bool few);   // more sentences: the layers side by side, a few positions behind each other
   int encoder_streams();
   int encode_positions(int mi, int l, int n, int pos0, int np, float* pre, int block);
   int each_member(int rows, const std::function<int(int)>& work);

@@ -177,6 +177,7 @@ int Engine::build_xw_tables() {
 // Up to here the encoder's products of a position are shaped like a step's, so that the next one's weights are under way (4 x 1000, 32
 // positions: one sentence 4.77 -> 4.73 ms a call, eight 14.34 -> 14.16; 64: 0.2 to 2 % slower).
 static constexpr int kBesideSentences = 48;
+static constexpr int kEncFewWords = 20, kEncFewHidden = 512;     // (see run_encoder_pipeline_tc)
 static constexpr int kEncRing = 4;
 int Engine::encoder_streams() {
   if (!enc_streams_.empty()) return LINMT_OK;
@@ -203,8 +204,10 @@ int Engine::run_encoder_tc(int n, int Smax) {
   stream_weights_ = false; beside_ = n <= kBesideSentences;
   if (enc_rows_)
     switch (encoder_form(EncoderModel{L, Hp, n_models, nt_ > 1}, n, Smax)) {
-      case EncoderForm::kLayers: return run_encoder_layers_tc(n, Smax);
-      case EncoderForm::kPipelined: return run_encoder_pipeline_tc(n, Smax);
+      case EncoderForm::kLayers:
+        if (L > 1 && n_models == 1 && !several_ && Hp >= kEncFewHidden && Smax >= kEncFewWords) return run_encoder_pipeline_tc(n, Smax, true);
+        return run_encoder_layers_tc(n, Smax);
+      case EncoderForm::kPipelined: return run_encoder_pipeline_tc(n, Smax, false);
       case EncoderForm::kWavefront: break;
     }
   constexpr int kRing = kEncRing;
@@ -310,13 +313,19 @@ int Engine::encode_positions(int mi, int l, int n, int pos0, int np, float* pre,
   return LINMT_OK;
 }
 
-// Encoder for more sentences and longer sources: the layers side by side on a stream each, every one kEncLag positions behind the layer below.
+// Encoder for more sentences and longer sources (`few`: few sentences): the layers side by side on a stream each, every one kEncLag positions behind the layer below.
 // As in the form above, the input parts of that many positions are one product, and what is left of the recurrence reads
 // half of a layer's weights, which all layers' together (67 MB in fp32 precision) stay in L2; but every layer's products are
 // shaped for their share of the SMs and run beside the others'.  Sources longer than the panels are taken in chunks: the
 // layers fall in line at the end of one, and the next starts from the states it ended with (4 x 1000, 500 words, two chunks,
 // against one position after another: 40 sentences 14.2 / 19.7 ms, 64 15.6 / 20.7).
-int Engine::run_encoder_pipeline_tc(int n, int Smax) {
+// few: the products of few sentences are those of the form above, in CTAs of half an SM that leave room for the other layers'.
+// Encoder and one scored word, ms, layer by layer / so: 4 x 1000 1 sentence of 16, 32 and 80 words 0.59 / 0.61, 0.98 / 0.99, 1.98 / 1.51,
+// 8 sentences 0.67 / 0.66, 1.01 / 0.86, 2.12 / 1.63, 32 0.79 / 0.76, 1.29 / 1.02, 2.85 / 2.02; in bf16 1 0.46 / 0.44, 0.73 / 0.64, 1.57 /
+// 1.26, 48 0.67 / 0.63, 1.13 / 0.88, 2.49 / 1.71; 5 x 512 1 0.56 / 0.53, 0.92 / 0.77, 2.00 / 1.46; of 8 words 2 to
+// 8 % slower.  (Narrower models gain less in whole calls: 3 x 250 with 1 to 30 sentences of 40 words 2 to 3 % of a call, with 11 ragged ones it
+// lost 2 %.)
+int Engine::run_encoder_pipeline_tc(int n, int Smax, bool few) {
   if (int rc = encoder_streams()) return rc;
   hs_sent_ = 1; hs_pos_ = n;
   const int per = enc_rows_ / n;               // positions per chunk
@@ -348,7 +357,7 @@ int Engine::run_encoder_pipeline_tc(int n, int Smax) {
         for (int l = 0; l < L && rc == LINMT_OK; ++l) {
           if (l > 0) CK(cudaStreamWaitEvent(enc_streams_[l], enc_events_[l - 1][0], 0));
           stream = enc_streams_[l];       // (tc_gemm: on the layer's stream, with its slice of the split-K workspace)
-          ws_part_ = l; ws_parts_ = L; plan_parts_ = L;
+          ws_part_ = l; ws_parts_ = L; plan_parts_ = few ? 1 : L;
           float* pre = s.enc_pre + (size_t)l * share * 4 * Hp;
           tc::TcEpiF32 ei{nullptr, pre, 4 * Hp, 0};
           rc = l == 0 ? tc_gemm(ts.enc_in, 0, enc_rows_, m.p_enc_w[0], np * n, 4 * Hp, Hp, ei, 0, 0, p0 * n)

@@ -562,3 +562,30 @@ def test_device_batches_of_a_call_at_once(cuda_lib, precision, beam, max_batch, 
     short = synth.make_sentences(1, 3, 3, d.Vs, 1.1, 3, lambda s: s + 3)      # one batch, after many
     assert dec.decode(short)["tok"].tobytes() == one.decode(short)["tok"].tobytes()
     dec.close(); one.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16"])
+@pytest.mark.parametrize("L,H,n,longest,max_src", [(2, 512, 1, 20, 64), (5, 500, 3, 41, 48), (3, 512, 32, 33, 33), (4, 448, 64, 21, 24), (2, 512, 7, 500, 512), (3, 512, 2, 21, 21)])
+def test_encoder_of_few_sentences_side_by_side(cuda_lib, precision, L, H, n, longest, max_src):
+    """Sources of 20 words and more of at most 64 sentences: the layers side by side from 449 units on (rounded to 512), one after
+    another below, against the encoder position by position; log-probabilities of given words to fp32 rounding, or within the
+    bar of bf16."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(L, H, 300, 200, 1)
+    blob = synth.make_blob(d, 11, family="peaked" if precision == "fp32" else "flat")
+    rng = np.random.default_rng(n)
+    lens = np.concatenate([[longest], rng.integers(1, longest + 1, size=n - 1)]).astype(np.int32)
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    sents = synth.Sentences(synth.zipf_ids(rng, int(off[-1]), 1, d.Vs, 1.1), off, np.full(n, 3, np.int32))
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 4, size=n)]
+    kw = dict(beam=2, precision=precision, max_batch=n, max_src_len=max_src, max_steps=8, cp_beta=0.0)
+    dec = decoder.Decoder(d, [blob], **kw)
+    ref = _with_env({"LINMT_TC_ROWS": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    a, again, b = dec.score(sents, targets), dec.score(sents, targets), ref.score(sents, targets)
+    dec.close(); ref.close()
+    assert np.array_equal(a[1], again[1])
+    if precision == "fp32":
+        scale = np.maximum(1, np.abs(b[1]).max(axis=1, keepdims=True))
+        assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
+    else:
+        assert (np.abs(a[1] - b[1]) <= 2e-2).all(), float(np.abs(a[1] - b[1]).max())
