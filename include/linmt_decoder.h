@@ -183,7 +183,8 @@ typedef struct linmt_trace {
  *   out_score [n][nbest]
  *   out_vit   [n][nbest][max_len]  viterbi alignment per position, may be NULL
  *   out_align [n][nbest][max_len][max_src_len]  dense alignments, may be NULL (print_info only)
- * Sentences are processed in device batches of at most max_batch. */
+ * Sentences are processed in device batches of at most max_batch.  A call of several device batches of up to 512 beam slots
+ * runs two or three of them at once, each with state of its own; it is made at the first such call and kept. */
 int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n,
                        const int32_t* steps, int32_t max_len, int32_t* out_tok, int32_t* out_len,
                        float* out_score, int32_t* out_vit, float* out_align, const linmt_trace* trace);

@@ -1024,7 +1024,10 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
     }
   };
   std::vector<std::thread> threads;
-  for (int ei = 1; ei < ne; ++ei) threads.emplace_back(worker, ei);
+  try {
+    threads.reserve(ne - 1);
+    for (int ei = 1; ei < ne; ++ei) threads.emplace_back(worker, ei);
+  } catch (const std::exception&) {}      // (no more threads: those there are take every item)
   worker(0);
   for (auto& t : threads) t.join();
   if (first_rc.load() != LINMT_OK) h->eng.err = err_text;
@@ -1035,9 +1038,11 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
 // that has several run at once, a stream and a host thread each.  ms a batch of 64 sentences of 20 to 30 words with 1, 2, 3 at
 // once: 4 x 1000 / 30k 64 rows 6.4, 5.3, 5.3; 32 rows 5.3, 3.6, 3.3; 256 rows 9.3, 7.8, 7.9; 768 rows 15.2, 14.8, 15.0; in bf16 64 rows
 // 5.0, 3.9, 3.8; scoring 128 sentences in bf16 3.2, 2.3, 2.4; 3 x 250 / 5k 256 rows 4.4, 2.6, 2.0.  (Ensembles' members run side by side
-// already.  Where events time the kernels, one after another.)
+// already.  Where events time the kernels, one after another; and where the encoder states of a batch of the longest sources are
+// more than 2 GB, which every engine has for itself.)
 int Engine::lanes_for(int rows) const {
-  if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512) return 1;
+  const size_t states = (size_t)B * opt.max_src_len * Hp * 12;
+  if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512 || states > ((size_t)2 << 30)) return 1;
   return rows <= 64 || !step_streams(false, rows) ? 3 : 2;
 }
 
@@ -1062,9 +1067,11 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
       for (auto& l : lanes)
         if (l->opt.device == of.opt.device && ++seen == j) lane = l.get();
       if (!lane && !no_more_lanes) {
-        std::unique_ptr<Engine> l(new (std::nothrow) Engine());
-        if (l && l->init_lane(of) == LINMT_OK) { lane = l.get(); lanes.push_back(std::move(l)); }
-        else { no_more_lanes = true; cudaGetLastError(); }
+        try {
+          std::unique_ptr<Engine> l(new Engine());
+          if (l->init_lane(of) == LINMT_OK) { lane = l.get(); lanes.push_back(std::move(l)); }
+        } catch (const std::bad_alloc&) { lane = nullptr; }
+        if (!lane) { no_more_lanes = true; cudaGetLastError(); }
       }
       if (lane) w.push_back(lane);
     }
