@@ -36,14 +36,26 @@ namespace linmt {
 
 #define LAUNCHED() (++stats.kernel_launches)
 
+// Device memory, for whatever an engine needs it.  A refusal is this call's result alone: the runtime would report it again to the
+// next check of a launch.
+int Engine::device_memory(void** p, size_t bytes, const char* what) {
+  const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 1));
+  if (e == cudaSuccess) return LINMT_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return fail(LINMT_ENOMEM, std::string("cudaMalloc failed (") + what + "): " + cudaGetErrorString(e));
+}
+int Engine::host_memory(void** p, size_t bytes, const char* what) {
+  const cudaError_t e = cudaMallocHost(p, bytes);
+  if (e == cudaSuccess) return LINMT_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return fail(LINMT_ENOMEM, std::string("cudaMallocHost failed (") + what + "): " + cudaGetErrorString(e));
+}
 template <class T>
 int Engine::dalloc(T** p, size_t count) {
   void* q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-  if (e != cudaSuccess) {
-    err = std::string("cudaMalloc failed: ") + cudaGetErrorString(e);
-    return LINMT_ENOMEM;
-  }
+  if (int rc = device_memory(&q, std::max<size_t>(count, 1) * sizeof(T), "engine")) return rc;
   allocs_.push_back(q);
   *p = static_cast<T*>(q);
   return LINMT_OK;
@@ -376,7 +388,7 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   // what one copy brings in and what one memset clears at the start of a decode lies together
   DA(d_off_, 4 * (B + 1)); d_len_ = d_off_ + (B + 1); d_steps_ = d_off_ + 2 * (B + 1); d_orig_ = d_off_ + 3 * (B + 1);
   CK(cudaMemset(d_off_, 0, sizeof(int32_t) * 4 * (B + 1)));   // (the attention's prefetch may go by a length before the first copy)
-  CK(cudaMallocHost(&h_meta_, sizeof(int32_t) * (4 * (B + 1) + 1)));
+  if (int rc = host_memory(reinterpret_cast<void**>(&h_meta_), sizeof(int32_t) * (4 * (B + 1) + 1), "batch metadata")) return rc;
   h_err_ = h_meta_ + 4 * (B + 1);
   DA(d_tok_, 3 * (size_t)R + B); d_parent_ = d_tok_ + R; d_score_ = reinterpret_cast<float*>(d_tok_ + 2 * (size_t)R); d_fin_n_ = d_tok_ + 3 * (size_t)R;
   DA(d_hist_tok_, (size_t)Tcap * R); DA(d_hist_parent_, (size_t)Tcap * R);
@@ -802,7 +814,7 @@ int Engine::reserve_host(size_t bytes) {
   if (bytes <= h_stage_cap_) return LINMT_OK;
   if (h_stage_) cudaFreeHost(h_stage_);
   h_stage_ = nullptr; h_stage_cap_ = 0;
-  if (cudaMallocHost(&h_stage_, bytes) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMallocHost failed (host staging)");
+  if (int rc = host_memory(reinterpret_cast<void**>(&h_stage_), bytes, "staging")) return rc;
   h_stage_cap_ = bytes;
   return LINMT_OK;
 }
@@ -886,7 +898,7 @@ int Engine::decode_host(const int32_t* src_ids, const int32_t* src_off, int n, c
       auto mk = [&](size_t count, size_t esz, void* host_dst, const void* host_src, void** dev) -> int {
         if (!host_dst && !host_src) { *dev = nullptr; return LINMT_OK; }
         void* q = nullptr;
-        if (cudaMalloc(&q, std::max<size_t>(count, 1) * esz) != cudaSuccess) return fail(LINMT_ENOMEM, "trace buffer allocation failed");
+        if (int rc = device_memory(&q, std::max<size_t>(count, 1) * esz, "trace")) return rc;
         trace_allocs_.push_back(q);
         if (host_src) {
           if (cudaMemcpyAsync(q, host_src, count * esz, cudaMemcpyHostToDevice, stream) != cudaSuccess) return fail(LINMT_ECUDA, "trace upload failed");
@@ -910,7 +922,7 @@ int Engine::decode_host(const int32_t* src_ids, const int32_t* src_off, int n, c
       td.pt = nullptr;
       if (trace->pt) {
         void* q = nullptr;
-        if (cudaMalloc(&q, std::max<size_t>(n_pt * n_models, 1) * 4) != cudaSuccess) return fail(LINMT_ENOMEM, "trace buffer allocation failed");
+        if (int rc_pt = device_memory(&q, std::max<size_t>(n_pt * n_models, 1) * 4, "trace")) return rc_pt;
         trace_allocs_.push_back(q);
         if (cudaMemsetAsync(q, 0xff, n_pt * n_models * 4, stream) != cudaSuccess) return fail(LINMT_ECUDA, "trace clear failed");
         td.pt = static_cast<float*>(q);

@@ -232,6 +232,8 @@ class Engine {
   std::vector<DevModel> models_;
   std::vector<DevState> states_;
   std::vector<void*> allocs_;
+  int device_memory(void** p, size_t bytes, const char* what);
+  int host_memory(void** p, size_t bytes, const char* what);      // (pinned)
   template <class T> int dalloc(T** p, size_t count);
   template <class T> int regrow(T** p, size_t count);
 
@@ -274,7 +276,7 @@ class Engine {
   size_t score_io_cap_ = 0;
   template <class T> int dalloc_bytes(T** p, size_t bytes) {
     void* q = nullptr;
-    if (cudaMalloc(&q, bytes) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMalloc failed (scoring workspace)");
+    if (int rc = device_memory(&q, bytes, "scoring workspace")) return rc;
     allocs_.push_back(q);
     *p = static_cast<T*>(q);
     return LINMT_OK;

@@ -32,7 +32,7 @@ int Engine::alloc_planes(tc::Planes& p, size_t rows, int ld) {
   for (int t = 0; t < nt_; ++t) {
     void* q = nullptr;
     const size_t bytes = rows * (size_t)ld * sizeof(__nv_bfloat16);
-    if (cudaMalloc(&q, bytes ? bytes : 2) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMalloc failed (operand planes)");
+    if (int rc = device_memory(&q, bytes, "operand planes")) return rc;
     allocs_.push_back(q);
     if (cudaMemset(q, 0, bytes) != cudaSuccess) return fail(LINMT_ECUDA, "cudaMemset failed (operand planes)");
     p.p[t] = static_cast<__nv_bfloat16*>(q);
@@ -47,7 +47,7 @@ int Engine::to_planes(const std::vector<float>& host, size_t rows, int ld, tc::P
   float* tmp = nullptr;
   const size_t n = rows * (size_t)ld;
   if (host.size() < n) return fail(LINMT_EINVAL, "internal: packed matrix smaller than its planes");
-  if (cudaMalloc(&tmp, n * sizeof(float)) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMalloc failed (weight staging)");
+  if ((rc = device_memory(reinterpret_cast<void**>(&tmp), n * sizeof(float), "weight staging"))) return rc;
   // stream-ordered copy: the split kernel must not start before the last byte has landed
   cudaError_t e = cudaMemcpyAsync(tmp, host.data(), n * sizeof(float), cudaMemcpyHostToDevice, stream);
   if (e == cudaSuccess) {
@@ -159,7 +159,7 @@ int Engine::build_xw_tables() {
     DevModel& m = models_[mi];
     void* q = nullptr;
     const size_t bytes = (size_t)desc.vocab_tgt * 4 * Hp * sizeof(float);
-    if (cudaMalloc(&q, bytes) != cudaSuccess) return fail(LINMT_ENOMEM, "cudaMalloc failed (input-term table)");
+    if (int rc = device_memory(&q, bytes, "input-term table")) return rc;
     allocs_.push_back(q);
     m.dec_xw = static_cast<float*>(q);
     tc::TcEpiF32 e{nullptr, m.dec_xw, 4 * Hp, 0};

@@ -15,7 +15,11 @@ namespace {
 struct DevBuf {
   void* p = nullptr;
   ~DevBuf() { if (p) cudaFree(p); }
-  cudaError_t alloc(size_t bytes) { return cudaMalloc(&p, bytes ? bytes : 1); }
+  cudaError_t alloc(size_t bytes) {
+    const cudaError_t e = cudaMalloc(&p, bytes ? bytes : 1);
+    if (e != cudaSuccess) cudaGetLastError();      // (or the next launch that is checked reports it again)
+    return e;
+  }
   template <class T> T* as() { return static_cast<T*>(p); }
 };
 #define KCK(x) do { if ((x) != cudaSuccess) return LINMT_ECUDA; } while (0)

@@ -1,0 +1,74 @@
+"""The engine's host side on the CPU: a child process decodes with tests/cpp/fake_cudart.cpp in the place of the CUDA runtime, whose
+kernels do nothing, and looks at what the engine asked the runtime for."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+HEAD = """
+import ctypes as C, os, sys
+fake = C.CDLL(os.environ["LD_PRELOAD"])
+fake.fake_get.restype = fake.fake_launches.restype = C.c_long
+sys.path.insert(0, %r)
+import numpy as np
+from linmt_b200 import decoder, synth
+
+def put(key, x): fake.fake_set(key.encode(), C.c_long(x))
+def get(key): return fake.fake_get(key.encode())
+def launches(part): return fake.fake_launches(part.encode())
+
+class refusing:
+    "From the n-th request for memory on, all are refused."
+    def __init__(self, n): self.n = n
+    def __enter__(self): put("refuse_after", self.n); put("refusing", 1)
+    def __exit__(self, *a): put("refusing", 0)
+
+def no_memory(call, n):
+    "Whether the call fails for memory when its n-th request and all after it are refused."
+    try:
+        with refusing(n): call()
+    except decoder.LinmtError as e:
+        assert "failed (4)" in str(e), e      # LINMT_ENOMEM
+        return True
+    return False
+
+D = synth.ModelDesc(2, 256, 3000, 300, 1)
+BLOB = synth.make_blob(D, 1)
+OPT = dict(beam=2, max_batch=4, max_src_len=16, max_steps=20)
+def make(**kw): return decoder.Decoder(D, [BLOB], **{**OPT, **kw})
+def some(n, seed=3): return synth.make_sentences(n, 2, 9, D.Vs, 1.1, seed, lambda s: s + 3)
+def words(n, m=2): return [np.arange(3, 3 + m)] * n
+""" % ROOT
+
+
+@pytest.fixture(scope="module")
+def child(cuda_lib, tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("cpp") / "fake_cudart.so")
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-O1", "-I/usr/local/cuda/include",
+                    os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), "-o", so], check=True)
+
+    def run(body, **env):
+        r = subprocess.run([sys.executable, "-c", HEAD + body + "\nassert get('violations') == 0, get('violations')\n"],
+                           env={**os.environ, "LD_PRELOAD": so, **env}, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+    return run
+
+
+def test_a_refused_request_is_not_reported_again(child):
+    """A call, or the creation of a handle, that fails for memory leaves nothing that the next one would fail by."""
+    child("""
+dec = make()
+dec.decode(some(2))
+assert no_memory(lambda: dec.decode(some(2), trace=True), 0)
+dec.decode(some(2))
+n = 0
+while no_memory(lambda: make().close(), n):
+    dec.decode(some(2))
+    n += 1
+assert n > 100
+dec.close()
+assert get("used") == 0, get("used")
+""")
