@@ -43,6 +43,22 @@ inline EncoderForm encoder_form(const EncoderModel& m, int n, int S) {
   return S >= 4 * kEncLag && (S + 6 * (L - 1)) * side < S * turn ? EncoderForm::kPipelined : other;
 }
 
+// Whether the layers of EncoderForm::kLayers run side by side all the same: the products of few sentences in CTAs of half an SM that
+// leave room for the other layers'.  Encoder and one scored word, ms, layer by layer / so: 4 x 1000 1 sentence of 16, 32 and 80 words
+// 0.59 / 0.61, 0.98 / 0.99, 1.98 / 1.51, 8 sentences 0.67 / 0.66, 1.01 / 0.86, 2.12 / 1.63, 32 0.79 / 0.76, 1.29 / 1.02, 2.85 / 2.02;
+// 5 x 512 1 0.56 / 0.53, 0.92 / 0.77, 2.00 / 1.46; of 8 words 2 to 8 % slower.  (Narrower models gain less in whole calls: 3 x 250
+// with 1 to 30 sentences of 40 words 2 to 3 % of a call, with 11 ragged ones it lost 2 %.)  Not where the batch shares the device with
+// others (`shared`), nor in one plane, which keeps its order of sums (see encoder_form).
+constexpr int kEncBesideWords = 20, kEncBesideHidden = 512;
+inline bool encoder_layers_beside(const EncoderModel& m, int S, bool shared) {
+  return m.split && m.members == 1 && m.layers > 1 && m.hp >= kEncBesideHidden && S >= kEncBesideWords && !shared;
+}
+
+// Up to here the encoder's products of a position are shaped like a step's, so that the next one's weights are under way (4 x 1000, 32
+// positions: one sentence 4.77 -> 4.73 ms a call, eight 14.34 -> 14.16; 64: 0.2 to 2 % slower).  One plane: as above.
+constexpr int kEncRoomSentences = 48;
+inline bool encoder_leaves_room(const EncoderModel& m, int n) { return m.split && n <= kEncRoomSentences; }
+
 // Sentences that the layers' panels of a handle are made for: those of the forms that its batches, of at most max_batch
 // sentences and max_words words, can take.
 inline int encoder_panel_sentences(const EncoderModel& m, int max_batch, int max_words) {

@@ -85,10 +85,12 @@ class Engine {
   int init(const linmt_model_desc& d, const float* const* blobs, int n_models, size_t blob_floats, const linmt_options& o);
   // An engine on the same device with the weights of `of`, which it must not outlive, and state, stream and workspaces of its own.
   int init_lane(const Engine& of);
-  // While one lives, the engine's device batch is one of several that run at once.
+  // While one lives, the engine's device batch is one of several that run at once, and its products leave room for theirs.  (Not in one
+  // plane: in other shapes the sums are in another order, which rounds a state to the other bf16 neighbour now and then.  A
+  // sentence has the bits there that it has in a batch by itself.)
   struct Several {
     Engine& g;
-    Several(Engine& e, bool on) : g(e) { g.several_ = on; }
+    Several(Engine& e, bool on) : g(e) { g.several_ = on && g.nt_ > 1; }
     ~Several() { g.several_ = false; }
   };
   // Device batches of a call that are worth running at once, of this engine's `rows` each.
@@ -197,7 +199,7 @@ class Engine {
   int l2_bytes_ = 0;
   bool rows_ = true;       // weight-streaming kernel for few rows (LINMT_TC_ROWS=0: test knob)
   bool ahead_ = true;      // recurrent products behind the step before (LINMT_AHEAD=0: test knob)
-  bool several_ = false;   // the device batch is one of several that run at once: products leave room for others
+  bool several_ = false;   // see Several
   bool lanes_ = true;      // device batches of a call at once (LINMT_LANES=0: test knob)
   bool persist_ = true;    // persistent kernel for the many-wave vocabulary GEMM (LINMT_TC_PERSIST=0: test knob)
   bool beside_ = false;      // the products issued leave room for the next one's CTAs (GemmLimits::beside)

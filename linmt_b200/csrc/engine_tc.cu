@@ -99,9 +99,10 @@ const CUtensorMap* Engine::maps(const tc::Planes& p, int col0, int rows, int K, 
 }
 
 // Products of a device batch that others run beside: up to 64 rows in CTAs of half an SM, as few of them as leave room for another
-// product's; beyond, in tiles for half of the SMs.  4 x 1000 / 30k, ms a call shaped for the whole
-// chip / so: 300 sentences greedily, 64 rows in a batch, 36.2 / 31.4; four batches, greedily 128 rows 25.3 / 21.5; beam 4, 128 rows 23.7 / 20.4, 256 rows
-// 28.6 / 27.1; beam 8, 512 rows 42.5 / 41.2; scoring 128 15.9 / 13.8, in bf16 8.6 / 8.1.  (Products of all positions fill the chip.)
+// product's; beyond, in tiles for half of the SMs.  4 x 1000 / 30k, ms a call shaped for the whole chip / so: 300 sentences greedily,
+// 64 rows in a batch, 36.2 / 31.4; four batches, greedily 128 rows 25.3 / 21.5; beam 4, 128 rows 23.7 / 20.4, 256 rows 28.6 / 27.1;
+// beam 8, 512 rows 42.5 / 41.2; scoring 128 15.9 / 13.8.  (Products of all positions fill the chip.  One plane: shaped for the whole
+// chip, see Engine::Several.)
 static constexpr int kSeveralFew = 64, kSeveralMost = 512;
 
 // C[M][N] = A[:, a_col0 : a_col0+K] . W[N][K]^T on the kernel and in the shape that plan_gemm chooses.
@@ -174,10 +175,6 @@ int Engine::build_xw_tables() {
   return LINMT_OK;
 }
 
-// Up to here the encoder's products of a position are shaped like a step's, so that the next one's weights are under way (4 x 1000, 32
-// positions: one sentence 4.77 -> 4.73 ms a call, eight 14.34 -> 14.16; 64: 0.2 to 2 % slower).
-static constexpr int kBesideSentences = 48;
-static constexpr int kEncFewWords = 20, kEncFewHidden = 512;     // (see run_encoder_pipeline_tc)
 static constexpr int kEncRing = 4;
 int Engine::encoder_streams() {
   if (!enc_streams_.empty()) return LINMT_OK;
@@ -199,14 +196,14 @@ int Engine::encoder_streams() {
 // the SMs (64 rows = one row tile), so the layers run as a wavefront: one stream per layer,
 // events for the cross-layer edges.  Besides the true dependencies, (l, p) waits for (l+1, p-2),
 // the last reader of the double-buffered input slot it overwrites.
-// Which of the three forms: encoder_form (encoder_form.h).
+// Which form, and in which shapes: encoder_form.h.
 int Engine::run_encoder_tc(int n, int Smax) {
-  stream_weights_ = false; beside_ = n <= kBesideSentences;
+  const EncoderModel model{L, Hp, n_models, nt_ > 1};
+  stream_weights_ = false; beside_ = encoder_leaves_room(model, n);
   if (enc_rows_)
-    switch (encoder_form(EncoderModel{L, Hp, n_models, nt_ > 1}, n, Smax)) {
+    switch (encoder_form(model, n, Smax)) {
       case EncoderForm::kLayers:
-        if (L > 1 && n_models == 1 && !several_ && Hp >= kEncFewHidden && Smax >= kEncFewWords) return run_encoder_pipeline_tc(n, Smax, true);
-        return run_encoder_layers_tc(n, Smax);
+        return encoder_layers_beside(model, Smax, several_) ? run_encoder_pipeline_tc(n, Smax, true) : run_encoder_layers_tc(n, Smax);
       case EncoderForm::kPipelined: return run_encoder_pipeline_tc(n, Smax, false);
       case EncoderForm::kWavefront: break;
     }
@@ -319,12 +316,7 @@ int Engine::encode_positions(int mi, int l, int n, int pos0, int np, float* pre,
 // shaped for their share of the SMs and run beside the others'.  Sources longer than the panels are taken in chunks: the
 // layers fall in line at the end of one, and the next starts from the states it ended with (4 x 1000, 500 words, two chunks,
 // against one position after another: 40 sentences 14.2 / 19.7 ms, 64 15.6 / 20.7).
-// few: the products of few sentences are those of the form above, in CTAs of half an SM that leave room for the other layers'.
-// Encoder and one scored word, ms, layer by layer / so: 4 x 1000 1 sentence of 16, 32 and 80 words 0.59 / 0.61, 0.98 / 0.99, 1.98 / 1.51,
-// 8 sentences 0.67 / 0.66, 1.01 / 0.86, 2.12 / 1.63, 32 0.79 / 0.76, 1.29 / 1.02, 2.85 / 2.02; in bf16 1 0.46 / 0.44, 0.73 / 0.64, 1.57 /
-// 1.26, 48 0.67 / 0.63, 1.13 / 0.88, 2.49 / 1.71; 5 x 512 1 0.56 / 0.53, 0.92 / 0.77, 2.00 / 1.46; of 8 words 2 to
-// 8 % slower.  (Narrower models gain less in whole calls: 3 x 250 with 1 to 30 sentences of 40 words 2 to 3 % of a call, with 11 ragged ones it
-// lost 2 %.)
+// few: the products of few sentences are those of the form above (encoder_layers_beside).
 int Engine::run_encoder_pipeline_tc(int n, int Smax, bool few) {
   if (int rc = encoder_streams()) return rc;
   hs_sent_ = 1; hs_pos_ = n;
@@ -583,7 +575,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc, in
 // while the attention, the softmax and the selection run on a few SMs; these products run beside them, those of the layers
 // between beside the attention, the rest beside the softmax.  What is left of the chain is half a product a layer, none of the
 // first (lstm_cell_kernel adds up its terms), and no state is gathered.  48 steps, ms a call without / with: 4 x 1000 / 30k 1 row
-// 3.92 / 3.81, 12 rows 4.74 / 4.02, 24 4.88 / 4.34, 60 5.57 / 5.47, in bf16 5 rows 3.41 / 3.22; 2 x 1000 12 rows 3.55 / 3.08, 48 3.69 / 3.46;
+// 3.92 / 3.81, 12 rows 4.74 / 4.02, 24 4.88 / 4.34, 60 5.57 / 5.47; 2 x 1000 12 rows 3.55 / 3.08, 48 3.69 / 3.46;
 // 3 x 250 / 5k 12 rows 2.50 / 2.36; beyond 48 rows their CTAs take longer than what they run beside (kRowsAhead; 32, kRowsAheadSelf, where there is no gather to save).
 //
 // They start without a wait for the kernel before them in the stream (RowsShape::ahead).  Before the attention that is where the
@@ -592,7 +584,7 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc, in
 // whether the launch was one of them.)  At their end they do wait, for those who wait for them.
 bool Engine::ahead_ok(int rows) const {
   tc::RowsShape sh;
-  return rows > 0 && rows <= rec_rows_ && tc::make_shape_ahead(rows, 4 * Hp, Hp, nt_, fmt_, n_sm_, 1, &sh);   // (more products: fewer slices each, see there)
+  return rows > 0 && rows <= rec_rows_ && tc::make_shape_ahead(rows, 4 * Hp, Hp, n_sm_, 1, &sh);   // (more products: fewer slices each, see there)
 }
 
 int Engine::recurrent_ahead(Ahead which, int mi, int t, int rows) {
@@ -613,7 +605,7 @@ int Engine::recurrent_ahead(Ahead which, int mi, int t, int rows) {
   }
   if (segs == 0) return LINMT_OK;
   tc::RowsShape sh;
-  if (!tc::make_shape_ahead(rows, 4 * Hp, Hp, nt_, fmt_, n_sm_, segs, &sh)) return fail(LINMT_EINVAL, "internal: no shape for the recurrent products");
+  if (!tc::make_shape_ahead(rows, 4 * Hp, Hp, n_sm_, segs, &sh)) return fail(LINMT_EINVAL, "internal: no shape for the recurrent products");
   sh.pdl = pdl_ ? 1 : 0;
   sh.ahead = pdl_ && got_late_ ? 1 : 0;
   tc::TmapSets<kSegs> tms{};
@@ -629,15 +621,9 @@ int Engine::recurrent_ahead(Ahead which, int mi, int t, int rows) {
   }
   const size_t stride = (size_t)rec_rows_ * 4 * Hp;
   const tc::TcEpiParts e{s.rec + slot * stride, (long long)stride, 4 * Hp};
-  auto launch = [&](auto nt, auto fmt) {
-    return tc::launch_gemm_tc_rows_of<decltype(nt)::value, decltype(fmt)::value, tc::TcEpiParts, kSegs, false>(tms, segs, rows, 4 * Hp, Hp, sh, e, d_tc_err_, stream, 0);
-  };
-  constexpr std::integral_constant<int, 0> zero{};
-  constexpr std::integral_constant<int, 1> one{};
-  constexpr std::integral_constant<int, 2> two{};
   if (int rc = kt(KC_LSTM)) return rc;
   if (kernel_timing) rec_flops_ += 2.0 * rows * 4.0 * H * (double)(segs * H);
-  CK(nt_ == 2 ? launch(two, one) : launch(one, zero));
+  CK((tc::launch_gemm_tc_rows_of<2, 1, tc::TcEpiParts, kSegs, false>(tms, segs, rows, 4 * Hp, Hp, sh, e, d_tc_err_, stream, 0)));
   LAUNCHED();
   return LINMT_OK;
 }

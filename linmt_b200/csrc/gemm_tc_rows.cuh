@@ -124,9 +124,9 @@ inline bool make_shape_rows(int rows, int N, int K, int nt, int fmt, int n_sm, b
 // flight (three products of 4096 x 1024 as launches of 256 CTAs each behind one another: 24 us more a step than these beside the
 // attention and the softmax, 12 rows).  Half an SM each, so that the next kernel's CTAs find room.
 constexpr int kRowsAhead = 60;
-inline bool make_shape_ahead(int rows, int N, int K, int nt, int fmt, int n_sm, int segs, RowsShape* out) {
+// (The f16 pair only: one plane keeps its order of sums.)
+inline bool make_shape_ahead(int rows, int N, int K, int n_sm, int segs, RowsShape* out) {
   if (rows < 1 || rows > kRowsAhead || K % 64 || K < 64 || N % 16) return false;
-  if (!(nt == 1 || (nt == 2 && fmt == 1))) return false;
   RowsShape s{};
   s.rp = (rows + 15) & ~15; s.units = (rows + 3) & ~3;
   s.tmem_cols = 256;
@@ -135,12 +135,12 @@ inline bool make_shape_ahead(int rows, int N, int K, int nt, int fmt, int n_sm, 
   while (s.splits > 1 && tiles * s.splits > places) s.splits >>= 1;
   for (; s.splits <= 8; s.splits *= 2) {
     if (s.splits > nkb) s.splits = nkb;
-    for (s.stacked = nt == 2 ? 1 : 0; s.stacked >= 0; --s.stacked) {     // (not stacked: more and shorter chains)
+    for (s.stacked = 1; s.stacked >= 0; --s.stacked) {     // (not stacked: more and shorter chains)
       s.acc_stride = s.stacked ? 2 * s.rp : (s.rp + 31) & ~31;
-      s.leads = nt == 1 ? 1 : (s.tmem_cols - s.rp) / s.acc_stride;
+      s.leads = (s.tmem_cols - s.rp) / s.acc_stride;
       if (s.leads > kRowsMaxLeads) s.leads = kRowsMaxLeads;
-      const bool chains = nt == 1 || (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
-      if (chains && rows_set_splits(&s, K, nt)) {
+      const bool chains = (nkb + s.splits - 1) / s.splits <= 3 * s.leads;   // a chain is at most three k-blocks
+      if (chains && rows_set_splits(&s, K, 2)) {
         *out = s;
         return true;
       }

@@ -54,3 +54,17 @@ def test_edges_of_the_rule(form):
                 assert form(4, 512, n, words) == plain
             elif words >= 100:
                 assert form(4, 512, n, words) == "pipelined"          # however long: in chunks
+
+
+def test_layers_side_by_side_and_room_for_the_next_product(tmp_path):
+    """Both change the order of sums: neither in one plane, whatever the sentences and words."""
+    out = str(tmp_path / "encoder_beside_main")
+    subprocess.run(["g++", "-std=c++17", "-I" + os.path.join(ROOT, "linmt_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "cpp", "encoder_beside_main.cpp"), "-o", out], check=True)
+    asked = [(layers, hp, members, split, n, words, shared) for layers in (1, 2, 5) for hp in (128, 448, 512, 1024) for members in (1, 2)
+             for split in (0, 1) for n in (1, 32, 48, 49, 64) for words in (1, 19, 20, 100) for shared in (0, 1)]
+    r = subprocess.run([out], input="".join("%d %d %d %d %d %d %d\n" % a for a in asked), capture_output=True, text=True, check=True)
+    for a, line in zip(asked, r.stdout.splitlines(), strict=True):
+        layers, hp, members, split, n, words, shared = a
+        beside = split and members == 1 and layers > 1 and hp >= 512 and words >= 20 and not shared
+        assert line == "%d %d" % (bool(beside), bool(split and n <= 48)), (a, line)

@@ -72,3 +72,15 @@ assert n > 100
 dec.close()
 assert get("used") == 0, get("used")
 """)
+
+
+def test_one_plane_makes_its_recurrent_products_in_place(child):
+    """Apart from the rest of a gate they are another order of sums, which bf16 states show."""
+    child("""
+for precision, ahead in (("fp32", True), ("bf16", False)):
+    before = launches("TcEpiParts")
+    dec = make(precision=precision)
+    dec.decode(some(2))
+    assert (launches("TcEpiParts") > before) == ahead, precision
+    dec.close()
+""")

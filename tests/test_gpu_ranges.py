@@ -589,3 +589,25 @@ def test_encoder_of_few_sentences_side_by_side(cuda_lib, precision, L, H, n, lon
         assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
     else:
         assert (np.abs(a[1] - b[1]) <= 2e-2).all(), float(np.abs(a[1] - b[1]).max())
+
+
+@pytest.mark.parametrize("L,H,n,beam,max_batch,longest", [
+    (3, 512, 1, 5, 8, 30), (2, 300, 40, 1, 40, 30),                            # one device batch
+    (3, 512, 9, 12, 3, 25), (2, 512, 70, 2, 32, 12), (2, 256, 200, 4, 96, 12)])    # several, of 36, 64 and 384 rows; scoring 3, 32 and 96
+def test_one_plane_has_one_order_of_sums(cuda_lib, L, H, n, beam, max_batch, longest):
+    """bf16 results do not go by what runs beside a step or beside a device batch: the same bits with and without."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(L, H, 2000, 300, 1)
+    blob = synth.make_blob(d, 40)
+    sents = synth.make_sentences(n, 2, longest, d.Vs, 1.1, 3, lambda s: s // 2 + 3)
+    rng = np.random.default_rng(n)
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 15, size=n)]
+    kw = dict(beam=beam, precision="bf16", cp_beta=0.0, max_batch=max_batch, max_src_len=32, max_steps=20)
+    dec = decoder.Decoder(d, [blob], **kw)
+    ref = _with_env({"LINMT_AHEAD": "0", "LINMT_LANES": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    a, b = dec.decode(sents), ref.decode(sents)
+    x, y = dec.score(sents, targets), ref.score(sents, targets)
+    dec.close(); ref.close()
+    for key in ("tok", "len", "score"):
+        assert a[key].tobytes() == b[key].tobytes(), key
+    assert x[1].tobytes() == y[1].tobytes()
