@@ -60,16 +60,19 @@ int Engine::dalloc(T** p, size_t count) {
   *p = static_cast<T*>(q);
   return LINMT_OK;
 }
-// Replaces *p by a fresh allocation of `count` elements and frees the old one.
+// Replaces *p by a fresh allocation of `count` elements and frees the old one; *cap says how many there are, also where that failed.
 template <class T>
-int Engine::regrow(T** p, size_t count) {
+int Engine::regrow(T** p, size_t count, size_t* cap) {
+  *cap = 0;
   if (*p) {
     auto it = std::find(allocs_.begin(), allocs_.end(), static_cast<void*>(*p));
     if (it != allocs_.end()) allocs_.erase(it);
     cudaFree(*p);
     *p = nullptr;
   }
-  return dalloc(p, count);
+  if (int rc = dalloc(p, count)) return rc;
+  *cap = count;
+  return LINMT_OK;
 }
 #define DA(p, n)                                  \
   do {                                            \
@@ -834,17 +837,13 @@ int Engine::decode_chunk(const HostJob& jb, const int* idx, int cn, const linmt_
   const size_t n_ids = (size_t)off[cn];
   // staging buffers grow with the longest input seen; the outgrown buffer is freed (the previous chunk's
   // work on it ended with the synchronisation in finish_timing)
-  if (n_ids > d_ids_cap_) {
-    if (int rc_ = regrow(&d_ids_, n_ids + 1024)) return rc_;
-    d_ids_cap_ = n_ids + 1024;
-  }
+  if (n_ids > d_ids_cap_)
+    if (int rc_ = regrow(&d_ids_, n_ids + 1024, &d_ids_cap_)) return rc_;
   const size_t need = (size_t)cn * nb, ml = (size_t)jb.max_len, per_align = ml * opt.max_src_len;
   // device results of the batch, one behind the other: len, score, tok, vit, align
   const size_t n_tok = need * ml, n_out = 2 * need + n_tok + (jb.out_vit ? n_tok : 0) + (jb.out_align ? need * per_align : 0);
-  if (n_out > out_cap_) {
-    if (int rc_ = regrow(&d_out_, n_out)) return rc_;
-    out_cap_ = n_out;
-  }
+  if (n_out > out_cap_)
+    if (int rc_ = regrow(&d_out_, n_out, &out_cap_)) return rc_;
   int32_t* d_len = d_out_;
   float* d_score = reinterpret_cast<float*>(d_out_ + need);
   int32_t* d_tok = d_out_ + 2 * need;
@@ -972,10 +971,8 @@ int Engine::score_chunk(const ScoreJob& jb, const int* idx, int cn) {
   }
   // ids | tokens read [steps][cn] | tokens asked for [rows], up in one copy; log-probabilities [rows] back
   const size_t n_up = n_ids + (size_t)steps * cn + rows;
-  if (n_up + rows > score_io_cap_) {
-    if (int rc = regrow(&score_io_, n_up + rows)) return rc;
-    score_io_cap_ = n_up + rows;
-  }
+  if (n_up + rows > score_io_cap_)
+    if (int rc = regrow(&score_io_, n_up + rows, &score_io_cap_)) return rc;
   if (int rc = reserve_host((n_up + rows) * 4)) return rc;
   int32_t *h_tok = h_stage_ + n_ids, *h_gold = h_tok + (size_t)steps * cn;
   for (int i = 0; i < cn; ++i)

@@ -237,7 +237,7 @@ class Engine {
   int device_memory(void** p, size_t bytes, const char* what);
   int host_memory(void** p, size_t bytes, const char* what);      // (pinned)
   template <class T> int dalloc(T** p, size_t count);
-  template <class T> int regrow(T** p, size_t count);
+  template <class T> int regrow(T** p, size_t count, size_t* cap);
 
   // batch metadata (device) and pinned staging
   int32_t *d_off_ = nullptr, *d_len_ = nullptr, *d_steps_ = nullptr, *d_orig_ = nullptr;

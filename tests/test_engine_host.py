@@ -84,3 +84,25 @@ for precision, ahead in (("fp32", True), ("bf16", False)):
     assert (launches("TcEpiParts") > before) == ahead, precision
     dec.close()
 """)
+
+
+def test_a_buffer_that_could_not_grow_is_not_taken_for_the_old_one(child):
+    """Calls that fail for memory at each request of theirs, and smaller ones after them: no copy goes to memory that is not there."""
+    child("""
+def all_refusals(dec, big, small):
+    "`big` fails at its first request, its second, ... until it goes through; `small` works after each."
+    small()
+    n = 0
+    while no_memory(big, n):
+        small()
+        n += 1
+    return n
+long = synth.make_sentences(4, 12, 16, D.Vs, 1.1, 3, lambda s: 20)
+dec = make(nbest=2)
+assert all_refusals(dec, lambda: dec.decode(long), lambda: dec.decode(some(1))) > 0
+dec.close()
+dec = make()
+assert all_refusals(dec, lambda: dec.score(long, words(4, 20)), lambda: dec.score(some(1), words(1))) > 0
+dec.close()
+assert get("used") == 0, get("used")
+""")
