@@ -34,7 +34,8 @@ int Engine::alloc_planes(tc::Planes& p, size_t rows, int ld) {
     const size_t bytes = rows * (size_t)ld * sizeof(__nv_bfloat16);
     if (int rc = device_memory(&q, bytes, "operand planes")) return rc;
     allocs_.push_back(q);
-    if (cudaMemset(q, 0, bytes) != cudaSuccess) return fail(LINMT_ECUDA, "cudaMemset failed (operand planes)");
+    // (on the engine's stream, whose kernels do not wait for the legacy one: scoring makes its panels in the middle of a call)
+    if (cudaMemsetAsync(q, 0, bytes, stream) != cudaSuccess) return fail(LINMT_ECUDA, "cudaMemsetAsync failed (operand planes)");
     p.p[t] = static_cast<__nv_bfloat16*>(q);
   }
   return LINMT_OK;

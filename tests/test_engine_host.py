@@ -106,3 +106,16 @@ assert all_refusals(dec, lambda: dec.score(long, words(4, 20)), lambda: dec.scor
 dec.close()
 assert get("used") == 0, get("used")
 """)
+
+
+def test_scoring_fills_its_panels_ahead_of_the_kernels_that_write_them(child):
+    """The engine's stream does not wait for a fill of the legacy stream: none of a call's is there."""
+    child("""
+for kw in (dict(), dict(precision="bf16"), dict(gemm_path="tensor3")):
+    dec = make(**kw)
+    put("races", 0)
+    dec.score(some(3), words(3))
+    dec.score(some(4), words(4, 12))       # (longer: the panels are made anew)
+    assert get("races") == 0, kw
+    dec.close()
+""")
