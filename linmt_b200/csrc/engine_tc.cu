@@ -713,6 +713,12 @@ int Engine::reserve_score(size_t rows) {
   }
   if (score_q_) return LINMT_OK;
   const size_t cap = std::max<size_t>(128, (((size_t)64 << 20) / Vp) & ~(size_t)127);
+  // (what a call that failed for memory here had got before that)
+  for (float* p : score_logits_) release(p);
+  for (void* p : {(void*)score_logits16_, (void*)score_combined_, (void*)score_idx_, (void*)score_candp_, (void*)score_eos_, (void*)score_stats_,
+                  (void*)score_pmax_, (void*)score_psum_})
+    release(p);
+  score_logits16_ = nullptr; score_combined_ = score_candp_ = score_eos_ = score_stats_ = score_pmax_ = score_psum_ = nullptr; score_idx_ = nullptr;
   score_logits_.assign(n_models, nullptr);
   if (logits16_) {
     if ((rc = dalloc_bytes(&score_logits16_, cap * Vp * 2))) return rc;

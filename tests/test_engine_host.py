@@ -119,3 +119,25 @@ for kw in (dict(), dict(precision="bf16"), dict(gemm_path="tensor3")):
     assert get("races") == 0, kw
     dec.close()
 """)
+
+
+def test_a_refused_scoring_workspace_is_not_kept_in_part(child):
+    """However often a call fails for memory, the handle holds what one that went through holds."""
+    child("""
+def held(refusals):
+    dec = make(precision=precision)
+    empty = get("used")
+    for n in refusals:
+        assert no_memory(lambda: dec.score(some(4), words(4, 12)), n), n
+    dec.score(some(4), words(4, 12))
+    mine = get("used") - empty
+    dec.close()
+    return mine
+for precision in ("fp32", "bf16"):
+    dec, n = make(precision=precision), 0
+    while no_memory(lambda: dec.score(some(4), words(4, 12)), n):
+        n += 1
+    dec.close()
+    assert n > 5
+    assert held(list(range(n)) * 3) == held([]), precision
+""")
