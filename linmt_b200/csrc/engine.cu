@@ -39,6 +39,7 @@ namespace linmt {
 // Device memory, for whatever an engine needs it.  A refusal is this call's result alone: the runtime would report it again to the
 // next check of a launch.
 int Engine::device_memory(void** p, size_t bytes, const char* what) {
+  asked_bytes_ += bytes;
   const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 1));
   if (e == cudaSuccess) return LINMT_OK;
   cudaGetLastError();
@@ -380,10 +381,13 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   const bool beside_softmax = logit_blocks(&some, &some, logit_blocks_ld(Vp), Vp, Hp, tc::BM, 32).sum != nullptr;
   if (ahead_ && beside_softmax && use_tc_ && rows_ && xw_table_ && nm == 1 && L > 1 && Hp >= 256 && fmt_ == 1) rec_rows_ = std::min(R, k > 1 ? tc::kRowsAhead : kRowsAheadSelf);
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);
+  size_t weight_bytes = 0;
   for (int i = 0; i < nm; ++i) {
     int rc = LINMT_OK;
+    const size_t before = asked_bytes_;
     if (of) models_[i] = of->models_[i];
     else if ((rc = pack_model(blobs[i], models_[i]))) return rc;
+    weight_bytes += asked_bytes_ - before;
     // fp16 storage of the logits needs them inside fp16's range with room to spare: |z| <= |w_row| |htilde| + |b| and
     // every component of htilde is below 1 in magnitude
     if (logits16_ && !(models_[i].voc_wnorm_max * std::sqrt((float)H) + models_[i].voc_babs_max < 3.0e4f)) logits16_ = false;
@@ -409,6 +413,7 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   if (o.print_info) {
     DA(d_rec_align_, (size_t)Tcap * R * rec_win); DA(d_rec_lo_, (size_t)Tcap * R); DA(d_rec_vit_, (size_t)Tcap * R);
   }
+  lane_bytes_ = asked_bytes_ - weight_bytes;
   if (use_tc_ && xw_table_ && !of) { const int rc_xw = build_xw_tables(); if (rc_xw) return rc_xw; }
   CK(cudaDeviceSynchronize());  // every weight upload has landed before the first decode
   return LINMT_OK;
@@ -1049,12 +1054,16 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
 // that has several run at once, a stream and a host thread each.  ms a batch of 64 sentences of 20 to 30 words with 1, 2, 3 at
 // once: 4 x 1000 / 30k 64 rows 6.4, 5.3, 5.3; 32 rows 5.3, 3.6, 3.3; 256 rows 9.3, 7.8, 7.9; 768 rows 15.2, 14.8, 15.0; in bf16 64 rows
 // 5.0, 3.9, 3.8; scoring 128 sentences in bf16 3.2, 2.3, 2.4; 3 x 250 / 5k 256 rows 4.4, 2.6, 2.0.  (Ensembles' members run side by side
-// already.  Where events time the kernels, one after another; and where the encoder states of a batch of the longest sources are
-// more than 2 GB, which every engine has for itself.)
+// already.  Where events time the kernels, one after another; and where an engine takes more than 3 GB beside the weights, which
+// are shared: states, panels and logits of a batch, records of alignments.)
 int Engine::lanes_for(int rows) const {
-  const size_t states = (size_t)B * opt.max_src_len * Hp * 12;
-  if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512 || states > ((size_t)2 << 30)) return 1;
+  if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512 || lane_bytes_ > ((size_t)3 << 30)) return 1;
   return rows <= 64 || !step_streams(false, rows) ? 3 : 2;
+}
+
+bool Engine::room_for_lane() const {
+  size_t free_bytes = 0, total = 0;
+  return cudaSetDevice(opt.device) == cudaSuccess && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && lane_bytes_ <= free_bytes / 4;
 }
 
 }  // namespace linmt
@@ -1080,7 +1089,7 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
       if (!lane && !no_more_lanes) {
         try {
           std::unique_ptr<Engine> l(new Engine());
-          if (l->init_lane(of) == LINMT_OK) { lane = l.get(); lanes.push_back(std::move(l)); }
+          if (of.room_for_lane() && l->init_lane(of) == LINMT_OK) { lane = l.get(); lanes.push_back(std::move(l)); }
         } catch (const std::bad_alloc&) { lane = nullptr; }
         if (!lane) { no_more_lanes = true; cudaGetLastError(); }
       }
@@ -1088,6 +1097,20 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
     }
   cudaSetDevice(eng.opt.device);
   return w;
+}
+
+int linmt_engine::with_lanes(const std::function<int()>& call) {
+  const int rc = call();
+  if (rc != LINMT_ENOMEM || lanes.empty()) return rc;
+  for (const auto& l : lanes) {      // (their counters stay the handle's)
+    eng.stats.kernel_launches += l->stats.kernel_launches;
+    eng.stats.pair_launches += l->stats.pair_launches;
+    eng.stats.decoder_row_steps += l->stats.decoder_row_steps;
+    eng.stats.sentence_steps += l->stats.sentence_steps;
+  }
+  lanes.clear();
+  no_more_lanes = true;
+  return call();
 }
 
 static std::string g_create_error;
@@ -1154,10 +1177,8 @@ const char* linmt_last_error(const linmt_engine* e) { return e ? e->eng.err.c_st
 
 int32_t linmt_beam(const linmt_engine* e) { return e ? e->eng.k : 0; }
 
-int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n, const int32_t* steps,
-                       int32_t max_len, int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit,
-                       float* out_align, const linmt_trace* trace) {
-  if (!e) return LINMT_EINVAL;
+static int decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n, const int32_t* steps, int32_t max_len, int32_t* out_tok,
+                        int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align, const linmt_trace* trace) {
   Engine& g0 = e->eng;
   const int B = g0.B;
   if ((g0.kernel_timing && e->n_engines() == 1) || trace || n <= B || !src_ids || !src_off || !steps || !out_tok || !out_len || !out_score)
@@ -1192,6 +1213,13 @@ int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* s
   return LINMT_OK;
 }
 
+int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n, const int32_t* steps,
+                       int32_t max_len, int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit,
+                       float* out_align, const linmt_trace* trace) {
+  if (!e) return LINMT_EINVAL;
+  return e->with_lanes([&] { return decode_batch(e, src_ids, src_off, n, steps, max_len, out_tok, out_len, out_score, out_vit, out_align, trace); });
+}
+
 int linmt_decode_batch_device(linmt_engine* e, const int32_t* d_src_ids, const int32_t* src_off_host, int32_t n,
                               const int32_t* steps_host, int32_t max_len, int32_t* d_out_tok, int32_t* d_out_len,
                               float* d_out_score) {
@@ -1202,9 +1230,8 @@ int linmt_decode_batch_device(linmt_engine* e, const int32_t* d_src_ids, const i
   return e->eng.finish_timing();
 }
 
-int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids,
-                      const int32_t* tgt_off, int32_t n, float* out_logprob, float* out_token_logp, int32_t max_tgt) {
-  if (!e || !src_ids || !src_off || !tgt_ids || !tgt_off || !out_logprob || n < 0) return LINMT_EINVAL;
+static int score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids, const int32_t* tgt_off, int32_t n,
+                       float* out_logprob, float* out_token_logp, int32_t max_tgt) {
   Engine& g = e->eng;
   if (g.n_models > 1 && g.opt.ensemble_mode != LINMT_ENS_PROB_MEAN) { g.err = "scoring supports single models and prob_mean ensembles"; return LINMT_EINVAL; }
   const int k = g.k;
@@ -1272,6 +1299,12 @@ int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* sr
     out_logprob[i] = sum;
   }
   return LINMT_OK;
+}
+
+int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids,
+                      const int32_t* tgt_off, int32_t n, float* out_logprob, float* out_token_logp, int32_t max_tgt) {
+  if (!e || !src_ids || !src_off || !tgt_ids || !tgt_off || !out_logprob || n < 0) return LINMT_EINVAL;
+  return e->with_lanes([&] { return score_batch(e, src_ids, src_off, tgt_ids, tgt_off, n, out_logprob, out_token_logp, max_tgt); });
 }
 
 int linmt_get_stats(const linmt_engine* e, linmt_stats* out) {

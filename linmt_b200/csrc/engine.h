@@ -95,6 +95,9 @@ class Engine {
   };
   // Device batches of a call that are worth running at once, of this engine's `rows` each.
   int lanes_for(int rows) const;
+  // Whether the device can spare what a lane takes: a quarter of its free memory at most, for calls grow an engine's buffers and others
+  // use the device as well.
+  bool room_for_lane() const;
   int decode_core(const int32_t* d_ids, const int32_t* off_host, int n, const int32_t* steps_host, int max_len,
                   int32_t* d_out_tok, int32_t* d_out_len, float* d_out_score, int32_t* d_out_vit, float* d_out_align,
                   const linmt_trace* trace_dev, int trace_Tm);
@@ -234,6 +237,7 @@ class Engine {
   std::vector<DevModel> models_;
   std::vector<DevState> states_;
   std::vector<void*> allocs_;
+  size_t asked_bytes_ = 0, lane_bytes_ = 0;     // device memory requested so far; what the handle's creation took beside the weights
   int device_memory(void** p, size_t bytes, const char* what);
   int host_memory(void** p, size_t bytes, const char* what);      // (pinned)
   template <class T> int dalloc(T** p, size_t count);
@@ -312,9 +316,12 @@ struct linmt_engine {
   linmt::Engine eng;
   std::vector<std::unique_ptr<linmt::Engine>> replicas;
   // Further engines on the devices above, with their weights: a call of several device batches runs some at once (Engine::lanes_for).
-  // Made when such a call first wants them, and kept; where memory does not suffice a call does with what there is.
+  // Made when such a call first wants them, and kept, unless memory is short (with_lanes).
   std::vector<std::unique_ptr<linmt::Engine>> lanes;
   bool no_more_lanes = false;
+  // Runs `call`, which may use the lanes; where it fails for memory, which they hold some of or were refused, it runs once more from its
+  // start without them, as every later one does.
+  int with_lanes(const std::function<int()>& call);
   // the engines that share `items` device batches of `rows` rows, on the first device alone or on all
   std::vector<linmt::Engine*> workers(size_t items, int rows, bool first_device);
   int n_engines() const { return 1 + (int)replicas.size(); }

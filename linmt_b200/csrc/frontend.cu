@@ -475,8 +475,9 @@ const char* linmt_translate(linmt_engine* h, const char* sentence) {
   std::vector<float> score(nb), align;
   const bool want_align = e.opt.print_info && e.print_align_scores;
   if (want_align) align.resize((size_t)nb * max_len * e.opt.max_src_len);
-  int rc = e.decode_host(ids.data(), off, 1, &steps, max_len, tok.data(), len.data(), score.data(), vit.data(),
-                         want_align ? align.data() : nullptr, nullptr);
+  int rc = h->with_lanes([&] {
+    return e.decode_host(ids.data(), off, 1, &steps, max_len, tok.data(), len.data(), score.data(), vit.data(), want_align ? align.data() : nullptr, nullptr);
+  });
   if (rc != LINMT_OK) return e.result_buf.c_str();
   e.result_buf = format_result(e, S, nb, max_len, tok.data(), len.data(), score.data(), vit.data(),
                                want_align ? align.data() : nullptr, e.opt.max_src_len);
@@ -530,7 +531,7 @@ int linmt_decode_file(linmt_engine* h, const char* in_path, const char* out_path
   std::vector<int> batch_ids;
   for (size_t b0 = 0; b0 < order.size(); b0 += B) batch_ids.push_back((int)(b0 / B));
   const bool together = batch_ids.size() > 1 && e.lanes_for(B * e.k) > 1;
-  const int rc_all = run_on_engines(h, h->workers(batch_ids.size(), B * e.k, false), batch_ids, [&](Engine& g, int bi) -> int {
+  auto one_batch = [&](Engine& g, int bi) -> int {
     const Engine::Several several(g, together);
     const size_t b0 = (size_t)bi * B;
     const int n = (int)std::min<size_t>(B, order.size() - b0);
@@ -566,7 +567,8 @@ int linmt_decode_file(linmt_engine* h, const char* in_path, const char* out_path
       results[order[b0 + i]] = out;
     }
     return LINMT_OK;
-  });
+  };
+  const int rc_all = h->with_lanes([&] { return run_on_engines(h, h->workers(batch_ids.size(), B * e.k, false), batch_ids, one_batch); });
   if (rc_all != LINMT_OK) return rc_all;
   std::ofstream outf(out_path);
   if (!outf) { e.err = std::string("can not open ") + out_path; return LINMT_EIO; }

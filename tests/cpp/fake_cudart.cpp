@@ -22,9 +22,11 @@ thread_local Call call;
 
 long& v(const char* key) { return value[key]; }
 
-// Whether a request for memory is refused: beyond `limit` bytes in all, or when the countdown `refuse_after` has run out.
+// Whether a request for memory is refused: beyond `limit` bytes in all, as the `refuse_one`-th from now on, or when the countdown
+// `refuse_after` has run out.
 bool refused(size_t bytes) {
   if (v("limit") && v("used") + (long)bytes > v("limit")) return true;
+  if (v("refuse_one") && --v("refuse_one") == 0) return true;
   return v("refusing") && v("refuse_after")-- <= 0;
 }
 bool inside(const void* p, size_t bytes) {

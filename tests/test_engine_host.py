@@ -141,3 +141,54 @@ for precision in ("fp32", "bf16"):
     assert n > 5
     assert held(list(range(n)) * 3) == held([]), precision
 """)
+
+
+LANES = """
+def calls(dec):
+    dec.decode(some(18)); dec.score(some(18), words(18, 12)); dec.decode(long); dec.decode(some(2), trace=True)
+long = synth.make_sentences(18, 12, 16, D.Vs, 1.1, 3, lambda s: 20)
+os.environ["LINMT_LANES"] = "0"
+dec = make(); created = get("used"); calls(dec); alone = get("used")
+per_call = dec.stats()["sentence_steps"]
+dec.close()
+del os.environ["LINMT_LANES"]
+"""
+
+
+def test_a_call_goes_through_in_the_memory_that_one_engine_needs(child):
+    """Whatever the device has beside that, and whenever the memory gets short: engines beside the handle's own are made of what is
+    to spare, and given up where it does not suffice."""
+    child(LANES + """
+kept = 0
+for early in (False, True):
+    for extra in range(0, 1200 << 20, 48 << 20):
+        dec = make()
+        if early:
+            dec.decode(some(18))
+            assert get("used") > created + (100 << 20), "no lanes made"
+        put("limit", max(get("used"), alone) + extra)
+        calls(dec)
+        calls(dec)
+        kept += get("used") > alone
+        put("limit", 0)
+        dec.close()
+        assert get("used") == 0
+assert 0 < kept < 50, kept
+""")
+
+
+def test_no_single_refusal_fails_a_call_of_several_batches(child):
+    child(LANES + """
+n, refused = 1, True
+while refused:
+    dec = make()
+    put("refuse_one", n)
+    calls(dec)
+    refused = get("refuse_one") == 0
+    put("refuse_one", 0)
+    assert dec.stats()["sentence_steps"] >= per_call
+    calls(dec)
+    dec.close()
+    n += 1
+assert get("used") == 0 and n > 100, n
+""")
