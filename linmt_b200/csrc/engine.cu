@@ -24,17 +24,15 @@
 
 namespace linmt {
 
-#define CK(call)                                                                              \
-  do {                                                                                        \
-    cudaError_t e_ = (call);                                                                  \
-    if (e_ != cudaSuccess) {                                                                  \
-      char b_[512];                                                                           \
-      snprintf(b_, sizeof b_, "CUDA error %s at %s:%d: %s", cudaGetErrorName(e_), __FILE__, __LINE__, cudaGetErrorString(e_)); \
-      return fail(LINMT_ECUDA, b_);                                                           \
-    }                                                                                         \
-  } while (0)
-
 #define LAUNCHED() (++stats.kernel_launches)
+
+int Engine::cuda_failed(cudaError_t e, const char* file, int line) {
+  char text[512];
+  snprintf(text, sizeof text, "CUDA error %s at %s:%d: %s", cudaGetErrorName(e), file, line, cudaGetErrorString(e));
+  if (e != cudaErrorMemoryAllocation) return fail(LINMT_ECUDA, text);
+  cudaGetLastError();       // (as device_memory)
+  return fail(LINMT_ENOMEM, text);
+}
 
 // Device memory, for whatever an engine needs it.  A refusal is this call's result alone: the runtime would report it again to the
 // next check of a launch.
@@ -90,11 +88,11 @@ Engine::~Engine() {
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   for (auto e : kt_ev_) cudaEventDestroy(e);
-  for (auto& v : enc_events_) for (auto e : v) cudaEventDestroy(e);
+  for (auto& v : enc_events_) for (auto e : v) if (e) cudaEventDestroy(e);
   if (enc_start_ev_) cudaEventDestroy(enc_start_ev_);
   for (auto e : mem_events_) if (e) cudaEventDestroy(e);
   for (auto st : mem_streams_) if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
-  for (auto st : enc_streams_) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
+  for (auto st : enc_streams_) if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -676,11 +674,11 @@ int Engine::each_member(int rows, const std::function<int(int)>& work) {
       if (int rc = work(mi)) return rc;
     return LINMT_OK;
   }
-  if (mem_streams_.empty()) {
+  if (mem_events_.empty() || !mem_events_.back()) {      // (the last to be made)
     mem_streams_.resize(n_models);
     mem_events_.resize(n_models + 1);
-    for (auto& st : mem_streams_) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    for (auto& ev : mem_events_) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    for (auto& st : mem_streams_) if (!st) CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    for (auto& ev : mem_events_) if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
   const cudaStream_t main_stream = stream;
   CK(cudaEventRecord(mem_events_[n_models], main_stream));

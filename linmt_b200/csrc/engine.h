@@ -73,6 +73,13 @@ struct DevState {
   std::vector<float*> enc_h[2], enc_c[2];            // [L] x [B][Hp], double buffered
 };
 
+// A call of the CUDA runtime in an Engine's method, which returns where it fails.
+#define CK(call)                                                             \
+  do {                                                                       \
+    const cudaError_t e_ = (call);                                           \
+    if (e_ != cudaSuccess) return cuda_failed(e_, __FILE__, __LINE__);       \
+  } while (0)
+
 // Kernel classes of a decoder step, in launch order (linmt_kernel_times reports one entry per class).
 enum KernelClass { KC_GATHER = 0, KC_LSTM, KC_PROJ, KC_ATTENTION, KC_ATTOUT, KC_VOCAB, KC_COMBINE, KC_SOFTMAX, KC_SELECT, KC_COUNT, KC_END = KC_COUNT };
 
@@ -139,6 +146,7 @@ class Engine {
  private:
   int init_state(const Engine* of, const float* const* blobs);
   int fail(int code, const std::string& msg) { err = msg; return code; }
+  int cuda_failed(cudaError_t e, const char* file, int line);
   // role of member mi in the alignment record of a step: 0 = single model, 1 / 2 / 3 = first / middle / last member
   int ens_member_code(int mi) const { return n_models == 1 ? 0 : (mi == 0 ? 1 : (mi == n_models - 1 ? 3 : 2)); }
   int pack_model(const float* blob, DevModel& m);

@@ -14,15 +14,6 @@
 
 namespace linmt {
 
-#define CK(call)                                                                              \
-  do {                                                                                        \
-    cudaError_t e_ = (call);                                                                  \
-    if (e_ != cudaSuccess) {                                                                  \
-      char b_[512];                                                                           \
-      snprintf(b_, sizeof b_, "CUDA error %s at %s:%d: %s", cudaGetErrorName(e_), __FILE__, __LINE__, cudaGetErrorString(e_)); \
-      return fail(LINMT_ECUDA, b_);                                                           \
-    }                                                                                         \
-  } while (0)
 #define LAUNCHED() (++stats.kernel_launches)
 
 int Engine::alloc_planes(tc::Planes& p, size_t rows, int ld) {
@@ -178,12 +169,13 @@ int Engine::build_xw_tables() {
 
 static constexpr int kEncRing = 4;
 int Engine::encoder_streams() {
-  if (!enc_streams_.empty()) return LINMT_OK;
+  if (enc_start_ev_) return LINMT_OK;      // (the last to be made)
   enc_streams_.resize(L);
-  enc_events_.assign(L, std::vector<cudaEvent_t>(kEncRing));
+  enc_events_.resize(L, std::vector<cudaEvent_t>(kEncRing));
   for (int l = 0; l < L; ++l) {
-    CK(cudaStreamCreateWithFlags(&enc_streams_[l], cudaStreamNonBlocking));
-    for (int r = 0; r < kEncRing; ++r) CK(cudaEventCreateWithFlags(&enc_events_[l][r], cudaEventDisableTiming));
+    if (!enc_streams_[l]) CK(cudaStreamCreateWithFlags(&enc_streams_[l], cudaStreamNonBlocking));
+    for (int r = 0; r < kEncRing; ++r)
+      if (!enc_events_[l][r]) CK(cudaEventCreateWithFlags(&enc_events_[l][r], cudaEventDisableTiming));
   }
   CK(cudaEventCreateWithFlags(&enc_start_ev_, cudaEventDisableTiming));
   return LINMT_OK;

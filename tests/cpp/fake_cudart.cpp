@@ -47,8 +47,9 @@ cudaError_t copy(void* d, const void* s, size_t bytes, cudaMemcpyKind kind) {
   if (ok_d && ok_s && bytes) std::memmove(d, s, bytes);
   return cudaSuccess;
 }
-cudaError_t launch(const void* f) {
+cudaError_t launch(const void* f, cudaStream_t s) {
   std::lock_guard<std::recursive_mutex> lock(mu);
+  if (!s) ++v("legacy");
   ++launched[names[f]];
   if (v("unordered")) ++v("races");     // a fill of the legacy stream, which this launch does not wait for, is under way
   return cudaSuccess;
@@ -60,6 +61,8 @@ CUresult encode_tiled(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void* p, co
 }
 template <class T>
 cudaError_t fresh(T* out) {
+  std::lock_guard<std::recursive_mutex> lock(mu);
+  if (refused(0)) return pending = cudaErrorMemoryAllocation;
   *out = reinterpret_cast<T>(std::malloc(1));
   return cudaSuccess;
 }
@@ -158,8 +161,8 @@ cudaError_t cudaGetDriverEntryPoint(const char*, void** f, unsigned long long, c
   if (r) *r = cudaDriverEntryPointSuccess;
   return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t, cudaStream_t) { return launch(f); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void* f, void**) { return launch(f); }
+cudaError_t cudaLaunchKernel(const void* f, dim3, dim3, void**, size_t, cudaStream_t s) { return launch(f, s); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) { return launch(f, c->stream); }
 
 void** __cudaRegisterFatBinary(void*) { static void* handle; return &handle; }
 void __cudaRegisterFatBinaryEnd(void**) {}

@@ -192,3 +192,22 @@ while refused:
     n += 1
 assert get("used") == 0 and n > 100, n
 """)
+
+
+def test_streams_that_could_not_be_made_are_not_used(child):
+    """The encoder's streams and those of ensemble members are made in a call: each refusal fails that one alone, for memory, and no
+    kernel runs on the legacy stream."""
+    child("""
+def ensemble(**kw): return decoder.Decoder(D, [BLOB, synth.make_blob(D, 2)], **{**OPT, **kw})
+for new in (lambda: make(gemm_path="tensor3"), ensemble, lambda: ensemble(gemm_path="tensor3")):
+    n, more = 0, True
+    while more:
+        dec = new()
+        more = no_memory(lambda: dec.decode(some(2)), n)
+        put("legacy", 0)
+        dec.decode(some(2))
+        assert get("legacy") == 0, n
+        dec.close()
+        n += 1
+    assert n > 4
+""")
