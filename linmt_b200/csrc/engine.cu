@@ -1014,8 +1014,18 @@ int Engine::score_chunk(const ScoreJob& jb, const int* idx, int cn) {
   return LINMT_OK;
 }
 
-int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& job) {
+int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& work) {
   const int ne = (int)workers.size();
+  // (no exception leaves a thread, nor this function while its threads run)
+  auto job = [&](Engine& g, int item) -> int {
+    try {
+      return work(g, item);
+    } catch (const std::exception& e) {
+      if (g.stream) cudaStreamSynchronize(g.stream);      // (copies from staging that the next batch reuses may be under way)
+      try { g.err = std::string("out of host memory: ") + e.what(); } catch (...) {}
+      return LINMT_ENOMEM;
+    }
+  };
   if (ne == 1 || order.size() <= 1) {
     for (int item : order)
       if (int rc = job(h->eng, item)) return rc;

@@ -338,7 +338,7 @@ struct linmt_engine {
 
 namespace linmt {
 std::vector<int> batch_order(const int32_t* src_off, int n, const int32_t* steps);
-// Runs job(engine, item) for item = order[0], order[1], ... on engines of a handle (linmt_engine::workers), one host thread per
+// Runs work(engine, item) for item = order[0], order[1], ... on engines of a handle (linmt_engine::workers), one host thread per
 // engine, each taking the next item when it is free.  Returns the first error; engine 0's `err` names it.
-int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& job);
+int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& work);
 }  // namespace linmt

@@ -8,6 +8,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 
 namespace {
@@ -129,7 +130,13 @@ cudaError_t cudaMemset2DAsync(void* p, size_t pitch, int c, size_t width, size_t
   return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind k) { fake_set("unordered", 0); return copy(d, s, n, k); }
-cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) { return copy(d, s, n, k); }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+  {
+    std::lock_guard<std::recursive_mutex> lock(mu);
+    if (v("throw_at") && --v("throw_at") == 0) throw std::bad_alloc();      // (stands for the engine's own host memory)
+  }
+  return copy(d, s, n, k);
+}
 cudaError_t cudaMemcpy2D(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind k) {
   for (size_t y = 0; y < h; ++y) copy(static_cast<char*>(d) + y * dp, static_cast<const char*>(s) + y * sp, w, k);
   return cudaSuccess;

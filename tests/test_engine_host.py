@@ -211,3 +211,21 @@ for new in (lambda: make(gemm_path="tensor3"), ensemble, lambda: ensemble(gemm_p
         n += 1
     assert n > 4
 """)
+
+
+def test_host_memory_that_runs_out_in_one_of_several_batches(child):
+    """Thrown in whichever engine's thread: the call goes through without the further engines; of a handle that has none it fails."""
+    child(LANES + """
+for n in range(1, 16):
+    dec = make()
+    put("throw_at", n)
+    dec.decode(some(18)); dec.decode(some(18))
+    assert get("throw_at") == 0, n
+    dec.close()
+os.environ["LINMT_LANES"] = "0"
+dec = make()
+put("throw_at", 3)
+assert no_memory(lambda: dec.decode(some(18)), 10**9)
+dec.decode(some(18))
+dec.close()
+""")
