@@ -1200,7 +1200,7 @@ static int decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* 
   std::vector<int> order(nchunks);
   std::iota(order.begin(), order.end(), 0);
   const std::vector<Engine*> workers = e->workers(nchunks, B * g0.k, false);
-  const bool together = nchunks > 1 && g0.lanes_for(B * g0.k) > 1;
+  const bool together = (int)workers.size() > e->n_engines();
   std::vector<float> ms_per_engine(workers.size(), 0.f);
   std::mutex stat_mutex;
   int rc = linmt::run_on_engines(e, workers, order, [&](Engine& g, int c) -> int {
@@ -1260,7 +1260,7 @@ static int score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* s
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(sents.begin(), sents.end(), [&](int a, int b) { return steps[a] > steps[b]; });
     const std::vector<Engine*> workers = e->workers(nchunks, B, true);
-    const bool together = nchunks > 1 && g.lanes_for(B) > 1;
+    const bool together = workers.size() > 1;
     std::vector<float> ms(workers.size(), 0.f);
     const int rc = linmt::run_on_engines(e, workers, order, [&](Engine& w, int c) -> int {
       const Engine::Several several(w, together);

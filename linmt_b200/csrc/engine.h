@@ -92,7 +92,8 @@ class Engine {
   int init(const linmt_model_desc& d, const float* const* blobs, int n_models, size_t blob_floats, const linmt_options& o);
   // An engine on the same device with the weights of `of`, which it must not outlive, and state, stream and workspaces of its own.
   int init_lane(const Engine& of);
-  // While one lives, the engine's device batch is one of several that run at once, and its products leave room for theirs.  (Not in one
+  // While one lives, the engine's device batch is one of a call's that run at once on a device, and its products leave room for others.
+  // That goes by the engines that the call has, not by what runs at the moment: a sentence's last bits do not depend on time.  (Not in one
   // plane: in other shapes the sums are in another order, which rounds a state to the other bf16 neighbour now and then.  A
   // sentence has the bits there that it has in a batch by itself.)
   struct Several {

@@ -530,7 +530,7 @@ int linmt_decode_file(linmt_engine* h, const char* in_path, const char* out_path
   // free (the batches are in descending step count, so the long ones go first)
   std::vector<int> batch_ids;
   for (size_t b0 = 0; b0 < order.size(); b0 += B) batch_ids.push_back((int)(b0 / B));
-  const bool together = batch_ids.size() > 1 && e.lanes_for(B * e.k) > 1;
+  bool together = false;
   auto one_batch = [&](Engine& g, int bi) -> int {
     const Engine::Several several(g, together);
     const size_t b0 = (size_t)bi * B;
@@ -568,7 +568,11 @@ int linmt_decode_file(linmt_engine* h, const char* in_path, const char* out_path
     }
     return LINMT_OK;
   };
-  const int rc_all = h->with_lanes([&] { return run_on_engines(h, h->workers(batch_ids.size(), B * e.k, false), batch_ids, one_batch); });
+  const int rc_all = h->with_lanes([&] {
+    const std::vector<Engine*> workers = h->workers(batch_ids.size(), B * e.k, false);
+    together = (int)workers.size() > h->n_engines();
+    return run_on_engines(h, workers, batch_ids, one_batch);
+  });
   if (rc_all != LINMT_OK) return rc_all;
   std::ofstream outf(out_path);
   if (!outf) { e.err = std::string("can not open ") + out_path; return LINMT_EIO; }

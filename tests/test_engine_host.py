@@ -229,3 +229,36 @@ assert no_memory(lambda: dec.decode(some(18)), 10**9)
 dec.decode(some(18))
 dec.close()
 """)
+
+
+def test_a_batch_that_has_its_device_to_itself_runs_as_one_by_itself(child):
+    """On several devices with a batch each, and where there is no memory for further engines: the launches of a handle without them.
+    (Batches that share a device encode layer by layer, a batch by itself with the layers side by side.)"""
+    child("""
+D5 = synth.ModelDesc(3, 512, 3000, 300, 1)
+B5 = synth.make_blob(D5, 1)
+def counted(n, limited=False, **kw):
+    dec = decoder.Decoder(D5, [B5], beam=2, max_batch=4, max_src_len=40, max_steps=20, **kw)
+    s = synth.make_sentences(n, 24, 30, D5.Vs, 1.1, 3, lambda s: 9)
+    dec.decode(synth.make_sentences(1, 24, 30, D5.Vs, 1.1, 3, lambda s: 9))
+    if limited: put("limit", get("used") + (200 << 20))
+    start = dec.stats()["kernel_launches"]
+    dec.decode(s)
+    one = dec.stats()["kernel_launches"] - start
+    if not kw: dec.score(s, words(n, 5))
+    put("limit", 0)
+    both = dec.stats()["kernel_launches"] - start
+    dec.close()
+    return one, both
+def alone(*a, **kw):
+    os.environ["LINMT_LANES"] = "0"
+    c = counted(*a, **kw)
+    del os.environ["LINMT_LANES"]
+    return c
+assert counted(8) != alone(8)                   # (one device: they share it)
+assert counted(8, devices=[0, 1]) == alone(8, devices=[0, 1])
+assert counted(12, devices=[0, 1, 2, 3]) == alone(12, devices=[0, 1, 2, 3])
+put("limit", 0)
+got, want = counted(8, limited=True), alone(8, limited=True)
+assert got == want, (got, want)
+""")
