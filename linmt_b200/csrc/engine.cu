@@ -37,7 +37,13 @@ int Engine::cuda_failed(cudaError_t e, const char* file, int line) {
 // Device memory, for whatever an engine needs it.  A refusal is this call's result alone: the runtime would report it again to the
 // next check of a launch.
 int Engine::device_memory(void** p, size_t bytes, const char* what) {
-  asked_bytes_ += bytes;
+  const size_t units = (std::max<size_t>(bytes, 1) + kMemoryUnit - 1) / kMemoryUnit * kMemoryUnit;
+  asked_bytes_ += units;
+  if (arena_used_ + units <= arena_bytes_) {
+    *p = arena_ + arena_used_;
+    arena_used_ += units;
+    return LINMT_OK;
+  }
   const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 1));
   if (e == cudaSuccess) return LINMT_OK;
   cudaGetLastError();
@@ -81,7 +87,9 @@ int Engine::regrow(T** p, size_t count, size_t* cap) {
 
 Engine::~Engine() {
   if (stream) { cudaSetDevice(opt.device); cudaStreamSynchronize(stream); }
-  for (void* p : allocs_) cudaFree(p);
+  for (void* p : allocs_)
+    if (!arena_ || static_cast<char*>(p) < arena_ || static_cast<char*>(p) >= arena_ + arena_used_) cudaFree(p);
+  if (arena_) cudaFree(arena_);
   for (void* p : trace_allocs_) cudaFree(p);
   if (h_meta_) cudaFreeHost(h_meta_);
   if (h_stage_) cudaFreeHost(h_stage_);
@@ -266,7 +274,7 @@ int Engine::alloc_state(DevState& s) {
   } else {
     DA(s.hs, (size_t)B * opt.max_src_len * Hp);
     // rows past a sentence's end are never written, but read as GEMM operand rows by the fold
-    CK(cudaMemset(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp));
+    CK(cudaMemsetAsync(s.hs, 0, sizeof(float) * (size_t)B * opt.max_src_len * Hp, stream));
   }
   if (att_fold_) DA(s.hs_wc1, (size_t)B * opt.max_src_len * Hp);
   if (rec_rows_) DA(s.rec, (size_t)(L + 1) * rec_rows_ * 4 * Hp);
@@ -323,13 +331,26 @@ int Engine::init(const linmt_model_desc& d, const float* const* blobs, int nm, s
   return init_state(nullptr, blobs);
 }
 
+int Engine::ready() {
+  if (!lane_of_) return broken_ ? LINMT_ENOMEM : LINMT_OK;
+  const Engine& of = *lane_of_;
+  lane_of_ = nullptr;
+  broken_ = init_lane(of) != LINMT_OK;       // (and stays what it was, broken, where that throws)
+  return broken_ ? LINMT_ENOMEM : LINMT_OK;
+}
+
 int Engine::init_lane(const Engine& of) {
-  desc = of.desc; opt = of.opt; n_models = of.n_models;
+  desc = of.desc; n_models = of.n_models;
   // (what the environment and the weights decided when the handle was made)
   use_tc_ = of.use_tc_; xw_table_ = of.xw_table_; pmax_on_ = of.pmax_on_; att_merge_ = of.att_merge_; att_fold_ = of.att_fold_;
   persist_ = of.persist_; rows_ = of.rows_; pair_ = of.pair_; pdl_ = of.pdl_; ahead_ = of.ahead_; fmt_ = of.fmt_; nt_ = of.nt_;
   nt_vocab_ = of.nt_vocab_; refine_ = of.refine_; logits16_ = of.logits16_;
-  return init_state(&of, nullptr);
+  CK(cudaSetDevice(opt.device));
+  if (int rc = device_memory(reinterpret_cast<void**>(&arena_), of.lane_bytes_, "engine")) return rc;
+  arena_bytes_ = of.lane_bytes_;
+  const int rc = init_state(&of, nullptr);
+  arena_bytes_ = arena_used_;      // (buffers of calls come and go by themselves)
+  return rc;
 }
 
 // What is left of a handle's creation once its options are settled: sizes, device buffers, and the weights, packed from `blobs` or
@@ -357,11 +378,11 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   CK(cudaEventCreate(&ev0_)); CK(cudaEventCreate(&ev1_));
   CK(cudaDeviceGetAttribute(&n_sm_, cudaDevAttrMultiProcessorCount, o.device));
   DA(d_tc_err_, 1);
-  CK(cudaMemset(d_tc_err_, 0, sizeof(int)));
+  CK(cudaMemsetAsync(d_tc_err_, 0, sizeof(int), stream));
   if (use_tc_) {
     DA(d_splitk_ws_, kSplitKWsFloats);
     DA(d_splitk_counters_, kSplitKMaxTiles);
-    CK(cudaMemset(d_splitk_counters_, 0, sizeof(int) * kSplitKMaxTiles));
+    CK(cudaMemsetAsync(d_splitk_counters_, 0, sizeof(int) * kSplitKMaxTiles, stream));
     CK(cudaDeviceGetAttribute(&l2_bytes_, cudaDevAttrL2CacheSize, o.device));
     if (pair_ && !pairs_available()) pair_ = false;   // (a device that cannot co-schedule two such CTAs keeps the one-tile kernels)
   }
@@ -394,14 +415,14 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   }
   // what one copy brings in and what one memset clears at the start of a decode lies together
   DA(d_off_, 4 * (B + 1)); d_len_ = d_off_ + (B + 1); d_steps_ = d_off_ + 2 * (B + 1); d_orig_ = d_off_ + 3 * (B + 1);
-  CK(cudaMemset(d_off_, 0, sizeof(int32_t) * 4 * (B + 1)));   // (the attention's prefetch may go by a length before the first copy)
+  CK(cudaMemsetAsync(d_off_, 0, sizeof(int32_t) * 4 * (B + 1), stream));   // (the attention's prefetch may go by a length before the first copy)
   if (int rc = host_memory(reinterpret_cast<void**>(&h_meta_), sizeof(int32_t) * (4 * (B + 1) + 1), "batch metadata")) return rc;
   h_err_ = h_meta_ + 4 * (B + 1);
   DA(d_tok_, 3 * (size_t)R + B); d_parent_ = d_tok_ + R; d_score_ = reinterpret_cast<float*>(d_tok_ + 2 * (size_t)R); d_fin_n_ = d_tok_ + 3 * (size_t)R;
   DA(d_hist_tok_, (size_t)Tcap * R); DA(d_hist_parent_, (size_t)Tcap * R);
   DA(d_fin_t_, (size_t)B * fin_cap); DA(d_fin_b_, (size_t)B * fin_cap);
   DA(d_rows_done_, B);
-  CK(cudaMemset(d_rows_done_, 0, sizeof(int) * B));
+  CK(cudaMemsetAsync(d_rows_done_, 0, sizeof(int) * B, stream));
   DA(d_fin_score_, (size_t)B * fin_cap); DA(d_fin_final_, (size_t)B * fin_cap);
   if (nm > 1) DA(d_combined_, (size_t)R * Vp);
   DA(d_cand_idx_, (size_t)R * kk); DA(d_cand_logp_, (size_t)R * kk); DA(d_eos_logp_, R); DA(d_row_stats_, 2 * (size_t)R);
@@ -413,7 +434,8 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   }
   lane_bytes_ = asked_bytes_ - weight_bytes;
   if (use_tc_ && xw_table_ && !of) { const int rc_xw = build_xw_tables(); if (rc_xw) return rc_xw; }
-  CK(cudaDeviceSynchronize());  // every weight upload has landed before the first decode
+  if (of) CK(cudaStreamSynchronize(stream));    // (others of the device's engines may be decoding)
+  else CK(cudaDeviceSynchronize());  // every weight upload has landed before the first decode
   return LINMT_OK;
 }
 
@@ -1019,7 +1041,7 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
   // (no exception leaves a thread, nor this function while its threads run)
   auto job = [&](Engine& g, int item) -> int {
     try {
-      return work(g, item);
+      return item < 0 ? g.ready() : work(g, item);
     } catch (const std::exception& e) {
       if (g.stream) cudaStreamSynchronize(g.stream);      // (copies from staging that the next batch reuses may be under way)
       try { g.err = std::string("out of host memory: ") + e.what(); } catch (...) {}
@@ -1037,10 +1059,15 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
   std::string err_text;
   auto worker = [&](int ei) {
     Engine& g = *workers[ei];
-    while (first_rc.load() == LINMT_OK) {
-      const size_t i = next.fetch_add(1);
-      if (i >= order.size()) break;
-      const int rc = job(g, order[i]);
+    for (bool made = false; first_rc.load() == LINMT_OK; made = true) {
+      int rc;
+      if (!made) {
+        rc = job(g, -1);
+      } else {
+        const size_t i = next.fetch_add(1);
+        if (i >= order.size()) break;
+        rc = job(g, order[i]);
+      }
       if (rc != LINMT_OK) {
         std::lock_guard<std::mutex> lock(err_mutex);
         if (first_rc.load() == LINMT_OK) { first_rc.store(rc); err_text = g.err; }
@@ -1069,9 +1096,9 @@ int Engine::lanes_for(int rows) const {
   return rows <= 64 || !step_streams(false, rows) ? 3 : 2;
 }
 
-bool Engine::room_for_lane() const {
+bool Engine::room_for_lanes(int n) const {
   size_t free_bytes = 0, total = 0;
-  return cudaSetDevice(opt.device) == cudaSuccess && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && lane_bytes_ <= free_bytes / 4;
+  return cudaSetDevice(opt.device) == cudaSuccess && cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && (size_t)n * lane_bytes_ <= free_bytes / 4;
 }
 
 }  // namespace linmt
@@ -1086,6 +1113,9 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
   const int devices = first_device ? 1 : n_engines();
   for (int i = 0; i < devices; ++i) w.push_back(&engine(i));
   const int per = eng.lanes_for(rows);
+  const auto broken = std::remove_if(lanes.begin(), lanes.end(), [](const auto& l) { return l->broken(); });
+  if (broken != lanes.end()) no_more_lanes = true;
+  lanes.erase(broken, lanes.end());
   for (int j = 1; j < per && w.size() < items; ++j)
     for (int i = 0; i < devices && w.size() < items; ++i) {
       Engine& of = engine(i);
@@ -1095,10 +1125,12 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
       for (auto& l : lanes)
         if (l->opt.device == of.opt.device && ++seen == j) lane = l.get();
       if (!lane && !no_more_lanes) {
-        try {
-          std::unique_ptr<Engine> l(new Engine());
-          if (of.room_for_lane() && l->init_lane(of) == LINMT_OK) { lane = l.get(); lanes.push_back(std::move(l)); }
-        } catch (const std::bad_alloc&) { lane = nullptr; }
+        if (of.room_for_lanes(1 + (int)std::count_if(lanes.begin(), lanes.end(), [&](const auto& l) { return l->planned() && l->opt.device == of.opt.device; })))
+          try {
+            std::unique_ptr<Engine> l(new Engine(&of));
+            lanes.push_back(std::move(l));
+            lane = lanes.back().get();
+          } catch (const std::bad_alloc&) {}
         if (!lane) { no_more_lanes = true; cudaGetLastError(); }
       }
       if (lane) w.push_back(lane);

@@ -90,8 +90,12 @@ class Engine {
   Engine() = default;
   ~Engine();
   int init(const linmt_model_desc& d, const float* const* blobs, int n_models, size_t blob_floats, const linmt_options& o);
-  // An engine on the same device with the weights of `of`, which it must not outlive, and state, stream and workspaces of its own.
-  int init_lane(const Engine& of);
+  // A lane: an engine on the device of `of` with its weights, which it must not outlive, and state, stream and workspaces of its own.
+  // Those are made by `ready`, in the thread that is going to use them; one that could not be is `broken` and of no use.
+  explicit Engine(const Engine* of) : lane_of_(of), broken_(true) { opt = of->opt; }
+  int ready();
+  bool planned() const { return lane_of_ != nullptr; }
+  bool broken() const { return broken_ && !lane_of_; }
   // While one lives, the engine's device batch is one of a call's that run at once on a device, and its products leave room for others.
   // That goes by the engines that the call has, not by what runs at the moment: a sentence's last bits do not depend on time.  (Not in one
   // plane: in other shapes the sums are in another order, which rounds a state to the other bf16 neighbour now and then.  A
@@ -103,9 +107,9 @@ class Engine {
   };
   // Device batches of a call that are worth running at once, of this engine's `rows` each.
   int lanes_for(int rows) const;
-  // Whether the device can spare what a lane takes: a quarter of its free memory at most, for calls grow an engine's buffers and others
-  // use the device as well.
-  bool room_for_lane() const;
+  // Whether the device can spare what so many lanes take: a quarter of its free memory at most, for calls grow an engine's buffers and
+  // others use the device as well.
+  bool room_for_lanes(int n) const;
   int decode_core(const int32_t* d_ids, const int32_t* off_host, int n, const int32_t* steps_host, int max_len,
                   int32_t* d_out_tok, int32_t* d_out_len, float* d_out_score, int32_t* d_out_vit, float* d_out_align,
                   const linmt_trace* trace_dev, int trace_Tm);
@@ -145,7 +149,10 @@ class Engine {
   std::string result_buf;
 
  private:
+  int init_lane(const Engine& of);
   int init_state(const Engine* of, const float* const* blobs);
+  const Engine* lane_of_ = nullptr;      // a lane that is not made yet
+  bool broken_ = false;
   int fail(int code, const std::string& msg) { err = msg; return code; }
   int cuda_failed(cudaError_t e, const char* file, int line);
   // role of member mi in the alignment record of a step: 0 = single model, 1 / 2 / 3 = first / middle / last member
@@ -246,7 +253,12 @@ class Engine {
   std::vector<DevModel> models_;
   std::vector<DevState> states_;
   std::vector<void*> allocs_;
-  size_t asked_bytes_ = 0, lane_bytes_ = 0;     // device memory requested so far; what the handle's creation took beside the weights
+  // device memory requested so far, in whole units; what the handle's creation took of it beside the weights
+  static constexpr size_t kMemoryUnit = 512;
+  size_t asked_bytes_ = 0, lane_bytes_ = 0;
+  // A lane's creation takes all that in one request, and its buffers from there: a request costs 0.3 to 2 ms, whatever its size.
+  char* arena_ = nullptr;
+  size_t arena_used_ = 0, arena_bytes_ = 0;
   int device_memory(void** p, size_t bytes, const char* what);
   int host_memory(void** p, size_t bytes, const char* what);      // (pinned)
   template <class T> int dalloc(T** p, size_t count);
@@ -296,6 +308,7 @@ class Engine {
     *p = static_cast<T*>(q);
     return LINMT_OK;
   }
+  // (buffers that are made when they are needed; those of the creation stay)
   void release(void* p) {
     for (auto it = allocs_.begin(); p && it != allocs_.end(); ++it)
       if (*it == p) { allocs_.erase(it); cudaFree(p); return; }
@@ -325,7 +338,7 @@ struct linmt_engine {
   linmt::Engine eng;
   std::vector<std::unique_ptr<linmt::Engine>> replicas;
   // Further engines on the devices above, with their weights: a call of several device batches runs some at once (Engine::lanes_for).
-  // Made when such a call first wants them, and kept, unless memory is short (with_lanes).
+  // Made when such a call first wants them, beside the batches that it has begun with, and kept, unless memory is short (with_lanes).
   std::vector<std::unique_ptr<linmt::Engine>> lanes;
   bool no_more_lanes = false;
   // Runs `call`, which may use the lanes; where it fails for memory, which they hold some of or were refused, it runs once more from its

@@ -705,24 +705,26 @@ int Engine::reserve_score(size_t rows) {
   }
   if (score_q_) return LINMT_OK;
   const size_t cap = std::max<size_t>(128, (((size_t)64 << 20) / Vp) & ~(size_t)127);
-  // (what a call that failed for memory here had got before that)
-  for (float* p : score_logits_) release(p);
-  for (void* p : {(void*)score_logits16_, (void*)score_combined_, (void*)score_idx_, (void*)score_candp_, (void*)score_eos_, (void*)score_stats_,
-                  (void*)score_pmax_, (void*)score_psum_})
-    release(p);
-  score_logits16_ = nullptr; score_combined_ = score_candp_ = score_eos_ = score_stats_ = score_pmax_ = score_psum_ = nullptr; score_idx_ = nullptr;
+  // (one request for all parts)
+  size_t at = 0;
+  auto part = [&](bool wanted, size_t bytes) {
+    const size_t here = at;
+    if (wanted) at += (bytes + kMemoryUnit - 1) / kMemoryUnit * kMemoryUnit;
+    return here;
+  };
+  const size_t logits16 = part(logits16_, cap * Vp * 2), logits = part(!logits16_, (size_t)n_models * cap * Vp * 4), combined = part(n_models > 1, cap * Vp * 4),
+               idx = part(true, cap * kk * 4), candp = part(true, cap * kk * 4), eos = part(true, cap * 4), statistics = part(true, cap * 8),
+               pmax = part(true, cap * pmax_ld_ * 4), psum = part(true, cap * pmax_ld_ * 4);
+  char* ws = nullptr;
+  if ((rc = dalloc_bytes(&ws, at))) return rc;
+  auto floats = [&](size_t offset) { return reinterpret_cast<float*>(ws + offset); };
   score_logits_.assign(n_models, nullptr);
-  if (logits16_) {
-    if ((rc = dalloc_bytes(&score_logits16_, cap * Vp * 2))) return rc;
-  } else {
-    for (int mi = 0; mi < n_models; ++mi)
-      if ((rc = dalloc_bytes(&score_logits_[mi], cap * Vp * 4))) return rc;
-  }
-  if (n_models > 1 && (rc = dalloc_bytes(&score_combined_, cap * Vp * 4))) return rc;
-  if ((rc = dalloc_bytes(&score_idx_, cap * kk * 4)) || (rc = dalloc_bytes(&score_candp_, cap * kk * 4)) || (rc = dalloc_bytes(&score_eos_, cap * 4)) ||
-      (rc = dalloc_bytes(&score_stats_, cap * 8)) || (rc = dalloc_bytes(&score_pmax_, cap * pmax_ld_ * 4)) ||
-      (rc = dalloc_bytes(&score_psum_, cap * pmax_ld_ * 4)))
-    return rc;
+  if (logits16_) score_logits16_ = reinterpret_cast<__half*>(ws + logits16);
+  else
+    for (int mi = 0; mi < n_models; ++mi) score_logits_[mi] = floats(logits) + (size_t)mi * cap * Vp;
+  if (n_models > 1) score_combined_ = floats(combined);
+  score_idx_ = reinterpret_cast<int32_t*>(ws + idx);
+  score_candp_ = floats(candp); score_eos_ = floats(eos); score_stats_ = floats(statistics); score_pmax_ = floats(pmax); score_psum_ = floats(psum);
   score_q_ = (int)cap;
   return LINMT_OK;
 }

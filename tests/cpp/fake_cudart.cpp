@@ -3,6 +3,7 @@
 // told to, and checks that every copy and fill stays inside one live allocation.
 #include <cuda.h>
 #include <cuda_runtime_api.h>
+#include <pthread.h>
 
 #include <cstdlib>
 #include <cstring>
@@ -20,6 +21,8 @@ thread_local cudaError_t pending = cudaSuccess;   // what cudaGetLastError retur
 thread_local int device = 0;
 struct Call { dim3 grid, block; size_t smem; void* stream; };
 thread_local Call call;
+
+const pthread_t main_thread = pthread_self();
 
 long& v(const char* key) { return value[key]; }
 
@@ -82,7 +85,7 @@ long fake_launches(const char* part) {
 
 cudaError_t cudaMalloc(void** p, size_t bytes) {
   std::lock_guard<std::recursive_mutex> lock(mu);
-  ++v("requests");
+  ++v(pthread_equal(pthread_self(), main_thread) ? "requests" : "requests_beside");
   if (refused(bytes)) return pending = cudaErrorMemoryAllocation;
   *p = std::calloc(bytes ? bytes : 1, 1);
   live[static_cast<char*>(*p)] = bytes;
@@ -101,7 +104,7 @@ cudaError_t cudaFree(void* p) {
 }
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
   std::lock_guard<std::recursive_mutex> lock(mu);
-  ++v("requests");
+  ++v(pthread_equal(pthread_self(), main_thread) ? "requests" : "requests_beside");
   if (refused(0)) return pending = cudaErrorMemoryAllocation;
   *p = std::calloc(bytes ? bytes : 1, 1);
   return cudaSuccess;
@@ -141,7 +144,12 @@ cudaError_t cudaMemcpy2D(void* d, size_t dp, const void* s, size_t sp, size_t w,
   for (size_t y = 0; y < h; ++y) copy(static_cast<char*>(d) + y * dp, static_cast<const char*>(s) + y * sp, w, k);
   return cudaSuccess;
 }
-cudaError_t cudaDeviceSynchronize() { fake_set("unordered", 0); return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize() {
+  std::lock_guard<std::recursive_mutex> lock(mu);
+  v("unordered") = 0;
+  ++v("device_waits");
+  return cudaSuccess;
+}
 cudaError_t cudaSetDevice(int d) { device = d; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* out, cudaDeviceAttr a, int) {
