@@ -156,7 +156,11 @@ cudaError_t cudaDeviceGetAttribute(int* out, cudaDeviceAttr a, int) {
   *out = a == cudaDevAttrComputeCapabilityMajor ? 10 : a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrL2CacheSize ? 126 << 20 : 0;
   return cudaSuccess;
 }
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { return fresh(s); }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+  std::lock_guard<std::recursive_mutex> lock(mu);
+  ++v("streams");
+  return fresh(s);
+}
 cudaError_t cudaStreamDestroy(cudaStream_t s) { std::free(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }

@@ -267,20 +267,91 @@ assert got == want, (got, want)
 def test_further_engines_are_made_beside_the_first_batches(child):
     """The first call of several batches does not wait for them: its thread asks for what it asks for without them, nothing waits for the
     whole device, and the two make a few requests each (an engine's creation is one)."""
-    child(LANES + """
-def asked(dec, call):
+    child("""
+same = synth.make_sentences(16, 9, 9, D.Vs, 1.1, 3, lambda s: s + 3)        # four batches of one size
+def asked(call):
     put("requests", 0); put("requests_beside", 0); put("device_waits", 0)
     call()
-    return get("requests")
-os.environ["LINMT_LANES"] = "0"
-dec = make()
-alone = [asked(dec, lambda: dec.decode(some(18))), asked(dec, lambda: dec.score(some(18), words(18, 12)))]
-dec.close()
-del os.environ["LINMT_LANES"]
-dec = make()
-for want, call in zip(alone, (lambda: dec.decode(some(18)), lambda: dec.score(some(18), words(18, 12)))):
-    assert asked(dec, call) <= want        # (less where another engine has taken every batch that wants more)
     assert get("device_waits") == 0
-    assert 0 < get("requests_beside") <= 2 * 20
+    return get("requests")
+for entry in (lambda dec: dec.decode(same), lambda dec: dec.score(same, words(16, 12))):
+    os.environ["LINMT_LANES"] = "0"
+    dec = make()
+    alone = asked(lambda: entry(dec))
+    dec.close()
+    del os.environ["LINMT_LANES"]
+    dec = make()
+    assert asked(lambda: entry(dec)) <= alone          # (less where the others have taken every batch)
+    assert 0 < get("requests_beside") <= 2 * 12
+    dec.close()
+""")
+
+
+def test_engines_of_a_call(child):
+    """Three up to 64 rows, and beyond where L2 holds a step's weights, else two; one from 513 rows on, for one batch, for an ensemble, and
+    while kernels are timed.  (An engine makes one stream; sources as short as these are encoded on that.)"""
+    child("""
+def engines(n, timing=False, **kw):
+    put("streams", 0)
+    dec = decoder.Decoder(d, blobs, max_src_len=16, max_steps=4, **kw)
+    dec.set_kernel_timing(timing)
+    dec.decode(synth.make_sentences(n, 2, 9, d.Vs, 1.1, 3, lambda s: 3))
+    dec.decode(synth.make_sentences(n, 2, 9, d.Vs, 1.1, 3, lambda s: 3))
+    dec.close()
+    return get("streams")
+d, blobs = D, [BLOB]
+assert engines(31, beam=2, max_batch=4) == 3
+assert engines(8, beam=2, max_batch=4) == 2
+assert engines(4, beam=2, max_batch=4) == 1
+assert engines(31, timing=True, beam=2, max_batch=4) == 1
+assert engines(200, beam=8, max_batch=64) == 3
+assert engines(200, beam=9, max_batch=57) == 1          # 513 rows
+d = synth.ModelDesc(5, 768, 3000, 300, 1)               # 104 MB a step in fp32 precision, of 126 MB of L2
+blobs = [synth.make_blob(d, 1)]
+assert engines(100, beam=2, max_batch=32) == 3
+assert engines(100, beam=2, max_batch=33) == 2
+assert engines(100, beam=2, max_batch=33, precision="bf16") == 3
+""")
+
+
+def test_an_error_in_a_further_engine_is_the_call_s(child):
+    """A sentence that cannot be decoded, in whichever of the batches: the code and the text that one engine gives, and a handle that
+    goes on working."""
+    child("""
+def bad(i, what):
+    s = some(18)
+    lens = s.lengths().copy()
+    lens[i] = 0 if what == "empty" else 17
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    return synth.Sentences(np.full(int(off[-1]), 5, np.int32), off, np.full(18, 5, np.int32))
+def error(call):
+    try:
+        call()
+    except decoder.LinmtError as e:
+        return str(e)
+dec = make()
+for i in range(18):
+    for what, code in (("empty", "(1): empty source"), ("long", "(5): source sentence longer")):
+        for call in (lambda: dec.decode(bad(i, what)), lambda: dec.score(bad(i, what), words(18))):
+            assert code in str(error(call)), (i, error(call))
+        dec.decode(some(18)); dec.score(some(18), words(18))
 dec.close()
+""")
+
+
+def test_layers_side_by_side_of_more_words_than_the_panels_hold(child):
+    """40 sentences of 500 words are 20000 rows, in two chunks of 409 and 91 positions: the layers side by side (512 units) make an input
+    product for every eight of them, layer by layer (448 units) one a chunk."""
+    child("""
+def launched(H, n, longest):
+    d = synth.ModelDesc(2, H, 3000, 300, 1)
+    dec = decoder.Decoder(d, [synth.make_blob(d, 1)], beam=2, max_batch=n, max_src_len=longest, max_steps=4)
+    before = dec.stats()["kernel_launches"]
+    dec.score(synth.make_sentences(n, longest, longest, d.Vs, 1.1, 3, lambda s: 3), words(n, 1))
+    count = dec.stats()["kernel_launches"] - before
+    dec.close()
+    return count
+assert launched(512, 40, 500) - launched(448, 40, 500) == 2 * (52 + 12 - 2)
+assert launched(512, 2, 20) - launched(448, 2, 20) == 2 * (3 - 1)
+assert launched(512, 2, 19) == launched(448, 2, 19)
 """)

@@ -611,3 +611,50 @@ def test_one_plane_has_one_order_of_sums(cuda_lib, L, H, n, beam, max_batch, lon
     for key in ("tok", "len", "score"):
         assert a[key].tobytes() == b[key].tobytes(), key
     assert x[1].tobytes() == y[1].tobytes()
+
+
+@pytest.mark.parametrize("L,H,beam,max_batch,n,lo,hi", [
+    (5, 768, 3, 32, 100, 2, 12),       # a step's weights are more than L2 keeps: two engines, of 96 rows
+    (3, 256, 1, 96, 200, 20, 40)])     # three engines, each with a pipelined encoder (96 sentences of 32 words and more)
+def test_engines_of_a_call_beyond_l2_and_with_pipelined_encoders(cuda_lib, L, H, beam, max_batch, n, lo, hi):
+    """Device batches at once: the same bits in every call, and the results of one batch after another to fp32 rounding."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(L, H, 3000, 300, 1)
+    blob = synth.make_blob(d, 40, family="peaked")
+    sents = synth.make_sentences(n, lo, hi, d.Vs, 1.1, 3, lambda s: s // 2 + 3)
+    rng = np.random.default_rng(n)
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 12, size=n)]
+    kw = dict(beam=beam, max_batch=max_batch, max_src_len=hi, max_steps=24, cp_beta=0.0)
+    one = _with_env({"LINMT_LANES": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    b, y = one.decode(sents), one.score(sents, targets)
+    one.close()
+    dec = decoder.Decoder(d, [blob], **kw)
+    a, x = dec.decode(sents), dec.score(sents, targets)
+    for _ in range(3):
+        again, z = dec.decode(sents), dec.score(sents, targets)
+        assert a["tok"].tobytes() == again["tok"].tobytes() and a["score"].tobytes() == again["score"].tobytes()
+        assert x[1].tobytes() == z[1].tobytes()
+    dec.close()
+    scale = np.maximum(1, np.abs(y[1]).max(axis=1, keepdims=True))
+    assert (np.abs(x[1] - y[1]) <= RTOL_FP32 * scale).all(), float((np.abs(x[1] - y[1]) / scale).max())
+    same = [i for i in range(n) if hyps(a, i) == hyps(b, i)]
+    assert len(same) >= 0.95 * n, len(same)       # (a tie may go the other way)
+    for i in same:
+        np.testing.assert_allclose(a["score"][i, 0], b["score"][i, 0], rtol=RTOL_FP32)
+
+
+def test_encoder_layers_side_by_side_in_two_chunks(cuda_lib):
+    """40 sentences of up to 500 words are more rows than the panels hold (16384): against the encoder position by position."""
+    from linmt_b200 import decoder
+    d = synth.ModelDesc(2, 512, 300, 200, 1)
+    blob = synth.make_blob(d, 11, family="peaked")
+    sents = synth.make_sentences(40, 380, 500, d.Vs, 1.1, 3, lambda s: 3)
+    rng = np.random.default_rng(4)
+    targets = [rng.integers(3, d.V, size=int(m)) for m in rng.integers(1, 4, size=40)]
+    kw = dict(beam=2, max_batch=40, max_src_len=500, max_steps=8, cp_beta=0.0)
+    dec = decoder.Decoder(d, [blob], **kw)
+    ref = _with_env({"LINMT_TC_ROWS": "0"}, lambda: decoder.Decoder(d, [blob], **kw))
+    a, b = dec.score(sents, targets), ref.score(sents, targets)
+    dec.close(); ref.close()
+    scale = np.maximum(1, np.abs(b[1]).max(axis=1, keepdims=True))
+    assert (np.abs(a[1] - b[1]) <= RTOL_FP32 * scale).all(), float((np.abs(a[1] - b[1]) / scale).max())
