@@ -396,9 +396,15 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   // batch of 128 sentences, beam 5, 35.0 -> 35.3 ms by the few steps of its longest sentences).
   // One plane makes them in place: the parts of a gate summed apart round a state to the other bf16 neighbour now and then, and a near
   // tie of two hypotheses is decided by that (4 x 1000 / 30k, one sentence, beam 5, would gain 5 %).
+  // Rows: from 49 on their CTAs, for 64 rows, take longer than what they run beside unless the layers are few or narrow.  40 steps, ms a
+  // call without / with them at 48, 52 and 60 rows: 4 x 1000 4.16 / 4.26 (60 steps: 6.22 / 6.16), 4.49 / 4.70, 4.56 / 4.82; 3 x 1000 3.63 /
+  // 3.58, 3.88 / 3.92, 3.95 / 4.04; 4 x 768 3.62 / 3.33, 3.91 / 3.93, 3.99 / 4.13; 2 x 1024 3.82 / 3.47, 3.87 / 3.79, 3.93 / 3.95;
+  // 3 x 768 3.30 / 3.10, 3.59 / 3.53, 3.69 / 3.69; 4 x 512 3.10 / 2.91, 3.33 / 3.08, 3.41 / 3.19; 3 x 250 2.86 / 2.69, 2.95 / 2.73, 2.98 /
+  // 2.73.  Rows that continue themselves have no gather to save: 4 x 1000 greedily 32 rows 3.93 / 3.77, 64 5.62 / 5.89 for 48 steps.
   float some = 0.f;
   const bool beside_softmax = logit_blocks(&some, &some, logit_blocks_ld(Vp), Vp, Hp, tc::BM, 32).sum != nullptr;
-  if (ahead_ && beside_softmax && use_tc_ && rows_ && xw_table_ && nm == 1 && L > 1 && Hp >= 256 && fmt_ == 1) rec_rows_ = std::min(R, k > 1 ? tc::kRowsAhead : kRowsAheadSelf);
+  if (ahead_ && beside_softmax && use_tc_ && rows_ && xw_table_ && nm == 1 && L > 1 && Hp >= 256 && fmt_ == 1)
+    rec_rows_ = std::min(R, k == 1 ? kRowsAheadSelf : (size_t)L * Hp * Hp > kWideLayers ? kRowsAheadWide : tc::kRowsAhead);
   models_.resize(nm); states_.resize(nm); tc_states_.resize(nm);
   size_t weight_bytes = 0;
   for (int i = 0; i < nm; ++i) {

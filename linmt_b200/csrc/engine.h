@@ -176,7 +176,8 @@ class Engine {
   bool ahead_ok(int rows) const;
   enum class Ahead { kBetween, kEnds };      // which of the recurrent products: the layers' between first and last, those two's
   // where they are in DevState::rec: the first layer's states, the last one's, the first layer's feed-input, the layers between
-  static constexpr int kRowsAheadSelf = 32;      // rows that continue themselves have no gather to save
+  static constexpr int kRowsAheadSelf = 32, kRowsAheadWide = 48;      // (see init_state; kRowsAhead otherwise)
+  static constexpr size_t kWideLayers = (size_t)2 << 20;              // layers x units x units
   static constexpr int kRecFeed = 2;
   int rec_slot(int l) const { return l == 0 ? 0 : l == L - 1 ? 1 : l + 2; }
   int recurrent_ahead(Ahead which, int mi, int t, int rows);

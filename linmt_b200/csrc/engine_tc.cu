@@ -568,8 +568,8 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc, in
 // while the attention, the softmax and the selection run on a few SMs; these products run beside them, those of the layers
 // between beside the attention, the rest beside the softmax.  What is left of the chain is half a product a layer, none of the
 // first (lstm_cell_kernel adds up its terms), and no state is gathered.  48 steps, ms a call without / with: 4 x 1000 / 30k 1 row
-// 3.92 / 3.81, 12 rows 4.74 / 4.02, 24 4.88 / 4.34, 60 5.57 / 5.47; 2 x 1000 12 rows 3.55 / 3.08, 48 3.69 / 3.46;
-// 3 x 250 / 5k 12 rows 2.50 / 2.36; beyond 48 rows their CTAs take longer than what they run beside (kRowsAhead; 32, kRowsAheadSelf, where there is no gather to save).
+// 3.92 / 3.81, 12 rows 4.74 / 4.02, 24 4.88 / 4.34; 2 x 1000 12 rows 3.55 / 3.08, 48 3.69 / 3.46;
+// 3 x 250 / 5k 12 rows 2.50 / 2.36.  (Up to how many rows: init_state.)
 //
 // They start without a wait for the kernel before them in the stream (RowsShape::ahead).  Before the attention that is where the
 // projections have let the attention start only behind their own wait, and it these products: the layers' states are complete.

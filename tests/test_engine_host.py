@@ -355,3 +355,21 @@ assert launched(512, 40, 500) - launched(448, 40, 500) == 2 * (52 + 12 - 2)
 assert launched(512, 2, 20) - launched(448, 2, 20) == 2 * (3 - 1)
 assert launched(512, 2, 19) == launched(448, 2, 19)
 """)
+
+
+def test_rows_whose_recurrent_products_are_made_ahead(child):
+    """Up to 60, of few or narrow layers; up to 48 of more than 2 Mi layers x units x units; up to 32 of one slot each."""
+    child("""
+def ahead(dec, n, beam):
+    before = launches("TcEpiParts")
+    dec.decode(synth.make_sentences(n, 4, 4, D.Vs, 1.1, 3, lambda s: 5))      # (all end together)
+    return launches("TcEpiParts") > before
+for L, H, most in ((2, 256, 60), (3, 768, 60), (3, 840, 48)):
+    d = synth.ModelDesc(L, H, 3000, 300, 1)
+    blob = synth.make_blob(d, 1)
+    for beam in (4, 1):
+        dec = decoder.Decoder(d, [blob], beam=beam, max_batch=70 // beam, max_src_len=16, max_steps=8)
+        bound = (32 if beam == 1 else most) // beam
+        assert ahead(dec, bound, beam) and not ahead(dec, bound + 1, beam), (L, H, beam)
+        dec.close()
+""")
