@@ -616,7 +616,8 @@ int Engine::launch_attention(int mi, int t, int rows, int kb, const float* u_alt
 }
 
 // Softmax statistics and top-k of rows whose logits vocab_gemm has just produced, from the block statistics it left if it did.
-cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel, bool late) {
+cudaError_t Engine::softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf,
+                                 const SelectArgs& sel, bool late) {
   return launch_topk(logits, logits16_ ? logits16 : nullptr, Vp, V, kk, rows, n_sm_, o, normalise, blocks_, rf, sel, stream, pdl_, late);
 }
 
@@ -777,7 +778,8 @@ int Engine::decode_core(const int32_t* d_ids, const int32_t* off_host, int n, co
     int n_next = n_act;       // sentences of the next step
     while (n_next > 0 && m_steps[n_next - 1] < t + 1) --n_next;
     const int rows = n_act * k, rows_next = ahead_ok(n_next * k) ? n_next * k : 0;
-    if ((rc = each_member(rows, [&](int mi) { return use_tc_ ? run_decoder_step_tc(mi, t, rows, nullptr, rows_next) : run_decoder_step(mi, t, rows); }))) return rc;
+    auto step = [&](int mi) { return use_tc_ ? run_decoder_step_tc(mi, t, rows, nullptr, rows_next) : run_decoder_step(mi, t, rows); };
+    if ((rc = each_member(rows, step))) return rc;
     if ((rc = step_tail(t, rows, rows_next > 0))) return rc;
     if (rows_next > 0) {
       if ((rc = recurrent_ahead(Ahead::kEnds, 0, t, rows_next))) return rc;
@@ -1131,7 +1133,8 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
       for (auto& l : lanes)
         if (l->opt.device == of.opt.device && ++seen == j) lane = l.get();
       if (!lane && !no_more_lanes) {
-        if (of.room_for_lanes(1 + (int)std::count_if(lanes.begin(), lanes.end(), [&](const auto& l) { return l->planned() && l->opt.device == of.opt.device; })))
+        auto coming = [&](const auto& l) { return l->planned() && l->opt.device == of.opt.device; };
+        if (of.room_for_lanes(1 + (int)std::count_if(lanes.begin(), lanes.end(), coming)))
           try {
             std::unique_ptr<Engine> l(new Engine(&of));
             lanes.push_back(std::move(l));
@@ -1223,8 +1226,8 @@ const char* linmt_last_error(const linmt_engine* e) { return e ? e->eng.err.c_st
 
 int32_t linmt_beam(const linmt_engine* e) { return e ? e->eng.k : 0; }
 
-static int decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n, const int32_t* steps, int32_t max_len, int32_t* out_tok,
-                        int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align, const linmt_trace* trace) {
+static int decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n, const int32_t* steps, int32_t max_len,
+                        int32_t* out_tok, int32_t* out_len, float* out_score, int32_t* out_vit, float* out_align, const linmt_trace* trace) {
   Engine& g0 = e->eng;
   const int B = g0.B;
   if ((g0.kernel_timing && e->n_engines() == 1) || trace || n <= B || !src_ids || !src_off || !steps || !out_tok || !out_len || !out_score)

@@ -67,7 +67,8 @@ struct DevState {
   float* hs = nullptr;                               // [B][max_src][Hp]
   tc::Planes hs16{};                                 // the same in bf16 (one plane: instead of hs)
   float* hs_wc1 = nullptr;                           // [B][max_src][Hp]  W_c1 . hs (tensor path with the attention fold)
-  float* rec = nullptr;                              // [L + 1][rec_rows_][4Hp]  recurrent products of the step before, by its rows (Engine::recurrent_ahead), in the order of rec_slot
+  // [L + 1][rec_rows_][4Hp]  recurrent products of the step before, by its rows (Engine::recurrent_ahead), in the order of rec_slot
+  float* rec = nullptr;
   float* enc_x = nullptr;                            // [B][Hp]
   float* enc_pre = nullptr;                          // [rows][4Hp]  W_x . input of every position (encoder layer by layer)
   std::vector<float*> enc_h[2], enc_c[2];            // [L] x [B][Hp], double buffered
@@ -184,7 +185,8 @@ class Engine {
   // rows that continue themselves: one beam slot (scoring aside)
   bool self_rows() const { return k == 1 && !trace_dev_.force_tok; }
   int vocab_gemm(int mi, const tc::Planes& ht, int rows_cap, int rows, float* logits, __half* logits16, float* pmax, float* psum);
-  cudaError_t softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel, bool late = false);
+  cudaError_t softmax_topk(const float* logits, const __half* logits16, int rows, const TopkOut& o, int normalise, const TopkRefine* rf, const SelectArgs& sel,
+                           bool late = false);
   int score_core_tc(int n, int Smax, const std::vector<int>& n_act, const int32_t* d_tok, const int32_t* d_gold, float* d_logp);
   int reserve_score(size_t rows);
   TopkRefine refinement(const tc::Planes& ht) const;    // of one-product logits of these attentional states

@@ -303,7 +303,8 @@ int Engine::encode_positions(int mi, int l, int n, int pos0, int np, float* pre,
   return LINMT_OK;
 }
 
-// Encoder for more sentences and longer sources (`few`: few sentences): the layers side by side on a stream each, every one kEncLag positions behind the layer below.
+// Encoder for more sentences and longer sources (`few`: few sentences): the layers side by side on a stream each, every one kEncLag
+// positions behind the layer below.
 // As in the form above, the input parts of that many positions are one product, and what is left of the recurrence reads
 // half of a layer's weights, which all layers' together (67 MB in fp32 precision) stay in L2; but every layer's products are
 // shaped for their share of the SMs and run beside the others'.  Sources longer than the panels are taken in chunks: the
@@ -490,7 +491,8 @@ int Engine::run_decoder_step_tc(int mi, int t, int rows, const ScoreStep* sc, in
     int rc;
     if (have_rec && l == 0) {
       e.xw = m.dec_xw; e.x_tok = tok; e.x_ld = 4 * Hp; e.x_vocab = V; e.x_unk = kUnk;
-      CK(tc::launch_k(pdl_, lstm_cell_kernel, dim3(rows, (Hp + 127) / 128), dim3(128), 0, stream, e, (const float*)s.rec, (const float*)(desc.feed_input ? s.rec + (size_t)kRecFeed * rec_rows_ * 4 * Hp : nullptr), Hp));
+      const float *pre = s.rec, *fed = desc.feed_input ? s.rec + (size_t)kRecFeed * rec_rows_ * 4 * Hp : nullptr;
+      CK(tc::launch_k(pdl_, lstm_cell_kernel, dim3(rows, (Hp + 127) / 128), dim3(128), 0, stream, e, pre, fed, Hp));
       LAUNCHED();
       rc = LINMT_OK;
     } else if (have_rec) {
@@ -712,8 +714,8 @@ int Engine::reserve_score(size_t rows) {
     if (wanted) at += (bytes + kMemoryUnit - 1) / kMemoryUnit * kMemoryUnit;
     return here;
   };
-  const size_t logits16 = part(logits16_, cap * Vp * 2), logits = part(!logits16_, (size_t)n_models * cap * Vp * 4), combined = part(n_models > 1, cap * Vp * 4),
-               idx = part(true, cap * kk * 4), candp = part(true, cap * kk * 4), eos = part(true, cap * 4), statistics = part(true, cap * 8),
+  const size_t logits16 = part(logits16_, cap * Vp * 2), logits = part(!logits16_, (size_t)n_models * cap * Vp * 4),
+               combined = part(n_models > 1, cap * Vp * 4), idx = part(true, cap * kk * 4), candp = part(true, cap * kk * 4), eos = part(true, cap * 4), statistics = part(true, cap * 8),
                pmax = part(true, cap * pmax_ld_ * 4), psum = part(true, cap * pmax_ld_ * 4);
   char* ws = nullptr;
   if ((rc = dalloc_bytes(&ws, at))) return rc;

@@ -476,7 +476,8 @@ const char* linmt_translate(linmt_engine* h, const char* sentence) {
   const bool want_align = e.opt.print_info && e.print_align_scores;
   if (want_align) align.resize((size_t)nb * max_len * e.opt.max_src_len);
   int rc = h->with_lanes([&] {
-    return e.decode_host(ids.data(), off, 1, &steps, max_len, tok.data(), len.data(), score.data(), vit.data(), want_align ? align.data() : nullptr, nullptr);
+    return e.decode_host(ids.data(), off, 1, &steps, max_len, tok.data(), len.data(), score.data(), vit.data(),
+                         want_align ? align.data() : nullptr, nullptr);
   });
   if (rc != LINMT_OK) return e.result_buf.c_str();
   e.result_buf = format_result(e, S, nb, max_len, tok.data(), len.data(), score.data(), vit.data(),

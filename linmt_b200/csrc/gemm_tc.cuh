@@ -381,7 +381,8 @@ struct TcEpiLstm {
   const float* xw = nullptr; const int32_t* x_tok = nullptr; int x_ld = 0; int x_vocab = 0; int x_unk = 0;
   bool x_parent = false;     // (without x_tok) the row of `xw` is the parent's, as c_prev's is
   __device__ __forceinline__ int x_row(int row) const {
-    if (!x_tok) return x_parent ? c_src_row(row) : row;    // one row of the table per row of the product (encoder: the input's share of every position)
+    // (encoder: one row of the table per row of the product, the input's share of every position)
+    if (!x_tok) return x_parent ? c_src_row(row) : row;
     const int t = x_tok[row];
     return (t < 0 || t >= x_vocab) ? x_unk : t;
   }

@@ -172,8 +172,12 @@ struct TmapSets { TmapSet s[SEGS]; };
 // first instruction, ahead of the first read of its parameters, which cost 1 to 3 % of a chain of small products.)
 template <int NT, int FMT, class Epi, int SEGS, bool LATE>
 __global__ void __launch_bounds__(kRowsThreads, 2)
-gemm_tc_rows_kernel(const __grid_constant__ TmapSets<SEGS> tms, int M, int N, int K, int x_row0, RowsShape sh, Epi epi_of, int* __restrict__ err_flag) {
-  auto chosen = [&]() -> std::conditional_t<(SEGS > 1), Epi, const Epi&> { if constexpr (SEGS > 1) return epi_of.of(blockIdx.y); else return epi_of; };
+gemm_tc_rows_kernel(const __grid_constant__ TmapSets<SEGS> tms, int M, int N, int K, int x_row0, RowsShape sh, Epi epi_of,
+                    int* __restrict__ err_flag) {
+  auto chosen = [&]() -> std::conditional_t<(SEGS > 1), Epi, const Epi&> {
+    if constexpr (SEGS > 1) return epi_of.of(blockIdx.y);
+    else return epi_of;
+  };
   const Epi& epi = chosen();
   const TmapSet& tm = tms.s[SEGS > 1 ? blockIdx.y : 0];
   constexpr int PC = product_code(NT, FMT);
@@ -390,7 +394,8 @@ gemm_tc_rows_kernel(const __grid_constant__ TmapSets<SEGS> tms, int M, int N, in
 
 // x_row0: first row of the product in the activations' tensor map
 template <int NT, int FMT, class Epi, int SEGS, bool LATE>
-inline cudaError_t launch_gemm_tc_rows_of(const TmapSets<SEGS>& tms, int segs, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0) {
+inline cudaError_t launch_gemm_tc_rows_of(const TmapSets<SEGS>& tms, int segs, int M, int N, int K, const RowsShape& sh, const Epi& epi,
+                                          int* err_flag, cudaStream_t st, int x_row0) {
   static std::atomic<bool> optin_done[kMaxDevices] = {};
   if (cudaError_t e = ensure_smem_optin(gemm_tc_rows_kernel<NT, FMT, Epi, SEGS, LATE>, optin_done, kRowsSmemWhole); e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
@@ -413,7 +418,8 @@ inline cudaError_t launch_gemm_tc_rows_of(const TmapSets<SEGS>& tms, int segs, i
   return cudaLaunchKernelEx(&cfg, gemm_tc_rows_kernel<NT, FMT, Epi, SEGS, LATE>, tms, M, N, K, x_row0, sh, epi, err_flag);
 }
 template <int NT, int FMT, class Epi>
-inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st, int x_row0 = 0, bool late = false) {
+inline cudaError_t launch_gemm_tc_rows(const TmapSet& tm, int M, int N, int K, const RowsShape& sh, const Epi& epi, int* err_flag, cudaStream_t st,
+                                       int x_row0 = 0, bool late = false) {
   if constexpr (Epi::kLate)
     if (late) return launch_gemm_tc_rows_of<NT, FMT, Epi, 1, true>(TmapSets<1>{{tm}}, 1, M, N, K, sh, epi, err_flag, st, x_row0);
   return launch_gemm_tc_rows_of<NT, FMT, Epi, 1, false>(TmapSets<1>{{tm}}, 1, M, N, K, sh, epi, err_flag, st, x_row0);

@@ -130,7 +130,8 @@ static __global__ void row_gather_kernel(GatherJobs jobs, const int32_t* __restr
 // First decoder layer of a step whose recurrent products are there already (Engine::recurrent_ahead): gates of row r = row
 // parent[r] of `pre` (its second part `feed` behind it, or null) plus the input term of its token, which the epilogue's preload looks
 // up.  A thread per hidden unit; grid = (rows, Hp / 128).
-static __global__ void __launch_bounds__(128) lstm_cell_kernel(tc::TcEpiLstm e, const float* __restrict__ pre, const float* __restrict__ feed, int Hp) {
+static __global__ void __launch_bounds__(128) lstm_cell_kernel(tc::TcEpiLstm e, const float* __restrict__ pre, const float* __restrict__ feed,
+                                                               int Hp) {
   tc::pdl_launch_dependents();
   tc::pdl_wait();
   const int row = blockIdx.x, col = (blockIdx.y * 128 + threadIdx.x) * 4;
