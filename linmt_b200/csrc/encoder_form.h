@@ -44,20 +44,27 @@ inline EncoderForm encoder_form(const EncoderModel& m, int n, int S) {
 }
 
 // Whether the layers of EncoderForm::kLayers run side by side all the same: the products of few sentences in CTAs of half an SM that
-// leave room for the other layers'.  Encoder and one scored word, ms, layer by layer / so: 4 x 1000 1 sentence of 16, 32 and 80 words
-// 0.59 / 0.61, 0.98 / 0.99, 1.98 / 1.51, 8 sentences 0.67 / 0.66, 1.01 / 0.86, 2.12 / 1.63, 32 0.79 / 0.76, 1.29 / 1.02, 2.85 / 2.02;
-// 5 x 512 1 0.56 / 0.53, 0.92 / 0.77, 2.00 / 1.46; of 8 words 2 to 8 % slower.  (Narrower models gain less in whole calls: 3 x 250
-// with 1 to 30 sentences of 40 words 2 to 3 % of a call, with 11 ragged ones it lost 2 %.)  Not where the batch shares the device with
-// others (`shared`), nor in one plane, which keeps its order of sums (see encoder_form).
-constexpr int kEncBesideWords = 20, kEncBesideHidden = 512;
-inline bool encoder_layers_beside(const EncoderModel& m, int S, bool shared) {
-  return m.split && m.members == 1 && m.layers > 1 && m.hp >= kEncBesideHidden && S >= kEncBesideWords && !shared;
+// leave room for the other layers'.  Encoder and two scored words, ms, layer by layer / so, at 20, 32 and 100 words: 4 x 1000 1 sentence
+// 0.71 / 0.66, 0.96 / 0.82, 2.42 / 1.82, 16 0.82 / 0.79, 1.10 / 1.01, 2.81 / 2.37, 48 (20 and 32 words) 1.13 / 0.98, 1.63 / 1.24; 5 x 768 4
+// 0.78 / 0.72, 1.07 / 0.92, 2.63 / 2.08; 2 x 512 4 0.34 / 0.33, 0.45 / 0.41, 1.04 / 0.86; of 8 words 2 to 8 % slower.  Not
+// * one sentence of a narrow model, until it is longer: its products are over before the next layer's start (2 x 512 20 words 0.333 /
+//   0.348, 32 0.437 / 0.454, 50 0.588 / 0.517);
+// * from 49 sentences on at 769 to 1024 units, where a layer's product fills the chip, in CTAs that leave no room (2 x 1000 64 sentences of 20
+//   and 50 words 0.726 / 0.745, 1.38 / 1.42; 4 x 1000 20 and 24 words 1.24 / 1.26, 1.44 / 1.42; 512, 768 and 1280 units gain 3 to 14 %);
+// * below 512 units (3 x 250 with 1 to 30 sentences of 40 words gained 2 to 3 % of a call, and lost 2 % with 11 ragged ones);
+// * where the batch shares the device with others (`shared`);
+// * in one plane, which keeps its order of sums (see encoder_form).
+constexpr int kEncBesideWords = 20, kEncBesideWordsOne = 40, kEncBesideHidden = 512, kEncRoomSentences = 48;
+inline bool encoder_layers_beside(const EncoderModel& m, int n, int S, bool shared) {
+  if (!m.split || m.members > 1 || m.layers < 2 || m.hp < kEncBesideHidden || shared) return false;
+  if (n > kEncRoomSentences && m.hp > 768 && m.hp <= 1024) return false;
+  return S >= (n == 1 && m.hp < 768 ? kEncBesideWordsOne : kEncBesideWords);
 }
 
-// Up to here the encoder's products of a position are shaped like a step's, so that the next one's weights are under way (4 x 1000, 32
-// positions: one sentence 4.77 -> 4.73 ms a call, eight 14.34 -> 14.16; 64: 0.2 to 2 % slower).  One plane: as above.
-constexpr int kEncRoomSentences = 48;
-inline bool encoder_leaves_room(const EncoderModel& m, int n) { return m.split && n <= kEncRoomSentences; }
+// Whether the encoder's products of a position are shaped like a step's, so that the next one's weights are under way: up to 48
+// sentences whose layers run side by side (4 x 1000, 20 words, ms as above with / without: 1 sentence 0.66 / 0.76, 40 0.96 / 1.08), up to 32
+// one layer after another (1 sentence 0.71 / 0.72; 40 of 10 words 0.73 / 0.70).  One plane: as above.
+inline bool encoder_leaves_room(const EncoderModel& m, int n, bool beside) { return m.split && n <= (beside ? kEncRoomSentences : kEncFew); }
 
 // Sentences that the layers' panels of a handle are made for: those of the forms that its batches, of at most max_batch
 // sentences and max_words words, can take.

@@ -192,11 +192,11 @@ int Engine::encoder_streams() {
 // Which form, and in which shapes: encoder_form.h.
 int Engine::run_encoder_tc(int n, int Smax) {
   const EncoderModel model{L, Hp, n_models, nt_ > 1};
-  stream_weights_ = false; beside_ = encoder_leaves_room(model, n);
+  const bool side = encoder_layers_beside(model, n, Smax, several_);
+  stream_weights_ = false; beside_ = encoder_leaves_room(model, n, side);
   if (enc_rows_)
     switch (encoder_form(model, n, Smax)) {
-      case EncoderForm::kLayers:
-        return encoder_layers_beside(model, Smax, several_) ? run_encoder_pipeline_tc(n, Smax, true) : run_encoder_layers_tc(n, Smax);
+      case EncoderForm::kLayers: return side ? run_encoder_pipeline_tc(n, Smax, true) : run_encoder_layers_tc(n, Smax);
       case EncoderForm::kPipelined: return run_encoder_pipeline_tc(n, Smax, false);
       case EncoderForm::kWavefront: break;
     }

@@ -9,6 +9,7 @@ int main() {
   int split, n, words, shared;
   while (std::scanf("%d %d %d %d %d %d %d", &m.layers, &m.hp, &m.members, &split, &n, &words, &shared) == 7) {
     m.split = split != 0;
-    std::printf("%d %d\n", linmt::encoder_layers_beside(m, words, shared != 0), linmt::encoder_leaves_room(m, n));
+    const bool beside = linmt::encoder_layers_beside(m, n, words, shared != 0);
+    std::printf("%d %d\n", beside, linmt::encoder_leaves_room(m, n, beside));
   }
 }
