@@ -183,8 +183,18 @@ typedef struct linmt_trace {
  *   out_score [n][nbest]
  *   out_vit   [n][nbest][max_len]  viterbi alignment per position, may be NULL
  *   out_align [n][nbest][max_len][max_src_len]  dense alignments, may be NULL (print_info only)
- * Sentences are processed in device batches of at most max_batch.  A call of several device batches of up to 512 beam slots
- * runs two or three of them at once, each with state of its own; it is made at the first such call and kept. */
+ * Sentences are processed in device batches of at most max_batch.  A call of a single model that has several device batches of up to
+ * 512 beam slots runs two or three of them at once on every device (linmt_score_batch, in batches of up to 512 sentences, and
+ * linmt_decode_file do the same), each on an engine with the handle's weights and state of its own:
+ *   - One or two further engines per device are made by the first such call, beside its first batches, and kept until the
+ *     handle is destroyed.  That call is up to 1.5 ms longer than without them, later ones are shorter (64 sentences a batch,
+ *     4 x 1000 / 30k: 300 greedily 46.5 ms one after another, 34 to 36 the first call, 32 after it).
+ *   - An engine takes 0.1 (2 x 128, greedily) to 0.7 GB of device memory (4 x 1000 / 30k, beam 12), and 0.2 GB more where it
+ *     scores.  None is made that takes more than 3 GB or a quarter of what the device has free, and a call that is refused memory
+ *     gives them up and runs on the handle's own engines.
+ *   - In fp32 precision the products of batches that share a device add in another order: the last bits of a score (4e-7 of it)
+ *     go by whether the call has one device batch or several that run at once.  Repeated calls give the same bits.  bf16
+ *     results do not depend on it. */
 int linmt_decode_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, int32_t n,
                        const int32_t* steps, int32_t max_len, int32_t* out_tok, int32_t* out_len,
                        float* out_score, int32_t* out_vit, float* out_align, const linmt_trace* trace);
@@ -232,7 +242,7 @@ const char* linmt_translate(linmt_engine* e, const char* sentence);
  *   tgt_ids, tgt_off  target token ids per sentence WITHOUT START / EOS
  *   out_logprob [n]   sum over the m_i tokens and the closing EOS of log p(token | source, prefix)
  *   out_token_logp    optional [n][max_tgt + 1]: the per-token terms (EOS last), zero padded
- * Every sentence needs 1 <= m_i <= max_steps. */
+ * Every sentence needs 1 <= m_i <= max_steps.  Several device batches run at once: see linmt_decode_batch. */
 int linmt_score_batch(linmt_engine* e, const int32_t* src_ids, const int32_t* src_off, const int32_t* tgt_ids,
                       const int32_t* tgt_off, int32_t n, float* out_logprob, float* out_token_logp, int32_t max_tgt);
 
@@ -248,7 +258,7 @@ int linmt_read_model_file(const char* path, linmt_model_desc* desc, float* blob,
  * EnsembleFactory::DecodeFile (src/decoder.h:1702-1776), Decoder::OutputKBestHypotheses
  * (src/decoder.h:529-699) and InputFilePreprocess::UnintFile
  * (src/input_file_preprocess.cc:1485-1572).  Needs an engine created from a config file; sentences
- * are decoded in length-sorted batches of --batch-size. */
+ * are decoded in length-sorted batches of --batch-size, several at once: see linmt_decode_batch. */
 int linmt_decode_file(linmt_engine* e, const char* in_path, const char* out_path);
 
 /* ------------------------------------------------------------------------------------
