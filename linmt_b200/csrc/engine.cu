@@ -1095,10 +1095,12 @@ int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const s
 
 // Few rows are a chain of launches in which most of the chip waits, for the next launch or for weights: the device batches of a call
 // that has several run at once, a stream and a host thread each.  ms a batch of 64 sentences of 20 to 30 words with 1, 2, 3 at
-// once: 4 x 1000 / 30k 64 rows 6.4, 5.3, 5.3; 32 rows 5.3, 3.6, 3.3; 256 rows 9.3, 7.8, 7.9; 768 rows 15.2, 14.8, 15.0; in bf16 64 rows
-// 5.0, 3.9, 3.8; scoring 128 sentences in bf16 3.2, 2.3, 2.4; 3 x 250 / 5k 256 rows 4.4, 2.6, 2.0.  (Ensembles' members run side by side
-// already.  Where events time the kernels, one after another; and where an engine takes more than 3 GB beside the weights, which
-// are shared: states, panels and logits of a batch, records of alignments.)
+// once: 4 x 1000 / 30k 64 rows 6.4, 5.3, 5.3; 32 rows 5.3, 3.6, 3.3; 256 rows 9.3, 7.8, 7.9; 768 rows 15.2, 14.8, 15.0; 3 x 250 / 5k 256 rows
+// 4.4, 2.6, 2.0.  In bf16 (shapes of one batch by itself), ms of five batches one after another / at once: 64 rows 13.9 / 10.8, 512 rows
+// 21.6 / 19.9, scoring 64 rows 12.3 / 10.0.  Two, three and five batches of 8 to 512 rows of 2 x 128, 3 x 250, 2 x 512, 4 x 1000 and 4 x 1024 /
+// 80k, both precisions, decoding and scoring: 1 to 60 % shorter.  (Ensembles' members run side by side already.  Where events time the
+// kernels, one after another; and where an engine takes more than 3 GB beside the weights, which are shared: states, panels and
+// logits of a batch, records of alignments.)
 int Engine::lanes_for(int rows) const {
   if (!lanes_ || !use_tc_ || n_models > 1 || kernel_timing || rows > 512 || lane_bytes_ > ((size_t)3 << 30)) return 1;
   return rows <= 64 || !step_streams(false, rows) ? 3 : 2;
