@@ -86,7 +86,7 @@ int Engine::regrow(T** p, size_t count, size_t* cap) {
   } while (0)
 
 Engine::~Engine() {
-  if (stream) { cudaSetDevice(opt.device); cudaStreamSynchronize(stream); }
+  if (main_stream_) { cudaSetDevice(opt.device); cudaStreamSynchronize(main_stream_); }
   for (void* p : allocs_)
     if (!arena_ || static_cast<char*>(p) < arena_ || static_cast<char*>(p) >= arena_ + arena_used_) cudaFree(p);
   if (arena_) cudaFree(arena_);
@@ -101,7 +101,26 @@ Engine::~Engine() {
   for (auto e : mem_events_) if (e) cudaEventDestroy(e);
   for (auto st : mem_streams_) if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
   for (auto st : enc_streams_) if (st) { cudaStreamSynchronize(st); cudaStreamDestroy(st); }
-  if (stream) cudaStreamDestroy(stream);
+  if (main_stream_) cudaStreamDestroy(main_stream_);
+}
+
+void Engine::recover() {
+  if (!main_stream_) return;
+  cudaSetDevice(opt.device);
+  cudaDeviceSynchronize();
+  stream = main_stream_;
+  ws_part_ = 0; ws_parts_ = 1; plan_parts_ = 0;
+  pdl_gemm_ = beside_ = want_late_ = got_late_ = false;
+}
+
+int Engine::guarded(const std::function<int()>& call) {
+  try {
+    return call();
+  } catch (const std::exception& e) {
+    recover();
+    try { err = std::string("out of host memory: ") + e.what(); } catch (...) {}
+    return LINMT_ENOMEM;
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -374,7 +393,8 @@ int Engine::init_state(const Engine* of, const float* const* blobs) {
   int cc_major = 0;
   CK(cudaDeviceGetAttribute(&cc_major, cudaDevAttrComputeCapabilityMajor, o.device));
   if (cc_major != 10) return fail(LINMT_ECUDA, "this library is built for sm_100a (B200) only");
-  CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&main_stream_, cudaStreamNonBlocking));
+  stream = main_stream_;
   CK(cudaEventCreate(&ev0_)); CK(cudaEventCreate(&ev1_));
   CK(cudaDeviceGetAttribute(&n_sm_, cudaDevAttrMultiProcessorCount, o.device));
   DA(d_tc_err_, 1);
@@ -888,7 +908,7 @@ int Engine::decode_chunk(const HostJob& jb, const int* idx, int cn, const linmt_
   CK(cudaMemcpyAsync(d_ids_, h_stage_, n_ids * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
   int rc = decode_core(d_ids_, off.data(), cn, st.data(), jb.max_len, d_tok, d_len, d_score, jb.out_vit ? d_vit : nullptr,
                        jb.out_align ? d_align : nullptr, td, Tm_all);
-  if (rc) { cudaStreamSynchronize(stream); return rc; }
+  if (rc) { recover(); return rc; }
   CK(cudaMemcpyAsync(h_stage_, d_out_, n_out * 4, cudaMemcpyDeviceToHost, stream));
   if ((rc = finish_timing())) return rc;
   const int32_t* h = h_stage_;
@@ -1025,7 +1045,7 @@ int Engine::score_chunk(const ScoreJob& jb, const int* idx, int cn) {
   kt_used_ = 0; rec_flops_ = 0.0;
   float* d_logp = reinterpret_cast<float*>(score_io_ + n_up);
   int rc = score_core_tc(cn, Smax, n_act, score_io_ + n_ids, score_io_ + n_ids + (size_t)steps * cn, d_logp);
-  if (rc) { cudaStreamSynchronize(stream); return rc; }
+  if (rc) { recover(); return rc; }
   if ((rc = kt(KC_END))) return rc;
   CK(cudaEventRecord(ev1_, stream));
   const float* h_logp = reinterpret_cast<const float*>(h_stage_ + n_up);
@@ -1047,15 +1067,7 @@ int Engine::score_chunk(const ScoreJob& jb, const int* idx, int cn) {
 int run_on_engines(linmt_engine* h, const std::vector<Engine*>& workers, const std::vector<int>& order, const std::function<int(Engine&, int)>& work) {
   const int ne = (int)workers.size();
   // (no exception leaves a thread, nor this function while its threads run)
-  auto job = [&](Engine& g, int item) -> int {
-    try {
-      return item < 0 ? g.ready() : work(g, item);
-    } catch (const std::exception& e) {
-      if (g.stream) cudaStreamSynchronize(g.stream);      // (copies from staging that the next batch reuses may be under way)
-      try { g.err = std::string("out of host memory: ") + e.what(); } catch (...) {}
-      return LINMT_ENOMEM;
-    }
-  };
+  auto job = [&](Engine& g, int item) { return g.guarded([&] { return item < 0 ? g.ready() : work(g, item); }); };
   if (ne == 1 || order.size() <= 1) {
     for (int item : order)
       if (int rc = job(h->eng, item)) return rc;
@@ -1151,7 +1163,7 @@ std::vector<Engine*> linmt_engine::workers(size_t items, int rows, bool first_de
 }
 
 int linmt_engine::with_lanes(const std::function<int()>& call) {
-  const int rc = call();
+  const int rc = eng.guarded(call);
   if (rc != LINMT_ENOMEM || lanes.empty()) return rc;
   for (const auto& l : lanes) {      // (their counters stay the handle's)
     eng.stats.kernel_launches += l->stats.kernel_launches;
@@ -1161,7 +1173,7 @@ int linmt_engine::with_lanes(const std::function<int()>& call) {
   }
   lanes.clear();
   no_more_lanes = true;
-  return call();
+  return eng.guarded(call);
 }
 
 static std::string g_create_error;

@@ -95,6 +95,10 @@ class Engine {
   // Those are made by `ready`, in the thread that is going to use them; one that could not be is `broken` and of no use.
   explicit Engine(const Engine* of) : lane_of_(of), broken_(true) { opt = of->opt; }
   int ready();
+  // After an exception or an error in the middle of a call: waits for what is under way, and the engine is as between two calls.
+  void recover();
+  // Runs `call`; an exception is its error (for host memory).
+  int guarded(const std::function<int()>& call);
   bool planned() const { return lane_of_ != nullptr; }
   bool broken() const { return broken_ && !lane_of_; }
   // While one lives, the engine's device batch is one of a call's that run at once on a device, and its products leave room for others.
@@ -204,6 +208,7 @@ class Engine {
   int tc_gemm(const tc::Planes& A, int a_col0, int a_rows_cap, const tc::Planes& W, int M, int N, int K, const Epi& e, int nt = 0, int drain = 0, int x_row0 = 0);
 
   bool use_tc_ = false;
+  cudaStream_t main_stream_ = nullptr;     // `stream`, but for a layer's or a member's work
   // encoder wavefront: one stream per layer, a small ring of events per layer
   std::vector<cudaStream_t> enc_streams_;
   std::vector<std::vector<cudaEvent_t>> enc_events_;

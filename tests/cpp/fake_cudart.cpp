@@ -54,6 +54,7 @@ cudaError_t copy(void* d, const void* s, size_t bytes, cudaMemcpyKind kind) {
 cudaError_t launch(const void* f, cudaStream_t s) {
   std::lock_guard<std::recursive_mutex> lock(mu);
   if (!s) ++v("legacy");
+  if (v("throw_launch") && --v("throw_launch") == 0) throw std::bad_alloc();      // (as `throw_at`)
   ++launched[names[f]];
   if (v("unordered")) ++v("races");     // a fill of the legacy stream, which this launch does not wait for, is under way
   return cudaSuccess;

@@ -373,3 +373,28 @@ for L, H, most in ((2, 256, 60), (3, 768, 60), (3, 840, 48)):
         assert ahead(dec, bound, beam) and not ahead(dec, bound + 1, beam), (L, H, beam)
         dec.close()
 """)
+
+
+def test_host_memory_that_runs_out_between_two_launches(child):
+    """Wherever in a call, on a layer's or a member's stream among them: that call fails for memory, and the next one runs as ever."""
+    child("""
+D5 = synth.ModelDesc(3, 512, 3000, 300, 1)
+long = synth.make_sentences(2, 20, 20, D5.Vs, 1.1, 3, lambda s: 3)
+def ensemble(): return decoder.Decoder(D, [BLOB, synth.make_blob(D, 2)], **OPT)
+def side_by_side(): return decoder.Decoder(D5, [synth.make_blob(D5, 1)], beam=2, max_batch=4, max_src_len=20, max_steps=8)
+for new, s in ((side_by_side, long), (lambda: make(gemm_path="tensor3"), some(2)), (ensemble, some(2))):
+    dec = new()
+    dec.decode(s)
+    before = dec.stats()["kernel_launches"]
+    dec.decode(s)
+    count = dec.stats()["kernel_launches"] - before
+    assert count > 20
+    for n in list(range(1, count, 3)) + [count]:
+        put("throw_launch", n)
+        assert no_memory(lambda: dec.decode(s), 10**9), n
+        before = dec.stats()["kernel_launches"]
+        dec.decode(s)
+        assert dec.stats()["kernel_launches"] - before == count, n
+    dec.close()
+assert get("used") == 0
+""")
